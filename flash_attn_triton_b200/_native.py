@@ -144,6 +144,24 @@ def lib():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The C++ host path (csrc/host_ext.cpp) driving the loaded library; raises if it has not been built."""
+    global _host
+    if _host is None:
+        l = lib()
+        try:
+            from . import _fa_host
+        except ImportError as e:
+            raise RuntimeError("the host extension is missing or does not load: build it with "
+                               f"`python -m flash_attn_triton_b200.build` ({e})") from e
+        _fa_host.init({name: C.cast(getattr(l, name), C.c_void_p).value for name in EXPORTS}, check)
+        _host = _fa_host
+    return _host
+
+
 class DeviceWaitError(RuntimeError):
     """A bounded wait inside a kernel ran out earlier on this device (FA_ERR_DEVICE_WAIT): the
     kernel that hit it left its outputs incomplete and the tcgen05 kernels refuse to launch

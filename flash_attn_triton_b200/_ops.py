@@ -1,4 +1,5 @@
-"""Operator layer: torch.autograd.Function wrappers that fill the C-ABI argument blocks.
+"""Operator layer: the differentiable attention calls (autograd nodes, allocation and argument blocks in
+C++, csrc/host_ext.cpp) and the C-ABI argument blocks of the calls that are not on a hot host path.
 
 Takes the place of the reference's `_attention`, `_attention_varlen` and
 `_attention_int8` autograd functions (flash_attn_triton/triton_kernel/attention_kernel.py:1158-1198,
@@ -35,9 +36,6 @@ class Features:
         self.bias, self.dropout_p, self.seed, self.row_stride = bias, float(dropout_p), int(seed), int(row_stride)
         self.seqused_q, self.seqused_k = seqused_q, seqused_k
 
-    def tensors(self):
-        return [t for t in (self.bias, self.seqused_q, self.seqused_k) if t is not None]
-
     def fill(self, a):
         if self.bias is not None:
             a.attn_bias = self.bias.data_ptr()
@@ -48,6 +46,7 @@ class Features:
 
 
 _NO_FEATURES = Features()
+_SEPARATE, PACK_QKV, PACK_KV = 0, 1, 2     # how the inputs of a call are packed
 
 
 def _fill_common(a, q, k, v, o, dims_q, dims_k, *, batch, sq, sk, hq, hkv, d, scale, causal, wl,
@@ -81,25 +80,30 @@ _BHSD = (0, 2, 1)      # (batch, heads, seq, dim)
 _THD = (None, 0, 1)    # packed (tokens, heads, dim)
 
 
+def dense_attention(q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl, layout, feat=None,
+                    want_lse=False):
+    """q (B,Sq,Hq,D), k/v (B,Sk,Hkv,D) ["bshd"] or head-major ["bhsd"] -> o like q (and the base-2 LSE
+    (B,Hq,Sq) when asked for); differentiable in q, k and v."""
+    f = feat or _NO_FEATURES
+    return N.host().dense(_SEPARATE, -1, q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl,
+                          layout == "bhsd", f.bias, f.dropout_p, f.seed, f.row_stride, want_lse)
+
+
+def dense_attention_packed(packing, dim, tensors, scale, causal, wl, wr, softcap, alibi, feat=None):
+    """The same for packed inputs: tensors = (qkv,) with packing QKV or (q, kv) with KV, the packed
+    dimension `dim`.  Gradients are written straight into packed tensors."""
+    f = feat or _NO_FEATURES
+    return N.host().dense(packing, dim, *tensors, scale, causal, wl, wr, softcap, alibi, 0, N.IMPL_AUTO, False,
+                          f.bias, f.dropout_p, f.seed, f.row_stride, False)
+
+
 def dense_forward(q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl, layout,
                   want_lse, feat=None):
-    dims = _BSHD if layout == "bshd" else _BHSD
-    B = q.shape[0]
-    Sq, Hq = q.shape[dims[1]], q.shape[dims[2]]
-    Sk, Hkv = k.shape[dims[1]], k.shape[dims[2]]
-    D = q.shape[-1]
+    """(o, base-2 LSE or None, the tensors as handed to the kernels), no autograd."""
     q, k, v = _prep(q), _prep(k), _prep(v)
-    o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    lse = torch.empty((B, Hq, Sq), dtype=torch.float32, device=q.device) if want_lse else None
-    a = N.AttnArgs()
-    _fill_common(a, q, k, v, o, dims, dims, batch=B, sq=Sq, sk=Sk, hq=Hq, hkv=Hkv, d=D,
-                 scale=scale, causal=causal, wl=wl, wr=wr, softcap=softcap, alibi=alibi,
-                 q_pos_offset=q_pos_offset, impl=impl, feat=feat)
-    if lse is not None:
-        a.lse2 = lse.data_ptr()
-        a.lse_stride = N._I64x3(Hq * Sq, 1, Sq)
-    with torch.cuda.device(q.device):
-        N.check(N.lib().fa_fwd(C.byref(a), N.stream_ptr(q.device)), "fa_fwd")
+    with torch.no_grad():
+        r = dense_attention(q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl, layout, feat, want_lse)
+    o, lse = r if want_lse else (r, None)
     return o, lse, (q, k, v)
 
 
@@ -128,81 +132,29 @@ def dense_probs(q, k, v, lse, scale, causal, wl, wr, softcap, alibi, q_pos_offse
 
 def dense_backward(q, k, v, o, lse, dout, scale, causal, wl, wr, softcap, alibi, q_pos_offset,
                    impl, layout, feat=None):
-    dims = _BSHD if layout == "bshd" else _BHSD
-    B = q.shape[0]
-    Sq, Hq = q.shape[dims[1]], q.shape[dims[2]]
-    Sk, Hkv = k.shape[dims[1]], k.shape[dims[2]]
-    D = q.shape[-1]
-    dout = _prep(dout)
-    dq = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    dk = torch.empty(k.shape, dtype=k.dtype, device=k.device)
-    dv = torch.empty(v.shape, dtype=v.dtype, device=v.device)
-    delta = torch.empty_like(lse)
-    a = N.AttnArgs()
-    _fill_common(a, q, k, v, o, dims, dims, batch=B, sq=Sq, sk=Sk, hq=Hq, hkv=Hkv, d=D,
-                 scale=scale, causal=causal, wl=wl, wr=wr, softcap=softcap, alibi=alibi,
-                 q_pos_offset=q_pos_offset, impl=impl, feat=feat)
-    a.lse2 = lse.data_ptr()
-    a.lse_stride = N._I64x3(Hq * Sq, 1, Sq)
-    a.dout, a.do_stride = dout.data_ptr(), N.strides3(dout, dims)
-    a.delta = delta.data_ptr()
-    a.dq, a.dk, a.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    a.dq_stride, a.dk_stride, a.dv_stride = (N.strides3(dq, dims), N.strides3(dk, dims),
-                                             N.strides3(dv, dims))
-    st = N.stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        L = N.lib()
-        N.check(L.fa_bwd_preprocess(C.byref(a), st), "fa_bwd_preprocess")
-        N.check(L.fa_bwd_dq(C.byref(a), st), "fa_bwd_dq")
-        N.check(L.fa_bwd_dkdv(C.byref(a), st), "fa_bwd_dkdv")
-    return dq, dk, dv
+    f = feat or _NO_FEATURES
+    return N.host().backward(_SEPARATE, -1, q, k, v, o, lse, dout, 1 if layout == "bhsd" else 0, None, None, 0, 0, scale,
+                             causal, wl, wr, softcap, alibi, q_pos_offset, impl, f.bias, f.dropout_p, f.seed,
+                             f.row_stride, None, None)
 
 
-class DenseAttention(torch.autograd.Function):
-    """q (B,Sq,Hq,D), k/v (B,Sk,Hkv,D) ["bshd"] or head-major ["bhsd"]; returns o like q."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl, layout, feat=None,
-                want_lse=False):
-        need = any(t.requires_grad for t in (q, k, v))
-        o, lse, (q, k, v) = dense_forward(q, k, v, scale, causal, wl, wr, softcap, alibi,
-                                          q_pos_offset, impl, layout, want_lse=need or want_lse, feat=feat)
-        if need:
-            ctx.save_for_backward(q, k, v, o, lse, alibi if alibi is not None else q.new_empty(0))
-            ctx.cfg = (scale, causal, wl, wr, softcap, alibi is not None, q_pos_offset, impl, layout)
-            ctx.feat = feat
-        if want_lse:
-            ctx.mark_non_differentiable(lse)
-            return o, lse
-        return o
-
-    @staticmethod
-    def backward(ctx, dout, *unused):
-        q, k, v, o, lse, alibi = ctx.saved_tensors
-        scale, causal, wl, wr, softcap, has_alibi, off, impl, layout = ctx.cfg
-        dq, dk, dv = dense_backward(q, k, v, o, lse, dout, scale, causal, wl, wr, softcap,
-                                    alibi if has_alibi else None, off, impl, layout, feat=ctx.feat)
-        return (dq, dk, dv) + (None,) * 11
+def varlen_attention(packing, dim, tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
+                     feat=None, want_lse=False):
+    """Packed sequences: tensors = (q (Tq,Hq,D), k, v (Tk,Hkv,D)), or packed as in dense_attention_packed; int32
+    cu_seqlens on the device; differentiable."""
+    f = feat or _NO_FEATURES
+    return N.host().varlen(packing, dim, *tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
+                           f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse)
 
 
 def varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
                    want_lse, feat=None):
-    Tq, Hq, D = q.shape
-    Hkv = k.shape[1]
-    batch = cu_q.numel() - 1
+    """(o, base-2 LSE (Hq, Tq) or None, the tensors as handed to the kernels), no autograd."""
     q, k, v = _prep(q), _prep(k), _prep(v)
-    o = torch.empty(q.shape, dtype=q.dtype, device=q.device)
-    # base-2 LSE laid out (heads, tokens): consecutive rows of a head are contiguous
-    lse = torch.empty((Hq, Tq), dtype=torch.float32, device=q.device) if want_lse else None
-    a = N.AttnArgs()
-    _fill_common(a, q, k, v, o, _THD, _THD, batch=batch, sq=max_q, sk=max_k, hq=Hq, hkv=Hkv, d=D,
-                 scale=scale, causal=causal, wl=wl, wr=wr, softcap=softcap, alibi=alibi,
-                 q_pos_offset=0, impl=impl, cu_q=cu_q, cu_k=cu_k, feat=feat)
-    if lse is not None:
-        a.lse2 = lse.data_ptr()
-        a.lse_stride = N._I64x3(0, 1, Tq)
-    with torch.cuda.device(q.device):
-        N.check(N.lib().fa_varlen_fwd(C.byref(a), N.stream_ptr(q.device)), "fa_varlen_fwd")
+    with torch.no_grad():
+        r = varlen_attention(_SEPARATE, -1, (q, k, v), cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi,
+                             impl, feat, want_lse)
+    o, lse = r if want_lse else (r, None)
     return o, lse, (q, k, v)
 
 
@@ -228,64 +180,9 @@ def varlen_probs(q, k, v, lse, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, 
 
 def varlen_backward(q, k, v, o, lse, dout, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr,
                     softcap, alibi, impl, feat=None):
-    Tq, Hq, D = q.shape
-    Hkv = k.shape[1]
-    batch = cu_q.numel() - 1
-    dout = _prep(dout)
-    # rows past cu_seqlens[-1] or past a sequence's used length never get a writer: start from zero
-    # when the packed tensors are not fully covered
-    partial = feat is not None and (feat.seqused_q is not None or feat.seqused_k is not None)
-    alloc = torch.zeros if partial else torch.empty
-    dq = alloc(q.shape, dtype=q.dtype, device=q.device)
-    dk = alloc(k.shape, dtype=k.dtype, device=k.device)
-    dv = alloc(v.shape, dtype=v.dtype, device=v.device)
-    delta = torch.empty_like(lse)
-    a = N.AttnArgs()
-    _fill_common(a, q, k, v, o, _THD, _THD, batch=batch, sq=max_q, sk=max_k, hq=Hq, hkv=Hkv, d=D,
-                 scale=scale, causal=causal, wl=wl, wr=wr, softcap=softcap, alibi=alibi,
-                 q_pos_offset=0, impl=impl, cu_q=cu_q, cu_k=cu_k, feat=feat)
-    a.lse2 = lse.data_ptr()
-    a.lse_stride = N._I64x3(0, 1, Tq)
-    a.dout, a.do_stride = dout.data_ptr(), N.strides3(dout, _THD)
-    a.delta = delta.data_ptr()
-    a.dq, a.dk, a.dv = dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    a.dq_stride, a.dk_stride, a.dv_stride = (N.strides3(dq, _THD), N.strides3(dk, _THD),
-                                             N.strides3(dv, _THD))
-    st = N.stream_ptr(q.device)
-    with torch.cuda.device(q.device):
-        L = N.lib()
-        N.check(L.fa_bwd_preprocess(C.byref(a), st), "fa_bwd_preprocess")
-        N.check(L.fa_varlen_bwd_dq(C.byref(a), st), "fa_varlen_bwd_dq")
-        N.check(L.fa_varlen_bwd_dkdv(C.byref(a), st), "fa_varlen_bwd_dkdv")
-    return dq, dk, dv
-
-
-class VarlenAttention(torch.autograd.Function):
-    """Packed q (Tq,Hq,D), k/v (Tk,Hkv,D) with int32 cu_seqlens on the device."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl, feat=None,
-                want_lse=False):
-        need = any(t.requires_grad for t in (q, k, v))
-        o, lse, (q, k, v) = varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl,
-                                           wr, softcap, alibi, impl, want_lse=need or want_lse, feat=feat)
-        if need:
-            ctx.save_for_backward(q, k, v, o, lse, cu_q, cu_k,
-                                  alibi if alibi is not None else q.new_empty(0))
-            ctx.cfg = (max_q, max_k, scale, causal, wl, wr, softcap, alibi is not None, impl)
-            ctx.feat = feat
-        if want_lse:
-            ctx.mark_non_differentiable(lse)
-            return o, lse
-        return o
-
-    @staticmethod
-    def backward(ctx, dout, *unused):
-        q, k, v, o, lse, cu_q, cu_k, alibi = ctx.saved_tensors
-        max_q, max_k, scale, causal, wl, wr, softcap, has_alibi, impl = ctx.cfg
-        dq, dk, dv = varlen_backward(q, k, v, o, lse, dout, cu_q, cu_k, max_q, max_k, scale,
-                                     causal, wl, wr, softcap, alibi if has_alibi else None, impl, feat=ctx.feat)
-        return (dq, dk, dv) + (None,) * 13
+    f = feat or _NO_FEATURES
+    return N.host().backward(_SEPARATE, -1, q, k, v, o, lse, dout, 2, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr,
+                             softcap, alibi, 0, impl, None, f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k)
 
 
 # ----------------------------------------------------------------------------------------
@@ -330,32 +227,9 @@ def int8_forward(q, k, v, causal, scale, impl=N.IMPL_AUTO, k_valid=0, q_pos_offs
     return o, lse, k8, s_k
 
 
-class Int8Attention(torch.autograd.Function):
+def int8_attention(q, k, v, causal, scale, impl, k_valid=0, q_pos_offset=0):
     """INT8-QK^T forward, fp16 backward (attention_kernel_int8.py:220-267).  [B,H,S,D]."""
-
-    @staticmethod
-    def forward(ctx, q, k, v, causal, scale, impl, k_valid=0, q_pos_offset=0):
-        o, lse, _, _ = int8_forward(q, k, v, causal, scale, impl, k_valid, q_pos_offset)
-        ctx.save_for_backward(q, k, v, o, lse)
-        ctx.cfg = (causal, scale, k_valid, q_pos_offset)
-        return o
-
-    @staticmethod
-    def backward(ctx, dout):
-        q, k, v, o, lse = ctx.saved_tensors
-        causal, scale, k_valid, off = ctx.cfg
-        S = k.shape[2]
-        if k_valid and k_valid < S:
-            # padded call: the keys past k_valid take no part; their gradients are zero
-            dq, dk_s, dv_s = dense_backward(q, k[:, :, :k_valid], v[:, :, :k_valid], o, lse, dout, scale,
-                                            causal, -1, -1, 0.0, None, off, N.IMPL_AUTO, "bhsd")
-            dk, dv = torch.zeros_like(k), torch.zeros_like(v)
-            dk[:, :, :k_valid] = dk_s
-            dv[:, :, :k_valid] = dv_s
-        else:
-            dq, dk, dv = dense_backward(q, k, v, o, lse, dout, scale, causal, -1, -1, 0.0, None, off,
-                                        N.IMPL_AUTO, "bhsd")
-        return dq, dk, dv, None, None, None, None, None
+    return N.host().int8(q, k, v, causal, scale, impl, k_valid, q_pos_offset)
 
 
 # ----------------------------------------------------------------------------------------

@@ -1,4 +1,5 @@
-"""Compile csrc/*.cu for sm_100a into libfa_b200.so next to this file.
+"""Compile csrc/*.cu for sm_100a into libfa_b200.so next to this file, and csrc/host_ext.cpp (the host
+path between PyTorch and that library) into _fa_host.so.
 
     python -m flash_attn_triton_b200.build [--force] [--verbose]
 
@@ -52,11 +53,35 @@ def _compile(src, defs, force, verbose):
     return src, r.stderr if verbose else "", True
 
 
+def build_host(force: bool = False) -> str:
+    """The host extension: plain C++ against PyTorch's headers, no device code."""
+    import sysconfig
+
+    import torch
+    src, out = os.path.join(CSRC, "host_ext.cpp"), os.path.join(HERE, "_fa_host.so")
+    header = os.path.join(os.path.dirname(HERE), "include", "fa_b200.h")
+    if not force and os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(f) for f in (src, header, __file__)):
+        return out
+    t = os.path.dirname(os.path.abspath(torch.__file__))
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{d}" for d in (t + "/include", t + "/include/torch/csrc/api/include", "/usr/local/cuda/include",
+                                sysconfig.get_paths()["include"])),
+           src, "-o", out, f"-L{t}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",
+           f"-Wl,-rpath,{t}/lib"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for host_ext.cpp:\n{r.stdout}\n{r.stderr}")
+    return out
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     os.makedirs(OBJ, exist_ok=True)
     srcs = _sources()
     defs = os.environ.get("FA_BUILD_DEFS", "").split()
     rebuilt = False
+    if not TAG:
+        build_host(force)
     with cf.ThreadPoolExecutor(max_workers=min(8, len(srcs))) as ex:
         for src, log, did in ex.map(lambda s: _compile(s, defs, force, verbose), srcs):
             rebuilt |= did

@@ -1,0 +1,568 @@
+// Host path between PyTorch and the C ABI: allocation of outputs, argument blocks, autograd nodes
+// and stream lookup in C++.
+//
+// A small attention call is bounded by the host, not by the GPU: the same steps as
+// torch.autograd.Function classes with ctypes argument blocks cost about 25 us per forward and
+// 70 us per backward on the host, against kernels of 5-20 us.  The kernels themselves are reached
+// through the addresses of libfa_b200.so's C functions, handed over once by init(), so that any build
+// of that library can be driven.
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/utils/pybind.h>
+#include <ATen/ATen.h>
+#include <ATen/core/LegacyTypeDispatch.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <string.h>
+
+#include "../../include/fa_b200.h"
+
+namespace {
+
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+// ---------------------------------------------------------------------------------------
+// the C ABI
+// ---------------------------------------------------------------------------------------
+typedef int (*AttnFn)(const fa_attn_args*, void*);
+struct Abi {
+  AttnFn fwd, varlen_fwd, preprocess, bwd_dq, bwd_dkdv, varlen_bwd_dq, varlen_bwd_dkdv;
+  int (*quantize_k)(const void*, int8_t*, float*, int64_t, int32_t, int32_t, void*);
+  int (*fwd_int8)(const fa_int8_args*, void*);
+  PyObject* check;   // _native.check(status, what): raises the Python exception of a status
+};
+Abi g_abi = {};
+
+// Raises the Python exception of a non-zero status, from whichever thread runs the call.
+void check(int status, const char* what) {
+  if (status == 0) return;
+  pybind11::gil_scoped_acquire gil;
+  PyObject* r = PyObject_CallFunction(g_abi.check, "is", status, what);
+  Py_XDECREF(r);
+  if (r == nullptr) {
+    python_error e;
+    e.persist();
+    throw std::move(e);
+  }
+  TORCH_CHECK(false, what, " failed (status ", status, ")");
+}
+
+// ---------------------------------------------------------------------------------------
+// tensors as the kernels see them
+// ---------------------------------------------------------------------------------------
+enum Layout { kBSHD = 0, kBHSD = 1, kTHD = 2 };
+enum Packing { kSeparate = 0, kQKV = 1, kKV = 2 };
+
+// unit inner stride, 16-byte aligned rows
+bool kernel_ready(const Tensor& t) {
+  const auto st = t.strides();
+  const size_t n = st.size();
+  if (n == 0 || st[n - 1] != 1 || (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0) return false;
+  for (size_t i = 0; i + 1 < n; ++i)
+    if (st[i] % 8 != 0) return false;
+  return true;
+}
+Tensor prep(const Tensor& t) { return kernel_ready(t) ? t : t.contiguous(); }
+
+struct View {
+  char* p;
+  int64_t stride[3];                 // batch, row, head
+  int64_t batch, rows, heads, dim;
+};
+
+// `packed` >= 0: dimension of t that holds q/k/v (or k/v), `which` the slice taken from it
+View view_of(const Tensor& t, Layout layout, int packed, int which) {
+  int64_t sz[4], st[4];
+  int n = 0;
+  for (int i = 0; i < t.dim(); ++i) {
+    if (i == packed) continue;
+    sz[n] = t.size(i);
+    st[n] = t.stride(i);
+    ++n;
+  }
+  View v;
+  v.p = static_cast<char*>(t.data_ptr());
+  if (packed >= 0) v.p += which * t.stride(packed) * t.element_size();
+  v.dim = sz[n - 1];
+  if (layout == kTHD) {
+    v.batch = 1; v.rows = sz[0]; v.heads = sz[1];
+    v.stride[0] = 0; v.stride[1] = st[0]; v.stride[2] = st[1];
+  } else {
+    const int r = layout == kBSHD ? 1 : 2, h = layout == kBSHD ? 2 : 1;
+    v.batch = sz[0]; v.rows = sz[r]; v.heads = sz[h];
+    v.stride[0] = st[0]; v.stride[1] = st[r]; v.stride[2] = st[h];
+  }
+  return v;
+}
+
+Tensor empty_cuda(at::IntArrayRef sizes, at::ScalarType dtype, const at::Device& dev) {
+  return Tensor(at::detail::empty_cuda(sizes, dtype, dev, std::nullopt));
+}
+
+// What a call is made with, beyond its tensors.
+struct Params {
+  Layout layout = kBSHD;
+  Packing packing = kSeparate;
+  int packed_dim = -1;
+  double scale = 1.0, softcap = 0.0;
+  int causal = 0, wl = -1, wr = -1, q_pos_offset = 0, impl = FA_IMPL_AUTO;
+  int max_q = 0, max_k = 0;          // packed sequences
+  int k_valid = 0;                   // keys used of each (batch, head); 0 = all (padded INT8 calls)
+  double dropout_p = 0.0;
+  uint64_t seed = 0;
+  int row_stride = 0;
+  // optional tensors
+  Tensor cu_q, cu_k, used_q, used_k, alibi, bias;
+};
+
+void split(const Params& c, const variable_list& in, View& q, View& k, View& v) {
+  switch (c.packing) {
+    case kSeparate:
+      q = view_of(in[0], c.layout, -1, 0); k = view_of(in[1], c.layout, -1, 0); v = view_of(in[2], c.layout, -1, 0);
+      break;
+    case kQKV:
+      q = view_of(in[0], c.layout, c.packed_dim, 0); k = view_of(in[0], c.layout, c.packed_dim, 1);
+      v = view_of(in[0], c.layout, c.packed_dim, 2);
+      break;
+    case kKV:
+      q = view_of(in[0], c.layout, -1, 0); k = view_of(in[1], c.layout, c.packed_dim, 0);
+      v = view_of(in[1], c.layout, c.packed_dim, 1);
+      break;
+  }
+  if (c.k_valid > 0) k.rows = v.rows = c.k_valid;
+}
+
+void set_strides(int64_t* dst, const View& v) { memcpy(dst, v.stride, sizeof(v.stride)); }
+
+void fill(fa_attn_args& a, const Params& c, const Tensor& first, const View& q, const View& k, const View& v,
+          const View& o, float* lse) {
+  memset(&a, 0, sizeof(a));
+  a.dtype = first.scalar_type() == at::kBFloat16 ? FA_BF16 : FA_F16;
+  TORCH_CHECK_VALUE(a.dtype == FA_BF16 || first.scalar_type() == at::kHalf, "unsupported dtype ", first.scalar_type());
+  a.device = first.device().index();
+  a.impl = c.impl;
+  const bool packed = c.layout == kTHD;
+  a.batch = packed ? (int)c.cu_q.numel() - 1 : (int)q.batch;
+  a.seqlen_q = packed ? c.max_q : (int)q.rows;
+  a.seqlen_k = packed ? c.max_k : (int)k.rows;
+  a.heads_q = (int)q.heads; a.heads_kv = (int)k.heads; a.head_dim = (int)q.dim;
+  a.q = q.p; a.k = k.p; a.v = v.p; a.o = o.p;
+  set_strides(a.q_stride, q); set_strides(a.k_stride, k); set_strides(a.v_stride, v); set_strides(a.o_stride, o);
+  if (packed) {
+    a.cu_seqlens_q = c.cu_q.const_data_ptr<int32_t>();
+    a.cu_seqlens_k = c.cu_k.const_data_ptr<int32_t>();
+    a.total_q = (int)q.rows; a.total_k = (int)k.rows;
+  }
+  // base-2 LSE: (batch, heads, rows), packed (heads, tokens)
+  a.lse2 = lse;
+  a.lse_stride[0] = packed ? 0 : q.heads * q.rows;
+  a.lse_stride[1] = 1;
+  a.lse_stride[2] = q.rows;
+  a.softmax_scale = (float)c.scale;
+  a.softcap = (float)c.softcap;
+  a.alibi_slopes = c.alibi.defined() ? c.alibi.const_data_ptr<float>() : nullptr;
+  a.causal = c.causal; a.window_left = c.wl; a.window_right = c.wr; a.q_pos_offset = c.q_pos_offset;
+  if (c.bias.defined()) {
+    a.attn_bias = c.bias.const_data_ptr<float>();
+    for (int i = 0; i < 4; ++i) a.bias_stride[i] = c.bias.stride(i);
+  }
+  if (c.dropout_p > 0.0) {
+    a.dropout_p = (float)c.dropout_p;
+    a.dropout_seed = c.seed;
+    a.dropout_row_stride = c.row_stride;
+  }
+  if (c.used_q.defined()) a.seqused_q = c.used_q.const_data_ptr<int32_t>();
+  if (c.used_k.defined()) a.seqused_k = c.used_k.const_data_ptr<int32_t>();
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+
+c10::SmallVector<int64_t, 4> lse_shape(const Params& c, const View& q) {
+  if (c.layout == kTHD) return {q.heads, q.rows};
+  return {q.batch, q.heads, q.rows};
+}
+
+// shape of one of q/k/v (the output has q's)
+c10::SmallVector<int64_t, 4> shape_of(const Params& c, const View& v) {
+  if (c.layout == kTHD) return {v.rows, v.heads, v.dim};
+  if (c.layout == kBSHD) return {v.batch, v.rows, v.heads, v.dim};
+  return {v.batch, v.heads, v.rows, v.dim};
+}
+
+// in: prepared inputs.  Fills out and (when wanted) lse.
+void run_forward(const Params& c, const variable_list& in, bool want_lse, Tensor& out, Tensor& lse) {
+  View q, k, v;
+  split(c, in, q, k, v);
+  const Tensor& t = in[0];
+  out = empty_cuda(shape_of(c, q), t.scalar_type(), t.device());
+  if (want_lse) lse = empty_cuda(lse_shape(c, q), at::kFloat, t.device());
+  fa_attn_args a;
+  fill(a, c, t, q, k, v, view_of(out, c.layout, -1, 0), want_lse ? lse.mutable_data_ptr<float>() : nullptr);
+  if (c.layout == kTHD) check(g_abi.varlen_fwd(&a, stream_of(t)), "fa_varlen_fwd");
+  else check(g_abi.fwd(&a, stream_of(t)), "fa_fwd");
+}
+
+// Gradients of the inputs, in the inputs' own packing.  need[0..2]: dq, dk, dv wanted.
+variable_list run_backward(const Params& c, const variable_list& in, const Tensor& out, const Tensor& lse,
+                           const Tensor& grad, bool need_dq, bool need_dkdv) {
+  View q, k, v;
+  split(c, in, q, k, v);
+  const Tensor& t = in[0];
+  const Tensor dout = prep(grad);
+  // rows past cu_seqlens[-1] or past a used length (and padded keys) get no writer: they start from zero
+  const bool partial = c.used_q.defined() || c.used_k.defined() || c.k_valid > 0;
+  auto alloc = [&](at::IntArrayRef sizes) {
+    return partial ? at::zeros(sizes, t.options()) : empty_cuda(sizes, t.scalar_type(), t.device());
+  };
+  variable_list g(in.size());
+  View dq = q, dk = k, dv = v;
+  switch (c.packing) {
+    case kSeparate:
+      if (need_dq) { g[0] = alloc(in[0].sizes()); dq = view_of(g[0], c.layout, -1, 0); }
+      if (need_dkdv) {
+        g[1] = alloc(in[1].sizes()); dk = view_of(g[1], c.layout, -1, 0);
+        g[2] = alloc(in[2].sizes()); dv = view_of(g[2], c.layout, -1, 0);
+      }
+      break;
+    case kQKV:
+      g[0] = alloc(in[0].sizes());
+      dq = view_of(g[0], c.layout, c.packed_dim, 0);
+      dk = view_of(g[0], c.layout, c.packed_dim, 1);
+      dv = view_of(g[0], c.layout, c.packed_dim, 2);
+      break;
+    case kKV:
+      if (need_dq) { g[0] = alloc(in[0].sizes()); dq = view_of(g[0], c.layout, -1, 0); }
+      if (need_dkdv) {
+        g[1] = alloc(in[1].sizes());
+        dk = view_of(g[1], c.layout, c.packed_dim, 0);
+        dv = view_of(g[1], c.layout, c.packed_dim, 1);
+      }
+      break;
+  }
+  Tensor delta = empty_cuda(lse.sizes(), at::kFloat, t.device());
+  fa_attn_args a;
+  fill(a, c, t, q, k, v, view_of(out, c.layout, -1, 0), lse.data_ptr<float>());
+  const View vd = view_of(dout, c.layout, -1, 0);
+  a.dout = vd.p;
+  set_strides(a.do_stride, vd);
+  a.delta = delta.mutable_data_ptr<float>();
+  a.dq = dq.p; a.dk = dk.p; a.dv = dv.p;
+  set_strides(a.dq_stride, dq); set_strides(a.dk_stride, dk); set_strides(a.dv_stride, dv);
+  void* st = stream_of(t);
+  check(g_abi.preprocess(&a, st), "fa_bwd_preprocess");
+  if (c.layout == kTHD) {
+    if (need_dq) check(g_abi.varlen_bwd_dq(&a, st), "fa_varlen_bwd_dq");
+    if (need_dkdv) check(g_abi.varlen_bwd_dkdv(&a, st), "fa_varlen_bwd_dkdv");
+  } else {
+    if (need_dq) check(g_abi.bwd_dq(&a, st), "fa_bwd_dq");
+    if (need_dkdv) check(g_abi.bwd_dkdv(&a, st), "fa_bwd_dkdv");
+  }
+  return g;
+}
+
+struct AttnBackward : public Node {
+  Params c;
+  std::vector<SavedVariable> in;
+  SavedVariable out;
+  Tensor lse;
+
+  variable_list apply(variable_list&& grads) override {
+    variable_list res(in.size());
+    if (!grads[0].defined()) return res;
+    at::AutoDispatchBelowADInplaceOrView below;
+    variable_list x;
+    x.reserve(in.size());
+    for (auto& s : in) x.push_back(s.unpack());
+    const Tensor o = out.unpack(getptr());
+    c10::cuda::CUDAGuard guard(x[0].device());
+    bool dq = true, dkdv = true;
+    if (c.packing != kQKV) {
+      dq = task_should_compute_output(0);
+      dkdv = task_should_compute_output(1) || (c.packing == kSeparate && task_should_compute_output(2));
+    }
+    return run_backward(c, x, o, lse, grads[0], dq, dkdv);
+  }
+  std::string name() const override { return "FlashAttnBackward"; }
+  void release_variables() override {
+    for (auto& s : in) s.reset_data();
+    out.reset_data();
+    lse.reset();
+  }
+};
+
+// Forward of `in` (1 to 3 tensors by packing) with the autograd node when a gradient is wanted.
+// `forward` computes out and lse from the prepared inputs.
+template <typename F>
+Tensor with_grad(const Params& c, variable_list in, bool want_lse, Tensor& lse, F forward) {
+  c10::cuda::CUDAGuard guard(in[0].device());
+  const bool need = at::GradMode::is_enabled() && torch::autograd::any_variable_requires_grad(in);
+  std::shared_ptr<AttnBackward> node;
+  if (need) {
+    node = std::shared_ptr<AttnBackward>(new AttnBackward(), torch::autograd::deleteNode);
+    node->set_next_edges(torch::autograd::collect_next_edges(in));
+  }
+  Tensor out;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    for (auto& t : in) t = prep(t);
+    forward(in, need || want_lse, out, lse);
+  }
+  if (need) {
+    torch::autograd::set_history(out, node);
+    node->c = c;
+    node->in.reserve(in.size());
+    for (auto& t : in) node->in.emplace_back(t, false);
+    node->out = SavedVariable(out, true);
+    node->lse = lse;
+  }
+  return out;
+}
+
+// ---------------------------------------------------------------------------------------
+// Python entry points (positional arguments only)
+// ---------------------------------------------------------------------------------------
+struct Args {
+  PyObject* const* v;
+  Py_ssize_t n, i = 0;
+  PyObject* next() {
+    TORCH_CHECK(i < n, "missing argument");
+    return v[i++];
+  }
+  Tensor tensor() {
+    PyObject* o = next();
+    TORCH_CHECK_TYPE(THPVariable_Check(o), "expected a tensor");
+    return THPVariable_Unpack(o);
+  }
+  Tensor tensor_or_none() {
+    PyObject* o = next();
+    if (o == Py_None) return Tensor();
+    TORCH_CHECK_TYPE(THPVariable_Check(o), "expected a tensor or None");
+    return THPVariable_Unpack(o);
+  }
+  int64_t integer() {
+    const long long x = PyLong_AsLongLong(next());
+    if (x == -1 && PyErr_Occurred()) throw python_error();
+    return x;
+  }
+  double real() {
+    const double x = PyFloat_AsDouble(next());
+    if (x == -1.0 && PyErr_Occurred()) throw python_error();
+    return x;
+  }
+  bool truth() {
+    const int x = PyObject_IsTrue(next());
+    if (x < 0) throw python_error();
+    return x != 0;
+  }
+};
+
+void score_params(Args& a, Params& c) {
+  c.scale = a.real();
+  c.causal = a.truth();
+  c.wl = (int)a.integer();
+  c.wr = (int)a.integer();
+  c.softcap = a.real();
+  c.alibi = a.tensor_or_none();
+}
+
+variable_list input_list(Args& a, Params& c) {
+  c.packing = (Packing)a.integer();
+  c.packed_dim = (int)a.integer();
+  variable_list in;
+  in.push_back(a.tensor());
+  for (int i = 1; i < (c.packing == kSeparate ? 3 : c.packing == kKV ? 2 : 1); ++i) in.push_back(a.tensor());
+  return in;
+}
+
+PyObject* result(const Tensor& out, const Tensor& lse, bool want_lse) {
+  if (!want_lse) return THPVariable_Wrap(out);
+  PyObject* t = PyTuple_New(2);
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(out));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(lse));
+  return t;
+}
+
+// dense(packing, packed_dim, inputs.., scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl, head_major,
+//       bias, dropout_p, seed, row_stride, want_lse) -> out | (out, lse2)
+PyObject* py_dense(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{args, n};
+  Params c;
+  variable_list in = input_list(a, c);
+  score_params(a, c);
+  c.q_pos_offset = (int)a.integer();
+  c.impl = (int)a.integer();
+  c.layout = a.truth() ? kBHSD : kBSHD;
+  c.bias = a.tensor_or_none();
+  c.dropout_p = a.real();
+  c.seed = (uint64_t)a.integer();
+  c.row_stride = (int)a.integer();
+  const bool want_lse = a.truth();
+  Tensor lse;
+  Tensor out = with_grad(c, std::move(in), want_lse, lse, [&](const variable_list& x, bool w, Tensor& o, Tensor& l) {
+    run_forward(c, x, w, o, l);
+  });
+  return result(out, lse, want_lse);
+  END_HANDLE_TH_ERRORS
+}
+
+// varlen(packing, packed_dim, inputs.., cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
+//        dropout_p, seed, row_stride, used_q, used_k, want_lse) -> out | (out, lse2)
+PyObject* py_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{args, n};
+  Params c;
+  variable_list in = input_list(a, c);
+  c.layout = kTHD;
+  c.cu_q = a.tensor();
+  c.cu_k = a.tensor();
+  c.max_q = (int)a.integer();
+  c.max_k = (int)a.integer();
+  score_params(a, c);
+  c.impl = (int)a.integer();
+  c.dropout_p = a.real();
+  c.seed = (uint64_t)a.integer();
+  c.row_stride = (int)a.integer();
+  c.used_q = a.tensor_or_none();
+  c.used_k = a.tensor_or_none();
+  const bool want_lse = a.truth();
+  Tensor lse;
+  Tensor out = with_grad(c, std::move(in), want_lse, lse, [&](const variable_list& x, bool w, Tensor& o, Tensor& l) {
+    run_forward(c, x, w, o, l);
+  });
+  return result(out, lse, want_lse);
+  END_HANDLE_TH_ERRORS
+}
+
+// backward(packing, packed_dim, inputs.., out, lse2, dout, layout, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr,
+//          softcap, alibi, q_pos_offset, impl, bias, dropout_p, seed, row_stride, used_q, used_k) -> gradients
+PyObject* py_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{args, n};
+  Params c;
+  variable_list in = input_list(a, c);
+  Tensor out = a.tensor(), lse = a.tensor(), dout = a.tensor();
+  c.layout = (Layout)a.integer();
+  c.cu_q = a.tensor_or_none();
+  c.cu_k = a.tensor_or_none();
+  c.max_q = (int)a.integer();
+  c.max_k = (int)a.integer();
+  score_params(a, c);
+  c.q_pos_offset = (int)a.integer();
+  c.impl = (int)a.integer();
+  c.bias = a.tensor_or_none();
+  c.dropout_p = a.real();
+  c.seed = (uint64_t)a.integer();
+  c.row_stride = (int)a.integer();
+  c.used_q = a.tensor_or_none();
+  c.used_k = a.tensor_or_none();
+  c10::cuda::CUDAGuard guard(in[0].device());
+  at::AutoDispatchBelowADInplaceOrView below;
+  const variable_list g = run_backward(c, in, out, lse, dout, true, true);
+  PyObject* t = PyTuple_New((Py_ssize_t)g.size());
+  for (size_t i = 0; i < g.size(); ++i) PyTuple_SET_ITEM(t, (Py_ssize_t)i, THPVariable_Wrap(g[i]));
+  return t;
+  END_HANDLE_TH_ERRORS
+}
+
+// int8(q, k, v, causal, scale, impl, k_valid, q_pos_offset) -> out; fp16 backward (head-major tensors)
+PyObject* py_int8(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{args, n};
+  Params c;
+  variable_list in;
+  for (int i = 0; i < 3; ++i) in.push_back(a.tensor());
+  c.layout = kBHSD;
+  c.causal = a.truth();
+  c.scale = a.real();
+  const int impl = (int)a.integer();
+  c.k_valid = (int)a.integer();
+  c.q_pos_offset = (int)a.integer();
+  Tensor lse;
+  Tensor out = with_grad(c, std::move(in), false, lse, [&](const variable_list& x, bool want_lse, Tensor& o, Tensor& l) {
+    const Tensor &q = x[0], &k = x[1], &v = x[2];
+    const auto dev = q.device();
+    const int64_t D = q.size(3), rows = k.numel() / D;
+    void* st = stream_of(q);
+    Tensor k8 = empty_cuda(k.sizes(), at::kChar, dev), s_k = empty_cuda({rows}, at::kFloat, dev), q8, s_q;
+    check(g_abi.quantize_k(k.data_ptr(), k8.data_ptr<int8_t>(), s_k.data_ptr<float>(), rows, (int)D, dev.index(), st),
+          "fa_quantize_k_int8");
+    o = empty_cuda(q.sizes(), at::kHalf, dev);
+    fa_int8_args p;
+    memset(&p, 0, sizeof(p));
+    p.device = dev.index();
+    p.impl = impl;
+    p.batch = (int)q.size(0); p.heads = (int)q.size(1); p.seqlen = (int)q.size(2); p.head_dim = (int)D;
+    p.q = q.data_ptr(); p.k8 = k8.data_ptr<int8_t>(); p.s_k = s_k.data_ptr<float>(); p.v = v.data_ptr();
+    p.o = o.data_ptr();
+    if (want_lse) {
+      l = empty_cuda({q.size(0), q.size(1), q.size(2)}, at::kFloat, dev);
+      p.lse2 = l.mutable_data_ptr<float>();
+    }
+    p.softmax_scale = (float)c.scale;
+    p.causal = c.causal;
+    p.seqlen_k_valid = c.k_valid;
+    p.q_pos_offset = c.q_pos_offset;
+    if (D == 128 && impl != FA_IMPL_MMA) {
+      q8 = empty_cuda(q.sizes(), at::kChar, dev);
+      s_q = empty_cuda({rows}, at::kFloat, dev);
+      p.q8_scratch = q8.data_ptr<int8_t>();
+      p.sq_scratch = s_q.data_ptr<float>();
+    }
+    check(g_abi.fwd_int8(&p, st), "fa_fwd_int8");
+  });
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
+// init({name: address}, check): addresses of the C functions, once per loaded library
+PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{args, n};
+  PyObject* addr = a.next();
+  PyObject* chk = a.next();
+  auto get = [&](const char* name) {
+    PyObject* o = PyDict_GetItemString(addr, name);
+    TORCH_CHECK(o != nullptr, "no address for ", name);
+    void* p = PyLong_AsVoidPtr(o);
+    if (p == nullptr && PyErr_Occurred()) throw python_error();
+    return p;
+  };
+  g_abi.fwd = (AttnFn)get("fa_fwd");
+  g_abi.varlen_fwd = (AttnFn)get("fa_varlen_fwd");
+  g_abi.preprocess = (AttnFn)get("fa_bwd_preprocess");
+  g_abi.bwd_dq = (AttnFn)get("fa_bwd_dq");
+  g_abi.bwd_dkdv = (AttnFn)get("fa_bwd_dkdv");
+  g_abi.varlen_bwd_dq = (AttnFn)get("fa_varlen_bwd_dq");
+  g_abi.varlen_bwd_dkdv = (AttnFn)get("fa_varlen_bwd_dkdv");
+  g_abi.quantize_k = (decltype(g_abi.quantize_k))get("fa_quantize_k_int8");
+  g_abi.fwd_int8 = (decltype(g_abi.fwd_int8))get("fa_fwd_int8");
+  Py_INCREF(chk);
+  Py_XDECREF(g_abi.check);
+  g_abi.check = chk;
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+#define FAST(f) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(f)), METH_FASTCALL
+PyMethodDef g_methods[] = {
+    {"init", FAST(py_init), "addresses of the C ABI functions and the status check"},
+    {"dense", FAST(py_dense), "dense attention"},
+    {"varlen", FAST(py_varlen), "packed variable-length attention"},
+    {"backward", FAST(py_backward), "gradients from a forward's output and LSE"},
+    {"int8", FAST(py_int8), "INT8 scores forward"},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_fa_host", "host path of the attention kernels", -1, g_methods};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__fa_host(void) { return PyModule_Create(&g_module); }

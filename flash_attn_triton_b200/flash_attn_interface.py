@@ -51,7 +51,7 @@ def _as_kernel_dtype(*tensors):
     return tensors
 
 
-def _dense_features(q, k, dropout_p, attn_bias):
+def _dense_features(shape_q, seqlen_k, device, dropout_p, attn_bias):
     """Bias and dropout settings of a dense call, or None when neither is used."""
     if attn_bias is None and not dropout_p:
         return None
@@ -59,10 +59,10 @@ def _dense_features(q, k, dropout_p, attn_bias):
     if attn_bias is not None:
         if attn_bias.requires_grad:
             raise ValueError("attn_bias gradients are not produced; pass a tensor that does not require grad")
-        B, Sq, Hq = q.shape[0], q.shape[1], q.shape[2]
-        bias = attn_bias.detach().to(device=q.device, dtype=torch.float32)
+        B, Sq, Hq = shape_q[:3]
+        bias = attn_bias.detach().to(device=device, dtype=torch.float32)
         try:
-            bias = bias.expand(B, Hq, Sq, k.shape[1])          # broadcast dimensions get stride 0
+            bias = bias.expand(B, Hq, Sq, seqlen_k)            # broadcast dimensions get stride 0
         except RuntimeError:
             raise ValueError("attn_bias must be broadcastable to (batch, nheads, seqlen_q, seqlen_k)")
     seed = row_stride = 0
@@ -70,7 +70,7 @@ def _dense_features(q, k, dropout_p, attn_bias):
         # one seed per call (attention_kernel.py:1238-1239); the counter of element (row, col) uses the
         # sequence length the reference pads to: the next multiple of 64 of the longer side (:168-184, :300-307)
         seed = random.randrange(2 ** 31 - 1)
-        row_stride = (max(q.shape[1], k.shape[1]) + 63) // 64 * 64
+        row_stride = (max(shape_q[1], seqlen_k) + 63) // 64 * 64
     return _ops.Features(bias=bias, dropout_p=dropout_p, seed=seed, row_stride=row_stride)
 
 
@@ -80,11 +80,12 @@ def _dense_call(q, k, v, dropout_p, softmax_scale, causal, window_size, softcap,
     q, k, v = _as_kernel_dtype(q, k, v)
     if softmax_scale is None:
         softmax_scale = 1.0 / math.sqrt(q.shape[-1])
-    feat = _dense_features(q, k, dropout_p, attn_bias)
+    feat = _dense_features(q.shape, k.shape[1], q.device, dropout_p, attn_bias)
     args = (softmax_scale, causal, window_size[0], window_size[1], softcap, alibi_slopes, int(q_pos_offset))
     if not return_attn_probs:
-        return _ops.DenseAttention.apply(q, k, v, *args, N.IMPL_AUTO, "bshd", feat).to(out_dtype)
-    out, lse2 = _ops.DenseAttention.apply(q, k, v, *args, N.IMPL_AUTO, "bshd", feat, True)
+        out = _ops.dense_attention(q, k, v, *args, N.IMPL_AUTO, "bshd", feat)
+        return out if out.dtype == out_dtype else out.to(out_dtype)
+    out, lse2 = _ops.dense_attention(q, k, v, *args, N.IMPL_AUTO, "bshd", feat, True)
     probs, lse = _ops.dense_probs(q.detach(), k.detach(), v.detach(), lse2, *args, "bshd", feat)
     return out.to(out_dtype), lse, probs
 
@@ -114,9 +115,23 @@ def _normalise_alibi(alibi_slopes, batch, heads, device):
     return alibi_slopes.contiguous()
 
 
+_HEAD_DIMS = (16, 32, 64, 128, 256)
+
+
 def _check_head_dim(d):
-    if d not in (16, 32, 64, 128, 256):
+    if d not in _HEAD_DIMS:
         raise ValueError("head dimension must be one of 16, 32, 64, 128, or 256")
+
+
+def _packed_call(packing, tensors, shape_q, seqlen_k, dropout_p, softmax_scale, causal, window_size, softcap, alibi_slopes):
+    """A checked dense call on packed inputs (dimension 2 holds q/k/v or k/v): the kernels read the slices
+    through their strides and write the gradients straight into a packed tensor."""
+    device = tensors[0].device
+    alibi_slopes = _normalise_alibi(alibi_slopes, shape_q[0], shape_q[2], device)
+    if softmax_scale is None:
+        softmax_scale = 1.0 / math.sqrt(shape_q[-1])
+    return _ops.dense_attention_packed(packing, 2, tensors, softmax_scale, causal, window_size[0], window_size[1], softcap,
+                                       alibi_slopes, _dense_features(shape_q, seqlen_k, device, dropout_p, None))
 
 
 def flash_attn_func(q, k, v, dropout_p=0.0, softmax_scale=None, causal=False,
@@ -200,6 +215,11 @@ def flash_attn_qkvpacked_func(qkv, dropout_p=0.0, softmax_scale=None, causal=Fal
     their strides (flash_attn_interface.py:337-371 copies them)."""
     if qkv.ndim != 5 or qkv.shape[2] != 3:
         raise ValueError("qkv must have shape (batch, seqlen, 3, nheads, headdim)")
+    batch, seqlen, _, heads, head_dim = qkv.shape
+    if (qkv.is_cuda and qkv.dtype in _KERNEL_DTYPES and heads and head_dim in _HEAD_DIMS and softcap >= 0.0
+            and 0.0 <= dropout_p < 1.0 and attn_bias is None and not return_attn_probs):
+        return _packed_call(_ops.PACK_QKV, (qkv,), (batch, seqlen, heads, head_dim), seqlen, dropout_p, softmax_scale, causal,
+                            window_size, softcap, alibi_slopes)
     q, k, v = qkv.unbind(dim=2)
     return flash_attn_func(q, k, v, dropout_p, softmax_scale, causal, window_size, softcap,
                            alibi_slopes, deterministic, return_attn_probs, use_native_gqa, attn_bias)
@@ -213,6 +233,13 @@ def flash_attn_kvpacked_func(q, kv, dropout_p=0.0, softmax_scale=None, causal=Fa
     (flash_attn_interface.py:374-406)."""
     if kv.ndim != 5 or kv.shape[2] != 2:
         raise ValueError("kv must have shape (batch, seqlen, 2, nheads_k, headdim)")
+    batch, seqlen_k, _, heads_k, head_dim = kv.shape
+    if (kv.is_cuda and kv.dtype in _KERNEL_DTYPES and q.dtype == kv.dtype and q.ndim == 4 and q.device == kv.device
+            and q.shape[0] == batch and q.shape[3] == head_dim and heads_k and q.shape[2] % heads_k == 0
+            and head_dim in _HEAD_DIMS and softcap >= 0.0 and 0.0 <= dropout_p < 1.0 and attn_bias is None
+            and not return_attn_probs):
+        return _packed_call(_ops.PACK_KV, (q, kv), q.shape, seqlen_k, dropout_p, softmax_scale, causal, window_size,
+                            softcap, alibi_slopes)
     k, v = kv.unbind(dim=2)
     return flash_attn_func(q, k, v, dropout_p, softmax_scale, causal, window_size, softcap,
                            alibi_slopes, deterministic, return_attn_probs, use_native_gqa, attn_bias)
@@ -479,10 +506,10 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
     args = (cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), softmax_scale, causal,
             window_size[0], window_size[1], softcap, alibi)
     if return_attn_probs:
-        out, lse2 = _ops.VarlenAttention.apply(q, k, v, *args, N.IMPL_AUTO, feat, True)
+        out, lse2 = _ops.varlen_attention(0, -1, (q, k, v), *args, N.IMPL_AUTO, feat, True)
         probs, lse = _ops.varlen_probs(q.detach(), k.detach(), v.detach(), lse2, *args, feat)
     else:
-        out = _ops.VarlenAttention.apply(q, k, v, *args, N.IMPL_AUTO, feat)
+        out = _ops.varlen_attention(0, -1, (q, k, v), *args, N.IMPL_AUTO, feat)
     if used_q is not None and not compacted:
         # the reference returns only the used rows, packed (flash_attn_interface.py:552-566); the one
         # host read of the lengths sizes that result
@@ -585,7 +612,7 @@ def attention_int8(q, k, v, causal=False, sm_scale=None, seq_len_k=None, seq_len
         raise ValueError("seq_len_k and seq_len_q must lie in (0, padded sequence length]")
     # Padded calls (attention_kernel_int8.py:108-118, :245): keys at or past seq_len_k are masked and
     # the causal diagonal is shifted by seq_len_k - seq_len_q, in the forward and in the backward.
-    return _ops.Int8Attention.apply(q, k, v, causal, sm_scale, N.IMPL_AUTO,
+    return _ops.int8_attention(q, k, v, causal, sm_scale, N.IMPL_AUTO,
                                     seq_len_k if seq_len_k < S else 0, seq_len_k - seq_len_q)
 
 
