@@ -60,6 +60,7 @@ class DecodeArgs(C.Structure):
         ("softmax_scale", C.c_float), ("alibi_slopes", C.c_void_p),
         ("causal", C.c_int32), ("window_left", C.c_int32), ("window_right", C.c_int32),
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("num_splits", C.c_int32),
+        ("counters", C.c_void_p), ("num_counters", C.c_int32),
     ]
 
 
@@ -98,6 +99,8 @@ EXPORTS = {
     "fa_varlen_bwd_dq": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fa_varlen_bwd_dkdv": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fa_decode_paged": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
+    "fa_decode_paged_checked": (C.c_int, [C.POINTER(DecodeArgs), C.POINTER(C.c_uint32), C.c_void_p]),
+    "fa_decode_counters": (C.c_int32, [C.POINTER(DecodeArgs)]),
     "fa_decode_workspace_bytes": (C.c_size_t, [C.POINTER(DecodeArgs)]),
     "fa_decode_paged_static": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
     "fa_decode_static_scratch_bytes": (C.c_size_t, []),

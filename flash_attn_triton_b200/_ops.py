@@ -235,67 +235,6 @@ def int8_attention(q, k, v, causal, scale, impl, k_valid=0, q_pos_offset=0):
 # ----------------------------------------------------------------------------------------
 # KV-cache decode
 # ----------------------------------------------------------------------------------------
-_workspaces = {}
-
-
-def _workspace(device, nbytes):
-    """Grow-only scratch for split-KV partials, one per (device, stream)."""
-    key = (device, torch.cuda.current_stream(device).cuda_stream)
-    buf = _workspaces.get(key)
-    if buf is None or buf.numel() < nbytes:
-        buf = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
-
-
-def kvcache_decode(q, k_cache, v_cache, k_new, v_new, cos, sin, cache_seqlens, cache_batch_idx,
-                   cache_leftpad, block_table, scale, causal, wl, wr, rotary_interleaved, alibi,
-                   num_splits=0):
-    B, Sq, Hq, D = q.shape
-    Hkv = k_cache.shape[2]
-    q = _prep(q)
-    o = torch.empty((B, Sq, Hq, D), dtype=q.dtype, device=q.device)
-    a = N.DecodeArgs()
-    a.dtype = N.dtype_code(q.dtype)
-    a.device = q.device.index if q.device.index is not None else torch.cuda.current_device()
-    a.batch, a.seqlen_q, a.heads_q, a.heads_kv, a.head_dim = B, Sq, Hq, Hkv, D
-    a.q, a.o = q.data_ptr(), o.data_ptr()
-    a.q_stride, a.o_stride = N.strides3(q, _BSHD), N.strides3(o, _BSHD)
-    a.k_cache, a.v_cache = k_cache.data_ptr(), v_cache.data_ptr()
-    a.kc_stride, a.vc_stride = N.strides3(k_cache, _BSHD), N.strides3(v_cache, _BSHD)
-    a.page_size, a.num_pages = k_cache.shape[1], k_cache.shape[0]
-    if block_table is not None:
-        a.block_table = block_table.data_ptr()
-        a.block_table_stride = block_table.stride(0)
-    a.cache_batch_idx = N.ptr(cache_batch_idx)
-    a.cache_seqlens = cache_seqlens.data_ptr()
-    a.cache_leftpad = N.ptr(cache_leftpad)
-    if k_new is not None:
-        k_new, v_new = _prep(k_new), _prep(v_new)
-        a.k_new, a.v_new = k_new.data_ptr(), v_new.data_ptr()
-        a.kn_stride, a.vn_stride = N.strides3(k_new, _BSHD), N.strides3(v_new, _BSHD)
-        a.seqlen_new = k_new.shape[1]
-    if cos is not None:
-        a.rotary_cos, a.rotary_sin = cos.data_ptr(), sin.data_ptr()
-        a.rotary_dim = cos.shape[-1] * 2
-        a.rotary_seqlen = cos.shape[0]
-        a.rotary_interleaved = int(bool(rotary_interleaved))
-    a.softmax_scale = float(scale)
-    a.alibi_slopes = _alibi_ptr(alibi)
-    a.causal = int(bool(causal))
-    a.window_left, a.window_right = int(wl), int(wr)
-    a.num_splits = int(num_splits)
-    L = N.lib()
-    need = L.fa_decode_workspace_bytes(C.byref(a))
-    ws = None
-    if need:
-        ws = _workspace(q.device, need)
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-    with torch.cuda.device(q.device):
-        N.check(L.fa_decode_paged(C.byref(a), N.stream_ptr(q.device)), "fa_decode_paged")
-    return o
-
-
 def kvcache_decode_static(q, out, k_cache, v_cache, cache_seqlens, block_table=None, k_new=None,
                           v_new=None, cos=None, sin=None, rotary_interleaved=True, scale=None,
                           causal=False, num_splits=0):

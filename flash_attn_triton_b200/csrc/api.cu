@@ -109,6 +109,8 @@ bool bwd_sm100_supported(const fa_attn_args&);
 int bwd_dq_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int bwd_dkdv_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int decode_paged(const fa_decode_args&, cudaStream_t);
+int decode_paged_checked(const fa_decode_args&, uint32_t*, cudaStream_t);
+int decode_num_counters(const fa_decode_args&);
 size_t decode_workspace_bytes(const fa_decode_args&);
 int decode_paged_static(const fa_decode_args&, cudaStream_t);
 size_t decode_static_scratch_bytes();
@@ -342,6 +344,18 @@ int fa_decode_paged(const fa_decode_args* a, void* stream) {
   if (int r = validate_decode(a)) return r;
   if (int r = ensure_device(a->device)) return r;
   return decode_paged(*a, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int fa_decode_paged_checked(const fa_decode_args* a, uint32_t* failed, void* stream) {
+  if (int r = validate_decode(a)) return r;
+  FA_REQUIRE(failed != nullptr, "failed is NULL");
+  if (int r = ensure_device(a->device)) return r;
+  return decode_paged_checked(*a, failed, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int32_t fa_decode_counters(const fa_decode_args* a) {
+  if (a == nullptr || a->heads_kv <= 0 || a->heads_q <= 0) return 0;
+  return decode_num_counters(*a);
 }
 
 int fa_decode_paged_static(const fa_decode_args* a, void* stream) {

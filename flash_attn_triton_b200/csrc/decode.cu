@@ -1,29 +1,95 @@
-// KV-cache decode: split-KV attention over a paged (or contiguous) cache with the in-place append
-// and the rotary embedding fused in, then a small combine.  HBM-bound: the job of the main
-// kernel is to stream every cached K/V byte exactly once at full bandwidth.
+// KV-cache decode: attention over a paged (or contiguous) cache with the in-place append and the rotary
+// embedding fused in.  HBM-bound: the job of the kernel is to stream every cached K/V byte exactly once at
+// full bandwidth.
 //
-//   decode_kernel    : CTA = (split, kv head x row group, sequence).  The query rows of one
-//                      GQA group (seqlen_q x group <= 16 per row group) form the M=16 side
-//                      of mma.sync m16n8k16, so one K/V byte serves the whole group.  K/V
-//                      tiles of 64 keys arrive through a 3-stage cp.async ring of 16-byte
-//                      page-row gathers; 4 warps take 16 keys each and merge at the end.
-//                      The new tokens (k_new rotated, v_new) never come from the cache: the CTAs
-//                      whose split holds their positions put them into the staged tile
-//                      themselves, and the CTA of row group 0 also writes them to their cache
-//                      slots -- one writer per (sequence, kv head, token), no separate launch.
-//   combine_kernel   : merges the per-split partial outputs with their base-2 LSEs.
+//   Work.  A unit is (sequence, kv head, group of 8 or 16 query rows): one K/V byte serves the whole
+//   GQA group.  The products are taken transposed, S^T = K Q^T and O^T = V^T P^T, with the keys (the head
+//   dimension) as the M=16 side of mma.sync m16n8k16 and the query rows as its N=8 side: with 4 or 8
+//   query rows per kv head, as in grouped-query decoding, that is half the products, exponentials
+//   and registers of query rows padded to 16.  A sequence has one work tile per 64 keys and is cut into
+//   pieces of equal size; a CTA takes a piece of one unit.  The piece size follows from the lengths, which are on the device, so every CTA works it out
+//   (see the kernel): a grid of (split, head, sequence) sized for the capacity of the cache has long
+//   pieces, a last wave that is nearly empty, and CTAs without work.  The U heads and row groups
+//   of a piece are neighbouring CTAs, which walk the same cache pages at the same time.
+//   Pipeline.  4 warps take 16 keys of a tile each.  Every warp has a 3-stage cp.async ring of its own
+//   (16-byte row gathers), so that the warps never wait for one another before they merge at the end.
+//   With 16-row products, a barrier per tile and the score options tested per element the compute of
+//   two CTAs per SM, not the memory, set the pace: 702 to 850 us for a 64-sequence step over
+//   4.3 GB of cache against 671 us now.
+//   Append.  The new tokens (k_new rotated, v_new) never come from the cache: the CTA whose tile holds
+//   their positions puts them into the staged tile itself, and the one of row group 0 also writes
+//   them to their cache slots -- one writer per (sequence, kv head, token), no separate launch.
+//   Merge.  A unit of one piece is written straight to the output.  Otherwise its pieces go to
+//   the workspace with their base-2 LSEs and the CTA that finishes last merges them, always in the
+//   same order.
+//   Value checks of the public call run at the start of the same kernel while the tables are small (one
+//   decode step of a few sequences is bounded by launches: 17 small kernels, a copy and a
+//   synchronisation took 150 us around a 16 us kernel), in decode_check_kernel otherwise.
+#include <sched.h>
+
+#include <cmath>
 #include <mutex>
 
 #include "common.cuh"
 
 namespace fa {
 
+constexpr int kTile = 64;             // keys per work tile
+constexpr int kMaxBalanced = 512;     // sequences up to which every CTA sums the lengths itself (2 CTAs per SM still fit)
+constexpr int kOneWave = 64;          // largest piece, in tiles, that is still run in one wave of CTAs
+constexpr int kWaves = 4;             // waves of CTAs beyond that
+
 struct DecodeGeom {
-  int chunk;       // keys per split (multiple of 64)
-  int num_splits;  // grid.x
-  int row_groups;  // ceil(seqlen_q * group / 16)
+  int shares;      // pieces the grid has room for
+  int splits;      // 0: pieces sized on the device; else that many pieces of every sequence
+  int resident;    // CTAs the GPU runs at a time
+  int max_tiles;   // tiles of a full cache
+  int row_groups;  // ceil(seqlen_q * group / rows of a unit)
   int page_shift;  // log2(page_size) or -1
 };
+
+// The value checks of one call: their result goes to a word in mapped host memory (bit 31 = done, low
+// bits = fa_decode_check of the checks that failed), and to a device word for the kernels behind them.
+constexpr uint32_t kCheckDone = 0x80000000u;
+constexpr int kInlineCheck = 1024;   // table entries up to which every attention CTA makes the checks itself
+struct DecodeCheck {
+  uint32_t* host;       // null = no checks in this kernel
+  const uint32_t* dev;  // null, or the result of decode_check_kernel
+};
+
+// All checks, by the threads of one CTA; every thread gets the mask of those that failed.
+__device__ __forceinline__ uint32_t decode_checks(const fa_decode_args& p, int tid, int nt) {
+  uint32_t bad = 0;
+  if (p.block_table) {
+    const int n = p.batch * p.block_table_stride;
+    for (int i = tid; i < n; i += nt)
+      if ((unsigned)p.block_table[i] >= (unsigned)p.num_pages) bad |= FA_CHECK_PAGES;
+  }
+  const long long cap = p.block_table ? (long long)p.block_table_stride * p.page_size : p.page_size;
+  for (int b = tid; b < p.batch; b += nt) {
+    if (p.cache_batch_idx && (unsigned)p.cache_batch_idx[b] >= (unsigned)p.num_pages) bad |= FA_CHECK_ROWS;
+    const int pad = p.cache_leftpad ? p.cache_leftpad[b] : 0;
+    if (pad < 0) bad |= FA_CHECK_LEFTPAD;
+    const int old = p.cache_seqlens[b];
+    const long long last = (long long)old + (p.k_new ? p.seqlen_new : 0) + pad;
+    if (old < 0 || last > cap) bad |= FA_CHECK_LENGTHS;
+    if (p.rotary_cos && last > p.rotary_seqlen) bad |= FA_CHECK_ROTARY;
+  }
+  return (__syncthreads_or(bad & FA_CHECK_PAGES) ? FA_CHECK_PAGES : 0u) |
+         (__syncthreads_or(bad & FA_CHECK_ROWS) ? FA_CHECK_ROWS : 0u) |
+         (__syncthreads_or(bad & FA_CHECK_LEFTPAD) ? FA_CHECK_LEFTPAD : 0u) |
+         (__syncthreads_or(bad & FA_CHECK_LENGTHS) ? FA_CHECK_LENGTHS : 0u) |
+         (__syncthreads_or(bad & FA_CHECK_ROTARY) ? FA_CHECK_ROTARY : 0u);
+}
+
+__global__ void __launch_bounds__(1024) decode_check_kernel(const fa_decode_args p, uint32_t* host, uint32_t* dev) {
+  const uint32_t bad = decode_checks(p, threadIdx.x, blockDim.x);
+  if (threadIdx.x == 0) {
+    *dev = bad;
+    *reinterpret_cast<volatile uint32_t*>(host) = bad | kCheckDone;
+    __threadfence_system();
+  }
+}
 
 template <typename T> __device__ __forceinline__ T hmul_rn(T a, T b);
 template <> __device__ __forceinline__ __half hmul_rn(__half a, __half b) { return __hmul_rn(a, b); }
@@ -82,352 +148,573 @@ __device__ __forceinline__ int64_t cache_row_offset(const fa_decode_args& p, int
 }
 
 // ---------------------------------------------------------------------------------------
-// split-KV attention
+// attention
 // ---------------------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void __launch_bounds__(128) decode_kernel(const fa_decode_args p, const ScoreCfg cfg,
-                                                     const DecodeGeom geo) {
-  constexpr int BN = 64, P = TilePitch<D>::value, NT = 128, NS = 3;
+// Tiles of a sequence: nt work tiles from tile lo on.  Keys that no query row sees (left of the window)
+// are skipped, new tokens never are: somebody has to append them.  An empty sequence has one
+// (empty) tile, which writes its zeros.
+struct SeqTiles {
+  int len_old, len, lo, nt;
+};
+__device__ __forceinline__ SeqTiles seq_tiles(const fa_decode_args& p, const ScoreCfg& cfg, int max_tiles, int b) {
+  SeqTiles s;
+  s.len_old = max(0, min(p.cache_seqlens[b], max_tiles * kTile));   // in bounds also with the value checks off
+  s.len = s.len_old + (p.k_new ? p.seqlen_new : 0);
+  const int first = cfg.wl >= 0 ? min(max(0, s.len - p.seqlen_q - cfg.wl), s.len_old) : 0;
+  s.lo = first / kTile;
+  s.nt = min(max(1, (s.len + kTile - 1) / kTile - s.lo), max_tiles);
+  return s;
+}
+
+// Elements [d, d + 4) of one output row, merged from `parts` pieces in slots s0, s0 + step, ...  Eight
+// pieces are loaded at a time, their common maximum taken first.
+template <typename T, int D, int kRows>
+__device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_l, int64_t s0, int step, int parts, int row,
+                                             int d, T* og) {
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+  float wsum = 0.f, m = -INFINITY;
+  for (int i0 = 0; i0 < parts; i0 += 8) {
+    float l[8];
+    float4 x[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int i = i0 + j;
+      const int64_t r = (s0 + (int64_t)i * step) * kRows + row;
+      l[j] = i < parts ? ws_l[r] : -INFINITY;
+      x[j] = i < parts ? *reinterpret_cast<const float4*>(ws_o + r * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float mn = m;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) mn = fmaxf(mn, l[j]);
+    if (mn == -INFINITY) continue;
+    const float sc = exp2f(m - mn);
+    acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
+    wsum *= sc;
+    m = mn;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float w = exp2f(l[j] - mn);
+      wsum += w;
+      acc.x += w * x[j].x; acc.y += w * x[j].y; acc.z += w * x[j].z; acc.w += w * x[j].w;
+    }
+  }
+  const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
+  uint2 pk;
+  pk.x = Elem<T>::pack(acc.x * inv, acc.y * inv);
+  pk.y = Elem<T>::pack(acc.z * inv, acc.w * inv);
+  *reinterpret_cast<uint2*>(og + d) = pk;
+}
+
+__device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
+  uint32_t y;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+
+// kRows: query rows of a unit (8 or 16)
+template <int D, int kRows> struct DecodeSmem {
+  static constexpr int P = TilePitch<D>::value, NS = 3, OP = D + 4;
+  static constexpr size_t ring = (size_t)2 * NS * kTile * P * 2;
+  static constexpr size_t q_bytes = kRows * P * 2, o_bytes = kRows * OP * 4;
+  static constexpr size_t merge = q_bytes > o_bytes ? q_bytes : o_bytes;   // Q rows, later the merged output of the warps
+  static constexpr size_t fixed = ring + merge + 4 * kRows * 2 * 4;       // + each warp's row maxima and sums
+};
+
+template <typename T, int D, int kRows>
+__global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
+    decode_kernel(const fa_decode_args p, const ScoreCfg cfg, const DecodeGeom geo, const DecodeCheck chk) {
+  using SM = DecodeSmem<D, kRows>;
+  constexpr int P = SM::P, NT = 128, NS = SM::NS, OP = SM::OP, NB = kRows / 8;
+  constexpr int CPR = D / 8, RPW = 32 / CPR, PASSES = 16 / RPW;     // a warp's loads: 16 rows of CPR 16-byte chunks
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* sQ = reinterpret_cast<T*>(smem_raw);  // 16 x P
-  T* sK = sQ + 16 * P;                     // NS x BN x P
-  T* sV = sK + NS * BN * P;                // NS x BN x P
-  // after the key loop the K/V ring is reused as the cross-warp merge buffer
+  T* ring = reinterpret_cast<T*>(smem_raw);      // [stage][warp][K, V][16][P]
+  T* sQ = reinterpret_cast<T*>(smem_raw + SM::ring);                       // kRows x P, and over it
+  float* sO = reinterpret_cast<float*>(sQ);      // kRows x OP
+  float* sM = reinterpret_cast<float*>(smem_raw + SM::ring + SM::merge);   // 4 x kRows
+  float* sL = sM + 4 * kRows;                    // 4 x kRows
+  int* pref = reinterpret_cast<int*>(sL + 4 * kRows);                      // batch + 1: first work tile of each sequence
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int split = blockIdx.x, b = blockIdx.z;
-  const int hk = blockIdx.y / geo.row_groups, rg = blockIdx.y % geo.row_groups;
+  if (chk.host) {
+    const uint32_t bad = decode_checks(p, tid, NT);
+    if (tid == 0 && blockIdx.x == 0) {
+      *reinterpret_cast<volatile uint32_t*>(chk.host) = bad | kCheckDone;
+      __threadfence_system();
+    }
+    if (bad) return;
+  } else if (chk.dev) {
+    // launched while the check kernel may still run (programmatic dependent launch)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (*chk.dev) return;
+  }
   const int G = p.heads_q / p.heads_kv;
-  const int R = p.seqlen_q * G;  // query rows of this kv head: r = sq * G + gi
-  const int len_old = p.cache_seqlens[b];
-  const int n_new = p.k_new ? p.seqlen_new : 0;
-  const int len = len_old + n_new;
-  const int pad = p.cache_leftpad ? p.cache_leftpad[b] : 0;
-  const int k_begin = split * geo.chunk;
-  if (k_begin >= len && split > 0) return;
-  const int k_end = min(len, k_begin + geo.chunk);
-  const int ntiles = max(0, (k_end - k_begin + BN - 1) / BN);
-  const T* kbase = reinterpret_cast<const T*>(p.k_cache) + (int64_t)hk * p.kc_stride[2];
-  const T* vbase = reinterpret_cast<const T*>(p.v_cache) + (int64_t)hk * p.vc_stride[2];
+  const int R = p.seqlen_q * G;                  // query rows of a kv head: r = sq * G + gi
+  const int U = p.heads_kv * geo.row_groups;     // units of a sequence
+  const int u = blockIdx.x % U, share = blockIdx.x / U;
+  const int hk = u / geo.row_groups, rg = u % geo.row_groups;
 
-  auto load_tile = [&](int ti, int st) {
-    constexpr int CPR = D / 8;
-    T* dK = sK + st * BN * P;
-    T* dV = sV + st * BN * P;
-    const int key0 = k_begin + ti * BN;
-    if (geo.page_shift >= 6 && pad == 0) {
-      // the 64-key tile lies inside one page (pages are a power of two >= 64 rows and tiles
-      // start on multiples of 64): one table lookup per thread and tile
-      const int64_t kt = cache_row_offset(p, b, key0, geo.page_shift, p.kc_stride);
-      const int64_t vt = cache_row_offset(p, b, key0, geo.page_shift, p.vc_stride);
-#pragma unroll
-      for (int i = tid; i < BN * CPR; i += NT) {
-        const int r = i / CPR, c = i % CPR;
-        const bool ok = key0 + r < min(k_end, len_old);     // new tokens are staged from k_new / v_new below
-        const int rr = ok ? r : 0;
-        cp_async16(smem_u32(dK + r * P + c * 8), kbase + kt + rr * p.kc_stride[1] + c * 8, ok ? 16 : 0);
-        cp_async16(smem_u32(dV + r * P + c * 8), vbase + vt + rr * p.vc_stride[1] + c * 8, ok ? 16 : 0);
+  // ---- this CTA's piece: tiles [tile0, tile0 + count) of sequence b ------------------------
+  int b, tile0, count, parts, base;              // base: first of the `parts` pieces of the sequence
+  SeqTiles w;
+  if (geo.splits == 0) {
+    for (int i = tid; i < p.batch; i += NT) pref[i + 1] = seq_tiles(p, cfg, geo.max_tiles, i).nt;
+    __syncthreads();
+    // piece size, the same in every warp
+    int sum = 0, longest = 0;
+    for (int i = lane; i < p.batch; i += 32) {
+      sum += pref[i + 1];
+      longest = max(longest, pref[i + 1]);
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    longest = __reduce_max_sync(0xffffffffu, longest);
+    const int64_t work = (int64_t)sum * U;
+    int size = (int)((work + geo.resident - 1) / geo.resident);
+    if (size > kOneWave) {
+      size = max(kOneWave / 2, (int)((work + kWaves * geo.resident - 1) / (kWaves * geo.resident)));
+    } else {
+      size = max(size, (int)ceilf((float)longest / ceilf(sqrtf(7.f * longest))));
+      for (; size < longest; size += max(1, size >> 3)) {
+        int n = 0;
+        for (int i = lane; i < p.batch; i += 32) n += (pref[i + 1] + size - 1) / size;
+        if (__reduce_add_sync(0xffffffffu, n) * U <= geo.resident) break;
       }
-      return;
     }
-    for (int i = tid; i < BN * CPR; i += NT) {
-      const int r = i / CPR, c = i % CPR;
-      const int key = key0 + r;
-      const bool ok = key < min(k_end, len_old);
-      const int pos = (ok ? key : k_begin) + pad;
-      const int64_t ko = cache_row_offset(p, b, pos, geo.page_shift, p.kc_stride);
-      const int64_t vo = cache_row_offset(p, b, pos, geo.page_shift, p.vc_stride);
-      cp_async16(smem_u32(dK + r * P + c * 8), kbase + ko + c * 8, ok ? 16 : 0);
-      cp_async16(smem_u32(dV + r * P + c * 8), vbase + vo + c * 8, ok ? 16 : 0);
+    __syncthreads();
+    // number of pieces before each sequence
+    const int per = (p.batch + NT - 1) / NT;
+    int mine = 0;
+    for (int i = 0; i < per; ++i) {
+      const int bb = tid * per + i;
+      if (bb < p.batch) {
+        mine += (pref[bb + 1] + size - 1) / size;
+        pref[bb + 1] = mine;
+      }
     }
+    int inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
+    }
+    int* wsum = reinterpret_cast<int*>(sM);
+    if (lane == 31) wsum[warp] = inc;
+    if (tid == 0) pref[0] = 0;
+    __syncthreads();
+    int before = inc - mine;
+    for (int i = 0; i < warp; ++i) before += wsum[i];
+    for (int i = 0; i < per; ++i) {
+      const int bb = tid * per + i;
+      if (bb < p.batch) pref[bb + 1] += before;
+    }
+    __syncthreads();
+    if (share >= pref[p.batch]) return;          // the grid is sized for a full cache
+    int lo = 0, hi = p.batch;                    // pref[lo] <= share < pref[hi]
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (pref[mid] <= share) lo = mid;
+      else hi = mid;
+    }
+    b = lo;
+    base = pref[lo];
+    parts = pref[lo + 1] - base;
+    w = seq_tiles(p, cfg, geo.max_tiles, b);
+  } else {
+    b = share / geo.splits;
+    base = b * geo.splits;
+    w = seq_tiles(p, cfg, geo.max_tiles, b);
+    parts = min(geo.splits, w.nt);
+    if (share - base >= parts) return;
+  }
+  const int len_old = w.len_old, len = w.len;
+  tile0 = (int)((int64_t)(share - base) * w.nt / parts);
+  count = (int)((int64_t)(share - base + 1) * w.nt / parts) - tile0;
+  tile0 += w.lo;
+
+  // ---- loading --------------------------------------------------------------------------
+  const int lc = (lane % CPR) * 8, lr = lane / CPR;         // this lane's 16-byte column and first row
+  const bool one_page = p.block_table == nullptr || geo.page_shift >= 4;   // a warp's 16 keys lie inside one page
+  const int pad = p.cache_leftpad ? p.cache_leftpad[b] : 0;
+  const int* table = p.block_table ? p.block_table + (int64_t)b * p.block_table_stride : nullptr;
+  int page = table ? 0 : (p.cache_batch_idx ? p.cache_batch_idx[b] : b);
+  int ld = tile0;                                           // next tile to load
+  auto ld_page = [&]() {                                    // read one tile ahead of its use
+    if (table && one_page) {
+      const int key = ld * kTile + warp * 16;
+      if (key < len_old) page = table[key >> geo.page_shift];
+    }
+  };
+  ld_page();
+  auto load_tile = [&](int st) {
+    if (ld == tile0 + count) return;
+    T* dK = ring + ((st * 4 + warp) * 2 * 16 + lr) * P + lc;
+    T* dV = dK + 16 * P;
+    const T* kb = reinterpret_cast<const T*>(p.k_cache) + (int64_t)hk * p.kc_stride[2] + lc;
+    const T* vb = reinterpret_cast<const T*>(p.v_cache) + (int64_t)hk * p.vc_stride[2] + lc;
+    const int key0 = ld * kTile + warp * 16 + lr;
+    if (one_page) {
+      const int row0 = table ? key0 & (p.page_size - 1) : key0 + pad;
+      const T* ks = kb + (int64_t)page * p.kc_stride[0] + (int64_t)row0 * p.kc_stride[1];
+      const T* vs = vb + (int64_t)page * p.vc_stride[0] + (int64_t)row0 * p.vc_stride[1];
+      const int64_t kstep = RPW * p.kc_stride[1], vstep = RPW * p.vc_stride[1];
+#pragma unroll
+      for (int i = 0; i < PASSES; ++i) {
+        // rows past the cached tokens are zero-filled (new tokens are staged from k_new / v_new later)
+        const int bytes = key0 + i * RPW < len_old ? 16 : 0;
+        cp_async16(smem_u32(dK + i * RPW * P), bytes ? ks + i * kstep : kb, bytes);
+        cp_async16(smem_u32(dV + i * RPW * P), bytes ? vs + i * vstep : vb, bytes);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < PASSES; ++i) {
+        const int key = key0 + i * RPW;
+        const int bytes = key < len_old ? 16 : 0;
+        int pi = 0, row = 0;
+        if (bytes) {
+          if (geo.page_shift >= 0) {
+            pi = key >> geo.page_shift;
+            row = key & (p.page_size - 1);
+          } else {
+            pi = key / p.page_size;
+            row = key - pi * p.page_size;
+          }
+          pi = table[pi];
+        }
+        cp_async16(smem_u32(dK + i * RPW * P), kb + (int64_t)pi * p.kc_stride[0] + (int64_t)row * p.kc_stride[1], bytes);
+        cp_async16(smem_u32(dV + i * RPW * P), vb + (int64_t)pi * p.vc_stride[0] + (int64_t)row * p.vc_stride[1], bytes);
+      }
+    }
+    ++ld;
+    ld_page();
   };
 
 #pragma unroll
   for (int i = 0; i < NS - 1; ++i) {
-    if (i < ntiles) load_tile(i, i);
+    load_tile(i);
     cp_async_commit();
   }
 
-  // ---- Q rows (rotary fused) -> shared memory -> A fragments held in registers ---------
-  {
-    const T* cos = reinterpret_cast<const T*>(p.rotary_cos);
-    const T* sin = reinterpret_cast<const T*>(p.rotary_sin);
-    for (int i = tid; i < 16 * D; i += NT) {
-      const int r = i / D, d = i % D;
-      const int gr = rg * 16 + r;
-      T val = Elem<T>::from_f(0.f);
-      if (gr < R) {
-        const int sq = gr / G, gi = gr % G;
-        const T* qrow = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + sq * p.q_stride[1] +
-                        (int64_t)(hk * G + gi) * p.q_stride[2];
-        if (cos) {
-          const int pos = len - p.seqlen_q + sq + pad;
-          val = rotary_elem<T>([&](int j) { return qrow[j]; }, d, cos, sin, pos, p.rotary_dim,
-                               p.rotary_interleaved, p.rotary_seqlen);
-        } else {
-          val = qrow[d];
-        }
+  float* ws_o = reinterpret_cast<float*>(p.workspace);
+  float* ws_l = ws_o + (int64_t)gridDim.x * kRows * D;
+  const T* cos = reinterpret_cast<const T*>(p.rotary_cos);
+  const T* sin = reinterpret_cast<const T*>(p.rotary_sin);
+  int stage = 0;
+
+  // Q rows (rotary fused) -> shared memory -> B fragments held in registers
+#pragma unroll 4
+  for (int i = tid; i < kRows * D; i += NT) {
+    const int r = i / D, d = i % D;
+    const int gr = rg * kRows + r;
+    T val = Elem<T>::from_f(0.f);
+    if (gr < R) {
+      const int sq = gr / G, gi = gr % G;
+      const T* qrow = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + sq * p.q_stride[1] +
+                      (int64_t)(hk * G + gi) * p.q_stride[2];
+      if (cos) {
+        val = rotary_elem<T>([&](int j) { return qrow[j]; }, d, cos, sin, len - p.seqlen_q + sq + pad, p.rotary_dim,
+                             p.rotary_interleaved, p.rotary_seqlen);
+      } else {
+        val = qrow[d];
       }
-      sQ[r * P + d] = val;
     }
+    sQ[r * P + d] = val;
   }
   __syncthreads();
-  uint32_t aq[D / 16][4];
+  uint32_t bq[NB][D / 16][2];
 #pragma unroll
-  for (int kk = 0; kk < D / 16; ++kk)
-    ldsm_x4(smem_u32(sQ + (lane & 15) * P + kk * 16 + (lane >> 4) * 8), aq[kk][0], aq[kk][1],
-            aq[kk][2], aq[kk][3]);
-
-  // per-thread rows g and g+8 of the row group
-  int qpos[2];
-  float slope[2];
+  for (int n = 0; n < NB; ++n) {
+    if constexpr (D >= 32) {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int gr = min(rg * 16 + g + i * 8, R - 1);
-    const int sq = gr / G, gi = gr % G;
-    qpos[i] = len - p.seqlen_q + sq;
-    slope[i] = cfg.has_alibi ? p.alibi_slopes[b * p.heads_q + hk * G + gi] : 0.f;
+      for (int kk = 0; kk < D / 32; ++kk)
+        ldsm_x4(smem_u32(sQ + (n * 8 + (lane & 7)) * P + kk * 32 + (lane >> 3) * 8), bq[n][2 * kk][0], bq[n][2 * kk][1],
+                bq[n][2 * kk + 1][0], bq[n][2 * kk + 1][1]);
+    } else {
+      const uint32_t* row = reinterpret_cast<const uint32_t*>(sQ + (n * 8 + g) * P);
+      bq[n][0][0] = row[t];
+      bq[n][0][1] = row[t + 4];
+    }
   }
-
-  float o[D / 8][4];
+  // this thread's score columns: query rows 8 n + 2 t and 8 n + 2 t + 1
+  int qpos[NB][2];
+  float slope[NB][2];
 #pragma unroll
-  for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-  float mrow[2] = {-INFINITY, -INFINITY}, lrow[2] = {0.f, 0.f};
-
-  for (int ti = 0; ti < ntiles; ++ti) {
-    cp_async_wait<NS - 2>();
-    __syncthreads();
-    {
-      const int nx = ti + NS - 1;
-      if (nx < ntiles) load_tile(nx, nx % NS);
-      cp_async_commit();
-    }
-    // ---- append: the new tokens of this tile, rotated, into the staged tile and the cache ----
-    {
-      const int key0 = k_begin + ti * BN;
-      const int first = max(key0, len_old), last = min(key0 + BN, k_end);   // new keys [first, last)
-      if (n_new > 0 && last > first) {
-        const T* cos = reinterpret_cast<const T*>(p.rotary_cos);
-        const T* sin = reinterpret_cast<const T*>(p.rotary_sin);
-        T* dK = sK + (ti % NS) * BN * P;
-        T* dV = sV + (ti % NS) * BN * P;
-        for (int i = tid; i < (last - first) * D; i += NT) {
-          const int key = first + i / D, d = i % D;
-          const int tok = key - len_old, pos = key + pad;
-          const T* kn = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] +
-                        hk * p.kn_stride[2];
-          const T* vn = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] +
-                        hk * p.vn_stride[2];
-          T kv = kn[d];
-          if (cos) kv = rotary_elem<T>([&](int j) { return kn[j]; }, d, cos, sin, pos, p.rotary_dim,
-                                         p.rotary_interleaved, p.rotary_seqlen);
-          const T vv = vn[d];
-          dK[(key - key0) * P + d] = kv;
-          dV[(key - key0) * P + d] = vv;
-          if (rg == 0) {
-            reinterpret_cast<T*>(p.k_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.kc_stride) +
-                                            (int64_t)hk * p.kc_stride[2] + d] = kv;
-            reinterpret_cast<T*>(p.v_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.vc_stride) +
-                                            (int64_t)hk * p.vc_stride[2] + d] = vv;
-          }
-        }
-        __syncthreads();
-      }
-    }
-    const T* cK = sK + (ti % NS) * BN * P + warp * 16 * P;
-    const T* cV = sV + (ti % NS) * BN * P + warp * 16 * P;
-
-    float s[2][4];
-    s[0][0] = s[0][1] = s[0][2] = s[0][3] = 0.f;
-    s[1][0] = s[1][1] = s[1][2] = s[1][3] = 0.f;
-#pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) {
-      uint32_t b0, b1, b2, b3;
-      ldsm_x4(smem_u32(cK + ((lane & 7) + ((lane >> 4) << 3)) * P + kk * 16 + ((lane >> 3) & 1) * 8),
-              b0, b1, b2, b3);
-      mma16816<T>(s[0], aq[kk], b0, b1);
-      mma16816<T>(s[1], aq[kk], b2, b3);
-    }
-    float tmax[2] = {-INFINITY, -INFINITY};
-    const int keyw = k_begin + ti * BN + warp * 16;
-#pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = e >> 1;
-        const int col = keyw + nb * 8 + 2 * t + (e & 1);
-        float th;
-        float v = score_log2(cfg, slope[i], s[nb][e], qpos[i], col, th);
-        if (!visible(cfg, qpos[i], col, k_end)) v = -INFINITY;
-        s[nb][e] = v;
-        tmax[i] = fmaxf(tmax[i], v);
-      }
-    }
-    float alpha[2], muse[2];
+  for (int n = 0; n < NB; ++n) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      float mnew = fmaxf(mrow[i], quad_max(tmax[i]));
-      muse[i] = (mnew == -INFINITY) ? 0.f : mnew;
-      alpha[i] = exp2f(mrow[i] - muse[i]);
-      mrow[i] = mnew;
+      const int gr = min(rg * kRows + n * 8 + 2 * t + i, R - 1);
+      const int sq = gr / G, gi = gr % G;
+      qpos[n][i] = len - p.seqlen_q + sq;
+      slope[n][i] = cfg.has_alibi ? p.alibi_slopes[b * p.heads_q + hk * G + gi] : 0.f;
     }
-    float psum[2] = {0.f, 0.f};
+  }
+  const int qmin = len - p.seqlen_q + rg * kRows / G, qmax = len - p.seqlen_q + min(rg * kRows + kRows - 1, R - 1) / G;
+  float o[NB][D / 16][4];
 #pragma unroll
-    for (int nb = 0; nb < 2; ++nb) {
+  for (int n = 0; n < NB; ++n) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float pv = exp2f(s[nb][e] - muse[e >> 1]);
-        s[nb][e] = pv;
-        psum[e >> 1] += pv;
+    for (int i = 0; i < D / 16; ++i) o[n][i][0] = o[n][i][1] = o[n][i][2] = o[n][i][3] = 0.f;
+  }
+  float mrow[NB][2], lrow[NB][2];                // the maximum all scores are taken relative to; sums of this lane's keys
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+    mrow[n][0] = mrow[n][1] = -INFINITY;
+    lrow[n][0] = lrow[n][1] = 0.f;
+  }
+
+  for (int ti = 0; ti < count; ++ti) {
+    const int keyw = (tile0 + ti) * kTile + warp * 16;   // this warp's first key
+    cp_async_wait<NS - 2>();
+    __syncwarp();
+    load_tile(stage == 0 ? NS - 1 : stage - 1);
+    cp_async_commit();
+    T* tK = ring + (stage * 4 + warp) * 2 * 16 * P;
+    T* tV = tK + 16 * P;
+    if (++stage == NS) stage = 0;
+    if (keyw >= len) continue;
+    // ---- append: new tokens among these keys, rotated, into the staged rows and the cache ----
+    const int nfirst = max(keyw, len_old), nlast = min(keyw + 16, len);   // new keys [nfirst, nlast)
+    if (nlast > nfirst) {
+#pragma unroll 4
+      for (int i = lane; i < (nlast - nfirst) * D; i += 32) {
+        const int key = nfirst + i / D, d = i % D;
+        const int tok = key - len_old, pos = key + pad;
+        const T* kn = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + hk * p.kn_stride[2];
+        const T* vn = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + hk * p.vn_stride[2];
+        T kv = kn[d];
+        if (cos) kv = rotary_elem<T>([&](int j) { return kn[j]; }, d, cos, sin, pos, p.rotary_dim,
+                                     p.rotary_interleaved, p.rotary_seqlen);
+        const T vv = vn[d];
+        tK[(key - keyw) * P + d] = kv;
+        tV[(key - keyw) * P + d] = vv;
+        if (rg == 0) {
+          reinterpret_cast<T*>(p.k_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.kc_stride) +
+                                          (int64_t)hk * p.kc_stride[2] + d] = kv;
+          reinterpret_cast<T*>(p.v_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.vc_stride) +
+                                          (int64_t)hk * p.vc_stride[2] + d] = vv;
+        }
+      }
+      __syncwarp();
+    }
+
+    // ---- S^T = K Q^T: keys keyw + g and keyw + g + 8 ------------------------------------
+    float s[NB][4];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < D / 16; ++kk) {
+      uint32_t a[4];
+      ldsm_x4(smem_u32(tK + (lane & 15) * P + kk * 16 + (lane >> 4) * 8), a[0], a[1], a[2], a[3]);
+#pragma unroll
+      for (int n = 0; n < NB; ++n) mma16816<T>(s[n], a, bq[n][kk][0], bq[n][kk][1]);
+    }
+    // ---- softmax.  Plain scores that every row sees need no test per element; their scale goes
+    // into the exponent's FMA --------------------------------------------------------------
+    const bool full = !cfg.has_alibi && keyw + 16 <= len && (!cfg.causal || keyw + 15 <= qmin) &&
+                      (cfg.wl < 0 || keyw >= qmax - cfg.wl) && (cfg.wr < 0 || keyw + 15 <= qmin + cfg.wr);
+    float mul = cfg.scale_log2;
+    if (!full) {
+      mul = 1.f;
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int i = e & 1, key = keyw + g + (e >> 1) * 8;
+          float th;
+          const float v = score_log2(cfg, slope[n][i], s[n][e], qpos[n][i], key, th);
+          s[n][e] = visible(cfg, qpos[n][i], key, len) ? v : -INFINITY;
+        }
       }
     }
-    lrow[0] = lrow[0] * alpha[0] + psum[0];
-    lrow[1] = lrow[1] * alpha[1] + psum[1];
-    uint32_t a[4];
-    a[0] = Elem<T>::pack(s[0][0], s[0][1]);
-    a[1] = Elem<T>::pack(s[0][2], s[0][3]);
-    a[2] = Elem<T>::pack(s[1][0], s[1][1]);
-    a[3] = Elem<T>::pack(s[1][2], s[1][3]);
+    float mx[NB][2];
+    bool grow = false;
 #pragma unroll
-    for (int db2 = 0; db2 < D / 16; ++db2) {
-      o[2 * db2][0] *= alpha[0]; o[2 * db2][1] *= alpha[0];
-      o[2 * db2][2] *= alpha[1]; o[2 * db2][3] *= alpha[1];
-      o[2 * db2 + 1][0] *= alpha[0]; o[2 * db2 + 1][1] *= alpha[0];
-      o[2 * db2 + 1][2] *= alpha[1]; o[2 * db2 + 1][3] *= alpha[1];
-      uint32_t b0, b1, b2, b3;
-      ldsm_x4_t(smem_u32(cV + ((lane & 7) + ((lane >> 3) & 1) * 8) * P + db2 * 16 + (lane >> 4) * 8),
-                b0, b1, b2, b3);
-      mma16816<T>(o[2 * db2], a, b0, b1);
-      mma16816<T>(o[2 * db2 + 1], a, b2, b3);
+    for (int n = 0; n < NB; ++n) {
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        // the scale may be negative: scale before the maximum
+        float m = fmaxf(s[n][i] * mul, s[n][2 + i] * mul);
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+        mx[n][i] = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        // raised only when it grows by more than 2^8: the sums stay in range and O is rarely touched
+        grow |= mx[n][i] > mrow[n][i] + 8.f;
+      }
+    }
+    if (__any_sync(0xffffffffu, grow)) {
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+        float alpha[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const bool up = mx[n][i] > mrow[n][i] + 8.f;
+          alpha[i] = up ? exp2f(mrow[n][i] - mx[n][i]) : 1.f;    // from -inf: 0
+          if (up) mrow[n][i] = mx[n][i];
+          lrow[n][i] *= alpha[i];
+        }
+#pragma unroll
+        for (int db = 0; db < D / 16; ++db) {
+          o[n][db][0] *= alpha[0]; o[n][db][1] *= alpha[1];
+          o[n][db][2] *= alpha[0]; o[n][db][3] *= alpha[1];
+        }
+      }
+    }
+    uint32_t pb[NB][2];
+#pragma unroll
+    for (int n = 0; n < NB; ++n) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float m = mrow[n][e & 1];
+        s[n][e] = m == -INFINITY ? 0.f : ex2(fmaf(s[n][e], mul, -m));
+        lrow[n][e & 1] += s[n][e];
+      }
+      // P^T[key][row] as the accumulator holds it -> B fragment [keys] x [rows]
+      pb[n][0] = transpose_8x8(Elem<T>::pack(s[n][0], s[n][1]));
+      pb[n][1] = transpose_8x8(Elem<T>::pack(s[n][2], s[n][3]));
+    }
+    // ---- O^T += V^T P^T -----------------------------------------------------------------
+#pragma unroll
+    for (int db = 0; db < D / 16; ++db) {
+      uint32_t a[4];
+      ldsm_x4_t(smem_u32(tV + ((lane & 7) + ((lane >> 4) << 3)) * P + db * 16 + ((lane >> 3) & 1) * 8), a[0], a[1], a[2], a[3]);
+#pragma unroll
+      for (int n = 0; n < NB; ++n) mma16816<T>(o[n][db], a, pb[n][0], pb[n][1]);
     }
   }
-  cp_async_wait<0>();
-  __syncthreads();
 
-  // ---- merge the 4 warps (each saw a quarter of every tile) ------------------------------
-  constexpr int OP = D + 4;  // fp32 pitch
-  float* sO = reinterpret_cast<float*>(sK);   // 4 x 16 x OP
-  float* sM = sO + 4 * 16 * OP;               // 4 x 16
-  float* sL = sM + 4 * 16;                    // 4 x 16
-  {
-    float l0 = quad_sum(lrow[0]), l1 = quad_sum(lrow[1]);
+  // ---- merge the 4 warps (each saw a quarter of every tile), one after the other into sO ------
 #pragma unroll
-    for (int nb = 0; nb < D / 8; ++nb) {
-      *reinterpret_cast<float2*>(sO + (warp * 16 + g) * OP + nb * 8 + 2 * t) = make_float2(o[nb][0], o[nb][1]);
-      *reinterpret_cast<float2*>(sO + (warp * 16 + g + 8) * OP + nb * 8 + 2 * t) = make_float2(o[nb][2], o[nb][3]);
-    }
-    if (t == 0) {
-      sM[warp * 16 + g] = mrow[0];
-      sM[warp * 16 + g + 8] = mrow[1];
-      sL[warp * 16 + g] = l0;
-      sL[warp * 16 + g + 8] = l1;
+  for (int n = 0; n < NB; ++n) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      float l = lrow[n][i];
+      l += __shfl_xor_sync(0xffffffffu, l, 4);
+      l += __shfl_xor_sync(0xffffffffu, l, 8);
+      l += __shfl_xor_sync(0xffffffffu, l, 16);
+      if (g == 0) {
+        sM[warp * kRows + n * 8 + 2 * t + i] = mrow[n][i];
+        sL[warp * kRows + n * 8 + 2 * t + i] = l;
+      }
     }
   }
   __syncthreads();
-  const bool direct = geo.num_splits == 1;
-  float* ws_o = reinterpret_cast<float*>(p.workspace);
-  float* ws_l = ws_o + (int64_t)p.batch * p.seqlen_q * p.heads_q * geo.num_splits * D;
-  for (int i = tid; i < 16 * (D / 4); i += NT) {
+  float wgt[NB][2];
+#pragma unroll
+  for (int n = 0; n < NB; ++n) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = n * 8 + 2 * t + i;
+      const float mstar = fmaxf(fmaxf(sM[r], sM[kRows + r]), fmaxf(sM[2 * kRows + r], sM[3 * kRows + r]));
+      wgt[n][i] = (mstar == -INFINITY) ? 0.f : exp2f(mrow[n][i] - mstar);
+    }
+  }
+#pragma unroll 1
+  for (int turn = 0; turn < 4; ++turn) {
+    if (warp == turn) {
+#pragma unroll
+      for (int n = 0; n < NB; ++n) {
+#pragma unroll
+        for (int db = 0; db < D / 16; ++db) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            float* x = sO + (n * 8 + 2 * t + (e & 1)) * OP + db * 16 + g + (e >> 1) * 8;
+            const float v = wgt[n][e & 1] * o[n][db][e];
+            *x = turn > 0 ? *x + v : v;
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+
+  // ---- output, or a piece of it -----------------------------------------------------------
+  const int slot = blockIdx.x;
+  for (int i = tid; i < kRows * (D / 4); i += NT) {
     const int r = i / (D / 4), c4 = (i % (D / 4)) * 4;
-    const int gr = rg * 16 + r;
+    const int gr = rg * kRows + r;
     if (gr >= R) continue;
-    float mstar = fmaxf(fmaxf(sM[r], sM[16 + r]), fmaxf(sM[32 + r], sM[48 + r]));
-    float w[4], lsum = 0.f;
+    const float mstar = fmaxf(fmaxf(sM[r], sM[kRows + r]), fmaxf(sM[2 * kRows + r], sM[3 * kRows + r]));
+    float lsum = 0.f;
+    if (mstar != -INFINITY) {
 #pragma unroll
-    for (int wv = 0; wv < 4; ++wv) {
-      w[wv] = (mstar == -INFINITY) ? 0.f : exp2f(sM[wv * 16 + r] - mstar);
-      lsum += w[wv] * sL[wv * 16 + r];
+      for (int wv = 0; wv < 4; ++wv) lsum += exp2f(sM[wv * kRows + r] - mstar) * sL[wv * kRows + r];
     }
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int wv = 0; wv < 4; ++wv) {
-      float4 x = *reinterpret_cast<const float4*>(sO + (wv * 16 + r) * OP + c4);
-      acc.x += w[wv] * x.x; acc.y += w[wv] * x.y; acc.z += w[wv] * x.z; acc.w += w[wv] * x.w;
-    }
+    float4 acc = *reinterpret_cast<const float4*>(sO + r * OP + c4);
     const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
     acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
     const int sq = gr / G, h = hk * G + gr % G;
-    if (direct) {
+    if (parts == 1) {
       T* og = reinterpret_cast<T*>(p.o) + b * p.o_stride[0] + sq * p.o_stride[1] + (int64_t)h * p.o_stride[2] + c4;
       uint2 pk;
       pk.x = Elem<T>::pack(acc.x, acc.y);
       pk.y = Elem<T>::pack(acc.z, acc.w);
       *reinterpret_cast<uint2*>(og) = pk;
     } else {
-      const int64_t row = (((int64_t)b * p.seqlen_q + sq) * p.heads_q + h) * geo.num_splits + split;
-      *reinterpret_cast<float4*>(ws_o + row * D + c4) = acc;
-      if (c4 == 0) ws_l[row] = lsum > 0.f ? mstar + log2f(lsum) : -INFINITY;
+      *reinterpret_cast<float4*>(ws_o + ((int64_t)slot * kRows + r) * D + c4) = acc;
+      if (c4 == 0) ws_l[(int64_t)slot * kRows + r] = lsum > 0.f ? mstar + log2f(lsum) : -INFINITY;
     }
   }
-}
-
-template <typename T, int D>
-__global__ void __launch_bounds__(128) decode_combine_kernel(const fa_decode_args p, const DecodeGeom geo) {
-  // one warp per output row (b, sq, h)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row = (int64_t)blockIdx.x * 4 + warp;
-  const int64_t nrows = (int64_t)p.batch * p.seqlen_q * p.heads_q;
-  if (row >= nrows) return;
-  const int h = row % p.heads_q;
-  const int sq = (row / p.heads_q) % p.seqlen_q;
-  const int b = row / ((int64_t)p.heads_q * p.seqlen_q);
-  const int len = p.cache_seqlens[b] + (p.k_new ? p.seqlen_new : 0);
-  const int nact = max(1, min(geo.num_splits, (len + geo.chunk - 1) / geo.chunk));
-  const float* ws_o = reinterpret_cast<const float*>(p.workspace);
-  const float* ws_l = ws_o + nrows * geo.num_splits * D;
-  const float* lrow = ws_l + row * geo.num_splits;
-  float mstar = -INFINITY;
-  for (int s = 0; s < nact; ++s) mstar = fmaxf(mstar, lrow[s]);
-  constexpr int EPL = (D + 31) / 32;  // elements per lane
-  float acc[EPL];
-#pragma unroll
-  for (int e = 0; e < EPL; ++e) acc[e] = 0.f;
-  float wsum = 0.f;
-  for (int s = 0; s < nact; ++s) {
-    const float w = (mstar == -INFINITY) ? 0.f : exp2f(lrow[s] - mstar);
-    wsum += w;
-    const float* orow = ws_o + (row * geo.num_splits + s) * D;
-#pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      const int d = e * 32 + lane;
-      if (d < D) acc[e] += w * orow[d];
+  if (parts > 1) {
+    // the CTA that comes last merges; the pieces are ordered before the count by each writer's fence
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) {
+      uint32_t* ctr = p.counters + ((int64_t)b * U + u);
+      last = atomicAdd(ctr, 1u) == (uint32_t)(parts - 1);
+      if (last) *ctr = 0u;
     }
-  }
-  const float inv = wsum > 0.f ? 1.f / wsum : 0.f;
-  T* og = reinterpret_cast<T*>(p.o) + b * p.o_stride[0] + sq * p.o_stride[1] + (int64_t)h * p.o_stride[2];
-#pragma unroll
-  for (int e = 0; e < EPL; ++e) {
-    const int d = e * 32 + lane;
-    if (d < D) og[d] = Elem<T>::from_f(acc[e] * inv);
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      const int rows = min(kRows, R - rg * kRows);
+      for (int i = tid; i < rows * (D / 4); i += NT) {
+        const int r = i / (D / 4), gr = rg * kRows + r;
+        const int sq = gr / G, h = hk * G + gr % G;
+        merge_pieces<T, D, kRows>(ws_o, ws_l, (int64_t)base * U + u, U, parts, r, (i % (D / 4)) * 4,
+                           reinterpret_cast<T*>(p.o) + b * p.o_stride[0] + sq * p.o_stride[1] + (int64_t)h * p.o_stride[2]);
+      }
+    }
   }
 }
 
 // ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
+static int decode_unit_rows(const fa_decode_args& a) { return a.seqlen_q * (a.heads_q / a.heads_kv) <= 8 ? 8 : 16; }
+static int decode_row_groups(const fa_decode_args& a) {
+  const int n = decode_unit_rows(a);
+  return (a.seqlen_q * (a.heads_q / a.heads_kv) + n - 1) / n;
+}
+int decode_num_counters(const fa_decode_args& a) { return a.batch * a.heads_kv * decode_row_groups(a); }
+
+// Room for the pieces the kernel may make.  It picks their size so that
+//   * one wave of CTAs (two per SM, one at head_dim 256) takes all of them, while that needs no more
+//     than kOneWave tiles each: every CTA costs about 3.5 us beside its tiles (16 sequences of 4000 keys,
+//     8 heads: one wave of 32-tile pieces 55 us, two of 16 61 us, 68 us without pieces);
+//   * a sequence has no more than sqrt(7 nt) pieces of its nt tiles: a tile costs about 0.7 us and a piece
+//     0.1 us in the merge (one sequence of 8000 keys, two heads: 126 pieces 20 us, 32 pieces 16.4 us);
+//   * more work than that runs as kWaves waves, which the hardware balances over SMs of unequal speed
+//     (64 sequences of 16000 keys: one wave of equal shares 688 us, 3.5 waves 656 us = 0.98 of the copy
+//     bandwidth).
+// An explicit num_splits, and batches too large to sum in every CTA, cut every sequence into the
+// same number of pieces.
 static DecodeGeom decode_geometry(const fa_decode_args& a) {
   DecodeGeom g;
-  const int G = a.heads_q / a.heads_kv;
-  g.row_groups = (a.seqlen_q * G + 15) / 16;
+  g.row_groups = decode_row_groups(a);
   const int64_t cap = a.block_table ? (int64_t)a.block_table_stride * a.page_size : a.page_size;
-  const int64_t max_len = cap > 0 ? cap : 1;
-  const int64_t base_ctas = (int64_t)a.batch * a.heads_kv * g.row_groups;
-  int splits;
-  if (a.num_splits > 0) {
-    splits = a.num_splits;
+  const int64_t nt = cap > 0 ? (cap + kTile - 1) / kTile : 1;
+  const int64_t U = (int64_t)a.heads_kv * g.row_groups;
+  g.max_tiles = (int)nt;
+  g.splits = 0;
+  g.resident = sm_count(a.device) * (a.head_dim == 256 ? 1 : 2);
+  if (a.num_splits > 0 || a.batch > kMaxBalanced || a.batch * nt > (1 << 30)) {
+    g.splits = a.num_splits > 0 ? (int)(a.num_splits < nt ? a.num_splits : nt) : 1;
+    g.shares = a.batch * g.splits;
   } else {
-    const int64_t target = 148 * 2 * 8;
-    splits = (int)((target + base_ctas - 1) / (base_ctas > 0 ? base_ctas : 1));
-    const int64_t max_splits = (max_len + 511) / 512;
-    if (splits > max_splits) splits = (int)max_splits;
-    if (splits < 1) splits = 1;
+    const int64_t most = a.batch * nt, whole = a.batch;
+    int64_t n = most * U <= (int64_t)kOneWave * g.resident ? g.resident / U : kWaves * g.resident / U + 1;
+    n += whole;                                // rounding up adds less than a piece per sequence
+    g.shares = (int)(n < most ? n : most);
   }
-  int64_t chunk = (max_len + splits - 1) / splits;
-  chunk = (chunk + 63) / 64 * 64;
-  if (chunk >= 256) chunk = (chunk + 255) / 256 * 256;
-  g.chunk = (int)chunk;
-  g.num_splits = (int)((max_len + chunk - 1) / chunk);
-  if (g.num_splits < 1) g.num_splits = 1;
   g.page_shift = -1;
   if (a.page_size > 0 && (a.page_size & (a.page_size - 1)) == 0) {
     int s = 0;
@@ -437,64 +724,197 @@ static DecodeGeom decode_geometry(const fa_decode_args& a) {
   return g;
 }
 
+// pieces (the rows of a unit in fp32 and their LSEs each), then the counters if the caller brings none
+static size_t decode_piece_bytes(const fa_decode_args& a, const DecodeGeom& g) {
+  if (g.splits == 1) return 0;
+  const size_t slots = (size_t)g.shares * a.heads_kv * g.row_groups;
+  return slots * decode_unit_rows(a) * (a.head_dim + 1) * sizeof(float);
+}
 size_t decode_workspace_bytes(const fa_decode_args& a) {
-  if (a.heads_kv <= 0 || a.heads_q <= 0) return 0;
-  DecodeGeom g = decode_geometry(a);
-  if (g.num_splits == 1) return 0;
-  return (size_t)a.batch * a.seqlen_q * a.heads_q * g.num_splits * (a.head_dim + 1) * sizeof(float);
+  if (a.heads_kv <= 0 || a.heads_q <= 0 || a.batch <= 0 || a.seqlen_q <= 0) return 0;
+  const size_t pieces = decode_piece_bytes(a, decode_geometry(a));
+  return pieces == 0 ? 0 : pieces + (a.counters ? 0 : (size_t)decode_num_counters(a) * sizeof(uint32_t));
+}
+
+template <typename T, int D, int kRows>
+static int launch_rows(const fa_decode_args& a, const ScoreCfg& cfg, const DecodeGeom& g, const DecodeCheck& chk,
+                         cudaStream_t st) {
+  const size_t smem = DecodeSmem<D, kRows>::fixed + (g.splits ? 0 : (a.batch + 1) * sizeof(int));
+  auto kern = decode_kernel<T, D, kRows>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    set_error("decode: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    return FA_ERR_LAUNCH;
+  }
+  cudaLaunchConfig_t lc = {};
+  cudaLaunchAttribute attr;
+  lc.gridDim = dim3((unsigned)g.shares * a.heads_kv * g.row_groups);
+  lc.blockDim = dim3(128);
+  lc.dynamicSmemBytes = smem;
+  lc.stream = st;
+  if (chk.dev) {
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = &attr;
+    lc.numAttrs = 1;
+  }
+  cudaLaunchKernelEx(&lc, kern, a, cfg, g, chk);
+  return check_launch("decode");
 }
 
 template <typename T, int D>
-static int launch_decode(const fa_decode_args& a, const ScoreCfg& cfg, const DecodeGeom& g, cudaStream_t st) {
-  constexpr int P = TilePitch<D>::value;
-  constexpr size_t ring = (size_t)(16 + 2 * 3 * 64) * P * sizeof(T);
-  constexpr size_t merge = (size_t)16 * P * sizeof(T) + (size_t)(4 * 16 * (D + 4) + 128) * sizeof(float);
-  constexpr size_t smem = ring > merge ? ring : merge;
-  auto kern = decode_kernel<T, D>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) {
-      set_error("decode: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-      return FA_ERR_LAUNCH;
-    }
-  }
-  dim3 grid(g.num_splits, a.heads_kv * g.row_groups, a.batch);
-  kern<<<grid, 128, smem, st>>>(a, cfg, g);
-  if (int r = check_launch("decode")) return r;
-  if (g.num_splits > 1) {
-    const int64_t rows = (int64_t)a.batch * a.seqlen_q * a.heads_q;
-    decode_combine_kernel<T, D><<<(unsigned)((rows + 3) / 4), 128, 0, st>>>(a, g);
-    return check_launch("decode_combine");
-  }
-  return FA_OK;
+static int launch_decode(const fa_decode_args& a, const ScoreCfg& cfg, const DecodeGeom& g, const DecodeCheck& chk,
+                         cudaStream_t st) {
+  return decode_unit_rows(a) == 8 ? launch_rows<T, D, 8>(a, cfg, g, chk, st) : launch_rows<T, D, 16>(a, cfg, g, chk, st);
 }
 
 template <typename T>
-static int decode_t(const fa_decode_args& a, const ScoreCfg& cfg, const DecodeGeom& g, cudaStream_t st) {
+static int decode_t(const fa_decode_args& a, const ScoreCfg& cfg, const DecodeGeom& g, const DecodeCheck& chk,
+                    cudaStream_t st) {
   switch (a.head_dim) {
-    case 16: return launch_decode<T, 16>(a, cfg, g, st);
-    case 32: return launch_decode<T, 32>(a, cfg, g, st);
-    case 64: return launch_decode<T, 64>(a, cfg, g, st);
-    case 128: return launch_decode<T, 128>(a, cfg, g, st);
-    case 256: return launch_decode<T, 256>(a, cfg, g, st);
+    case 16: return launch_decode<T, 16>(a, cfg, g, chk, st);
+    case 32: return launch_decode<T, 32>(a, cfg, g, chk, st);
+    case 64: return launch_decode<T, 64>(a, cfg, g, chk, st);
+    case 128: return launch_decode<T, 128>(a, cfg, g, chk, st);
+    case 256: return launch_decode<T, 256>(a, cfg, g, chk, st);
   }
   set_error("head_dim %d not in {16,32,64,128,256}", a.head_dim);
   return FA_ERR_UNSUPPORTED;
 }
 
-int decode_paged(const fa_decode_args& a, cudaStream_t st) {
-  if (a.batch == 0 || a.seqlen_q == 0 || a.heads_q == 0) return FA_OK;
-  DecodeGeom g = decode_geometry(a);
-  size_t need = decode_workspace_bytes(a);
+static int decode_run(const fa_decode_args& args, const DecodeCheck& chk, cudaStream_t st) {
+  fa_decode_args a = args;
+  const DecodeGeom g = decode_geometry(a);
+  const size_t pieces = decode_piece_bytes(a, g), need = decode_workspace_bytes(a);
   if (need > 0 && (a.workspace == nullptr || a.workspace_bytes < need)) {
     set_error("decode workspace too small: need %zu bytes, got %zu", need, a.workspace_bytes);
     return FA_ERR_WORKSPACE;
+  }
+  FA_REQUIRE(a.counters == nullptr || a.num_counters >= decode_num_counters(a), "decode: too few counters");
+  if (need > 0 && a.counters == nullptr) {
+    a.counters = reinterpret_cast<uint32_t*>(static_cast<char*>(a.workspace) + pieces);
+    const cudaError_t e = cudaMemsetAsync(a.counters, 0, need - pieces, st);
+    if (e != cudaSuccess) {
+      set_error("decode: cudaMemsetAsync: %s", cudaGetErrorString(e));
+      return FA_ERR_LAUNCH;
+    }
   }
   // bottom-right alignment: the causal mask and window are relative to the query's
   // position at the end of the cached sequence
   ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, a.window_left, a.window_right,
                                 a.alibi_slopes != nullptr);
-  return a.dtype == FA_BF16 ? decode_t<__nv_bfloat16>(a, cfg, g, st) : decode_t<__half>(a, cfg, g, st);
+  return a.dtype == FA_BF16 ? decode_t<__nv_bfloat16>(a, cfg, g, chk, st) : decode_t<__half>(a, cfg, g, chk, st);
+}
+
+int decode_paged(const fa_decode_args& a, cudaStream_t st) {
+  if (a.batch == 0 || a.seqlen_q == 0 || a.heads_q == 0) return FA_OK;
+  return decode_run(a, DecodeCheck{nullptr, nullptr}, st);
+}
+
+// ---------------------------------------------------------------------------------------
+// Value checks.  A call takes a slot -- one word in mapped host memory and one on the device --
+// launches, and polls the host word: it changes as soon as the checks have run, so the host goes on
+// while the attention is still running, without a stream synchronisation.
+// ---------------------------------------------------------------------------------------
+constexpr int kCheckSlots = 256;
+alignas(4096) static volatile uint32_t g_check_host[kCheckSlots * 16];      // a cache line per slot
+static __device__ uint32_t g_check_dev[kCheckSlots];
+
+namespace {
+struct CheckSlots {
+  std::mutex mu;
+  int free_list[kCheckSlots], nfree = 0;
+  int state = 0;                       // 0 not tried, 1 mapped, -1 unavailable
+  uint32_t* dev[64] = {nullptr};
+  // index of a free slot, or -1 (error set)
+  int acquire(int device, uint32_t** host_dptr, uint32_t** dev_ptr) {
+    for (;;) {
+      {
+        std::lock_guard<std::mutex> lock(mu);
+        if (state == 0) {
+          cudaError_t e = cudaHostRegister(const_cast<uint32_t*>(g_check_host), sizeof(g_check_host),
+                                           cudaHostRegisterPortable | cudaHostRegisterMapped);
+          state = e == cudaSuccess ? 1 : -1;
+          for (int i = 0; i < kCheckSlots; ++i) free_list[nfree++] = kCheckSlots - 1 - i;
+          if (e != cudaSuccess) cudaGetLastError();
+        }
+        if (state < 0 || device < 0 || device >= 64) {
+          set_error("decode: no mapped host memory for the value checks");
+          return -1;
+        }
+        if (dev[device] == nullptr) {
+          void* q = nullptr;
+          if (cudaGetSymbolAddress(&q, g_check_dev) != cudaSuccess) {
+            set_error("decode: cudaGetSymbolAddress: %s", cudaGetErrorString(cudaGetLastError()));
+            return -1;
+          }
+          dev[device] = static_cast<uint32_t*>(q);
+        }
+        if (nfree > 0) {
+          const int i = free_list[--nfree];
+          void* h = nullptr;
+          if (cudaHostGetDevicePointer(&h, const_cast<uint32_t*>(&g_check_host[i * 16]), 0) != cudaSuccess) {
+            set_error("decode: cudaHostGetDevicePointer: %s", cudaGetErrorString(cudaGetLastError()));
+            free_list[nfree++] = i;
+            return -1;
+          }
+          *host_dptr = static_cast<uint32_t*>(h);
+          *dev_ptr = dev[device] + i;
+          g_check_host[i * 16] = 0u;
+          return i;
+        }
+      }
+      sched_yield();                   // as many threads as slots are inside this function
+    }
+  }
+  void release(int i) {
+    std::lock_guard<std::mutex> lock(mu);
+    free_list[nfree++] = i;
+  }
+} g_slots;
+}  // namespace
+
+int decode_paged_checked(const fa_decode_args& a, uint32_t* failed, cudaStream_t st) {
+  *failed = 0;
+  if (a.batch == 0 || a.seqlen_q == 0 || a.heads_q == 0) return FA_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    set_error("value checks cannot run while the stream is being captured; turn them off with set_validation(False)");
+    return FA_ERR_LAUNCH;
+  }
+  uint32_t *host = nullptr, *dev = nullptr;
+  const int slot = g_slots.acquire(a.device, &host, &dev);
+  if (slot < 0) return FA_ERR_LAUNCH;
+  const int64_t entries = (int64_t)a.batch * (a.block_table ? a.block_table_stride : 1);
+  int r;
+  if (entries <= kInlineCheck) {
+    r = decode_run(a, DecodeCheck{host, nullptr}, st);
+  } else {
+    decode_check_kernel<<<1, 1024, 0, st>>>(a, host, dev);
+    r = check_launch("decode_check");
+    if (r == FA_OK) r = decode_run(a, DecodeCheck{nullptr, dev}, st);
+  }
+  volatile uint32_t* word = &g_check_host[slot * 16];
+  if (r == FA_OK) {
+    for (uint32_t it = 1; *word == 0u; ++it) {
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+      if ((it & 0x3fffu) == 0) {       // every few hundred microseconds: has the stream died?
+        const cudaError_t e = cudaStreamQuery(st);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess || *word == 0u) {
+          set_error("decode: value checks did not run: %s", cudaGetErrorString(e));
+          r = FA_ERR_LAUNCH;
+          break;
+        }
+      }
+    }
+    *failed = *word & ~kCheckDone;
+  }
+  g_slots.release(slot);
+  return r;
 }
 
 // ---------------------------------------------------------------------------------------

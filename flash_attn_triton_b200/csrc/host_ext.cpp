@@ -21,6 +21,9 @@
 
 #include <string.h>
 
+#include <list>
+#include <mutex>
+
 #include "../../include/fa_b200.h"
 
 namespace {
@@ -38,6 +41,10 @@ struct Abi {
   AttnFn fwd, varlen_fwd, preprocess, bwd_dq, bwd_dkdv, varlen_bwd_dq, varlen_bwd_dkdv;
   int (*quantize_k)(const void*, int8_t*, float*, int64_t, int32_t, int32_t, void*);
   int (*fwd_int8)(const fa_int8_args*, void*);
+  int (*decode)(const fa_decode_args*, void*);
+  int (*decode_checked)(const fa_decode_args*, uint32_t*, void*);
+  int32_t (*decode_counters)(const fa_decode_args*);
+  size_t (*decode_workspace)(const fa_decode_args*);
   PyObject* check;   // _native.check(status, what): raises the Python exception of a status
 };
 Abi g_abi = {};
@@ -524,6 +531,116 @@ PyObject* py_int8(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
+// Zeroed counters of the split-KV merge, one buffer per (device, stream): calls on a stream run one
+// after the other and leave them zero.  At most kCounterBuffers of them are kept (least recently
+// used first out; the allocator hands a dropped one out again on the same stream only).
+constexpr int kCounterWords = 8192;
+constexpr size_t kCounterBuffers = 32;
+Tensor decode_counters(const at::Device& dev, cudaStream_t stream) {
+  struct Entry {
+    int device;
+    cudaStream_t stream;
+    Tensor words;
+  };
+  static std::mutex mu;
+  static std::list<Entry>* pool = new std::list<Entry>();     // never destroyed: outlives the CUDA context's teardown
+  std::lock_guard<std::mutex> lock(mu);
+  for (auto it = pool->begin(); it != pool->end(); ++it)
+    if (it->device == dev.index() && it->stream == stream) {
+      pool->splice(pool->begin(), *pool, it);
+      return it->words;
+    }
+  if (pool->size() >= kCounterBuffers) pool->pop_back();
+  pool->push_front(Entry{dev.index(), stream, at::zeros({kCounterWords}, at::TensorOptions().device(dev).dtype(at::kInt))});
+  return pool->front().words;
+}
+
+// kvcache(q, k_cache, v_cache, k_new, v_new, cos, sin, seqlens, batch_idx, leftpad, block_table, scale, causal, wl, wr,
+//         interleaved, alibi, num_splits, checks) -> out, or the mask of the value checks that failed
+PyObject* py_kvcache(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{args, n};
+  Tensor q = a.tensor(), kc = a.tensor(), vc = a.tensor(), kn = a.tensor_or_none(), vn = a.tensor_or_none();
+  Tensor cos = a.tensor_or_none(), sin = a.tensor_or_none(), lens = a.tensor(), idx = a.tensor_or_none();
+  Tensor pads = a.tensor_or_none(), table = a.tensor_or_none();
+  fa_decode_args p;
+  memset(&p, 0, sizeof(p));
+  p.softmax_scale = (float)a.real();
+  p.causal = a.truth();
+  p.window_left = (int)a.integer();
+  p.window_right = (int)a.integer();
+  p.rotary_interleaved = a.truth();
+  Tensor alibi = a.tensor_or_none();
+  p.num_splits = (int)a.integer();
+  const bool checks = a.truth();
+
+  c10::cuda::CUDAGuard guard(q.device());
+  at::AutoDispatchBelowADInplaceOrView below;
+  const auto dev = q.device();
+  q = prep(q);
+  Tensor out = empty_cuda(q.sizes(), q.scalar_type(), dev);
+  p.dtype = q.scalar_type() == at::kBFloat16 ? FA_BF16 : FA_F16;
+  p.device = dev.index();
+  const View vq = view_of(q, kBSHD, -1, 0), vo = view_of(out, kBSHD, -1, 0), vkc = view_of(kc, kBSHD, -1, 0),
+             vvc = view_of(vc, kBSHD, -1, 0);
+  p.batch = (int)vq.batch; p.seqlen_q = (int)vq.rows; p.heads_q = (int)vq.heads; p.head_dim = (int)vq.dim;
+  p.heads_kv = (int)vkc.heads;
+  p.q = vq.p; p.o = vo.p;
+  set_strides(p.q_stride, vq); set_strides(p.o_stride, vo);
+  p.k_cache = vkc.p; p.v_cache = vvc.p;
+  set_strides(p.kc_stride, vkc); set_strides(p.vc_stride, vvc);
+  p.page_size = (int)vkc.rows; p.num_pages = (int)vkc.batch;
+  if (table.defined()) {
+    p.block_table = table.const_data_ptr<int32_t>();
+    p.block_table_stride = (int)table.size(1);       // contiguous
+  }
+  if (idx.defined()) p.cache_batch_idx = idx.const_data_ptr<int32_t>();
+  p.cache_seqlens = lens.const_data_ptr<int32_t>();
+  if (pads.defined()) p.cache_leftpad = pads.const_data_ptr<int32_t>();
+  if (kn.defined()) {
+    kn = prep(kn);
+    vn = prep(vn);
+    const View vkn = view_of(kn, kBSHD, -1, 0), vvn = view_of(vn, kBSHD, -1, 0);
+    p.k_new = vkn.p; p.v_new = vvn.p;
+    set_strides(p.kn_stride, vkn); set_strides(p.vn_stride, vvn);
+    p.seqlen_new = (int)vkn.rows;
+  }
+  if (cos.defined()) {
+    p.rotary_cos = cos.data_ptr(); p.rotary_sin = sin.data_ptr();
+    p.rotary_dim = (int)cos.size(1) * 2;
+    p.rotary_seqlen = (int)cos.size(0);
+  }
+  if (alibi.defined()) p.alibi_slopes = alibi.const_data_ptr<float>();
+  const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+  Tensor ws, ctr;
+  if (const size_t need = g_abi.decode_workspace(&p)) {
+    ws = empty_cuda({(int64_t)need}, at::kByte, dev);
+    p.workspace = ws.data_ptr();
+    p.workspace_bytes = need;
+    const int words = g_abi.decode_counters(&p);
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (words <= kCounterWords && cudaStreamIsCapturing(st, &cap) == cudaSuccess) {
+      // a captured call keeps counters of its own, zeroed inside the graph
+      ctr = cap == cudaStreamCaptureStatusNone ? decode_counters(dev, st)
+                                               : at::zeros({words}, at::TensorOptions().device(dev).dtype(at::kInt));
+      p.counters = reinterpret_cast<uint32_t*>(ctr.data_ptr<int32_t>());
+      p.num_counters = (int)ctr.numel();
+    }
+  }
+  uint32_t failed = 0;
+  int status;
+  if (checks) {
+    pybind11::gil_scoped_release nogil;
+    status = g_abi.decode_checked(&p, &failed, st);
+  } else {
+    status = g_abi.decode(&p, st);
+  }
+  check(status, "fa_decode_paged");
+  if (failed) return PyLong_FromUnsignedLong(failed);
+  return THPVariable_Wrap(out);
+  END_HANDLE_TH_ERRORS
+}
+
 // init({name: address}, check): addresses of the C functions, once per loaded library
 PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
@@ -546,6 +663,10 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t n) {
   g_abi.varlen_bwd_dkdv = (AttnFn)get("fa_varlen_bwd_dkdv");
   g_abi.quantize_k = (decltype(g_abi.quantize_k))get("fa_quantize_k_int8");
   g_abi.fwd_int8 = (decltype(g_abi.fwd_int8))get("fa_fwd_int8");
+  g_abi.decode = (decltype(g_abi.decode))get("fa_decode_paged");
+  g_abi.decode_checked = (decltype(g_abi.decode_checked))get("fa_decode_paged_checked");
+  g_abi.decode_counters = (decltype(g_abi.decode_counters))get("fa_decode_counters");
+  g_abi.decode_workspace = (decltype(g_abi.decode_workspace))get("fa_decode_workspace_bytes");
   Py_INCREF(chk);
   Py_XDECREF(g_abi.check);
   g_abi.check = chk;
@@ -559,6 +680,7 @@ PyMethodDef g_methods[] = {
     {"dense", FAST(py_dense), "dense attention"},
     {"varlen", FAST(py_varlen), "packed variable-length attention"},
     {"backward", FAST(py_backward), "gradients from a forward's output and LSE"},
+    {"kvcache", FAST(py_kvcache), "append to a KV cache and attend to it"},
     {"int8", FAST(py_int8), "INT8 scores forward"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_fa_host", "host path of the attention kernels", -1, g_methods};

@@ -246,6 +246,8 @@ def flash_attn_kvpacked_func(q, kv, dropout_p=0.0, softmax_scale=None, causal=Fa
 
 
 def _as_i32(x, device):
+    if isinstance(x, torch.Tensor) and x.dtype == torch.int32 and x.ndim == 1 and x.device == device and x.is_contiguous():
+        return x
     return torch.as_tensor(x, device=device).to(torch.int32).flatten().contiguous()
 
 
@@ -265,22 +267,22 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, rotary_cos=None
     measured from there (also without `causal`: the reference only shifts the causal mask,
     flash_attn_interface.py:523).  `num_splits` (0 = automatic) is an extra tuning knob.
 
-    With value checks on (the default) the call reads ONE flag back from the device (page indices
-    in range, lengths fit the cache and the rotary tables, reduced on the device);
-    `set_validation(False)` or FA_B200_VALIDATE=0 turns them off and the call then never
-    synchronises."""
+    With value checks on (the default) the kernel makes them first (page indices in range, lengths
+    fit the cache and the rotary tables) and the call waits for that one flag, not for the attention;
+    `set_validation(False)` or FA_B200_VALIDATE=0 turns them off and the call then never waits."""
     paged = block_table is not None
-    checks = []          # value checks, evaluated together just before the launch (one host read)
     if (rotary_cos is None) != (rotary_sin is None):
         raise ValueError("rotary_cos and rotary_sin must be supplied together")
     if q.ndim != 4 or k_cache.ndim != 4 or v_cache.ndim != 4:
         raise ValueError("q and KV caches must be rank-4 tensors")
-    if k_cache.shape != v_cache.shape:
+    shape, cache_shape = q.shape, k_cache.shape
+    if cache_shape != v_cache.shape:
         raise ValueError("k_cache and v_cache must have the same shape")
     if not (q.is_cuda and k_cache.is_cuda and v_cache.is_cuda):
         raise ValueError("All attention tensors must be CUDA tensors")
-    B = q.shape[0]
-    dev = q.device
+    B, seqlen_q, heads_q, head_dim = shape
+    rows_cache, cache_rows, heads_kv, cache_dim = cache_shape
+    dev, dtype = q.device, q.dtype
     if paged:
         if block_table.ndim != 2 or block_table.shape[0] != B:
             raise ValueError("block_table must have shape (batch, max_num_pages)")
@@ -290,97 +292,99 @@ def flash_attn_with_kvcache(q, k_cache, v_cache, k=None, v=None, rotary_cos=None
             raise ValueError("cache_leftpad cannot be combined with paged KV caches")
         if cache_batch_idx is not None:
             raise ValueError("cache_batch_idx cannot be combined with paged KV caches")
-        page_size = k_cache.shape[1]
-        cache_capacity = block_table.shape[1] * page_size
         block_table = block_table.to(device=dev, dtype=torch.int32).contiguous()
-        if _VALIDATE:
-            checks.append((torch.any((block_table < 0) | (block_table >= k_cache.shape[0])),
-                           "block_table contains an invalid physical page index"))
+        cache_capacity = block_table.shape[1] * cache_rows
     else:
-        cache_capacity = k_cache.shape[1]
-    if q.shape[-1] != k_cache.shape[-1]:
+        cache_capacity = cache_rows
+    if head_dim != cache_dim:
         raise ValueError("q and KV cache dimensions are incompatible")
-    if q.device != k_cache.device or q.device != v_cache.device:
+    if dev != k_cache.device or dev != v_cache.device:
         raise ValueError("q and KV caches must be on the same device")
-    if q.dtype != k_cache.dtype or q.dtype != v_cache.dtype:
+    if dtype != k_cache.dtype or dtype != v_cache.dtype:
         raise ValueError("q and KV caches must have the same dtype")
-    if q.dtype not in _KERNEL_DTYPES:
+    if dtype not in _KERNEL_DTYPES:
         raise ValueError("flash_attn_with_kvcache supports FP16 and BF16 tensors")
-    _check_head_dim(q.shape[-1])
-    if k_cache.shape[2] == 0 or q.shape[2] % k_cache.shape[2] != 0:
+    _check_head_dim(head_dim)
+    if heads_kv == 0 or heads_q % heads_kv != 0:
         raise ValueError("The number of query heads must be divisible by KV heads")
-    if k_cache.stride(-1) != 1 or v_cache.stride(-1) != 1 or not (
-            N.kernel_ready(k_cache) and N.kernel_ready(v_cache)):
+    if not (N.kernel_ready(k_cache) and N.kernel_ready(v_cache)):
         raise ValueError("KV caches must have a unit head-dim stride and 16-byte aligned rows")
     rows = None
     if cache_batch_idx is not None:
         rows = _as_i32(cache_batch_idx, dev)
         if rows.numel() != B:
             raise ValueError("cache_batch_idx must contain valid cache-row indices")
-        if _VALIDATE:
-            checks.append((torch.any((rows < 0) | (rows >= k_cache.shape[0])),
-                           "cache_batch_idx must contain valid cache-row indices"))
-    elif not paged and k_cache.shape[0] < B:
+    elif not paged and rows_cache < B:
         raise ValueError("cache_batch_idx must contain valid cache-row indices")
     pads = None
     if cache_leftpad is not None:
         pads = _as_i32(cache_leftpad, dev)
         if pads.numel() != B:
             raise ValueError("cache_leftpad must contain one non-negative value per query batch")
-        if _VALIDATE:
-            checks.append((torch.any(pads < 0), "cache_leftpad must contain one non-negative value per query batch"))
-    n_new = 0
+    lengths_error = "cache_seqlens must contain valid lengths for every batch item"
     if k is not None or v is not None:
         if k is None or v is None or k.shape != v.shape:
             raise ValueError("k and v must be supplied together with matching shapes")
-        if k.ndim != 4 or k.shape[0] != B or k.shape[2:] != k_cache.shape[2:]:
+        if k.ndim != 4 or k.shape[0] != B or k.shape[2:] != cache_shape[2:]:
             raise ValueError("new k/v tensors are incompatible with the cache")
-        if k.dtype != q.dtype or v.dtype != q.dtype:
+        if k.dtype != dtype or v.dtype != dtype:
             raise ValueError("q and KV caches must have the same dtype")
-        n_new = k.shape[1]
+        lengths_error = "new KV tensors do not fit in the cache"
         if cache_seqlens is None:
             cache_seqlens = torch.zeros(B, dtype=torch.int32, device=dev)
-        lengths = _as_i32(cache_seqlens, dev)
-        if lengths.numel() != B:
-            raise ValueError("new KV tensors do not fit in the cache")
-        if _VALIDATE:
-            total = lengths.long() + n_new + (pads.long() if pads is not None else 0)
-            checks.append((torch.any((lengths < 0) | (total > cache_capacity)), "new KV tensors do not fit in the cache"))
-        if n_new == 0:
+        if k.shape[1] == 0:
             k = v = None
-    else:
-        if cache_seqlens is None:
-            lengths = torch.full((B,), cache_capacity, dtype=torch.int32, device=dev)
-        else:
-            lengths = _as_i32(cache_seqlens, dev)
-        if lengths.numel() != B:
-            raise ValueError("cache_seqlens must contain valid lengths for every batch item")
-        if _VALIDATE:
-            total = lengths.long() + (pads.long() if pads is not None else 0)
-            checks.append((torch.any((lengths < 0) | (total > cache_capacity)),
-                           "cache_seqlens must contain valid lengths for every batch item"))
-    cos = sin = None
+    elif cache_seqlens is None:
+        cache_seqlens = torch.full((B,), cache_capacity, dtype=torch.int32, device=dev)
+    lengths = _as_i32(cache_seqlens, dev)
+    if lengths.numel() != B:
+        raise ValueError(lengths_error)
     if rotary_cos is not None:
         if rotary_cos.shape != rotary_sin.shape or rotary_cos.ndim != 2:
             raise ValueError("rotary_cos and rotary_sin must be (seqlen_ro, rotary_dim / 2)")
-        if rotary_cos.shape[-1] * 2 > q.shape[-1]:
+        if rotary_cos.shape[-1] * 2 > head_dim:
             raise ValueError("rotary tables exceed the head dimension")
+        rotary_cos = rotary_cos.to(device=dev, dtype=dtype).contiguous()
+        rotary_sin = rotary_sin.to(device=dev, dtype=dtype).contiguous()
+    alibi = _normalise_alibi(alibi_slopes, B, heads_q, dev)
+    if B == 0 or seqlen_q == 0:
         if _VALIDATE:
-            # every rotated position (new keys and query rows) must have a table row
-            last = lengths.long() + n_new + (pads.long() if pads is not None else 0)
-            checks.append((torch.any(last > rotary_cos.shape[0]),
-                           "rotary tables are shorter than the longest sequence after the append"))
-        cos = rotary_cos.to(device=dev, dtype=q.dtype).contiguous()
-        sin = rotary_sin.to(device=dev, dtype=q.dtype).contiguous()
-    alibi = _normalise_alibi(alibi_slopes, B, q.shape[2], dev)
-    _raise_first(checks)
-    if B == 0 or q.shape[1] == 0:
-        return q.new_empty(q.shape)
+            _check_cache_values(block_table, rows, pads, lengths, 0 if k is None else k.shape[1], rows_cache, cache_capacity,
+                                rotary_cos, lengths_error)
+        return q.new_empty(shape)
     if softmax_scale is None:
-        softmax_scale = 1.0 / math.sqrt(q.shape[-1])
-    return _ops.kvcache_decode(q, k_cache, v_cache, k, v, cos, sin, lengths, rows, pads,
-                               block_table, softmax_scale, causal, window_size[0], window_size[1],
-                               rotary_interleaved, alibi, num_splits)
+        softmax_scale = 1.0 / math.sqrt(head_dim)
+    out = N.host().kvcache(q, k_cache, v_cache, k, v, rotary_cos, rotary_sin, lengths, rows, pads, block_table, softmax_scale,
+                           causal, window_size[0], window_size[1], rotary_interleaved, alibi, num_splits, _VALIDATE)
+    if isinstance(out, int):
+        raise ValueError(_cache_value_errors(lengths_error)[(out & -out).bit_length() - 1])
+    return out
+
+
+def _cache_value_errors(lengths_error):
+    """Messages of the value checks of a cache call, in order of precedence (the bits of fa_decode_check)."""
+    return ("block_table contains an invalid physical page index",
+            "cache_batch_idx must contain valid cache-row indices",
+            "cache_leftpad must contain one non-negative value per query batch",
+            lengths_error,
+            "rotary tables are shorter than the longest sequence after the append")
+
+
+def _check_cache_values(block_table, rows, pads, lengths, n_new, cache_rows, capacity, cos, lengths_error):
+    """The value checks of a cache call that launches no attention kernel (no query rows)."""
+    checks = []
+    errors = _cache_value_errors(lengths_error)
+    if block_table is not None:
+        checks.append((torch.any((block_table < 0) | (block_table >= cache_rows)), errors[0]))
+    if rows is not None:
+        checks.append((torch.any((rows < 0) | (rows >= cache_rows)), errors[1]))
+    if pads is not None:
+        checks.append((torch.any(pads < 0), errors[2]))
+    last = lengths.long() + n_new + (pads.long() if pads is not None else 0)
+    checks.append((torch.any((lengths < 0) | (last > capacity)), errors[3]))
+    if cos is not None:
+        checks.append((torch.any(last > cos.shape[0]), errors[4]))
+    _raise_first(checks)
 
 
 def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k,

@@ -200,9 +200,30 @@ typedef struct fa_decode_args {
   void* workspace; /* split-KV partials; size from fa_decode_workspace_bytes */
   size_t workspace_bytes;
   int32_t num_splits; /* 0 = choose */
+  /* Optional: fa_decode_counters() zeroed words that calls in flight at the same time do not share.  The
+   * kernel that finishes a row's last split merges the partials itself (no second launch) and
+   * leaves the words zero again. */
+  uint32_t* counters;
+  int32_t num_counters;
 } fa_decode_args;
 
 int fa_decode_paged(const fa_decode_args* args, void* stream);
+
+/* fa_decode_paged with the value checks of the public call made on the device.  `failed` receives the
+ * checks that did not hold (0 = all held); if any did not, nothing was written.  Returns as soon as the
+ * checks have run on the GPU, while the attention itself may still be running.  Not for streams
+ * under capture. */
+typedef enum fa_decode_check {
+  FA_CHECK_PAGES = 1,   /* block_table entries lie in [0, num_pages) */
+  FA_CHECK_ROWS = 2,    /* cache_batch_idx entries lie in [0, num_pages) */
+  FA_CHECK_LEFTPAD = 4, /* cache_leftpad is not negative */
+  FA_CHECK_LENGTHS = 8, /* 0 <= cache_seqlens, and old + new + padding tokens fit the cache */
+  FA_CHECK_ROTARY = 16  /* every rotated position has a table row */
+} fa_decode_check;
+int fa_decode_paged_checked(const fa_decode_args* args, uint32_t* failed, void* stream);
+
+/* Words fa_decode_args.counters needs for this problem. */
+int32_t fa_decode_counters(const fa_decode_args* args);
 
 /* Bytes of workspace fa_decode_paged needs for this problem (host-only, no CUDA call). */
 size_t fa_decode_workspace_bytes(const fa_decode_args* args);
