@@ -7,7 +7,7 @@
 //   dimension) as the M=16 side of mma.sync m16n8k16 and the query rows as its N=8 side: with 4 or 8
 //   query rows per kv head, as in grouped-query decoding, that is half the products, exponentials
 //   and registers of query rows padded to 16.  A sequence has one work tile per 64 keys and is cut into
-//   pieces of equal size; a CTA takes a piece of one unit.  The piece size follows from the lengths, which are on the device, so every CTA works it out
+//   pieces of equal size; a CTA takes a piece of one unit.  The piece size follows from the lengths, which are on the device, so every warp works it out
 //   (see the kernel): a grid of (split, head, sequence) sized for the capacity of the cache has long
 //   pieces, a last wave that is nearly empty, and CTAs without work.  The U heads and row groups
 //   of a piece are neighbouring CTAs, which walk the same cache pages at the same time.
@@ -35,7 +35,7 @@
 namespace fa {
 
 constexpr int kTile = 64;             // keys per work tile
-constexpr int kMaxBalanced = 512;     // sequences up to which every CTA sums the lengths itself (2 CTAs per SM still fit)
+constexpr int kMaxBalanced = 512;     // sequences up to which every warp sums the lengths itself
 constexpr int kOneWave = 64;          // largest piece, in tiles, that is still run in one wave of CTAs
 constexpr int kWaves = 4;             // waves of CTAs beyond that
 
@@ -75,6 +75,7 @@ __device__ __forceinline__ uint32_t decode_checks(const fa_decode_args& p, int t
     if (old < 0 || last > cap) bad |= FA_CHECK_LENGTHS;
     if (p.rotary_cos && last > p.rotary_seqlen) bad |= FA_CHECK_ROTARY;
   }
+  if (!__syncthreads_or(bad)) return 0u;
   return (__syncthreads_or(bad & FA_CHECK_PAGES) ? FA_CHECK_PAGES : 0u) |
          (__syncthreads_or(bad & FA_CHECK_ROWS) ? FA_CHECK_ROWS : 0u) |
          (__syncthreads_or(bad & FA_CHECK_LEFTPAD) ? FA_CHECK_LEFTPAD : 0u) |
@@ -232,7 +233,6 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
   float* sO = reinterpret_cast<float*>(sQ);      // kRows x OP
   float* sM = reinterpret_cast<float*>(smem_raw + SM::ring + SM::merge);   // 4 x kRows
   float* sL = sM + 4 * kRows;                    // 4 x kRows
-  int* pref = reinterpret_cast<int*>(sL + 4 * kRows);                      // batch + 1: first work tile of each sequence
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   if (chk.host) {
@@ -257,66 +257,62 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
   int b, tile0, count, parts, base;              // base: first of the `parts` pieces of the sequence
   SeqTiles w;
   if (geo.splits == 0) {
-    for (int i = tid; i < p.batch; i += NT) pref[i + 1] = seq_tiles(p, cfg, geo.max_tiles, i).nt;
-    __syncthreads();
-    // piece size, the same in every warp
+    // Every warp does this on its own, without shared memory or barriers (which cost a small step 2 to 4
+    // us); lane i looks after the sequences [i per, (i + 1) per).
+    const int per = (p.batch + 31) / 32, b0 = min(lane * per, p.batch), b1 = min(b0 + per, p.batch);
     int sum = 0, longest = 0;
-    for (int i = lane; i < p.batch; i += 32) {
-      sum += pref[i + 1];
-      longest = max(longest, pref[i + 1]);
+    for (int i = b0; i < b1; ++i) {
+      const int nt = seq_tiles(p, cfg, geo.max_tiles, i).nt;
+      sum += nt;
+      longest = max(longest, nt);
     }
     sum = __reduce_add_sync(0xffffffffu, sum);
     longest = __reduce_max_sync(0xffffffffu, longest);
     const int64_t work = (int64_t)sum * U;
-    int size = (int)((work + geo.resident - 1) / geo.resident);
+    int size = (int)((work + geo.resident - 1) / geo.resident), mine = 0;
+    auto count_pieces = [&]() {
+      mine = 0;
+      for (int i = b0; i < b1; ++i) mine += (seq_tiles(p, cfg, geo.max_tiles, i).nt + size - 1) / size;
+    };
     if (size > kOneWave) {
       size = max(kOneWave / 2, (int)((work + kWaves * geo.resident - 1) / (kWaves * geo.resident)));
+      count_pieces();
     } else {
       size = max(size, (int)ceilf((float)longest / ceilf(sqrtf(7.f * longest))));
       for (; size < longest; size += max(1, size >> 3)) {
-        int n = 0;
-        for (int i = lane; i < p.batch; i += 32) n += (pref[i + 1] + size - 1) / size;
-        if (__reduce_add_sync(0xffffffffu, n) * U <= geo.resident) break;
+        count_pieces();
+        if (__reduce_add_sync(0xffffffffu, mine) * U <= geo.resident) break;
       }
     }
-    __syncthreads();
-    // number of pieces before each sequence
-    const int per = (p.batch + NT - 1) / NT;
-    int mine = 0;
-    for (int i = 0; i < per; ++i) {
-      const int bb = tid * per + i;
-      if (bb < p.batch) {
-        mine += (pref[bb + 1] + size - 1) / size;
-        pref[bb + 1] = mine;
-      }
-    }
-    int inc = mine;
+    if (size >= longest) {                       // every sequence in one piece
+      if (share >= p.batch) return;
+      b = base = share;
+      parts = 1;
+    } else {
+      int inc = mine;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int x = __shfl_up_sync(0xffffffffu, inc, o);
-      if (lane >= o) inc += x;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += x;
+      }
+      const bool owner = share >= inc - mine && share < inc;
+      const unsigned who = __ballot_sync(0xffffffffu, owner);
+      if (who == 0u) return;                       // the grid is sized for a full cache
+      base = inc - mine;
+      b = b0;
+      parts = 0;
+      if (owner) {
+        for (;; ++b) {
+          parts = (seq_tiles(p, cfg, geo.max_tiles, b).nt + size - 1) / size;
+          if (share < base + parts) break;
+          base += parts;
+        }
+      }
+      const int src = __ffs(who) - 1;
+      b = __shfl_sync(0xffffffffu, b, src);
+      base = __shfl_sync(0xffffffffu, base, src);
+      parts = __shfl_sync(0xffffffffu, parts, src);
     }
-    int* wsum = reinterpret_cast<int*>(sM);
-    if (lane == 31) wsum[warp] = inc;
-    if (tid == 0) pref[0] = 0;
-    __syncthreads();
-    int before = inc - mine;
-    for (int i = 0; i < warp; ++i) before += wsum[i];
-    for (int i = 0; i < per; ++i) {
-      const int bb = tid * per + i;
-      if (bb < p.batch) pref[bb + 1] += before;
-    }
-    __syncthreads();
-    if (share >= pref[p.batch]) return;          // the grid is sized for a full cache
-    int lo = 0, hi = p.batch;                    // pref[lo] <= share < pref[hi]
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (pref[mid] <= share) lo = mid;
-      else hi = mid;
-    }
-    b = lo;
-    base = pref[lo];
-    parts = pref[lo + 1] - base;
     w = seq_tiles(p, cfg, geo.max_tiles, b);
   } else {
     b = share / geo.splits;
@@ -695,7 +691,7 @@ int decode_num_counters(const fa_decode_args& a) { return a.batch * a.heads_kv *
 //   * more work than that runs as kWaves waves, which the hardware balances over SMs of unequal speed
 //     (64 sequences of 16000 keys: one wave of equal shares 688 us, 3.5 waves 656 us = 0.98 of the copy
 //     bandwidth).
-// An explicit num_splits, and batches too large to sum in every CTA, cut every sequence into the
+// An explicit num_splits, and batches too large to sum in every warp, cut every sequence into the
 // same number of pieces.
 static DecodeGeom decode_geometry(const fa_decode_args& a) {
   DecodeGeom g;
@@ -739,7 +735,7 @@ size_t decode_workspace_bytes(const fa_decode_args& a) {
 template <typename T, int D, int kRows>
 static int launch_rows(const fa_decode_args& a, const ScoreCfg& cfg, const DecodeGeom& g, const DecodeCheck& chk,
                          cudaStream_t st) {
-  const size_t smem = DecodeSmem<D, kRows>::fixed + (g.splits ? 0 : (a.batch + 1) * sizeof(int));
+  const size_t smem = DecodeSmem<D, kRows>::fixed;
   auto kern = decode_kernel<T, D, kRows>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) {
