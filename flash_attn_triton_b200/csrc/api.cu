@@ -108,6 +108,9 @@ int fwd_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 bool bwd_sm100_supported(const fa_attn_args&);
 int bwd_dq_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int bwd_dkdv_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
+int fwd_alt_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
+int fwd_alt_sm100_status();
+int fwd_alt_sm100_clear_status();
 int decode_paged(const fa_decode_args&, cudaStream_t);
 int decode_paged_checked(const fa_decode_args&, uint32_t*, cudaStream_t);
 int decode_num_counters(const fa_decode_args&);
@@ -465,6 +468,7 @@ int fa_device_wait_status(int device) {
   }
   int s = fwd_sm100_status();
   if (s == 0) s = bwd_sm100_status();
+  if (s == 0) s = fwd_alt_sm100_status();
   if (s == 0) s = host_wait_status(device);
   if (s != 0 && device >= 0 && device < 1024) g_host_wait[device] = s;   // remembered for the launchers
   return s;
@@ -479,6 +483,7 @@ int fa_device_wait_clear(int device) {
   }
   fwd_sm100_clear_status();
   bwd_sm100_clear_status();
+  fwd_alt_sm100_clear_status();
   if (device >= 0 && device < 1024) g_host_wait[device] = 0;
   return FA_OK;
 }

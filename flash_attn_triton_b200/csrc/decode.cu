@@ -30,6 +30,7 @@
 #include <cmath>
 #include <mutex>
 
+#include "cache_geo.cuh"
 #include "common.cuh"
 
 namespace fa {
@@ -82,6 +83,9 @@ __device__ __forceinline__ uint32_t decode_checks(const fa_decode_args& p, int t
          (__syncthreads_or(bad & FA_CHECK_LENGTHS) ? FA_CHECK_LENGTHS : 0u) |
          (__syncthreads_or(bad & FA_CHECK_ROTARY) ? FA_CHECK_ROTARY : 0u);
 }
+
+int cache_attention_sm100(const fa_decode_args& d, const void* q, const int64_t* q_stride, const CacheGeo& geo,
+                          const ScoreCfg& cfg, cudaStream_t st);
 
 __global__ void __launch_bounds__(1024) decode_check_kernel(const fa_decode_args p, uint32_t* host, uint32_t* dev) {
   const uint32_t bad = decode_checks(p, threadIdx.x, blockDim.x);
@@ -675,12 +679,137 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
 // ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
+static int page_shift_of(const fa_decode_args& a) {
+  if (a.page_size <= 0 || (a.page_size & (a.page_size - 1)) != 0) return -1;
+  int s = 0;
+  while ((1 << s) < a.page_size) ++s;
+  return s;
+}
 static int decode_unit_rows(const fa_decode_args& a) { return a.seqlen_q * (a.heads_q / a.heads_kv) <= 8 ? 8 : 16; }
 static int decode_row_groups(const fa_decode_args& a) {
   const int n = decode_unit_rows(a);
   return (a.seqlen_q * (a.heads_q / a.heads_kv) + n - 1) / n;
 }
-int decode_num_counters(const fa_decode_args& a) { return a.batch * a.heads_kv * decode_row_groups(a); }
+
+// ---------------------------------------------------------------------------------------
+// Chunks of tokens: more than 16 query rows per KV head.  The kernel above would read the cache once per 16
+// rows; these calls append and rotate in a kernel of their own and attend on the tensor cores
+// (fwd_alt_sm100.cu), which takes about as long for 128 rows as the kernel above for 16.
+// ---------------------------------------------------------------------------------------
+// 8 elements of a head row, rotated like rotary_elem.
+template <typename T>
+__device__ __forceinline__ uint4 rotary_chunk(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
+                                              int interleaved, int rotary_seqlen) {
+  union { uint4 v; T e[8]; } out, self, other, c, s;
+  self.v = *reinterpret_cast<const uint4*>(x + d);
+  if (cos == nullptr || d >= rotary_dim || pos < 0 || pos >= rotary_seqlen) return self.v;
+  const int half = rotary_dim >> 1;
+  if (!interleaved && half % 8 == 0 && ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 15) == 0) {
+    const bool first = d < half;
+    const int i = first ? d : d - half;
+    other.v = *reinterpret_cast<const uint4*>(x + (first ? d + half : d - half));
+    c.v = *reinterpret_cast<const uint4*>(cos + (int64_t)pos * half + i);
+    s.v = *reinterpret_cast<const uint4*>(sin + (int64_t)pos * half + i);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      out.e[k] = first ? hsub_rn(hmul_rn(self.e[k], c.e[k]), hmul_rn(other.e[k], s.e[k]))
+                       : hadd_rn(hmul_rn(other.e[k], s.e[k]), hmul_rn(self.e[k], c.e[k]));
+    return out.v;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    out.e[k] = rotary_elem<T>([&](int j) { return x[j]; }, d + k, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+  return out.v;
+}
+
+// New keys (rotated) and values into the cache, rotated queries into q_out (batch, tokens, heads, D); one
+// 16-byte chunk per thread, HBM-bound.  host / dev: value checks made by every CTA, see decode_kernel.
+template <typename T>
+__global__ void __launch_bounds__(256) cache_append_kernel(const fa_decode_args p, T* q_out, int page_shift, uint32_t* host,
+                                                           uint32_t* dev, bool check_here) {
+  if (check_here) {
+    const uint32_t bad = decode_checks(p, threadIdx.x, 256);
+    if (threadIdx.x == 0 && blockIdx.x == 0) {
+      *dev = bad;
+      *reinterpret_cast<volatile uint32_t*>(host) = bad | kCheckDone;
+      __threadfence_system();
+    }
+    if (bad) return;
+  } else if (dev && *dev) {
+    return;
+  }
+  const int D = p.head_dim, cpr = D / 8;
+  const int n_new = p.k_new ? p.seqlen_new : 0;
+  const int64_t nq = q_out ? (int64_t)p.batch * p.seqlen_q * p.heads_q * cpr : 0;
+  const int64_t nk = (int64_t)p.batch * n_new * p.heads_kv * cpr;
+  const T* cos = reinterpret_cast<const T*>(p.rotary_cos);
+  const T* sin = reinterpret_cast<const T*>(p.rotary_sin);
+  int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i < nq) {
+    const int d = (int)(i % cpr) * 8, h = (int)(i / cpr % p.heads_q);
+    const int64_t bt = i / ((int64_t)cpr * p.heads_q);
+    const int tok = (int)(bt % p.seqlen_q), b = (int)(bt / p.seqlen_q);
+    const int pos = p.cache_seqlens[b] + n_new - p.seqlen_q + tok + (p.cache_leftpad ? p.cache_leftpad[b] : 0);
+    const T* x = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + tok * p.q_stride[1] + h * p.q_stride[2];
+    *reinterpret_cast<uint4*>(q_out + i * 8) =
+        rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+    return;
+  }
+  i -= nq;
+  if (i >= 2 * nk) return;
+  const bool val = i >= nk;
+  if (val) i -= nk;
+  const int d = (int)(i % cpr) * 8, h = (int)(i / cpr % p.heads_kv);
+  const int64_t bt = i / ((int64_t)cpr * p.heads_kv);
+  const int tok = (int)(bt % n_new), b = (int)(bt / n_new);
+  const int pos = p.cache_seqlens[b] + tok + (p.cache_leftpad ? p.cache_leftpad[b] : 0);
+  if (val) {
+    const T* x = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + h * p.vn_stride[2];
+    T* dst = reinterpret_cast<T*>(p.v_cache) + cache_row_offset(p, b, pos, page_shift, p.vc_stride) + h * p.vc_stride[2];
+    *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(x + d);
+  } else {
+    const T* x = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + h * p.kn_stride[2];
+    T* dst = reinterpret_cast<T*>(p.k_cache) + cache_row_offset(p, b, pos, page_shift, p.kc_stride) + h * p.kc_stride[2];
+    *reinterpret_cast<uint4*>(dst + d) = rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+  }
+}
+
+struct ChunkPlan {
+  int pack_log2, units, parts, capacity;
+  size_t q_bytes, piece_bytes;   // workspace: rotated queries, pieces, then the counters if the caller brings none
+};
+// Whether a call is a chunk, and how it is cut.
+static bool chunk_plan(const fa_decode_args& a, ChunkPlan& c) {
+  const int G = a.heads_q / a.heads_kv;
+  if (a.num_splits != 0 || a.seqlen_q * G <= 16 || a.softmax_scale < 0.f) return false;
+  if (a.head_dim != 64 && a.head_dim != 128 && a.head_dim != 256) return false;
+  if (a.block_table) {       // a tile of 128 keys is whole pages, or lies inside one
+    const bool pow2 = (a.page_size & (a.page_size - 1)) == 0;
+    if (!(pow2 && a.page_size >= 16 && a.page_size < 128) && a.page_size % 128 != 0) return false;
+  }
+  c.pack_log2 = 0;
+  if ((G & (G - 1)) == 0 && G <= 64)
+    while ((1 << c.pack_log2) < G) ++c.pack_log2;
+  const int64_t cap = a.block_table ? (int64_t)a.block_table_stride * a.page_size : a.page_size;
+  const int mtiles = (int)((((int64_t)a.seqlen_q << c.pack_log2) + 127) / 128);
+  const int64_t units = (int64_t)a.batch * (a.heads_q >> c.pack_log2) * mtiles;
+  if (units > (1 << 28) || cap > (1 << 30)) return false;
+  c.units = (int)units;
+  c.capacity = (int)cap;
+  // pieces of at least four key tiles, only while the units leave SMs idle
+  const int64_t fill = sm_count(a.device) / units, most = (cap + 511) / 512;
+  c.parts = (int)(fill < most ? fill : most);
+  if (c.parts < 1) c.parts = 1;
+  c.q_bytes = a.rotary_cos ? (size_t)a.batch * a.seqlen_q * a.heads_q * a.head_dim * 2 : 0;
+  c.piece_bytes = c.parts > 1 ? (size_t)c.units * c.parts * 128 * (a.head_dim + 1) * sizeof(float) : 0;
+  return true;
+}
+
+int decode_num_counters(const fa_decode_args& a) {
+  ChunkPlan c;
+  if (chunk_plan(a, c)) return c.parts > 1 ? c.units : 0;
+  return a.batch * a.heads_kv * decode_row_groups(a);
+}
 
 // Room for the pieces the kernel may make.  It picks their size so that
 //   * one wave of CTAs (two per SM, one at head_dim 256) takes all of them, while that needs no more
@@ -711,12 +840,7 @@ static DecodeGeom decode_geometry(const fa_decode_args& a) {
     n += whole;                                // rounding up adds less than a piece per sequence
     g.shares = (int)(n < most ? n : most);
   }
-  g.page_shift = -1;
-  if (a.page_size > 0 && (a.page_size & (a.page_size - 1)) == 0) {
-    int s = 0;
-    while ((1 << s) < a.page_size) ++s;
-    g.page_shift = s;
-  }
+  g.page_shift = page_shift_of(a);
   return g;
 }
 
@@ -728,6 +852,11 @@ static size_t decode_piece_bytes(const fa_decode_args& a, const DecodeGeom& g) {
 }
 size_t decode_workspace_bytes(const fa_decode_args& a) {
   if (a.heads_kv <= 0 || a.heads_q <= 0 || a.batch <= 0 || a.seqlen_q <= 0) return 0;
+  ChunkPlan c;
+  if (chunk_plan(a, c)) {
+    if (c.q_bytes + c.piece_bytes == 0) return 0;
+    return c.q_bytes + c.piece_bytes + (c.parts > 1 && !a.counters ? (size_t)c.units * sizeof(uint32_t) : 0);
+  }
   const size_t pieces = decode_piece_bytes(a, decode_geometry(a));
   return pieces == 0 ? 0 : pieces + (a.counters ? 0 : (size_t)decode_num_counters(a) * sizeof(uint32_t));
 }
@@ -802,8 +931,68 @@ static int decode_run(const fa_decode_args& args, const DecodeCheck& chk, cudaSt
   return a.dtype == FA_BF16 ? decode_t<__nv_bfloat16>(a, cfg, g, chk, st) : decode_t<__half>(a, cfg, g, chk, st);
 }
 
+// host / dev: the slot of the value checks, or null; `inside`: made by the append kernel itself
+static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* host, uint32_t* dev, bool inside, cudaStream_t st) {
+  fa_decode_args a = args;
+  if (const int code = host_wait_status(a.device)) {
+    set_error("fa_decode_paged: a bounded device-side wait ran out earlier on device %d (code %d); the tcgen05 kernels stay "
+              "off until fa_device_wait_clear()", a.device, code);
+    return FA_ERR_DEVICE_WAIT;
+  }
+  const size_t need = decode_workspace_bytes(a);
+  if (need > 0 && (a.workspace == nullptr || a.workspace_bytes < need)) {
+    set_error("decode workspace too small: need %zu bytes, got %zu", need, a.workspace_bytes);
+    return FA_ERR_WORKSPACE;
+  }
+  char* ws = static_cast<char*>(a.workspace);
+  CacheGeo geo = {};
+  geo.seqlens = a.cache_seqlens;
+  geo.table = a.block_table;
+  geo.table_stride = a.block_table_stride;
+  geo.batch_idx = a.cache_batch_idx;
+  geo.leftpad = a.cache_leftpad;
+  geo.page_size = a.page_size;
+  geo.box_rows = a.block_table && a.page_size < 128 ? a.page_size : 128;
+  geo.n_new = a.k_new ? a.seqlen_new : 0;
+  geo.tokens = a.seqlen_q;
+  geo.pack_log2 = c.pack_log2;
+  geo.parts = c.parts;
+  geo.capacity = c.capacity;
+  geo.ws = reinterpret_cast<float*>(ws + c.q_bytes);
+  geo.bad = dev;
+  if (c.parts > 1) {
+    FA_REQUIRE(a.counters == nullptr || a.num_counters >= c.units, "decode: too few counters");
+    geo.counters = a.counters;
+    if (geo.counters == nullptr) {
+      geo.counters = reinterpret_cast<uint32_t*>(ws + c.q_bytes + c.piece_bytes);
+      const cudaError_t e = cudaMemsetAsync(geo.counters, 0, (size_t)c.units * sizeof(uint32_t), st);
+      if (e != cudaSuccess) {
+        set_error("decode: cudaMemsetAsync: %s", cudaGetErrorString(e));
+        return FA_ERR_LAUNCH;
+      }
+    }
+  }
+  void* q_out = c.q_bytes ? ws : nullptr;
+  const int64_t chunks = ((q_out ? (int64_t)a.batch * a.seqlen_q * a.heads_q : 0) + 2ll * a.batch * geo.n_new * a.heads_kv) *
+                         (a.head_dim / 8);
+  if (chunks > 0 || inside) {
+    const unsigned grid = (unsigned)(chunks > 0 ? (chunks + 255) / 256 : 1);
+    const int shift = page_shift_of(a);
+    if (a.dtype == FA_BF16)
+      cache_append_kernel<<<grid, 256, 0, st>>>(a, static_cast<__nv_bfloat16*>(q_out), shift, host, dev, inside);
+    else
+      cache_append_kernel<<<grid, 256, 0, st>>>(a, static_cast<__half*>(q_out), shift, host, dev, inside);
+    if (int r = check_launch("cache_append")) return r;
+  }
+  const int64_t qs[3] = {(int64_t)a.seqlen_q * a.heads_q * a.head_dim, (int64_t)a.heads_q * a.head_dim, a.head_dim};
+  const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, a.window_left, a.window_right, a.alibi_slopes != nullptr);
+  return cache_attention_sm100(a, q_out ? q_out : a.q, q_out ? qs : a.q_stride, geo, cfg, st);
+}
+
 int decode_paged(const fa_decode_args& a, cudaStream_t st) {
   if (a.batch == 0 || a.seqlen_q == 0 || a.heads_q == 0) return FA_OK;
+  ChunkPlan c;
+  if (chunk_plan(a, c)) return chunk_run(a, c, nullptr, nullptr, false, st);
   return decode_run(a, DecodeCheck{nullptr, nullptr}, st);
 }
 
@@ -884,7 +1073,15 @@ int decode_paged_checked(const fa_decode_args& a, uint32_t* failed, cudaStream_t
   if (slot < 0) return FA_ERR_LAUNCH;
   const int64_t entries = (int64_t)a.batch * (a.block_table ? a.block_table_stride : 1);
   int r;
-  if (entries <= kInlineCheck) {
+  ChunkPlan c;
+  if (chunk_plan(a, c)) {
+    r = FA_OK;
+    if (entries > kInlineCheck) {
+      decode_check_kernel<<<1, 1024, 0, st>>>(a, host, dev);
+      r = check_launch("decode_check");
+    }
+    if (r == FA_OK) r = chunk_run(a, c, host, dev, entries <= kInlineCheck, st);
+  } else if (entries <= kInlineCheck) {
     r = decode_run(a, DecodeCheck{host, nullptr}, st);
   } else {
     decode_check_kernel<<<1, 1024, 0, st>>>(a, host, dev);

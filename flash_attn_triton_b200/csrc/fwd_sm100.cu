@@ -752,7 +752,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 // host side
 // ---------------------------------------------------------------------------------------
 bool fwd_sm100_supported(const fa_attn_args& a) {
-  if (a.head_dim != 128 && a.head_dim != 64) return false;
+  if (a.head_dim != 256 && a.head_dim != 128 && a.head_dim != 64) return false;
   if (a.softmax_scale < 0.f) return false;
   if (a.batch == 0 || a.seqlen_q == 0 || a.seqlen_k == 0) return false;
   // tiny problems are launch-bound; the warp-level kernel has less fixed cost
@@ -806,7 +806,10 @@ int fwd_persist_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t s
 int fwd_persist_sm100_status();
 int fwd_persist_sm100_clear_status();
 
+int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st);
+
 int fwd_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
+  if (a.head_dim == 256) return fwd_alt_sm100(a, cfg, st);
   // FA_B200_FWD_PERSISTENT_FROM in the environment overrides the threshold (tests run the
   // persistent kernel on small shapes with it; 0 = never)
   int from = FA_FWD_PERSISTENT_FROM;
