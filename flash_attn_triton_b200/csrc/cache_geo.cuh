@@ -11,6 +11,7 @@ struct CacheGeo {
   const int* leftpad;      // or null
   int table_stride;
   int page_size;           // rows of a page (of a sequence when contiguous)
+  int page_log2;           // of page_size, or -1
   int box_rows;            // rows of one TMA box: min(page_size, 128)
   int n_new;               // tokens appended by the call
   int tokens;              // query tokens of a sequence

@@ -952,6 +952,7 @@ static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* h
   geo.batch_idx = a.cache_batch_idx;
   geo.leftpad = a.cache_leftpad;
   geo.page_size = a.page_size;
+  geo.page_log2 = page_shift_of(a);
   geo.box_rows = a.block_table && a.page_size < 128 ? a.page_size : 128;
   geo.n_new = a.k_new ? a.seqlen_new : 0;
   geo.tokens = a.seqlen_q;

@@ -235,7 +235,7 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   } else if (warp == 8) {
     // ------------------------------- TMA producer ---------------------------------------
     reg_dealloc<72>();
-    if (nt > 0) {
+    if (nt > 0 && (lane == 0 || (kCache && geo.box_rows < kBN))) {
       if (lane == 0) {
         prefetch_tmap(&tmQ);
         prefetch_tmap(&tmK);
@@ -249,42 +249,48 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      // page of box `lane` of a key tile (boxes of one page each; a contiguous cache is one page);
-      // read one tile ahead of its use
-      const int boxes = kCache ? kBN / geo.box_rows : 1;
+      // Page of box `lane` of a key tile (boxes of one page each; a contiguous cache is one page); read one
+      // tile ahead of its use.  No divisions here and no lock-step of the warp unless a tile has several
+      // boxes: with both, a load took this warp 900 cycles, and two of them per tile were what bounded
+      // the kernel.
+      const bool many = kCache && geo.box_rows < kBN;
+      const int box_log2 = many ? 31 - __clz(geo.box_rows) : 7;
       auto page_of = [&](int tile) {
         int pg = w.batch_row;
         if (kCache && geo.table) {
-          const int key = tile * kBN + lane * geo.box_rows;
-          pg = (lane < boxes && key < w.k_len) ? geo.table[(int64_t)w.b * geo.table_stride + key / geo.page_size] : 0;
+          const int key = tile * kBN + (many ? lane << box_log2 : 0);
+          pg = (lane < (kBN >> box_log2) && key < w.k_len)
+                   ? geo.table[(int64_t)w.b * geo.table_stride + (geo.page_log2 >= 0 ? key >> geo.page_log2 : key / geo.page_size)]
+                   : 0;
         }
         return pg;
       };
       auto load_tile = [&](const CUtensorMap* tm, int tile, int pages) {
-        for (int un = 0; un < NU && ok; ++un) {
-          if (lane == 0) ok = wait_bar(&sh->kv_empty[stage], phase ^ 1, sh, 11);
-          ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
-          if (!ok) return;
+#pragma unroll
+        for (int un = 0; un < NU; ++un) {
           const uint32_t bar = smem_u32(&sh->kv_full[stage]);
           const uint32_t dst = sKV + stage * C::kUnitBytes;
-          if (kCache) {
+          if (many) {
             // boxes that start past the last key are not loaded (their rows are masked, and zeroed in V)
-            const int key0 = tile * kBN;
-            const int n = min(boxes, (w.k_len - key0 + geo.box_rows - 1) / geo.box_rows);
-            if (lane == 0) mbar_expect_tx(bar, n * geo.box_rows * C::kUnitCols * 2);
-            for (int i = 0; i < n; ++i) {
-              const int pg = __shfl_sync(0xffffffffu, pages, i);
-              const int key = key0 + i * geo.box_rows;
-              const int row = geo.table ? key % geo.page_size : key + w.key_off;
-              if (lane == 0) {
-                for (int bx = 0; bx < C::kBoxes; ++bx)
-                  tma_load_4d(dst + bx * (kBN * 128) + i * geo.box_rows * 128, tm, bar, un * C::kUnitCols + bx * 64, w.hk, row, pg);
-              }
+            if (lane == 0) ok = ok && wait_bar(&sh->kv_empty[stage], phase ^ 1, sh, 11);
+            ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+            if (!ok) return;
+            const int n = min(kBN >> box_log2, ((w.k_len - tile * kBN - 1) >> box_log2) + 1);
+            if (lane == 0) mbar_expect_tx(bar, n * (C::kUnitCols * 2 << box_log2));
+            __syncwarp();
+            if (lane < n) {
+              for (int bx = 0; bx < C::kBoxes; ++bx)
+                tma_load_4d(dst + bx * (kBN * 128) + (lane << box_log2) * 128, tm, bar, un * C::kUnitCols + bx * 64, w.hk, 0, pages);
             }
           } else if (lane == 0) {
+            ok = ok && wait_bar(&sh->kv_empty[stage], phase ^ 1, sh, 11);
+            if (!ok) return;
+            const int row = !kCache || geo.table == nullptr ? tile * kBN + w.key_off
+                            : geo.page_log2 >= 0            ? (tile * kBN) & (geo.page_size - 1)
+                                                            : (tile * kBN) % geo.page_size;
             mbar_expect_tx(bar, C::kUnitBytes);
             for (int bx = 0; bx < C::kBoxes; ++bx)
-              tma_load_4d(dst + bx * (kBN * 128), tm, bar, un * C::kUnitCols + bx * 64, w.hk, w.key_off + tile * kBN, pages);
+              tma_load_4d(dst + bx * (kBN * 128), tm, bar, un * C::kUnitCols + bx * 64, w.hk, row, pages);
           }
           if (++stage == S) { stage = 0; phase ^= 1; }
         }
@@ -678,28 +684,48 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           __threadfence();
           const int64_t s0 = (int64_t)(blockIdx.x / geo.parts) * geo.parts;
           const int rows = min(kBM, w.rows - w.m0);
-          for (int i = tid; i < rows * (D / 4); i += 256) {
-            const int r = i / (D / 4), d = (i % (D / 4)) * 4, gr = w.m0 + r;
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            float wsum = 0.f, m = -INFINITY;
+          // weights of the pieces per row, over the ring (every K/V tile has been read)
+          float* wt = reinterpret_cast<float*>(tiles + C::kQBytes);
+          if (tid < rows) {
+            float m = -INFINITY, sum = 0.f;
+            for (int s = 0; s < w.parts; ++s) m = fmaxf(m, ws_l[(s0 + s) * kBM + tid]);
             for (int s = 0; s < w.parts; ++s) {
-              const float ls = ws_l[(s0 + s) * kBM + r];
-              const float4 v = *reinterpret_cast<const float4*>(geo.ws + ((s0 + s) * kBM + r) * D + d);
-              const float mn = fmaxf(m, ls);
-              if (mn == -INFINITY) continue;
-              const float a = exp2f(m - mn), b = exp2f(ls - mn);
-              acc.x = acc.x * a + b * v.x; acc.y = acc.y * a + b * v.y;
-              acc.z = acc.z * a + b * v.z; acc.w = acc.w * a + b * v.w;
-              wsum = wsum * a + b;
-              m = mn;
+              const float v = m == -INFINITY ? 0.f : exp2f(ws_l[(s0 + s) * kBM + tid] - m);
+              wt[s * kBM + tid] = v;
+              sum += v;
             }
-            const float f = wsum > 0.f ? 1.f / wsum : 0.f;
-            uint2 pk;
-            pk.x = Elem<T>::pack(acc.x * f, acc.y * f);
-            pk.y = Elem<T>::pack(acc.z * f, acc.w * f);
-            *reinterpret_cast<uint2*>(reinterpret_cast<T*>(p.o) + (int64_t)w.q_boff * p.o_stride[0] +
-                                      (int64_t)(gr >> w.pack_log2) * p.o_stride[1] +
-                                      (int64_t)(w.h + (gr & ((1 << w.pack_log2) - 1))) * p.o_stride[2] + d) = pk;
+            const float f = sum > 0.f ? 1.f / sum : 0.f;
+            for (int s = 0; s < w.parts; ++s) wt[s * kBM + tid] *= f;
+          }
+          asm volatile("bar.sync 1, 256;\n" ::: "memory");
+          // four elements of four rows per thread at a time, two pieces in flight each
+          constexpr int kStep = 256 / (D / 4);             // rows between a thread's items
+          const int d = (tid % (D / 4)) * 4;
+          for (int r0 = tid / (D / 4); r0 < rows; r0 += 4 * kStep) {
+            float4 acc[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+            for (int s = 0; s < w.parts; ++s) {
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const int r = min(r0 + k * kStep, rows - 1);
+                const float4 v = *reinterpret_cast<const float4*>(geo.ws + ((s0 + s) * kBM + r) * D + d);
+                const float f = wt[s * kBM + r];
+                acc[k].x += f * v.x; acc[k].y += f * v.y; acc[k].z += f * v.z; acc[k].w += f * v.w;
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const int r = r0 + k * kStep, gr = w.m0 + r;
+              if (r >= rows) break;
+              uint2 pk;
+              pk.x = Elem<T>::pack(acc[k].x, acc[k].y);
+              pk.y = Elem<T>::pack(acc[k].z, acc[k].w);
+              *reinterpret_cast<uint2*>(reinterpret_cast<T*>(p.o) + (int64_t)w.q_boff * p.o_stride[0] +
+                                        (int64_t)(gr >> w.pack_log2) * p.o_stride[1] +
+                                        (int64_t)(w.h + (gr & ((1 << w.pack_log2) - 1))) * p.o_stride[2] + d) = pk;
+            }
           }
         }
       }
