@@ -93,6 +93,11 @@ EXPORTS = {
     "fa_bwd_preprocess": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fa_bwd_dq": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fa_bwd_dkdv": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
+    "fa_dropout_bits_bytes": (C.c_size_t, [C.POINTER(AttnArgs), C.c_int32]),
+    "fa_dropout_bits": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.c_void_p]),
+    "fa_fwd_dropout": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.c_void_p]),
+    "fa_bwd_dq_dropout": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.c_void_p]),
+    "fa_bwd_dkdv_dropout": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.c_void_p]),
     "fa_attn_probs": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p, C.POINTER(C.c_int64 * 4), C.c_void_p, C.c_int64,
                                 C.c_void_p]),
     "fa_varlen_fwd": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),

@@ -110,6 +110,8 @@ int bwd_dq_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int bwd_dkdv_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int fwd_alt_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int fwd_alt_sm100_status();
+int64_t dropout_bits_words(int, int);
+int dropout_bits(const fa_attn_args&, const ScoreCfg&, uint32_t*, cudaStream_t);
 int fwd_alt_sm100_clear_status();
 int decode_paged(const fa_decode_args&, cudaStream_t);
 int decode_paged_checked(const fa_decode_args&, uint32_t*, cudaStream_t);
@@ -198,6 +200,20 @@ static ScoreCfg cfg_of(const fa_attn_args* a) {
 // Bias and dropout are features of the mma.sync kernels.
 static bool needs_mma(const fa_attn_args* a) { return a->attn_bias != nullptr || a->dropout_p > 0.f; }
 
+// Calls whose dropout mask the tcgen05 kernels read as bits: the plain dense variants of both kernels.
+// 64 MiB for the two copies is a square problem of 16384; longer ones draw per score.
+constexpr int64_t kDropoutBitsLimit = 64ll << 20;
+static int64_t dropout_bits_bytes(const fa_attn_args* a, bool backward) {
+  if (a == nullptr || !(a->dropout_p > 0.f) || a->impl != FA_IMPL_AUTO || a->cu_seqlens_q != nullptr || a->attn_bias != nullptr ||
+      a->alibi_slopes != nullptr || a->softcap > 0.f)
+    return 0;
+  if (a->head_dim != 64 && a->head_dim != 128) return 0;
+  if (!(a->softmax_scale * FA_LOG2E > 2e-5f)) return 0;     // see launch_dkdv in bwd_sm100.cu
+  if (!(backward ? bwd_sm100_supported(*a) : fwd_sm100_supported(*a))) return 0;
+  const int64_t bytes = 2 * 4 * dropout_bits_words(a->seqlen_q, a->seqlen_k);
+  return bytes <= kDropoutBitsLimit ? bytes : 0;
+}
+
 // A bounded wait that ran out earlier on this device (host mirror of the status word): the tcgen05
 // kernels would return at their first wait, so the call is refused before anything is launched.
 static int refuse_after_timeout(int device, const char* what) {
@@ -273,6 +289,30 @@ static int dkdv_impl(const fa_attn_args* a, void* stream, bool need_cu) {
   return bwd_dkdv_mma(*a, cfg, st);
 }
 
+enum DropoutOp { kDropFwd, kDropDq, kDropDkdv };
+
+static int dropout_impl(const fa_attn_args* a, const void* bits, void* stream, DropoutOp op) {
+  if (int r = validate_common(a, false)) return r;
+  FA_REQUIRE(dropout_bits_bytes(a, op != kDropFwd) > 0, "the call does not take its dropout mask as bits");
+  FA_REQUIRE(bits != nullptr && aligned16(bits), "dropout bits must be a 16-byte aligned buffer");
+  if (op != kDropFwd)
+    if (int r = validate_bwd(a)) return r;
+  if (op == kDropDq) FA_REQUIRE(a->dq && aligned16(a->dq) && mult8(a->dq_stride, 3), "dq pointer/alignment/stride");
+  if (op == kDropDkdv)
+    FA_REQUIRE(a->dk && a->dv && aligned16(a->dk) && aligned16(a->dv) && mult8(a->dk_stride, 3) && mult8(a->dv_stride, 3),
+               "dk/dv pointer/alignment/stride");
+  if (int r = refuse_after_timeout(a->device, op == kDropFwd ? "fa_fwd_dropout" : "fa_bwd_dropout")) return r;
+  if (int r = ensure_device(a->device)) return r;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  ScoreCfg cfg = cfg_of(a);
+  const int64_t tiles_q = (a->seqlen_q + 127) / 128, tiles_k = (a->seqlen_k + 127) / 128;
+  const uint32_t* words = static_cast<const uint32_t*>(bits);
+  cfg.drop_log2 = log2f(cfg.dropout_scale);
+  cfg.keep = op == kDropDkdv ? words + dropout_bits_words(a->seqlen_q, a->seqlen_k) : words;
+  cfg.keep_words = 4 * (op == kDropDkdv ? tiles_q : tiles_k);
+  return op == kDropFwd ? fwd_sm100(*a, cfg, st) : op == kDropDq ? bwd_dq_sm100(*a, cfg, st) : bwd_dkdv_sm100(*a, cfg, st);
+}
+
 }  // namespace fa
 
 using namespace fa;
@@ -302,6 +342,18 @@ int fa_bwd_dq(const fa_attn_args* a, void* stream) { return dq_impl(a, stream, f
 int fa_varlen_bwd_dq(const fa_attn_args* a, void* stream) { return dq_impl(a, stream, true); }
 int fa_bwd_dkdv(const fa_attn_args* a, void* stream) { return dkdv_impl(a, stream, false); }
 int fa_varlen_bwd_dkdv(const fa_attn_args* a, void* stream) { return dkdv_impl(a, stream, true); }
+
+size_t fa_dropout_bits_bytes(const fa_attn_args* a, int32_t backward) { return (size_t)dropout_bits_bytes(a, backward != 0); }
+int fa_dropout_bits(const fa_attn_args* a, void* bits, void* stream) {
+  if (int r = validate_common(a, false)) return r;
+  FA_REQUIRE(dropout_bits_bytes(a, false) > 0, "the call does not take its dropout mask as bits");
+  FA_REQUIRE(bits != nullptr && aligned16(bits), "dropout bits must be a 16-byte aligned buffer");
+  if (int r = ensure_device(a->device)) return r;
+  return dropout_bits(*a, cfg_of(a), static_cast<uint32_t*>(bits), reinterpret_cast<cudaStream_t>(stream));
+}
+int fa_fwd_dropout(const fa_attn_args* a, const void* bits, void* stream) { return dropout_impl(a, bits, stream, kDropFwd); }
+int fa_bwd_dq_dropout(const fa_attn_args* a, const void* bits, void* stream) { return dropout_impl(a, bits, stream, kDropDq); }
+int fa_bwd_dkdv_dropout(const fa_attn_args* a, const void* bits, void* stream) { return dropout_impl(a, bits, stream, kDropDkdv); }
 
 static int validate_decode(const fa_decode_args* a) {
   FA_REQUIRE(a != nullptr, "args is NULL");

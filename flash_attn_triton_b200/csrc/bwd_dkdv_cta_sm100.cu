@@ -159,7 +159,9 @@ __device__ __forceinline__ void mma_from_tmem(uint32_t d_tmem, uint32_t a_tmem, 
 // =======================================================================================
 // dK, dV
 // =======================================================================================
-template <typename T, int D, bool kExtras>
+// kDrop: P^T and dS^T are zero where the bit of (key, query row) in cfg.keep is 0, and scaled by
+// dropout_scale, which is folded into the statistics operand (its log2 is added to -lse2).
+template <typename T, int D, bool kExtras, bool kDrop>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -311,7 +313,7 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const int i = lane + 32 * k;
         // NEGATED; rows that do not exist or see no key get a large finite value instead of
         // infinity (an infinity would meet the zeros of the other GEMM's key-side operand): P = 0
-        float nl2 = -rl[k];
+        float nl2 = kDrop ? cfg.drop_log2 - rl[k] : -rl[k];
         const float ndl = fminf(fmaxf(-rd[k], -60000.f), 60000.f);   // kept inside the 16-bit range
         if (!(fabsf(nl2) < 60000.f)) nl2 = -60000.f;
         // the feature variant adds the LSE after the soft cap, in the element-wise warps
@@ -449,6 +451,8 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           st[i4 * 4] = l4.x; st[i4 * 4 + 1] = l4.y; st[i4 * 4 + 2] = l4.z; st[i4 * 4 + 3] = l4.w;
         }
       }
+      uint2 keep2;                                   // this thread's 64 bits of the tile, on their way during the wait
+      if (kDrop) keep2 = __ldg(reinterpret_cast<const uint2*>(cfg.keep + key * cfg.keep_words + (q0 >> 5)));
       ok = bwait(&sh->s_full[0], it & 1, sh, 46);
       if (!ok) break;
       tc_fence_after();
@@ -477,6 +481,7 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             else sc = sv * cfg.scale_log2;
             float pe = ex2(sc);
             if (masked) pe = col_visible(cm, i) ? pe : 0.f;
+            if (kDrop) pe = ((i < 32 ? keep2.x : keep2.y) >> (i & 31)) & 1u ? pe : 0.f;
             pf[i] = pe;
             // the tanh factor of the soft cap is folded into the copy kept for dS
             if (kExtras && cfg.softcap > 0.f) st[i] = 1.f - th * th;
@@ -487,7 +492,12 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           for (int i = 0; i < kHalfT; i += 2) {
             const uint32_t* rr = i < 32 ? r0 : r1;
             const float2 a = f2mul(make_float2(__uint_as_float(rr[i & 31]), __uint_as_float(rr[(i & 31) + 1])), c2);
-            const float2 pe = ex2_pair<kPolyEvery>(a, i >> 1);
+            float2 pe = ex2_pair<kPolyEvery>(a, i >> 1);
+            if (kDrop) {
+              const uint32_t kw = i < 32 ? keep2.x : keep2.y;
+              pe.x = (kw >> (i & 31)) & 1u ? pe.x : 0.f;
+              pe.y = (kw >> ((i & 31) + 1)) & 1u ? pe.y : 0.f;
+            }
             pf[i] = pe.x;
             pf[i + 1] = pe.y;
           }
@@ -659,7 +669,8 @@ int launch_dkdv(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
     set_error("bwd_dkdv_cta_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  auto kern = bwd_dkdv_cta_kernel<T, D, false>;   // the feature variants always take the persistent kernel
+  // the feature variants always take the persistent kernel
+  auto kern = cfg.keep != nullptr ? bwd_dkdv_cta_kernel<T, D, false, true> : bwd_dkdv_cta_kernel<T, D, false, false>;
   if (int r = set_smem_attr(kern, BCfg<D>::kSmemBytes, "bwd_dkdv_cta_sm100")) return r;
   dim3 grid((a.seqlen_k + kT - 1) / kT, a.heads_kv, a.batch);
   kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytes, st>>>(m.q, m.k, m.v, m.dout, m.dk, m.dv, a, cfg, host_wait_word(a.device));

@@ -1145,7 +1145,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 // =======================================================================================
 // dQ
 // =======================================================================================
-template <typename T, int D, bool kExtras>
+// kDrop: dS is zero where the bit of (query row, key) in cfg.keep is 0; the scale of the kept probabilities
+// is folded into the row's LSE.
+template <typename T, int D, bool kExtras, bool kDrop>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -1352,6 +1354,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         l2 = p.lse2[idx];
         dl = p.delta[idx];
         if (l2 == -INFINITY) l2 = INFINITY;
+        if (kDrop) l2 -= cfg.drop_log2;
       }
     };
     float l2n = INFINITY, dln = 0.f;
@@ -1396,6 +1399,8 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (cfg.wl >= 0) masked |= (k0 < w.m0 + kT - 1 + off - cfg.wl);
         if (cfg.wr >= 0) masked |= (k0 + kHalfT - 1 > w.m0 + off + cfg.wr);
 
+        uint2 keep2;                                   // this thread's 64 bits of the tile, on their way during the wait
+        if (kDrop) keep2 = __ldg(reinterpret_cast<const uint2*>(cfg.keep + row * cfg.keep_words + (k0 >> 5)));
         ok = bwait(&sh->s_full[tg & 1], (tg >> 1) & 1, sh, 56);
         if (!ok) break;
         tc_fence_after();
@@ -1447,6 +1452,11 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               if (kMask) {
                 pe.x = col_visible(cm, i) ? pe.x : 0.f;
                 pe.y = col_visible(cm, i + 1) ? pe.y : 0.f;
+              }
+              if (kDrop) {
+                const uint32_t kw = i < 32 ? keep2.x : keep2.y;
+                pe.x = (kw >> (i & 31)) & 1u ? pe.x : 0.f;
+                pe.y = (kw >> ((i & 31) + 1)) & 1u ? pe.y : 0.f;
               }
               pf[i] = pe.x;
               pf[i + 1] = pe.y;
@@ -1625,7 +1635,9 @@ int launch_dq(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
     return FA_ERR_LAUNCH;
   }
   const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
-  auto kern = extras ? bwd_dq_sm100_kernel<T, D, true> : bwd_dq_sm100_kernel<T, D, false>;
+  auto kern = cfg.keep != nullptr ? bwd_dq_sm100_kernel<T, D, false, true>
+              : extras            ? bwd_dq_sm100_kernel<T, D, true, false>
+                                  : bwd_dq_sm100_kernel<T, D, false, false>;
   if (int r = set_smem_attr(kern, BCfg<D>::kSmemBytesDq, "bwd_dq_sm100")) return r;
   const int nmb = (a.seqlen_q + kT - 1) / kT;
   int ncand = 0;
@@ -1672,7 +1684,7 @@ int bwd_dkdv_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) 
   const bool features = cfg.has_alibi || cfg.softcap > 0.f || !(cfg.scale_log2 > 2e-5f);
   double below = FA_DKDV_CTA_BELOW;
   if (const char* e = getenv("FA_B200_DKDV_CTA_BELOW")) below = atof(e);   // tuning / tests: 0 = never
-  if (!features && a.cu_seqlens_q == nullptr && dkdv_tiles_per_item(a, cfg) < below)
+  if (cfg.keep != nullptr || (!features && a.cu_seqlens_q == nullptr && dkdv_tiles_per_item(a, cfg) < below))
     return bwd_dkdv_cta_sm100(a, cfg, st);
   if (a.head_dim == 128)
     return a.dtype == FA_BF16 ? launch_dkdv<__nv_bfloat16, 128>(a, cfg, st) : launch_dkdv<__half, 128>(a, cfg, st);

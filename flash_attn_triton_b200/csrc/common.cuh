@@ -59,6 +59,11 @@ struct ScoreCfg {
   float dropout_scale;      // 1 / (1 - p)
   uint32_t seed_lo, seed_hi;
   uint32_t drop_stride;     // counter of element (row, col) = (row0 + row) * drop_stride + col
+  // the mask as bits (dropout_bits.cu), when the kernel reads it instead of drawing it: bit (j & 31) of word
+  // i * keep_words + (j >> 5), i = query row, j = key (dK/dV kernel: i = key, j = query row)
+  const uint32_t* keep;
+  int64_t keep_words;
+  float drop_log2;          // log2(dropout_scale)
 };
 
 __host__ __device__ inline ScoreCfg make_score_cfg(float scale, float softcap, int causal, int wl,
@@ -77,6 +82,9 @@ __host__ __device__ inline ScoreCfg make_score_cfg(float scale, float softcap, i
   c.dropout_p = 0.f;
   c.dropout_scale = 1.f;
   c.seed_lo = c.seed_hi = c.drop_stride = 0u;
+  c.keep = nullptr;
+  c.keep_words = 0;
+  c.drop_log2 = 0.f;
   return c;
 }
 

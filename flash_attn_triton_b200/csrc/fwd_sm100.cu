@@ -111,13 +111,16 @@ static_assert(sizeof(Shared) <= 4096, "Shared must fit its reserve");
 // kInt8: Q and K are int8 codes (tensor maps over the code buffers, 1 byte per element), QK^T is
 // tcgen05.mma.kind::i8 with an int32 accumulator, and the per-row / per-key scales sq, sk are
 // folded into the score epilogue; P@V stays in T.
-template <typename T, int D, bool kExtras, bool kInt8>
+// kDrop: probabilities whose bit in cfg.keep is 0 do not enter P@V (they stay in the row sum); the scale of
+// the kept ones goes into the normalisation of the output.
+template <typename T, int D, bool kExtras, bool kInt8, bool kDrop>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                  const fa_attn_args p, const ScoreCfg cfg, const float* __restrict__ sq,
                  const float* __restrict__ sk, int* const host_status) {
   static_assert(!kInt8 || D == 128, "the INT8 variant stages 128-byte code rows");
+  static_assert(!kDrop || (!kExtras && !kInt8), "dropout bits are read by the plain variant");
   // measured: 2-3 % faster on the plain variants, 2 % slower on the feature variant (whose
   // element-wise phase is three times as long, so the extra wait for the store costs more than
   // the early start gains)
@@ -403,6 +406,9 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (cfg.wl >= 0) masked |= (k0 < tq_max - cfg.wl);
       if (cfg.wr >= 0) masked |= (k0 + kBN - 1 > tq_min + cfg.wr);
 
+      uint4 keep4;                                   // the row's 128 bits of the tile, on their way during the wait
+      if (kDrop) keep4 = __ldg(reinterpret_cast<const uint4*>(cfg.keep + row * cfg.keep_words + (k0 >> 5)));
+
       PROF_T0();
       ok = wait_bar(&sh->s_full[x], t & 1, sh, 31 + x);
 #ifdef FA_PROF
@@ -647,9 +653,14 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           for (int i = 0; i < 32; i += 2) {
             const float2 a = f2fma(make_float2(__uint_as_float(r[cc][i]), __uint_as_float(r[cc][i + 1])), mul2, nm2);
             // the unmasked fast path holds no -inf scores: part of its exponentials may run on the FMA pipe
-            const float2 pe = prescaled ? make_float2(ex2(a.x), ex2(a.y)) : ex2_pair<kPolyEvery>(a, i >> 1);
-            pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
+            float2 pe = prescaled ? make_float2(ex2(a.x), ex2(a.y)) : ex2_pair<kPolyEvery>(a, i >> 1);
             acc2[(i >> 1) & 1] = f2add(acc2[(i >> 1) & 1], pe);
+            if (kDrop) {
+              const uint32_t kw = cc == 0 ? keep4.x : cc == 1 ? keep4.y : cc == 2 ? keep4.z : keep4.w;
+              pe.x = (kw >> i) & 1u ? pe.x : 0.f;
+              pe.y = (kw >> (i + 1)) & 1u ? pe.y : 0.f;
+            }
+            pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
           }
           tmem_st16(tSx + cc * 16, pk);
           if (kPvSplit && cc == 1) {
@@ -684,7 +695,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (ok && my_tiles == 0 && nsteps > 0) ok = wait_bar(&sh->q_full, 0, sh, 37);
     tc_fence_after();
     if (m0 < si.q_len && ok && sh->abort_flag == 0) {
-      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const float inv = l > 0.f ? (kDrop ? cfg.dropout_scale : 1.f) / l : 0.f;
       const bool row_ok = row < si.q_len;
       // The tile is staged in shared memory (over this stream's Q tile, which no MMA reads any
       // more) in the swizzled box layout and written by the TMA unit as full rows; a packed
@@ -783,7 +794,9 @@ static int launch(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st, i
     return FA_ERR_LAUNCH;
   }
   const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
-  auto kern = extras ? fwd_sm100_kernel<T, D, true, false> : fwd_sm100_kernel<T, D, false, false>;
+  auto kern = cfg.keep != nullptr ? fwd_sm100_kernel<T, D, false, false, true>
+              : extras            ? fwd_sm100_kernel<T, D, true, false, false>
+                                  : fwd_sm100_kernel<T, D, false, false, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
@@ -814,7 +827,8 @@ int fwd_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   // persistent kernel on small shapes with it; 0 = never)
   int from = FA_FWD_PERSISTENT_FROM;
   if (const char* e = getenv("FA_B200_FWD_PERSISTENT_FROM")) from = atoi(e);
-  if (from > 0 && a.seqlen_k >= from) return fwd_persist_sm100(a, cfg, st);
+  // with dropout bits this kernel takes every length: the persistent one has no such variant
+  if (cfg.keep == nullptr && from > 0 && a.seqlen_k >= from) return fwd_persist_sm100(a, cfg, st);
   // Row extents of the tensor maps.  Dense: the sequence length.  Packed: the caller does
   // not pass the total token count, so the map covers rows up to the int32 limit of the
   // cu_seqlens; tiles never start past cu_seqlens[batch], and rows past a sequence's end
@@ -875,7 +889,7 @@ int fwd_int8_sm100(const fa_int8_args& a, cudaStream_t st) {
   p.causal = a.causal;
   p.window_left = p.window_right = -1;
   const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
-  auto kern = fwd_sm100_kernel<__half, D, false, true>;
+  auto kern = fwd_sm100_kernel<__half, D, false, true, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_int8_sm100: cudaFuncSetAttribute: %s", cudaGetErrorString(e));

@@ -39,6 +39,11 @@ using torch::autograd::variable_list;
 typedef int (*AttnFn)(const fa_attn_args*, void*);
 struct Abi {
   AttnFn fwd, varlen_fwd, preprocess, bwd_dq, bwd_dkdv, varlen_bwd_dq, varlen_bwd_dkdv;
+  size_t (*bits_bytes)(const fa_attn_args*, int32_t);
+  int (*bits)(const fa_attn_args*, void*, void*);
+  int (*fwd_bits)(const fa_attn_args*, const void*, void*);
+  int (*bwd_dq_bits)(const fa_attn_args*, const void*, void*);
+  int (*bwd_dkdv_bits)(const fa_attn_args*, const void*, void*);
   int (*quantize_k)(const void*, int8_t*, float*, int64_t, int32_t, int32_t, void*);
   int (*fwd_int8)(const fa_int8_args*, void*);
   int (*decode)(const fa_decode_args*, void*);
@@ -205,6 +210,17 @@ c10::SmallVector<int64_t, 4> shape_of(const Params& c, const View& v) {
   return {v.batch, v.heads, v.rows, v.dim};
 }
 
+// The dropout mask of a call as bits, where its kernels read it that way; an undefined tensor otherwise.  It
+// is drawn again in the backward: that costs a few microseconds, keeping it would hold memory per layer.
+Tensor dropout_bits(const fa_attn_args& a, const Tensor& t, bool backward) {
+  if (!(a.dropout_p > 0.f)) return Tensor();
+  const size_t bytes = g_abi.bits_bytes(&a, backward);
+  if (bytes == 0) return Tensor();
+  Tensor bits = empty_cuda({(int64_t)bytes}, at::kByte, t.device());
+  check(g_abi.bits(&a, bits.mutable_data_ptr(), stream_of(t)), "fa_dropout_bits");
+  return bits;
+}
+
 // in: prepared inputs.  Fills out and (when wanted) lse.
 void run_forward(const Params& c, const variable_list& in, bool want_lse, Tensor& out, Tensor& lse) {
   View q, k, v;
@@ -214,7 +230,9 @@ void run_forward(const Params& c, const variable_list& in, bool want_lse, Tensor
   if (want_lse) lse = empty_cuda(lse_shape(c, q), at::kFloat, t.device());
   fa_attn_args a;
   fill(a, c, t, q, k, v, view_of(out, c.layout, -1, 0), want_lse ? lse.mutable_data_ptr<float>() : nullptr);
-  if (c.layout == kTHD) check(g_abi.varlen_fwd(&a, stream_of(t)), "fa_varlen_fwd");
+  const Tensor bits = dropout_bits(a, t, false);
+  if (bits.defined()) check(g_abi.fwd_bits(&a, bits.const_data_ptr(), stream_of(t)), "fa_fwd_dropout");
+  else if (c.layout == kTHD) check(g_abi.varlen_fwd(&a, stream_of(t)), "fa_varlen_fwd");
   else check(g_abi.fwd(&a, stream_of(t)), "fa_fwd");
 }
 
@@ -266,7 +284,11 @@ variable_list run_backward(const Params& c, const variable_list& in, const Tenso
   set_strides(a.dq_stride, dq); set_strides(a.dk_stride, dk); set_strides(a.dv_stride, dv);
   void* st = stream_of(t);
   check(g_abi.preprocess(&a, st), "fa_bwd_preprocess");
-  if (c.layout == kTHD) {
+  const Tensor bits = dropout_bits(a, t, true);
+  if (bits.defined()) {
+    if (need_dq) check(g_abi.bwd_dq_bits(&a, bits.const_data_ptr(), st), "fa_bwd_dq_dropout");
+    if (need_dkdv) check(g_abi.bwd_dkdv_bits(&a, bits.const_data_ptr(), st), "fa_bwd_dkdv_dropout");
+  } else if (c.layout == kTHD) {
     if (need_dq) check(g_abi.varlen_bwd_dq(&a, st), "fa_varlen_bwd_dq");
     if (need_dkdv) check(g_abi.varlen_bwd_dkdv(&a, st), "fa_varlen_bwd_dkdv");
   } else {
@@ -661,6 +683,11 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t n) {
   g_abi.bwd_dkdv = (AttnFn)get("fa_bwd_dkdv");
   g_abi.varlen_bwd_dq = (AttnFn)get("fa_varlen_bwd_dq");
   g_abi.varlen_bwd_dkdv = (AttnFn)get("fa_varlen_bwd_dkdv");
+  g_abi.bits_bytes = (decltype(g_abi.bits_bytes))get("fa_dropout_bits_bytes");
+  g_abi.bits = (decltype(g_abi.bits))get("fa_dropout_bits");
+  g_abi.fwd_bits = (decltype(g_abi.fwd_bits))get("fa_fwd_dropout");
+  g_abi.bwd_dq_bits = (decltype(g_abi.bwd_dq_bits))get("fa_bwd_dq_dropout");
+  g_abi.bwd_dkdv_bits = (decltype(g_abi.bwd_dkdv_bits))get("fa_bwd_dkdv_dropout");
   g_abi.quantize_k = (decltype(g_abi.quantize_k))get("fa_quantize_k_int8");
   g_abi.fwd_int8 = (decltype(g_abi.fwd_int8))get("fa_fwd_int8");
   g_abi.decode = (decltype(g_abi.decode))get("fa_decode_paged");

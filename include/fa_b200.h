@@ -112,7 +112,7 @@ typedef struct fa_attn_args {
    * (row0 + row) * dropout_row_stride + col) mapped to [0, 1) exceeds dropout_p; kept
    * probabilities are scaled by 1 / (1 - p); row0 = cu_seqlens_q[b] in the packed layout, else 0.
    * The same mask for every batch entry and head, as in the reference.  0 = off.
-   * Taken by the mma.sync kernels. */
+   * Taken by the mma.sync kernels, and by the tcgen05 ones through fa_fwd_dropout and its companions. */
   float dropout_p;
   int32_t dropout_row_stride;
   uint64_t dropout_seed;
@@ -137,6 +137,20 @@ int fa_bwd_dq(const fa_attn_args* args, void* stream);
  * Replaces the dK/dV half of _attn_bwd (attention_kernel.py:567-673, :873-962) and
  * _varlen_bwd_dkdv (attention_kernel.py:188-272). */
 int fa_bwd_dkdv(const fa_attn_args* args, void* stream);
+
+/*
+ * The same three operations with the dropout mask read as bits from `bits` instead of drawn per score, which
+ * lets the tcgen05 kernels take the call: the mask is the same for every batch entry and head.
+ * fa_dropout_bits_bytes gives the size of `bits` for a call, or 0 when the call keeps to fa_fwd / fa_bwd_dq /
+ * fa_bwd_dkdv (no dropout, packed layout, other features, shapes without a tcgen05 kernel, more than 64 MiB);
+ * `backward` != 0 asks for the two backward operations, which need both.  fa_dropout_bits fills it.
+ * 16-byte aligned, device memory of the caller.
+ */
+size_t fa_dropout_bits_bytes(const fa_attn_args* args, int32_t backward);
+int fa_dropout_bits(const fa_attn_args* args, void* bits, void* stream);
+int fa_fwd_dropout(const fa_attn_args* args, const void* bits, void* stream);
+int fa_bwd_dq_dropout(const fa_attn_args* args, const void* bits, void* stream);
+int fa_bwd_dkdv_dropout(const fa_attn_args* args, const void* bits, void* stream);
 
 /*
  * Attention probabilities as a matrix (the `return_attn_probs` surface,
