@@ -346,7 +346,8 @@ int fa_varlen_bwd_dkdv(const fa_attn_args* a, void* stream) { return dkdv_impl(a
 size_t fa_dropout_bits_bytes(const fa_attn_args* a, int32_t backward) { return (size_t)dropout_bits_bytes(a, backward != 0); }
 int fa_dropout_bits(const fa_attn_args* a, void* bits, void* stream) {
   if (int r = validate_common(a, false)) return r;
-  FA_REQUIRE(dropout_bits_bytes(a, false) > 0, "the call does not take its dropout mask as bits");
+  FA_REQUIRE(dropout_bits_bytes(a, false) > 0 || dropout_bits_bytes(a, true) > 0,
+             "the call does not take its dropout mask as bits");
   FA_REQUIRE(bits != nullptr && aligned16(bits), "dropout bits must be a 16-byte aligned buffer");
   if (int r = ensure_device(a->device)) return r;
   return dropout_bits(*a, cfg_of(a), static_cast<uint32_t*>(bits), reinterpret_cast<cudaStream_t>(stream));

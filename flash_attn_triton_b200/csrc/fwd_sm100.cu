@@ -766,8 +766,10 @@ bool fwd_sm100_supported(const fa_attn_args& a) {
   if (a.head_dim != 256 && a.head_dim != 128 && a.head_dim != 64) return false;
   if (a.softmax_scale < 0.f) return false;
   if (a.batch == 0 || a.seqlen_q == 0 || a.seqlen_k == 0) return false;
-  // tiny problems are launch-bound; the warp-level kernel has less fixed cost
-  if (a.impl == FA_IMPL_AUTO && a.seqlen_k < 256) return false;
+  // Below one key tile the warp-level kernel has less fixed cost (2 x 64 tokens, 4 heads of 64: 5.1 against
+  // 7.0 us; 16 x 100 of 32 heads 20 against 24); from a full tile on it is behind (16 x 128, 16 heads of 128:
+  // 20 against 16; 2 x 255, 4 heads of 128: 13.7 against 10.2; 16 x 200 of 16 heads 46 against 21).
+  if (a.impl == FA_IMPL_AUTO && a.seqlen_k < 128) return false;
   return true;
 }
 

@@ -45,7 +45,8 @@ def test_bits_are_the_reference_stream(Sq, Sk, p):
     (1, 257, 257, 2, 1, 128, dict(causal=True)),                      # one row, one key past the tiles
     (1, 300, 1000, 4, 2, 64, dict(causal=True)),
     (1, 700, 321, 2, 2, 128, dict(causal=True, window=(130, -1))),    # query tiles that see few keys
-    (1, 70, 513, 2, 2, 64, dict()),                                   # forward on bits, backward drawn per score
+    (1, 70, 513, 2, 2, 64, dict()),                                   # one short query tile
+    (2, 100, 90, 4, 2, 128, dict(causal=True)),                       # forward drawn per score, backward on bits
     (1, 2200, 2100, 1, 1, 64, dict(window=(300, 200))),               # longer than the persistent forward starts at
 ])
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
