@@ -3,6 +3,8 @@
 // fwd_persist_sm100.cu) do not fit:
 //
 //   head_dim 256   two output accumulators and two score buffers would need 768 tensor-memory columns;
+//   few tiles      dense problems of head_dim 64 and 128 with few tiles per SM, or very long ones: see
+//                  one_tile_is_faster() in fwd_sm100.cu;
 //   KV cache       a chunk of new tokens against a paged or contiguous cache.  The query heads of a KV head
 //                  are packed into the rows of a tile (row = token * group + head), so a K/V tile is
 //                  read once per group and a short chunk still fills its tile.
@@ -762,10 +764,9 @@ static int launch_alt(K kern, int smem, dim3 grid, cudaStream_t st, const CUtens
   return check_launch("fwd_alt_sm100");
 }
 
-// Dense or packed forward at head_dim 256.
-template <typename T>
-static int launch_256(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
-  constexpr int D = 256;
+// Dense or packed forward.  With ALiBi or a soft cap only head_dim 256 comes here (one_tile_is_faster()).
+template <typename T, int D>
+static int launch_rows(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   const bool packed = a.cu_seqlens_q != nullptr;
   const int64_t q_rows = packed ? a.total_q : a.seqlen_q, k_rows = packed ? a.total_k : a.seqlen_k;
   const int64_t batch = packed ? 1 : a.batch;
@@ -781,13 +782,17 @@ static int launch_256(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t s
   }
   const dim3 grid((a.seqlen_q + kBM - 1) / kBM, a.heads_q, a.batch);
   const CacheGeo geo = {};
-  if (cfg.has_alibi || cfg.softcap > 0.f)
-    return launch_alt(fwd_alt_sm100_kernel<T, D, true, false>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+  if constexpr (D == 256)
+    if (cfg.has_alibi || cfg.softcap > 0.f)
+      return launch_alt(fwd_alt_sm100_kernel<T, D, true, false>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
   return launch_alt(fwd_alt_sm100_kernel<T, D, false, false>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
 }
 
 int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
-  return a.dtype == FA_BF16 ? launch_256<__nv_bfloat16>(a, cfg, st) : launch_256<__half>(a, cfg, st);
+  const bool bf = a.dtype == FA_BF16;
+  if (a.head_dim == 64) return bf ? launch_rows<__nv_bfloat16, 64>(a, cfg, st) : launch_rows<__half, 64>(a, cfg, st);
+  if (a.head_dim == 128) return bf ? launch_rows<__nv_bfloat16, 128>(a, cfg, st) : launch_rows<__half, 128>(a, cfg, st);
+  return bf ? launch_rows<__nv_bfloat16, 256>(a, cfg, st) : launch_rows<__half, 256>(a, cfg, st);
 }
 
 template <typename T, int D>

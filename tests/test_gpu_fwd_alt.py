@@ -123,3 +123,29 @@ def test_cache_chunk_vs_oracle(case):
                                    cache_seqlens=dev(bad), cache_leftpad=dev(pad), block_table=dev(bt), **common)
     assert torch.equal(torch.nan_to_num(kcd.cpu(), nan=7.0), torch.nan_to_num(rkc, nan=7.0))
     assert N.lib().fa_device_wait_status(0) == 0
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,Sq,Sk,Hq,Hkv,causal,window", [
+    (1, 128, 128, 2, 1, True, (-1, -1)),          # one tile
+    (2, 129, 385, 2, 2, False, (-1, -1)),         # a row and a key past the tiles
+    (1, 640, 300, 4, 1, True, (-1, -1)),          # query tiles past the last key
+    (1, 700, 700, 2, 2, True, (150, -1)),         # tiles skipped, rows that see part of two tiles
+    (1, 2100, 2100, 12, 3, True, (-1, -1)),       # more CTAs than SMs
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_dense_routes(monkeypatch, B, Sq, Sk, Hq, Hkv, causal, window, D, dtype):
+    """The three dense forward kernels against the oracle on the same problem, rows past it untouched."""
+    from flash_attn_triton_b200 import _native as N, _ops
+    q, k, v, _ = (t.to(dtype) for t in cases.dense_case(Sq + Sk + D, B, Sq, Sk, Hq, Hkv, D))
+    ro, rl = orc.attention_ref(q, k, v, causal=causal, window=window)
+    for route in (None, "0", "1"):                # by the rule (the one-tile kernel here), two-tile, persistent
+        if route is None:
+            monkeypatch.delenv("FA_B200_FWD_PERSISTENT_FROM", raising=False)
+        else:
+            monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", route)
+        o, lse, _ = _ops.dense_forward(dev(q), dev(k), dev(v), D ** -0.5, causal, *window, 0.0, None, 0, N.IMPL_TCGEN05,
+                                       "bshd", True)
+        assert maxdiff(o, ro) <= util.tols(dtype)[0], route
+        assert maxdiff(lse * util.LN2, rl) <= util.tols(dtype)[0], route
+    assert N.lib().fa_device_wait_status(0) == 0
