@@ -12,7 +12,7 @@
 // lane collects its own column (a warp for the whole block left the chip idle: 6 us for 512 x 512).
 //
 // Bound: integer issue, 50 instructions per 1 / (batch * heads) of a score.  Measured on B200, forward + backward
-// of 8 x 512 tokens, 16 heads of 64, without a mask: 834 -> 123 us with the three attention kernels on tcgen05
+// of 8 x 512 tokens, 16 heads of 64, without a mask: 834 -> 117 us with the three attention kernels on tcgen05
 // and the bits drawn twice (once per direction: keeping them would hold memory per layer).
 #include "common.cuh"
 
