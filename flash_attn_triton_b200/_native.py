@@ -112,6 +112,8 @@ EXPORTS = {
     "fa_quantize_k_int8": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32,
                                      C.c_int32, C.c_void_p]),
     "fa_fwd_int8": (C.c_int, [C.POINTER(Int8Args), C.c_void_p]),
+    "fa_int8_codes16_bytes": (C.c_size_t, [C.POINTER(Int8Args)]),
+    "fa_fwd_int8_codes16": (C.c_int, [C.POINTER(Int8Args), C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "fa_rotary": (C.c_int, [C.POINTER(RotaryArgs), C.c_void_p]),
     "fa_gather_rows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64,
                                  C.c_int32, C.c_void_p]),

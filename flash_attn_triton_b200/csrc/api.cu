@@ -123,6 +123,9 @@ int quantize_k(const void*, int8_t*, float*, int64_t, int, cudaStream_t);
 int fwd_int8_mma(const fa_int8_args&, cudaStream_t);
 bool fwd_int8_sm100_supported(const fa_int8_args&);
 int fwd_int8_sm100(const fa_int8_args&, cudaStream_t);
+bool int8_codes16_supported(const fa_int8_args&);
+int quantize_codes16(const void*, void*, float*, int64_t, bool, cudaStream_t);
+int fwd_int8_codes16(const fa_int8_args&, const void*, const void*, cudaStream_t);
 int rotary(const fa_rotary_args&, cudaStream_t);
 int gather_rows(const void*, void*, const int64_t*, int64_t, int64_t, int64_t, int, cudaStream_t);
 int scatter_rows(const void*, void*, const int64_t*, int64_t, int64_t, int64_t, int, int, cudaStream_t);
@@ -461,6 +464,29 @@ int fa_fwd_int8(const fa_int8_args* a, void* stream) {
   }
   if (a->impl == FA_IMPL_AUTO && fwd_int8_sm100_supported(*a)) return fwd_int8_sm100(*a, st);
   return fwd_int8_mma(*a, st);
+}
+
+size_t fa_int8_codes16_bytes(const fa_int8_args* a) {
+  if (a == nullptr || a->batch <= 0 || a->heads <= 0 || a->seqlen <= 0 || !int8_codes16_supported(*a)) return 0;
+  return (size_t)a->batch * a->heads * a->seqlen * a->head_dim * 4;
+}
+
+int fa_fwd_int8_codes16(const fa_int8_args* a, const void* k, float* s_k, void* codes, void* stream) {
+  FA_REQUIRE(a != nullptr, "args is NULL");
+  FA_REQUIRE(fa_int8_codes16_bytes(a) > 0, "the call does not take its codes as 16-bit floats");
+  FA_REQUIRE(a->q && k && s_k && a->v && a->o && a->sq_scratch && codes, "NULL pointer");
+  FA_REQUIRE(a->seqlen_k_valid >= 0 && a->seqlen_k_valid <= a->seqlen, "seqlen_k_valid must lie in [0, seqlen]");
+  FA_REQUIRE(aligned16(a->q) && aligned16(k) && aligned16(a->v) && aligned16(a->o) && aligned16(codes), "16-byte alignment");
+  if (int r = refuse_after_timeout(a->device, "fa_fwd_int8_codes16")) return r;
+  if (int r = ensure_device(a->device)) return r;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const int64_t rows = (int64_t)a->batch * a->heads * a->seqlen;
+  void* k16 = static_cast<char*>(codes) + rows * a->head_dim * 2;
+  if (int r = quantize_codes16(a->q, codes, a->sq_scratch, rows, true, st)) return r;
+  if (int r = quantize_codes16(k, k16, s_k, rows, false, st)) return r;
+  fa_int8_args p = *a;
+  p.s_k = s_k;
+  return fwd_int8_codes16(p, codes, k16, st);
 }
 
 int fa_rotary(const fa_rotary_args* a, void* stream) {

@@ -108,18 +108,22 @@ static_assert(sizeof(Shared) <= 4096, "Shared must fit its reserve");
 
 }  // namespace
 
-// kInt8: Q and K are int8 codes (tensor maps over the code buffers, 1 byte per element), QK^T is
-// tcgen05.mma.kind::i8 with an int32 accumulator, and the per-row / per-key scales sq, sk are
-// folded into the score epilogue; P@V stays in T.
+// kInt8: INT8 scores; the per-row / per-key scales sq, sk are folded into the score epilogue, P@V stays in T.
+//   1  Q and K are int8 codes (tensor maps over the code buffers, 1 byte per element), QK^T is
+//      tcgen05.mma.kind::i8 with an int32 accumulator;
+//   2  the same codes as 16-bit floats (head_dim 64, whose rows of codes are half of the swizzle's 128 bytes): every
+//      product and partial sum is a whole number below 2^24, so the fp32 accumulator holds exactly the int32
+//      sums, and the conversion of a score to float falls away.  At head_dim 128 this form was measured 1-29 %
+//      slower than kind::i8 (twice the tensor cycles of the score GEMM, codes of twice the size).
 // kDrop: probabilities whose bit in cfg.keep is 0 do not enter P@V (they stay in the row sum); the scale of
 // the kept ones goes into the normalisation of the output.
-template <typename T, int D, bool kExtras, bool kInt8, bool kDrop>
+template <typename T, int D, bool kExtras, int kInt8, bool kDrop>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                  const fa_attn_args p, const ScoreCfg cfg, const float* __restrict__ sq,
                  const float* __restrict__ sk, int* const host_status) {
-  static_assert(!kInt8 || D == 128, "the INT8 variant stages 128-byte code rows");
+  static_assert(kInt8 != 1 || D == 128, "kind::i8 stages 128-byte code rows");
   static_assert(!kDrop || (!kExtras && !kInt8), "dropout bits are read by the plain variant");
   // measured: 2-3 % faster on the plain variants, 2 % slower on the feature variant (whose
   // element-wise phase is three times as long, so the extra wait for the store costs more than
@@ -228,7 +232,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       {
         const uint32_t bar = smem_u32(&sh->q_full);
         const int ntile = q1_loaded ? 2 : 1;
-        if (kInt8) {
+        if (kInt8 == 1) {
           mbar_expect_tx(bar, ntile * kBM * D);
           for (int x = 0; x < ntile; ++x)
             tma_load_4d(sQ + x * C::kTileBytes, &tmQ, bar, 0, h, (int)si.q_row0 + m00 + x * kBM, (int)si.q_boff);
@@ -260,10 +264,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (++stage == C::kStages) { stage = 0; phase ^= 1; }
       };
       // order of use: K_0, then V_j, K_{j+1}
-      load_kv(&tmK, n_hi - 1, kInt8);
+      load_kv(&tmK, n_hi - 1, kInt8 == 1);
       for (int j = 0; j < nsteps; ++j) {
         load_kv(&tmV, n_hi - 1 - j, false);
-        if (j + 1 < nsteps) load_kv(&tmK, n_hi - 2 - j, kInt8);
+        if (j + 1 < nsteps) load_kv(&tmK, n_hi - 2 - j, kInt8 == 1);
       }
     }
   } else if (warp == 9) {
@@ -287,7 +291,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       auto issue_qk = [&](int x, uint32_t kbase) {
         const uint64_t dq = make_smem_desc(sQ + x * C::kTileBytes, 16, 1024);
         const uint64_t dk = make_smem_desc(kbase, 16, 1024);
-        if (kInt8) {
+        if (kInt8 == 1) {
           constexpr uint32_t idesc_i8 = make_idesc(2, 1, 0, 0, kBM, kBN);  // s32 <- s8 x s8
           if (leader) {
 #pragma unroll
@@ -453,10 +457,13 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             for (int i4 = 0; i4 < 8; ++i4) {
               const float4 s4 = S4[cc * 8 + i4];
               const int i = i4 * 4;
-              const float2 a01 = f2add(make_float2(__uint_as_float(0x4B400000u + r[cc][i]),
-                                                   __uint_as_float(0x4B400000u + r[cc][i + 1])), nb2);
-              const float2 a23 = f2add(make_float2(__uint_as_float(0x4B400000u + r[cc][i + 2]),
-                                                   __uint_as_float(0x4B400000u + r[cc][i + 3])), nb2);
+              constexpr uint32_t kBias = kInt8 == 1 ? 0x4B400000u : 0u;
+              float2 a01 = make_float2(__uint_as_float(kBias + r[cc][i]), __uint_as_float(kBias + r[cc][i + 1]));
+              float2 a23 = make_float2(__uint_as_float(kBias + r[cc][i + 2]), __uint_as_float(kBias + r[cc][i + 3]));
+              if (kInt8 == 1) {
+                a01 = f2add(a01, nb2);
+                a23 = f2add(a23, nb2);
+              }
               // the per-query scale (positive, one value per thread) is applied after the maximum,
               // inside the FMA that forms the exp2 argument
               const float2 v01 = f2mul(a01, make_float2(s4.x, s4.y));
@@ -796,9 +803,9 @@ static int launch(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st, i
     return FA_ERR_LAUNCH;
   }
   const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
-  auto kern = cfg.keep != nullptr ? fwd_sm100_kernel<T, D, false, false, true>
-              : extras            ? fwd_sm100_kernel<T, D, true, false, false>
-                                  : fwd_sm100_kernel<T, D, false, false, false>;
+  auto kern = cfg.keep != nullptr ? fwd_sm100_kernel<T, D, false, 0, true>
+              : extras            ? fwd_sm100_kernel<T, D, true, 0, false>
+                                  : fwd_sm100_kernel<T, D, false, 0, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
@@ -873,6 +880,27 @@ int fwd_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
 // ---------------------------------------------------------------------------------------
 int quantize_q(const void* q, int8_t* q8, float* s_q, int64_t rows, int head_dim, cudaStream_t st);
 
+// The attention problem behind an INT8 call on contiguous head-major tensors.
+static fa_attn_args int8_problem(const fa_int8_args& a) {
+  fa_attn_args p;
+  memset(&p, 0, sizeof(p));
+  p.dtype = FA_F16;
+  const int B = a.batch, H = a.heads, S = a.seqlen, D = a.head_dim;
+  p.device = a.device;
+  p.batch = B; p.seqlen_q = S; p.heads_q = H; p.heads_kv = H; p.head_dim = D;
+  p.seqlen_k = a.seqlen_k_valid > 0 ? a.seqlen_k_valid : S;   // keys past it are padding (masked, tiles skipped)
+  p.total_q = p.total_k = S;                                  // rows of q8 / k8 and of the scale arrays
+  p.q_pos_offset = a.q_pos_offset;
+  p.o = a.o;
+  p.o_stride[0] = (int64_t)H * S * D; p.o_stride[1] = D; p.o_stride[2] = (int64_t)S * D;
+  p.lse2 = a.lse2;
+  p.lse_stride[0] = (int64_t)H * S; p.lse_stride[1] = 1; p.lse_stride[2] = S;
+  p.softmax_scale = a.softmax_scale;
+  p.causal = a.causal;
+  p.window_left = p.window_right = -1;
+  return p;
+}
+
 bool fwd_int8_sm100_supported(const fa_int8_args& a) {
   if (a.head_dim != 128 || a.softmax_scale < 0.f) return false;
   if (a.q8_scratch == nullptr || a.sq_scratch == nullptr) return false;
@@ -898,23 +926,9 @@ int fwd_int8_sm100(const fa_int8_args& a, cudaStream_t st) {
       return FA_ERR_LAUNCH;
     }
   }
-  fa_attn_args p;
-  memset(&p, 0, sizeof(p));
-  p.dtype = FA_F16;
-  p.device = a.device;
-  p.batch = B; p.seqlen_q = S; p.heads_q = H; p.heads_kv = H; p.head_dim = D;
-  p.seqlen_k = a.seqlen_k_valid > 0 ? a.seqlen_k_valid : S;   // keys past it are padding (masked, tiles skipped)
-  p.total_q = p.total_k = S;                                  // rows of q8 / k8 and of the scale arrays
-  p.q_pos_offset = a.q_pos_offset;
-  p.o = a.o;
-  p.o_stride[0] = (int64_t)H * S * D; p.o_stride[1] = D; p.o_stride[2] = (int64_t)S * D;
-  p.lse2 = a.lse2;
-  p.lse_stride[0] = (int64_t)H * S; p.lse_stride[1] = 1; p.lse_stride[2] = S;
-  p.softmax_scale = a.softmax_scale;
-  p.causal = a.causal;
-  p.window_left = p.window_right = -1;
+  const fa_attn_args p = int8_problem(a);
   const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
-  auto kern = fwd_sm100_kernel<__half, D, false, true, false>;
+  auto kern = fwd_sm100_kernel<__half, D, false, 1, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_int8_sm100: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -925,6 +939,39 @@ int fwd_int8_sm100(const fa_int8_args& a, cudaStream_t st) {
   return check_launch("fwd_int8_sm100");
 }
 
+
+// INT8 scores at head_dim 64, on codes held as 16-bit floats (kInt8 = 2).
+int fwd_int8_codes16(const fa_int8_args& a, const void* q16, const void* k16, cudaStream_t st) {
+  constexpr int D = 64;
+  using C = Cfg<D>;
+  const fa_attn_args p = int8_problem(a);
+  const int64_t stride[3] = {p.o_stride[0], p.o_stride[1], p.o_stride[2]};
+  CUtensorMap tq, tk, tv, to;
+  if (!make_map(&tq, q16, stride, a.seqlen, a.heads, a.batch, D, false) || !make_map(&tk, k16, stride, a.seqlen, a.heads, a.batch, D, false) ||
+      !make_map(&tv, a.v, stride, a.seqlen, a.heads, a.batch, D, false) || !make_map(&to, a.o, stride, a.seqlen, a.heads, a.batch, D, false)) {
+    set_error("fwd_int8_codes16: cuTensorMapEncodeTiled failed");
+    return FA_ERR_LAUNCH;
+  }
+  const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
+  auto kern = fwd_sm100_kernel<__half, D, false, 2, false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+  if (e != cudaSuccess) {
+    set_error("fwd_int8_codes16: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+    return FA_ERR_LAUNCH;
+  }
+  dim3 grid((a.seqlen + 2 * kBM - 1) / (2 * kBM), a.heads, a.batch);
+  kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, cfg, a.sq_scratch, a.s_k, host_wait_word(a.device));
+  return check_launch("fwd_int8_codes16");
+}
+
+// Whole calls against the mma.sync kernel, launches interleaved, with and without the causal mask: from 3e7 (query, key)
+// pairs over all heads on -5 to -49 % (32 heads x 1024 51 -> 41 us, 256 x 4096 2739 -> 1630 us causal, 32 x 8192
+// without a mask 2585 -> 1317 us); below that the two quantiser launches and the fixed cost of a CTA weigh more
+// (8 x 1024: 32 -> 38 us, 256 x 320: 46 -> 58 us).
+bool int8_codes16_supported(const fa_int8_args& a) {
+  if (a.head_dim != 64 || a.softmax_scale < 0.f || a.impl != FA_IMPL_AUTO || a.seqlen < 256) return false;
+  return (int64_t)a.batch * a.heads * a.seqlen * a.seqlen >= 30000000;
+}
 
 int fwd_sm100_status() {
   int v = 0;

@@ -46,6 +46,8 @@ struct Abi {
   int (*bwd_dkdv_bits)(const fa_attn_args*, const void*, void*);
   int (*quantize_k)(const void*, int8_t*, float*, int64_t, int32_t, int32_t, void*);
   int (*fwd_int8)(const fa_int8_args*, void*);
+  size_t (*int8_codes16_bytes)(const fa_int8_args*);
+  int (*fwd_int8_codes16)(const fa_int8_args*, const void*, float*, void*, void*);
   int (*decode)(const fa_decode_args*, void*);
   int (*decode_checked)(const fa_decode_args*, uint32_t*, void*);
   int32_t (*decode_counters)(const fa_decode_args*);
@@ -522,16 +524,14 @@ PyObject* py_int8(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const auto dev = q.device();
     const int64_t D = q.size(3), rows = k.numel() / D;
     void* st = stream_of(q);
-    Tensor k8 = empty_cuda(k.sizes(), at::kChar, dev), s_k = empty_cuda({rows}, at::kFloat, dev), q8, s_q;
-    check(g_abi.quantize_k(k.data_ptr(), k8.data_ptr<int8_t>(), s_k.data_ptr<float>(), rows, (int)D, dev.index(), st),
-          "fa_quantize_k_int8");
+    Tensor s_k = empty_cuda({rows}, at::kFloat, dev), k8, q8, s_q;
     o = empty_cuda(q.sizes(), at::kHalf, dev);
     fa_int8_args p;
     memset(&p, 0, sizeof(p));
     p.device = dev.index();
     p.impl = impl;
     p.batch = (int)q.size(0); p.heads = (int)q.size(1); p.seqlen = (int)q.size(2); p.head_dim = (int)D;
-    p.q = q.data_ptr(); p.k8 = k8.data_ptr<int8_t>(); p.s_k = s_k.data_ptr<float>(); p.v = v.data_ptr();
+    p.q = q.data_ptr(); p.s_k = s_k.data_ptr<float>(); p.v = v.data_ptr();
     p.o = o.data_ptr();
     if (want_lse) {
       l = empty_cuda({q.size(0), q.size(1), q.size(2)}, at::kFloat, dev);
@@ -541,6 +541,17 @@ PyObject* py_int8(PyObject*, PyObject* const* args, Py_ssize_t n) {
     p.causal = c.causal;
     p.seqlen_k_valid = c.k_valid;
     p.q_pos_offset = c.q_pos_offset;
+    if (const size_t bytes = g_abi.int8_codes16_bytes(&p)) {
+      const Tensor codes = empty_cuda({(int64_t)bytes}, at::kByte, dev);
+      s_q = empty_cuda({rows}, at::kFloat, dev);
+      p.sq_scratch = s_q.data_ptr<float>();
+      check(g_abi.fwd_int8_codes16(&p, k.data_ptr(), s_k.data_ptr<float>(), codes.data_ptr(), st), "fa_fwd_int8_codes16");
+      return;
+    }
+    k8 = empty_cuda(k.sizes(), at::kChar, dev);
+    check(g_abi.quantize_k(k.data_ptr(), k8.data_ptr<int8_t>(), s_k.data_ptr<float>(), rows, (int)D, dev.index(), st),
+          "fa_quantize_k_int8");
+    p.k8 = k8.data_ptr<int8_t>();
     if (D == 128 && impl != FA_IMPL_MMA) {
       q8 = empty_cuda(q.sizes(), at::kChar, dev);
       s_q = empty_cuda({rows}, at::kFloat, dev);
@@ -690,6 +701,8 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t n) {
   g_abi.bwd_dkdv_bits = (decltype(g_abi.bwd_dkdv_bits))get("fa_bwd_dkdv_dropout");
   g_abi.quantize_k = (decltype(g_abi.quantize_k))get("fa_quantize_k_int8");
   g_abi.fwd_int8 = (decltype(g_abi.fwd_int8))get("fa_fwd_int8");
+  g_abi.int8_codes16_bytes = (decltype(g_abi.int8_codes16_bytes))get("fa_int8_codes16_bytes");
+  g_abi.fwd_int8_codes16 = (decltype(g_abi.fwd_int8_codes16))get("fa_fwd_int8_codes16");
   g_abi.decode = (decltype(g_abi.decode))get("fa_decode_paged");
   g_abi.decode_checked = (decltype(g_abi.decode_checked))get("fa_decode_paged_checked");
   g_abi.decode_counters = (decltype(g_abi.decode_counters))get("fa_decode_counters");

@@ -20,6 +20,12 @@ __device__ __forceinline__ int round_i8_fast(float x) {
   return x < 0.f ? -m : m;
 }
 
+// ... and as a float
+__device__ __forceinline__ float round_f_fast(float x) {
+  const float t = __fadd_rn(fabsf(x), 0.5f);
+  return copysignf(__fsub_rn(__fadd_rd(t, 8388608.0f), 8388608.0f), x);
+}
+
 // ---------------------------------------------------------------------------------------
 // K quantiser: rows x D fp16 -> int8 codes + fp32 scale per row.  HBM-bound: 2 B read and
 // 1 B written per element.  D/8 lanes share a row, 16 bytes each; every thread keeps kRows
@@ -35,9 +41,10 @@ __device__ __forceinline__ int round_i8_fast(float x) {
 #define FA_QUANT_BLOCKS 8
 #endif
 constexpr int kQuantRows = FA_QUANT_ROWS;
-template <int D, bool kDivide = false>
+// kHalf: the codes as 16-bit floats (exact) for the tcgen05 forward that multiplies them in that form.
+template <int D, bool kDivide, bool kHalf>
 __global__ void __launch_bounds__(256) quantize_k_kernel(const __half* __restrict__ k,
-                                                         int8_t* __restrict__ k8,
+                                                         void* __restrict__ codes,
                                                          float* __restrict__ s_k, int64_t rows) {
   constexpr int LPR = D / 8;
   constexpr int RPB = 256 / LPR;                     // rows per block and sub-step
@@ -76,26 +83,36 @@ __global__ void __launch_bounds__(256) quantize_k_kernel(const __half* __restric
       for (int i = 0; i < 4; ++i) {
         const float a = kDivide ? __fdiv_rn(x[i], sc) : __fmul_rn(x[i], inv);
         const float c2 = kDivide ? __fdiv_rn(x[4 + i], sc) : __fmul_rn(x[4 + i], inv);
-        lo |= (uint32_t)(uint8_t)(int8_t)round_i8_fast(a) << (8 * i);
-        hi |= (uint32_t)(uint8_t)(int8_t)round_i8_fast(c2) << (8 * i);
+        if (kHalf) {
+          x[i] = round_f_fast(a);
+          x[4 + i] = round_f_fast(c2);
+        } else {
+          lo |= (uint32_t)(uint8_t)(int8_t)round_i8_fast(a) << (8 * i);
+          hi |= (uint32_t)(uint8_t)(int8_t)round_i8_fast(c2) << (8 * i);
+        }
       }
       if (row < rows) {
-        __stcs(reinterpret_cast<uint2*>(k8 + row * D + c * 8), make_uint2(lo, hi));
+        if (kHalf)
+          __stcs(reinterpret_cast<uint4*>(static_cast<__half*>(codes) + row * D + c * 8),
+                 make_uint4(Elem<__half>::pack(x[0], x[1]), Elem<__half>::pack(x[2], x[3]), Elem<__half>::pack(x[4], x[5]),
+                            Elem<__half>::pack(x[6], x[7])));
+        else
+          __stcs(reinterpret_cast<uint2*>(static_cast<int8_t*>(codes) + row * D + c * 8), make_uint2(lo, hi));
         if (c == 0) __stcs(s_k + row, sc);
       }
     }
   }
 }
 
-template <int D, bool kDivide>
-static int launch_quantiser(const void* x, int8_t* x8, float* s, int64_t rows, cudaStream_t st, const char* what) {
+template <int D, bool kDivide, bool kHalf = false>
+static int launch_quantiser(const void* x, void* codes, float* s, int64_t rows, cudaStream_t st, const char* what) {
   constexpr int RPB = 256 / (D / 8);
   const int64_t need = (rows + RPB * kQuantRows - 1) / (RPB * kQuantRows);
   int device = 0;
   cudaGetDevice(&device);
   const int64_t cap = (int64_t)sm_count(device) * FA_QUANT_BLOCKS;  // 8 blocks of 256 threads fill an SM
-  quantize_k_kernel<D, kDivide><<<(unsigned)(need < cap ? need : cap), 256, 0, st>>>(
-      reinterpret_cast<const __half*>(x), x8, s, rows);
+  quantize_k_kernel<D, kDivide, kHalf><<<(unsigned)(need < cap ? need : cap), 256, 0, st>>>(
+      reinterpret_cast<const __half*>(x), codes, s, rows);
   return check_launch(what);
 }
 
@@ -120,6 +137,13 @@ int quantize_q(const void* q, int8_t* q8, float* s_q, int64_t rows, int head_dim
     return FA_ERR_UNSUPPORTED;
   }
   return launch_quantiser<128, true>(q, q8, s_q, rows, st, "quantize_q");
+}
+
+// Codes of Q (division form) and K (reciprocal form) as 16-bit floats, head_dim 64.
+int quantize_codes16(const void* x, void* codes, float* s, int64_t rows, bool divide, cudaStream_t st) {
+  if (rows == 0) return FA_OK;
+  return divide ? launch_quantiser<64, true, true>(x, codes, s, rows, st, "quantize_codes16")
+                : launch_quantiser<64, false, true>(x, codes, s, rows, st, "quantize_codes16");
 }
 
 // ---------------------------------------------------------------------------------------

@@ -307,6 +307,15 @@ typedef struct fa_int8_args {
 int fa_fwd_int8(const fa_int8_args* args, void* stream);
 
 /*
+ * Quantisation of q and k and the forward in one call, with the codes held as 16-bit floats in `codes`
+ * (fa_int8_codes16_bytes; 0 = the call keeps to fa_quantize_k_int8 + fa_fwd_int8).  Codes and scales are those of
+ * the int8 calls, and so are the scores: sums of products of codes are exact in the fp32 accumulator.  s_k
+ * (batch*heads, seqlen) is written; args->k8, s_k and q8_scratch are not used.
+ */
+size_t fa_int8_codes16_bytes(const fa_int8_args* args);
+int fa_fwd_int8_codes16(const fa_int8_args* args, const void* k, float* s_k, void* codes, void* stream);
+
+/*
  * Rotary position embedding on x (batch, seqlen, heads, head_dim) -- or packed (tokens, heads,
  * head_dim) with cu_seqlens -- into out (same layout; out == x rotates in place):
  *   non-interleaved: pairs (x[i], x[i + rotary_dim/2]);  interleaved: pairs (x[2i], x[2i+1])

@@ -162,3 +162,16 @@ def test_config5_shape():
             sl = (slice(b, b + 1), slice(h, h + 1))
             ro, _, _, _ = orc.attention_int8_ref(q[sl].cpu(), k[sl].cpu(), v[sl].cpu(), causal=causal)
             assert maxdiff(out[sl], ro) <= util.FWD_TOL, (b, h, causal)
+
+
+@pytest.mark.parametrize("B,H,S,lk,causal", [(2, 60, 512, 512, True), (1, 26, 1088, 1088, False), (1, 8, 2048, 2048, True),
+                                             (1, 26, 1088, 900, True)])
+def test_head_dim_64_on_tcgen05(B, H, S, lk, causal):
+    """Problems large enough for the codes held as 16-bit floats, key columns of very different scales among them."""
+    import flash_attn_triton_b200 as fa
+    q, k, v = cases.int8_case(700 + S, B, H, S, 64)
+    k[0, 0, :, 5] *= 8
+    kw = {} if lk == S else dict(seq_len_k=lk, seq_len_q=lk)
+    out = fa.attention_int8(q.to(DEV), k.to(DEV), v.to(DEV), causal=causal, **kw)
+    ro, _, _, _ = orc.attention_int8_ref(q, k, v, causal=causal, **kw)
+    assert maxdiff(out[:, :, :lk], ro[:, :, :lk]) <= util.FWD_TOL
