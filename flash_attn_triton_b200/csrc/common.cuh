@@ -64,6 +64,12 @@ struct ScoreCfg {
   const uint32_t* keep;
   int64_t keep_words;
   float drop_log2;          // log2(dropout_scale)
+  // log2 by which a row maximum must exceed the one its exponents are relative to before O is rescaled (tcgen05
+  // forward kernels).  8 saves most rescales, but a row's largest probability is then 2^x and is rounded to 16 bits,
+  // where relative to its own maximum it is exactly 1: errors against float64 grow by 1 to 10 %.  0 where the
+  // mma.sync kernels, which always rescale, set the precision of a call: head_dim 256, fewer than 256 keys, KV-cache
+  // chunks, INT8 at head_dim 64 (bf16, 2 x 1999 tokens, head_dim 256: 2.017e-3 both, 2.075e-3 with 8).
+  float rescale_at;
 };
 
 __host__ __device__ inline ScoreCfg make_score_cfg(float scale, float softcap, int causal, int wl,
@@ -85,6 +91,7 @@ __host__ __device__ inline ScoreCfg make_score_cfg(float scale, float softcap, i
   c.keep = nullptr;
   c.keep_words = 0;
   c.drop_log2 = 0.f;
+  c.rescale_at = 8.f;
   return c;
 }
 

@@ -20,7 +20,7 @@
 // takes the buffer next is issued right after P_j V_j, which reads them, in the in-order pipe.  Neither
 // group waits for the other's exponentials: what a tile needs from the tile before it is only the
 // row maximum that all exponents are taken relative to.  It sits in shared memory (mref), is read and
-// raised in tile order -- only when a row's maximum grows by more than 2^8, and the accumulator is then
+// raised in tile order -- only when a row's maximum grows by more than cfg.rescale_at, and the accumulator is then
 // rescaled by the group that raised it -- and each group keeps its own row sums.
 //
 // Bound: the tensor pipe needs 2 * head_dim * 8 cycles per tile (128 x 128 scores), the exponentials
@@ -45,7 +45,6 @@ namespace {
 constexpr int kBM = 128;          // query rows of the tile
 constexpr int kBN = 128;          // keys per tile
 constexpr int kThreads = 384;
-constexpr float kRescaleThreshold = 8.0f;
 constexpr int kMaxStages = 8;
 
 template <int D> struct ACfg {
@@ -541,7 +540,7 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         ok = wait_bar(&sh->decided[x ^ 1], ((j - 1) >> 1) & 1, sh, 33 + x);
         if (!ok) break;
         const float m_old = sh->mref[row_in_tile];
-        const bool need = mx > m_old + kRescaleThreshold;
+        const bool need = mx > m_old + cfg.rescale_at;
         m_use = need ? mx : m_old;
         if (__any_sync(0xffffffffu, need)) {
           // The accumulator may be touched once P V of the tile before is finished: the one of this
@@ -797,7 +796,9 @@ int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
 
 template <typename T, int D>
 static int launch_cache(const fa_decode_args& d, const void* q, const int64_t* q_stride, const CacheGeo& geo,
-                        const ScoreCfg& cfg, cudaStream_t st) {
+                        const ScoreCfg& plain, cudaStream_t st) {
+  ScoreCfg cfg = plain;
+  cfg.rescale_at = 0.f;
   fa_attn_args a = {};
   a.dtype = d.dtype;
   a.device = d.device;

@@ -53,7 +53,6 @@ namespace {
 constexpr int kBM = 128;          // query rows per tile (two tiles per CTA)
 constexpr int kBN = 128;          // keys per K/V tile
 constexpr int kThreads = 384;     // 8 softmax warps + a warpgroup holding producer and MMA warps
-constexpr float kRescaleThreshold = 8.0f;
 // Share of the exponentials of the unmasked fast path that run on the FMA pipe (every n-th;
 // 0 = none: measured slower here, the softmax warps are short of issue slots, not of MUFU).
 #ifndef FA_POLY_FWD
@@ -591,7 +590,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (t == 0) {
         m_used = mx;
       } else {
-        const bool need = mx > m_used + kRescaleThreshold;
+        const bool need = mx > m_used + cfg.rescale_at;
         if (__any_sync(0xffffffffu, need)) {
           // The previous P V of this stream is its (t-1)-th; the one of this tile cannot
           // complete before P is written below, so the barrier is at most one phase ahead
@@ -851,7 +850,9 @@ static bool one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
   return nk >= 96 || (a.head_dim == 128 && (nk >= 48 || 3 * ctas <= nk * sms));
 }
 
-int fwd_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
+int fwd_sm100(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
+  ScoreCfg cfg = plain;
+  if (a.head_dim == 256 || a.seqlen_k < 256) cfg.rescale_at = 0.f;
   if (a.head_dim == 256) return fwd_alt_sm100(a, cfg, st);
   // FA_B200_FWD_PERSISTENT_FROM in the environment overrides the threshold (tests run the
   // persistent kernel on small shapes with it; 0 = never)
@@ -952,7 +953,8 @@ int fwd_int8_codes16(const fa_int8_args& a, const void* q16, const void* k16, cu
     set_error("fwd_int8_codes16: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
+  ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
+  cfg.rescale_at = 0.f;
   auto kern = fwd_sm100_kernel<__half, D, false, 2, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
