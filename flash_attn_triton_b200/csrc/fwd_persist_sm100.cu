@@ -39,7 +39,6 @@ namespace {
 constexpr int kBM = 128;          // query rows per tile (two tiles per work item)
 constexpr int kBN = 128;          // keys per K/V tile
 constexpr int kThreads = 384;
-constexpr float kRescaleThreshold = 8.0f;
 constexpr int kMaxStages = 8;
 constexpr int kSched = 4;         // depth of the in-CTA ring of work-queue entries
 constexpr int kConsumers = 9;     // warps that read the queue: 8 softmax warps and the MMA issuer
@@ -531,7 +530,7 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         if (t == 0) {
           m_used = mx;
         } else {
-          const bool need = mx > m_used + kRescaleThreshold;
+          const bool need = mx > m_used + cfg.rescale_at;
           if (__any_sync(0xffffffffu, need)) {
             // The previous P V of this stream is its (tc-1)-th; the one of this tile cannot
             // complete before P is written below, so the barrier is at most one phase ahead
