@@ -105,6 +105,7 @@ EXPORTS = {
     "fa_varlen_bwd_dkdv": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fa_decode_paged": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
     "fa_decode_paged_checked": (C.c_int, [C.POINTER(DecodeArgs), C.POINTER(C.c_uint32), C.c_void_p]),
+    "fa_decode_checked_workspace_bytes": (C.c_size_t, [C.POINTER(DecodeArgs)]),
     "fa_decode_counters": (C.c_int32, [C.POINTER(DecodeArgs)]),
     "fa_decode_workspace_bytes": (C.c_size_t, [C.POINTER(DecodeArgs)]),
     "fa_decode_paged_static": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),

@@ -117,6 +117,7 @@ int decode_paged(const fa_decode_args&, cudaStream_t);
 int decode_paged_checked(const fa_decode_args&, uint32_t*, cudaStream_t);
 int decode_num_counters(const fa_decode_args&);
 size_t decode_workspace_bytes(const fa_decode_args&);
+size_t decode_checked_workspace_bytes(const fa_decode_args&);
 int decode_paged_static(const fa_decode_args&, cudaStream_t);
 size_t decode_static_scratch_bytes();
 int quantize_k(const void*, int8_t*, float*, int64_t, int, cudaStream_t);
@@ -425,6 +426,10 @@ int fa_decode_paged_static(const fa_decode_args* a, void* stream) {
 
 size_t fa_decode_static_scratch_bytes(void) { return decode_static_scratch_bytes(); }
 
+size_t fa_decode_checked_workspace_bytes(const fa_decode_args* a) {
+  if (a == nullptr || a->heads_kv <= 0 || a->heads_q <= 0 || a->page_size <= 0) return 0;
+  return decode_checked_workspace_bytes(*a);
+}
 size_t fa_decode_workspace_bytes(const fa_decode_args* a) {
   if (a == nullptr || a->heads_kv <= 0 || a->heads_q <= 0 || a->page_size <= 0) return 0;
   return decode_workspace_bytes(*a);

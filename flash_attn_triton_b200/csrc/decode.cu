@@ -50,7 +50,9 @@ struct DecodeGeom {
 };
 
 // The value checks of one call: their result goes to a word in mapped host memory (bit 31 = done, low
-// bits = fa_decode_check of the checks that failed), and to a device word for the kernels behind them.
+// bits = fa_decode_check of the checks that failed), and to a word of the call's own workspace for the kernels
+// behind them.  The host word is handed to the next call once the host has read it; the kernels read theirs until the
+// last CTA has started, long after the call has returned, so no other call may write to it.
 constexpr uint32_t kCheckDone = 0x80000000u;
 constexpr int kInlineCheck = 1024;   // table entries up to which every attention CTA makes the checks itself
 struct DecodeCheck {
@@ -90,7 +92,7 @@ int cache_attention_sm100(const fa_decode_args& d, const void* q, const int64_t*
 __global__ void __launch_bounds__(1024) decode_check_kernel(const fa_decode_args p, uint32_t* host, uint32_t* dev) {
   const uint32_t bad = decode_checks(p, threadIdx.x, blockDim.x);
   if (threadIdx.x == 0) {
-    *dev = bad;
+    if (dev) *dev = bad;
     *reinterpret_cast<volatile uint32_t*>(host) = bad | kCheckDone;
     __threadfence_system();
   }
@@ -907,15 +909,27 @@ static int decode_t(const fa_decode_args& a, const ScoreCfg& cfg, const DecodeGe
   return FA_ERR_UNSUPPORTED;
 }
 
-static int decode_run(const fa_decode_args& args, const DecodeCheck& chk, cudaStream_t st) {
-  fa_decode_args a = args;
-  const DecodeGeom g = decode_geometry(a);
-  const size_t pieces = decode_piece_bytes(a, g), need = decode_workspace_bytes(a);
+// What a call is refused for, before any of its kernels is launched.  c: its cut as a chunk, or null.
+static int decode_refused(const fa_decode_args& a, const ChunkPlan* c) {
+  if (c != nullptr)
+    if (const int code = host_wait_status(a.device)) {
+      set_error("fa_decode_paged: a bounded device-side wait ran out earlier on device %d (code %d); the tcgen05 kernels "
+                "stay off until fa_device_wait_clear()", a.device, code);
+      return FA_ERR_DEVICE_WAIT;
+    }
+  const size_t need = decode_workspace_bytes(a);
   if (need > 0 && (a.workspace == nullptr || a.workspace_bytes < need)) {
     set_error("decode workspace too small: need %zu bytes, got %zu", need, a.workspace_bytes);
     return FA_ERR_WORKSPACE;
   }
   FA_REQUIRE(a.counters == nullptr || a.num_counters >= decode_num_counters(a), "decode: too few counters");
+  return FA_OK;
+}
+
+static int decode_run(const fa_decode_args& args, const DecodeCheck& chk, cudaStream_t st) {
+  fa_decode_args a = args;
+  const DecodeGeom g = decode_geometry(a);
+  const size_t pieces = decode_piece_bytes(a, g), need = decode_workspace_bytes(a);
   if (need > 0 && a.counters == nullptr) {
     a.counters = reinterpret_cast<uint32_t*>(static_cast<char*>(a.workspace) + pieces);
     const cudaError_t e = cudaMemsetAsync(a.counters, 0, need - pieces, st);
@@ -931,19 +945,11 @@ static int decode_run(const fa_decode_args& args, const DecodeCheck& chk, cudaSt
   return a.dtype == FA_BF16 ? decode_t<__nv_bfloat16>(a, cfg, g, chk, st) : decode_t<__half>(a, cfg, g, chk, st);
 }
 
-// host / dev: the slot of the value checks, or null; `inside`: made by the append kernel itself
-static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* host, uint32_t* dev, bool inside, cudaStream_t st) {
+// dev: the call's word with the result of the value checks, or null.  host != null: the append kernel makes the
+// checks; *queued is set once it is on the stream and will write the host word.
+static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* host, uint32_t* dev, bool* queued, cudaStream_t st) {
   fa_decode_args a = args;
-  if (const int code = host_wait_status(a.device)) {
-    set_error("fa_decode_paged: a bounded device-side wait ran out earlier on device %d (code %d); the tcgen05 kernels stay "
-              "off until fa_device_wait_clear()", a.device, code);
-    return FA_ERR_DEVICE_WAIT;
-  }
-  const size_t need = decode_workspace_bytes(a);
-  if (need > 0 && (a.workspace == nullptr || a.workspace_bytes < need)) {
-    set_error("decode workspace too small: need %zu bytes, got %zu", need, a.workspace_bytes);
-    return FA_ERR_WORKSPACE;
-  }
+  const bool inside = host != nullptr;
   char* ws = static_cast<char*>(a.workspace);
   CacheGeo geo = {};
   geo.seqlens = a.cache_seqlens;
@@ -962,7 +968,6 @@ static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* h
   geo.ws = reinterpret_cast<float*>(ws + c.q_bytes);
   geo.bad = dev;
   if (c.parts > 1) {
-    FA_REQUIRE(a.counters == nullptr || a.num_counters >= c.units, "decode: too few counters");
     geo.counters = a.counters;
     if (geo.counters == nullptr) {
       geo.counters = reinterpret_cast<uint32_t*>(ws + c.q_bytes + c.piece_bytes);
@@ -984,6 +989,7 @@ static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* h
     else
       cache_append_kernel<<<grid, 256, 0, st>>>(a, static_cast<__half*>(q_out), shift, host, dev, inside);
     if (int r = check_launch("cache_append")) return r;
+    if (inside) *queued = true;
   }
   const int64_t qs[3] = {(int64_t)a.seqlen_q * a.heads_q * a.head_dim, (int64_t)a.heads_q * a.head_dim, a.head_dim};
   const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, a.window_left, a.window_right, a.alibi_slopes != nullptr);
@@ -993,27 +999,26 @@ static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* h
 int decode_paged(const fa_decode_args& a, cudaStream_t st) {
   if (a.batch == 0 || a.seqlen_q == 0 || a.heads_q == 0) return FA_OK;
   ChunkPlan c;
-  if (chunk_plan(a, c)) return chunk_run(a, c, nullptr, nullptr, false, st);
-  return decode_run(a, DecodeCheck{nullptr, nullptr}, st);
+  const bool chunk = chunk_plan(a, c);
+  if (int r = decode_refused(a, chunk ? &c : nullptr)) return r;
+  return chunk ? chunk_run(a, c, nullptr, nullptr, nullptr, st) : decode_run(a, DecodeCheck{nullptr, nullptr}, st);
 }
 
 // ---------------------------------------------------------------------------------------
-// Value checks.  A call takes a slot -- one word in mapped host memory and one on the device --
-// launches, and polls the host word: it changes as soon as the checks have run, so the host goes on
-// while the attention is still running, without a stream synchronisation.
+// Value checks.  A call takes a slot -- one word in mapped host memory --, launches, and polls the word: it
+// changes as soon as the checks have run, so the host goes on while the attention is still running, without
+// a stream synchronisation.
 // ---------------------------------------------------------------------------------------
 constexpr int kCheckSlots = 256;
 alignas(4096) static volatile uint32_t g_check_host[kCheckSlots * 16];      // a cache line per slot
-static __device__ uint32_t g_check_dev[kCheckSlots];
 
 namespace {
 struct CheckSlots {
   std::mutex mu;
   int free_list[kCheckSlots], nfree = 0;
   int state = 0;                       // 0 not tried, 1 mapped, -1 unavailable
-  uint32_t* dev[64] = {nullptr};
   // index of a free slot, or -1 (error set)
-  int acquire(int device, uint32_t** host_dptr, uint32_t** dev_ptr) {
+  int acquire(uint32_t** host_dptr) {
     for (;;) {
       {
         std::lock_guard<std::mutex> lock(mu);
@@ -1024,17 +1029,9 @@ struct CheckSlots {
           for (int i = 0; i < kCheckSlots; ++i) free_list[nfree++] = kCheckSlots - 1 - i;
           if (e != cudaSuccess) cudaGetLastError();
         }
-        if (state < 0 || device < 0 || device >= 64) {
+        if (state < 0) {
           set_error("decode: no mapped host memory for the value checks");
           return -1;
-        }
-        if (dev[device] == nullptr) {
-          void* q = nullptr;
-          if (cudaGetSymbolAddress(&q, g_check_dev) != cudaSuccess) {
-            set_error("decode: cudaGetSymbolAddress: %s", cudaGetErrorString(cudaGetLastError()));
-            return -1;
-          }
-          dev[device] = static_cast<uint32_t*>(q);
         }
         if (nfree > 0) {
           const int i = free_list[--nfree];
@@ -1045,7 +1042,6 @@ struct CheckSlots {
             return -1;
           }
           *host_dptr = static_cast<uint32_t*>(h);
-          *dev_ptr = dev[device] + i;
           g_check_host[i * 16] = 0u;
           return i;
         }
@@ -1053,12 +1049,52 @@ struct CheckSlots {
       sched_yield();                   // as many threads as slots are inside this function
     }
   }
+  // Waits until the kernel that was given the slot has written it: only then may another call have it.
+  int await(int i, uint32_t* failed, cudaStream_t st) {
+    volatile uint32_t* word = &g_check_host[i * 16];
+    for (uint32_t it = 1; *word == 0u; ++it) {
+#if defined(__x86_64__)
+      __builtin_ia32_pause();
+#endif
+      if ((it & 0x3fffu) == 0) {       // every few hundred microseconds: has the stream died?
+        const cudaError_t e = cudaStreamQuery(st);
+        if (e == cudaErrorNotReady) continue;
+        if (e != cudaSuccess || *word == 0u) {
+          set_error("decode: value checks did not run: %s", cudaGetErrorString(e));
+          return FA_ERR_LAUNCH;
+        }
+      }
+    }
+    *failed = *word & ~kCheckDone;
+    return FA_OK;
+  }
   void release(int i) {
     std::lock_guard<std::mutex> lock(mu);
     free_list[nfree++] = i;
   }
 } g_slots;
+
+// What the checks of a call need: `inside`, its first kernel makes them, in every CTA, because the tables are
+// small; `word`, kernels behind that one read the result from device memory.
+struct CheckPlan {
+  bool chunk, inside, word;
+  ChunkPlan c;
+};
+CheckPlan check_plan(const fa_decode_args& a) {
+  CheckPlan k;
+  k.chunk = chunk_plan(a, k.c);
+  k.inside = (int64_t)a.batch * (a.block_table ? a.block_table_stride : 1) <= kInlineCheck;
+  k.word = k.chunk || !k.inside;
+  return k;
+}
+constexpr size_t kWordBytes = 16;
+size_t word_offset(const fa_decode_args& a) { return (decode_workspace_bytes(a) + kWordBytes - 1) / kWordBytes * kWordBytes; }
 }  // namespace
+
+size_t decode_checked_workspace_bytes(const fa_decode_args& a) {
+  if (a.heads_kv <= 0 || a.heads_q <= 0 || a.batch <= 0 || a.seqlen_q <= 0) return 0;
+  return check_plan(a).word ? word_offset(a) + kWordBytes : decode_workspace_bytes(a);
+}
 
 int decode_paged_checked(const fa_decode_args& a, uint32_t* failed, cudaStream_t st) {
   *failed = 0;
@@ -1069,46 +1105,38 @@ int decode_paged_checked(const fa_decode_args& a, uint32_t* failed, cudaStream_t
     set_error("value checks cannot run while the stream is being captured; turn them off with set_validation(False)");
     return FA_ERR_LAUNCH;
   }
-  uint32_t *host = nullptr, *dev = nullptr;
-  const int slot = g_slots.acquire(a.device, &host, &dev);
+  CheckPlan k = check_plan(a);
+  if (int r = decode_refused(a, k.chunk ? &k.c : nullptr)) return r;
+  uint32_t* word = nullptr;
+  if (k.word && a.workspace != nullptr && a.workspace_bytes >= word_offset(a) + kWordBytes)
+    word = reinterpret_cast<uint32_t*>(static_cast<char*>(a.workspace) + word_offset(a));
+  const bool host_order = k.word && word == nullptr;   // no room for the word: launch nothing before the result is here
+  if (host_order) k.inside = false;
+  uint32_t* host = nullptr;
+  const int slot = g_slots.acquire(&host);
   if (slot < 0) return FA_ERR_LAUNCH;
-  const int64_t entries = (int64_t)a.batch * (a.block_table ? a.block_table_stride : 1);
-  int r;
-  ChunkPlan c;
-  if (chunk_plan(a, c)) {
-    r = FA_OK;
-    if (entries > kInlineCheck) {
-      decode_check_kernel<<<1, 1024, 0, st>>>(a, host, dev);
-      r = check_launch("decode_check");
-    }
-    if (r == FA_OK) r = chunk_run(a, c, host, dev, entries <= kInlineCheck, st);
-  } else if (entries <= kInlineCheck) {
-    r = decode_run(a, DecodeCheck{host, nullptr}, st);
-  } else {
-    decode_check_kernel<<<1, 1024, 0, st>>>(a, host, dev);
+  int r = FA_OK;
+  bool queued = false;                                 // a kernel that writes the host word is on the stream
+  if (!k.inside) {
+    decode_check_kernel<<<1, 1024, 0, st>>>(a, host, word);
     r = check_launch("decode_check");
-    if (r == FA_OK) r = decode_run(a, DecodeCheck{nullptr, dev}, st);
+    queued = r == FA_OK;
   }
-  volatile uint32_t* word = &g_check_host[slot * 16];
-  if (r == FA_OK) {
-    for (uint32_t it = 1; *word == 0u; ++it) {
-#if defined(__x86_64__)
-      __builtin_ia32_pause();
-#endif
-      if ((it & 0x3fffu) == 0) {       // every few hundred microseconds: has the stream died?
-        const cudaError_t e = cudaStreamQuery(st);
-        if (e == cudaErrorNotReady) continue;
-        if (e != cudaSuccess || *word == 0u) {
-          set_error("decode: value checks did not run: %s", cudaGetErrorString(e));
-          r = FA_ERR_LAUNCH;
-          break;
-        }
-      }
+  if (r == FA_OK && !host_order) {
+    if (k.chunk) {
+      r = chunk_run(a, k.c, k.inside ? host : nullptr, word, &queued, st);
+    } else {
+      r = decode_run(a, k.inside ? DecodeCheck{host, nullptr} : DecodeCheck{nullptr, word}, st);
+      queued = queued || r == FA_OK;
     }
-    *failed = *word & ~kCheckDone;
+  }
+  if (queued) {
+    const int w = g_slots.await(slot, failed, st);
+    if (r == FA_OK) r = w;
   }
   g_slots.release(slot);
-  return r;
+  if (r != FA_OK || *failed || !host_order) return r;
+  return k.chunk ? chunk_run(a, k.c, nullptr, nullptr, nullptr, st) : decode_run(a, DecodeCheck{nullptr, nullptr}, st);
 }
 
 // ---------------------------------------------------------------------------------------

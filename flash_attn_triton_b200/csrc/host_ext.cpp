@@ -52,6 +52,7 @@ struct Abi {
   int (*decode_checked)(const fa_decode_args*, uint32_t*, void*);
   int32_t (*decode_counters)(const fa_decode_args*);
   size_t (*decode_workspace)(const fa_decode_args*);
+  size_t (*decode_checked_workspace)(const fa_decode_args*);
   PyObject* check;   // _native.check(status, what): raises the Python exception of a status
 };
 Abi g_abi = {};
@@ -646,7 +647,7 @@ PyObject* py_kvcache(PyObject*, PyObject* const* args, Py_ssize_t n) {
   if (alibi.defined()) p.alibi_slopes = alibi.const_data_ptr<float>();
   const cudaStream_t st = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
   Tensor ws, ctr;
-  if (const size_t need = g_abi.decode_workspace(&p)) {
+  if (const size_t need = checks ? g_abi.decode_checked_workspace(&p) : g_abi.decode_workspace(&p)) {
     ws = empty_cuda({(int64_t)need}, at::kByte, dev);
     p.workspace = ws.data_ptr();
     p.workspace_bytes = need;
@@ -707,6 +708,7 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t n) {
   g_abi.decode_checked = (decltype(g_abi.decode_checked))get("fa_decode_paged_checked");
   g_abi.decode_counters = (decltype(g_abi.decode_counters))get("fa_decode_counters");
   g_abi.decode_workspace = (decltype(g_abi.decode_workspace))get("fa_decode_workspace_bytes");
+  g_abi.decode_checked_workspace = (decltype(g_abi.decode_checked_workspace))get("fa_decode_checked_workspace_bytes");
   Py_INCREF(chk);
   Py_XDECREF(g_abi.check);
   g_abi.check = chk;

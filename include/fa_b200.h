@@ -226,7 +226,9 @@ int fa_decode_paged(const fa_decode_args* args, void* stream);
 /* fa_decode_paged with the value checks of the public call made on the device.  `failed` receives the
  * checks that did not hold (0 = all held); if any did not, nothing was written.  Returns as soon as the
  * checks have run on the GPU, while the attention itself may still be running.  Not for streams
- * under capture. */
+ * under capture.  With fa_decode_checked_workspace_bytes() of workspace the attention is queued behind the
+ * checks, which leave their result there; with less (fa_decode_workspace_bytes() will do) the call waits for
+ * it first. */
 typedef enum fa_decode_check {
   FA_CHECK_PAGES = 1,   /* block_table entries lie in [0, num_pages) */
   FA_CHECK_ROWS = 2,    /* cache_batch_idx entries lie in [0, num_pages) */
@@ -235,6 +237,10 @@ typedef enum fa_decode_check {
   FA_CHECK_ROTARY = 16  /* every rotated position has a table row */
 } fa_decode_check;
 int fa_decode_paged_checked(const fa_decode_args* args, uint32_t* failed, void* stream);
+
+/* Bytes of workspace for fa_decode_paged_checked, 0 where fa_decode_paged needs none and no kernel has to read the
+ * result of the checks. */
+size_t fa_decode_checked_workspace_bytes(const fa_decode_args* args);
 
 /* Words fa_decode_args.counters needs for this problem. */
 int32_t fa_decode_counters(const fa_decode_args* args);

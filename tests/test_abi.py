@@ -130,3 +130,20 @@ def test_wait_status_refusal_without_gpu(built):
                 N.check(r, "probe")
     finally:
         assert lib.fa_debug_set_wait_status(0, 0) == 0
+
+
+def test_checked_decode_result_has_room_of_its_own(built):
+    """Kernels behind the value checks read the result until their last CTA has started: it lies in the workspace of the
+    call, not in memory that a call on another stream may be given.  No word where one kernel does it all."""
+    from flash_attn_triton_b200 import _native as N
+    lib = N.lib()
+
+    def sizes(tokens, table):
+        d = N.DecodeArgs()
+        d.heads_q, d.heads_kv, d.head_dim, d.batch, d.seqlen_q = 8, 2, 128, 4, tokens
+        d.page_size, d.block_table, d.block_table_stride, d.softmax_scale = 64, 4096, table, 0.1
+        return lib.fa_decode_workspace_bytes(ctypes.byref(d)), lib.fa_decode_checked_workspace_bytes(ctypes.byref(d))
+
+    for tokens, table, word in ((1, 256, False), (1, 257, True), (64, 8, True), (64, 300, True)):
+        plain, checked = sizes(tokens, table)
+        assert (checked >= plain + 4) if word else (checked == plain), (tokens, table, plain, checked)
