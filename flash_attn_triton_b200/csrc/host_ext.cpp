@@ -21,6 +21,7 @@
 
 #include <string.h>
 
+#include <array>
 #include <list>
 #include <mutex>
 
@@ -301,11 +302,18 @@ variable_list run_backward(const Params& c, const variable_list& in, const Tenso
   return g;
 }
 
+// Every tensor that the backward reads is a saved variable: one that was changed in place since the forward is
+// refused, and the saved-tensor hooks (offloading, checkpointing) see all of them.  Params::bias alone is held as it
+// is: expanded over broadcast dimensions, it would be written out in full by a hook that copies.
 struct AttnBackward : public Node {
-  Params c;
+  Params c;                                      // without the tensors of `side`
   std::vector<SavedVariable> in;
-  SavedVariable out;
-  Tensor lse;
+  SavedVariable out, lse;
+  SavedVariable side[5];                         // cu_q, cu_k, used_q, used_k, alibi
+
+  static std::array<Tensor Params::*, 5> side_members() {
+    return {&Params::cu_q, &Params::cu_k, &Params::used_q, &Params::used_k, &Params::alibi};
+  }
 
   variable_list apply(variable_list&& grads) override {
     variable_list res(in.size());
@@ -314,20 +322,23 @@ struct AttnBackward : public Node {
     variable_list x;
     x.reserve(in.size());
     for (auto& s : in) x.push_back(s.unpack());
-    const Tensor o = out.unpack(getptr());
+    const Tensor o = out.unpack(getptr()), l = lse.unpack();
+    Params p = c;
+    for (size_t i = 0; i < 5; ++i) p.*side_members()[i] = side[i].unpack();
     c10::cuda::CUDAGuard guard(x[0].device());
     bool dq = true, dkdv = true;
-    if (c.packing != kQKV) {
+    if (p.packing != kQKV) {
       dq = task_should_compute_output(0);
-      dkdv = task_should_compute_output(1) || (c.packing == kSeparate && task_should_compute_output(2));
+      dkdv = task_should_compute_output(1) || (p.packing == kSeparate && task_should_compute_output(2));
     }
-    return run_backward(c, x, o, lse, grads[0], dq, dkdv);
+    return run_backward(p, x, o, l, grads[0], dq, dkdv);
   }
   std::string name() const override { return "FlashAttnBackward"; }
   void release_variables() override {
     for (auto& s : in) s.reset_data();
+    for (auto& s : side) s.reset_data();
     out.reset_data();
-    lse.reset();
+    lse.reset_data();
   }
 };
 
@@ -354,7 +365,12 @@ Tensor with_grad(const Params& c, variable_list in, bool want_lse, Tensor& lse, 
     node->in.reserve(in.size());
     for (auto& t : in) node->in.emplace_back(t, false);
     node->out = SavedVariable(out, true);
-    node->lse = lse;
+    node->lse = SavedVariable(lse, false);
+    for (size_t i = 0; i < 5; ++i) {
+      Tensor& t = node->c.*AttnBackward::side_members()[i];
+      node->side[i] = SavedVariable(t, false);
+      t.reset();
+    }
   }
   return out;
 }

@@ -1,0 +1,52 @@
+"""The autograd node of the attention calls (csrc/host_ext.cpp) under what PyTorch does with nodes."""
+import pytest
+import torch
+
+from util import DEV
+
+pytestmark = pytest.mark.gpu
+
+
+def mk(*s, seed=0):
+    g = torch.Generator(DEV).manual_seed(seed + sum(s))
+    return torch.randn(*s, device=DEV, dtype=torch.half, generator=g)
+
+
+def fa():
+    import flash_attn_triton_b200 as m
+    return m
+
+
+def varlen(q, k, v, cu, **kw):
+    return fa().flash_attn_varlen_func(q, k, v, cu, cu, 156, 156, **kw)
+
+
+@pytest.mark.parametrize("side", ["cu_seqlens", "alibi", "used"])
+def test_side_tensor_changed_in_place_is_refused(side):
+    q, k, v = (mk(256, 4, 64, seed=i).requires_grad_() for i in range(3))
+    cu = torch.tensor([0, 100, 256], dtype=torch.int32, device=DEV)
+    used = torch.tensor([90, 156], dtype=torch.int32, device=DEV)
+    slopes = torch.rand(2, 4, device=DEV)
+    out = varlen(q, k, v, cu, alibi_slopes=slopes, seqused_k=used if side == "used" else None)
+    changed = dict(cu_seqlens=cu, alibi=slopes, used=used)[side]
+    changed[1:2] += 1
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out.float().sum().backward()
+
+
+def test_hooks_see_every_saved_tensor():
+    q, k, v = (mk(256, 4, 64, seed=i).requires_grad_() for i in range(3))
+    cu = torch.tensor([0, 100, 256], dtype=torch.int32, device=DEV)
+    slopes = torch.rand(4, device=DEV)
+    want = torch.autograd.grad(varlen(q, k, v, cu, alibi_slopes=slopes).float().sum(), (q, k, v))
+    seen = []
+
+    def pack(t):
+        seen.append(tuple(t.shape))
+        return t.cpu()
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.to(DEV)):
+        out = varlen(q, k, v, cu, alibi_slopes=slopes)
+    assert sorted(seen) == sorted([(256, 4, 64)] * 4 + [(4, 256), (3,), (3,), (2, 4)])      # inputs, output, LSE, lengths, slopes
+    for a, b in zip(torch.autograd.grad(out.float().sum(), (q, k, v)), want):
+        assert torch.equal(a, b)
