@@ -318,13 +318,15 @@ struct AttnBackward : public Node {
   variable_list apply(variable_list&& grads) override {
     variable_list res(in.size());
     if (!grads[0].defined()) return res;
-    at::AutoDispatchBelowADInplaceOrView below;
+    // Unpacked before autograd is switched off: the hook of a checkpointed region runs that region's forward again
+    // here, and its nodes have to save what this one saved.
     variable_list x;
     x.reserve(in.size());
     for (auto& s : in) x.push_back(s.unpack());
     const Tensor o = out.unpack(getptr()), l = lse.unpack();
     Params p = c;
     for (size_t i = 0; i < 5; ++i) p.*side_members()[i] = side[i].unpack();
+    at::AutoDispatchBelowADInplaceOrView below;
     c10::cuda::CUDAGuard guard(x[0].device());
     bool dq = true, dkdv = true;
     if (p.packing != kQKV) {

@@ -50,3 +50,32 @@ def test_hooks_see_every_saved_tensor():
     assert sorted(seen) == sorted([(256, 4, 64)] * 4 + [(4, 256), (3,), (3,), (2, 4)])      # inputs, output, LSE, lengths, slopes
     for a, b in zip(torch.autograd.grad(out.float().sum(), (q, k, v)), want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("call", ["dense", "packed", "varlen", "int8"])
+def test_checkpointed_region_that_ends_in_attention(call):
+    """projection -> attention -> reshape: the backward of the attention node is what runs the region again."""
+    from torch.utils.checkpoint import checkpoint
+    torch.manual_seed(0)
+    proj = torch.nn.Linear(64, 192, device=DEV, dtype=torch.half)
+    x = mk(2, 256, 4, 64).requires_grad_()
+    cu = torch.tensor([0, 256, 512], dtype=torch.int32, device=DEV)
+
+    def region(x):
+        y = proj(x)
+        q, k, v = y.split(64, -1)
+        if call == "dense":
+            out = fa().flash_attn_func(q, k, v, causal=True)
+        elif call == "packed":
+            out = fa().flash_attn_qkvpacked_func(y.view(2, 256, 4, 3, 64).transpose(2, 3), causal=True)
+        elif call == "varlen":
+            out = fa().flash_attn_varlen_func(*(t.reshape(512, 4, 64) for t in (q, k, v)), cu, cu, 256, 256, causal=True)
+        else:
+            out = fa().attention_int8(*(t.transpose(1, 2).contiguous() for t in (q, k, v)), causal=True)
+        return out.reshape(2, -1)
+
+    wrt = (x, proj.weight)
+    want = torch.autograd.grad(region(x).float().sum(), wrt)
+    got = torch.autograd.grad(checkpoint(region, x, use_reentrant=False).float().sum(), wrt)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
