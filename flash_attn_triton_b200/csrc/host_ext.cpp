@@ -349,6 +349,12 @@ struct AttnBackward : public Node {
 template <typename F>
 Tensor with_grad(const Params& c, variable_list in, bool want_lse, Tensor& lse, F forward) {
   c10::cuda::CUDAGuard guard(in[0].device());
+  auto no_tangent = [](const Tensor& t) {
+    TORCH_CHECK_NOT_IMPLEMENTED(!t.defined() || !t._fw_grad(/*level=*/0).defined(),
+                                "the attention functions have no forward-mode derivative");
+  };
+  for (const auto& t : in) no_tangent(t);
+  no_tangent(c.alibi);
   const bool need = at::GradMode::is_enabled() && torch::autograd::any_variable_requires_grad(in);
   std::shared_ptr<AttnBackward> node;
   if (need) {

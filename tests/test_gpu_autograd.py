@@ -79,3 +79,18 @@ def test_checkpointed_region_that_ends_in_attention(call):
     got = torch.autograd.grad(checkpoint(region, x, use_reentrant=False).float().sum(), wrt)
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("call", ["dense", "packed", "varlen", "int8"])
+def test_forward_mode_is_refused(call):
+    import torch.autograd.forward_ad as fw
+    cu = torch.tensor([0, 256], dtype=torch.int32, device=DEV)
+    shape = dict(dense=(1, 256, 4, 64), packed=(1, 256, 3, 4, 64), varlen=(256, 4, 64), int8=(1, 4, 256, 64))[call]
+    x = mk(*shape)
+    run = dict(dense=lambda t: fa().flash_attn_func(x, t, x), packed=lambda t: fa().flash_attn_qkvpacked_func(t),
+               varlen=lambda t: fa().flash_attn_varlen_func(x, x, t, cu, cu, 256, 256),
+               int8=lambda t: fa().attention_int8(t, x, x))[call]
+    with fw.dual_level():
+        run(x)
+        with pytest.raises(NotImplementedError):
+            run(fw.make_dual(x, torch.ones_like(x)))
