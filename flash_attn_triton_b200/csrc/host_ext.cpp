@@ -316,8 +316,9 @@ struct AttnBackward : public Node {
   }
 
   variable_list apply(variable_list&& grads) override {
-    variable_list res(in.size());
-    if (!grads[0].defined()) return res;
+    std::lock_guard<std::mutex> lock(mutex_);    // against release_variables() of a backward on another thread
+    // no gradient came back to the output (a node behind it returned none): the inputs have one of zeros
+    const Tensor grad = grads[0].defined() ? grads[0] : input_metadata(0).zeros_like();
     // Unpacked before autograd is switched off: the hook of a checkpointed region runs that region's forward again
     // here, and its nodes have to save what this one saved.
     variable_list x;
@@ -333,10 +334,11 @@ struct AttnBackward : public Node {
       dq = task_should_compute_output(0);
       dkdv = task_should_compute_output(1) || (p.packing == kSeparate && task_should_compute_output(2));
     }
-    return run_backward(p, x, o, l, grads[0], dq, dkdv);
+    return run_backward(p, x, o, l, grad, dq, dkdv);
   }
   std::string name() const override { return "FlashAttnBackward"; }
   void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
     for (auto& s : in) s.reset_data();
     for (auto& s : side) s.reset_data();
     out.reset_data();

@@ -94,3 +94,39 @@ def test_forward_mode_is_refused(call):
         run(x)
         with pytest.raises(NotImplementedError):
             run(fw.make_dual(x, torch.ones_like(x)))
+
+
+def test_output_without_a_gradient_gives_zeros():
+    class Dropped(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.clone()
+
+        @staticmethod
+        def backward(ctx, grad):
+            return None
+
+    q, k, v = (mk(1, 256, 4, 64, seed=i).requires_grad_() for i in range(3))
+    w = mk(1, 256, 4, 64, seed=3).requires_grad_()
+    (Dropped.apply(fa().flash_attn_func(q, k, v)) * w).sum().backward()
+    for t in (q, k, v):
+        assert t.grad is not None and not t.grad.any()
+
+
+def test_backward_of_one_graph_from_several_threads():
+    import threading
+    q, k, v = (mk(1, 256, 4, 64, seed=i).requires_grad_() for i in range(3))
+    out = fa().flash_attn_func(q, k, v, causal=True)
+    want = torch.autograd.grad(out.float().sum(), (q, k, v), retain_graph=True)
+    got = [None] * 4
+
+    def run(i):
+        got[i] = torch.autograd.grad(out.float().sum(), (q, k, v), retain_graph=True)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for g in got:
+        assert all(torch.equal(a, b) for a, b in zip(g, want))
