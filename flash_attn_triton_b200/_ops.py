@@ -80,21 +80,61 @@ _BHSD = (0, 2, 1)      # (batch, heads, seq, dim)
 _THD = (None, 0, 1)    # packed (tokens, heads, dim)
 
 
+class _TracedCall(torch.autograd.Function):
+    """A differentiable call as one operation that torch.jit.trace records: it does not see the C++ nodes and
+    would take their results for constants.  `call` and what it holds are constants of the trace, `tensors` (None among
+    them) its inputs."""
+
+    @staticmethod
+    def forward(ctx, call, *tensors):
+        state = torch._C._get_tracing_state()
+        torch._C._set_tracing_state(None)           # the call's own autograd graph is no part of the trace
+        try:
+            ctx.tensors = [None if t is None else t.detach().requires_grad_(t.requires_grad) for t in tensors]
+            with torch.enable_grad():
+                result = call(*ctx.tensors)
+            ctx.result, lse = result if isinstance(result, tuple) else (result, None)
+            out = ctx.result.detach()
+        finally:
+            torch._C._set_tracing_state(state)
+        out = out.view(out.shape)                   # the trace wants an operation behind an output
+        if lse is None:
+            return out
+        lse = lse.view(lse.shape)
+        ctx.mark_non_differentiable(lse)
+        return out, lse
+
+    @staticmethod
+    def backward(ctx, grad, *unused):
+        wanted = [t for t in ctx.tensors if t is not None and t.requires_grad]
+        grads = iter(torch.autograd.grad(ctx.result, wanted, grad, retain_graph=True))
+        return (None, *(next(grads) if t is not None and t.requires_grad else None for t in ctx.tensors))
+
+
+_tracing = torch._C._get_tracing_state
+
+
 def dense_attention(q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl, layout, feat=None,
                     want_lse=False):
     """q (B,Sq,Hq,D), k/v (B,Sk,Hkv,D) ["bshd"] or head-major ["bhsd"] -> o like q (and the base-2 LSE
     (B,Hq,Sq) when asked for); differentiable in q, k and v."""
     f = feat or _NO_FEATURES
-    return N.host().dense(_SEPARATE, -1, q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl,
-                          layout == "bhsd", f.bias, f.dropout_p, f.seed, f.row_stride, want_lse)
+    tail = (q_pos_offset, impl, layout == "bhsd", f.bias, f.dropout_p, f.seed, f.row_stride, want_lse)
+    if _tracing() is not None:
+        return _TracedCall.apply(lambda q, k, v, alibi: N.host().dense(
+            _SEPARATE, -1, q, k, v, scale, causal, wl, wr, softcap, alibi, *tail), q, k, v, alibi)
+    return N.host().dense(_SEPARATE, -1, q, k, v, scale, causal, wl, wr, softcap, alibi, *tail)
 
 
 def dense_attention_packed(packing, dim, tensors, scale, causal, wl, wr, softcap, alibi, feat=None):
     """The same for packed inputs: tensors = (qkv,) with packing QKV or (q, kv) with KV, the packed
     dimension `dim`.  Gradients are written straight into packed tensors."""
     f = feat or _NO_FEATURES
-    return N.host().dense(packing, dim, *tensors, scale, causal, wl, wr, softcap, alibi, 0, N.IMPL_AUTO, False,
-                          f.bias, f.dropout_p, f.seed, f.row_stride, False)
+    tail = (0, N.IMPL_AUTO, False, f.bias, f.dropout_p, f.seed, f.row_stride, False)
+    if _tracing() is not None:
+        return _TracedCall.apply(lambda alibi, *tensors: N.host().dense(
+            packing, dim, *tensors, scale, causal, wl, wr, softcap, alibi, *tail), alibi, *tensors)
+    return N.host().dense(packing, dim, *tensors, scale, causal, wl, wr, softcap, alibi, *tail)
 
 
 def dense_forward(q, k, v, scale, causal, wl, wr, softcap, alibi, q_pos_offset, impl, layout,
@@ -143,8 +183,12 @@ def varlen_attention(packing, dim, tensors, cu_q, cu_k, max_q, max_k, scale, cau
     """Packed sequences: tensors = (q (Tq,Hq,D), k, v (Tk,Hkv,D)), or packed as in dense_attention_packed; int32
     cu_seqlens on the device; differentiable."""
     f = feat or _NO_FEATURES
-    return N.host().varlen(packing, dim, *tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
-                           f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse)
+    tail = (impl, f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse)
+    if _tracing() is not None:
+        return _TracedCall.apply(lambda cu_q, cu_k, alibi, *tensors: N.host().varlen(
+            packing, dim, *tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail),
+            cu_q, cu_k, alibi, *tensors)
+    return N.host().varlen(packing, dim, *tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail)
 
 
 def varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
@@ -229,6 +273,8 @@ def int8_forward(q, k, v, causal, scale, impl=N.IMPL_AUTO, k_valid=0, q_pos_offs
 
 def int8_attention(q, k, v, causal, scale, impl, k_valid=0, q_pos_offset=0):
     """INT8-QK^T forward, fp16 backward (attention_kernel_int8.py:220-267).  [B,H,S,D]."""
+    if _tracing() is not None:
+        return _TracedCall.apply(lambda q, k, v: N.host().int8(q, k, v, causal, scale, impl, k_valid, q_pos_offset), q, k, v)
     return N.host().int8(q, k, v, causal, scale, impl, k_valid, q_pos_offset)
 
 

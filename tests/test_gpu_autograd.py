@@ -130,3 +130,27 @@ def test_backward_of_one_graph_from_several_threads():
         t.join()
     for g in got:
         assert all(torch.equal(a, b) for a, b in zip(g, want))
+
+
+@pytest.mark.filterwarnings("ignore")
+@pytest.mark.parametrize("call", ["dense", "packed", "varlen", "int8"])
+def test_traced_calls_are_operations_of_the_trace(call):
+    slopes = torch.rand(2, 4, device=DEV)
+
+    def run(x, y, cu):
+        if call == "dense":
+            return fa().flash_attn_func(x, y, y, causal=True, alibi_slopes=slopes)
+        if call == "packed":
+            return fa().flash_attn_qkvpacked_func(torch.stack((x, y, y), dim=2), causal=True) + 1
+        if call == "varlen":
+            flat = [t.reshape(512, 4, 64) for t in (x, y)]
+            return fa().flash_attn_varlen_func(flat[0], flat[1], flat[1], cu, cu, 400, 400, causal=True)
+        return fa().attention_int8(*(t.transpose(1, 2).contiguous() for t in (x, y, y)), causal=True) + 1
+
+    cu = [torch.tensor([0, n, 512], dtype=torch.int32, device=DEV) for n in (200, 300)]
+    args = [(mk(2, 256, 4, 64, seed=i).requires_grad_(), mk(2, 256, 4, 64, seed=9 + i).requires_grad_(), cu[i]) for i in (0, 1)]
+    traced = torch.jit.trace(run, args[0], check_trace=False)
+    got, want = traced(*args[1]), run(*args[1])
+    assert torch.equal(got, want)
+    for a, b in zip(torch.autograd.grad(got.float().sum(), args[1][:2]), torch.autograd.grad(want.float().sum(), args[1][:2])):
+        assert torch.equal(a, b)
