@@ -14,6 +14,7 @@
 #include <cstddef>
 #include <type_traits>
 
+#include "bwd_stats.cuh"
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -50,8 +51,7 @@ template <int D> struct BCfg {
   static constexpr int kSmemTiles = (2 + kStagesQ + kStagesO) * kTileBytes;
   // dK/dV kernel: 128 x 16 operand tiles that carry the row statistics into the GEMMs
   // (two constant ones on the key side, one per ring stage on the query side)
-  static constexpr int kAugBytes = kT * 16 * 2;
-  static constexpr int kAugTotal = (2 + kStagesQ) * kAugBytes;
+  static constexpr int kAugTotal = (2 + kStagesQ) * kStatBlock;
   static constexpr int kSmemBytes = kSmemTiles + kAugTotal + 1024 + 8192;
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
   // dQ kernel: the K ring is one stage deeper than the V ring.  K(k+1) is needed by S(k+1) at
@@ -174,10 +174,9 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   BShared* sh = reinterpret_cast<BShared*>(tiles + C::kSmemTiles + C::kAugTotal);
   const uint32_t sV = smem_u32(tiles), sK = sV + C::kTileBytes;
   const uint32_t sRingQ = sK + C::kTileBytes, sRingO = sRingQ + C::kStagesQ * C::kTileBytes;
-  // statistics operands: [0] key side of the score GEMM, [1] key side of the dP GEMM,
-  // [2 + stage] query side (written per streamed query tile by the statistics warp)
+  // statistics operands: one block per ring stage, then the two of the key side (bwd_stats.cuh)
   unsigned char* aug = tiles + C::kSmemTiles;
-  const uint32_t sAug = sV + C::kSmemTiles;
+  const uint32_t sAug = sV + C::kSmemTiles, sAugKeys = sAug + C::kStagesQ * kStatBlock;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nblk = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
@@ -214,27 +213,8 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     sh->abort_flag = 0;
     fence_barrier_init();
   }
-  {
-    // Statistics operands, no-swizzle K-major layout: columns 0-7 of row r at
-    // (r / 8) * 128 + (r % 8) * 16, columns 8-15 (always zero) 2048 bytes further.
-    // Query side, per row:  [l_hi, l_hi, l_lo, l_lo, d_hi, d_lo, 0, 0]  with l = -lse2, d = -delta
-    // key side, scores:     [w_hi, w_lo, w_hi, w_lo, 0, 0, 0, 0]        with w = 1 / scale_log2
-    // key side, dP:         [0, 0, 0, 0, 1, 1, 0, 0]
-    // so the score GEMM yields S - lse2 / scale_log2 and the dP GEMM dP - delta.
-    const float w = 1.f / cfg.scale_log2;
-    const T w_hi = Elem<T>::from_f(w), w_lo = Elem<T>::from_f(w - Elem<T>::to_f(w_hi));
-    const uint32_t wp = (uint32_t)(*reinterpret_cast<const uint16_t*>(&w_hi)) |
-                        ((uint32_t)(*reinterpret_cast<const uint16_t*>(&w_lo)) << 16);
-    const uint32_t ones = Elem<T>::pack(1.f, 1.f);
-    uint4* a4 = reinterpret_cast<uint4*>(aug);
-    for (int i = tid; i < C::kAugTotal / 16; i += kBwdThreads) {
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (i < kT) val = make_uint4(wp, wp, 0u, 0u);
-      else if (i >= C::kAugBytes / 16 && i < C::kAugBytes / 16 + kT) val = make_uint4(0u, 0u, ones, 0u);
-      a4[i] = val;
-    }
-    fence_proxy_async();
-  }
+  stat_write_keys<T>(aug + C::kStagesQ * kStatBlock, cfg.scale_log2, tid, kBwdThreads);
+  fence_proxy_async();
   if (warp == 8) {
     tmem_alloc(smem_u32(&sh->tmem_base), 512);
     tmem_relinquish();
@@ -282,11 +262,13 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     // ------------------------------- statistics loader ----------------------------------
     // The loads of tile it+1 are ISSUED right after tile it has been written and only consumed
     // after the wait for the next slot, so their latency hides behind that wait (nothing reads
-    // the registers in between: a scoreboard stall before the poll would serialise the two).
+    // the registers in between: a scoreboard stall before the poll would serialise the two; the pieces worked
+    // out there too cost 4 x 1024 x 1531 of 32 heads of 64 387 -> 488 us).
     reg_dealloc<kRegsService>();
     int stage = 0;
     uint32_t phase = 0;
     float rl[kT / 32], rd[kT / 32];                  // statistics of rows lane, lane + 32, ... as loaded
+    const float unit = stat_score_unit(cfg.scale_log2);
     auto fetch = [&](int it) {
       const int hq = hk * G + it / ntiles, m = m_lo + it % ntiles;
 #pragma unroll
@@ -307,23 +289,13 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       bool w = true;
       if (lane == 0) w = bwait_relaxed(&sh->empty_a[stage], phase ^ 1, sh, 42);
       if (!__all_sync(0xffffffffu, w)) break;
-      uint4* q4 = reinterpret_cast<uint4*>(aug + (2 + stage) * C::kAugBytes);
 #pragma unroll
       for (int k = 0; k < kT / 32; ++k) {
         const int i = lane + 32 * k;
-        // NEGATED; rows that do not exist or see no key get a large finite value instead of
-        // infinity (an infinity would meet the zeros of the other GEMM's key-side operand): P = 0
-        float nl2 = kDrop ? cfg.drop_log2 - rl[k] : -rl[k];
-        const float ndl = fminf(fmaxf(-rd[k], -60000.f), 60000.f);   // kept inside the 16-bit range
-        if (!(fabsf(nl2) < 60000.f)) nl2 = -60000.f;
-        // the feature variant adds the LSE after the soft cap, in the element-wise warps
-        if (kExtras) sh->lse[stage][i] = nl2 == -60000.f ? -INFINITY : nl2;
-        const float lf = kExtras ? 0.f : nl2;
-        const T l_hi = Elem<T>::from_f(lf), l_lo = Elem<T>::from_f(lf - Elem<T>::to_f(l_hi));
-        const T d_hi = Elem<T>::from_f(ndl), d_lo = Elem<T>::from_f(ndl - Elem<T>::to_f(d_hi));
-        const uint32_t lh = *reinterpret_cast<const uint16_t*>(&l_hi), ll = *reinterpret_cast<const uint16_t*>(&l_lo);
-        const uint32_t dh = *reinterpret_cast<const uint16_t*>(&d_hi), dl = *reinterpret_cast<const uint16_t*>(&d_lo);
-        q4[i] = make_uint4(lh | (lh << 16), ll | (ll << 16), dh | (dl << 16), 0u);
+        // NEGATED.  The feature variant adds the LSE after the soft cap, in the element-wise warps.
+        const float nl2 = kDrop ? cfg.drop_log2 - rl[k] : -rl[k];
+        if (kExtras) sh->lse[stage][i] = isinf(nl2) ? -INFINITY : nl2;
+        stat_write_row<T, !kExtras>(aug + stage * kStatBlock, i, nl2, -rd[k], unit);
       }
       fence_proxy_async();
       __syncwarp();
@@ -346,11 +318,10 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       };
       auto slotQ = [&](int it) { return sRingQ + (it % C::kStagesQ) * C::kTileBytes; };
       auto slotO = [&](int it) { return sRingO + (it % C::kStagesO) * C::kTileBytes; };
-      auto stat_desc = [&](int it) {
-        return make_smem_desc_noswizzle(sAug + (2 + it % C::kStagesQ) * C::kAugBytes, 2048, 128);
+      auto stat_desc = [&](int it, bool dp) {
+        return stat_desc_query(sAugKeys, sAug + (it % C::kStagesQ) * kStatBlock, dp);
       };
-      const uint64_t dstat_s = make_smem_desc_noswizzle(sAug, 2048, 128);
-      const uint64_t dstat_dp = make_smem_desc_noswizzle(sAug + C::kAugBytes, 2048, 128);
+      const uint64_t dstat_s = stat_desc_key(sAugKeys, false), dstat_dp = stat_desc_key(sAugKeys, true);
       // S^T(i) = K Q(i)^T - lse2 / scale_log2; waits for Q(i) and its statistics
       auto issue_s = [&](int i) {
         const int st = i % C::kStagesQ;
@@ -359,7 +330,7 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (i > 0) wq(&sh->r_free, 1, 49);                                     // dP(i-1) read out
         if (!ok) return;
         mma_kmajor<D>(tR, sK, slotQ(i), idesc_s, leader);
-        if (!kExtras) mma_f16_ss_lp(tR, dstat_s, stat_desc(i), idesc_s, 1u, leader);
+        if (!kExtras) mma_f16_ss_lp(tR, dstat_s, stat_desc(i, false), idesc_s, 1u, leader);
         mma_commit_lp(smem_u32(&sh->s_full[0]), leader);
       };
       // This warp issues the GEMMs into the fp32 region R: dP(i), then S(i+1) -- each once the
@@ -374,7 +345,7 @@ bwd_dkdv_cta_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         wq(&sh->r_free, 0, 49);                                                // S(i) read out
         if (!ok) break;
         mma_kmajor<D>(tR, sV, slotO(i), idesc_s, leader);                      // dP^T(i) = V dO(i)^T
-        mma_f16_ss_lp(tR, dstat_dp, stat_desc(i), idesc_s, 1u, leader);        //           - delta
+        mma_f16_ss_lp(tR, dstat_dp, stat_desc(i, true), idesc_s, 1u, leader);  //           - delta
         mma_commit_lp(smem_u32(&sh->dp_full), leader);
         mma_commit_lp(smem_u32(&sh->empty_b[so]), leader);   // this warp's last reads of dO(i) and of
         mma_commit_lp(smem_u32(&sh->empty_a[st]), leader);   // Q(i) and its statistics

@@ -45,6 +45,7 @@
 #include <type_traits>
 
 #include <cstdlib>
+#include "bwd_stats.cuh"
 #include "common.cuh"
 #define PROF_TAG bwd
 #include "prof.cuh"
@@ -85,8 +86,7 @@ template <int D> struct BCfg {
   static constexpr int kSmemTiles = (1 + kStagesQ + kStagesO) * kTileBytes;
   // dK/dV kernel: 128 x 16 operand tiles that carry the row statistics into the GEMMs
   // (two constant ones on the key side, one per ring stage on the query side)
-  static constexpr int kAugBytes = kT * 16 * 2;
-  static constexpr int kAugTotal = (2 + kStagesQ) * kAugBytes;
+  static constexpr int kAugTotal = (2 + kStagesQ) * kStatBlock;
   static constexpr int kSmemBytes = kSmemTiles + kAugTotal + 1024 + 4096;
   static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
   // dQ kernel: Q and dO resident, ring A of K tiles (dQ is staged over the last one), ring B of V tiles.  The K
@@ -427,10 +427,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   BShared* sh = reinterpret_cast<BShared*>(tiles + C::kSmemTiles + C::kAugTotal);
   const uint32_t sV = smem_u32(tiles);
   const uint32_t sRingQ = sV + C::kTileBytes, sRingO = sRingQ + SQ * C::kTileBytes;
-  // statistics operands: [0] key side of the score GEMM, [1] key side of the dP GEMM,
-  // [2 + stage] query side (written per streamed query tile by the statistics warp)
+  // statistics operands: one block per ring stage, then the two of the key side (bwd_stats.cuh)
   unsigned char* aug = tiles + C::kSmemTiles;
-  const uint32_t sAug = sV + C::kSmemTiles;
+  const uint32_t sAug = sV + C::kSmemTiles, sAugKeys = sAug + SQ * kStatBlock;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.heads_q / p.heads_kv;
@@ -467,27 +466,8 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     sh->abort_flag = 0;
     fence_barrier_init();
   }
-  {
-    // Statistics operands, no-swizzle K-major layout: columns 0-7 of row r at
-    // (r / 8) * 128 + (r % 8) * 16, columns 8-15 (always zero) 2048 bytes further.
-    // Query side, per row:  [l_hi, l_hi, l_lo, l_lo, d_hi, d_lo, 0, 0]  with l = -lse2, d = -delta
-    // key side, scores:     [w_hi, w_lo, w_hi, w_lo, 0, 0, 0, 0]        with w = 1 / scale_log2
-    // key side, dP:         [0, 0, 0, 0, 1, 1, 0, 0]
-    // so the score GEMM yields S - lse2 / scale_log2 and the dP GEMM dP - delta.
-    const float w = 1.f / cfg.scale_log2;
-    const T w_hi = Elem<T>::from_f(w), w_lo = Elem<T>::from_f(w - Elem<T>::to_f(w_hi));
-    const uint32_t wp = (uint32_t)(*reinterpret_cast<const uint16_t*>(&w_hi)) |
-                        ((uint32_t)(*reinterpret_cast<const uint16_t*>(&w_lo)) << 16);
-    const uint32_t ones = Elem<T>::pack(1.f, 1.f);
-    uint4* a4 = reinterpret_cast<uint4*>(aug);
-    for (int i = tid; i < C::kAugTotal / 16; i += kBwdThreads) {
-      uint4 val = make_uint4(0u, 0u, 0u, 0u);
-      if (i < kT) val = make_uint4(wp, wp, 0u, 0u);
-      else if (i >= C::kAugBytes / 16 && i < C::kAugBytes / 16 + kT) val = make_uint4(0u, 0u, ones, 0u);
-      a4[i] = val;
-    }
-    fence_proxy_async();
-  }
+  stat_write_keys<T>(aug + SQ * kStatBlock, cfg.scale_log2, tid, kBwdThreads);
+  fence_proxy_async();
   if (warp == 8) {
     tmem_alloc(smem_u32(&sh->tmem_base), 512);
     tmem_relinquish();
@@ -580,6 +560,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     // consumed after the wait for the next slot, so their latency hides behind that wait.
     reg_dealloc<kRegsService>();
     float rl[kT / 32], rd[kT / 32];                  // statistics of rows lane, lane + 32, ... as loaded
+    const float unit = stat_score_unit(cfg.scale_log2);
     auto fetch = [&](const KItem& w, int it) {
       const int hq = w.hk * G + it / w.ntiles, m = w.m_lo + it % w.ntiles;
 #pragma unroll
@@ -611,24 +592,12 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         bool wt = true;
         if (lane == 0) wt = bwait_relaxed(&sh->empty_a[stage], ((posA / SQ) & 1) ^ 1, sh, 42);
         if (!__all_sync(0xffffffffu, wt)) { ok = false; break; }
-        uint4* q4 = reinterpret_cast<uint4*>(aug + (2 + stage) * C::kAugBytes);
 #pragma unroll
         for (int k = 0; k < kT / 32; ++k) {
           const int i = lane + 32 * k;
-          // NEGATED; rows that do not exist or see no key get a large finite value instead of
-          // infinity (an infinity would meet the zeros of the other GEMM's key-side operand): P = 0.
-          // delta is clamped into the 16-bit range for the same reason.
-          float nl2 = -rl[k];
-          float ndl = fminf(fmaxf(-rd[k], -60000.f), 60000.f);
-          if (!(fabsf(nl2) < 60000.f)) nl2 = -60000.f;
-          // the feature variant adds the LSE after the soft cap, in the element-wise warps
-          if (kExtras) sh->lse[stage][i] = nl2 == -60000.f ? -INFINITY : nl2;
-          const float lf = kExtras ? 0.f : nl2;
-          const T l_hi = Elem<T>::from_f(lf), l_lo = Elem<T>::from_f(lf - Elem<T>::to_f(l_hi));
-          const T d_hi = Elem<T>::from_f(ndl), d_lo = Elem<T>::from_f(ndl - Elem<T>::to_f(d_hi));
-          const uint32_t lh = *reinterpret_cast<const uint16_t*>(&l_hi), ll = *reinterpret_cast<const uint16_t*>(&l_lo);
-          const uint32_t dh = *reinterpret_cast<const uint16_t*>(&d_hi), dl = *reinterpret_cast<const uint16_t*>(&d_lo);
-          q4[i] = make_uint4(lh | (lh << 16), ll | (ll << 16), dh | (dl << 16), 0u);
+          // NEGATED.  The feature variant adds the LSE after the soft cap, in the element-wise warps.
+          if (kExtras) sh->lse[stage][i] = isinf(rl[k]) ? -INFINITY : -rl[k];
+          stat_write_row<T, !kExtras>(aug + stage * kStatBlock, i, -rl[k], -rd[k], unit);
         }
         fence_proxy_async();
         __syncwarp();
@@ -662,11 +631,8 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (ok) ok = bwait(bar, parity, sh, code);
       tc_fence_after();
     };
-    const uint64_t dstat_s = make_smem_desc_noswizzle(sAug, 2048, 128);
-    const uint64_t dstat_dp = make_smem_desc_noswizzle(sAug + C::kAugBytes, 2048, 128);
-    auto stat_desc = [&](int pos) {
-      return make_smem_desc_noswizzle(sAug + (2 + pos % SQ) * C::kAugBytes, 2048, 128);
-    };
+    const uint64_t dstat_s = stat_desc_key(sAugKeys, false), dstat_dp = stat_desc_key(sAugKeys, true);
+    auto stat_desc = [&](int pos, bool dp) { return stat_desc_query(sAugKeys, sAug + (pos % SQ) * kStatBlock, dp); };
     PROF_VARS(8);
     int posA = 0, posB = 0, wi = 0, tg = 0;          // tg: tiles issued so far by this CTA
     // The last query tile of a packed sequence also stages rows of the NEXT sequence.  Their P is
@@ -684,7 +650,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       PROF_ADD(2);
       if (!ok) return;
       mma_kmajor_ts<D>(tR, tK, slotA(qpos), idesc_s, leader);
-      if (!kExtras) mma_f16_ss_lp(tR, dstat_s, stat_desc(qpos), idesc_s, 1u, leader);
+      if (!kExtras) mma_f16_ss_lp(tR, dstat_s, stat_desc(qpos, false), idesc_s, 1u, leader);
       mma_commit_lp(smem_u32(&sh->s_full[0]), leader);
     };
     int sidx = 0;
@@ -722,7 +688,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         PROF_ADD(5);
         if (!ok) break;
         mma_kmajor<D>(tR, sV, slotB(opos), idesc_s, leader);                    // dP^T(i) = V dO(i)^T
-        mma_f16_ss_lp(tR, dstat_dp, stat_desc(qpos), idesc_s, 1u, leader);      //           - delta
+        mma_f16_ss_lp(tR, dstat_dp, stat_desc(qpos, true), idesc_s, 1u, leader); //           - delta
         mma_commit_lp(smem_u32(&sh->dp_full), leader);
         if (i + 1 < w.total) {
           mma_commit_lp(smem_u32(&sh->empty_b[opos % SO]), leader);   // this warp's last reads of dO(i) and of
