@@ -123,6 +123,12 @@ def _check_head_dim(d):
         raise ValueError("head dimension must be one of 16, 32, 64, 128, or 256")
 
 
+def _in_place(packed):
+    """Whether the kernels can read the slices of a packed tensor where they are.  Otherwise (an address that is not a
+    multiple of 16 bytes, rows of an odd pitch) it goes the way of separate tensors, which copies the slices."""
+    return packed.data_ptr() % 16 == 0 and (packed.is_contiguous() or N.kernel_ready(packed))
+
+
 def _packed_call(packing, tensors, shape_q, seqlen_k, dropout_p, softmax_scale, causal, window_size, softcap, alibi_slopes):
     """A checked dense call on packed inputs (dimension 2 holds q/k/v or k/v): the kernels read the slices
     through their strides and write the gradients straight into a packed tensor."""
@@ -217,7 +223,7 @@ def flash_attn_qkvpacked_func(qkv, dropout_p=0.0, softmax_scale=None, causal=Fal
         raise ValueError("qkv must have shape (batch, seqlen, 3, nheads, headdim)")
     batch, seqlen, _, heads, head_dim = qkv.shape
     if (qkv.is_cuda and qkv.dtype in _KERNEL_DTYPES and heads and head_dim in _HEAD_DIMS and softcap >= 0.0
-            and 0.0 <= dropout_p < 1.0 and attn_bias is None and not return_attn_probs):
+            and 0.0 <= dropout_p < 1.0 and attn_bias is None and not return_attn_probs and _in_place(qkv)):
         return _packed_call(_ops.PACK_QKV, (qkv,), (batch, seqlen, heads, head_dim), seqlen, dropout_p, softmax_scale, causal,
                             window_size, softcap, alibi_slopes)
     q, k, v = qkv.unbind(dim=2)
@@ -237,7 +243,7 @@ def flash_attn_kvpacked_func(q, kv, dropout_p=0.0, softmax_scale=None, causal=Fa
     if (kv.is_cuda and kv.dtype in _KERNEL_DTYPES and q.dtype == kv.dtype and q.ndim == 4 and q.device == kv.device
             and q.shape[0] == batch and q.shape[3] == head_dim and heads_k and q.shape[2] % heads_k == 0
             and head_dim in _HEAD_DIMS and softcap >= 0.0 and 0.0 <= dropout_p < 1.0 and attn_bias is None
-            and not return_attn_probs):
+            and not return_attn_probs and _in_place(kv)):
         return _packed_call(_ops.PACK_KV, (q, kv), q.shape, seqlen_k, dropout_p, softmax_scale, causal, window_size,
                             softcap, alibi_slopes)
     k, v = kv.unbind(dim=2)
