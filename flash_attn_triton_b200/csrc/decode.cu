@@ -173,11 +173,11 @@ __device__ __forceinline__ SeqTiles seq_tiles(const fa_decode_args& p, const Sco
   return s;
 }
 
-// Elements [d, d + 4) of one output row, merged from `parts` pieces in slots s0, s0 + step, ...  Eight
+// Elements [d, d + 4) of one output row, merged from the `parts` workspace rows r0, r0 + step, ...  Eight
 // pieces are loaded at a time, their common maximum taken first.
-template <typename T, int D, int kRows>
-__device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_l, int64_t s0, int step, int parts, int row,
-                                             int d, T* og) {
+template <typename T, int D>
+__device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_l, int64_t r0, int64_t step, int parts, int d,
+                                             T* og) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float wsum = 0.f, m = -INFINITY;
   for (int i0 = 0; i0 < parts; i0 += 8) {
@@ -186,7 +186,7 @@ __device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int i = i0 + j;
-      const int64_t r = (s0 + (int64_t)i * step) * kRows + row;
+      const int64_t r = r0 + i * step;
       l[j] = i < parts ? ws_l[r] : -INFINITY;
       x[j] = i < parts ? *reinterpret_cast<const float4*>(ws_o + r * D + d) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
   }
 
   float* ws_o = reinterpret_cast<float*>(p.workspace);
-  float* ws_l = ws_o + (int64_t)gridDim.x * kRows * D;
+  float* ws_l = ws_o + (int64_t)(gridDim.x / U) * p.heads_kv * R * D;
   const T* cos = reinterpret_cast<const T*>(p.rotary_cos);
   const T* sin = reinterpret_cast<const T*>(p.rotary_sin);
   int stage = 0;
@@ -628,7 +628,8 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
   }
 
   // ---- output, or a piece of it -----------------------------------------------------------
-  const int slot = blockIdx.x;
+  // workspace: the R query rows of every (piece, kv head), not padded to units
+  const int64_t ws_row = ((int64_t)share * p.heads_kv + hk) * R + rg * kRows;
   for (int i = tid; i < kRows * (D / 4); i += NT) {
     const int r = i / (D / 4), c4 = (i % (D / 4)) * 4;
     const int gr = rg * kRows + r;
@@ -650,8 +651,8 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
       pk.y = Elem<T>::pack(acc.z, acc.w);
       *reinterpret_cast<uint2*>(og) = pk;
     } else {
-      *reinterpret_cast<float4*>(ws_o + ((int64_t)slot * kRows + r) * D + c4) = acc;
-      if (c4 == 0) ws_l[(int64_t)slot * kRows + r] = lsum > 0.f ? mstar + log2f(lsum) : -INFINITY;
+      *reinterpret_cast<float4*>(ws_o + (ws_row + r) * D + c4) = acc;
+      if (c4 == 0) ws_l[ws_row + r] = lsum > 0.f ? mstar + log2f(lsum) : -INFINITY;
     }
   }
   if (parts > 1) {
@@ -671,7 +672,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
       for (int i = tid; i < rows * (D / 4); i += NT) {
         const int r = i / (D / 4), gr = rg * kRows + r;
         const int sq = gr / G, h = hk * G + gr % G;
-        merge_pieces<T, D, kRows>(ws_o, ws_l, (int64_t)base * U + u, U, parts, r, (i % (D / 4)) * 4,
+        merge_pieces<T, D>(ws_o, ws_l, ((int64_t)base * p.heads_kv + hk) * R + gr, (int64_t)p.heads_kv * R, parts, (i % (D / 4)) * 4,
                            reinterpret_cast<T*>(p.o) + b * p.o_stride[0] + sq * p.o_stride[1] + (int64_t)h * p.o_stride[2]);
       }
     }
@@ -846,11 +847,10 @@ static DecodeGeom decode_geometry(const fa_decode_args& a) {
   return g;
 }
 
-// pieces (the rows of a unit in fp32 and their LSEs each), then the counters if the caller brings none
+// pieces (their query rows in fp32, then the LSEs of those), then the counters if the caller brings none
 static size_t decode_piece_bytes(const fa_decode_args& a, const DecodeGeom& g) {
   if (g.splits == 1) return 0;
-  const size_t slots = (size_t)g.shares * a.heads_kv * g.row_groups;
-  return slots * decode_unit_rows(a) * (a.head_dim + 1) * sizeof(float);
+  return (size_t)g.shares * a.seqlen_q * a.heads_q * (a.head_dim + 1) * sizeof(float);
 }
 size_t decode_workspace_bytes(const fa_decode_args& a) {
   if (a.heads_kv <= 0 || a.heads_q <= 0 || a.batch <= 0 || a.seqlen_q <= 0) return 0;
@@ -1172,9 +1172,29 @@ static void* static_scratch_ptr(int device) {
 
 size_t decode_static_scratch_bytes() { return kStaticScratchBytes; }
 
+// Pieces of a full cache when each is a multiple of 64 keys, from 256 keys on of 256.
+static int whole_splits(const fa_decode_args& a) {
+  const int64_t cap = a.block_table ? (int64_t)a.block_table_stride * a.page_size : a.page_size;
+  int64_t keys = (cap + a.num_splits - 1) / a.num_splits;
+  keys = (keys + 63) / 64 * 64;
+  if (keys >= 256) keys = (keys + 255) / 256 * 256;
+  const int64_t n = keys > 0 ? (cap + keys - 1) / keys : 1;
+  return n < 1 ? 1 : (int)n;
+}
+
 int decode_paged_static(const fa_decode_args& a, cudaStream_t st) {
   if (a.batch == 0 || a.seqlen_q == 0 || a.heads_q == 0) return FA_OK;
-  const size_t need = decode_workspace_bytes(a);
+  fa_decode_args b = a;
+  // Fewer pieces rather than a refusal: they cost time where a sequence is long and the batch small, and such
+  // calls fit.  A number of pieces that the caller asked for stands for pieces of whole 64 or 256 keys.
+  if (decode_workspace_bytes(b) > kStaticScratchBytes) {
+    if (a.num_splits > 0) {
+      b.num_splits = whole_splits(a);
+    } else {
+      for (b.num_splits = 8; b.num_splits > 1 && decode_workspace_bytes(b) > kStaticScratchBytes;) b.num_splits /= 2;
+    }
+  }
+  const size_t need = decode_workspace_bytes(b);
   if (need > kStaticScratchBytes) {
     set_error("fa_decode_paged_static: this problem needs %zu bytes of split-KV scratch but the "
               "built-in array holds %zu; pass a smaller num_splits or use fa_decode_paged with "
@@ -1183,7 +1203,6 @@ int decode_paged_static(const fa_decode_args& a, cudaStream_t st) {
   }
   void* p = static_scratch_ptr(a.device);
   if (p == nullptr) return FA_ERR_LAUNCH;
-  fa_decode_args b = a;
   b.workspace = p;
   b.workspace_bytes = kStaticScratchBytes;
   return decode_paged(b, st);

@@ -245,7 +245,7 @@ size_t fa_decode_checked_workspace_bytes(const fa_decode_args* args);
 /* Words fa_decode_args.counters needs for this problem. */
 int32_t fa_decode_counters(const fa_decode_args* args);
 
-/* Bytes of workspace fa_decode_paged needs for this problem (host-only, no CUDA call). */
+/* Bytes of workspace fa_decode_paged needs for this problem (no stream operation; asks the device for its number of SMs). */
 size_t fa_decode_workspace_bytes(const fa_decode_args* args);
 
 /*
@@ -259,9 +259,10 @@ size_t fa_decode_workspace_bytes(const fa_decode_args* args);
  * args->workspace_bytes are ignored; q, o, the caches and every other buffer are still the
  * caller's.  The call makes no cudaMalloc/cudaFree and calls no allocating library routine.
  *
- *  - A problem whose partials exceed the array (fa_decode_workspace_bytes(args) >
- *    fa_decode_static_scratch_bytes()) is refused with FA_ERR_WORKSPACE and a message;
- *    a smaller args->num_splits shrinks the need.
+ *  - Where the partials of the automatic choice (num_splits = 0) exceed the array, the sequences are cut
+ *    into fewer pieces, at last into one, which needs no scratch.  An explicit num_splits whose partials exceed
+ *    it, also with pieces of whole 64 or 256 keys, is refused with FA_ERR_WORKSPACE and a message; a smaller one
+ *    shrinks the need.
  *  - The first call on each device looks up the array's device address
  *    (cudaGetSymbolAddress, with that device current) and keeps it; make that first call
  *    outside any stream capture.

@@ -68,3 +68,28 @@ def test_static_scratch_rejects_oversized_problem():
     with pytest.raises(RuntimeError, match="built-in array"):
         _ops.kvcache_decode_static(q, torch.empty_like(q), kc, kc.clone(), cl, block_table=bt,
                                    num_splits=40)
+
+
+@pytest.mark.parametrize("B,Sq,Hq,Hkv,rotary,splits", [
+    (512, 1, 32, 8, False, 0),      # pieces of the automatic choice: a slot per sequence and more
+    (120, 1, 32, 32, False, 0),
+    (16, 256, 32, 8, True, 0),      # a chunk: its rotated queries alone are 32 MiB
+    (16, 1, 32, 32, False, 16),     # one query row per kv head, asked for in 16 pieces
+    (64, 1, 32, 8, False, 15),      # 15 pieces of 3200 keys are 13 of 256
+])
+def test_static_scratch_takes_what_fits_in_fewer_pieces(B, Sq, Hq, Hkv, rotary, splits):
+    import flash_attn_triton_b200 as fa
+    from flash_attn_triton_b200 import _ops
+    D, page, pages = 128, 64, 50
+    g = torch.Generator(DEV).manual_seed(B)
+    mk = lambda *s: torch.randn(*s, device=DEV, dtype=torch.half, generator=g)
+    q, kc, vc = mk(B, Sq, Hq, D), mk(pages, page, Hkv, D), mk(pages, page, Hkv, D)
+    bt = torch.arange(pages, dtype=torch.int32, device=DEV).repeat(B, 1)          # every sequence reads the same cache
+    cl = torch.randint(Sq, pages * page + 1, (B,), dtype=torch.int32, device=DEV, generator=g)
+    cos, sin = (t.to(DEV) for t in cases.rotary_tables(pages * page + 1, D)) if rotary else (None, None)
+    want = fa.flash_attn_with_kvcache(q, kc, vc, rotary_cos=cos, rotary_sin=sin, cache_seqlens=cl, block_table=bt, causal=True,
+                                      rotary_interleaved=False)
+    out = torch.full_like(q, float("nan"))
+    _ops.kvcache_decode_static(q, out, kc, vc, cl, block_table=bt, cos=cos, sin=sin, rotary_interleaved=False, causal=True,
+                               num_splits=splits)
+    assert maxdiff(out, want) <= util.FWD_TOL
