@@ -193,14 +193,15 @@ __device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_
     float mn = m;
 #pragma unroll
     for (int j = 0; j < 8; ++j) mn = fmaxf(mn, l[j]);
-    if (mn == -INFINITY) continue;
-    const float sc = exp2f(m - mn);
+    // pieces without a finite score weigh 0, which a NaN in them survives
+    const float mf = mn == -INFINITY ? 0.f : mn;
+    const float sc = exp2f(m - mf);
     acc.x *= sc; acc.y *= sc; acc.z *= sc; acc.w *= sc;
     wsum *= sc;
     m = mn;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float w = exp2f(l[j] - mn);
+      const float w = exp2f(l[j] - mf);
       wsum += w;
       acc.x += w * x[j].x; acc.y += w * x[j].y; acc.z += w * x[j].z; acc.w += w * x[j].w;
     }
@@ -564,8 +565,9 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
     for (int n = 0; n < NB; ++n) {
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float m = mrow[n][e & 1];
-        s[n][e] = m == -INFINITY ? 0.f : ex2(fmaf(s[n][e], mul, -m));
+        // no finite score yet: exponents relative to 0, so that -inf gives 0 and NaN stays NaN
+        const float m = mrow[n][e & 1] == -INFINITY ? 0.f : mrow[n][e & 1];
+        s[n][e] = ex2(fmaf(s[n][e], mul, -m));
         lrow[n][e & 1] += s[n][e];
       }
       // P^T[key][row] as the accumulator holds it -> B fragment [keys] x [rows]

@@ -191,3 +191,20 @@ def test_config4_shape():
         qb = orc.apply_rotary_ref(q[b].cpu(), cos, sin, torch.tensor([L]), False)
         ro, _ = orc.attention_ref(qb[None], kb[None], vb[None])
         assert maxdiff(out[b:b + 1], ro) <= util.FWD_TOL
+
+
+@pytest.mark.parametrize("tokens,length,splits", [(1, 100, 0), (1, 4000, 0), (1, 4000, 4), (2, 700, 0), (64, 4000, 0)])
+@pytest.mark.parametrize("D", [64, 256])
+def test_nan_query_gives_nan(tokens, length, splits, D):
+    """A broken row shows, in one piece and in several; its neighbours, rows without keys among them, stay what they are."""
+    g = torch.Generator(DEV).manual_seed(length)
+    mk = lambda *s: torch.randn(*s, device=DEV, dtype=torch.half, generator=g)
+    q, kc, vc = mk(3, tokens, 8, D), mk(3, 4096, 2, D), mk(3, 4096, 2, D)
+    lens = torch.tensor([length, length, 0], dtype=torch.int32, device=DEV)
+    call = lambda x: fa().flash_attn_with_kvcache(x, kc, vc, cache_seqlens=lens, num_splits=splits)
+    want = call(q)
+    q[0, 0, 1] = float("nan")
+    out = call(q)
+    assert out[0, 0, 1].isnan().all()
+    out[0, 0, 1] = want[0, 0, 1]
+    assert torch.equal(out, want) and not out[2].any()
