@@ -730,6 +730,11 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           }
         }
       }
+    } else if (kCache && w.parts > 1 && tid == 0) {
+      // A piece whose wait ran out counts too: the counters outlive the call and have to be zero again once the
+      // status has been cleared.  (If another CTA is the last, it merges what there is: the call has failed.)
+      uint32_t* ctr = geo.counters + blockIdx.x / geo.parts;
+      if (atomicAdd(ctr, 1u) == (uint32_t)(w.parts - 1)) *ctr = 0u;
     }
   }
 
