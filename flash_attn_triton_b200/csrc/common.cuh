@@ -67,8 +67,8 @@ struct ScoreCfg {
   // log2 by which a row maximum must exceed the one its exponents are relative to before O is rescaled (tcgen05
   // forward kernels).  8 saves most rescales, but a row's largest probability is then 2^x and is rounded to 16 bits,
   // where relative to its own maximum it is exactly 1: errors against float64 grow by 1 to 10 %.  0 where the
-  // mma.sync kernels, which always rescale, set the precision of a call: head_dim 256, fewer than 256 keys, KV-cache
-  // chunks, INT8 at head_dim 64 (bf16, 2 x 1999 tokens, head_dim 256: 2.017e-3 both, 2.075e-3 with 8).
+  // mma.sync kernels, which always rescale, set the precision of a call: head_dim 256, fewer than 256 keys, dropout,
+  // KV-cache chunks, INT8 at head_dim 64; decode has the same rule in its own kernel (bf16, 2 x 1999 tokens, head_dim 256: 2.017e-3 both, 2.075e-3 with 8).
   float rescale_at;
 };
 

@@ -538,8 +538,8 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
         mx[n][i] = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
-        // raised only when it grows by more than 2^8: the sums stay in range and O is rarely touched
-        grow |= mx[n][i] > mrow[n][i] + 8.f;
+        // raised whenever it grows: the largest probability is then exactly 1 (ScoreCfg::rescale_at)
+        grow |= mx[n][i] > mrow[n][i];
       }
     }
     if (__any_sync(0xffffffffu, grow)) {
@@ -548,7 +548,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
         float alpha[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-          const bool up = mx[n][i] > mrow[n][i] + 8.f;
+          const bool up = mx[n][i] > mrow[n][i];
           alpha[i] = up ? exp2f(mrow[n][i] - mx[n][i]) : 1.f;    // from -inf: 0
           if (up) mrow[n][i] = mx[n][i];
           lrow[n][i] *= alpha[i];

@@ -852,7 +852,7 @@ static bool one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
 
 int fwd_sm100(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
   ScoreCfg cfg = plain;
-  if (a.head_dim == 256 || a.seqlen_k < 256) cfg.rescale_at = 0.f;
+  if (a.head_dim == 256 || a.seqlen_k < 256 || cfg.keep != nullptr) cfg.rescale_at = 0.f;
   if (a.head_dim == 256) return fwd_alt_sm100(a, cfg, st);
   // FA_B200_FWD_PERSISTENT_FROM in the environment overrides the threshold (tests run the
   // persistent kernel on small shapes with it; 0 = never)
