@@ -1521,7 +1521,9 @@ bool bwd_sm100_supported(const fa_attn_args& a) {
   if (a.batch == 0 || a.seqlen_q == 0 || a.seqlen_k == 0) return false;
   // No lower bound on the lengths: even where one tile is mostly padding these kernels are ahead of the
   // mma.sync ones (GPU time of the three backward launches, causal: 2 x 16 tokens, 4 heads of 64 28 -> 16 us,
-  // 2 x 128 42 -> 17, 16 x 64 of 16 heads 32 -> 26, 16 x 200 of 16 heads of 128 295 -> 68 us).
+  // 2 x 128 42 -> 17, 16 x 64 of 16 heads 32 -> 26, 16 x 200 of 16 heads of 128 295 -> 68 us).  With a soft cap they
+  // start where the tanh of these kernels, good to 2^-11 of the capped score, always set the precision.
+  if (a.impl == FA_IMPL_AUTO && a.softcap > 0.f && (a.seqlen_k < 256 || a.seqlen_q < 128)) return false;
   return true;
 }
 

@@ -265,7 +265,8 @@ template <bool kCap> __device__ __forceinline__ FeatK feat_k(const ScoreCfg& c, 
   k.kb = make_float2(kb, kb);
   return k;
 }
-template <bool kCap, bool kAbs>
+// kExact: the tanh of the mma.sync kernels (absolute error 1e-7), for the calls whose precision they set.
+template <bool kCap, bool kAbs, bool kExact = false>
 __device__ __forceinline__ float2 score_unit_feat2(const FeatK& k, float2 dot2, float2 d2) {
   if (kAbs) {
     d2.x = fabsf(d2.x);
@@ -273,6 +274,7 @@ __device__ __forceinline__ float2 score_unit_feat2(const FeatK& k, float2 dot2, 
   }
   const float2 y = f2fma(k.ka, d2, f2mul(dot2, k.kb));
   if (!kCap) return y;
+  if (kExact) return make_float2(fast_tanh(y.x), fast_tanh(y.y));
   return make_float2(tanh_approx(y.x), tanh_approx(y.y));
 }
 // score in the log2 domain = score_unit_feat() * soft_cap_factor()

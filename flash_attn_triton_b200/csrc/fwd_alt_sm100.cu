@@ -449,7 +449,7 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             for (int cc = 0; cc < 4; ++cc) {
 #pragma unroll
               for (int i = 0; i < 32; i += 2) {
-                float2 v = score_unit_feat2<kCap, kAbs>(
+                float2 v = score_unit_feat2<kCap, kAbs, true>(
                     fk, make_float2(__uint_as_float(r[cc][i]), __uint_as_float(r[cc][i + 1])), d2);
                 if (kMask) {
                   v.x = col_visible(cm, cc * 32 + i) ? v.x : -INFINITY;

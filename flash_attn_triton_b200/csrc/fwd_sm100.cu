@@ -776,6 +776,9 @@ bool fwd_sm100_supported(const fa_attn_args& a) {
   // 7.0 us; 16 x 100 of 32 heads 20 against 24); from a full tile on it is behind (16 x 128, 16 heads of 128:
   // 20 against 16; 2 x 255, 4 heads of 128: 13.7 against 10.2; 16 x 200 of 16 heads 46 against 21).
   if (a.impl == FA_IMPL_AUTO && a.seqlen_k < 128) return false;
+  // ... and up to 256 keys a soft cap stays with its tanh: the one of the two-tile kernel is good to 2^-11 of the capped
+  // score.  (At head_dim 256 the one-tile kernel has the same tanh.)
+  if (a.impl == FA_IMPL_AUTO && a.softcap > 0.f && a.seqlen_k < 256 && a.head_dim != 256) return false;
   return true;
 }
 
