@@ -21,7 +21,10 @@
 // group waits for the other's exponentials: what a tile needs from the tile before it is only the
 // row maximum that all exponents are taken relative to.  It sits in shared memory (mref), is read and
 // raised in tile order -- only when a row's maximum grows by more than cfg.rescale_at, and the accumulator is then
-// rescaled by the group that raised it -- and each group keeps its own row sums.
+// rescaled by the group that raised it.  The row sum travels with it, one tile late: a group adds the sum of its tile
+// j when it settles tile j + 2, so that nothing waits for it and the sums are added in tile order all the same.  The results
+// are therefore those of the two-tile kernels bit for bit, and which kernel a call takes may depend on its batch:
+// an entry has the same result in any batch.
 //
 // Bound: the tensor pipe needs 2 * head_dim * 8 cycles per tile (128 x 128 scores), the exponentials
 // 1024, and two groups have the load-max-exp-store chain of about 2200 cycles per tile half each.
@@ -74,7 +77,7 @@ struct AShared {
   volatile int abort_flag;
   int last;                // split keys: this CTA merges the pieces
   alignas(16) float mref[kBM];
-  float l[2][kBM];         // row sums of the groups at the end
+  float lrun[kBM];         // row sums, up to the tile before the last one each group has settled
 };
 static_assert(sizeof(AShared) <= 2048, "AShared must fit its reserve");
 
@@ -116,8 +119,9 @@ struct Tile {
 
 }  // namespace
 
+// kPoly > 0: every kPoly-th pair of exponentials of unmasked tiles on the FMA pipe, as in fwd_persist_sm100.cu.
 // kCache: K/V through the page table of a cache, query heads packed into rows, optional key pieces.
-template <typename T, int D, bool kExtras, bool kCache>
+template <typename T, int D, bool kExtras, bool kCache, int kPoly>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -189,6 +193,7 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   }
   const int tq_min = w.pos0 + (w.m0 >> w.pack_log2);
   const int tq_max = w.pos0 + ((min(w.m0 + kBM, w.rows) - 1) >> w.pack_log2);
+  const int tq_end = w.pos0 + ((w.m0 + kBM - 1) >> w.pack_log2);     // of the tile's last row, existing or not
   {
     int klo, khi;
     visible_key_range(cfg, tq_min, tq_max, w.k_len, klo, khi);
@@ -402,7 +407,8 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     float slope = 0.f;
     if (kExtras && cfg.has_alibi)
       slope = p.alibi_slopes[w.b * p.heads_q + w.h + (row & ((1 << w.pack_log2) - 1))];
-    float m_mine = -INFINITY, l = 0.f;               // this group's row sum and the maximum it is relative to
+    // of this group's latest tile: the factor its maximum asked of what came before, and its row sum
+    float alpha = 1.f, sum = 0.f;
     bool ok = true;
     const bool zero_tail = kCache || packed;         // rows past k_len of the last V tile are not ours
 
@@ -413,7 +419,7 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       const int k0 = (w.n_hi - 1 - j) * kBN;
       bool masked = (k0 + kBN > w.k_len);
       if (cfg.causal) masked |= (k0 + kBN - 1 > tq_min);
-      if (cfg.wl >= 0) masked |= (k0 < tq_max - cfg.wl);
+      if (cfg.wl >= 0) masked |= (k0 < tq_end - cfg.wl);
       if (cfg.wr >= 0) masked |= (k0 + kBN - 1 > tq_min + cfg.wr);
 
       ok = wait_bar(&sh->s_full[buf], par, sh, 31 + x);
@@ -536,12 +542,15 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (j == 0) {
         m_use = mx;
         sh->mref[row_in_tile] = mx;
+        sh->lrun[row_in_tile] = 0.f;
       } else {
         ok = wait_bar(&sh->decided[x ^ 1], ((j - 1) >> 1) & 1, sh, 33 + x);
         if (!ok) break;
         const float m_old = sh->mref[row_in_tile];
+        if (j >= 2) sh->lrun[row_in_tile] = __fadd_rn(__fmul_rn(sh->lrun[row_in_tile], alpha), sum);
         const bool need = mx > m_old + cfg.rescale_at;
         m_use = need ? mx : m_old;
+        alpha = 1.f;
         if (__any_sync(0xffffffffu, need)) {
           // The accumulator may be touched once P V of the tile before is finished: the one of this
           // tile cannot start before P is written below.  (Score buffers come round in order, so the
@@ -550,7 +559,7 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           ok = wait_bar(&sh->o_done[pb], ((j - 1) / NB) & 1, sh, 35 + x);
           if (!ok) break;
           tc_fence_after();
-          const float alpha = need ? exp2f(m_old - mx) : 1.f;     // m_old = -inf -> 0
+          if (need) alpha = exp2f(m_old - mx);                    // m_old = -inf -> 0
           if (need) sh->mref[row_in_tile] = mx;
 #pragma unroll
           for (int cc = 0; cc < D / 32; ++cc) {
@@ -566,14 +575,38 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
       }
       mbar_arrive(smem_u32(&sh->decided[x]));
-      if (m_use != m_mine) {
-        l *= exp2f(m_mine - m_use);                      // from -inf: l is 0
-        m_mine = m_use;
-      }
       const float m_safe = (m_use == -INFINITY) ? 0.f : m_use;
 
       // ---- P = exp2(s - m), row sum, P -> TMEM in place over S ----------------------------
-      {
+      if (kPoly > 0 && !prescaled) {
+        // the scores once more from tensor memory, a quarter at a time: the polynomial wants the registers
+        const float2 mul2 = make_float2(mul, mul), nm2 = make_float2(-m_safe, -m_safe);
+        float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        uint32_t ra[32], rb[32];
+        tmem_ld32(tS, ra);
+#pragma unroll
+        for (int cc = 0; cc < 4; ++cc) {
+          uint32_t (&cur)[32] = (cc & 1) ? rb : ra;
+          uint32_t (&nxt)[32] = (cc & 1) ? ra : rb;
+          tmem_wait_ld();
+          if (cc < 3) tmem_ld32(tS + (cc + 1) * 32, nxt);
+          uint32_t pk[16];
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) {
+            const float2 a = f2fma(make_float2(__uint_as_float(cur[i]), __uint_as_float(cur[i + 1])), mul2, nm2);
+            const float2 pe = ex2_pair<kPoly>(a, i >> 1);
+            pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
+            acc2[(i >> 1) & 1] = f2add(acc2[(i >> 1) & 1], pe);
+          }
+          tmem_st16(tS + cc * 16, pk);
+          if (kPvSplit && cc == 1) {
+            tmem_wait_st();
+            tc_fence_before();
+            mbar_arrive(smem_u32(&sh->p_half[buf]));
+          }
+        }
+        sum = (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
+      } else {
         const float2 mul2 = make_float2(mul, mul), nm2 = make_float2(-m_safe, -m_safe);
         float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
@@ -593,7 +626,7 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             mbar_arrive(smem_u32(&sh->p_half[buf]));
           }
         }
-        l += (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
+        sum = (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
       }
       tmem_wait_st();
       tc_fence_before();
@@ -603,11 +636,18 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // ---- epilogue: both groups, half of the columns each ----------------------------------
     asm volatile("bar.sync 1, 256;\n" ::: "memory");     // every decision is made
     const float m_fin = nt > 0 ? sh->mref[row_in_tile] : -INFINITY;
-    sh->l[x][row_in_tile] = l == 0.f ? 0.f : l * exp2f(m_mine - m_fin);
+    // the row sum: the tile before the last, then the last
+    const bool last_group = ((nt - 1) & 1) == x;
+    if (nt > 0 && !last_group) sh->lrun[row_in_tile] = __fadd_rn(__fmul_rn(sh->lrun[row_in_tile], alpha), sum);
     if (ok && nt > 0) ok = wait_bar(&sh->o_done[(nt - 1) % NB], ((nt - 1) / NB) & 1, sh, 37 + x);
     const bool failed = any_of_256(!ok || sh->abort_flag != 0);
     tc_fence_after();
-    const float l_all = sh->l[0][row_in_tile] + sh->l[1][row_in_tile];
+    float l_all = 0.f;
+    if (nt > 0) {
+      if (last_group) sh->lrun[row_in_tile] = __fadd_rn(__fmul_rn(sh->lrun[row_in_tile], alpha), sum);
+      asm volatile("bar.sync 1, 256;\n" ::: "memory");
+      l_all = sh->lrun[row_in_tile];
+    }
     if (!failed) {
       const float inv = l_all > 0.f ? 1.f / l_all : 0.f;
       const float lse = l_all > 0.f ? m_fin + log2f(l_all) : -INFINITY;
@@ -768,9 +808,9 @@ static int launch_alt(K kern, int smem, dim3 grid, cudaStream_t st, const CUtens
   return check_launch("fwd_alt_sm100");
 }
 
-// Dense or packed forward.  With ALiBi or a soft cap only head_dim 256 comes here (one_tile_is_faster()).
+// Dense or packed forward; poly: exponentials as the persistent kernel would take them.  With ALiBi or a soft cap only head_dim 256 comes here (one_tile_is_faster()).
 template <typename T, int D>
-static int launch_rows(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
+static int launch_rows(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStream_t st) {
   const bool packed = a.cu_seqlens_q != nullptr;
   const int64_t q_rows = packed ? a.total_q : a.seqlen_q, k_rows = packed ? a.total_k : a.seqlen_k;
   const int64_t batch = packed ? 1 : a.batch;
@@ -786,17 +826,20 @@ static int launch_rows(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t 
   }
   const dim3 grid((a.seqlen_q + kBM - 1) / kBM, a.heads_q, a.batch);
   const CacheGeo geo = {};
-  if constexpr (D == 256)
+  if constexpr (D == 256) {
     if (cfg.has_alibi || cfg.softcap > 0.f)
-      return launch_alt(fwd_alt_sm100_kernel<T, D, true, false>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
-  return launch_alt(fwd_alt_sm100_kernel<T, D, false, false>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+      return launch_alt(fwd_alt_sm100_kernel<T, D, true, false, 0>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+  } else if (poly) {
+    return launch_alt(fwd_alt_sm100_kernel<T, D, false, false, 4>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+  }
+  return launch_alt(fwd_alt_sm100_kernel<T, D, false, false, 0>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
 }
 
-int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
+int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStream_t st) {
   const bool bf = a.dtype == FA_BF16;
-  if (a.head_dim == 64) return bf ? launch_rows<__nv_bfloat16, 64>(a, cfg, st) : launch_rows<__half, 64>(a, cfg, st);
-  if (a.head_dim == 128) return bf ? launch_rows<__nv_bfloat16, 128>(a, cfg, st) : launch_rows<__half, 128>(a, cfg, st);
-  return bf ? launch_rows<__nv_bfloat16, 256>(a, cfg, st) : launch_rows<__half, 256>(a, cfg, st);
+  if (a.head_dim == 64) return bf ? launch_rows<__nv_bfloat16, 64>(a, cfg, poly, st) : launch_rows<__half, 64>(a, cfg, poly, st);
+  if (a.head_dim == 128) return bf ? launch_rows<__nv_bfloat16, 128>(a, cfg, poly, st) : launch_rows<__half, 128>(a, cfg, poly, st);
+  return bf ? launch_rows<__nv_bfloat16, 256>(a, cfg, poly, st) : launch_rows<__half, 256>(a, cfg, poly, st);
 }
 
 template <typename T, int D>
@@ -827,8 +870,8 @@ static int launch_cache(const fa_decode_args& d, const void* q, const int64_t* q
   const int mtiles = (d.seqlen_q * pack + kBM - 1) / kBM;
   const dim3 grid((unsigned)d.batch * (d.heads_q / pack) * mtiles * geo.parts);
   if (cfg.has_alibi)
-    return launch_alt(fwd_alt_sm100_kernel<T, D, true, true>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
-  return launch_alt(fwd_alt_sm100_kernel<T, D, false, true>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+    return launch_alt(fwd_alt_sm100_kernel<T, D, true, true, 0>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+  return launch_alt(fwd_alt_sm100_kernel<T, D, false, true, 0>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
 }
 
 int cache_attention_sm100(const fa_decode_args& d, const void* q, const int64_t* q_stride, const CacheGeo& geo,

@@ -830,7 +830,8 @@ int fwd_persist_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t s
 int fwd_persist_sm100_status();
 int fwd_persist_sm100_clear_status();
 
-int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st);
+bool fwd_poly_pays(const fa_attn_args& a, const ScoreCfg& cfg);
+int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStream_t st);
 
 // Plain dense problems for the one-tile kernel (fwd_alt_sm100.cu): a tile of its costs 1.8 k cycles of an SM
 // where a pair of tiles costs the others 4.3 k, but it has twice as many CTAs to start, drain and balance.
@@ -843,26 +844,34 @@ int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st);
 //   no mask, D = 128   -1 to -24 % while rounds <= key tiles / 3, +2 to +9 % beyond, -1 to -26 % from 6144 keys up
 //   no mask, D = 64    within +-7 % (the persistent kernel has part of its exponentials on the FMA pipe), -1 to -12 %
 //                      from 12288 keys up
-static bool one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
-  if (cfg.keep != nullptr || a.cu_seqlens_q != nullptr || cfg.has_alibi || cfg.softcap > 0.f) return false;
+// A choice by the number of CTAs must not show in the results (a batch may be computed in parts): there the kernel
+// takes its exponentials as the one it stands in for (`poly`).
+enum OneTile { kNotOneTile, kOneTileByLength, kOneTileByCtas };
+static OneTile one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
+  if (cfg.keep != nullptr || a.cu_seqlens_q != nullptr || cfg.has_alibi || cfg.softcap > 0.f) return kNotOneTile;
   const int64_t ctas = (int64_t)((a.seqlen_q + kBM - 1) / kBM) * a.heads_q * a.batch;
   const int64_t sms = sm_count(a.device), nk = (a.seqlen_k + kBN - 1) / kBN;
-  if (ctas <= sms) return true;
-  if (cfg.wl >= 0 || cfg.wr >= 0 || nk < 16) return false;
-  if (cfg.causal) return nk >= 96 || 2 * ctas <= nk * sms;
-  return nk >= 96 || (a.head_dim == 128 && (nk >= 48 || 3 * ctas <= nk * sms));
+  const bool window = cfg.wl >= 0 || cfg.wr >= 0;
+  if (!window && (nk >= 96 || (!cfg.causal && a.head_dim == 128 && nk >= 48))) return kOneTileByLength;
+  if (ctas <= sms) return kOneTileByCtas;
+  if (window || nk < 16) return kNotOneTile;
+  if (cfg.causal) return 2 * ctas <= nk * sms ? kOneTileByCtas : kNotOneTile;
+  return a.head_dim == 128 && 3 * ctas <= nk * sms ? kOneTileByCtas : kNotOneTile;
 }
 
 int fwd_sm100(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
   ScoreCfg cfg = plain;
   if (a.head_dim == 256 || a.seqlen_k < 256 || cfg.keep != nullptr) cfg.rescale_at = 0.f;
-  if (a.head_dim == 256) return fwd_alt_sm100(a, cfg, st);
+  if (a.head_dim == 256) return fwd_alt_sm100(a, cfg, false, st);
   // FA_B200_FWD_PERSISTENT_FROM in the environment overrides the threshold (tests run the
   // persistent kernel on small shapes with it; 0 = never)
   int from = FA_FWD_PERSISTENT_FROM;
   const char* e = getenv("FA_B200_FWD_PERSISTENT_FROM");
-  if (e != nullptr) from = atoi(e);
-  else if (one_tile_is_faster(a, cfg)) return fwd_alt_sm100(a, cfg, st);
+  if (e != nullptr) {
+    from = atoi(e);
+  } else if (const OneTile why = one_tile_is_faster(a, cfg)) {
+    return fwd_alt_sm100(a, cfg, why == kOneTileByCtas && from > 0 && a.seqlen_k >= from && fwd_poly_pays(a, cfg), st);
+  }
   // with dropout bits this kernel takes every length: the persistent one has no such variant
   if (cfg.keep == nullptr && from > 0 && a.seqlen_k >= from) return fwd_persist_sm100(a, cfg, st);
   // Row extents of the tensor maps.  Dense: the sequence length.  Packed: the caller does

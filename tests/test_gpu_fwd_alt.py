@@ -149,3 +149,34 @@ def test_dense_routes(monkeypatch, B, Sq, Sk, Hq, Hkv, causal, window, D, dtype)
         assert maxdiff(o, ro) <= util.tols(dtype)[0], route
         assert maxdiff(lse * util.LN2, rl) <= util.tols(dtype)[0], route
     assert N.lib().fa_device_wait_status(0) == 0
+
+
+@pytest.mark.parametrize("B,H,Sq,Sk,D,causal,window", [
+    (16, 16, 2048, 2048, 128, True, None),     # one entry: one-tile kernel, all: persistent
+    (16, 16, 4096, 4096, 64, True, None),
+    (16, 16, 2048, 2048, 128, False, None),    # ... with part of the exponentials on the FMA pipe
+    (16, 16, 2049, 2175, 64, False, None),
+    (20, 16, 2048, 1930, 128, False, None),    # as many key tiles, but below the persistent kernel's first length
+    (24, 8, 8192, 8192, 128, True, None),
+    (16, 16, 1024, 1024, 64, False, None),     # one entry: one-tile kernel, all: two-tile
+    (32, 16, 300, 500, 128, False, None),
+    (32, 16, 384, 384, 64, True, None),
+    (32, 16, 700, 700, 128, False, (200, 60)),
+    (16, 16, 2500, 2500, 64, False, (300, -1)),
+])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_an_entry_has_the_same_result_in_any_batch(B, H, Sq, Sk, D, causal, window, dtype):
+    """The kernel depends on the number of tiles of the call; the results (and the LSE) do not."""
+    from flash_attn_triton_b200 import _native as N, _ops
+    g = torch.Generator(DEV).manual_seed(Sk)
+    q, k, v = (2 * torch.randn(B, s, H, D, device=DEV, dtype=dtype, generator=g) for s in (Sq, Sk, Sk))
+    wl, wr = window or (-1, -1)
+
+    def run(n):
+        o, lse, _ = _ops.dense_forward(q[:n], k[:n], v[:n], D ** -0.5, causal, wl, wr, 0.0, None, 0, N.IMPL_AUTO, "bshd", True)
+        return o, lse
+
+    whole = run(B)
+    for n in (1, 2):
+        for a, b in zip(run(n), whole):
+            assert torch.equal(a, b[:n])
