@@ -414,7 +414,7 @@ int fa_decode_paged_checked(const fa_decode_args* a, uint32_t* failed, void* str
 }
 
 int32_t fa_decode_counters(const fa_decode_args* a) {
-  if (a == nullptr || a->heads_kv <= 0 || a->heads_q <= 0) return 0;
+  if (a == nullptr || a->heads_kv <= 0 || a->heads_q <= 0 || a->batch <= 0 || a->seqlen_q <= 0) return 0;
   return decode_num_counters(*a);
 }
 

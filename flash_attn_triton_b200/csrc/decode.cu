@@ -163,9 +163,18 @@ __device__ __forceinline__ int64_t cache_row_offset(const fa_decode_args& p, int
 struct SeqTiles {
   int len_old, len, lo, nt;
 };
+// Rows a sequence can hold behind its left padding: lengths are taken up to here and new tokens stored up to here, so
+// that a call whose values are not checked stays inside its rows of the cache and of the table.
+__host__ __device__ __forceinline__ int cache_capacity(const fa_decode_args& p) {
+  const int64_t cap = p.block_table ? (int64_t)p.block_table_stride * p.page_size : p.page_size;
+  return (int)(cap < (1 << 30) ? cap : (1 << 30));
+}
+__device__ __forceinline__ int seq_capacity(const fa_decode_args& p, int b) {
+  return cache_capacity(p) - (p.cache_leftpad ? max(0, p.cache_leftpad[b]) : 0);
+}
 __device__ __forceinline__ SeqTiles seq_tiles(const fa_decode_args& p, const ScoreCfg& cfg, int max_tiles, int b) {
   SeqTiles s;
-  s.len_old = max(0, min(p.cache_seqlens[b], max_tiles * kTile));   // in bounds also with the value checks off
+  s.len_old = max(0, min(p.cache_seqlens[b], seq_capacity(p, b)));
   s.len = s.len_old + (p.k_new ? p.seqlen_new : 0);
   const int first = cfg.wl >= 0 ? min(max(0, s.len - p.seqlen_q - cfg.wl), s.len_old) : 0;
   s.lo = first / kTile;
@@ -336,7 +345,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
   // ---- loading --------------------------------------------------------------------------
   const int lc = (lane % CPR) * 8, lr = lane / CPR;         // this lane's 16-byte column and first row
   const bool one_page = p.block_table == nullptr || geo.page_shift >= 4;   // a warp's 16 keys lie inside one page
-  const int pad = p.cache_leftpad ? p.cache_leftpad[b] : 0;
+  const int pad = p.cache_leftpad ? max(0, p.cache_leftpad[b]) : 0;
   const int* table = p.block_table ? p.block_table + (int64_t)b * p.block_table_stride : nullptr;
   int page = table ? 0 : (p.cache_batch_idx ? p.cache_batch_idx[b] : b);
   int ld = tile0;                                           // next tile to load
@@ -488,7 +497,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
         const T vv = vn[d];
         tK[(key - keyw) * P + d] = kv;
         tV[(key - keyw) * P + d] = vv;
-        if (rg == 0) {
+        if (rg == 0 && pos < cache_capacity(p)) {
           reinterpret_cast<T*>(p.k_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.kc_stride) +
                                           (int64_t)hk * p.kc_stride[2] + d] = kv;
           reinterpret_cast<T*>(p.v_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.vc_stride) +
@@ -767,7 +776,8 @@ __global__ void __launch_bounds__(256) cache_append_kernel(const fa_decode_args 
   const int d = (int)(i % cpr) * 8, h = (int)(i / cpr % p.heads_kv);
   const int64_t bt = i / ((int64_t)cpr * p.heads_kv);
   const int tok = (int)(bt % n_new), b = (int)(bt / n_new);
-  const int pos = p.cache_seqlens[b] + tok + (p.cache_leftpad ? p.cache_leftpad[b] : 0);
+  const int pos = max(0, min(p.cache_seqlens[b], seq_capacity(p, b))) + tok + (p.cache_leftpad ? max(0, p.cache_leftpad[b]) : 0);
+  if (pos >= cache_capacity(p)) return;
   if (val) {
     const T* x = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + h * p.vn_stride[2];
     T* dst = reinterpret_cast<T*>(p.v_cache) + cache_row_offset(p, b, pos, page_shift, p.vc_stride) + h * p.vc_stride[2];

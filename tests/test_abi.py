@@ -147,3 +147,12 @@ def test_checked_decode_result_has_room_of_its_own(built):
     for tokens, table, word in ((1, 256, False), (1, 257, True), (64, 8, True), (64, 300, True)):
         plain, checked = sizes(tokens, table)
         assert (checked >= plain + 4) if word else (checked == plain), (tokens, table, plain, checked)
+
+
+def test_decode_counters_of_an_empty_call(built):
+    from flash_attn_triton_b200 import _native as N
+    d = N.DecodeArgs()
+    d.heads_q, d.heads_kv, d.head_dim, d.seqlen_q, d.page_size, d.softmax_scale = 8, 2, 128, 64, 8192, 0.1
+    assert N.lib().fa_decode_counters(ctypes.byref(d)) == 0        # batch 0, a chunk of tokens
+    d.batch = 1
+    assert N.lib().fa_decode_counters(ctypes.byref(d)) > 0

@@ -208,3 +208,23 @@ def test_nan_query_gives_nan(tokens, length, splits, D):
     assert out[0, 0, 1].isnan().all()
     out[0, 0, 1] = want[0, 0, 1]
     assert torch.equal(out, want) and not out[2].any()
+
+
+@pytest.mark.parametrize("tokens", [1, 64])
+@pytest.mark.parametrize("padded", [False, True])
+def test_unchecked_lengths_stay_inside_the_cache(tokens, padded):
+    """Value checks off and lengths past the capacity: the rows of the neighbours in the same buffer stay untouched."""
+    B, cap, Hkv, D = 2, 100, 2, 64
+    buf = [torch.randn(B + 2, cap, Hkv, D, device=DEV, dtype=torch.half) for _ in range(2)]
+    kept = [t.clone() for t in buf]
+    q, kn, vn = (torch.randn(B, tokens, h, D, device=DEV, dtype=torch.half) for h in (8, Hkv, Hkv))
+    lens = torch.tensor([cap + 20, cap - 1], dtype=torch.int32, device=DEV)
+    pads = torch.tensor([3, 0], dtype=torch.int32, device=DEV) if padded else None
+    fa().set_validation(False)
+    try:
+        fa().flash_attn_with_kvcache(q, buf[0][1:B + 1], buf[1][1:B + 1], kn, vn, cache_seqlens=lens, cache_leftpad=pads, causal=True)
+    finally:
+        fa().set_validation(True)
+    for t, was, new in zip(buf, kept, (kn, vn)):
+        assert torch.equal(t[0], was[0]) and torch.equal(t[3], was[3]) and torch.equal(t[1], was[1])
+        assert torch.equal(t[2, :cap - 1], was[2, :cap - 1]) and torch.equal(t[2, cap - 1], new[1, 0])
