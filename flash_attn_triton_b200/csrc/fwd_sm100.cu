@@ -978,13 +978,13 @@ int fwd_int8_codes16(const fa_int8_args& a, const void* q16, const void* k16, cu
   return check_launch("fwd_int8_codes16");
 }
 
-// Whole calls against the mma.sync kernel, launches interleaved, with and without the causal mask: from 3e7 (query, key)
-// pairs over all heads on -5 to -49 % (32 heads x 1024 51 -> 41 us, 256 x 4096 2739 -> 1630 us causal, 32 x 8192
-// without a mask 2585 -> 1317 us); below that the two quantiser launches and the fixed cost of a CTA weigh more
-// (8 x 1024: 32 -> 38 us, 256 x 320: 46 -> 58 us).
+// By the length alone: the two kernels round differently, and an entry has the same result in any batch.  Whole calls
+// against the mma.sync kernel, batch * heads from 1 to 256, with and without the causal mask:
+//    512   +32 % (8) to -14 % (256)            1024   +29 % (1), +15 % (8, 40 -> 46 us), -16 to -34 % from 32 on
+//    768   +21 % (1) to -24 % (256)            2048   +17 % (1), +-3 % (8), -20 to -41 % from 32 on; less above
+// What the small calls lose is the 6 to 10 us of the two quantiser launches and the fixed cost of a CTA.
 bool int8_codes16_supported(const fa_int8_args& a) {
-  if (a.head_dim != 64 || a.softmax_scale < 0.f || a.impl != FA_IMPL_AUTO || a.seqlen < 256) return false;
-  return (int64_t)a.batch * a.heads * a.seqlen * a.seqlen >= 30000000;
+  return a.head_dim == 64 && a.softmax_scale >= 0.f && a.impl == FA_IMPL_AUTO && a.seqlen >= 1024;
 }
 
 int fwd_sm100_status() {

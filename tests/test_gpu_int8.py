@@ -175,3 +175,14 @@ def test_head_dim_64_on_tcgen05(B, H, S, lk, causal):
     out = fa.attention_int8(q.to(DEV), k.to(DEV), v.to(DEV), causal=causal, **kw)
     ro, _, _, _ = orc.attention_int8_ref(q, k, v, causal=causal, **kw)
     assert maxdiff(out[:, :, :lk], ro[:, :, :lk]) <= util.FWD_TOL
+
+
+@pytest.mark.parametrize("S", [960, 1024, 2048])
+@pytest.mark.parametrize("D", [64, 128])
+def test_an_entry_has_the_same_result_in_any_batch(S, D):
+    import flash_attn_triton_b200 as fa
+    g = torch.Generator(DEV).manual_seed(S)
+    q, k, v = (torch.randn(6, 16, S, D, device=DEV, dtype=torch.half, generator=g) for _ in range(3))
+    whole = fa.attention_int8(q, k, v, causal=True)
+    assert torch.equal(fa.attention_int8(q[:1], k[:1], v[:1], causal=True), whole[:1])
+    assert torch.equal(fa.attention_int8(*(t[:1, :2].contiguous() for t in (q, k, v)), causal=True), whole[:1, :2])
