@@ -178,17 +178,15 @@ def dense_backward(q, k, v, o, lse, dout, scale, causal, wl, wr, softcap, alibi,
                              f.row_stride, None, None)
 
 
-def varlen_attention(packing, dim, tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
-                     feat=None, want_lse=False):
-    """Packed sequences: tensors = (q (Tq,Hq,D), k, v (Tk,Hkv,D)), or packed as in dense_attention_packed; int32
-    cu_seqlens on the device; differentiable."""
+def varlen_attention(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl, feat=None,
+                     want_lse=False):
+    """Packed sequences: q (Tq,Hq,D), k/v (Tk,Hkv,D), int32 cu_seqlens on the device; differentiable."""
     f = feat or _NO_FEATURES
     tail = (impl, f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse)
     if _tracing() is not None:
-        return _TracedCall.apply(lambda cu_q, cu_k, alibi, *tensors: N.host().varlen(
-            packing, dim, *tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail),
-            cu_q, cu_k, alibi, *tensors)
-    return N.host().varlen(packing, dim, *tensors, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail)
+        return _TracedCall.apply(lambda q, k, v, cu_q, cu_k, alibi: N.host().varlen(
+            q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail), q, k, v, cu_q, cu_k, alibi)
+    return N.host().varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail)
 
 
 def varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
@@ -196,8 +194,7 @@ def varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, sof
     """(o, base-2 LSE (Hq, Tq) or None, the tensors as handed to the kernels), no autograd."""
     q, k, v = _prep(q), _prep(k), _prep(v)
     with torch.no_grad():
-        r = varlen_attention(_SEPARATE, -1, (q, k, v), cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi,
-                             impl, feat, want_lse)
+        r = varlen_attention(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl, feat, want_lse)
     o, lse = r if want_lse else (r, None)
     return o, lse, (q, k, v)
 

@@ -81,6 +81,6 @@ def attention_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seql
         feat = _ops.Features(dropout_p=dropout_p, seed=int(dropout_seed), row_stride=int(max_seqlen_k))
     cu_q = cu_seqlens_q.to(dtype=torch.int32).contiguous()
     cu_k = cu_seqlens_k.to(dtype=torch.int32).contiguous()
-    return _ops.varlen_attention(0, -1, (q, k, v), cu_q, cu_k, int(max_seqlen_q), int(max_seqlen_k), sm_scale,
+    return _ops.varlen_attention(q, k, v, cu_q, cu_k, int(max_seqlen_q), int(max_seqlen_k), sm_scale,
                                       bool(causal), int(window_left), int(window_right), float(softcap), alibi,
                                       N.IMPL_AUTO, feat)

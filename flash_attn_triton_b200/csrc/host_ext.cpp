@@ -473,13 +473,14 @@ PyObject* py_dense(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// varlen(packing, packed_dim, inputs.., cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
+// varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
 //        dropout_p, seed, row_stride, used_q, used_k, want_lse) -> out | (out, lse2)
 PyObject* py_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a{args, n};
   Params c;
-  variable_list in = input_list(a, c);
+  variable_list in;
+  for (int i = 0; i < 3; ++i) in.push_back(a.tensor());
   c.layout = kTHD;
   c.cu_q = a.tensor();
   c.cu_k = a.tensor();

@@ -516,10 +516,10 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
     args = (cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), softmax_scale, causal,
             window_size[0], window_size[1], softcap, alibi)
     if return_attn_probs:
-        out, lse2 = _ops.varlen_attention(0, -1, (q, k, v), *args, N.IMPL_AUTO, feat, True)
+        out, lse2 = _ops.varlen_attention(q, k, v, *args, N.IMPL_AUTO, feat, True)
         probs, lse = _ops.varlen_probs(q.detach(), k.detach(), v.detach(), lse2, *args, feat)
     else:
-        out = _ops.varlen_attention(0, -1, (q, k, v), *args, N.IMPL_AUTO, feat)
+        out = _ops.varlen_attention(q, k, v, *args, N.IMPL_AUTO, feat)
     if used_q is not None and not compacted:
         # the reference returns only the used rows, packed (flash_attn_interface.py:552-566); the one
         # host read of the lengths sizes that result
