@@ -168,6 +168,9 @@ def host():
         except ImportError as e:
             raise RuntimeError("the host extension is missing or does not load: build it with "
                                f"`python -m flash_attn_triton_b200.build` ({e})") from e
+        if _fa_host.built_for != f"torch=={torch.__version__}":
+            raise RuntimeError(f"the host extension was built for {_fa_host.built_for}, this is {torch.__version__}: build it "
+                               "again with `python -m flash_attn_triton_b200.build`")
         _fa_host.init({name: C.cast(getattr(l, name), C.c_void_p).value for name in EXPORTS}, check)
         _host = _fa_host
     return _host

@@ -54,17 +54,20 @@ def _compile(src, defs, force, verbose):
 
 
 def build_host(force: bool = False) -> str:
-    """The host extension: plain C++ against PyTorch's headers, no device code."""
+    """The host extension: plain C++ against PyTorch's headers, no device code.  It names the PyTorch it was compiled
+    against and is rebuilt for another one."""
     import sysconfig
 
     import torch
     src, out = os.path.join(CSRC, "host_ext.cpp"), os.path.join(HERE, "_fa_host.so")
     header = os.path.join(os.path.dirname(HERE), "include", "fa_b200.h")
     if not force and os.path.exists(out) and os.path.getmtime(out) > max(os.path.getmtime(f) for f in (src, header, __file__)):
-        return out
+        with open(out, "rb") as f:
+            if f"torch=={torch.__version__}\0".encode() in f.read():
+                return out
     t = os.path.dirname(os.path.abspath(torch.__file__))
     cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f'-DFA_TORCH="torch=={torch.__version__}"',
            *(f"-I{d}" for d in (t + "/include", t + "/include/torch/csrc/api/include", "/usr/local/cuda/include",
                                 sysconfig.get_paths()["include"])),
            src, "-o", out, f"-L{t}/lib", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda",

@@ -756,4 +756,8 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_fa_host", "host path of the att
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__fa_host(void) { return PyModule_Create(&g_module); }
+PyMODINIT_FUNC PyInit__fa_host(void) {
+  PyObject* m = PyModule_Create(&g_module);
+  if (m != nullptr && PyModule_AddStringConstant(m, "built_for", FA_TORCH) != 0) Py_CLEAR(m);
+  return m;
+}

@@ -69,3 +69,23 @@ def test_missing_library_fails_loudly(monkeypatch):
     monkeypatch.setattr(N, "LIB_PATH", "/nonexistent/libfa_b200.so")
     with pytest.raises(RuntimeError, match="no CPU fallback"):
         N.lib()
+
+
+def test_host_extension_of_another_pytorch_is_rebuilt(monkeypatch):
+    """The extension names the PyTorch it was compiled against: the build makes it again for another one, and loading it
+    under another one fails loudly."""
+    import subprocess
+
+    from flash_attn_triton_b200 import _native as N, build as B
+    B.build_host()
+    made = []
+    monkeypatch.setattr(subprocess, "run", lambda cmd, **kw: made.append(cmd) or subprocess.CompletedProcess(cmd, 0, "", ""))
+    B.build_host()
+    assert not made
+    N.host()
+    monkeypatch.setattr(N, "_host", None)
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    B.build_host()
+    assert len(made) == 1
+    with pytest.raises(RuntimeError, match="host extension was built for"):
+        N.host()
