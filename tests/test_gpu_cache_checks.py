@@ -82,3 +82,81 @@ def test_without_room_for_the_result(tokens, page, lens):
     assert failed.value == 1                    # FA_CHECK_PAGES
     torch.cuda.synchronize()
     assert not out.any()
+
+
+def decode_call(stream_no, tokens=1):
+    """A call whose sequences are cut into pieces (the merge counters are per stream), and what it gives alone."""
+    import flash_attn_triton_b200 as fa
+    p = problem(tokens, 64, [3000, 700, 4100], seed=stream_no)
+    return p, fa.flash_attn_with_kvcache(**p)
+
+
+def test_more_streams_than_counter_buffers():
+    """Every stream has merge counters of its own; the 33rd takes the place of the first."""
+    import flash_attn_triton_b200 as fa
+    calls = [decode_call(i) for i in range(3)]
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1) for _ in range(32)]      # 32 streams of each priority exist
+    got = []
+    torch.cuda.synchronize()
+    for again in range(2):
+        for i, s in enumerate(streams):
+            with torch.cuda.stream(s):
+                got.append((i % 3, fa.flash_attn_with_kvcache(**calls[i % 3][0])))
+    torch.cuda.synchronize()
+    for i, out in got:
+        assert torch.equal(out, calls[i][1])
+
+
+@pytest.mark.parametrize("tokens", [1, 40])
+def test_threads_with_a_stream_each(tokens):
+    import threading
+
+    import flash_attn_triton_b200 as fa
+    calls = [decode_call(i, tokens) for i in range(4)]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def run(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                if not torch.equal(fa.flash_attn_with_kvcache(**calls[i][0]), calls[i][1]):
+                    wrong.append(i)
+
+    threads = [threading.Thread(target=run, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+
+
+@pytest.mark.parametrize("tokens", [1, 40])
+def test_captured_call_replays(tokens):
+    """Value checks off: the call goes into a CUDA graph, with merge counters of its own that the graph sets to zero."""
+    import flash_attn_triton_b200 as fa
+    (p, want), (other, want_other) = decode_call(0, tokens), decode_call(1, tokens)
+    fa.set_validation(False)
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = fa.flash_attn_with_kvcache(**p)
+        for _ in range(3):
+            out.zero_()
+            graph.replay()
+            assert torch.equal(out, want)
+        for name in ("q", "k", "v", "k_cache", "v_cache", "cache_seqlens", "block_table"):
+            p[name].copy_(other[name])
+        graph.replay()
+        assert torch.equal(out, want_other)
+    finally:
+        fa.set_validation(True)
+
+
+def test_checked_call_under_capture_is_refused():
+    import flash_attn_triton_b200 as fa
+    p, want = decode_call(0)
+    with pytest.raises(RuntimeError, match="captured"):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            fa.flash_attn_with_kvcache(**p)
+    torch.cuda.synchronize()
+    assert torch.equal(fa.flash_attn_with_kvcache(**p), want)
