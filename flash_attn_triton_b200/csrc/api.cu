@@ -201,7 +201,8 @@ static ScoreCfg cfg_of(const fa_attn_args* a) {
   return c;
 }
 
-// Bias and dropout are features of the mma.sync kernels.
+// Bias and dropout drawn per score are features of the mma.sync kernels (dropout as bits: fa_fwd_dropout and its
+// companions).
 static bool needs_mma(const fa_attn_args* a) { return a->attn_bias != nullptr || a->dropout_p > 0.f; }
 
 // Calls whose dropout mask the tcgen05 kernels read as bits: the plain dense variants of both kernels.
