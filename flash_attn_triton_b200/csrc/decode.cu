@@ -1028,22 +1028,23 @@ namespace {
 struct CheckSlots {
   std::mutex mu;
   int free_list[kCheckSlots], nfree = 0;
-  int state = 0;                       // 0 not tried, 1 mapped, -1 unavailable
+  bool mapped = false;
   // index of a free slot, or -1 (error set)
   int acquire(uint32_t** host_dptr) {
     for (;;) {
       {
         std::lock_guard<std::mutex> lock(mu);
-        if (state == 0) {
-          cudaError_t e = cudaHostRegister(const_cast<uint32_t*>(g_check_host), sizeof(g_check_host),
-                                           cudaHostRegisterPortable | cudaHostRegisterMapped);
-          state = e == cudaSuccess ? 1 : -1;
+        if (!mapped) {
+          // tried again by the next call where it fails (another thread may be capturing a graph right now)
+          const cudaError_t e = cudaHostRegister(const_cast<uint32_t*>(g_check_host), sizeof(g_check_host),
+                                                 cudaHostRegisterPortable | cudaHostRegisterMapped);
+          if (e != cudaSuccess) {
+            cudaGetLastError();
+            set_error("decode: no mapped host memory for the value checks: %s", cudaGetErrorString(e));
+            return -1;
+          }
+          mapped = true;
           for (int i = 0; i < kCheckSlots; ++i) free_list[nfree++] = kCheckSlots - 1 - i;
-          if (e != cudaSuccess) cudaGetLastError();
-        }
-        if (state < 0) {
-          set_error("decode: no mapped host memory for the value checks");
-          return -1;
         }
         if (nfree > 0) {
           const int i = free_list[--nfree];
