@@ -68,7 +68,7 @@ struct ScoreCfg {
   // forward kernels).  8 saves most rescales, but a row's largest probability is then 2^x and is rounded to 16 bits,
   // where relative to its own maximum it is exactly 1: errors against float64 grow by 1 to 10 %.  0 where the
   // mma.sync kernels, which always rescale, set the precision of a call: head_dim 256, fewer than 256 keys, dropout,
-  // KV-cache chunks, INT8 at head_dim 64; decode has the same rule in its own kernel (bf16, 2 x 1999 tokens, head_dim 256: 2.017e-3 both, 2.075e-3 with 8).
+  // INT8 at head_dim 64; decode has the same rule in its own kernel, KV-cache chunks have P in two parts (bf16, 2 x 1999 tokens, head_dim 256: 2.017e-3 both, 2.075e-3 with 8).
   float rescale_at;
 };
 

@@ -15,6 +15,12 @@
 //   warp  9     MMA issuer      : S[j] = Q K_j^T (SS);  O += P_j V_j (A = P_j from tensor memory)
 //   warps 10-11 idle (they complete the warpgroup that gives its registers to the softmax groups)
 //
+// For a KV cache P is held in two 16-bit parts, the second in the other 64 columns of its score buffer, and P V is two
+// products per 16 keys.  The kernel these calls came from had a maximum per warp and 16 keys, and every new maximum is a
+// probability without rounding; with one per 128 keys the outputs were 4 to 8 % further from float64 over chunks of 4 to
+// 600 tokens, with two parts they are 16 to 23 % closer.  Rounding no longer depends on the maximum then, so the
+// accumulator is rescaled past 2^8 only.  Four chunks of 256 tokens against 1024 to 8192: 194 -> 207 us.
+//
 // Tensor memory (512 columns): two score buffers and a 256-column accumulator at head_dim 256, else
 // three score buffers.  P_j overwrites the first 64 columns of its score buffer; Q K^T of the tile that
 // takes the buffer next is issued right after P_j V_j, which reads them, in the in-order pipe.  Neither
@@ -99,6 +105,16 @@ __device__ __forceinline__ bool any_of_256(bool x) {
   return r != 0;
 }
 
+// First of two parts: rounded from a little less, so that the rest is never negative (an infinite value times two parts
+// of one sign stays infinite).
+template <typename T> __device__ __forceinline__ float2 first_part(float2 p);
+template <> __device__ __forceinline__ float2 first_part<__half>(float2 p) {
+  return f2mul(p, make_float2(1.f - 0x1p-11f, 1.f - 0x1p-11f));
+}
+template <> __device__ __forceinline__ float2 first_part<__nv_bfloat16>(float2 p) {
+  return f2mul(p, make_float2(1.f - 0x1p-8f, 1.f - 0x1p-8f));
+}
+
 template <typename T> struct AFmt;
 template <> struct AFmt<__half> { static constexpr int code = 0; };
 template <> struct AFmt<__nv_bfloat16> { static constexpr int code = 1; };
@@ -126,7 +142,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                      const fa_attn_args p, const ScoreCfg cfg, const CacheGeo geo, int* const host_status) {
-  constexpr bool kPvSplit = !kExtras;
+  constexpr bool kPvSplit = !kExtras, kTwoParts = kCache;
   using C = ACfg<D>;
   constexpr int S = C::kStages, NB = C::kSBuf, NU = C::kUnits;
   extern __shared__ unsigned char smem_raw[];
@@ -374,9 +390,12 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int un = 0; un < NU; ++un) {
             const uint64_t dv = make_smem_desc(sKV + st[un] * C::kUnitBytes, kBN * 128, 1024);
 #pragma unroll
-            for (int kk = 0; kk < kBN / 32; ++kk)
+            for (int kk = 0; kk < kBN / 32; ++kk) {
               mma_f16_ts_lp(tmem + C::kOCol + un * C::kUnitCols, a + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv,
                             (j > 0 || kk > 0) ? 1u : 0u, leader);
+              if (kTwoParts)
+                mma_f16_ts_lp(tmem + C::kOCol + un * C::kUnitCols, a + 64 + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv, 1u, leader);
+            }
           }
         }
         wwait(&sh->p_ready[buf], par, 26);
@@ -385,9 +404,12 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         for (int un = 0; un < NU; ++un) {
           const uint64_t dv = make_smem_desc(sKV + st[un] * C::kUnitBytes, kBN * 128, 1024);
 #pragma unroll
-          for (int kk = kPvSplit ? kBN / 32 : 0; kk < kBN / 16; ++kk)
+          for (int kk = kPvSplit ? kBN / 32 : 0; kk < kBN / 16; ++kk) {
             mma_f16_ts_lp(tmem + C::kOCol + un * C::kUnitCols, a + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv,
                           (j > 0 || kk > 0) ? 1u : 0u, leader);
+            if (kTwoParts)
+              mma_f16_ts_lp(tmem + C::kOCol + un * C::kUnitCols, a + 64 + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv, 1u, leader);
+          }
           mma_commit_lp(smem_u32(&sh->kv_empty[st[un]]), leader);
         }
         mma_commit_lp(smem_u32(&sh->o_done[buf]), leader);
@@ -611,15 +633,23 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
-          uint32_t pk[16];
+          uint32_t pk[16], rest[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
             const float2 a = f2fma(make_float2(__uint_as_float(r[cc][i]), __uint_as_float(r[cc][i + 1])), mul2, nm2);
             const float2 pe = make_float2(ex2(a.x), ex2(a.y));
-            pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
             acc2[(i >> 1) & 1] = f2add(acc2[(i >> 1) & 1], pe);
+            if (kTwoParts) {
+              const float2 first = first_part<T>(pe);
+              pk[i >> 1] = Elem<T>::pack(first.x, first.y);
+              const float2 left = f2fma(Elem<T>::unpack(pk[i >> 1]), make_float2(-1.f, -1.f), pe);
+              rest[i >> 1] = Elem<T>::pack(left.x, left.y);
+            } else {
+              pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
+            }
           }
           tmem_st16(tS + cc * 16, pk);
+          if (kTwoParts) tmem_st16(tS + 64 + cc * 16, rest);
           if (kPvSplit && cc == 1) {
             tmem_wait_st();
             tc_fence_before();
@@ -844,9 +874,7 @@ int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStr
 
 template <typename T, int D>
 static int launch_cache(const fa_decode_args& d, const void* q, const int64_t* q_stride, const CacheGeo& geo,
-                        const ScoreCfg& plain, cudaStream_t st) {
-  ScoreCfg cfg = plain;
-  cfg.rescale_at = 0.f;
+                        const ScoreCfg& cfg, cudaStream_t st) {
   fa_attn_args a = {};
   a.dtype = d.dtype;
   a.device = d.device;

@@ -180,3 +180,46 @@ def test_an_entry_has_the_same_result_in_any_batch(B, H, Sq, Sk, D, causal, wind
     for n in (1, 2):
         for a, b in zip(run(n), whole):
             assert torch.equal(a, b[:n])
+
+
+def _exact_chunk(q, k, v, start):
+    """float64 attention of the tokens at start.. over all keys, causal; (tokens, heads, dim) each"""
+    g = q.shape[1] // k.shape[1]
+    k, v = (t.double().repeat_interleave(g, 1) for t in (k, v))
+    s = torch.einsum("ihd,jhd->hij", q.double(), k) / q.shape[-1] ** 0.5
+    i = torch.arange(q.shape[0], device=q.device)[:, None] + start
+    return torch.einsum("hij,jhd->ihd", s.masked_fill(torch.arange(k.shape[0], device=q.device) > i, -torch.inf).softmax(-1), v)
+
+
+@pytest.mark.parametrize("tokens,length,Hq,Hkv,D,size", [(40, 300, 8, 2, 64, 1.0), (100, 3000, 16, 4, 128, 1.0), (100, 3000, 16, 4, 128, 4.0),
+                                                         (20, 900, 8, 8, 256, 1.0), (130, 127, 8, 8, 128, 2.0)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_cache_chunk_is_as_exact_as_decode(tokens, length, Hq, Hkv, D, size, dtype):
+    """Against float64, not above the decode kernel (which an explicit number of pieces takes), whose probabilities are rounded
+    once and relative to finer maxima.  Both round the output; in two parts P adds next to nothing to that."""
+    import flash_attn_triton_b200 as fa
+    g = torch.Generator(DEV).manual_seed(length)
+    mk = lambda *s, f=1.0: (torch.randn(*s, device=DEV, generator=g) * f).to(dtype)
+    q, kc, vc = mk(2, tokens, Hq, D, f=size), mk(2, length + tokens, Hkv, D), mk(2, length + tokens, Hkv, D)
+    lens = torch.full((2,), length + tokens, dtype=torch.int32, device=DEV)
+    err = []
+    for splits in (0, 1):
+        out = fa.flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, causal=True, num_splits=splits)
+        ref = torch.stack([_exact_chunk(q[b], kc[b], vc[b], length) for b in range(2)])
+        err.append(((out.double() - ref).norm() / ref.norm()).item())
+    assert err[0] <= err[1], err
+
+
+def test_cache_chunk_keeps_infinite_values():
+    """An infinite value of a visible key makes its column infinite and no other, not NaN, for every row that sees the key."""
+    import flash_attn_triton_b200 as fa
+    g = torch.Generator(DEV).manual_seed(1)
+    q, kc, vc = (torch.randn(1, n, h, 64, device=DEV, dtype=torch.half, generator=g) for n, h in ((64, 8), (500, 2), (500, 2)))
+    vc[0, 70, 1, 5], vc[0, 333, 0, 9] = float("inf"), float("-inf")
+    kc[0, 333, 0] = 8 * q[0, 10, 2] / q[0, 10, 2].norm()            # close to the whole weight of one row
+    lens = torch.tensor([500], dtype=torch.int32, device=DEV)
+    out = fa.flash_attn_with_kvcache(q, kc, vc, cache_seqlens=lens, causal=True)
+    want = torch.zeros_like(out)
+    want[0, :, 4:, 5], want[0, :, :4, 9] = float("inf"), float("-inf")
+    assert torch.equal(out.isinf(), want.isinf()) and torch.equal(out[out.isinf()], want[want.isinf()])
+    assert torch.isfinite(out[~out.isinf()]).all()
