@@ -23,8 +23,8 @@
 // Both kernels are software-pipelined through the ORDER in which the MMA warps feed the (in-
 // order) tensor pipe, so that the element-wise warps always work while independent MMAs run:
 //
-//   dK/dV, per query tile i:   S(i) | dK += dS(i-1)^T Q(i-1) | dV += P(i-1)^T dO(i-1) | dP(i)
-//       S(i) and dP(i) take turns in ONE fp32 TMEM region, P and dS (16-bit) share a second one.
+//   dK/dV, per query tile i:   dV += P(i)^T dO(i) | S(i+1)   then   dK += dS(i)^T Q(i) | dP(i+1)
+//       S and dP have an fp32 TMEM region each, which P and dS (16-bit) overwrite at head_dim 128.
 //   dQ, per key tile k:        S(k+1) -> other S buffer | dQ += dS(k) K(k) | dP(k+1)
 //
 // Roles (384 threads):
@@ -34,9 +34,14 @@
 //   warp 9           MMA issuer (uniform control flow, one elected lane issues)
 //   warp 10          dK/dV kernel: loads the per-row statistics (base-2 LSE, delta) of the
 //                    streamed query tile and writes them as a 16-column GEMM operand
-//   warp 11          dK/dV kernel: second MMA issuer (the accumulating GEMMs)
+//   warp 11          dK/dV kernel: hands the staged dV and dK tiles to the TMA unit
 //
-// TMEM, dK/dV kernel: S^T or dP^T (128 columns) | P^T or dS^T (64) | K (64) | dV (128) | dK (128).
+// TMEM, dK/dV kernel: S^T, P^T (128 columns) | dP^T, dS^T (128) | dV (128) | dK (128); at head_dim 64
+//                     S^T | dP^T | P^T (64) | dS^T (64) | dV (64) | dK (64).
+// What it measured, against the two kernels it replaced (one with S and dP in turns in one region, one with a CTA per
+// key block): 32 packed sequences of 256 to 4096 tokens with window, ALiBi and soft cap 3610 -> 3045 us; 16 x 16 heads
+// x 4096 tokens of 128, causal, 1980 -> 1880 us (3.3 k cycles per tile instead of 4.2 k, of which the
+// power limit gives most back); 4 x 32 heads x 1024 x 1531 of 64 168 -> 157 us.
 // TMEM, dQ kernel:    S[0] | S[1] | dP | dQ    (4 x 128 columns).
 // All operand tiles are written by TMA with the 128-byte swizzle; the same tile is read
 // K-major (contraction over head_dim) or MN-major (contraction over its rows) through
@@ -78,12 +83,14 @@ static_assert((kRegsEw - 168) * 256 <= (168 - kRegsService) * 128, "register spl
 template <int D> struct BCfg {
   static constexpr int kTileBytes = kT * D * 2;
   static constexpr int kBoxes = D / 64;
-  // dK/dV kernel: V resident, ring A of K / Q entries (Q(i) lives from S(i) to dK(i); dK is
+  // dK/dV kernel: K and V resident, ring A of Q entries (Q(i) lives from S(i) to dK(i); dK is
   // staged over the last Q), ring B of dO entries (dO(i) lives from dP(i) to dV(i); dV is
   // staged over the last dO).
-  static constexpr int kStagesQ = (D == 128) ? 3 : 4;
+  static constexpr int kStagesQ = (D == 128) ? 2 : 4;
   static constexpr int kStagesO = (D == 128) ? 2 : 4;
-  static constexpr int kSmemTiles = (1 + kStagesQ + kStagesO) * kTileBytes;
+  static constexpr int kSmemTiles = (2 + kStagesQ + kStagesO) * kTileBytes;
+  // head_dim 64 leaves tensor-memory columns for P and dS beside S and dP
+  static constexpr bool kApart = D == 64;
   // dK/dV kernel: 128 x 16 operand tiles that carry the row statistics into the GEMMs
   // (two constant ones on the key side, one per ring stage on the query side)
   static constexpr int kAugTotal = (2 + kStagesQ) * kStatBlock;
@@ -106,20 +113,21 @@ struct BShared {
   uint64_t empty_b[4];    // ring B entry released
   uint64_t res_full;      // resident tiles of the item landed (dK/dV: V; dQ: Q and dO)
   uint64_t res_free;      // last MMA reading the resident tiles of the item finished
+  uint64_t k_full, k_free;  // dK/dV kernel: the same for K
   uint64_t s_full[2];     // S computed ([buffer] in the dQ kernel, [0] in the dK/dV kernel)
   uint64_t dp_full;       // dP computed
-  uint64_t p_ready;       // P written back (256 arrivals; dK/dV kernel)
+  uint64_t p_ready;       // dK/dV kernel: P written back (256 arrivals)
   uint64_t ds_ready;      // dS written back (256 arrivals)
-  uint64_t r_free;        // dK/dV kernel: scores, then dP, read out of their shared TMEM region (256 arrivals)
-  uint64_t p_free;        // dK/dV kernel: dV MMA that read P finished
-  uint64_t ds_free;       // dK/dV kernel: dK MMA that read dS finished
-  uint64_t k_copied;      // dK/dV kernel: K of the item copied from its ring slot into TMEM (256 arrivals)
+  // dK/dV kernel, P and dS in regions of their own:
+  uint64_t s_read, dp_read;   // scores, dP in registers (256 arrivals)
+  uint64_t p_free, ds_free;   // dV MMA that read P, dK MMA that read dS finished
+  uint64_t dv_done;       // dK/dV kernel: every dV MMA of the item finished
   uint64_t acc_done;      // every accumulation MMA of the item finished
   uint64_t sched_full[kSched];   // work-queue entry published by the producer thread
   uint64_t sched_empty[kSched];  // ... read by every consuming warp
   int4 sched_item[kSched][3];    // the item, decoded once by the producer thread (KItem / QItem)
-  uint64_t stg_ready[2];  // [group] result tile of an item staged for the store lane (and its message written)
-  uint64_t stg_taken[2];  // [group] the store lane has read the message
+  uint64_t stg_ready[2];  // result tile of an item staged for the store lane (and its message written); dK/dV: dV, dK
+  uint64_t stg_taken[2];  // [group] the store lane has read the message; dK/dV: [0], both tiles seen by the agent
   // [group] message to the store lane: shared-memory address of the staged tile (0 = nothing to
   // store, -1 = no more items), tensor-map coordinates head / row / batch, barrier to release
   volatile int stg_msg[2][5];
@@ -149,18 +157,22 @@ __device__ __forceinline__ bool bwait_relaxed(uint64_t* bar, uint32_t parity, BS
   return bwait(bar, parity, sh, code);
 }
 
-// Work queue.  `counter[0]` hands out candidate indices, `counter[1]` counts the CTAs that have
-// finished; the last one to finish puts both back to zero, so a launch always finds them at zero.
-// The producer thread draws a candidate, decodes it into an item (12 ints: KItem / QItem) and
+// Work queue.  A CTA's first candidate is its own index; `counter[0]` hands out the others,
+// `counter[1]` counts the CTAs that have finished; the last one to finish puts both back to zero, so a
+// launch always finds them at zero.  A launch without others (ncand <= gridDim.x) does not touch them.
+// The producer thread draws a candidate (just before the last loads of the current item, so that the
+// round trip to the counter is over when they are issued), decodes it into an item (12 ints: KItem / QItem) and
 // publishes the item to the other roles; entry number i of this CTA travels in ring slot
 // i % kSched.  Candidates outside their sequence are skipped; an item with total < 0 ends the queue.
+__device__ __forceinline__ unsigned int sched_draw(unsigned int* counter, int ncand) {
+  return ncand <= (int)gridDim.x ? (unsigned int)ncand : gridDim.x + atomicAdd(&counter[0], 1u);
+}
 template <typename Item, typename F>
-__device__ __forceinline__ Item sched_publish(BShared* sh, unsigned int* counter, int ncand, int& fidx, bool& ok,
-                                              F decode) {
+__device__ __forceinline__ Item sched_publish(BShared* sh, unsigned int* counter, int ncand, unsigned int u, int& fidx,
+                                              bool& ok, F decode) {
   static_assert(sizeof(Item) == 48, "an item travels as three 16-byte words");
   Item w;
-  for (;;) {
-    const unsigned int u = atomicAdd(&counter[0], 1u);
+  for (;; u = sched_draw(counter, ncand)) {
     if (u >= (unsigned int)ncand) {
       w.total = -1;
       break;
@@ -208,6 +220,23 @@ __device__ __forceinline__ void sched_release(BShared* sh, int idx) {
   if ((threadIdx.x & 31) == 0) mbar_arrive(smem_u32(&sh->sched_empty[idx % kSched]));
 }
 
+// For an agent that waits for a whole item (tens of microseconds; items differ in length by orders of magnitude):
+// sleeps between polls instead of spinning next to the other roles.
+__device__ __forceinline__ bool bwait_long(uint64_t* bar, uint32_t parity, BShared* sh, int code) {
+  const uint32_t a = smem_u32(bar);
+  const long long t0 = clock64();
+  while (!mbar_try_wait(a, parity)) {
+    __nanosleep(200);
+    if (sh->abort_flag || *reinterpret_cast<volatile int*>(&g_bwd_sm100_status) != 0) return false;
+    if (clock64() - t0 > 4 * FA_WAIT_CLOCKS) {
+      sh->abort_flag = code;
+      atomicCAS(&g_bwd_sm100_status, 0, code);
+      return false;
+    }
+  }
+  return true;
+}
+
 // Store lane: one thread that writes the result tiles the element-wise warps stage, so that none of
 // them has to wait for the TMA unit.  Per item it waits for the tile (and the message that
 // describes it), issues the store, waits until the unit has read the tile and releases the ring
@@ -215,23 +244,7 @@ __device__ __forceinline__ void sched_release(BShared* sh, int idx) {
 template <int D>
 __device__ __forceinline__ void store_lane(BShared* sh, int x, const CUtensorMap* tm, uint32_t release_count) {
   for (uint32_t n = 0;; ++n) {
-    // an item takes tens of microseconds: sleep between polls instead of spinning next to the
-    // producer lane (a spinning lane of the same warp takes its issue slots)
-    {
-      const uint32_t bar = smem_u32(&sh->stg_ready[x]);
-      const long long t0 = clock64();
-      bool done = false;
-      while (!(done = mbar_try_wait(bar, n & 1))) {
-        __nanosleep(400);
-        if (sh->abort_flag || *reinterpret_cast<volatile int*>(&g_bwd_sm100_status) != 0) break;
-        if (clock64() - t0 > 4 * FA_WAIT_CLOCKS) {   // items differ in length by orders of magnitude
-          sh->abort_flag = 62;
-          atomicCAS(&g_bwd_sm100_status, 0, 62);
-          break;
-        }
-      }
-      if (!done) return;
-    }
+    if (!bwait_long(&sh->stg_ready[x], n & 1, sh, 62)) return;
     const int addr = sh->stg_msg[x][0], head = sh->stg_msg[x][1], row = sh->stg_msg[x][2],
               batch = sh->stg_msg[x][3], rel = sh->stg_msg[x][4];
     mbar_arrive(smem_u32(&sh->stg_taken[x]));
@@ -259,7 +272,8 @@ __device__ __forceinline__ bool post_store(BShared* sh, int x, int n, int addr, 
   return true;
 }
 
-__device__ __forceinline__ void sched_finish(unsigned int* counter) {
+__device__ __forceinline__ void sched_finish(unsigned int* counter, int ncand) {
+  if (ncand <= (int)gridDim.x) return;
   __threadfence();
   const unsigned int done = atomicAdd(&counter[1], 1u);
   if (done == gridDim.x - 1) {
@@ -290,22 +304,10 @@ __device__ __forceinline__ void mma_kmajor(uint32_t d_tmem, uint32_t a_smem, uin
   }
 }
 
-// 128 x 128 x D product with A (128 rows x D, 16-bit pairs, D/2 columns) in TMEM and B a K-major tile.
-template <int D>
-__device__ __forceinline__ void mma_kmajor_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_smem,
-                                              uint32_t idesc, uint32_t leader) {
-  const uint64_t db = make_smem_desc(b_smem, 16, 1024);
-#pragma unroll
-  for (int kk = 0; kk < D / 16; ++kk) {
-    const uint32_t o = ((kk / 4) * (kT * 128) + (kk % 4) * 32) >> 4;
-    mma_f16_ts_lp(d_tmem, a_tmem + kk * 8, db + o, idesc, kk > 0, leader);
-  }
-}
-
 // acc(128 x D) += A(128 x 128, fp16 pairs in TMEM) * B(128 rows x D, MN-major smem tile).
 // A is stored as two 32-column blocks (written by the two element-wise groups) at
 // a_tmem and a_tmem + kGroupStride.
-template <int D, int kGroupStride = 64>
+template <int D, int kGroupStride>
 __device__ __forceinline__ void mma_from_tmem(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_smem,
                                               uint32_t idesc, bool accumulate, uint32_t leader) {
   const uint64_t db = make_smem_desc(b_smem, kT * 128, 1024);
@@ -322,18 +324,19 @@ __device__ __forceinline__ void mma_from_tmem(uint32_t d_tmem, uint32_t a_tmem, 
 template <typename T, int kCols>
 __device__ __forceinline__ void drain_acc(uint32_t tsrc, float mul, bool staged, uint32_t stg, int lrow,
                                           int col0, T* grow) {
+  uint32_t r[kCols / 32][32];
+#pragma unroll
+  for (int cc = 0; cc < kCols / 32; ++cc) tmem_ld32(tsrc + cc * 32, r[cc]);
+  tmem_wait_ld();
 #pragma unroll
   for (int cc = 0; cc < kCols / 32; ++cc) {
-    uint32_t r[32];
-    tmem_ld32(tsrc + cc * 32, r);
-    tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 32; i += 8) {
       uint4 v;
-      v.x = Elem<T>::pack(__uint_as_float(r[i]) * mul, __uint_as_float(r[i + 1]) * mul);
-      v.y = Elem<T>::pack(__uint_as_float(r[i + 2]) * mul, __uint_as_float(r[i + 3]) * mul);
-      v.z = Elem<T>::pack(__uint_as_float(r[i + 4]) * mul, __uint_as_float(r[i + 5]) * mul);
-      v.w = Elem<T>::pack(__uint_as_float(r[i + 6]) * mul, __uint_as_float(r[i + 7]) * mul);
+      v.x = Elem<T>::pack(__uint_as_float(r[cc][i]) * mul, __uint_as_float(r[cc][i + 1]) * mul);
+      v.y = Elem<T>::pack(__uint_as_float(r[cc][i + 2]) * mul, __uint_as_float(r[cc][i + 3]) * mul);
+      v.z = Elem<T>::pack(__uint_as_float(r[cc][i + 4]) * mul, __uint_as_float(r[cc][i + 5]) * mul);
+      v.w = Elem<T>::pack(__uint_as_float(r[cc][i + 6]) * mul, __uint_as_float(r[cc][i + 7]) * mul);
       const int col = col0 + cc * 32 + i;
       if (staged) st_shared_v4(sw128_addr(stg + (col / 64) * (kT * 128), lrow, (col % 64) / 8), v);
       else if (grow != nullptr) *reinterpret_cast<uint4*>(grow + cc * 32 + i) = v;
@@ -411,7 +414,9 @@ __device__ __forceinline__ bool dq_item(const fa_attn_args& p, const ScoreCfg& c
 // =======================================================================================
 // dK, dV
 // =======================================================================================
-template <typename T, int D, bool kExtras>
+// kDrop: P^T and dS^T are zero where the bit of (key, query row) in cfg.keep is 0, and scaled by
+// dropout_scale, which is folded into the statistics operand (its log2 is added to -lse2).
+template <typename T, int D, bool kExtras, bool kDrop>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -420,16 +425,17 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                       unsigned int* const queue, int* const host_status) {
   using C = BCfg<D>;
   constexpr int SQ = C::kStagesQ, SO = C::kStagesO;
-  constexpr int kConsumers = 11;   // warps that read the work queue: 8 element-wise, 2 issuers, statistics
+  constexpr bool kApart = C::kApart;
+  constexpr int kConsumers = 11;   // warps that read the work queue: 8 element-wise, issuer, statistics, store agent
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   BShared* sh = reinterpret_cast<BShared*>(tiles + C::kSmemTiles + C::kAugTotal);
-  const uint32_t sV = smem_u32(tiles);
+  const uint32_t sK = smem_u32(tiles), sV = sK + C::kTileBytes;
   const uint32_t sRingQ = sV + C::kTileBytes, sRingO = sRingQ + SQ * C::kTileBytes;
   // statistics operands: one block per ring stage, then the two of the key side (bwd_stats.cuh)
   unsigned char* aug = tiles + C::kSmemTiles;
-  const uint32_t sAug = sV + C::kSmemTiles, sAugKeys = sAug + SQ * kStatBlock;
+  const uint32_t sAug = sK + C::kSmemTiles, sAugKeys = sAug + SQ * kStatBlock;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int G = p.heads_q / p.heads_kv;
@@ -441,28 +447,31 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (tid == 0) {
     mbar_init(smem_u32(&sh->res_full), 1);
     mbar_init(smem_u32(&sh->res_free), 1);
+    mbar_init(smem_u32(&sh->k_full), 1);
+    mbar_init(smem_u32(&sh->k_free), 1);
     mbar_init(smem_u32(&sh->s_full[0]), 1);
-    mbar_init(smem_u32(&sh->s_full[1]), 1);
     mbar_init(smem_u32(&sh->dp_full), 1);
     mbar_init(smem_u32(&sh->p_ready), 256);
     mbar_init(smem_u32(&sh->ds_ready), 256);
-    mbar_init(smem_u32(&sh->r_free), 256);
+    mbar_init(smem_u32(&sh->s_read), 256);
+    mbar_init(smem_u32(&sh->dp_read), 256);
     mbar_init(smem_u32(&sh->p_free), 1);
     mbar_init(smem_u32(&sh->ds_free), 1);
+    mbar_init(smem_u32(&sh->dv_done), 1);
     mbar_init(smem_u32(&sh->acc_done), 1);
-    mbar_init(smem_u32(&sh->k_copied), 256);
     for (int i = 0; i < 4; ++i) {
-      mbar_init(smem_u32(&sh->full_a[i]), 2);   // the TMA load and the statistics warp (or two stand-in arrivals)
+      mbar_init(smem_u32(&sh->full_a[i]), 2);   // the TMA load and the statistics warp
       mbar_init(smem_u32(&sh->full_b[i]), 1);
-      mbar_init(smem_u32(&sh->empty_a[i]), 2);  // one commit from each of the two issuer warps (or a stand-in)
-      mbar_init(smem_u32(&sh->empty_b[i]), 2);
+      mbar_init(smem_u32(&sh->empty_a[i]), 1);  // commit behind the slot's last reader, or the store agent
+      mbar_init(smem_u32(&sh->empty_b[i]), 1);
     }
     for (int i = 0; i < kSched; ++i) {
       mbar_init(smem_u32(&sh->sched_full[i]), 1);
       mbar_init(smem_u32(&sh->sched_empty[i]), kConsumers);
     }
-    mbar_init(smem_u32(&sh->stg_ready[0]), 128);
-    mbar_init(smem_u32(&sh->stg_ready[1]), 128);
+    mbar_init(smem_u32(&sh->stg_ready[0]), 256);
+    mbar_init(smem_u32(&sh->stg_ready[1]), 256);
+    mbar_init(smem_u32(&sh->stg_taken[0]), 1);
     sh->abort_flag = 0;
     fence_barrier_init();
   }
@@ -476,16 +485,19 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sh->tmem_base;
-  // TMEM: R (128 fp32 columns: S^T, then dP^T of a tile) | X (64: P^T, then dS^T) | K (64) | dV | dK
-  const uint32_t tR = tmem, tX = tmem + 128, tK = tmem + 192, tdV = tmem + 256, tdK = tmem + 384;
+  // TMEM: R0 (128 fp32 columns: S^T) | R1 (128: dP^T) | [P^T (64) | dS^T (64)] | dV (D) | dK (D).
+  // Without regions of their own (head_dim 128) P^T overwrites S^T and dS^T overwrites dP^T, each
+  // element-wise group over its own columns.
+  constexpr int kPStride = kApart ? kHalfT / 2 : kHalfT;     // columns between the groups' blocks of P, of dS
+  const uint32_t tR0 = tmem, tR1 = tmem + 128;
+  const uint32_t tP = kApart ? tmem + 256 : tR0, tdS = kApart ? tmem + 320 : tR1;
+  const uint32_t tdV = tmem + 512 - 2 * D, tdK = tmem + 512 - D;
 
-  // Ring bookkeeping shared by every role.  An item with `total` query tiles takes, in order,
-  //   ring A:  K | Q(0) ... Q(total-1)        (total + 1 entries)
-  //   ring B:  dO(0) ... dO(total-1)          (total entries)
-  // and every role advances the same two position counters; entry `pos` lives in slot
-  // pos % stages and completes phase (pos / stages) & 1 of that slot's barriers.  The entries of
-  // the LAST tile are released by the epilogue (which stages dK and dV over them), the others
-  // by the commits of the two issuer warps.
+  // Ring bookkeeping shared by every role.  An item with `total` query tiles takes ring A entries
+  // Q(0) ... Q(total-1) and ring B entries dO(0) ... dO(total-1); every role advances one position
+  // counter, entry `pos` lives in slot pos % stages and completes phase (pos / stages) & 1 of that
+  // slot's barriers.  The entries of the LAST tile are released by the store agent (the epilogue stages
+  // dK and dV over them), the others by the commits of the issuer.
 
   if (warp == 8) {
     // ------------------------------- TMA producer ---------------------------------------
@@ -497,67 +509,56 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       prefetch_tmap(&tmdO);
       prefetch_tmap(&tmdK);
       prefetch_tmap(&tmdV);
-      int posA = 0, posB = 0, wi = 0, fidx = 0;
+      int pos = 0, wi = 0, fidx = 0;
+      unsigned int u = blockIdx.x;
       bool ok = true;
-      auto acquire_a = [&]() { return bwait_relaxed(&sh->empty_a[posA % SQ], ((posA / SQ) & 1) ^ 1, sh, 41); };
-      auto acquire_b = [&]() { return bwait_relaxed(&sh->empty_b[posB % SO], ((posB / SO) & 1) ^ 1, sh, 41); };
       auto decode = [&](int c, KItem& w) { return dkdv_item(p, cfg, c, nkb, w); };
-      // An item is drawn from the queue as late as possible -- when the loads of the previous one
-      // are all issued, a tile or two before it ends -- so that the CTAs share the work evenly;
-      // the other roles look one entry ahead only at the end of an item.
-      PROF_VARS(4);
+      // An item is drawn from the queue as late as possible -- before the last loads of the previous one,
+      // two tiles or three before it ends -- so that the CTAs share the work evenly.
       for (;;) {
-        PROF_T0();
-        const KItem w = sched_publish<KItem>(sh, queue, ncand, fidx, ok, decode);
-        PROF_ADD(0);
+        const KItem w = sched_publish<KItem>(sh, queue, ncand, u, fidx, ok, decode);
         if (!ok || w.total < 0) break;
-        if (w.total == 0) continue;
-        PROF_T0();
-        // K: a ring A entry; the second arrival of its barrier is made here
-        if (!(ok = acquire_a())) break;
-        {
-          const uint32_t bar = smem_u32(&sh->full_a[posA % SQ]);
-          mbar_expect_tx(bar, C::kTileBytes);
-          load_tile<D>(slotA(posA), &tmK, bar, w.g.k_row0 + w.n0, w.hk, w.g.k_boff);
-          mbar_arrive(bar);
-          ++posA;
+        if (w.total == 0) {
+          u = sched_draw(queue, ncand);
+          continue;
         }
-        for (int it = 0; it < w.total; ++it) {
+        // K: its slot is free once the last score GEMM of the previous item has read it
+        if (wi > 0 && !(ok = bwait_relaxed(&sh->k_free, (wi - 1) & 1, sh, 41))) break;
+        mbar_expect_tx(smem_u32(&sh->k_full), C::kTileBytes);
+        load_tile<D>(sK, &tmK, smem_u32(&sh->k_full), w.g.k_row0 + w.n0, w.hk, w.g.k_boff);
+        for (int it = 0; it < w.total; ++it, ++pos) {
           const int hq = w.hk * G + it / w.ntiles, m = w.m_lo + it % w.ntiles;
-          if (!(ok = acquire_a())) break;
+          if (it + 1 == w.total) u = sched_draw(queue, ncand);
+          if (!(ok = bwait_relaxed(&sh->empty_a[pos % SQ], ((pos / SQ) & 1) ^ 1, sh, 41))) break;
           {
-            const uint32_t bar = smem_u32(&sh->full_a[posA % SQ]);
+            const uint32_t bar = smem_u32(&sh->full_a[pos % SQ]);
             mbar_expect_tx(bar, C::kTileBytes);
-            load_tile<D>(slotA(posA), &tmQ, bar, w.g.q_row0 + m * kT, hq, w.g.q_boff);
-            ++posA;
-          }
-          if (!(ok = acquire_b())) break;
-          {
-            const uint32_t bar = smem_u32(&sh->full_b[posB % SO]);
-            mbar_expect_tx(bar, C::kTileBytes);
-            load_tile<D>(slotB(posB), &tmdO, bar, w.g.q_row0 + m * kT, hq, w.g.q_boff);
-            ++posB;
+            load_tile<D>(slotA(pos), &tmQ, bar, w.g.q_row0 + m * kT, hq, w.g.q_boff);
           }
           if (it == 0) {
-            // V (first needed by dP(0), after the first score tile): its slot is free once the last
-            // dP GEMM of the previous item has read it.  Requested after the first Q and dO tiles so
-            // that those never queue behind this wait.
+            // V: after the last dP GEMM of the previous item
             if (wi > 0 && !(ok = bwait_relaxed(&sh->res_free, (wi - 1) & 1, sh, 41))) break;
             const uint32_t bar = smem_u32(&sh->res_full);
             mbar_expect_tx(bar, C::kTileBytes);
             load_tile<D>(sV, &tmV, bar, w.g.k_row0 + w.n0, w.hk, w.g.k_boff);
           }
+          if (!(ok = bwait_relaxed(&sh->empty_b[pos % SO], ((pos / SO) & 1) ^ 1, sh, 41))) break;
+          {
+            const uint32_t bar = smem_u32(&sh->full_b[pos % SO]);
+            mbar_expect_tx(bar, C::kTileBytes);
+            load_tile<D>(slotB(pos), &tmdO, bar, w.g.q_row0 + m * kT, hq, w.g.q_boff);
+          }
         }
         if (!ok) break;
         ++wi;
-        PROF_ADD(1);
       }
-      PROF_FLUSH(true, 28, 4);
     }
   } else if (warp == 10) {
     // ------------------------------- statistics loader ----------------------------------
-    // The loads of the next tile are ISSUED right after the current one has been written and only
-    // consumed after the wait for the next slot, so their latency hides behind that wait.
+    // The loads of the next tile are ISSUED right after the current one has been written and only consumed
+    // after the wait for the next slot, so their latency hides behind that wait (nothing reads
+    // the registers in between: a scoreboard stall before the poll would serialise the two; the pieces worked
+    // out there too cost 4 x 1024 x 1531 of 32 heads of 64 387 -> 488 us).
     reg_dealloc<kRegsService>();
     float rl[kT / 32], rd[kT / 32];                  // statistics of rows lane, lane + 32, ... as loaded
     const float unit = stat_score_unit(cfg.scale_log2);
@@ -576,7 +577,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       }
     };
-    int posA = 0, sidx = 0;
+    int pos = 0, sidx = 0;
     bool ok = true, fetched = false;                 // fetched: tile 0 of the item about to run is in rl/rd
     KItem w = sched_get<KItem>(sh, sidx++, true, ok);
     while (ok && w.total >= 0) {
@@ -586,18 +587,18 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       bool haven = false;
       if (!fetched) fetch(w, 0);
-      ++posA;                                        // the K entry
-      for (int it = 0; it < w.total; ++it, ++posA) {
-        const int stage = posA % SQ;
+      for (int it = 0; it < w.total; ++it, ++pos) {
+        const int stage = pos % SQ;
         bool wt = true;
-        if (lane == 0) wt = bwait_relaxed(&sh->empty_a[stage], ((posA / SQ) & 1) ^ 1, sh, 42);
+        if (lane == 0) wt = bwait_relaxed(&sh->empty_a[stage], ((pos / SQ) & 1) ^ 1, sh, 42);
         if (!__all_sync(0xffffffffu, wt)) { ok = false; break; }
 #pragma unroll
         for (int k = 0; k < kT / 32; ++k) {
           const int i = lane + 32 * k;
           // NEGATED.  The feature variant adds the LSE after the soft cap, in the element-wise warps.
-          if (kExtras) sh->lse[stage][i] = isinf(rl[k]) ? -INFINITY : -rl[k];
-          stat_write_row<T, !kExtras>(aug + stage * kStatBlock, i, -rl[k], -rd[k], unit);
+          const float nl2 = kDrop ? cfg.drop_log2 - rl[k] : -rl[k];
+          if (kExtras) sh->lse[stage][i] = isinf(nl2) ? -INFINITY : nl2;
+          stat_write_row<T, !kExtras>(aug + stage * kStatBlock, i, nl2, -rd[k], unit);
         }
         fence_proxy_async();
         __syncwarp();
@@ -618,12 +619,17 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       w = sched_get<KItem>(sh, sidx++, true, ok);
     }
   } else if (warp == 9) {
-    // ------------------------------- MMA issuer, GEMMs into the fp32 region -------------
-    // This warp issues dP(i), then S(i+1) -- each once the element-wise warps have read its
-    // predecessor out of R (r_free).  Warp 11 issues the accumulating GEMMs dV(i), dK(i) that
-    // read P, dS from region X.
+    // ------------------------------- MMA issuer -----------------------------------------
+    // The GEMMs of tile i+1 follow, in the in-order tensor pipe, the accumulation of tile i that
+    // reads the region they overwrite:
+    //   P(i) stored:   dV += P(i)^T dO(i)   S(i+1)        (under the dS phase of tile i)
+    //   dS(i) stored:  dK += dS(i)^T Q(i)   dP(i+1)       (under the exp2 phase of tile i+1)
+    // so no barrier protects R0 and R1, and two stages of Q and of dO are enough.  Where P and dS
+    // have regions of their own, S(i+1) and dP(i+1) go ahead of the accumulations, as soon as S(i),
+    // dP(i) have been read.
     reg_dealloc<kRegsService>();
     constexpr uint32_t idesc_s = make_idesc(1, BFmt<T>::code, 0, 0, kT, kT);
+    constexpr uint32_t idesc_acc = make_idesc(1, BFmt<T>::code, 0, 1, kT, D);
     const uint32_t leader = elect_one() ? 1u : 0u;
     bool ok = true;
     // every lane polls (uniform control flow, no vote needed: a completed phase is seen by all)
@@ -632,151 +638,126 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       tc_fence_after();
     };
     const uint64_t dstat_s = stat_desc_key(sAugKeys, false), dstat_dp = stat_desc_key(sAugKeys, true);
-    auto stat_desc = [&](int pos, bool dp) { return stat_desc_query(sAugKeys, sAug + (pos % SQ) * kStatBlock, dp); };
-    PROF_VARS(8);
-    int posA = 0, posB = 0, wi = 0, tg = 0;          // tg: tiles issued so far by this CTA
+    auto stat_desc = [&](int ps, bool dp) { return stat_desc_query(sAugKeys, sAug + (ps % SQ) * kStatBlock, dp); };
     // The last query tile of a packed sequence also stages rows of the NEXT sequence.  Their P is
     // 0 (the statistics say so), but 0 * inf is NaN and dS^T Q, P^T dO contract over those rows:
     // this warp, the first reader of every staged Q and dO tile, zeroes them once the tile has
     // landed (scores and dP of those rows then are 0 too).
-    // S^T = K Q^T (K from TMEM) - lse2 / scale_log2 for the tile at ring position qpos
-    auto issue_s = [&](int qpos, int tile_no, int tail) {
-      PROF_T0();
-      wq(&sh->full_a[qpos % SQ], (qpos / SQ) & 1, 44);
-      PROF_ADD(1);
-      if (ok && tail < kT) zero_tile_tail<C::kBoxes, kT>(slotA(qpos), tail, lane);
-      PROF_T0();
-      if (tile_no > 0) wq(&sh->r_free, 1, 49);                                  // the previous dP read out
-      PROF_ADD(2);
+    // S^T = K Q^T - lse2 / scale_log2 for the tile at ring position ps
+    auto issue_s = [&](int ps, int tail) {
+      wq(&sh->full_a[ps % SQ], (ps / SQ) & 1, 44);
       if (!ok) return;
-      mma_kmajor_ts<D>(tR, tK, slotA(qpos), idesc_s, leader);
-      if (!kExtras) mma_f16_ss_lp(tR, dstat_s, stat_desc(qpos, false), idesc_s, 1u, leader);
+      if (tail < kT) zero_tile_tail<C::kBoxes, kT>(slotA(ps), tail, lane);
+      mma_kmajor<D>(tR0, sK, slotA(ps), idesc_s, leader);
+      if (!kExtras) mma_f16_ss_lp(tR0, dstat_s, stat_desc(ps, false), idesc_s, 1u, leader);
       mma_commit_lp(smem_u32(&sh->s_full[0]), leader);
     };
-    int sidx = 0;
+    // dP^T = V dO^T - delta
+    auto issue_dp = [&](int ps, int tail) {
+      wq(&sh->full_b[ps % SO], (ps / SO) & 1, 44);
+      if (!ok) return;
+      if (tail < kT) zero_tile_tail<C::kBoxes, kT>(slotB(ps), tail, lane);
+      mma_kmajor<D>(tR1, sV, slotB(ps), idesc_s, leader);
+      mma_f16_ss_lp(tR1, dstat_dp, stat_desc(ps, true), idesc_s, 1u, leader);
+      mma_commit_lp(smem_u32(&sh->dp_full), leader);
+    };
+    int pos = 0, wi = 0, sidx = 0;
     for (;;) {
-      PROF_T0();
       const KItem w = sched_get<KItem>(sh, sidx++, true, ok);
       if (!ok || w.total < 0) break;
-      PROF_ADD(6);
       if (w.total == 0) continue;
-      // K is in TMEM: its ring slot may be refilled (stand-in for the two MMA commits of a Q entry)
-      PROF_T0();
-      wq(&sh->k_copied, wi & 1, 43);
-      PROF_ADD(0);
-      if (!ok) break;
-      if (leader) mbar_arrive_cnt(smem_u32(&sh->empty_a[posA % SQ]), 2);
-      __syncwarp();
-      const int q0pos = posA + 1;
+      const int last = w.total - 1;
       // the query tile that crosses the end of its sequence (-1: none) and its first row to zero;
-      // m_cur / m_nxt: query tile of stream position i / i + 1 (the tiles repeat per query head)
+      // m_nxt: query tile of stream position i + 1 (the tiles repeat per query head)
       const int tail_m = (p.cu_seqlens_q != nullptr && (w.g.q_len % kT) != 0) ? w.g.q_len / kT : -1;
       const int tail_first = w.g.q_len % kT, m_end = w.m_lo + w.ntiles;
-      int m_cur = w.m_lo, m_nxt = (w.m_lo + 1 == m_end) ? w.m_lo : w.m_lo + 1;
-      issue_s(q0pos, tg, m_cur == tail_m ? tail_first : kT);
-      for (int i = 0; i < w.total && ok; ++i, ++tg, m_cur = m_nxt, m_nxt = (m_nxt + 1 == m_end) ? w.m_lo : m_nxt + 1) {
-        const int qpos = q0pos + i, opos = posB + i;
-        PROF_T0();
-        wq(&sh->full_b[opos % SO], (opos / SO) & 1, 44);
-        PROF_ADD(3);
-        if (ok && m_cur == tail_m) zero_tile_tail<C::kBoxes, kT>(slotB(opos), tail_first, lane);
-        PROF_T0();
-        if (i == 0) wq(&sh->res_full, wi & 1, 43);                              // V of this item
-        PROF_ADD(4);
-        PROF_T0();
-        wq(&sh->r_free, 0, 49);                                                 // S(i) read out
-        PROF_ADD(5);
+      int m_nxt = w.m_lo;
+      wq(&sh->k_full, wi & 1, 43);
+      issue_s(pos, m_nxt == tail_m ? tail_first : kT);
+      if (ok && last == 0) mma_commit_lp(smem_u32(&sh->k_free), leader);
+      wq(&sh->res_full, wi & 1, 43);
+      issue_dp(pos, m_nxt == tail_m ? tail_first : kT);
+      if (ok && last == 0) mma_commit_lp(smem_u32(&sh->res_free), leader);
+      for (int i = 0; i < w.total && ok; ++i, ++pos) {
+        const bool more = i < last;
+        m_nxt = (m_nxt + 1 == m_end) ? w.m_lo : m_nxt + 1;
+        const int tail = m_nxt == tail_m ? tail_first : kT;    // of tile i + 1
+        auto next_s = [&]() {
+          if (!more || !ok) return;
+          issue_s(pos + 1, tail);
+          if (ok && i + 1 == last) mma_commit_lp(smem_u32(&sh->k_free), leader);     // K's last reader
+        };
+        auto next_dp = [&]() {
+          if (!more || !ok) return;
+          issue_dp(pos + 1, tail);
+          if (ok && i + 1 == last) mma_commit_lp(smem_u32(&sh->res_free), leader);   // V's last reader
+        };
+        if (kApart && more) {
+          wq(&sh->s_read, pos & 1, 49);
+          next_s();
+        }
+        wq(&sh->p_ready, pos & 1, 45);
         if (!ok) break;
-        mma_kmajor<D>(tR, sV, slotB(opos), idesc_s, leader);                    // dP^T(i) = V dO(i)^T
-        mma_f16_ss_lp(tR, dstat_dp, stat_desc(qpos, true), idesc_s, 1u, leader); //           - delta
-        mma_commit_lp(smem_u32(&sh->dp_full), leader);
-        if (i + 1 < w.total) {
-          mma_commit_lp(smem_u32(&sh->empty_b[opos % SO]), leader);   // this warp's last reads of dO(i) and of
-          mma_commit_lp(smem_u32(&sh->empty_a[qpos % SQ]), leader);   // Q(i) and its statistics
-          issue_s(qpos + 1, tg + 1, m_nxt == tail_m ? tail_first : kT);
-        } else {
-          mma_commit_lp(smem_u32(&sh->res_free), leader);             // ... and of V (the epilogue releases
-        }                                                             // the last tile's ring entries)
-      }
-      posA += w.total + 1;
-      posB += w.total;
-      ++wi;
-    }
-    PROF_FLUSH(lane == 0, 16, 8);
-    __syncwarp();
-  } else if (warp == 11) {
-    // ------------------------------- MMA issuer, accumulations --------------------------
-    reg_dealloc<kRegsService>();
-    constexpr uint32_t idesc_acc = make_idesc(1, BFmt<T>::code, 0, 1, kT, D);
-    const uint32_t leader = elect_one() ? 1u : 0u;
-    bool ok = true;
-    auto wq = [&](uint64_t* bar, uint32_t parity, int code) {
-      if (ok) ok = bwait(bar, parity, sh, code);
-      tc_fence_after();
-    };
-    int posA = 0, posB = 0, tg = 0, sidx = 0, wi = 0;
-    PROF_VARS(4);
-    for (;;) {
-      PROF_T0();
-      const KItem w = sched_get<KItem>(sh, sidx++, true, ok);
-      if (!ok || w.total < 0) break;
-      PROF_ADD(3);
-      if (w.total == 0) continue;
-      for (int i = 0; i < w.total && ok; ++i, ++tg) {
-        const int qpos = posA + 1 + i, opos = posB + i;
-        // dO(i) may land after P(i) is ready; Q(i) has been read by S(i) long before dS(i) exists
-        PROF_T0();
-        wq(&sh->full_b[opos % SO], (opos / SO) & 1, 44);
-        PROF_ADD(0);
-        PROF_T0();
-        wq(&sh->p_ready, tg & 1, 45);
-        PROF_ADD(1);
+        mma_from_tmem<D, kPStride>(tdV, tP, slotB(pos), idesc_acc, i > 0, leader);    // dV += P(i)^T dO(i)
+        if (kApart) mma_commit_lp(smem_u32(&sh->p_free), leader);
+        // (dO(i)'s other reader, dP(i), precedes in the pipe)
+        mma_commit_lp(smem_u32(more ? &sh->empty_b[pos % SO] : &sh->dv_done), leader);
+        if (!kApart) next_s();
+        if (kApart && more) {
+          wq(&sh->dp_read, pos & 1, 49);
+          next_dp();
+        }
+        wq(&sh->ds_ready, pos & 1, 46);
         if (!ok) break;
-        const bool last = i + 1 == w.total;          // its ring entries are released by the epilogue
-        mma_from_tmem<D, 32>(tdV, tX, slotB(opos), idesc_acc, i > 0, leader);   // dV += P(i)^T dO(i)
-        if (!last) mma_commit_lp(smem_u32(&sh->empty_b[opos % SO]), leader);
-        mma_commit_lp(smem_u32(&sh->p_free), leader);
-        PROF_T0();
-        wq(&sh->ds_ready, tg & 1, 46);
-        PROF_ADD(2);
-        if (!ok) break;
-        mma_from_tmem<D, 32>(tdK, tX, slotA(qpos), idesc_acc, i > 0, leader);   // dK += dS(i)^T Q(i)
-        if (!last) mma_commit_lp(smem_u32(&sh->empty_a[qpos % SQ]), leader);
-        mma_commit_lp(smem_u32(&sh->ds_free), leader);
+        mma_from_tmem<D, kPStride>(tdK, tdS, slotA(pos), idesc_acc, i > 0, leader);   // dK += dS(i)^T Q(i)
+        if (kApart) mma_commit_lp(smem_u32(&sh->ds_free), leader);
+        if (more) mma_commit_lp(smem_u32(&sh->empty_a[pos % SQ]), leader);
+        if (!kApart) next_dp();
       }
       if (ok) mma_commit_lp(smem_u32(&sh->acc_done), leader);
-      // The element-wise warps now stage dV and dK over the item's last dO and Q tiles.  This warp
-      // has nothing to issue until the first P of the next item exists, so it hands the staged
-      // tiles to the TMA unit and releases the two ring entries once the unit has read them.
-      {
-        const int stgA = posA + w.total, stgB = posB + w.total - 1;
-        const bool via_tma = (p.cu_seqlens_k == nullptr) || (w.n0 + kT <= w.g.k_len);
-        wq(&sh->stg_ready[0], wi & 1, 62);
-        if (ok && via_tma && leader) {
-#pragma unroll
-          for (int bx = 0; bx < D / 64; ++bx)
-            tma_store_4d(&tmdV, slotB(stgB) + bx * (kT * 128), bx * 64, w.hk, w.g.k_row0 + w.n0, w.g.k_boff);
-        }
-        wq(&sh->stg_ready[1], wi & 1, 62);
-        if (ok && leader) {
-          if (via_tma) {
-#pragma unroll
-            for (int bx = 0; bx < D / 64; ++bx)
-              tma_store_4d(&tmdK, slotA(stgA) + bx * (kT * 128), bx * 64, w.hk, w.g.k_row0 + w.n0, w.g.k_boff);
-            tma_store_commit();
-            tma_store_wait_read();
-          }
-          // released like tiles whose two readers have finished
-          mbar_arrive_cnt(smem_u32(&sh->empty_b[stgB % SO]), 2);
-          mbar_arrive_cnt(smem_u32(&sh->empty_a[stgA % SQ]), 2);
-        }
-        __syncwarp();
-      }
-      posA += w.total + 1;
-      posB += w.total;
       ++wi;
     }
-    PROF_FLUSH(lane == 0, 24, 4);
+    __syncwarp();
+  } else if (warp == 11) {
+    // ------------------------------- store agent ----------------------------------------
+    // The element-wise warps stage dV and dK over the item's last dO and Q tiles; this warp hands them
+    // to the TMA unit and releases the two ring entries once the unit has read them.
+    reg_dealloc<kRegsService>();
+    const uint32_t leader = elect_one() ? 1u : 0u;
+    int pos = 0, sidx = 0, wi = 0;
+    bool ok = true;
+    for (;;) {
+      const KItem w = sched_get<KItem>(sh, sidx++, true, ok);
+      if (!ok || w.total < 0) break;
+      if (w.total == 0) continue;
+      pos += w.total;
+      const int stg = pos - 1;
+      const bool via_tma = (p.cu_seqlens_k == nullptr) || (w.n0 + kT <= w.g.k_len);
+      ok = bwait_long(&sh->stg_ready[0], wi & 1, sh, 62);
+      if (ok && via_tma && leader) {
+#pragma unroll
+        for (int bx = 0; bx < D / 64; ++bx)
+          tma_store_4d(&tmdV, slotB(stg) + bx * (kT * 128), bx * 64, w.hk, w.g.k_row0 + w.n0, w.g.k_boff);
+        tma_store_commit();
+      }
+      if (ok) ok = bwait_long(&sh->stg_ready[1], wi & 1, sh, 62);
+      if (!ok) break;
+      if (leader) {
+        mbar_arrive(smem_u32(&sh->stg_taken[0]));
+        if (via_tma) {
+#pragma unroll
+          for (int bx = 0; bx < D / 64; ++bx)
+            tma_store_4d(&tmdK, slotA(stg) + bx * (kT * 128), bx * 64, w.hk, w.g.k_row0 + w.n0, w.g.k_boff);
+          tma_store_commit();
+          tma_store_wait_read();
+        }
+        // released like tiles whose last reader has finished
+        mbar_arrive(smem_u32(&sh->empty_b[stg % SO]));
+        mbar_arrive(smem_u32(&sh->empty_a[stg % SQ]));
+      }
+      __syncwarp();
+      ++wi;
+    }
     __syncwarp();
   } else {
     // ------------------------------- element-wise groups --------------------------------
@@ -784,80 +765,46 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int x = warp >> 2;                         // column half
     const int lrow = (warp & 3) * 32 + lane;         // TMEM lane = key inside the tile
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tRx = tR + lane_addr + x * kHalfT;            // fp32 scores / dP: this group's 64 columns
-    const uint32_t tXx = tX + lane_addr + x * (kHalfT / 2);      // P^T, then dS^T, as 16-bit pairs: 32 columns
+    const uint32_t tSx = tR0 + lane_addr + x * kHalfT, tdPx = tR1 + lane_addr + x * kHalfT;    // this group's 64 columns
+    const uint32_t tPx = tP + lane_addr + x * kPStride, tdSx = tdS + lane_addr + x * kPStride;  // 16-bit pairs: 32 columns
     bool ok = true;
-    int posA = 0, posB = 0, wi = 0, tg = 0, sidx = 0;
-    bool k_in_tmem = false;                          // K of the item about to run is already in TMEM
+    int pos = 0, wi = 0, sidx = 0;
     PROF_VARS(16);
 #ifdef FA_PROF
     const long long prof_start = clock64();
-    long long prof_t1 = 0;
 #endif
 
-    // K of an item: from its ring slot into TMEM, where the score GEMM reads it as the A operand.
-    // This thread copies its key row, group x the x-th half of it.
-    auto copy_k = [&](int kpos) {
-      ok = bwait(&sh->full_a[kpos % SQ], (kpos / SQ) & 1, sh, 43);
-      if (!ok) return;
-      constexpr int kChunks = D / 16;                // 16-byte chunks per group
-      const uint32_t src = slotA(kpos);
-      uint32_t kr[kChunks / 4][16];
-#pragma unroll
-      for (int c = 0; c < kChunks; ++c) {
-        const int g = x * kChunks + c;
-        const uint4 v = ld_shared_v4(sw128_addr(src + (g / 8) * (kT * 128), lrow, g % 8));
-        kr[c / 4][(c % 4) * 4] = v.x; kr[c / 4][(c % 4) * 4 + 1] = v.y;
-        kr[c / 4][(c % 4) * 4 + 2] = v.z; kr[c / 4][(c % 4) * 4 + 3] = v.w;
-      }
-#pragma unroll
-      for (int c = 0; c < kChunks / 4; ++c) tmem_st16(tK + lane_addr + x * (D / 4) + c * 16, kr[c]);
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(smem_u32(&sh->k_copied));
-    };
-
-    KItem w, wn;                                     // wn: the entry after the current one, once looked at
-    bool peeked = false;
-    for (;;) {
-      PROF_T0();
-      if (peeked) {
-        sched_release(sh, sidx++);
-        w = wn;
-      } else {
-        w = sched_get<KItem>(sh, sidx++, true, ok);
-      }
-      if (!ok || w.total < 0) break;
-      peeked = false;
-      PROF_ADD(7);
+    KItem w = sched_get<KItem>(sh, sidx++, true, ok);
+    while (ok && w.total >= 0) {
       const int key = w.n0 + lrow;
-      // group A stores dV, group B stores dK * softmax_scale
-      T* grow = nullptr;
-      if (key < w.g.k_len)
-        grow = (x == 0) ? reinterpret_cast<T*>(p.dv) + (int64_t)w.g.k_boff * p.dv_stride[0] +
-                              (int64_t)(w.g.k_row0 + key) * p.dv_stride[1] + (int64_t)w.hk * p.dv_stride[2]
-                        : reinterpret_cast<T*>(p.dk) + (int64_t)w.g.k_boff * p.dk_stride[0] +
-                              (int64_t)(w.g.k_row0 + key) * p.dk_stride[1] + (int64_t)w.hk * p.dk_stride[2];
+      // each group stores half of the head_dim columns of dV and of dK * softmax_scale
+      constexpr int DH = D / 2;
+      T *gdv = nullptr, *gdk = nullptr;
+      if (key < w.g.k_len) {
+        gdv = reinterpret_cast<T*>(p.dv) + (int64_t)w.g.k_boff * p.dv_stride[0] +
+              (int64_t)(w.g.k_row0 + key) * p.dv_stride[1] + (int64_t)w.hk * p.dv_stride[2] + x * DH;
+        gdk = reinterpret_cast<T*>(p.dk) + (int64_t)w.g.k_boff * p.dk_stride[0] +
+              (int64_t)(w.g.k_row0 + key) * p.dk_stride[1] + (int64_t)w.hk * p.dk_stride[2] + x * DH;
+      }
       if (w.total == 0) {
         // no query can see these keys: their gradients are zero
-        if (grow != nullptr) {
+        if (gdv != nullptr) {
 #pragma unroll
-          for (int c = 0; c < D / 8; ++c) reinterpret_cast<uint4*>(grow)[c] = make_uint4(0u, 0u, 0u, 0u);
+          for (int c = 0; c < DH / 8; ++c) {
+            reinterpret_cast<uint4*>(gdv)[c] = make_uint4(0u, 0u, 0u, 0u);
+            reinterpret_cast<uint4*>(gdk)[c] = make_uint4(0u, 0u, 0u, 0u);
+          }
         }
+        w = sched_get<KItem>(sh, sidx++, true, ok);
         continue;
       }
       int vq_lo, vq_hi;                              // query positions that see this thread's key
       visible_q_interval(cfg, key, vq_lo, vq_hi);
-      PROF_T0();
-      if (!k_in_tmem) copy_k(posA);
-      PROF_ADD(4);
-      if (!ok) break;
-      const int q0pos = posA + 1;
       PROF_COUNT(9, w.total);
       PROF_COUNT(10, 1);
 
-      for (int it = 0; it < w.total && ok; ++it, ++tg) {
-        const int stage = (q0pos + it) % SQ;
+      for (int it = 0; it < w.total && ok; ++it, ++pos) {
+        const int stage = pos % SQ;
         const int hq = w.hk * G + it / w.ntiles, m = w.m_lo + it % w.ntiles;
         const int q0 = m * kT + x * kHalfT;            // first query row of this thread's columns
         const float slope = (kExtras && cfg.has_alibi) ? p.alibi_slopes[w.b * p.heads_q + hq] : 0.f;
@@ -870,9 +817,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // it is fetched into registers BEFORE the wait for the scores: shared-memory loads issued
         // while the tensor pipe streams its operands take hundreds of cycles, and here that
         // latency hides behind the wait.  Otherwise the GEMMs deliver S - lse and dP - delta.
-        float st[kHalfT];                              // -lse, later the soft cap's tanh factor
+        float st[kHalfT];                              // -lse
         if (kExtras) {
-          ok = bwait(&sh->full_a[stage], ((q0pos + it) / SQ) & 1, sh, 47);
+          ok = bwait(&sh->full_a[stage], (pos / SQ) & 1, sh, 47);
           if (!ok) break;
           const float4* L4 = reinterpret_cast<const float4*>(&sh->lse[stage][x * kHalfT]);
 #pragma unroll
@@ -881,32 +828,36 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             st[i4 * 4] = l4.x; st[i4 * 4 + 1] = l4.y; st[i4 * 4 + 2] = l4.z; st[i4 * 4 + 3] = l4.w;
           }
         }
+        uint2 keep2;                                   // this thread's 64 bits of the tile, on their way during the wait
+        if (kDrop) keep2 = __ldg(reinterpret_cast<const uint2*>(cfg.keep + key * cfg.keep_words + (q0 >> 5)));
         PROF_T0();
-        ok = bwait(&sh->s_full[0], tg & 1, sh, 46);
+        ok = bwait(&sh->s_full[0], pos & 1, sh, 46);
 #ifdef FA_PROF
         if (it == 0) PROF_ADD(11); else PROF_ADD(0);
-        prof_t1 = clock64();
+        PROF_T0();
 #endif
         if (!ok) break;
         tc_fence_after();
 
         // ---- exp phase: P = exp2(score - lse), written back as T pairs ---------------------
         uint32_t r0[32], r1[32];
-        tmem_ld32(tRx, r0);
-        tmem_ld32(tRx + 32, r1);
+        tmem_ld32(tSx, r0);
+        tmem_ld32(tSx + 32, r1);
         tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(smem_u32(&sh->r_free));            // the scores are in registers: dP may take the region
+        if (kApart) {
+          tc_fence_before();
+          mbar_arrive(smem_u32(&sh->s_read));          // the scores are in registers: S(i+1) may take R0
+        }
         float pf[kHalfT];                              // P in fp32, kept for the dS phase
         const float dist0 = (float)(q0 + off - key);   // query position - key position of column 0
         // columns (query rows) of this tile that see this thread's key
         const ColMask cm = make_col_mask(vq_lo - (q0 + off), vq_hi - (q0 + off));
         // One body, compiled per (masked tile, soft cap): no branch inside the unrolled loops.
-        uint32_t pkx[kExtras ? 32 : 1];                // feature variant: P as T pairs, packed inside the loop
-        auto exp_body = [&](auto mask_tag, auto cap_tag, auto abs_tag) {
+        // Half h of the group's columns: 32 scores to 16 pairs of P.
+        auto exp_body = [&](const int h, const uint32_t (&rr)[32], auto mask_tag, auto cap_tag, auto abs_tag) {
           constexpr bool kMask = decltype(mask_tag)::value;
-          constexpr bool kCap = decltype(cap_tag)::value;
-          constexpr bool kAbs = decltype(abs_tag)::value;
+          [[maybe_unused]] constexpr bool kCap = decltype(cap_tag)::value, kAbs = decltype(abs_tag)::value;
+          uint32_t pk[16];
           if constexpr (kExtras) {
             // Packed pairs throughout (the loop body is what the instruction cache has to hold:
             // as 64 scalar chains this variant stalled more on instruction fetch than on anything
@@ -917,13 +868,14 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             const float cl = cfg.softcap * FA_LOG2E;
             const float2 ka2 = make_float2(ka, ka), kb2 = make_float2(kb, kb), cl2 = make_float2(cl, cl);
             const float2 one2 = make_float2(1.f, 1.f), none2 = make_float2(-1.f, -1.f), two2 = make_float2(2.f, 2.f);
-            float2 d2 = make_float2(dist0, dist0 + 1.f);
+            const float dh = dist0 + 32.f * h;
+            float2 d2 = make_float2(dh, dh + 1.f);
 #pragma unroll
-            for (int i = 0; i < kHalfT; i += 2) {
-              const uint32_t* rr = i < 32 ? r0 : r1;
-              const float2 sv2 = make_float2(__uint_as_float(rr[i & 31]), __uint_as_float(rr[(i & 31) + 1]));
+            for (int i = 0; i < 32; i += 2) {
+              const int c = h * 32 + i;
+              const float2 sv2 = make_float2(__uint_as_float(rr[i]), __uint_as_float(rr[i + 1]));
               const float2 da = kAbs ? make_float2(fabsf(d2.x), fabsf(d2.y)) : d2;
-              const float2 st2 = make_float2(st[i], st[i + 1]);
+              const float2 st2 = make_float2(st[c], st[c + 1]);
               float2 pe;
               if (kCap) {
                 const float2 y2 = f2fma(ka2, da, f2mul(sv2, kb2));
@@ -931,179 +883,160 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 const float2 a2 = f2fma(th2, cl2, st2);
                 pe = make_float2(ex2(a2.x), ex2(a2.y));
                 if (kMask) {
-                  pe.x = col_visible(cm, i) ? pe.x : 0.f;
-                  pe.y = col_visible(cm, i + 1) ? pe.y : 0.f;
+                  pe.x = col_visible(cm, c) ? pe.x : 0.f;
+                  pe.y = col_visible(cm, c + 1) ? pe.y : 0.f;
                 }
-                pkx[i >> 1] = Elem<T>::pack(pe.x, pe.y);
+                pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
                 // the tanh factor of the soft cap goes into the copy kept for dS
                 pe = f2mul(pe, f2fma(f2mul(th2, th2), none2, one2));
               } else {
                 const float2 a2 = f2fma(ka2, da, f2fma(sv2, kb2, st2));
                 pe = make_float2(ex2(a2.x), ex2(a2.y));
                 if (kMask) {
-                  pe.x = col_visible(cm, i) ? pe.x : 0.f;
-                  pe.y = col_visible(cm, i + 1) ? pe.y : 0.f;
+                  pe.x = col_visible(cm, c) ? pe.x : 0.f;
+                  pe.y = col_visible(cm, c + 1) ? pe.y : 0.f;
                 }
-                pkx[i >> 1] = Elem<T>::pack(pe.x, pe.y);
+                pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
               }
-              pf[i] = pe.x;
-              pf[i + 1] = pe.y;
+              pf[c] = pe.x;
+              pf[c + 1] = pe.y;
               d2 = f2add(d2, two2);
             }
           } else {
             const float2 c2 = make_float2(cfg.scale_log2, cfg.scale_log2);
 #pragma unroll
-            for (int i = 0; i < kHalfT; i += 2) {
-              const uint32_t* rr = i < 32 ? r0 : r1;
-              const float2 a = f2mul(make_float2(__uint_as_float(rr[i & 31]), __uint_as_float(rr[(i & 31) + 1])), c2);
-              float2 pe = ex2_pair<kPolyEvery>(a, i >> 1);
+            for (int i = 0; i < 32; i += 2) {
+              const int c = h * 32 + i;
+              const float2 a = f2mul(make_float2(__uint_as_float(rr[i]), __uint_as_float(rr[i + 1])), c2);
+              float2 pe = make_float2(ex2(a.x), ex2(a.y));
               if (kMask) {
-                pe.x = col_visible(cm, i) ? pe.x : 0.f;
-                pe.y = col_visible(cm, i + 1) ? pe.y : 0.f;
+                pe.x = col_visible(cm, c) ? pe.x : 0.f;
+                pe.y = col_visible(cm, c + 1) ? pe.y : 0.f;
               }
-              pf[i] = pe.x;
-              pf[i + 1] = pe.y;
+              if (kDrop) {
+                const uint32_t kw = h == 0 ? keep2.x : keep2.y;
+                pe.x = (kw >> i) & 1u ? pe.x : 0.f;
+                pe.y = (kw >> (i + 1)) & 1u ? pe.y : 0.f;
+              }
+              pf[c] = pe.x;
+              pf[c + 1] = pe.y;
+              pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
             }
           }
+          tmem_st16(tPx + h * 16, pk);
         };
         const bool cap = kExtras && cfg.softcap > 0.f;
         // |distance| only where a visible element can lie on the other side of the diagonal
         const bool need_abs = kExtras && !cfg.causal;
+        auto both = [&](auto mask_tag, auto cap_tag, auto abs_tag) {
+          exp_body(0, r0, mask_tag, cap_tag, abs_tag);
+          exp_body(1, r1, mask_tag, cap_tag, abs_tag);
+        };
         auto run_exp = [&](auto mask_tag) {
           if (cap) {
-            if (need_abs) exp_body(mask_tag, std::true_type{}, std::true_type{});
-            else exp_body(mask_tag, std::true_type{}, std::false_type{});
+            if (need_abs) both(mask_tag, std::true_type{}, std::true_type{});
+            else both(mask_tag, std::true_type{}, std::false_type{});
           } else {
-            if (need_abs) exp_body(mask_tag, std::false_type{}, std::true_type{});
-            else exp_body(mask_tag, std::false_type{}, std::false_type{});
+            if (need_abs) both(mask_tag, std::false_type{}, std::true_type{});
+            else both(mask_tag, std::false_type{}, std::false_type{});
           }
         };
-        if (masked) run_exp(std::true_type{});
-        else run_exp(std::false_type{});
-#ifdef FA_PROF
-        prof_acc[masked ? 13 : 12] += (unsigned int)(clock64() - prof_t1);
-        if (masked) prof_acc[14] += 1;
-#endif
-        // X holds dS of the previous tile until its dK MMA has finished (ds_free)
-        if (tg > 0) {
-          PROF_T0();
-          ok = bwait(&sh->ds_free, (tg - 1) & 1, sh, 50);
-          PROF_ADD(1);
+        // with a region of its own, P(i-1) has to be read by its dV GEMM: long ago by now
+        if (kApart && pos > 0) {
+          ok = bwait(&sh->p_free, (pos - 1) & 1, sh, 51);
           if (!ok) break;
           tc_fence_after();
         }
-        if constexpr (kExtras) {
-          uint32_t pk[16];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) pk[i] = pkx[c * 16 + i];
-            tmem_st16(tXx + c * 16, pk);
-          }
-        } else {
-          uint32_t pk[16];
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-#pragma unroll
-            for (int i = 0; i < 16; ++i) pk[i] = Elem<T>::pack(pf[c * 32 + 2 * i], pf[c * 32 + 2 * i + 1]);
-            tmem_st16(tXx + c * 16, pk);
-          }
-        }
+        if (masked) run_exp(std::true_type{});
+        else run_exp(std::false_type{});
         tmem_wait_st();
         tc_fence_before();
         mbar_arrive(smem_u32(&sh->p_ready));
+#ifdef FA_PROF
+        if (masked) { PROF_ADD(13); prof_acc[14] += 1; } else PROF_ADD(12);
+#endif
 
         // ---- dS phase: dS = P (dP - delta) -------------------------------------------------
         PROF_T0();
-        ok = bwait(&sh->dp_full, tg & 1, sh, 48);
+        ok = bwait(&sh->dp_full, pos & 1, sh, 48);
         PROF_ADD(2);
-#ifdef FA_PROF
-        prof_t1 = clock64();
-#endif
         if (!ok) break;
-        tc_fence_after();
-        tmem_ld32(tRx, r0);
-        tmem_ld32(tRx + 32, r1);
-        tmem_wait_ld();
-        tc_fence_before();
-        mbar_arrive(smem_u32(&sh->r_free));            // dP is in registers: the next S may take the region
-        uint32_t pk0[16], pk1[16];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int e = 2 * i;
-          const uint32_t* rr = e < 32 ? r0 : r1;
-          const float2 ds = f2mul(make_float2(pf[e], pf[e + 1]),
-                                  make_float2(__uint_as_float(rr[e & 31]), __uint_as_float(rr[(e & 31) + 1])));
-          if (i < 16) pk0[i] = Elem<T>::pack(ds.x, ds.y);
-          else pk1[i - 16] = Elem<T>::pack(ds.x, ds.y);
-        }
-#ifdef FA_PROF
-        prof_acc[15] += (unsigned int)(clock64() - prof_t1);
-#endif
-        // X holds P of this tile until its dV MMA has finished (p_free)
         PROF_T0();
-        ok = bwait(&sh->p_free, tg & 1, sh, 51);
-        PROF_ADD(3);
-        if (!ok) break;
         tc_fence_after();
-        tmem_st16(tXx, pk0);
-        tmem_st16(tXx + 16, pk1);
+        tmem_ld32(tdPx, r0);
+        tmem_ld32(tdPx + 32, r1);
+        tmem_wait_ld();
+        if (kApart) {
+          tc_fence_before();
+          mbar_arrive(smem_u32(&sh->dp_read));
+          if (pos > 0) {
+            ok = bwait(&sh->ds_free, (pos - 1) & 1, sh, 50);
+            if (!ok) break;
+            tc_fence_after();
+          }
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          uint32_t pk[16];
+          const uint32_t* rr = c == 0 ? r0 : r1;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float2 ds = f2mul(make_float2(pf[c * 32 + 2 * i], pf[c * 32 + 2 * i + 1]),
+                                    make_float2(__uint_as_float(rr[2 * i]), __uint_as_float(rr[2 * i + 1])));
+            pk[i] = Elem<T>::pack(ds.x, ds.y);
+          }
+          tmem_st16(tdSx + c * 16, pk);
+        }
         tmem_wait_st();
         tc_fence_before();
         mbar_arrive(smem_u32(&sh->ds_ready));
+        PROF_ADD(15);
       }
       if (!ok) break;
 
-      // ---- end of the item ------------------------------------------------------------------
-      // K of the next item goes into TMEM first (every score GEMM of this item has finished, and
-      // the last dK GEMM still runs), so that the issuer can start on it during the epilogue.
-      const int stgA = posA + w.total, stgB = posB + w.total - 1;   // the last Q and dO tiles of the item
-      {
-        PROF_T0();
-        wn = sched_get<KItem>(sh, sidx, false, ok);
-        if (!ok) break;
-        peeked = true;
-        k_in_tmem = wn.total > 0;
-        PROF_ADD(7);
-        PROF_T0();
-        if (k_in_tmem) copy_k(stgA + 1);
-        PROF_ADD(4);
-        if (!ok) break;
-      }
-      // Epilogue: each group stages its tile over the item's last dO / Q tile (every MMA is done;
-      // swizzled box layout) and hands it to the second issuer warp, which lets the TMA unit write
+      // Epilogue: dV is staged over the item's last dO tile while the last dK GEMM still runs, then dK over
+      // the last Q tile (swizzled box layout), for the store agent, which lets the TMA unit write
       // full rows; a packed tile that reaches past the end of its sequence is stored row by row instead.
+      // The first score and dP GEMMs of the next item run meanwhile.
       PROF_T0();
-      ok = bwait(&sh->acc_done, wi & 1, sh, 49);
+      const KItem wn = sched_get<KItem>(sh, sidx++, true, ok);
+      PROF_ADD(7);
+      if (!ok) break;
+      const bool via_tma = (p.cu_seqlens_k == nullptr) || (w.n0 + kT <= w.g.k_len);
+      PROF_T0();
+      ok = bwait(&sh->dv_done, wi & 1, sh, 49);
       PROF_ADD(5);
       if (!ok) break;
       tc_fence_after();
       PROF_T0();
-      const uint32_t stg = (x == 0) ? slotB(stgB) : slotA(stgA);
-      const bool via_tma = (p.cu_seqlens_k == nullptr) || (w.n0 + kT <= w.g.k_len);
-      drain_acc<T, D>((x == 0 ? tdV : tdK) + lane_addr, (x == 0) ? 1.f : cfg.scale, via_tma, stg, lrow, 0, grow);
+      drain_acc<T, DH>(tdV + lane_addr + x * DH, 1.f, via_tma, slotB(pos - 1), lrow, x * DH, gdv);
       tc_fence_before();
       if (via_tma) fence_proxy_async();
-      mbar_arrive(smem_u32(&sh->stg_ready[x]));
+      // (the agent has seen the previous item's tiles: its barrier is never a whole phase behind)
+      if (wi > 0 && !(ok = bwait(&sh->stg_taken[0], (wi - 1) & 1, sh, 63))) break;
+      mbar_arrive(smem_u32(&sh->stg_ready[0]));
+      ok = bwait(&sh->acc_done, wi & 1, sh, 49);
+      if (!ok) break;
+      tc_fence_after();
+      drain_acc<T, DH>(tdK + lane_addr + x * DH, cfg.scale, via_tma, slotA(pos - 1), lrow, x * DH, gdk);
+      tc_fence_before();
+      if (via_tma) fence_proxy_async();
+      mbar_arrive(smem_u32(&sh->stg_ready[1]));
+      w = wn;
       PROF_ADD(6);
-      posA += w.total + 1;
-      posB += w.total;
       ++wi;
     }
 #ifdef FA_PROF
     prof_acc[8] = (unsigned int)(clock64() - prof_start);
 #endif
-    PROF_FLUSH(tid == 0, 0, 12);
-#ifdef FA_PROF
-    if (tid == 0) for (int pi = 11; pi < 16; ++pi) atomicAdd(&PROF_ARRAY[32 + pi], (unsigned long long)prof_acc[pi]);
-#endif
+    PROF_FLUSH(tid == 0, 0, 16);
   }
 
   tc_fence_before();
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, 512);
   if (tid == 0) {
-    if (sh->abort_flag == 0) sched_finish(queue);
+    if (sh->abort_flag == 0) sched_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }
@@ -1188,13 +1121,16 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       prefetch_tmap(&tmV);
       prefetch_tmap(&tmdO);
       int posA = 0, posB = 0, wi = 0, fidx = 0;
+      unsigned int u = blockIdx.x;
       bool ok = true;
       auto decode = [&](int c, QItem& w) { return dq_item(p, cfg, c, nmb, w); };
-      // an item is drawn from the queue only when the loads of the previous one are all issued
       for (;;) {
-        const QItem w = sched_publish<QItem>(sh, queue, ncand, fidx, ok, decode);
+        const QItem w = sched_publish<QItem>(sh, queue, ncand, u, fidx, ok, decode);
         if (!ok || w.total < 0) break;
-        if (w.total == 0) continue;
+        if (w.total == 0) {
+          u = sched_draw(queue, ncand);
+          continue;
+        }
         const int hk = w.h / (p.heads_q / p.heads_kv);
         // Q and dO: their slots are free once the last S and dP GEMMs of the previous item are done
         if (wi > 0 && !(ok = bwait_relaxed(&sh->res_free, (wi - 1) & 1, sh, 51))) break;
@@ -1223,6 +1159,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         };
         ok = load_k(0);
         for (int j = 0; j < w.total && ok; ++j) {
+          if (j + 1 == w.total) u = sched_draw(queue, ncand);
           if (j + 1 < w.total) ok = load_k(j + 1);
           if (ok) ok = load_v(j);
         }
@@ -1281,7 +1218,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         wq(&sh->ds_ready, tg & 1, 55);
         if (!ok) break;
-        mma_from_tmem<D>(tdQ, tdP, slotK(kpos), idesc_acc, k > 0, leader);        // dQ += dS(k) K(k)
+        mma_from_tmem<D, kHalfT>(tdQ, tdP, slotK(kpos), idesc_acc, k > 0, leader);        // dQ += dS(k) K(k)
         if (more) mma_commit_lp(smem_u32(&sh->empty_a[kpos % SK]), leader);       // (the epilogue releases the last)
         if (more) {
           wq(&sh->full_b[v1pos % SV], (v1pos / SV) & 1, 54);
@@ -1507,7 +1444,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, 512);
   if (tid == 0) {
-    if (sh->abort_flag == 0) sched_finish(queue);
+    if (sh->abort_flag == 0) sched_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }
@@ -1581,7 +1518,9 @@ int launch_dkdv(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   // scale so small that its reciprocal leaves the fp16 range takes the feature variant, whose
   // element-wise warps add the LSE themselves.
   const bool extras = cfg.has_alibi || cfg.softcap > 0.f || !(cfg.scale_log2 > 2e-5f);
-  auto kern = extras ? bwd_dkdv_sm100_kernel<T, D, true> : bwd_dkdv_sm100_kernel<T, D, false>;
+  auto kern = cfg.keep != nullptr ? bwd_dkdv_sm100_kernel<T, D, false, true>
+              : extras            ? bwd_dkdv_sm100_kernel<T, D, true, false>
+                                  : bwd_dkdv_sm100_kernel<T, D, false, false>;
   if (int r = set_smem_attr(kern, BCfg<D>::kSmemBytes, "bwd_dkdv_sm100")) return r;
   const int nkb = (a.seqlen_k + kT - 1) / kT;
   int ncand = 0;
@@ -1625,37 +1564,7 @@ int launch_dq(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
 
 }  // namespace
 
-int bwd_dkdv_cta_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st);
-
-#ifndef FA_DKDV_CTA_BELOW
-#define FA_DKDV_CTA_BELOW 1e9    // plain dense work items shorter than this many tiles go to the one-CTA-per-key-block kernel
-#endif
-// Average number of query tiles a block of 128 keys meets (times the GQA group): what one work
-// item of the dK/dV kernels amounts to.  Dense layout only (the lengths of a packed batch live
-// on the device).
-static double dkdv_tiles_per_item(const fa_attn_args& a, const ScoreCfg& cfg) {
-  const int nkb = (a.seqlen_k + kT - 1) / kT, off = a.q_pos_offset;
-  long long sum = 0;
-  for (int n = 0; n < nkb; ++n) {
-    int qlo, qhi;
-    const int k_last = (n * kT + kT < a.seqlen_k ? n * kT + kT : a.seqlen_k) - 1;
-    visible_query_range(cfg, n * kT, k_last, off, a.seqlen_q + off, qlo, qhi);
-    const int m_lo = (qlo - off > 0 ? qlo - off : 0) / kT, m_hi = ((qhi - off > 0 ? qhi - off : 0) + kT - 1) / kT;
-    if (m_hi > m_lo) sum += m_hi - m_lo;
-  }
-  return (double)sum / nkb * (a.heads_q / a.heads_kv);
-}
-
 int bwd_dkdv_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
-  // Two kernels (see bwd_dkdv_cta_sm100.cu): a plain dense problem goes to the one-CTA-per-key-block
-  // kernel (since it keeps K in shared memory and P, dS apart it wins at every item length: 2-7 %
-  // without a mask, 10-15 % with the causal mask or GQA, measured at 16-66 tiles per item),
-  // packed batches and the feature variants to the persistent one.
-  const bool features = cfg.has_alibi || cfg.softcap > 0.f || !(cfg.scale_log2 > 2e-5f);
-  double below = FA_DKDV_CTA_BELOW;
-  if (const char* e = getenv("FA_B200_DKDV_CTA_BELOW")) below = atof(e);   // tuning / tests: 0 = never
-  if (cfg.keep != nullptr || (!features && a.cu_seqlens_q == nullptr && dkdv_tiles_per_item(a, cfg) < below))
-    return bwd_dkdv_cta_sm100(a, cfg, st);
   if (a.head_dim == 128)
     return a.dtype == FA_BF16 ? launch_dkdv<__nv_bfloat16, 128>(a, cfg, st) : launch_dkdv<__half, 128>(a, cfg, st);
   return a.dtype == FA_BF16 ? launch_dkdv<__nv_bfloat16, 64>(a, cfg, st) : launch_dkdv<__half, 64>(a, cfg, st);
@@ -1667,19 +1576,15 @@ int bwd_dq_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   return a.dtype == FA_BF16 ? launch_dq<__nv_bfloat16, 64>(a, cfg, st) : launch_dq<__half, 64>(a, cfg, st);
 }
 
-int bwd_dkdv_cta_status();
-void bwd_dkdv_cta_clear_status();
-
 void bwd_sm100_clear_status() {
   const int z = 0;
   cudaMemcpyToSymbol(g_bwd_sm100_status, &z, sizeof(int));
-  bwd_dkdv_cta_clear_status();
 }
 
 int bwd_sm100_status() {
   int v = 0;
   cudaMemcpyFromSymbol(&v, g_bwd_sm100_status, sizeof(int));
-  return v != 0 ? v : bwd_dkdv_cta_status();
+  return v;
 }
 
 }  // namespace fa
