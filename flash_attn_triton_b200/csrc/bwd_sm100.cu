@@ -416,7 +416,7 @@ __device__ __forceinline__ bool dq_item(const fa_attn_args& p, const ScoreCfg& c
 // =======================================================================================
 // kDrop: P^T and dS^T are zero where the bit of (key, query row) in cfg.keep is 0, and scaled by
 // dropout_scale, which is folded into the statistics operand (its log2 is added to -lse2).
-template <typename T, int D, bool kExtras, bool kDrop>
+template <typename T, int D, Feat kFeat, bool kDrop>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -424,6 +424,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                       const fa_attn_args p, const ScoreCfg cfg, const int nkb, const int ncand,
                       unsigned int* const queue, int* const host_status) {
   using C = BCfg<D>;
+  constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr int SQ = C::kStagesQ, SO = C::kStagesO;
   constexpr bool kApart = C::kApart;
   constexpr int kConsumers = 11;   // warps that read the work queue: 8 element-wise, issuer, statistics, store agent
@@ -852,11 +853,11 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const float dist0 = (float)(q0 + off - key);   // query position - key position of column 0
         // columns (query rows) of this tile that see this thread's key
         const ColMask cm = make_col_mask(vq_lo - (q0 + off), vq_hi - (q0 + off));
-        // One body, compiled per (masked tile, soft cap): no branch inside the unrolled loops.
+        // One body, compiled per masked tile: no branch inside the unrolled loops.
         // Half h of the group's columns: 32 scores to 16 pairs of P.
-        auto exp_body = [&](const int h, const uint32_t (&rr)[32], auto mask_tag, auto cap_tag, auto abs_tag) {
+        auto exp_body = [&](const int h, const uint32_t (&rr)[32], auto mask_tag, auto abs_tag) {
           constexpr bool kMask = decltype(mask_tag)::value;
-          [[maybe_unused]] constexpr bool kCap = decltype(cap_tag)::value, kAbs = decltype(abs_tag)::value;
+          [[maybe_unused]] constexpr bool kAbs = decltype(abs_tag)::value;
           uint32_t pk[16];
           if constexpr (kExtras) {
             // Packed pairs throughout (the loop body is what the instruction cache has to hold:
@@ -925,20 +926,15 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
           tmem_st16(tPx + h * 16, pk);
         };
-        const bool cap = kExtras && cfg.softcap > 0.f;
         // |distance| only where a visible element can lie on the other side of the diagonal
         const bool need_abs = kExtras && !cfg.causal;
-        auto both = [&](auto mask_tag, auto cap_tag, auto abs_tag) {
-          exp_body(0, r0, mask_tag, cap_tag, abs_tag);
-          exp_body(1, r1, mask_tag, cap_tag, abs_tag);
-        };
         auto run_exp = [&](auto mask_tag) {
-          if (cap) {
-            if (need_abs) both(mask_tag, std::true_type{}, std::true_type{});
-            else both(mask_tag, std::true_type{}, std::false_type{});
+          if (need_abs) {
+            exp_body(0, r0, mask_tag, std::true_type{});
+            exp_body(1, r1, mask_tag, std::true_type{});
           } else {
-            if (need_abs) both(mask_tag, std::false_type{}, std::true_type{});
-            else both(mask_tag, std::false_type{}, std::false_type{});
+            exp_body(0, r0, mask_tag, std::false_type{});
+            exp_body(1, r1, mask_tag, std::false_type{});
           }
         };
         // with a region of its own, P(i-1) has to be read by its dV GEMM: long ago by now
@@ -1046,7 +1042,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 // =======================================================================================
 // kDrop: dS is zero where the bit of (query row, key) in cfg.keep is 0; the scale of the kept probabilities
 // is folded into the row's LSE.
-template <typename T, int D, bool kExtras, bool kDrop>
+template <typename T, int D, Feat kFeat, bool kDrop>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -1054,6 +1050,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                     const int nmb, const int ncand, unsigned int* const queue,
                     int* const host_status) {
   using C = BCfg<D>;
+  constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr int SK = C::kStagesK, SV = C::kStagesV;
   constexpr int kConsumers = 9;    // warps that read the work queue: 8 element-wise and the issuer
   extern __shared__ unsigned char smem_raw[];
@@ -1317,10 +1314,9 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         float pf[kHalfT];
         // columns (keys) of this tile that this thread's query row sees
         const ColMask cm = make_col_mask(vk_lo - k0, vk_hi - k0);
-        // One body, compiled per (masked tile, soft cap): no branch inside the unrolled loops.
-        auto exp_body = [&](auto mask_tag, auto cap_tag, auto abs_tag) {
+        // One body, compiled per masked tile: no branch inside the unrolled loops.
+        auto exp_body = [&](auto mask_tag, auto abs_tag) {
           constexpr bool kMask = decltype(mask_tag)::value;
-          constexpr bool kCap = decltype(cap_tag)::value;
           constexpr bool kAbs = decltype(abs_tag)::value;
           if (kExtras) {
             // packed pairs; the distance of a pair's columns goes down by (2, 2)
@@ -1366,16 +1362,10 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
           }
         };
-        const bool cap = kExtras && cfg.softcap > 0.f;
         const bool need_abs = kExtras && !cfg.causal;    // under the causal mask visible keys lie at distance >= 0
         auto run_exp = [&](auto mask_tag) {
-          if (cap) {
-            if (need_abs) exp_body(mask_tag, std::true_type{}, std::true_type{});
-            else exp_body(mask_tag, std::true_type{}, std::false_type{});
-          } else {
-            if (need_abs) exp_body(mask_tag, std::false_type{}, std::true_type{});
-            else exp_body(mask_tag, std::false_type{}, std::false_type{});
-          }
+          if (need_abs) exp_body(mask_tag, std::true_type{});
+          else exp_body(mask_tag, std::false_type{});
         };
         if (masked) run_exp(std::true_type{});
         else run_exp(std::false_type{});
@@ -1518,9 +1508,10 @@ int launch_dkdv(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   // scale so small that its reciprocal leaves the fp16 range takes the feature variant, whose
   // element-wise warps add the LSE themselves.
   const bool extras = cfg.has_alibi || cfg.softcap > 0.f || !(cfg.scale_log2 > 2e-5f);
-  auto kern = cfg.keep != nullptr ? bwd_dkdv_sm100_kernel<T, D, false, true>
-              : extras            ? bwd_dkdv_sm100_kernel<T, D, true, false>
-                                  : bwd_dkdv_sm100_kernel<T, D, false, false>;
+  auto kern = cfg.keep != nullptr  ? bwd_dkdv_sm100_kernel<T, D, Feat::kNone, true>
+              : cfg.softcap > 0.f ? bwd_dkdv_sm100_kernel<T, D, Feat::kCap, false>
+              : extras            ? bwd_dkdv_sm100_kernel<T, D, Feat::kAlibi, false>
+                                  : bwd_dkdv_sm100_kernel<T, D, Feat::kNone, false>;
   if (int r = set_smem_attr(kern, BCfg<D>::kSmemBytes, "bwd_dkdv_sm100")) return r;
   const int nkb = (a.seqlen_k + kT - 1) / kT;
   int ncand = 0;
@@ -1543,10 +1534,10 @@ int launch_dq(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
     set_error("bwd_dq_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
-  auto kern = cfg.keep != nullptr ? bwd_dq_sm100_kernel<T, D, false, true>
-              : extras            ? bwd_dq_sm100_kernel<T, D, true, false>
-                                  : bwd_dq_sm100_kernel<T, D, false, false>;
+  auto kern = cfg.keep != nullptr  ? bwd_dq_sm100_kernel<T, D, Feat::kNone, true>
+              : cfg.softcap > 0.f ? bwd_dq_sm100_kernel<T, D, Feat::kCap, false>
+              : cfg.has_alibi     ? bwd_dq_sm100_kernel<T, D, Feat::kAlibi, false>
+                                  : bwd_dq_sm100_kernel<T, D, Feat::kNone, false>;
   if (int r = set_smem_attr(kern, BCfg<D>::kSmemBytesDq, "bwd_dq_sm100")) return r;
   const int nmb = (a.seqlen_q + kT - 1) / kT;
   int ncand = 0;

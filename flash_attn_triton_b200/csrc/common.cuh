@@ -72,6 +72,11 @@ struct ScoreCfg {
   float rescale_at;
 };
 
+// Score options a kernel is compiled for; kCap takes ALiBi too (a zero slope leaves the score unchanged, exactly).  With the
+// soft cap as a branch inside one feature kernel, four copies of each unrolled score loop more than a launch needs
+// stood in its way to the instruction caches.
+enum class Feat { kNone, kAlibi, kCap };
+
 __host__ __device__ inline ScoreCfg make_score_cfg(float scale, float softcap, int causal, int wl,
                                                    int wr, bool alibi) {
   ScoreCfg c;

@@ -142,12 +142,13 @@ __device__ __forceinline__ int sched_get(PShared* sh, int idx, bool& ok) {
 // the FMA pipe (ex2_fma2) and the scores are read from tensor memory a second time for the exp2
 // pass, 32 columns at a time and one chunk ahead, instead of staying in 128 registers (the
 // polynomial needs the registers; without them it was a loss).  The host picks it for long items.
-template <typename T, int D, bool kExtras, int kPoly>
+template <typename T, int D, Feat kFeat, int kPoly>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                          const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                          const fa_attn_args p, const ScoreCfg cfg, const int npair, const int ncand,
                          unsigned int* const queue, int* const host_status) {
+  constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr bool kPvSplit = !kExtras;     // P V in two key halves (measured: helps the plain variants only)
   using C = PCfg<D>;
   constexpr int S = C::kStages;
@@ -427,11 +428,10 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         }
         if (prescaled) {
           // score pipeline and mask applied once, in place; values end up in the log2 domain.
-          // One body, compiled per (masked tile, soft cap): no branch inside the unrolled loops.
+          // One body, compiled per masked tile: no branch inside the unrolled loops.
           const float dist0 = (float)(qpos - k0);
-          auto score_tile = [&](auto mask_tag, auto cap_tag, auto abs_tag) {
+          auto score_tile = [&](auto mask_tag, auto abs_tag) {
             constexpr bool kMask = decltype(mask_tag)::value;
-            constexpr bool kCap = decltype(cap_tag)::value;
             constexpr bool kAbs = decltype(abs_tag)::value;
             if (kExtras) {
               // packed pairs; the distance of a pair's columns goes down by (2, 2)
@@ -465,16 +465,10 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
               }
             }
           };
-          const bool cap = kExtras && cfg.softcap > 0.f;
           const bool need_abs = kExtras && !cfg.causal;    // under the causal mask visible keys lie at distance >= 0
           auto run_score = [&](auto mask_tag) {
-            if (cap) {
-              if (need_abs) score_tile(mask_tag, std::true_type{}, std::true_type{});
-              else score_tile(mask_tag, std::true_type{}, std::false_type{});
-            } else {
-              if (need_abs) score_tile(mask_tag, std::false_type{}, std::true_type{});
-              else score_tile(mask_tag, std::false_type{}, std::false_type{});
-            }
+            if (need_abs) score_tile(mask_tag, std::true_type{});
+            else score_tile(mask_tag, std::false_type{});
           };
           if (masked) run_score(std::true_type{});
           else run_score(std::false_type{});
@@ -523,7 +517,7 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
         }
         // what the stored values are multiplied by to give log2-domain scores: softmax_scale log2e
         // on the plain path, cap log2e for capped scores (stored as tanh), else 1; all >= 0
-        const float mul = !prescaled ? cfg.scale_log2 : ((kExtras && cfg.softcap > 0.f) ? cfg.softcap * FA_LOG2E : 1.f);
+        const float mul = !prescaled ? cfg.scale_log2 : (kCap ? cfg.softcap * FA_LOG2E : 1.f);
         mx *= mul;
 
         // ---- lazy rescale ----------------------------------------------------------------
@@ -758,8 +752,10 @@ static int launch_p(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st,
   const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
   bool poly = fwd_poly_pays(a, cfg);
   if (const char* e = getenv("FA_B200_FWD_POLY")) poly = !extras && atoi(e) != 0;   // tests: 0 = never, 1 = always
-  auto kern = extras ? fwd_persist_sm100_kernel<T, D, true, 0>
-                     : (poly ? fwd_persist_sm100_kernel<T, D, false, 4> : fwd_persist_sm100_kernel<T, D, false, 0>);
+  auto kern = cfg.softcap > 0.f ? fwd_persist_sm100_kernel<T, D, Feat::kCap, 0>
+              : cfg.has_alibi   ? fwd_persist_sm100_kernel<T, D, Feat::kAlibi, 0>
+              : poly            ? fwd_persist_sm100_kernel<T, D, Feat::kNone, 4>
+                                : fwd_persist_sm100_kernel<T, D, Feat::kNone, 0>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_persist_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));

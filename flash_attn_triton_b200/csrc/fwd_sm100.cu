@@ -116,13 +116,14 @@ static_assert(sizeof(Shared) <= 4096, "Shared must fit its reserve");
 //      slower than kind::i8 (twice the tensor cycles of the score GEMM, codes of twice the size).
 // kDrop: probabilities whose bit in cfg.keep is 0 do not enter P@V (they stay in the row sum); the scale of
 // the kept ones goes into the normalisation of the output.
-template <typename T, int D, bool kExtras, int kInt8, bool kDrop>
+template <typename T, int D, Feat kFeat, int kInt8, bool kDrop>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                  const fa_attn_args p, const ScoreCfg cfg, const float* __restrict__ sq,
                  const float* __restrict__ sk, int* const host_status) {
   static_assert(kInt8 != 1 || D == 128, "kind::i8 stages 128-byte code rows");
+  constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   static_assert(!kDrop || (!kExtras && !kInt8), "dropout bits are read by the plain variant");
   // measured: 2-3 % faster on the plain variants, 2 % slower on the feature variant (whose
   // element-wise phase is three times as long, so the extra wait for the store costs more than
@@ -482,11 +483,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         mbar_arrive(smem_u32(&sh->sk_empty[j % kSkSlots]));
       } else if (prescaled) {
         // score pipeline and mask applied once, in place; values end up in the log2 domain.
-        // One body, compiled per (masked tile, soft cap): no branch inside the unrolled loops.
+        // One body, compiled per masked tile: no branch inside the unrolled loops.
         const float dist0 = (float)(qpos - k0);
-        auto score_tile = [&](auto mask_tag, auto cap_tag, auto abs_tag) {
+        auto score_tile = [&](auto mask_tag, auto abs_tag) {
           constexpr bool kMask = decltype(mask_tag)::value;
-          constexpr bool kCap = decltype(cap_tag)::value;
           constexpr bool kAbs = decltype(abs_tag)::value;
           if (kExtras) {
             // packed pairs; the distance of a pair's columns goes down by (2, 2)
@@ -520,16 +520,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             }
           }
         };
-        const bool cap = kExtras && cfg.softcap > 0.f;
         const bool need_abs = kExtras && !cfg.causal;    // under the causal mask visible keys lie at distance >= 0
         auto run_score = [&](auto mask_tag) {
-          if (cap) {
-            if (need_abs) score_tile(mask_tag, std::true_type{}, std::true_type{});
-            else score_tile(mask_tag, std::true_type{}, std::false_type{});
-          } else {
-            if (need_abs) score_tile(mask_tag, std::false_type{}, std::true_type{});
-            else score_tile(mask_tag, std::false_type{}, std::false_type{});
-          }
+          if (need_abs) score_tile(mask_tag, std::true_type{});
+          else score_tile(mask_tag, std::false_type{});
         };
         if (masked) run_score(std::true_type{});
         else run_score(std::false_type{});
@@ -578,7 +572,7 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       // what the stored values are multiplied by to give log2-domain scores: softmax_scale log2e
       // on the plain path, cap log2e for capped scores (stored as tanh), else 1; all >= 0
-      const float mul = !prescaled ? cfg.scale_log2 : ((kExtras && cfg.softcap > 0.f) ? cfg.softcap * FA_LOG2E : 1.f);
+      const float mul = !prescaled ? cfg.scale_log2 : (kCap ? cfg.softcap * FA_LOG2E : 1.f);
       mx *= mul;
       if (kInt8) mx *= sq_row;               // s_q > 0
 
@@ -804,10 +798,10 @@ static int launch(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st, i
     set_error("fwd_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
-  auto kern = cfg.keep != nullptr ? fwd_sm100_kernel<T, D, false, 0, true>
-              : extras            ? fwd_sm100_kernel<T, D, true, 0, false>
-                                  : fwd_sm100_kernel<T, D, false, 0, false>;
+  auto kern = cfg.keep != nullptr  ? fwd_sm100_kernel<T, D, Feat::kNone, 0, true>
+              : cfg.softcap > 0.f ? fwd_sm100_kernel<T, D, Feat::kCap, 0, false>
+              : cfg.has_alibi     ? fwd_sm100_kernel<T, D, Feat::kAlibi, 0, false>
+                                  : fwd_sm100_kernel<T, D, Feat::kNone, 0, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
@@ -941,7 +935,7 @@ int fwd_int8_sm100(const fa_int8_args& a, cudaStream_t st) {
   }
   const fa_attn_args p = int8_problem(a);
   const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
-  auto kern = fwd_sm100_kernel<__half, D, false, 1, false>;
+  auto kern = fwd_sm100_kernel<__half, D, Feat::kNone, 1, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_int8_sm100: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -967,7 +961,7 @@ int fwd_int8_codes16(const fa_int8_args& a, const void* q16, const void* k16, cu
   }
   ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
   cfg.rescale_at = 0.f;
-  auto kern = fwd_sm100_kernel<__half, D, false, 2, false>;
+  auto kern = fwd_sm100_kernel<__half, D, Feat::kNone, 2, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_int8_codes16: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
