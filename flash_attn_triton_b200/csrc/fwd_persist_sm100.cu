@@ -61,6 +61,8 @@ struct PShared {
   uint64_t p_ready[2];           // [stream]: P written back (128 arrivals)
   uint64_t p_half[2];            // [stream]: the first 64 keys of P written back (128 arrivals)
   uint64_t o_ready[2];           // [stream]: its latest P V finished
+  uint64_t o_slot[2];            // [stream]: the output entry of its item is free
+  uint64_t o_seen[2];            // [stream]: ... and the group knows (128 arrivals)
   uint64_t sched_full[kSched];   // queue entry published by the producer lane
   uint64_t sched_empty[kSched];  // ... read by every consuming warp
   int sched_item[kSched];        // candidate index, -1 = no more work
@@ -168,6 +170,8 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_u32(&sh->s_full[i]), 1);
       mbar_init(smem_u32(&sh->o_ready[i]), 1);
+      mbar_init(smem_u32(&sh->o_slot[i]), 1);
+      mbar_init(smem_u32(&sh->o_seen[i]), 128);
       mbar_init(smem_u32(&sh->p_ready[i]), 128);
       mbar_init(smem_u32(&sh->p_half[i]), 128);
     }
@@ -268,6 +272,9 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
           const int slot = pos % S;
           ok = wait_bar(&sh->kv_empty[slot], ((pos / S) & 1) ^ 1, sh, 13);
           if (ok) mbar_arrive(smem_u32(&sh->kv_full[slot]));
+          // one item ahead of the group at most, so that it never finds o_slot a whole phase ahead
+          if (ok && qi > 1) ok = wait_bar(&sh->o_seen[x], qi & 1, sh, 14);
+          if (ok) mbar_arrive(smem_u32(&sh->o_slot[x]));
           ++pos;
         }
       }
@@ -624,22 +631,13 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       const bool via_tma = uses_ring && in_seq && my_tiles > 0 &&
                            ((p.cu_seqlens_q == nullptr) || (m0 + kBM <= si.q_len));
       if (uses_ring) {
-        // The entry is ours once the producer has passed it (its previous occupant is released).
-        // A parity wait must not run a whole phase ahead of its barrier, and a stream with few or
-        // no tiles gets here long before the ring does: walk up the entries of that slot from the
-        // last position this stream KNOWS to have landed -- its own last V tile, or, without
-        // tiles, everything before this item once the item's Q tiles have landed (the producer
-        // passes the previous item's output entries before it loads them).
-        int known = pos + 2 * my_je - 1;
-        if (my_tiles == 0) {
-          ok = wait_bar(&sh->q_full, qi & 1, sh, 37);
-          if (!ok) break;
-          known = pos - 1;
-        }
-        ++qi;
-        for (int q = opos - S * ((opos - known - 1) / S); q <= opos && ok; q += S)
-          ok = wait_bar(&sh->kv_full[q % S], (q / S) & 1, sh, 36);
+        // The entry is ours once the producer has passed it (its previous occupant is released).  A stream with few
+        // or no tiles gets here long before the ring does, or long after: the other stream's tiles and the next item's
+        // loads do not wait for it.  So the entry has a barrier of its own, which waits for every group.
+        ok = wait_bar(&sh->o_slot[x], qi & 1, sh, 36);
         if (!ok) break;
+        mbar_arrive(smem_u32(&sh->o_seen[x]));
+        ++qi;
       }
       if (in_seq) {
         const float inv = l > 0.f ? 1.f / l : 0.f;
