@@ -518,4 +518,35 @@ __device__ __forceinline__ SeqInfo seq_info(const fa_attn_args& p, int b) {
   return s;
 }
 
+// Packed forwards have a CTA per tile that their sequences can have together, not per tile of the longest one: they
+// differ in length, and a CTA without a tile still waits for an SM to itself.
+template <int kBM> inline int64_t packed_tiles(const fa_attn_args& a) {
+  const int64_t most = (int64_t)((a.seqlen_q + kBM - 1) / kBM) * a.batch, sum = a.total_q / kBM + (int64_t)a.batch;
+  return sum < most ? sum : most;
+}
+// The t-th tile, counting those of sequence 0, 1, ... (with a causal mask the last, heaviest tile of a sequence first).
+// Called by whole warps; false when there are fewer.
+template <int kBM>
+__device__ __forceinline__ bool packed_tile(const fa_attn_args& p, bool causal, int t, int lane, int& b, int& mt) {
+  for (int b0 = 0; b0 < p.batch; b0 += 32) {
+    const int n = b0 + lane < p.batch ? (min(seq_info(p, b0 + lane).q_len, p.seqlen_q) + kBM - 1) / kBM : 0;
+    int end = n;                                   // tiles up to and with this lane's sequence
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, end, o);
+      if (lane >= o) end += v;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, t < end);
+    if (past != 0u) {
+      const int src = __ffs(past) - 1;
+      const int first = __shfl_sync(0xffffffffu, end - n, src), tiles = __shfl_sync(0xffffffffu, n, src);
+      b = b0 + src;
+      mt = causal ? first + tiles - 1 - t : t - first;
+      return true;
+    }
+    t -= __shfl_sync(0xffffffffu, end, 31);
+  }
+  return false;
+}
+
 }  // namespace fa

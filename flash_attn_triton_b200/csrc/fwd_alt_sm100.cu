@@ -194,9 +194,12 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     w.q_row0 = 0;
     w.q_boff = w.b;
   } else {
-    const SeqInfo si = seq_info(p, blockIdx.z);
-    const int mt = cfg.causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;     // heavy tiles first
+    packed = p.cu_seqlens_q != nullptr;
     w.b = blockIdx.z;
+    int mt = cfg.causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;           // heavy tiles first
+    // packed: blockIdx.x counts the tiles of the sequences one after the other
+    if (packed && !packed_tile<kBM>(p, cfg.causal, blockIdx.x, lane, w.b, mt)) return;
+    const SeqInfo si = seq_info(p, w.b);
     w.h = blockIdx.y;
     w.hk = w.h / (p.heads_q / p.heads_kv);
     w.m0 = mt * kBM;
@@ -210,7 +213,6 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     w.q_row0 = (int)si.q_row0;
     w.q_boff = (int)si.q_boff;
     w.part = 0;
-    packed = p.cu_seqlens_q != nullptr;
   }
   const int tq_min = w.pos0 + (w.m0 >> w.pack_log2);
   const int tq_max = w.pos0 + ((min(w.m0 + kBM, w.rows) - 1) >> w.pack_log2);
@@ -887,7 +889,7 @@ static int launch_rows(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cu
     set_error("fwd_alt_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  const dim3 grid((a.seqlen_q + kBM - 1) / kBM, a.heads_q, a.batch);
+  const dim3 grid((unsigned)(packed ? packed_tiles<kBM>(a) : (a.seqlen_q + kBM - 1) / kBM), a.heads_q, packed ? 1 : a.batch);
   const CacheGeo geo = {};
   if constexpr (D == 256) {
     if (cfg.has_alibi || cfg.softcap > 0.f)
