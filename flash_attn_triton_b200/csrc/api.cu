@@ -110,9 +110,11 @@ int bwd_dq_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int bwd_dkdv_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int fwd_alt_sm100(const fa_attn_args&, const ScoreCfg&, cudaStream_t);
 int fwd_alt_sm100_status();
+int fwd_duo_sm100_status();
 int64_t dropout_bits_words(int, int);
 int dropout_bits(const fa_attn_args&, const ScoreCfg&, uint32_t*, cudaStream_t);
 int fwd_alt_sm100_clear_status();
+int fwd_duo_sm100_clear_status();
 int decode_paged(const fa_decode_args&, cudaStream_t);
 int decode_paged_checked(const fa_decode_args&, uint32_t*, cudaStream_t);
 int decode_num_counters(const fa_decode_args&);
@@ -554,6 +556,7 @@ int fa_device_wait_status(int device) {
   int s = fwd_sm100_status();
   if (s == 0) s = bwd_sm100_status();
   if (s == 0) s = fwd_alt_sm100_status();
+  if (s == 0) s = fwd_duo_sm100_status();
   if (s == 0) s = host_wait_status(device);
   if (s != 0 && device >= 0 && device < 1024) g_host_wait[device] = s;   // remembered for the launchers
   return s;
@@ -569,6 +572,7 @@ int fa_device_wait_clear(int device) {
   fwd_sm100_clear_status();
   bwd_sm100_clear_status();
   fwd_alt_sm100_clear_status();
+  fwd_duo_sm100_clear_status();
   if (device >= 0 && device < 1024) g_host_wait[device] = 0;
   return FA_OK;
 }

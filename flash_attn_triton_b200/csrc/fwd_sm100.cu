@@ -33,6 +33,7 @@
 //
 // Every mbarrier wait is bounded; on timeout the CTA raises a device-side status word,
 // releases its TMEM and returns.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
@@ -826,6 +827,7 @@ int fwd_persist_sm100_clear_status();
 
 bool fwd_poly_pays(const fa_attn_args& a, const ScoreCfg& cfg);
 int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStream_t st);
+int fwd_duo_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st);
 
 // Plain dense problems for the one-tile kernel (fwd_alt_sm100.cu): a tile of its costs 1.8 k cycles of an SM
 // where a pair of tiles costs the others 4.3 k, but it has twice as many CTAs to start, drain and balance.
@@ -853,6 +855,35 @@ static OneTile one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
   return a.head_dim == 128 && 3 * ctas <= nk * sms ? kOneTileByCtas : kNotOneTile;
 }
 
+// Calls for the kernel with two CTAs per SM (fwd_duo_sm100.cu), whose starts and ends lie under each other's work but whose
+// tiles cost more at head_dim 128 (2.9 k cycles of an SM per tile, against 2.1 k: K and V of a CTA pass through two
+// ring slots, and every tile is loaded for 128 rows instead of 256).  Measured against the rule without it, launches
+// interleaved, 32 to 512 heads * batch, 128 to 4096 tokens, and packed batches of 12 to 48 sequences of 17 to 4096:
+//   up to 2.5 CTAs per SM        +1 to +15 %
+//   head_dim 64, plain           -2 to -22 % dense (16 x 32 heads x 1024, causal: 205 -> 191 us; no mask, 1531 tokens: 550 -> 518),
+//                                -2 to -11 % packed; +3 to +7 % where part of the exponentials would go to the FMA pipe
+//   others, by the key tiles of a row tile on average: up to 6.5  -2 to -26 % (head_dim 128, 512 x 1024, causal: 245 -> 235;
+//                                packed 17 to 2048, causal: 396 -> 370), 8 and more  0 to +15 %
+//   windows, up to 10            -4 to -12 % (32 packed sequences of 256 to 4096, window 1024, ALiBi and soft cap, head_dim
+//                                128: 1686 -> 1621): two thirds of a short window's tiles are masked, and the pair of
+//                                tiles of the other kernels sees one more than either needs
+static bool two_ctas_are_faster(const fa_attn_args& a, const ScoreCfg& cfg, int persistent_from) {
+  const bool packed = a.cu_seqlens_q != nullptr, plain = !cfg.has_alibi && !(cfg.softcap > 0.f);
+  const int64_t tiles = packed ? a.total_q / kBM + a.batch / 2 : (int64_t)((a.seqlen_q + kBM - 1) / kBM) * a.batch;
+  if (2 * tiles * a.heads_q <= 5 * (int64_t)sm_count(a.device)) return false;
+  // the choice between the kernels must not show in the results
+  if (cfg.keep == nullptr && persistent_from > 0 && a.seqlen_k >= persistent_from && fwd_poly_pays(a, cfg)) return false;
+  if (!packed && a.seqlen_k >= 96 * kBN) return false;                      // one_tile_is_faster()
+  if (plain && a.head_dim == 64) return true;
+  // of a packed batch only the sum and the longest are known here
+  const int64_t keys = packed ? (a.total_k / a.batch + a.seqlen_k) / 2 : a.seqlen_k;
+  const int64_t nk = (keys + kBN - 1) / kBN;
+  int64_t twice = cfg.causal ? nk + 1 : 2 * nk;
+  const int right = cfg.causal ? 0 : cfg.wr;
+  if (cfg.wl < 0 || right < 0) return twice <= 13;
+  return std::min<int64_t>(twice, 2 * (((int64_t)cfg.wl + right) / kBN + 2)) <= 20;
+}
+
 int fwd_sm100(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
   ScoreCfg cfg = plain;
   if (a.head_dim == 256 || a.seqlen_k < 256 || cfg.keep != nullptr) cfg.rescale_at = 0.f;
@@ -863,6 +894,8 @@ int fwd_sm100(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
   const char* e = getenv("FA_B200_FWD_PERSISTENT_FROM");
   if (e != nullptr) {
     from = atoi(e);
+  } else if (two_ctas_are_faster(a, cfg, from)) {
+    return fwd_duo_sm100(a, cfg, st);
   } else if (const OneTile why = one_tile_is_faster(a, cfg)) {
     return fwd_alt_sm100(a, cfg, why == kOneTileByCtas && from > 0 && a.seqlen_k >= from && fwd_poly_pays(a, cfg), st);
   }
