@@ -226,7 +226,7 @@ __device__ __forceinline__ bool bwait_long(uint64_t* bar, uint32_t parity, BShar
   const uint32_t a = smem_u32(bar);
   const long long t0 = clock64();
   while (!mbar_try_wait(a, parity)) {
-    __nanosleep(64);
+    __nanosleep(200);
     if (sh->abort_flag || *reinterpret_cast<volatile int*>(&g_bwd_sm100_status) != 0) return false;
     if (clock64() - t0 > 4 * FA_WAIT_CLOCKS) {
       sh->abort_flag = code;
@@ -359,17 +359,16 @@ __device__ __forceinline__ Geo geo_of(const fa_attn_args& p, int b) {
   return g;
 }
 
-// dK/dV: candidate c = ((b * heads_kv + hk) * key_blocks + key block), or with by_block = batch * heads_kv > 0
-// c = key block * by_block + (b * heads_kv + hk); key block 0 sees the most query tiles under a causal mask.
-// Returns false when the key block lies outside its sequence.
+// dK/dV: candidates in the order of block_of(), units = (batch entry, kv head); key block 0 sees the most
+// query tiles under a causal mask.  Returns false when the key block lies outside its sequence.
 struct KItem {
   Geo g;
   int n0, hk, b;
   int m_lo, ntiles, total;   // query tiles [m_lo, m_lo + ntiles) per query head; total = ntiles * group
 };
-__device__ __forceinline__ bool dkdv_item(const fa_attn_args& p, const ScoreCfg& cfg, int cand, int nkb, int by_block,
-                                          KItem& w) {
-  const int nblk = by_block > 0 ? cand / by_block : cand % nkb, rem = by_block > 0 ? cand % by_block : cand / nkb;
+__device__ __forceinline__ bool dkdv_item(const fa_attn_args& p, const ScoreCfg& cfg, int cand, int nkb, KItem& w) {
+  int nblk, rem;
+  block_of(cand, nkb, p.batch * p.heads_kv, cfg.unit_group, rem, nblk);
   w.hk = rem % p.heads_kv;
   w.b = rem / p.heads_kv;
   w.n0 = nblk * kT;
@@ -386,7 +385,7 @@ __device__ __forceinline__ bool dkdv_item(const fa_attn_args& p, const ScoreCfg&
   return true;
 }
 
-// dQ: candidate c = ((b * heads_q + h) * query_blocks + i), or with by_block as above; with a causal mask block i counts
+// dQ: the same with units = (batch entry, head); with a causal mask block i counts
 // down from the last (heaviest) query block.  Returns false when the block lies outside its sequence.
 struct QItem {
   Geo g;
@@ -394,9 +393,9 @@ struct QItem {
   int n_hi, total;           // step j works on key tile n_hi - 1 - j (masked tiles first)
   int pad;
 };
-__device__ __forceinline__ bool dq_item(const fa_attn_args& p, const ScoreCfg& cfg, int cand, int nmb, int by_block,
-                                        QItem& w) {
-  const int i = by_block > 0 ? cand / by_block : cand % nmb, rem = by_block > 0 ? cand % by_block : cand / nmb;
+__device__ __forceinline__ bool dq_item(const fa_attn_args& p, const ScoreCfg& cfg, int cand, int nmb, QItem& w) {
+  int i, rem;
+  block_of(cand, nmb, p.batch * p.heads_q, cfg.unit_group, rem, i);
   w.h = rem % p.heads_q;
   w.b = rem / p.heads_q;
   w.m0 = (cfg.causal ? (nmb - 1 - i) : i) * kT;
@@ -424,7 +423,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                       const __grid_constant__ CUtensorMap tmdK, const __grid_constant__ CUtensorMap tmdV,
-                      const fa_attn_args p, const ScoreCfg cfg, const int nkb, const int by_block, const int ncand,
+                      const fa_attn_args p, const ScoreCfg cfg, const int nkb, const int ncand,
                       unsigned int* const queue, int* const host_status) {
   using C = BCfg<D>;
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
@@ -512,7 +511,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       int pos = 0, wi = 0, fidx = 0;
       unsigned int u = blockIdx.x;
       bool ok = true;
-      auto decode = [&](int c, KItem& w) { return dkdv_item(p, cfg, c, nkb, by_block, w); };
+      auto decode = [&](int c, KItem& w) { return dkdv_item(p, cfg, c, nkb, w); };
       // An item is drawn from the queue as late as possible -- before the last loads of the previous one,
       // two tiles or three before it ends -- so that the CTAs share the work evenly.
       for (;;) {
@@ -1018,7 +1017,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1)
 bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                     const __grid_constant__ CUtensorMap tmdQ, const fa_attn_args p, const ScoreCfg cfg,
-                    const int nmb, const int by_block, const int ncand, unsigned int* const queue,
+                    const int nmb, const int ncand, unsigned int* const queue,
                     int* const host_status) {
   using C = BCfg<D>;
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
@@ -1091,7 +1090,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       int posA = 0, posB = 0, wi = 0, fidx = 0;
       unsigned int u = blockIdx.x;
       bool ok = true;
-      auto decode = [&](int c, QItem& w) { return dq_item(p, cfg, c, nmb, by_block, w); };
+      auto decode = [&](int c, QItem& w) { return dq_item(p, cfg, c, nmb, w); };
       for (;;) {
         const QItem w = sched_publish<QItem>(sh, queue, ncand, u, fidx, ok, decode);
         if (!ok || w.total < 0) break;
@@ -1468,15 +1467,12 @@ bool candidate_count(int64_t blocks, int64_t heads, int64_t batch, int* out) {
   return true;
 }
 
-// Order of the candidates.  One head after the other keeps the tiles that the CTAs stream in L2, but the last heads' heavy
-// blocks come late.  Where everything a call reads stays in L2 anyway, the heaviest blocks of all heads go first: with
-// few items per CTA the time is the balance of the last ones (6 x 8 heads x 802 tokens of 128, causal, dK/dV 47 -> 34 us; 1 x 16 x 2048: dK/dV 58 -> 42, dQ 40 -> 30).
-int order_by_block(const fa_attn_args& a, int heads) {
+ScoreCfg with_order(const fa_attn_args& a, const ScoreCfg& cfg, int heads, int blocks) {
   const bool packed = a.cu_seqlens_q != nullptr;
   const int64_t q = packed ? a.total_q : (int64_t)a.batch * a.seqlen_q, k = packed ? a.total_k : (int64_t)a.batch * a.seqlen_k;
-  const int64_t bytes = 4 * a.head_dim * (q * a.heads_q + k * a.heads_kv);
-  const int64_t units = (int64_t)a.batch * heads;
-  return bytes <= (int64_t)64 << 20 && units <= 0x7fffffff ? (int)units : 0;
+  ScoreCfg c = cfg;
+  c.unit_group = unit_group(a, cfg, heads, blocks, 4 * a.head_dim * (q * a.heads_q + k * a.heads_kv));
+  return c;
 }
 
 template <typename T, int D>
@@ -1504,7 +1500,7 @@ int launch_dkdv(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   unsigned int* queue = work_queue(a.device);
   if (queue == nullptr) return FA_ERR_LAUNCH;
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
-  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytes, st>>>(m.q, m.k, m.v, m.dout, m.dk, m.dv, a, cfg, nkb, order_by_block(a, a.heads_kv), ncand, queue,
+  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytes, st>>>(m.q, m.k, m.v, m.dout, m.dk, m.dv, a, with_order(a, cfg, a.heads_kv, nkb), nkb, ncand, queue,
                                                            host_wait_word(a.device));
   return check_launch("bwd_dkdv_sm100");
 }
@@ -1530,7 +1526,7 @@ int launch_dq(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   unsigned int* queue = work_queue(a.device);
   if (queue == nullptr) return FA_ERR_LAUNCH;
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
-  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytesDq, st>>>(m.q, m.k, m.v, m.dout, m.dq, a, cfg, nmb, order_by_block(a, a.heads_q), ncand, queue,
+  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytesDq, st>>>(m.q, m.k, m.v, m.dout, m.dq, a, with_order(a, cfg, a.heads_q, nmb), nmb, ncand, queue,
                                                              host_wait_word(a.device));
   return check_launch("bwd_dq_sm100");
 }

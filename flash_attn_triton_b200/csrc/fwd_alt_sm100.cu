@@ -195,12 +195,16 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     w.q_boff = w.b;
   } else {
     packed = p.cu_seqlens_q != nullptr;
-    w.b = blockIdx.z;
-    int mt = cfg.causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;           // heavy tiles first
-    // packed: blockIdx.x counts the tiles of the sequences one after the other
-    if (packed && !packed_tile<kBM>(p, cfg.causal, blockIdx.x, lane, w.b, mt)) return;
+    int mt;
+    if (packed) {                                  // the tiles of the sequences one after the other, each for all heads
+      w.h = blockIdx.x % p.heads_q;
+      if (!packed_tile<kBM>(p, cfg.causal, blockIdx.x / p.heads_q, lane, w.b, mt)) return;
+    } else {
+      const int mtiles = (p.seqlen_q + kBM - 1) / kBM;
+      dense_block(p, cfg, mtiles, w.b, w.h, mt);
+      if (cfg.causal) mt = mtiles - 1 - mt;        // heavy tiles first
+    }
     const SeqInfo si = seq_info(p, w.b);
-    w.h = blockIdx.y;
     w.hk = w.h / (p.heads_q / p.heads_kv);
     w.m0 = mt * kBM;
     w.rows = si.q_len;
@@ -875,7 +879,7 @@ static int launch_alt(K kern, int smem, dim3 grid, cudaStream_t st, const CUtens
 
 // Dense or packed forward; poly: exponentials as the persistent kernel would take them.  With ALiBi or a soft cap only head_dim 256 comes here (one_tile_is_faster()).
 template <typename T, int D>
-static int launch_rows(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStream_t st) {
+static int launch_rows(const fa_attn_args& a, const ScoreCfg& plain, bool poly, cudaStream_t st) {
   const bool packed = a.cu_seqlens_q != nullptr;
   const int64_t q_rows = packed ? a.total_q : a.seqlen_q, k_rows = packed ? a.total_k : a.seqlen_k;
   const int64_t batch = packed ? 1 : a.batch;
@@ -889,7 +893,8 @@ static int launch_rows(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cu
     set_error("fwd_alt_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  const dim3 grid((unsigned)(packed ? packed_tiles<kBM>(a) : (a.seqlen_q + kBM - 1) / kBM), a.heads_q, packed ? 1 : a.batch);
+  ScoreCfg cfg = plain;
+  const dim3 grid = packed ? dim3((unsigned)(packed_tiles<kBM>(a) * a.heads_q)) : dense_grid(a, (a.seqlen_q + kBM - 1) / kBM, cfg);
   const CacheGeo geo = {};
   if constexpr (D == 256) {
     if (cfg.has_alibi || cfg.softcap > 0.f)

@@ -84,10 +84,15 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const uint32_t sQ = smem_u32(tiles), sKV = sQ + C::kTileBytes;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
-  const int h = blockIdx.y;
-  int b = blockIdx.z, mt = cfg.causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;    // heavy tiles first
-  // packed: blockIdx.x counts the tiles of the sequences one after the other
-  if (p.cu_seqlens_q != nullptr && !packed_tile<kBM>(p, cfg.causal, blockIdx.x, lane, b, mt)) return;
+  int h, b, mt;
+  if (p.cu_seqlens_q != nullptr) {                 // the tiles of the sequences one after the other, each for all heads
+    h = blockIdx.x % p.heads_q;
+    if (!packed_tile<kBM>(p, cfg.causal, blockIdx.x / p.heads_q, lane, b, mt)) return;
+  } else {
+    const int mtiles = (p.seqlen_q + kBM - 1) / kBM;
+    dense_block(p, cfg, mtiles, b, h, mt);
+    if (cfg.causal) mt = mtiles - 1 - mt;          // heavy tiles first
+  }
   const SeqInfo si = seq_info(p, b);
   const int m0 = mt * kBM;
   if (m0 >= si.q_len) return;
@@ -464,7 +469,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // host side
 // ---------------------------------------------------------------------------------------
 template <typename T, int D>
-static int launch_duo(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
+static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
   using C = DCfg<D>;
   const bool packed = a.cu_seqlens_q != nullptr;
   const int64_t q_rows = packed ? a.total_q : a.seqlen_q, k_rows = packed ? a.total_k : a.seqlen_k;
@@ -482,16 +487,17 @@ static int launch_duo(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t s
     set_error("fwd_duo_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  auto kern = cfg.keep != nullptr  ? fwd_duo_sm100_kernel<T, D, Feat::kNone, true>
-              : cfg.softcap > 0.f ? fwd_duo_sm100_kernel<T, D, Feat::kCap, false>
-              : cfg.has_alibi     ? fwd_duo_sm100_kernel<T, D, Feat::kAlibi, false>
-                                  : fwd_duo_sm100_kernel<T, D, Feat::kNone, false>;
+  auto kern = plain.keep != nullptr  ? fwd_duo_sm100_kernel<T, D, Feat::kNone, true>
+              : plain.softcap > 0.f ? fwd_duo_sm100_kernel<T, D, Feat::kCap, false>
+              : plain.has_alibi     ? fwd_duo_sm100_kernel<T, D, Feat::kAlibi, false>
+                                    : fwd_duo_sm100_kernel<T, D, Feat::kNone, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_duo_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
     return FA_ERR_LAUNCH;
   }
-  const dim3 grid((unsigned)(packed ? packed_tiles<kBM>(a) : (a.seqlen_q + kBM - 1) / kBM), a.heads_q, packed ? 1 : a.batch);
+  ScoreCfg cfg = plain;
+  const dim3 grid = packed ? dim3((unsigned)(packed_tiles<kBM>(a) * a.heads_q)) : dense_grid(a, (a.seqlen_q + kBM - 1) / kBM, cfg);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, host_wait_word(a.device));
   return check_launch("fwd_duo_sm100");
 }

@@ -91,9 +91,10 @@ struct Geo {
 
 // false: the candidate lies outside its sequence (packed batches) and is skipped
 __device__ __forceinline__ bool item_geo(const fa_attn_args& p, const ScoreCfg& cfg, int c, int npair, Geo& g) {
-  const int pr = c % npair;
-  g.h = (c / npair) % p.heads_q;
-  g.b = c / (npair * p.heads_q);
+  int unit, pr;
+  block_of(c, npair, p.heads_q * p.batch, cfg.unit_group, unit, pr);
+  g.h = unit % p.heads_q;
+  g.b = unit / p.heads_q;
   const int mblk = cfg.causal ? (npair - 1 - pr) : pr;      // heavy blocks first
   g.si = seq_info(p, g.b);
   g.m00 = mblk * 2 * kBM;
@@ -736,7 +737,7 @@ bool fwd_poly_pays(const fa_attn_args& a, const ScoreCfg& cfg) {
 }
 
 template <typename T, int D>
-static int launch_p(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st, int q_rows, int k_rows) {
+static int launch_p(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st, int q_rows, int k_rows) {
   using C = PCfg<D>;
   CUtensorMap tq, tk, tv, to;
   const bool packed = a.cu_seqlens_q != nullptr;
@@ -747,13 +748,13 @@ static int launch_p(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st,
     set_error("fwd_persist_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
-  bool poly = fwd_poly_pays(a, cfg);
+  const bool extras = plain.has_alibi || plain.softcap > 0.f;
+  bool poly = fwd_poly_pays(a, plain);
   if (const char* e = getenv("FA_B200_FWD_POLY")) poly = !extras && atoi(e) != 0;   // tests: 0 = never, 1 = always
-  auto kern = cfg.softcap > 0.f ? fwd_persist_sm100_kernel<T, D, Feat::kCap, 0>
-              : cfg.has_alibi   ? fwd_persist_sm100_kernel<T, D, Feat::kAlibi, 0>
-              : poly            ? fwd_persist_sm100_kernel<T, D, Feat::kNone, 4>
-                                : fwd_persist_sm100_kernel<T, D, Feat::kNone, 0>;
+  auto kern = plain.softcap > 0.f ? fwd_persist_sm100_kernel<T, D, Feat::kCap, 0>
+              : plain.has_alibi   ? fwd_persist_sm100_kernel<T, D, Feat::kAlibi, 0>
+              : poly              ? fwd_persist_sm100_kernel<T, D, Feat::kNone, 4>
+                                  : fwd_persist_sm100_kernel<T, D, Feat::kNone, 0>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_persist_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
@@ -768,6 +769,8 @@ static int launch_p(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st,
     return FA_ERR_UNSUPPORTED;
   }
   const int ncand = (int)ncand64;
+  ScoreCfg cfg = plain;
+  cfg.unit_group = fwd_unit_group(a, plain, npair);
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, npair, ncand, queue, host_wait_word(a.device));
   return check_launch("fwd_persist_sm100");

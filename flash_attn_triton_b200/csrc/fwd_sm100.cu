@@ -140,8 +140,10 @@ fwd_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   const uint32_t sKV = sQ + 2 * C::kTileBytes;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int h = blockIdx.y, b = blockIdx.z;
-  const int mblk = cfg.causal ? (gridDim.x - 1 - blockIdx.x) : blockIdx.x;  // heavy blocks first
+  const int npair = (p.seqlen_q + 2 * kBM - 1) / (2 * kBM);
+  int b, h, mblk;
+  dense_block(p, cfg, npair, b, h, mblk);
+  if (cfg.causal) mblk = npair - 1 - mblk;             // heavy blocks first
   const SeqInfo si = seq_info(p, b);
   const int m00 = mblk * 2 * kBM;
   if (m00 >= si.q_len) return;
@@ -788,7 +790,7 @@ static bool make_map(CUtensorMap* m, const void* base, const int64_t* stride, in
 }
 
 template <typename T, int D>
-static int launch(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st, int q_rows, int k_rows) {
+static int launch(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st, int q_rows, int k_rows) {
   using C = Cfg<D>;
   CUtensorMap tq, tk, tv, to;
   const bool packed = a.cu_seqlens_q != nullptr;
@@ -799,16 +801,17 @@ static int launch(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st, i
     set_error("fwd_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  auto kern = cfg.keep != nullptr  ? fwd_sm100_kernel<T, D, Feat::kNone, 0, true>
-              : cfg.softcap > 0.f ? fwd_sm100_kernel<T, D, Feat::kCap, 0, false>
-              : cfg.has_alibi     ? fwd_sm100_kernel<T, D, Feat::kAlibi, 0, false>
-                                  : fwd_sm100_kernel<T, D, Feat::kNone, 0, false>;
+  auto kern = plain.keep != nullptr  ? fwd_sm100_kernel<T, D, Feat::kNone, 0, true>
+              : plain.softcap > 0.f ? fwd_sm100_kernel<T, D, Feat::kCap, 0, false>
+              : plain.has_alibi     ? fwd_sm100_kernel<T, D, Feat::kAlibi, 0, false>
+                                    : fwd_sm100_kernel<T, D, Feat::kNone, 0, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
     return FA_ERR_LAUNCH;
   }
-  dim3 grid((a.seqlen_q + 2 * kBM - 1) / (2 * kBM), a.heads_q, a.batch);
+  ScoreCfg cfg = plain;
+  const dim3 grid = dense_grid(a, (a.seqlen_q + 2 * kBM - 1) / (2 * kBM), cfg);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, nullptr, nullptr, host_wait_word(a.device));
   return check_launch("fwd_sm100");
 }
@@ -967,14 +970,14 @@ int fwd_int8_sm100(const fa_int8_args& a, cudaStream_t st) {
     }
   }
   const fa_attn_args p = int8_problem(a);
-  const ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
+  ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
+  const dim3 grid = dense_grid(p, (a.seqlen + 2 * kBM - 1) / (2 * kBM), cfg);
   auto kern = fwd_sm100_kernel<__half, D, Feat::kNone, 1, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_int8_sm100: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return FA_ERR_LAUNCH;
   }
-  dim3 grid((S + 2 * kBM - 1) / (2 * kBM), H, B);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, cfg, a.sq_scratch, a.s_k, host_wait_word(a.device));
   return check_launch("fwd_int8_sm100");
 }
@@ -994,13 +997,13 @@ int fwd_int8_codes16(const fa_int8_args& a, const void* q16, const void* k16, cu
   }
   ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
   cfg.rescale_at = 0.f;
+  const dim3 grid = dense_grid(p, (a.seqlen + 2 * kBM - 1) / (2 * kBM), cfg);
   auto kern = fwd_sm100_kernel<__half, D, Feat::kNone, 2, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_int8_codes16: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     return FA_ERR_LAUNCH;
   }
-  dim3 grid((a.seqlen + 2 * kBM - 1) / (2 * kBM), a.heads, a.batch);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, p, cfg, a.sq_scratch, a.s_k, host_wait_word(a.device));
   return check_launch("fwd_int8_codes16");
 }
