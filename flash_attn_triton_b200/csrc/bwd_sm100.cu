@@ -1471,7 +1471,10 @@ ScoreCfg with_order(const fa_attn_args& a, const ScoreCfg& cfg, int heads, int b
   const bool packed = a.cu_seqlens_q != nullptr;
   const int64_t q = packed ? a.total_q : (int64_t)a.batch * a.seqlen_q, k = packed ? a.total_k : (int64_t)a.batch * a.seqlen_k;
   ScoreCfg c = cfg;
-  c.unit_group = unit_group(a, cfg, heads, blocks, 4 * a.head_dim * (q * a.heads_q + k * a.heads_kv));
+  // with many blocks per SM the last ones weigh little, and groups cost (16 x 16 heads x 4096: dQ 1325 -> 1359 us, dK/dV
+  // 1913 -> 1929 in groups of 16; the forwards do not mind)
+  if (!packed && (int64_t)a.batch * heads * blocks > 16 * (int64_t)sm_count(a.device)) c.unit_group = 1;
+  else c.unit_group = unit_group(a, cfg, heads, 4 * a.head_dim * (q * a.heads_q + k * a.heads_kv));
   return c;
 }
 

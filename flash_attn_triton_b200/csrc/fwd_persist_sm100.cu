@@ -770,7 +770,7 @@ static int launch_p(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t s
   }
   const int ncand = (int)ncand64;
   ScoreCfg cfg = plain;
-  cfg.unit_group = fwd_unit_group(a, plain, npair);
+  cfg.unit_group = fwd_unit_group(a, plain);
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, npair, ncand, queue, host_wait_word(a.device));
   return check_launch("fwd_persist_sm100");
