@@ -54,6 +54,7 @@
 #include "common.cuh"
 #define PROF_TAG bwd
 #include "prof.cuh"
+#include "skew.cuh"
 #include "sm100.cuh"
 
 namespace fa {
@@ -117,9 +118,9 @@ struct BShared {
   uint64_t res_full;      // resident tiles of the item landed (dK/dV: V; dQ: Q and dO)
   uint64_t res_free;      // last MMA reading the resident tiles of the item finished
   uint64_t k_full, k_free;  // dK/dV kernel: the same for K
-  uint64_t s_full[2];     // S computed ([buffer] in the dQ kernel, [0] in the dK/dV kernel)
+  uint64_t s_full[2];     // [buffer]: S computed
   uint64_t dp_full;       // dP computed
-  uint64_t p_ready;       // dK/dV kernel: P written back (256 arrivals)
+  uint64_t p_ready[2];    // dK/dV kernel, [score buffer]: P written back (256 arrivals)
   uint64_t ds_ready;      // dS written back (256 arrivals)
   uint64_t dv_done;       // dK/dV kernel: every dV MMA of the item finished
   uint64_t acc_done;      // every accumulation MMA of the item finished
@@ -454,7 +455,8 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_init(smem_u32(&sh->s_full[0]), 1);
     mbar_init(smem_u32(&sh->s_full[1]), 1);
     mbar_init(smem_u32(&sh->dp_full), 1);
-    mbar_init(smem_u32(&sh->p_ready), 256);
+    mbar_init(smem_u32(&sh->p_ready[0]), 256);
+    mbar_init(smem_u32(&sh->p_ready[1]), 256);
     mbar_init(smem_u32(&sh->ds_ready), 256);
     mbar_init(smem_u32(&sh->dv_done), 1);
     mbar_init(smem_u32(&sh->acc_done), 1);
@@ -623,7 +625,11 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     // reads the region they overwrite:
     //   P(i) stored:   dV += P(i)^T dO(i)   S(i + buffers)   (under the dS phase of tile i)
     //   dS(i) stored:  dK += dS(i)^T Q(i)   dP(i+1)          (under the exp2 phase of tile i+1)
-    // so no barrier protects the regions, and with one score buffer two stages of Q and of dO are enough.
+    // so no barrier protects the regions from the GEMMs, and with one score buffer two stages of Q and of dO are
+    // enough.  What protects them, and the barriers, from the warps: no warp arrives on a barrier again before its phase
+    // is complete, because the scores that it needs first, S(i + buffers) after P(i), are issued behind that phase.  With
+    // two score buffers that holds per buffer only: a warp can store P(i+1) while another has not stored P(i), so
+    // each buffer has a barrier of its own.  For dS: dP(i+1), which dS(i+1) needs, is issued behind dS(i) of all warps.
     reg_dealloc<kRegsService>();
     constexpr uint32_t idesc_s = make_idesc(1, BFmt<T>::code, 0, 0, kT, kT);
     constexpr uint32_t idesc_acc = make_idesc(1, BFmt<T>::code, 0, 1, kT, D);
@@ -690,7 +696,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       for (int i = 0; i < w.total && ok; ++i) {
         const int ps = pos + i;
         const bool more = i < last;
-        wq(&sh->p_ready, ps & 1, 45);
+        wq(&sh->p_ready[sbuf(ps)], sphase(ps), 45);
         if (!ok) break;
         mma_from_tmem<D, kHalfT>(tdV, tS + sbuf(ps) * 128, slotB(ps), idesc_acc, i > 0, leader);   // dV += P(i)^T dO(i)
         // (dO(i)'s other reader, dP(i), precedes in the pipe)
@@ -826,6 +832,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         PROF_T0();
 #endif
         if (!ok) break;
+        SKEW(warp, pos, 0);
         tc_fence_after();
 
         // ---- exp phase: P = exp2(score - lse), written back as T pairs ---------------------
@@ -926,7 +933,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         else run_exp(std::false_type{});
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(smem_u32(&sh->p_ready));
+        mbar_arrive(smem_u32(&sh->p_ready[sbuf(pos)]));
 #ifdef FA_PROF
         if (masked) { PROF_ADD(13); prof_acc[14] += 1; } else PROF_ADD(12);
 #endif
@@ -936,6 +943,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ok = bwait(&sh->dp_full, pos & 1, sh, 48);
         PROF_ADD(2);
         if (!ok) break;
+        SKEW(warp, pos, 1);
         PROF_T0();
         tc_fence_after();
         tmem_ld32(tdPx, r0);
@@ -973,6 +981,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       ok = bwait(&sh->dv_done, wi & 1, sh, 49);
       PROF_ADD(5);
       if (!ok) break;
+      SKEW(warp, wi, 2);
       tc_fence_after();
       PROF_T0();
       drain_acc<T, DH>(tdV + lane_addr + x * DH, 1.f, via_tma, slotB(pos - 1), lrow, x * DH, gdv);
@@ -983,6 +992,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_arrive(smem_u32(&sh->stg_ready[0]));
       ok = bwait(&sh->acc_done, wi & 1, sh, 49);
       if (!ok) break;
+      SKEW(warp, wi, 3);
       tc_fence_after();
       drain_acc<T, DH>(tdK + lane_addr + x * DH, cfg.scale, via_tma, slotA(pos - 1), lrow, x * DH, gdk);
       tc_fence_before();

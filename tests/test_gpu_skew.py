@@ -1,0 +1,87 @@
+"""Backward kernels whose element-wise warps are made to drift apart (csrc/skew.cuh, a build of its own): the gradients stay
+bit for bit those of the shipped build, whichever warps are late."""
+import hashlib
+import json
+import os
+import random
+import subprocess
+import sys
+
+import pytest
+import torch
+
+import cases
+from util import DEV
+
+pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "flash_attn_triton_b200")
+LIB = os.path.join(PKG, "libfa_b200_skew.so")
+
+CALLS = {                                        # several items of each kind per CTA
+    "causal": dict(B=12, Sq=400, Sk=400, causal=True),
+    "odd": dict(B=10, Sq=385, Sk=640),
+    "window": dict(B=8, Sq=700, Sk=700, window_size=(100, 30)),
+    "dropout": dict(B=12, Sq=512, Sk=512, causal=True, dropout_p=0.2),
+    "options": dict(B=12, Sq=384, Sk=384, causal=True, softcap=20.0, alibi=True, window_size=(200, 0)),
+    "packed": dict(lens=[1, 300, 128, 513, 64, 257, 400, 129, 700, 31, 256, 512] * 3, causal=True),
+}
+
+
+def gradients():
+    """Digests of dQ, dK, dV of every call."""
+    import flash_attn_triton_b200 as fa
+    from flash_attn_triton_b200 import _native as N
+    out = {}
+    for name, call in CALLS.items():
+        for D in (64, 128):
+            kw, H = dict(call), 8
+            slopes = torch.tensor([0.5 ** (i + 1) for i in range(H)], device=DEV) if kw.pop("alibi", False) else None
+            if "lens" in kw:
+                lens = kw.pop("lens")
+                q, k, v, do, cu, _ = cases.varlen_case(11 + D, lens, lens, H, H, D)
+                fn, extra = fa.flash_attn_varlen_func, (cu.to(DEV), cu.to(DEV), max(lens), max(lens))
+            else:
+                q, k, v, do = cases.dense_case(D, kw.pop("B"), kw.pop("Sq"), kw.pop("Sk"), H, H // 2, D)
+                fn, extra = fa.flash_attn_func, ()
+            ts = [t.to(DEV).requires_grad_() for t in (q, k, v)]
+            random.seed(3)                       # the dropout mask
+            grads = torch.autograd.grad(fn(*ts, *extra, alibi_slopes=slopes, **kw), ts, do.to(DEV))
+            for g, what in zip(grads, ("dq", "dk", "dv")):
+                assert torch.isfinite(g).all(), (name, D, what)
+                out[f"{name}-{D}-{what}"] = hashlib.sha256(g.cpu().numpy().tobytes()).hexdigest()
+    assert N.lib().fa_device_wait_status(0) == 0
+    return out
+
+
+def skewed():
+    from flash_attn_triton_b200 import _native as N
+    modes = {}
+    for mode in range(5):
+        assert N.lib().fa_debug_skew(mode) == 0
+        modes[mode] = gradients()
+    print("digests " + json.dumps(modes))
+
+
+def library():
+    """The build with delays, made where it is missing or older than a source."""
+    files = [os.path.join(PKG, "csrc", f) for f in os.listdir(os.path.join(PKG, "csrc"))]
+    if not os.path.exists(LIB) or os.path.getmtime(LIB) < max(map(os.path.getmtime, files)):
+        env = dict(os.environ, FA_BUILD_TAG="skew", FA_BUILD_DEFS="-DFA_SKEW")
+        subprocess.run([sys.executable, "-m", "flash_attn_triton_b200.build"], cwd=ROOT, env=env, check=True, timeout=900)
+
+
+def test_late_warps_do_not_change_gradients():
+    library()
+    r = subprocess.run([sys.executable, os.path.abspath(__file__)], capture_output=True, text=True, timeout=600,
+                       env=dict(os.environ, FA_B200_LIB=LIB, PYTHONPATH=os.pathsep.join(sys.path)))
+    assert r.returncode == 0, r.stdout + r.stderr
+    modes = json.loads(r.stdout.split("digests ", 1)[1])
+    want = gradients()
+    for mode, got in modes.items():
+        wrong = [n for n in want if got[n] != want[n]]
+        assert not wrong, (mode, wrong)
+
+
+if __name__ == "__main__":
+    skewed()
