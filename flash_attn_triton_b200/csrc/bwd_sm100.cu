@@ -1193,7 +1193,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           mma_commit_lp(smem_u32(&sh->s_full[(tg + 1) & 1]), leader);
           if (k + 1 == last) mma_commit_lp(smem_u32(&sh->res_free), leader);      // Q's last reader
         }
-        wq(&sh->ds_ready, tg & 1, 55);
+        wq(&sh->ds_ready, tg & 1, 55);                // (dP(k+1), which dS(k+1) needs, is issued behind this phase)
         if (!ok) break;
         mma_from_tmem<D, kHalfT>(tdQ, tdP, slotK(kpos), idesc_acc, k > 0, leader);        // dQ += dS(k) K(k)
         if (more) mma_commit_lp(smem_u32(&sh->empty_a[kpos % SK]), leader);       // (the epilogue releases the last)
@@ -1283,6 +1283,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         if (kDrop) keep2 = __ldg(reinterpret_cast<const uint2*>(cfg.keep + row * cfg.keep_words + (k0 >> 5)));
         ok = bwait(&sh->s_full[tg & 1], (tg >> 1) & 1, sh, 56);
         if (!ok) break;
+        SKEW(warp, tg, 0);
         tc_fence_after();
         uint32_t r0[32], r1[32];
         const uint32_t tSx = tS + (tg & 1) * kT + lane_addr + x * kHalfT;
@@ -1353,6 +1354,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // ---- dS phase --------------------------------------------------------------------
         ok = bwait(&sh->dp_full, tg & 1, sh, 57);
         if (!ok) break;
+        SKEW(warp, tg, 1);
         tc_fence_after();
         tmem_ld32(tdPx, r0);
         tmem_ld32(tdPx + 32, r1);
@@ -1390,6 +1392,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int spos = posA + w.total - 1;
       ok = bwait(&sh->acc_done, wi & 1, sh, 58);
       if (!ok) break;
+      SKEW(warp, wi, 2);
       tc_fence_after();
       const bool via_tma = (p.cu_seqlens_q == nullptr) || (w.m0 + kT <= w.g.q_len);
       const uint32_t stg = slotK(spos);
@@ -1403,7 +1406,9 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       posA += w.total;
       ++wi;
     }
-    // no more items: the store lane may leave
+    // No more items: the store lane may leave.  Between items the products of the next one wait for every warp, so that none
+    // arrives on stg_ready twice in a phase; here the warps wait for one another (all of them get here, whatever `ok` says).
+    asm volatile("bar.sync 1, 256;\n" ::: "memory");
     if (ok) {
       if (tid == 0) ok = post_store(sh, 0, wi, -1, 0, 0, 0, 0);
       mbar_arrive(smem_u32(&sh->stg_ready[0]));

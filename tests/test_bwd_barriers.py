@@ -119,6 +119,40 @@ def dkdv(items, buffers, p_barriers, rng):
     run([tensor_pipe(), issuer()] + [warp(w) for w in range(WARPS)], rng)
 
 
+def dq_results(items, last_waits, rng):
+    """Result tiles of the dQ kernel on their way to the store lane; `last_waits`: the warps wait for one another
+    before the message that ends it."""
+    ready, taken, products, last = Barrier(WARPS), Barrier(1), Barrier(WARPS), Barrier(WARPS)
+    staged, message = [-1] * WARPS, None
+
+    def store_lane():
+        for n in range(items + 1):
+            yield lambda: ready.done(n & 1)
+            need(message == n, f"message {message} instead of {n}")
+            need(n == items or min(staged) >= n, f"tile {n} stored before every warp has staged it")
+            taken.arrive()
+
+    def warp(w):
+        nonlocal message
+        for n in range(items + 1):
+            if n < items:
+                products.arrive()                # the item's products need dS of every warp
+                yield lambda: products.done(n & 1)
+                yield None
+            elif last_waits:
+                last.arrive()
+                yield lambda: last.done(0)
+            if w == 0:
+                if n > 0:
+                    yield lambda: taken.done((n - 1) & 1)
+                message = n
+            if n < items:
+                staged[w] = n
+            ready.arrive()
+
+    run([store_lane()] + [warp(w) for w in range(WARPS)], rng)
+
+
 ITEMS = [[5], [1, 1, 1, 1], [3, 2, 1], [2, 7]]
 
 
@@ -143,3 +177,17 @@ def test_the_model_sees_an_early_phase():
     with pytest.raises(Fault):
         for seed in range(400):
             dkdv([7], 2, 1, random.Random(seed))
+
+
+@pytest.mark.parametrize("items", [0, 1, 2, 5])
+def test_dq_results(items):
+    end = kernel_source().split("No more items: the store lane may leave")[-1]
+    last_waits = "bar.sync 1, 256" in end.split("post_store(sh, 0, wi, -1")[0]
+    for seed in range(100):
+        dq_results(items, last_waits, random.Random(seed))
+
+
+def test_the_model_sees_a_tile_stored_early():
+    with pytest.raises(Fault):
+        for seed in range(400):
+            dq_results(1, False, random.Random(seed))
