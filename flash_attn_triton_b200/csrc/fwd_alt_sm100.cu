@@ -196,15 +196,15 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   } else {
     packed = p.cu_seqlens_q != nullptr;
     int mt;
-    if (packed) {                                  // the tiles of the sequences one after the other, each for all heads
-      w.h = blockIdx.x % p.heads_q;
-      if (!packed_tile<kBM>(p, cfg.causal, blockIdx.x / p.heads_q, lane, w.b, mt)) return;
+    SeqInfo si;
+    if (packed) {
+      if (!packed_tile<kBM>(p, cfg, lane, w.h, w.b, si, mt)) return;
     } else {
       const int mtiles = (p.seqlen_q + kBM - 1) / kBM;
       dense_block(p, cfg, mtiles, w.b, w.h, mt);
       if (cfg.causal) mt = mtiles - 1 - mt;        // heavy tiles first
+      si = seq_info(p, w.b);
     }
-    const SeqInfo si = seq_info(p, w.b);
     w.hk = w.h / (p.heads_q / p.heads_kv);
     w.m0 = mt * kBM;
     w.rows = si.q_len;
@@ -894,7 +894,7 @@ static int launch_rows(const fa_attn_args& a, const ScoreCfg& plain, bool poly, 
     return FA_ERR_LAUNCH;
   }
   ScoreCfg cfg = plain;
-  const dim3 grid = packed ? dim3((unsigned)(packed_tiles<kBM>(a) * a.heads_q)) : dense_grid(a, (a.seqlen_q + kBM - 1) / kBM, cfg);
+  const dim3 grid = packed ? packed_grid<kBM>(a, cfg) : dense_grid(a, (a.seqlen_q + kBM - 1) / kBM, cfg);
   const CacheGeo geo = {};
   if constexpr (D == 256) {
     if (cfg.has_alibi || cfg.softcap > 0.f)

@@ -85,15 +85,15 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   int h, b, mt;
-  if (p.cu_seqlens_q != nullptr) {                 // the tiles of the sequences one after the other, each for all heads
-    h = blockIdx.x % p.heads_q;
-    if (!packed_tile<kBM>(p, cfg.causal, blockIdx.x / p.heads_q, lane, b, mt)) return;
+  SeqInfo si;
+  if (p.cu_seqlens_q != nullptr) {
+    if (!packed_tile<kBM>(p, cfg, lane, h, b, si, mt)) return;
   } else {
     const int mtiles = (p.seqlen_q + kBM - 1) / kBM;
     dense_block(p, cfg, mtiles, b, h, mt);
     if (cfg.causal) mt = mtiles - 1 - mt;          // heavy tiles first
+    si = seq_info(p, b);
   }
-  const SeqInfo si = seq_info(p, b);
   const int m0 = mt * kBM;
   if (m0 >= si.q_len) return;
   const int hk = h / (p.heads_q / p.heads_kv);
@@ -497,7 +497,7 @@ static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t
     return FA_ERR_LAUNCH;
   }
   ScoreCfg cfg = plain;
-  const dim3 grid = packed ? dim3((unsigned)(packed_tiles<kBM>(a) * a.heads_q)) : dense_grid(a, (a.seqlen_q + kBM - 1) / kBM, cfg);
+  const dim3 grid = packed ? packed_grid<kBM>(a, cfg) : dense_grid(a, (a.seqlen_q + kBM - 1) / kBM, cfg);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, host_wait_word(a.device));
   return check_launch("fwd_duo_sm100");
 }

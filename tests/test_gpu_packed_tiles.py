@@ -13,8 +13,10 @@ pytestmark = pytest.mark.gpu
 LENS = {
     "one": [130],
     "empty": [0, 256, 0, 0, 129, 1, 0],
-    "many": [(37 * i * i) % 300 for i in range(70)],       # two full scans of 32 and a remainder; some without a tile
+    "many": [(37 * i * i) % 300 for i in range(70)],       # the search takes three sequences per lane, then one; some without a tile
     "long_last": [1] * 33 + [513],
+    "same_length": [128] * 40,                              # an entry for each: nothing to search
+    "two_steps": [(7 * i) % 40 for i in range(1100)] + [300, 0, 129],
 }
 
 
