@@ -137,7 +137,10 @@ struct Tile {
 
 // kPoly > 0: every kPoly-th pair of exponentials of unmasked tiles on the FMA pipe, as in fwd_persist_sm100.cu.
 // kCache: K/V through the page table of a cache, query heads packed into rows, optional key pieces.
-template <typename T, int D, bool kExtras, bool kCache, int kPoly>
+// kGrid: the CTA's tile is its grid index (dense calls whose order does not matter, packed ones without a list); as one of
+// several ways in one kernel it took a CTA 0.2 us longer to start: 4096 packed sequences of 16 to 128, 8 heads of 256,
+// 2063 -> 2001 us.
+template <typename T, int D, bool kExtras, bool kCache, int kPoly, bool kGrid = false>
 __global__ void __launch_bounds__(kThreads, 1)
 fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
@@ -197,7 +200,12 @@ fwd_alt_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     packed = p.cu_seqlens_q != nullptr;
     int mt;
     SeqInfo si;
-    if (packed) {
+    if constexpr (kGrid) {
+      mt = cfg.causal ? gridDim.x - 1 - blockIdx.x : blockIdx.x;   // heavy tiles first
+      w.h = blockIdx.y;
+      w.b = blockIdx.z;
+      si = seq_info(p, w.b);
+    } else if (packed) {
       if (!packed_tile<kBM>(p, cfg, lane, w.h, w.b, si, mt)) return;
     } else {
       const int mtiles = (p.seqlen_q + kBM - 1) / kBM;
@@ -896,13 +904,16 @@ static int launch_rows(const fa_attn_args& a, const ScoreCfg& plain, bool poly, 
   ScoreCfg cfg = plain;
   const dim3 grid = packed ? packed_grid<kBM>(a, cfg) : dense_grid(a, (a.seqlen_q + kBM - 1) / kBM, cfg);
   const CacheGeo geo = {};
+  auto go = [&](auto kern) { return launch_alt(kern, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo); };
   if constexpr (D == 256) {
-    if (cfg.has_alibi || cfg.softcap > 0.f)
-      return launch_alt(fwd_alt_sm100_kernel<T, D, true, false, 0>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+    const bool extras = cfg.has_alibi || cfg.softcap > 0.f;
+    if (packed ? !cfg.packed_list : cfg.unit_group == 0)
+      return extras ? go(fwd_alt_sm100_kernel<T, D, true, false, 0, true>) : go(fwd_alt_sm100_kernel<T, D, false, false, 0, true>);
+    if (extras) return go(fwd_alt_sm100_kernel<T, D, true, false, 0>);
   } else if (poly) {
-    return launch_alt(fwd_alt_sm100_kernel<T, D, false, false, 4>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+    return go(fwd_alt_sm100_kernel<T, D, false, false, 4>);
   }
-  return launch_alt(fwd_alt_sm100_kernel<T, D, false, false, 0>, ACfg<D>::kSmemBytes, grid, st, tm, a, cfg, geo);
+  return go(fwd_alt_sm100_kernel<T, D, false, false, 0>);
 }
 
 int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStream_t st) {
