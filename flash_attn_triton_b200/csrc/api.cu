@@ -573,6 +573,14 @@ int fa_device_wait_clear(int device) {
   bwd_sm100_clear_status();
   fwd_alt_sm100_clear_status();
   fwd_duo_sm100_clear_status();
+  // a launch whose CTAs gave up has not put its pair of counters back to zero; the next one to get the pair would skip items
+  static const unsigned int zero[kWorkQueues][2] = {};
+  e = cudaMemcpyToSymbol(g_work_queues, zero, sizeof(zero));
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) {
+    set_error("clearing the work queues: %s", cudaGetErrorString(e));
+    return FA_ERR_LAUNCH;
+  }
   if (device >= 0 && device < 1024) g_host_wait[device] = 0;
   return FA_OK;
 }
@@ -589,6 +597,15 @@ int fa_mma_peak_probe(int32_t device, int32_t kind, int32_t iters, void* stream)
   if (int r = ensure_device(device)) return r;
   return mma_peak_probe(device, kind, iters, reinterpret_cast<cudaStream_t>(stream));
 }
+
+#ifdef FA_SKEW
+// Side build of the tests: the counters as launches whose CTAs gave up on a wait may leave them.
+int fa_debug_dirty_queues(unsigned int value) {
+  unsigned int pairs[kWorkQueues][2];
+  for (auto& pair : pairs) pair[0] = pair[1] = value;
+  return (int)cudaMemcpyToSymbol(g_work_queues, pairs, sizeof(pairs));
+}
+#endif
 
 int fa_debug_set_wait_status(int32_t device, int32_t code) {
   FA_REQUIRE(device >= 0 && device < 1024, "device ordinal out of range");

@@ -379,7 +379,8 @@ int fa_fwd_uses_tcgen05(const fa_attn_args* args);
  * until fa_device_wait_clear() is called.
  *
  * fa_device_wait_status: 0, or the code of the wait that ran out.  Synchronises the device.
- * fa_device_wait_clear:  synchronises, then puts the words of `device` back to zero.
+ * fa_device_wait_clear:  synchronises, then puts the words of `device`, and the counters that its launches hand out
+ *                        work with, back to zero.
  * fa_wait_probe:         launches ONE warp that waits, for at most `clocks` cycles, on a barrier
  *                        nothing ever arrives at (no copy or MMA in flight): exercises the
  *                        time-out path for bring-up and tests.  Leaves the status set (code 99).

@@ -63,6 +63,19 @@ def skewed():
     print("digests " + json.dumps(modes))
 
 
+def after_a_failed_wait():
+    """fa_device_wait_clear() also puts the counters of the work queues back to zero: a launch that gave up leaves them."""
+    from flash_attn_triton_b200 import _native as N
+    L = N.lib()
+    want = gradients()
+    assert L.fa_debug_dirty_queues(3) == 0 and L.fa_device_wait_clear(0) == 0
+    for _ in range(4):                           # more launches than there are queues
+        got = gradients()
+        wrong = [n for n in want if got[n] != want[n]]
+        assert not wrong, wrong
+    print("queues ok")
+
+
 def library():
     """The build with delays, made where it is missing or older than a source."""
     files = [os.path.join(PKG, "csrc", f) for f in os.listdir(os.path.join(PKG, "csrc"))]
@@ -71,17 +84,25 @@ def library():
         subprocess.run([sys.executable, "-m", "flash_attn_triton_b200.build"], cwd=ROOT, env=env, check=True, timeout=900)
 
 
-def test_late_warps_do_not_change_gradients():
+def child(what):
     library()
-    r = subprocess.run([sys.executable, os.path.abspath(__file__)], capture_output=True, text=True, timeout=600,
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), what], capture_output=True, text=True, timeout=600,
                        env=dict(os.environ, FA_B200_LIB=LIB, PYTHONPATH=os.pathsep.join(sys.path)))
     assert r.returncode == 0, r.stdout + r.stderr
-    modes = json.loads(r.stdout.split("digests ", 1)[1])
+    return r.stdout
+
+
+def test_late_warps_do_not_change_gradients():
+    modes = json.loads(child("skewed").split("digests ", 1)[1])
     want = gradients()
     for mode, got in modes.items():
         wrong = [n for n in want if got[n] != want[n]]
         assert not wrong, (mode, wrong)
 
 
+def test_queues_are_cleared_with_the_wait_status():
+    assert "queues ok" in child("after_a_failed_wait")
+
+
 if __name__ == "__main__":
-    skewed()
+    globals()[sys.argv[1]]()
