@@ -1,31 +1,46 @@
 """The forward with two CTAs per SM against the two-tile kernel: bit for bit the same, whatever the options, head groups,
-ragged ends and strides."""
+ragged ends and strides, dense and packed."""
 import random
 
 import pytest
 import torch
 
-from util import DEV
+import cases
+import util
+from oracle import attention_oracle as orc
+from util import DEV, maxdiff
 
 pytestmark = pytest.mark.gpu
 
-
-@pytest.mark.parametrize("kw", [
+OPTIONS = [
     dict(causal=True), dict(), dict(window_size=(150, 0)), dict(window_size=(60, 90)),
     dict(causal=True, softcap=20.0), dict(alibi=True), dict(causal=True, alibi=True, window_size=(200, -1)),
-    dict(causal=True, dropout_p=0.2), dict(dropout_p=0.1),
-], ids=str)
-@pytest.mark.parametrize("D", [64, 128])
-@pytest.mark.parametrize("Sq,Sk,Hkv,packed", [(400, 400, 16, True), (385, 640, 4, False)])
-def test_two_ctas_against_two_tiles(monkeypatch, kw, D, Sq, Sk, Hkv, packed):
-    import flash_attn_triton_b200 as fa
+]
+
+
+def enough_tiles(tiles, heads):
+    """More than 2.5 CTAs per SM: the calls that the rule of the kernel takes."""
+    return 2 * tiles * heads > 5 * torch.cuda.get_device_properties(0).multi_processor_count
+
+
+def slopes(kw):
     kw = dict(kw)
+    if kw.pop("alibi", False):
+        kw["alibi_slopes"] = torch.tensor([0.5 ** (i + 1) for i in range(16)], device=DEV)
+    return kw
+
+
+@pytest.mark.parametrize("kw", OPTIONS + [dict(causal=True, dropout_p=0.2), dict(dropout_p=0.1)], ids=str)
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("Sq,Sk,Hkv", [(400, 400, 16), (385, 640, 4)])
+def test_two_ctas_against_two_tiles(monkeypatch, kw, D, Sq, Sk, Hkv):
+    import flash_attn_triton_b200 as fa
+    assert enough_tiles(10 * -(-Sq // 128), 16)
+    kw = slopes(kw)
     g = torch.Generator(DEV).manual_seed(D)
     q = torch.randn(10, Sq, 16, D, device=DEV, dtype=torch.half, generator=g)
     kv = torch.randn(10, Sk, 2, Hkv, D, device=DEV, dtype=torch.half, generator=g)      # k and v: slices of one tensor
     k, v = kv[:, :, 0], kv[:, :, 1]
-    if kw.pop("alibi", False):
-        kw["alibi_slopes"] = torch.tensor([0.5 ** (i + 1) for i in range(16)], device=DEV)
 
     def run():
         random.seed(3)                                                                   # the dropout mask
@@ -34,3 +49,33 @@ def test_two_ctas_against_two_tiles(monkeypatch, kw, D, Sq, Sk, Hkv, packed):
     got = run()
     monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
     assert torch.equal(got, run())
+
+
+@pytest.mark.parametrize("kw", OPTIONS, ids=str)
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_packed_two_ctas(monkeypatch, kw, D, dtype):
+    """Empty and one-token sequences, ends inside and on the edge of a tile, and a neighbour full of NaN and infinities."""
+    import flash_attn_triton_b200 as fa
+    lens = [400, 0, 1, 385, 130, 300, 129, 256, 17, 511] * 3
+    assert enough_tiles(sum(lens) // 128 + len(lens) // 2, 16)
+    q, k, v, _, cu, _ = cases.varlen_case(7 + D, lens, lens, 16, 4, D)
+    q, k, v = (t.to(dtype) for t in (q, k, v))
+    opts = slopes(kw)
+    run = lambda k, v: fa.flash_attn_varlen_func(q.to(DEV), k.to(DEV), v.to(DEV), cu.to(DEV), cu.to(DEV), max(lens), max(lens), **opts)
+    got = run(k, v)
+    bad = slice(int(cu[4]), int(cu[5]))                                                  # the 130 tokens after the 385
+    kb, vb = k.clone(), v.clone()
+    kb[bad], vb[bad] = float("nan"), float("inf")
+    beside = run(kb, vb)
+    assert torch.equal(beside[:bad.start], got[:bad.start]) and torch.equal(beside[bad.stop:], got[bad.stop:])
+    ref = dict(kw)
+    ref["window"] = ref.pop("window_size", (-1, -1))
+    ref["alibi_slopes"] = opts["alibi_slopes"].cpu() if ref.pop("alibi", False) else None
+    for b in range(len(lens) // 3):
+        if lens[b]:
+            r = slice(int(cu[b]), int(cu[b + 1]))
+            want, _ = orc.attention_ref(q[None, r], k[None, r], v[None, r], **ref)
+            assert maxdiff(got[r], want[0]) <= util.tols(dtype)[0], b
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    assert torch.equal(got, run(k, v))
