@@ -366,7 +366,7 @@ def decode_bench(dev, peaks, iters=20, batch_lo=0, batch_hi=64):
 def profile_case(args):
     """Small cases for ncu captures (a few hundred MB on the device, more than the 126 MB L2), W+K
     steps of one kernel family each:
-      dense     forward + backward, B2 H16 S4096 D128 causal (per-CTA dK/dV kernel)
+      dense     forward + backward, B2 H16 S4096 D128 causal
       dense_nc  the same without the mask (persistent dK/dV kernel)
       varlen    8 packed sequences, H8 D128, causal + window 1024 + ALiBi + soft cap (feature variants)
       decode    16 sequences of the paged-decode workload

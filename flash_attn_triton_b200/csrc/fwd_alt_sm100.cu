@@ -75,6 +75,9 @@ struct AShared {
   uint64_t kv_full[kMaxStages];
   uint64_t kv_empty[kMaxStages];
   uint64_t s_full[3];      // [buffer]: scores computed
+  // (Barriers that count threads: none may arrive for a phase before the one ahead of it is complete.  For P: the next scores
+  // of the same buffer are issued behind its p_ready.  For `decided`: a group settles tile j + 2 after the other group's
+  // tile j + 1, which each of that group's threads settled after tile j was settled by all.)
   uint64_t p_half[3];      // [buffer]: the first 64 keys of P written back (128 arrivals)
   uint64_t p_ready[3];     // [buffer]: P written back (128 arrivals)
   uint64_t o_done[3];      // [buffer]: its P V finished

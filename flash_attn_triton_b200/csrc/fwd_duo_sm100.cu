@@ -49,6 +49,8 @@ struct DShared {
   uint64_t kv_full[4];
   uint64_t kv_empty[4];
   uint64_t s_full;         // scores computed
+  // (Barriers that count threads: none may arrive for a phase before the one ahead of it is complete.  For P: the next
+  // scores, which a thread needs first, are issued behind p_ready.)
   uint64_t p_half;         // the first 64 keys of P written back (128 arrivals)
   uint64_t p_ready;        // P written back (128 arrivals)
   uint64_t o_ready;        // the latest P V finished

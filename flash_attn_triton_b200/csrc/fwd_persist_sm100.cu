@@ -58,6 +58,8 @@ struct PShared {
   uint64_t kv_full[kMaxStages];
   uint64_t kv_empty[kMaxStages];
   uint64_t s_full[2];            // [stream]: its score tile computed
+  // (Barriers that count threads: none may arrive for a phase before the one ahead of it is complete.  For P: the next
+  // scores of the stream are issued behind its p_ready.  For o_seen: the producer frees the next entry behind it.)
   uint64_t p_ready[2];           // [stream]: P written back (128 arrivals)
   uint64_t p_half[2];            // [stream]: the first 64 keys of P written back (128 arrivals)
   uint64_t o_ready[2];           // [stream]: its latest P V finished

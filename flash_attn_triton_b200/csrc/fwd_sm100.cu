@@ -82,6 +82,8 @@ struct Shared {
   uint64_t kv_full[kMaxStages];
   uint64_t kv_empty[kMaxStages];
   uint64_t s_full[2];      // [stream]: its score tile computed
+  // (Barriers that count threads: none may arrive for a phase before the one ahead of it is complete.  For P: the next
+  // scores of the stream are issued behind its p_ready.  For sk_empty: the slot is written again behind it.)
   uint64_t p_ready[2];     // [stream]: P written back (128 arrivals)
   uint64_t p_half[2];      // [stream]: the first 64 keys of P written back (128 arrivals)
   uint64_t o_ready[2];     // [stream]: its latest P V finished
@@ -816,7 +818,8 @@ static int launch(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st,
   return check_launch("fwd_sm100");
 }
 
-// Two kernels.  The persistent one (fwd_persist_sm100.cu) takes the calls with long work items:
+// Four kernels: two for the calls that their rules below take (fwd_duo_sm100.cu, fwd_alt_sm100.cu), and two for the
+// rest.  Of these the persistent one (fwd_persist_sm100.cu) takes the calls with long work items:
 // measured with launches interleaved on one GPU it is 3-4 % faster at 4096-8192 keys (dense, GQA
 // and the packed workload) and 9 % slower at 1024 keys, where an item is four or five steps and
 // the hand-over between items costs more than a fresh CTA.  This file keeps the one-CTA-per-item
@@ -892,7 +895,7 @@ int fwd_sm100(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
   if (a.head_dim == 256 || a.seqlen_k < 256 || cfg.keep != nullptr) cfg.rescale_at = 0.f;
   if (a.head_dim == 256) return fwd_alt_sm100(a, cfg, false, st);
   // FA_B200_FWD_PERSISTENT_FROM in the environment overrides the threshold (tests run the
-  // persistent kernel on small shapes with it; 0 = never)
+  // persistent kernel on small shapes with it; 0 = never) and keeps the other two kernels off
   int from = FA_FWD_PERSISTENT_FROM;
   const char* e = getenv("FA_B200_FWD_PERSISTENT_FROM");
   if (e != nullptr) {
