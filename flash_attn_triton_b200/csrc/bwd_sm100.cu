@@ -40,8 +40,8 @@
 //                     S^T, P^T [0] | S^T, P^T [1] | dP^T, dS^T | dV (64) | dK (64).
 // What it measured, against the two kernels it replaced (one with S and dP in turns in one region, one with a CTA per
 // key block): 32 packed sequences of 256 to 4096 tokens with window, ALiBi and soft cap 3610 -> 3045 us; 16 x 16 heads
-// x 4096 tokens of 128, causal, 1980 -> 1880 us (3.3 k cycles per tile instead of 4.2 k, of which the
-// power limit gives most back); 4 x 32 heads x 1024 x 1531 of 64 171 -> 141 us.
+// x 4096 tokens of 128, causal, unchanged within calls (3.3 k cycles per tile instead of 4.2 k; the power limit
+// gives it back); 4 x 32 heads x 1024 x 1531 of 64 171 -> 141 us.
 // TMEM, dQ kernel:    S[0] | S[1] | dP | dQ    (4 x 128 columns).
 // All operand tiles are written by TMA with the 128-byte swizzle; the same tile is read
 // K-major (contraction over head_dim) or MN-major (contraction over its rows) through
@@ -127,6 +127,7 @@ struct BShared {
   uint64_t sched_full[kSched];   // work-queue entry published by the producer thread
   uint64_t sched_empty[kSched];  // ... read by every consuming warp
   int4 sched_item[kSched][3];    // the item, decoded once by the producer thread (KItem / QItem)
+  // (dK/dV: every warp has seen the previous item's tiles taken; dQ: see the end of its element-wise groups)
   uint64_t stg_ready[2];  // result tile of an item staged for the store lane (and its message written); dK/dV: dV, dK
   uint64_t stg_taken[2];  // [group] the store lane has read the message; dK/dV: [0], both tiles seen by the agent
   // [group] message to the store lane: shared-memory address of the staged tile (0 = nothing to
@@ -1482,14 +1483,15 @@ bool candidate_count(int64_t blocks, int64_t heads, int64_t batch, int* out) {
   return true;
 }
 
-ScoreCfg with_order(const fa_attn_args& a, const ScoreCfg& cfg, int heads, int blocks) {
+// Q, dO, K and V of a group: 64 MB.  dQ and dK/dV together without groups, in groups of 16, 32, 64 and 96 MB (us), causal:
+// 16 x 16 x 4096 of 128 3964, 3973, 3954, 3869, 3854; 16 x 16 x 2048 of 64 836, 740, 725, 717, 717; 64 x 16 x 512 of 64
+// 438, 366, 357, 356, 358; 1 x 16 x 8192 of 128 972, 897, 881, 877, 880; window of 200, 16 x 16 x 2048 of 64 446, 388, 382, 377, 377;
+// 48 packed sequences of 64 to 4096, 16 heads of 128 4655, 4576, 4488, 4461, 4510.
+ScoreCfg with_order(const fa_attn_args& a, const ScoreCfg& cfg, int heads) {
   const bool packed = a.cu_seqlens_q != nullptr;
   const int64_t q = packed ? a.total_q : (int64_t)a.batch * a.seqlen_q, k = packed ? a.total_k : (int64_t)a.batch * a.seqlen_k;
   ScoreCfg c = cfg;
-  // with many blocks per SM the last ones weigh little, and groups cost (16 x 16 heads x 4096: dQ 1325 -> 1359 us, dK/dV
-  // 1913 -> 1929 in groups of 16; the forwards do not mind)
-  if (!packed && (int64_t)a.batch * heads * blocks > 16 * (int64_t)sm_count(a.device)) c.unit_group = 1;
-  else c.unit_group = unit_group(a, cfg, heads, 4 * a.head_dim * (q * a.heads_q + k * a.heads_kv));
+  c.unit_group = unit_group(a, cfg, heads, 4 * a.head_dim * (q * a.heads_q + k * a.heads_kv), (int64_t)64 << 20);
   return c;
 }
 
@@ -1518,7 +1520,7 @@ int launch_dkdv(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   unsigned int* queue = work_queue(a.device);
   if (queue == nullptr) return FA_ERR_LAUNCH;
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
-  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytes, st>>>(m.q, m.k, m.v, m.dout, m.dk, m.dv, a, with_order(a, cfg, a.heads_kv, nkb), nkb, ncand, queue,
+  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytes, st>>>(m.q, m.k, m.v, m.dout, m.dk, m.dv, a, with_order(a, cfg, a.heads_kv), nkb, ncand, queue,
                                                            host_wait_word(a.device));
   return check_launch("bwd_dkdv_sm100");
 }
@@ -1544,7 +1546,7 @@ int launch_dq(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   unsigned int* queue = work_queue(a.device);
   if (queue == nullptr) return FA_ERR_LAUNCH;
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
-  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytesDq, st>>>(m.q, m.k, m.v, m.dout, m.dq, a, with_order(a, cfg, a.heads_q, nmb), nmb, ncand, queue,
+  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytesDq, st>>>(m.q, m.k, m.v, m.dout, m.dq, a, with_order(a, cfg, a.heads_q), nmb, ncand, queue,
                                                              host_wait_word(a.device));
   return check_launch("bwd_dq_sm100");
 }

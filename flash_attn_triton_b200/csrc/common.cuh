@@ -536,25 +536,29 @@ __device__ __forceinline__ void block_of(int c, int blocks, int units, int group
   block = r / n;
   unit = first + r % n;
 }
-// Units per group: what they read again and again stays in half of the L2.  Blocks of one size have no order to keep.  In
-// packed batches groups also bring the blocks that lie outside their sequences together, where all SMs skip them at once.
-inline int unit_group(const fa_attn_args& a, const ScoreCfg& cfg, int heads, int64_t bytes) {
+// Units per group: groups of one size (a last group of one unit brings back its light blocks at the end: 1 x 16 heads x 8192 of
+// 128, where 15 fitted, 277 -> 300 us by the order it should have gained from), as few as what their units read again and
+// again allows.  Blocks of one size have no order to keep.  In packed batches groups also bring the blocks that lie outside their
+// sequences together, where all SMs skip them at once.
+inline int unit_group(const fa_attn_args& a, const ScoreCfg& cfg, int heads, int64_t bytes, int64_t limit) {
   const int64_t units = (int64_t)a.batch * heads;
   if (!cfg.causal || units <= 1) return 1;
-  const int64_t n = ((int64_t)64 << 20) / (bytes / units + 1);
-  return (int)(n < 1 ? 1 : n < units ? n : units);
+  const int64_t groups = bytes > limit ? (bytes + limit - 1) / limit : 1;
+  return (int)((units + groups - 1) / groups);
 }
 
+// Keys and values of a group: 32 MB.  Without groups, 16, 32 and 64 MB (us): 1 x 16 x 8192 of 128 277, 263, 264, 263;
+// 8 x 16 x 2048 of 128 209, 194, 197, 190; 64 x 16 x 512 of 128 179, 174, 174, 181; 32 x 16 x 256 of 256 84, 82, 85, 89.
 inline int fwd_unit_group(const fa_attn_args& a, const ScoreCfg& cfg) {
   const int64_t keys = a.cu_seqlens_q != nullptr ? a.total_k : (int64_t)a.batch * a.seqlen_k;
-  return unit_group(a, cfg, a.heads_q, 4 * keys * a.heads_kv * a.head_dim);
+  return unit_group(a, cfg, a.heads_q, 4 * keys * a.heads_kv * a.head_dim, (int64_t)32 << 20);
 }
 
 // The same for a kernel with one CTA per block of a dense call: where the order does not matter (blocks of one size, or a
 // CTA for each at once) the grid has three dimensions and unit_group is 0, which saves the divisions (0.3 us).
 inline dim3 dense_grid(const fa_attn_args& a, int blocks, ScoreCfg& cfg) {
   const int64_t all = (int64_t)blocks * a.heads_q * a.batch;
-  cfg.unit_group = fwd_unit_group(a, cfg);
+  cfg.unit_group = blocks == 1 ? 1 : fwd_unit_group(a, cfg);
   if ((cfg.unit_group == 1 || all <= sm_count(a.device)) && a.heads_q <= 65535 && a.batch <= 65535) {
     cfg.unit_group = 0;
     return dim3(blocks, a.heads_q, a.batch);
