@@ -41,7 +41,7 @@
 // What it measured, against the two kernels it replaced (one with S and dP in turns in one region, one with a CTA per
 // key block): 32 packed sequences of 256 to 4096 tokens with window, ALiBi and soft cap 3610 -> 3045 us; 16 x 16 heads
 // x 4096 tokens of 128, causal, unchanged within calls (3.3 k cycles per tile instead of 4.2 k; the power limit
-// gives it back); 4 x 32 heads x 1024 x 1531 of 64 171 -> 141 us.
+// gives it back); 4 x 32 heads x 1024 x 1531 of 64 171 -> 139 us.
 // TMEM, dQ kernel:    S[0] | S[1] | dP | dQ    (4 x 128 columns).
 // All operand tiles are written by TMA with the 128-byte swizzle; the same tile is read
 // K-major (contraction over head_dim) or MN-major (contraction over its rows) through
@@ -92,7 +92,7 @@ template <int D> struct BCfg {
   static constexpr int kSmemTiles = (2 + kStagesQ + kStagesO) * kTileBytes;
   // head_dim 64 leaves tensor-memory columns for a second score buffer.  The element-wise warps then find their scores
   // ready (they waited 0.4 k of 2.3 k cycles per tile for them, or, with P and dS in columns of their own instead, spent
-  // as much on four more barriers): 4 x 32 heads x 1024 x 1531 153 -> 141 us, 2 x 16 over 4 heads x 1024, causal, 50 -> 45.
+  // as much on four more barriers): 4 x 32 heads x 1024 x 1531 153 -> 139 us, 2 x 16 over 4 heads x 1024, causal, 50 -> 46.
   // (Tried with those columns: one group half a tile behind the other, so that their exponentials do not meet, 4 % slower.)
   static constexpr int kSBuf = D == 64 ? 2 : 1;
   // dK/dV kernel: 128 x 16 operand tiles that carry the row statistics into the GEMMs
