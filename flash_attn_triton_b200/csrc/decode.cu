@@ -22,6 +22,12 @@
 //   Merge.  A unit of one piece is written straight to the output.  Otherwise its pieces go to
 //   the workspace with their base-2 LSEs and the CTA that finishes last merges them, always in the
 //   same order.
+//   Latency.  A small step is one chain: lengths, piece, tiles and Q, the append, the merge of the warps, the merge of the
+//   pieces.  So Q and the new tokens are read and rotated 16 bytes at a time (they came element by element), what the
+//   append reads is fetched to L1 under the first tiles, the warps write their outputs side by side and add them up after
+//   one barrier (not in four turns), and sixteen pieces are merged per trip to L2.  Kernel time, before -> after (us):
+//   1 x 1900 tokens, 32 heads over 8 of 128: 15.2 -> 12.2; 28 x 66 to 2112, 8 over 2: 20.0 -> 15.9; 47 x 192, 2 new tokens, 32
+//   over 8 of 64: 22.6 -> 17.1; 4 x 600 to 2400, 4 new tokens, 16 over 4 of 128: 34.7 -> 21.1; 17 x 18450, 8 over 2: 68.9 -> 63.5.
 //   Value checks of the public call run at the start of the same kernel while the tables are small (one
 //   decode step of a few sequences is bounded by launches: 17 small kernels, a copy and a
 //   synchronisation took 150 us around a 16 us kernel), in decode_check_kernel otherwise.
@@ -134,6 +140,32 @@ __device__ __forceinline__ T rotary_elem(F get, int d, const T* cos, const T* si
   return first ? hsub_rn(hmul_rn(x, c), hmul_rn(y, s)) : hadd_rn(hmul_rn(y, s), hmul_rn(x, c));
 }
 
+// 8 elements of a head row, rotated like rotary_elem.
+template <typename T>
+__device__ __forceinline__ uint4 rotary_chunk(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
+                                              int interleaved, int rotary_seqlen) {
+  union { uint4 v; T e[8]; } out, self, other, c, s;
+  self.v = *reinterpret_cast<const uint4*>(x + d);
+  if (cos == nullptr || d >= rotary_dim || pos < 0 || pos >= rotary_seqlen) return self.v;
+  const int half = rotary_dim >> 1;
+  if (!interleaved && half % 8 == 0 && ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 15) == 0) {
+    const bool first = d < half;
+    const int i = first ? d : d - half;
+    other.v = *reinterpret_cast<const uint4*>(x + (first ? d + half : d - half));
+    c.v = *reinterpret_cast<const uint4*>(cos + (int64_t)pos * half + i);
+    s.v = *reinterpret_cast<const uint4*>(sin + (int64_t)pos * half + i);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      out.e[k] = first ? hsub_rn(hmul_rn(self.e[k], c.e[k]), hmul_rn(other.e[k], s.e[k]))
+                       : hadd_rn(hmul_rn(other.e[k], s.e[k]), hmul_rn(self.e[k], c.e[k]));
+    return out.v;
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    out.e[k] = rotary_elem<T>([&](int j) { return x[j]; }, d + k, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+  return out.v;
+}
+
 __device__ __forceinline__ int64_t cache_row_offset(const fa_decode_args& p, int b, int pos,
                                                     int page_shift, const int64_t* stride) {
   int page, row;
@@ -182,18 +214,19 @@ __device__ __forceinline__ SeqTiles seq_tiles(const fa_decode_args& p, const Sco
   return s;
 }
 
-// Elements [d, d + 4) of one output row, merged from the `parts` workspace rows r0, r0 + step, ...  Eight
-// pieces are loaded at a time, their common maximum taken first.
+// Elements [d, d + 4) of one output row, merged from the `parts` workspace rows r0, r0 + step, ...  Sixteen
+// pieces are loaded at a time (a small step seldom has more: one trip to L2), their common maximum taken first.
+constexpr int kMergeBatch = 16;
 template <typename T, int D>
 __device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_l, int64_t r0, int64_t step, int parts, int d,
                                              T* og) {
   float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
   float wsum = 0.f, m = -INFINITY;
-  for (int i0 = 0; i0 < parts; i0 += 8) {
-    float l[8];
-    float4 x[8];
+  for (int i0 = 0; i0 < parts; i0 += kMergeBatch) {
+    float l[kMergeBatch];
+    float4 x[kMergeBatch];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < kMergeBatch; ++j) {
       const int i = i0 + j;
       const int64_t r = r0 + i * step;
       l[j] = i < parts ? ws_l[r] : -INFINITY;
@@ -201,7 +234,7 @@ __device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_
     }
     float mn = m;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) mn = fmaxf(mn, l[j]);
+    for (int j = 0; j < kMergeBatch; ++j) mn = fmaxf(mn, l[j]);
     // pieces without a finite score weigh 0, which a NaN in them survives
     const float mf = mn == -INFINITY ? 0.f : mn;
     const float sc = exp2f(m - mf);
@@ -209,7 +242,7 @@ __device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_
     wsum *= sc;
     m = mn;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
+    for (int j = 0; j < kMergeBatch; ++j) {
       const float w = exp2f(l[j] - mf);
       wsum += w;
       acc.x += w * x[j].x; acc.y += w * x[j].y; acc.z += w * x[j].z; acc.w += w * x[j].w;
@@ -232,9 +265,9 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
 template <int D, int kRows> struct DecodeSmem {
   static constexpr int P = TilePitch<D>::value, NS = 3, OP = D + 4;
   static constexpr size_t ring = (size_t)2 * NS * kTile * P * 2;
-  static constexpr size_t q_bytes = kRows * P * 2, o_bytes = kRows * OP * 4;
-  static constexpr size_t merge = q_bytes > o_bytes ? q_bytes : o_bytes;   // Q rows, later the merged output of the warps
-  static constexpr size_t fixed = ring + merge + 4 * kRows * 2 * 4;       // + each warp's row maxima and sums
+  static constexpr size_t q_bytes = kRows * P * 2;
+  static constexpr size_t fixed = ring + q_bytes + 4 * kRows * 2 * 4;     // Q rows; each warp's row maxima and sums
+  static_assert((size_t)4 * kRows * OP * 4 <= ring, "the warps' outputs, over the ring");
 };
 
 template <typename T, int D, int kRows>
@@ -245,9 +278,9 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
   constexpr int CPR = D / 8, RPW = 32 / CPR, PASSES = 16 / RPW;     // a warp's loads: 16 rows of CPR 16-byte chunks
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* ring = reinterpret_cast<T*>(smem_raw);      // [stage][warp][K, V][16][P]
-  T* sQ = reinterpret_cast<T*>(smem_raw + SM::ring);                       // kRows x P, and over it
-  float* sO = reinterpret_cast<float*>(sQ);      // kRows x OP
-  float* sM = reinterpret_cast<float*>(smem_raw + SM::ring + SM::merge);   // 4 x kRows
+  float* sO = reinterpret_cast<float*>(smem_raw); // over the ring, when it is done with: 4 x kRows x OP
+  T* sQ = reinterpret_cast<T*>(smem_raw + SM::ring);                       // kRows x P
+  float* sM = reinterpret_cast<float*>(smem_raw + SM::ring + SM::q_bytes); // 4 x kRows
   float* sL = sM + 4 * kRows;                    // 4 x kRows
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
@@ -411,24 +444,40 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
   const T* sin = reinterpret_cast<const T*>(p.rotary_sin);
   int stage = 0;
 
+  // What the append of this piece's new tokens will read, on its way to L1 meanwhile: it is the last thing that the piece
+  // with the end of the sequence does, and a small step waits for that piece.
+  if (p.k_new && (tile0 + count) * kTile > len_old) {
+    const int from = max(len_old, tile0 * kTile), n = min(min(len, (tile0 + count) * kTile) - from, 8);
+    for (int i = tid; i < n * 4; i += NT) {
+      const int key = from + (i >> 2), tok = key - len_old, what = i & 3;
+      const char* a = nullptr;
+      int bytes = D * 2;
+      if (what == 0) a = reinterpret_cast<const char*>(reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + hk * p.kn_stride[2]);
+      if (what == 1) a = reinterpret_cast<const char*>(reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + hk * p.vn_stride[2]);
+      if (what >= 2 && cos && key + pad < p.rotary_seqlen) {
+        bytes = p.rotary_dim;
+        a = reinterpret_cast<const char*>((what == 2 ? cos : sin) + (int64_t)(key + pad) * (p.rotary_dim >> 1));
+      }
+      if (a != nullptr)
+        for (int o = 0; o < bytes; o += 128) asm volatile("prefetch.global.L1 [%0];" ::"l"(a + o));
+    }
+  }
+
   // Q rows (rotary fused) -> shared memory -> B fragments held in registers
-#pragma unroll 4
-  for (int i = tid; i < kRows * D; i += NT) {
-    const int r = i / D, d = i % D;
+#pragma unroll
+  for (int i0 = 0; i0 < kRows * CPR; i0 += NT) {
+    const int i = i0 + tid;
+    if (kRows * CPR % NT != 0 && i >= kRows * CPR) break;
+    const int r = i / CPR, d = i % CPR * 8;
     const int gr = rg * kRows + r;
-    T val = Elem<T>::from_f(0.f);
+    uint4 val = make_uint4(0u, 0u, 0u, 0u);
     if (gr < R) {
       const int sq = gr / G, gi = gr % G;
       const T* qrow = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + sq * p.q_stride[1] +
                       (int64_t)(hk * G + gi) * p.q_stride[2];
-      if (cos) {
-        val = rotary_elem<T>([&](int j) { return qrow[j]; }, d, cos, sin, len - p.seqlen_q + sq + pad, p.rotary_dim,
-                             p.rotary_interleaved, p.rotary_seqlen);
-      } else {
-        val = qrow[d];
-      }
+      val = rotary_chunk<T>(qrow, d, cos, sin, len - p.seqlen_q + sq + pad, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
     }
-    sQ[r * P + d] = val;
+    *reinterpret_cast<uint4*>(sQ + r * P + d) = val;
   }
   __syncthreads();
   uint32_t bq[NB][D / 16][2];
@@ -485,23 +534,20 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
     // ---- append: new tokens among these keys, rotated, into the staged rows and the cache ----
     const int nfirst = max(keyw, len_old), nlast = min(keyw + 16, len);   // new keys [nfirst, nlast)
     if (nlast > nfirst) {
-#pragma unroll 4
-      for (int i = lane; i < (nlast - nfirst) * D; i += 32) {
-        const int key = nfirst + i / D, d = i % D;
+      for (int i = lane; i < (nlast - nfirst) * CPR; i += 32) {
+        const int key = nfirst + i / CPR, d = i % CPR * 8;
         const int tok = key - len_old, pos = key + pad;
         const T* kn = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + hk * p.kn_stride[2];
         const T* vn = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + hk * p.vn_stride[2];
-        T kv = kn[d];
-        if (cos) kv = rotary_elem<T>([&](int j) { return kn[j]; }, d, cos, sin, pos, p.rotary_dim,
-                                     p.rotary_interleaved, p.rotary_seqlen);
-        const T vv = vn[d];
-        tK[(key - keyw) * P + d] = kv;
-        tV[(key - keyw) * P + d] = vv;
+        const uint4 vv = *reinterpret_cast<const uint4*>(vn + d);
+        const uint4 kv = rotary_chunk<T>(kn, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+        *reinterpret_cast<uint4*>(tK + (key - keyw) * P + d) = kv;
+        *reinterpret_cast<uint4*>(tV + (key - keyw) * P + d) = vv;
         if (rg == 0 && pos < cache_capacity(p)) {
-          reinterpret_cast<T*>(p.k_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.kc_stride) +
-                                          (int64_t)hk * p.kc_stride[2] + d] = kv;
-          reinterpret_cast<T*>(p.v_cache)[cache_row_offset(p, b, pos, geo.page_shift, p.vc_stride) +
-                                          (int64_t)hk * p.vc_stride[2] + d] = vv;
+          *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.k_cache) + cache_row_offset(p, b, pos, geo.page_shift, p.kc_stride) +
+                                    (int64_t)hk * p.kc_stride[2] + d) = kv;
+          *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.v_cache) + cache_row_offset(p, b, pos, geo.page_shift, p.vc_stride) +
+                                    (int64_t)hk * p.vc_stride[2] + d) = vv;
         }
       }
       __syncwarp();
@@ -593,7 +639,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
     }
   }
 
-  // ---- merge the 4 warps (each saw a quarter of every tile), one after the other into sO ------
+  // ---- merge the 4 warps (each saw a quarter of every tile) -----------------------------------
 #pragma unroll
   for (int n = 0; n < NB; ++n) {
 #pragma unroll
@@ -619,24 +665,16 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
       wgt[n][i] = (mstar == -INFINITY) ? 0.f : exp2f(mrow[n][i] - mstar);
     }
   }
-#pragma unroll 1
-  for (int turn = 0; turn < 4; ++turn) {
-    if (warp == turn) {
 #pragma unroll
-      for (int n = 0; n < NB; ++n) {
+  for (int n = 0; n < NB; ++n) {
 #pragma unroll
-        for (int db = 0; db < D / 16; ++db) {
+    for (int db = 0; db < D / 16; ++db) {
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float* x = sO + (n * 8 + 2 * t + (e & 1)) * OP + db * 16 + g + (e >> 1) * 8;
-            const float v = wgt[n][e & 1] * o[n][db][e];
-            *x = turn > 0 ? *x + v : v;
-          }
-        }
-      }
+      for (int e = 0; e < 4; ++e)
+        sO[(warp * kRows + n * 8 + 2 * t + (e & 1)) * OP + db * 16 + g + (e >> 1) * 8] = wgt[n][e & 1] * o[n][db][e];
     }
-    __syncthreads();
   }
+  __syncthreads();
 
   // ---- output, or a piece of it -----------------------------------------------------------
   // workspace: the R query rows of every (piece, kv head), not padded to units
@@ -652,6 +690,11 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
       for (int wv = 0; wv < 4; ++wv) lsum += exp2f(sM[wv * kRows + r] - mstar) * sL[wv * kRows + r];
     }
     float4 acc = *reinterpret_cast<const float4*>(sO + r * OP + c4);
+#pragma unroll
+    for (int wv = 1; wv < 4; ++wv) {
+      const float4 x = *reinterpret_cast<const float4*>(sO + (wv * kRows + r) * OP + c4);
+      acc.x += x.x; acc.y += x.y; acc.z += x.z; acc.w += x.w;
+    }
     const float inv = lsum > 0.f ? 1.f / lsum : 0.f;
     acc.x *= inv; acc.y *= inv; acc.z *= inv; acc.w *= inv;
     const int sq = gr / G, h = hk * G + gr % G;
@@ -710,32 +753,6 @@ static int decode_row_groups(const fa_decode_args& a) {
 // rows; these calls append and rotate in a kernel of their own and attend on the tensor cores
 // (fwd_alt_sm100.cu), which takes about as long for 128 rows as the kernel above for 16.
 // ---------------------------------------------------------------------------------------
-// 8 elements of a head row, rotated like rotary_elem.
-template <typename T>
-__device__ __forceinline__ uint4 rotary_chunk(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
-                                              int interleaved, int rotary_seqlen) {
-  union { uint4 v; T e[8]; } out, self, other, c, s;
-  self.v = *reinterpret_cast<const uint4*>(x + d);
-  if (cos == nullptr || d >= rotary_dim || pos < 0 || pos >= rotary_seqlen) return self.v;
-  const int half = rotary_dim >> 1;
-  if (!interleaved && half % 8 == 0 && ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 15) == 0) {
-    const bool first = d < half;
-    const int i = first ? d : d - half;
-    other.v = *reinterpret_cast<const uint4*>(x + (first ? d + half : d - half));
-    c.v = *reinterpret_cast<const uint4*>(cos + (int64_t)pos * half + i);
-    s.v = *reinterpret_cast<const uint4*>(sin + (int64_t)pos * half + i);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      out.e[k] = first ? hsub_rn(hmul_rn(self.e[k], c.e[k]), hmul_rn(other.e[k], s.e[k]))
-                       : hadd_rn(hmul_rn(other.e[k], s.e[k]), hmul_rn(self.e[k], c.e[k]));
-    return out.v;
-  }
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    out.e[k] = rotary_elem<T>([&](int j) { return x[j]; }, d + k, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
-  return out.v;
-}
-
 // New keys (rotated) and values into the cache, rotated queries into q_out (batch, tokens, heads, D); one
 // 16-byte chunk per thread, HBM-bound.  host / dev: value checks made by every CTA, see decode_kernel.
 template <typename T>

@@ -228,3 +228,21 @@ def test_unchecked_lengths_stay_inside_the_cache(tokens, padded):
     for t, was, new in zip(buf, kept, (kn, vn)):
         assert torch.equal(t[0], was[0]) and torch.equal(t[3], was[3]) and torch.equal(t[1], was[1])
         assert torch.equal(t[2, :cap - 1], was[2, :cap - 1]) and torch.equal(t[2, cap - 1], new[1, 0])
+
+
+@pytest.mark.parametrize("pieces", [15, 16, 17, 33])
+@pytest.mark.parametrize("D,rotary,interleaved,tokens", [(64, 24, False, 1), (64, 24, True, 3), (64, 48, False, 2), (128, 128, False, 2),
+                                                         (128, 96, True, 1), (16, 16, False, 4), (256, 256, False, 1)])
+def test_merge_batches_and_rotated_chunks(pieces, D, rotary, interleaved, tokens):
+    """Numbers of pieces around the 16 that are merged at a time; rotary dimensions that end inside a 16-byte chunk, new tokens
+    in the last tile and across two of them.  The cache rows are the reference's arithmetic to the last bit."""
+    cap, lens, Hq, Hkv = 2304, [2300 - tokens, 63 if tokens > 1 else 2111, 0], 8, 4
+    q, kc, vc, kn, vn = _contig_case(pieces + D + rotary, 3, 3, cap, Hq, Hkv, D, tokens, tokens)
+    cl = torch.tensor(lens, dtype=torch.int32)
+    cos, sin = cases.rotary_tables(cap, rotary)
+    ro, rkc, rvc = orc.kvcache_ref(q, kc, vc, kn, vn, cos, sin, cache_seqlens=cl, causal=True, rotary_interleaved=interleaved)
+    kcd, vcd = kc.to(DEV), vc.to(DEV)
+    out = fa().flash_attn_with_kvcache(dev(q), kcd, vcd, dev(kn), dev(vn), dev(cos), dev(sin), cache_seqlens=dev(cl), causal=True,
+                                       rotary_interleaved=interleaved, num_splits=pieces)
+    assert maxdiff(out, ro) <= util.FWD_TOL
+    assert torch.equal(kcd.cpu(), rkc) and torch.equal(vcd.cpu(), rvc)
