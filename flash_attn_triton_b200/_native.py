@@ -103,6 +103,9 @@ EXPORTS = {
     "fa_varlen_fwd": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fa_varlen_bwd_dq": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
     "fa_varlen_bwd_dkdv": (C.c_int, [C.POINTER(AttnArgs), C.c_void_p]),
+    "fa_varlen_check": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32, C.c_int64, C.c_int64, C.c_int32, C.c_int64, C.c_int64,
+                                  C.c_int32, C.POINTER(C.c_int32), C.c_void_p]),
+    "fa_check_result": (C.c_int, [C.c_int32, C.POINTER(C.c_uint32), C.c_void_p]),
     "fa_decode_paged": (C.c_int, [C.POINTER(DecodeArgs), C.c_void_p]),
     "fa_decode_paged_checked": (C.c_int, [C.POINTER(DecodeArgs), C.POINTER(C.c_uint32), C.c_void_p]),
     "fa_decode_checked_workspace_bytes": (C.c_size_t, [C.POINTER(DecodeArgs)]),

@@ -178,11 +178,20 @@ def dense_backward(q, k, v, o, lse, dout, scale, causal, wl, wr, softcap, alibi,
                              f.row_stride, None, None)
 
 
+VARLEN_UNCHECKED, VARLEN_EXACT, VARLEN_KV_AT_MOST = 0, 1, 2     # value checks of a packed call
+
+
+def varlen_check(q, k, cu_q, cu_k, max_q, max_k, checks):
+    """ValueError where the values of cu_seqlens do not describe q and k."""
+    N.host().varlen_check(q, k, cu_q, cu_k, int(max_q), int(max_k), checks == VARLEN_KV_AT_MOST)
+
+
 def varlen_attention(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl, feat=None,
-                     want_lse=False):
-    """Packed sequences: q (Tq,Hq,D), k/v (Tk,Hkv,D), int32 cu_seqlens on the device; differentiable."""
+                     want_lse=False, checks=VARLEN_UNCHECKED):
+    """Packed sequences: q (Tq,Hq,D), k/v (Tk,Hkv,D), int32 cu_seqlens on the device; differentiable.  `checks`: the
+    values of cu_seqlens are looked at, on the device, before the attention is launched."""
     f = feat or _NO_FEATURES
-    tail = (impl, f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse)
+    tail = (impl, f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse, checks)
     if _tracing() is not None:
         return _TracedCall.apply(lambda q, k, v, cu_q, cu_k, alibi: N.host().varlen(
             q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail), q, k, v, cu_q, cu_k, alibi)

@@ -49,6 +49,8 @@ struct Abi {
   int (*fwd_int8)(const fa_int8_args*, void*);
   size_t (*int8_codes16_bytes)(const fa_int8_args*);
   int (*fwd_int8_codes16)(const fa_int8_args*, const void*, float*, void*, void*);
+  int (*varlen_check)(const int32_t*, const int32_t*, int32_t, int64_t, int64_t, int32_t, int64_t, int64_t, int32_t, int32_t*, void*);
+  int (*check_result)(int32_t, uint32_t*, void*);
   int (*decode)(const fa_decode_args*, void*);
   int (*decode_checked)(const fa_decode_args*, uint32_t*, void*);
   int32_t (*decode_counters)(const fa_decode_args*);
@@ -225,8 +227,68 @@ Tensor dropout_bits(const fa_attn_args& a, const Tensor& t, bool backward) {
   return bits;
 }
 
+// The value checks of a packed call (the reference's, flash_attn_interface.py:588-626): started before the host work
+// of the call, whose result is awaited before anything reads by cu_seqlens.
+class VarlenCheck {
+ public:
+  void start(const Tensor& q, const Tensor& k, const Tensor& cu_q, const Tensor& cu_k, bool k_at_most, int64_t max_q, int64_t max_k) {
+    stream_ = stream_of(q);
+    const int n = (int)cu_q.numel() - 1;
+    const int r = g_abi.varlen_check(cu_q.const_data_ptr<int32_t>(), cu_k.const_data_ptr<int32_t>(), n, q.size(0), k.size(0), k_at_most,
+                                     max_q, max_k, q.device().index(), &ticket_, stream_);
+    if (r != FA_ERR_UNSUPPORTED) {
+      check(r, "fa_varlen_check");
+      return;
+    }
+    // no mapped host memory: by a copy
+    const Tensor hq = cu_q.cpu(), hk = cu_k.cpu();
+    const int32_t *a = hq.const_data_ptr<int32_t>(), *b = hk.const_data_ptr<int32_t>();
+    if (a[0] != 0 || b[0] != 0) failed_ |= FA_VARLEN_START;
+    for (int i = 0; i < n; ++i) {
+      const int64_t lq = (int64_t)a[i + 1] - a[i], lk = (int64_t)b[i + 1] - b[i];
+      if (lq < 0 || lk < 0) failed_ |= FA_VARLEN_ORDER;
+      if (lq > max_q || lk > max_k) failed_ |= FA_VARLEN_LONGEST;
+    }
+    if (a[n] != q.size(0) || (k_at_most ? b[n] > k.size(0) : b[n] != k.size(0))) failed_ |= FA_VARLEN_COVER;
+  }
+  // Raises what the values are refused for.
+  void finish() {
+    check(result(), "fa_check_result");
+    const char* what = failed_ & FA_VARLEN_START     ? "cu_seqlens arrays must start at zero and contain a batch boundary"
+                       : failed_ & FA_VARLEN_ORDER   ? "cu_seqlens arrays must be monotonically non-decreasing"
+                       : failed_ & FA_VARLEN_COVER   ? "cu_seqlens arrays must cover the packed q and KV tensors"
+                       : failed_ & FA_VARLEN_LONGEST ? "max sequence lengths must cover every packed sequence"
+                                                     : nullptr;
+    if (what == nullptr) return;
+    PyErr_SetString(PyExc_ValueError, what);
+    throw python_error();
+  }
+  ~VarlenCheck() { result(); }     // an exception in between: the ticket is handed in all the same
+  VarlenCheck() = default;
+  VarlenCheck(const VarlenCheck&) = delete;
+  VarlenCheck& operator=(const VarlenCheck&) = delete;
+
+ private:
+  int result() {
+    if (ticket_ < 0) return FA_OK;
+    const int32_t t = ticket_;
+    ticket_ = -1;
+    uint32_t bad = 0;
+    int r;
+    {
+      pybind11::gil_scoped_release nogil;
+      r = g_abi.check_result(t, &bad, stream_);
+    }
+    failed_ |= bad;
+    return r;
+  }
+  int32_t ticket_ = -1;
+  uint32_t failed_ = 0;
+  void* stream_ = nullptr;
+};
+
 // in: prepared inputs.  Fills out and (when wanted) lse.
-void run_forward(const Params& c, const variable_list& in, bool want_lse, Tensor& out, Tensor& lse) {
+void run_forward(const Params& c, const variable_list& in, bool want_lse, Tensor& out, Tensor& lse, VarlenCheck* values = nullptr) {
   View q, k, v;
   split(c, in, q, k, v);
   const Tensor& t = in[0];
@@ -235,6 +297,7 @@ void run_forward(const Params& c, const variable_list& in, bool want_lse, Tensor
   fa_attn_args a;
   fill(a, c, t, q, k, v, view_of(out, c.layout, -1, 0), want_lse ? lse.mutable_data_ptr<float>() : nullptr);
   const Tensor bits = dropout_bits(a, t, false);
+  if (values != nullptr) values->finish();
   if (bits.defined()) check(g_abi.fwd_bits(&a, bits.const_data_ptr(), stream_of(t)), "fa_fwd_dropout");
   else if (c.layout == kTHD) check(g_abi.varlen_fwd(&a, stream_of(t)), "fa_varlen_fwd");
   else check(g_abi.fwd(&a, stream_of(t)), "fa_fwd");
@@ -474,7 +537,8 @@ PyObject* py_dense(PyObject*, PyObject* const* args, Py_ssize_t n) {
 }
 
 // varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
-//        dropout_p, seed, row_stride, used_q, used_k, want_lse) -> out | (out, lse2)
+//        dropout_p, seed, row_stride, used_q, used_k, want_lse, checks) -> out | (out, lse2)
+// checks: 0 none, 1 the values of cu_seqlens, 2 the same with rows of k and v past the last sequence
 PyObject* py_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a{args, n};
@@ -494,11 +558,34 @@ PyObject* py_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
   c.used_q = a.tensor_or_none();
   c.used_k = a.tensor_or_none();
   const bool want_lse = a.truth();
+  const int checks = (int)a.integer();
   Tensor lse;
+  VarlenCheck values;
+  if (checks != 0) {
+    c10::cuda::CUDAGuard guard(in[0].device());
+    at::AutoDispatchBelowADInplaceOrView below;
+    values.start(in[0], in[1], c.cu_q, c.cu_k, checks == 2, c.max_q, c.max_k);
+  }
   Tensor out = with_grad(c, std::move(in), want_lse, lse, [&](const variable_list& x, bool w, Tensor& o, Tensor& l) {
-    run_forward(c, x, w, o, l);
+    run_forward(c, x, w, o, l, checks != 0 ? &values : nullptr);
   });
   return result(out, lse, want_lse);
+  END_HANDLE_TH_ERRORS
+}
+
+// varlen_check(q, k, cu_q, cu_k, max_q, max_k, k_at_most): the same checks by themselves
+PyObject* py_varlen_check(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  Args a{args, n};
+  const Tensor q = a.tensor(), k = a.tensor(), cu_q = a.tensor(), cu_k = a.tensor();
+  const int64_t max_q = a.integer(), max_k = a.integer();
+  const bool k_at_most = a.truth();
+  c10::cuda::CUDAGuard guard(q.device());
+  at::AutoDispatchBelowADInplaceOrView below;
+  VarlenCheck values;
+  values.start(q, k, cu_q, cu_k, k_at_most, max_q, max_k);
+  values.finish();
+  Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
 
@@ -731,6 +818,8 @@ PyObject* py_init(PyObject*, PyObject* const* args, Py_ssize_t n) {
   g_abi.fwd_int8 = (decltype(g_abi.fwd_int8))get("fa_fwd_int8");
   g_abi.int8_codes16_bytes = (decltype(g_abi.int8_codes16_bytes))get("fa_int8_codes16_bytes");
   g_abi.fwd_int8_codes16 = (decltype(g_abi.fwd_int8_codes16))get("fa_fwd_int8_codes16");
+  g_abi.varlen_check = (decltype(g_abi.varlen_check))get("fa_varlen_check");
+  g_abi.check_result = (decltype(g_abi.check_result))get("fa_check_result");
   g_abi.decode = (decltype(g_abi.decode))get("fa_decode_paged");
   g_abi.decode_checked = (decltype(g_abi.decode_checked))get("fa_decode_paged_checked");
   g_abi.decode_counters = (decltype(g_abi.decode_counters))get("fa_decode_counters");
@@ -748,6 +837,7 @@ PyMethodDef g_methods[] = {
     {"init", FAST(py_init), "addresses of the C ABI functions and the status check"},
     {"dense", FAST(py_dense), "dense attention"},
     {"varlen", FAST(py_varlen), "packed variable-length attention"},
+    {"varlen_check", FAST(py_varlen_check), "value checks of a packed call"},
     {"backward", FAST(py_backward), "gradients from a forward's output and LSE"},
     {"kvcache", FAST(py_kvcache), "append to a KV cache and attend to it"},
     {"int8", FAST(py_int8), "INT8 scores forward"},

@@ -452,20 +452,15 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
         raise ValueError("max sequence lengths must be non-negative")
     cu_seqlens_q = cu_seqlens_q.to(dtype=torch.int32).contiguous()
     cu_seqlens_k = cu_seqlens_k.to(dtype=torch.int32).contiguous()
+    checks = _ops.VARLEN_UNCHECKED
     if _VALIDATE:
-        # one device->host transfer for every value check the reference makes (:588-626)
-        both = torch.cat((cu_seqlens_q, cu_seqlens_k)).tolist()
-        cq, ck = both[:batch_size + 1], both[batch_size + 1:]
-        if cq[0] != 0 or ck[0] != 0:
-            raise ValueError("cu_seqlens arrays must start at zero and contain a batch boundary")
-        if any(b < a for a, b in zip(cq, cq[1:])) or any(b < a for a, b in zip(ck, ck[1:])):
-            raise ValueError("cu_seqlens arrays must be monotonically non-decreasing")
-        # gathered pages are sized by batch * max_seqlen_k, an upper bound of cu_seqlens_k[-1]
-        if cq[-1] != q.shape[0] or (ck[-1] > k.shape[0] if paged else ck[-1] != k.shape[0]):
-            raise ValueError("cu_seqlens arrays must cover the packed q and KV tensors")
-        if max_seqlen_q < max(b - a for a, b in zip(cq, cq[1:])) or \
-                max_seqlen_k < max(b - a for a, b in zip(ck, ck[1:])):
-            raise ValueError("max sequence lengths must cover every packed sequence")
+        # every value check the reference makes (:588-626).  Gathered pages are sized by batch * max_seqlen_k, an upper bound
+        # of cu_seqlens_k[-1].  The plain call makes them itself, under its own host work.
+        checks = _ops.VARLEN_KV_AT_MOST if paged else _ops.VARLEN_EXACT
+        if dropout_p or used_q is not None or used_k is not None or not (0 < max_seqlen_q < 2 ** 31) or \
+                not (0 < max_seqlen_k < 2 ** 31):
+            _ops.varlen_check(q, k, cu_seqlens_q, cu_seqlens_k, min(max_seqlen_q, 2 ** 62), min(max_seqlen_k, 2 ** 62), checks)
+            checks = _ops.VARLEN_UNCHECKED
     if max_seqlen_q == 0 or max_seqlen_k == 0:
         return q.new_zeros((q.shape[0], q.shape[1], q.shape[2]))
     alibi = _normalise_alibi(alibi_slopes, batch_size, q.shape[1], q.device)
@@ -516,10 +511,10 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
     args = (cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), softmax_scale, causal,
             window_size[0], window_size[1], softcap, alibi)
     if return_attn_probs:
-        out, lse2 = _ops.varlen_attention(q, k, v, *args, N.IMPL_AUTO, feat, True)
+        out, lse2 = _ops.varlen_attention(q, k, v, *args, N.IMPL_AUTO, feat, True, checks)
         probs, lse = _ops.varlen_probs(q.detach(), k.detach(), v.detach(), lse2, *args, feat)
     else:
-        out = _ops.varlen_attention(q, k, v, *args, N.IMPL_AUTO, feat)
+        out = _ops.varlen_attention(q, k, v, *args, N.IMPL_AUTO, feat, False, checks)
     if used_q is not None and not compacted:
         # the reference returns only the used rows, packed (flash_attn_interface.py:552-566); the one
         # host read of the lengths sizes that result

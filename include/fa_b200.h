@@ -238,6 +238,22 @@ typedef enum fa_decode_check {
 } fa_decode_check;
 int fa_decode_paged_checked(const fa_decode_args* args, uint32_t* failed, void* stream);
 
+/*
+ * The value checks of a packed call, without a stream synchronisation: fa_varlen_check queues a kernel that reads both
+ * cu_seqlens arrays (batch + 1 entries) and gives a ticket; fa_check_result waits until that kernel has run -- not for what
+ * is queued behind it -- and returns the checks that did not hold.  Every ticket is handed in exactly once.
+ * FA_ERR_UNSUPPORTED: no mapped host memory, the caller has to look at the values itself.  Not for streams under capture.
+ */
+typedef enum fa_varlen_check_bit {
+  FA_VARLEN_START = 1,   /* both arrays start at zero */
+  FA_VARLEN_ORDER = 2,   /* and never decrease */
+  FA_VARLEN_COVER = 4,   /* cu_seqlens_q[batch] == total_q; cu_seqlens_k[batch] == total_k, or <= with k_at_most */
+  FA_VARLEN_LONGEST = 8  /* no sequence is longer than max_q, max_k */
+} fa_varlen_check_bit;
+int fa_varlen_check(const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int32_t batch, int64_t total_q, int64_t total_k,
+                    int32_t k_at_most, int64_t max_q, int64_t max_k, int32_t device, int32_t* ticket, void* stream);
+int fa_check_result(int32_t ticket, uint32_t* failed, void* stream);
+
 /* Bytes of workspace for fa_decode_paged_checked, 0 where fa_decode_paged needs none and no kernel has to read the
  * result of the checks. */
 size_t fa_decode_checked_workspace_bytes(const fa_decode_args* args);

@@ -169,3 +169,67 @@ def test_config3_shape_reduced_and_full():
         assert maxdiff(out[s:e, hs], ro[0]) <= util.FWD_TOL, b
         for n, a, r in (("dq", dq, rdq), ("dk", dk, rdk), ("dv", dv, rdv)):
             assert maxdiff(a[s:e, hs], r[0]) <= util.GRAD_TOL, (b, n)
+
+
+@pytest.mark.parametrize("batch", [1, 128, 129, 1024, 2500])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64])
+def test_values_of_cu_seqlens_are_checked(batch, dtype):
+    """Every value check, at the first, a middle and the last sequence, in both arrays; with dropout they are made by themselves.
+    What is refused in several ways is refused for the first of them, and the call after a refused one works."""
+    total, H, D = 4 * batch, 1, 16
+    q, k, v = (torch.randn(total, H, D, device=DEV, dtype=torch.half) for _ in range(3))
+    good = torch.arange(0, total + 1, 4, dtype=dtype, device=DEV)
+
+    def call(cu_q, cu_k, max_q=4, max_k=4, **kw):
+        return fa().flash_attn_varlen_func(q, k, v, cu_q, cu_k, max_q, max_k, **kw)
+
+    def refused(text, *args, **kw):
+        for more in (dict(), dict(dropout_p=0.5)):
+            with pytest.raises(ValueError, match=text):
+                call(*args, **kw, **more)
+
+    want = call(good, good)
+    for which in (0, 1):
+        def bad(i, x):
+            cu = good.clone()
+            cu[i] = x
+            return (cu, good) if which == 0 else (good, cu)
+        refused("start at zero", *bad(0, 1))
+        refused("cover the packed", *bad(batch, total + 1), max_q=9, max_k=9)
+        for i in {1, batch // 2, batch - 1} - {0, batch}:
+            refused("non-decreasing", *bad(i, total + 7))
+            refused("cover every packed sequence", *bad(i, 4 * i + 1))
+    refused("cover every packed sequence", good, good, max_q=3)
+    refused("cover every packed sequence", good, good, max_k=3)
+    if batch > 1:
+        both = good.clone()
+        both[0], both[1] = 1, 0
+        refused("start at zero", both, good, max_q=1)
+    assert torch.equal(call(good, good), want)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert torch.equal(call(good, good), want)
+        refused("cover every packed sequence", good, good, max_q=3)
+    torch.cuda.current_stream().wait_stream(side)
+
+
+@pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
+def test_value_checks_are_refused_under_capture():
+    q = torch.randn(64, 2, 64, device=DEV, dtype=torch.half)
+    cu = torch.tensor([0, 30, 64], dtype=torch.int32, device=DEV)
+    call = lambda: fa().flash_attn_varlen_func(q, q, q, cu, cu, 34, 34)
+    want = call()
+    with pytest.raises(RuntimeError):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            call()
+    assert torch.equal(call(), want)
+    fa().set_validation(False)
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = call()
+        graph.replay()
+    finally:
+        fa().set_validation(True)
+    assert torch.equal(out, want)
