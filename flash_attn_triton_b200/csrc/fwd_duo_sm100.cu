@@ -10,11 +10,14 @@
 //   warp  5     MMA issuer: S = Q K_j^T (SS);  O += P V_j (A = P from tensor memory)
 //   warps 6-7   idle (they complete the warpgroup that gives its registers to the softmax warps)
 //
-// P (fp16/bf16) overwrites the first 64 columns of S; Q K_{j+1}^T may overwrite it because P V_j precedes it in the
-// in-order tensor pipe.  Arithmetic, order of the tiles and of the sums are those of the two-tile kernels
+// At head_dim 128 P (fp16/bf16) overwrites the first 64 columns of S; Q K_{j+1}^T may overwrite it because P V_j precedes it
+// in the in-order tensor pipe.  At head_dim 64 the accumulator leaves 64 columns, which P has to itself: Q K_{j+1}^T follows
+// as soon as the scores of tile j are in registers and runs under their exponentials, where it came behind P V_j, with
+// nothing of this CTA to do meanwhile (us, before -> after: 4 x 32 heads x 1024 x 1531 92.1 -> 88.0, 4 x 16 x 4096 causal 225 -> 219,
+// 8 x 16 x 512 with dropout 25.3 -> 24.3, 24 packed of 64 to 2048 211 -> 206; rows of two or three tiles +-1 %).  Arithmetic, order of the tiles and of the sums are those of the two-tile kernels
 // (fwd_sm100.cu, fwd_persist_sm100.cu): results are equal bit for bit.
 //
-// TMEM (256 columns): S (128) | O (head_dim).  Every mbarrier wait is bounded.
+// TMEM (256 columns): S (128) | O (head_dim) | at head_dim 64 P (64).  Every mbarrier wait is bounded.
 #include <type_traits>
 
 #include "common.cuh"
@@ -49,8 +52,10 @@ struct DShared {
   uint64_t kv_full[4];
   uint64_t kv_empty[4];
   uint64_t s_full;         // scores computed
+  uint64_t s_free;         // head_dim 64: scores in registers (128 arrivals)
   // (Barriers that count threads: none may arrive for a phase before the one ahead of it is complete.  For P: the next
-  // scores, which a thread needs first, are issued behind p_ready.)
+  // scores, which a thread needs first, are issued behind p_ready -- at head_dim 64 behind s_free, but a thread writes
+  // P only when the P V before, which was issued behind p_ready, has finished.)
   uint64_t p_half;         // the first 64 keys of P written back (128 arrivals)
   uint64_t p_ready;        // P written back (128 arrivals)
   uint64_t o_ready;        // the latest P V finished
@@ -77,6 +82,8 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
                      const fa_attn_args p, const ScoreCfg cfg, int* const host_status) {
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr bool kPvSplit = !kExtras;     // P V in two key halves (measured: helps the plain variants only)
+  constexpr bool kOwnP = D == 64;         // P in columns of its own
+  constexpr int kPCol = kOwnP ? kBN + D : 0;
   using C = DCfg<D>;
   constexpr int S = C::kStages;
   extern __shared__ unsigned char smem_raw[];
@@ -111,6 +118,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   if (tid == 0) {
     mbar_init(smem_u32(&sh->q_full), 1);
     mbar_init(smem_u32(&sh->s_full), 1);
+    mbar_init(smem_u32(&sh->s_free), 128);
     mbar_init(smem_u32(&sh->o_ready), 1);
     mbar_init(smem_u32(&sh->p_half), 128);
     mbar_init(smem_u32(&sh->p_ready), 128);
@@ -172,7 +180,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         if (ok) ok = wait_bar(bar, parity, sh, code);
         tc_fence_after();
       };
-      auto issue_qk = [&]() {                        // S = Q K^T with the next tile of the ring
+      auto issue_qk = [&]() {                        // S = Q K^T with this tile of the ring
         wwait(&sh->kv_full[stage], phase, 22);
         if (!ok) return;
         const uint64_t dq = make_smem_desc(sQ, 16, 1024), dk = make_smem_desc(sKV + stage * C::kTileBytes, 16, 1024);
@@ -183,29 +191,58 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         }
         mma_commit_lp(smem_u32(&sh->s_full), leader);
         mma_commit_lp(smem_u32(&sh->kv_empty[stage]), leader);
+      };
+      auto advance = [&]() {
         if (++stage == S) { stage = 0; phase ^= 1; }
       };
-      wwait(&sh->q_full, 0, 21);
-      if (ok) issue_qk();
-      for (int j = 0; j < nt && ok; ++j) {
-        wwait(&sh->kv_full[stage], phase, 24);       // V_j
+      auto issue_pv = [&](int j) {                   // O += P V_j with this tile of the ring
+        wwait(&sh->kv_full[stage], phase, 24);
         const uint64_t dv = make_smem_desc(sKV + stage * C::kTileBytes, kBN * 128, 1024);
         if (kPvSplit) {
           wwait(&sh->p_half, j & 1, 25);
-          if (!ok) break;
+          if (!ok) return;
 #pragma unroll
           for (int kk = 0; kk < kBN / 32; ++kk)
-            mma_f16_ts_lp(tmem + kBN, tmem + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u, leader);
+            mma_f16_ts_lp(tmem + kBN, tmem + kPCol + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u, leader);
         }
         wwait(&sh->p_ready, j & 1, 25);
-        if (!ok) break;
+        if (!ok) return;
 #pragma unroll
         for (int kk = kPvSplit ? kBN / 32 : 0; kk < kBN / 16; ++kk)
-          mma_f16_ts_lp(tmem + kBN, tmem + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u, leader);
+          mma_f16_ts_lp(tmem + kBN, tmem + kPCol + kk * 8, dv + ((kk * 2048) >> 4), idesc_pv, (j > 0 || kk > 0) ? 1u : 0u, leader);
         mma_commit_lp(smem_u32(&sh->o_ready), leader);
         mma_commit_lp(smem_u32(&sh->kv_empty[stage]), leader);
-        if (++stage == S) { stage = 0; phase ^= 1; }
-        if (j + 1 < nt) issue_qk();
+      };
+      wwait(&sh->q_full, 0, 21);
+      if constexpr (kOwnP) {
+        // S(j + 1) goes before P V_j, while the softmax warps have S(j) in registers.  K_j is entry 2 j of the ring, V_j the
+        // one behind it.
+        static_assert(S == 4, "K tiles take slots 0 and 2, V tiles 1 and 3");
+        for (int j = 0; j <= nt && ok; ++j) {
+          if (j < nt) {
+            if (j > 0) wwait(&sh->s_free, (j - 1) & 1, 25);
+            stage = 2 * (j & 1);
+            phase = (j >> 1) & 1;
+            if (ok) issue_qk();
+          }
+          if (j > 0 && ok) {
+            stage = 2 * ((j - 1) & 1) + 1;
+            phase = ((j - 1) >> 1) & 1;
+            issue_pv(j - 1);
+          }
+        }
+      } else {
+        if (ok) issue_qk();
+        advance();
+        for (int j = 0; j < nt && ok; ++j) {
+          issue_pv(j);
+          if (!ok) break;
+          advance();
+          if (j + 1 < nt) {
+            issue_qk();
+            advance();
+          }
+        }
       }
     }
   } else {
@@ -240,6 +277,10 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc) tmem_ld32(tSx + cc * 32, r[cc]);
       tmem_wait_ld();
+      if (kOwnP) {                                   // (behind the last tile too: a branch here undoes the gain)
+        tc_fence_before();
+        mbar_arrive(smem_u32(&sh->s_free));
+      }
 
       const bool prescaled = kExtras || masked;
       // columns (keys) of this tile that this thread's query row sees (used by masked tiles only)
@@ -374,6 +415,11 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
       // ---- P = exp2(s - m), row sum, P -> TMEM in place over S ----------------------------
       // packed pairs: one FMA, two exponentials, one conversion and one add per two scores
+      if (kOwnP && j > 0) {                          // the P V before has read its P (as good as always)
+        ok = wait_bar(&sh->o_ready, (j - 1) & 1, sh, 33);
+        if (!ok) break;
+        tc_fence_after();
+      }
       const float2 mul2 = make_float2(mul, mul), nm2 = make_float2(-m_safe, -m_safe);
       float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
       auto half_done = [&]() {
@@ -398,7 +444,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           }
           pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
         }
-        tmem_st16(tSx + cc * 16, pk);
+        tmem_st16(tSx + kPCol + cc * 16, pk);
         if (kPvSplit && cc == 1) half_done();
       }
       l += (acc2[0].x + acc2[0].y) + (acc2[1].x + acc2[1].y);
