@@ -26,6 +26,16 @@ __device__ __forceinline__ float round_f_fast(float x) {
   return copysignf(__fsub_rn(__fadd_rd(t, 8388608.0f), 8388608.0f), x);
 }
 
+// x / s to the last bit from the correctly rounded reciprocal `inv` of s: the estimate x inv is within one unit in the last
+// place, its remainder is exact, and one more step rounds correctly (P. Markstein, Computation of elementary functions on the
+// IBM RISC System/6000 processor, 1990).  For |x| <= 127 s, s = max(amax, 1) / 127 of finite 16-bit floats: compared with the
+// division for every pair of x and amax.  kSign: a zero keeps x's sign too.  The division itself, inlined per element, kept
+// the quantiser of 8 x 32 x 8192 query rows of 128 at 206 us; 167 now, 138 with a multiplication (the keys).
+template <bool kSign> __device__ __forceinline__ float div_by(float x, float s, float inv) {
+  const float q = __fmul_rn(x, inv), d = __fmaf_rn(__fmaf_rn(-q, s, x), inv, q);
+  return kSign ? copysignf(d, x) : d;
+}
+
 // ---------------------------------------------------------------------------------------
 // K quantiser: rows x D fp16 -> int8 codes + fp32 scale per row.  HBM-bound: 2 B read and
 // 1 B written per element.  D/8 lanes share a row, 16 bytes each; every thread keeps kRows
@@ -79,10 +89,22 @@ __global__ void __launch_bounds__(256) quantize_k_kernel(const __half* __restric
       const float sc = __fdiv_rn(fmaxf(amax, 1.0f), 127.0f);
       const float inv = __fdiv_rn(1.0f, sc);
       uint32_t lo = 0, hi = 0;
+      if (kDivide) {
+        if (amax < INFINITY) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] = div_by<kHalf>(x[i], sc, inv);
+        } else {                                     // an infinity among the row
+#pragma unroll 1
+          for (int i = 0; i < 8; ++i) {
+#pragma unroll
+            for (int n = 0; n < 8; ++n) x[n] = n == i ? __fdiv_rn(x[n], sc) : x[n];
+          }
+        }
+      }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const float a = kDivide ? __fdiv_rn(x[i], sc) : __fmul_rn(x[i], inv);
-        const float c2 = kDivide ? __fdiv_rn(x[4 + i], sc) : __fmul_rn(x[4 + i], inv);
+        const float a = kDivide ? x[i] : __fmul_rn(x[i], inv);
+        const float c2 = kDivide ? x[4 + i] : __fmul_rn(x[4 + i], inv);
         if (kHalf) {
           x[i] = round_f_fast(a);
           x[4 + i] = round_f_fast(c2);

@@ -186,3 +186,22 @@ def test_an_entry_has_the_same_result_in_any_batch(S, D):
     whole = fa.attention_int8(q, k, v, causal=True)
     assert torch.equal(fa.attention_int8(q[:1], k[:1], v[:1], causal=True), whole[:1])
     assert torch.equal(fa.attention_int8(*(t[:1, :2].contiguous() for t in (q, k, v)), causal=True), whole[:1, :2])
+
+
+@pytest.mark.parametrize("S,D", [(256, 128), (1088, 128), (1088, 64)])
+def test_query_rows_with_infinities_and_zeros(S, D):
+    """A row with an infinity has an infinite scale and a path of its own; rows of zeros, of both signs, and of the largest and
+    the smallest values beside it stay what they are without it."""
+    import flash_attn_triton_b200 as fa
+    g = torch.Generator(DEV).manual_seed(S + D)
+    q, k, v = (torch.randn(2, 32, S, D, device=DEV, dtype=torch.half, generator=g) for _ in range(3))
+    q[0, 0, 0] = 0.0
+    q[0, 0, 1] = -0.0
+    q[0, 0, 2, ::2], q[0, 0, 3] = 65504.0, 6e-8
+    want = fa.attention_int8(q, k, v)
+    q[0, 0, 5, 7] = float("inf")
+    out = fa.attention_int8(q, k, v)
+    out[0, 0, 5] = want[0, 0, 5]
+    assert torch.equal(out, want)
+    mean = v[0, 0].float().mean(0)                   # scores of zero: every key alike
+    assert (out[0, 0, :2].float() - mean).abs().max() <= 2e-3
