@@ -35,6 +35,7 @@
 
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "cache_geo.cuh"
 #include "common.cuh"
@@ -753,10 +754,12 @@ static int decode_row_groups(const fa_decode_args& a) {
 // rows; these calls append and rotate in a kernel of their own and attend on the tensor cores
 // (fwd_alt_sm100.cu), which takes about as long for 128 rows as the kernel above for 16.
 // ---------------------------------------------------------------------------------------
-// New keys (rotated) and values into the cache, rotated queries into q_out (batch, tokens, heads, D); one
-// 16-byte chunk per thread, HBM-bound.  host / dev: value checks made by every CTA, see decode_kernel.
-template <typename T>
-__global__ void __launch_bounds__(256) cache_append_kernel(const fa_decode_args p, T* q_out, int page_shift, uint32_t* host,
+// New keys (rotated) and values into the cache, rotated queries into q_out (batch, tokens, heads, D); a
+// 16-byte chunk per thread and step, HBM-bound.  host / dev: value checks made by every CTA, see decode_kernel.
+// Index: of a chunk.  With 64-bit indices the five divisions of a thread were most of the kernel; and as every CTA makes the
+// checks, there are no more CTAs than run at a time (4 x 256 tokens of 32 heads over 8 of 128: 15.5 -> 10.9 us).
+template <typename T, typename Index>
+__global__ void __launch_bounds__(256, 5) cache_append_kernel(const fa_decode_args p, T* q_out, int page_shift, uint32_t* host,
                                                            uint32_t* dev, bool check_here) {
   if (check_here) {
     const uint32_t bad = decode_checks(p, threadIdx.x, 256);
@@ -769,40 +772,40 @@ __global__ void __launch_bounds__(256) cache_append_kernel(const fa_decode_args 
   } else if (dev && *dev) {
     return;
   }
-  const int D = p.head_dim, cpr = D / 8;
+  const int D = p.head_dim, cpr_log2 = 31 - __clz(D / 8);      // (a power of two)
   const int n_new = p.k_new ? p.seqlen_new : 0;
-  const int64_t nq = q_out ? (int64_t)p.batch * p.seqlen_q * p.heads_q * cpr : 0;
-  const int64_t nk = (int64_t)p.batch * n_new * p.heads_kv * cpr;
+  const Index nq = q_out ? ((Index)p.batch * p.seqlen_q * p.heads_q) << cpr_log2 : 0;
+  const Index nk = ((Index)p.batch * n_new * p.heads_kv) << cpr_log2;
   const T* cos = reinterpret_cast<const T*>(p.rotary_cos);
   const T* sin = reinterpret_cast<const T*>(p.rotary_sin);
-  int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-  if (i < nq) {
-    const int d = (int)(i % cpr) * 8, h = (int)(i / cpr % p.heads_q);
-    const int64_t bt = i / ((int64_t)cpr * p.heads_q);
-    const int tok = (int)(bt % p.seqlen_q), b = (int)(bt / p.seqlen_q);
-    const int pos = p.cache_seqlens[b] + n_new - p.seqlen_q + tok + (p.cache_leftpad ? p.cache_leftpad[b] : 0);
-    const T* x = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + tok * p.q_stride[1] + h * p.q_stride[2];
-    *reinterpret_cast<uint4*>(q_out + i * 8) =
-        rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
-    return;
-  }
-  i -= nq;
-  if (i >= 2 * nk) return;
-  const bool val = i >= nk;
-  if (val) i -= nk;
-  const int d = (int)(i % cpr) * 8, h = (int)(i / cpr % p.heads_kv);
-  const int64_t bt = i / ((int64_t)cpr * p.heads_kv);
-  const int tok = (int)(bt % n_new), b = (int)(bt / n_new);
-  const int pos = max(0, min(p.cache_seqlens[b], seq_capacity(p, b))) + tok + (p.cache_leftpad ? max(0, p.cache_leftpad[b]) : 0);
-  if (pos >= cache_capacity(p)) return;
-  if (val) {
-    const T* x = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + h * p.vn_stride[2];
-    T* dst = reinterpret_cast<T*>(p.v_cache) + cache_row_offset(p, b, pos, page_shift, p.vc_stride) + h * p.vc_stride[2];
-    *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(x + d);
-  } else {
-    const T* x = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + h * p.kn_stride[2];
-    T* dst = reinterpret_cast<T*>(p.k_cache) + cache_row_offset(p, b, pos, page_shift, p.kc_stride) + h * p.kc_stride[2];
-    *reinterpret_cast<uint4*>(dst + d) = rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+  for (Index at = (Index)blockIdx.x * 256 + threadIdx.x; at < nq + 2 * nk; at += (Index)gridDim.x * 256) {
+    Index i = at;
+    const int d = (int)(i & ((1 << cpr_log2) - 1)) * 8;
+    if (i < nq) {
+      const Index row = i >> cpr_log2, bt = row / (Index)p.heads_q;
+      const int h = (int)(row - bt * p.heads_q), b = (int)(bt / (Index)p.seqlen_q), tok = (int)(bt - (Index)b * p.seqlen_q);
+      const int pos = p.cache_seqlens[b] + n_new - p.seqlen_q + tok + (p.cache_leftpad ? p.cache_leftpad[b] : 0);
+      const T* x = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + tok * p.q_stride[1] + h * p.q_stride[2];
+      *reinterpret_cast<uint4*>(q_out + (int64_t)i * 8) =
+          rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+      continue;
+    }
+    i -= nq;
+    const bool val = i >= nk;
+    if (val) i -= nk;
+    const Index row = i >> cpr_log2, bt = row / (Index)p.heads_kv;
+    const int h = (int)(row - bt * p.heads_kv), b = (int)(bt / (Index)n_new), tok = (int)(bt - (Index)b * n_new);
+    const int pos = max(0, min(p.cache_seqlens[b], seq_capacity(p, b))) + tok + (p.cache_leftpad ? max(0, p.cache_leftpad[b]) : 0);
+    if (pos >= cache_capacity(p)) continue;
+    if (val) {
+      const T* x = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + h * p.vn_stride[2];
+      T* dst = reinterpret_cast<T*>(p.v_cache) + cache_row_offset(p, b, pos, page_shift, p.vc_stride) + h * p.vc_stride[2];
+      *reinterpret_cast<uint4*>(dst + d) = *reinterpret_cast<const uint4*>(x + d);
+    } else {
+      const T* x = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + h * p.kn_stride[2];
+      T* dst = reinterpret_cast<T*>(p.k_cache) + cache_row_offset(p, b, pos, page_shift, p.kc_stride) + h * p.kc_stride[2];
+      *reinterpret_cast<uint4*>(dst + d) = rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+    }
   }
 }
 
@@ -1011,12 +1014,17 @@ static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* h
   const int64_t chunks = ((q_out ? (int64_t)a.batch * a.seqlen_q * a.heads_q : 0) + 2ll * a.batch * geo.n_new * a.heads_kv) *
                          (a.head_dim / 8);
   if (chunks > 0 || inside) {
-    const unsigned grid = (unsigned)(chunks > 0 ? (chunks + 255) / 256 : 1);
+    const int64_t need = chunks > 0 ? (chunks + 255) / 256 : 1, fit = (int64_t)sm_count(a.device) * 5;
+    const unsigned grid = (unsigned)(need < fit ? need : fit);
     const int shift = page_shift_of(a);
-    if (a.dtype == FA_BF16)
-      cache_append_kernel<<<grid, 256, 0, st>>>(a, static_cast<__nv_bfloat16*>(q_out), shift, host, dev, inside);
-    else
-      cache_append_kernel<<<grid, 256, 0, st>>>(a, static_cast<__half*>(q_out), shift, host, dev, inside);
+    const bool small = chunks < (int64_t)1 << 31;
+    auto append = [&](auto* q) {
+      using T = std::remove_pointer_t<decltype(q)>;
+      auto kern = small ? cache_append_kernel<T, uint32_t> : cache_append_kernel<T, int64_t>;
+      kern<<<grid, 256, 0, st>>>(a, q, shift, host, dev, inside);
+    };
+    if (a.dtype == FA_BF16) append(static_cast<__nv_bfloat16*>(q_out));
+    else append(static_cast<__half*>(q_out));
     if (int r = check_launch("cache_append")) return r;
     if (inside) *queued = true;
   }

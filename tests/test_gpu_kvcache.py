@@ -246,3 +246,19 @@ def test_merge_batches_and_rotated_chunks(pieces, D, rotary, interleaved, tokens
                                        rotary_interleaved=interleaved, num_splits=pieces)
     assert maxdiff(out, ro) <= util.FWD_TOL
     assert torch.equal(kcd.cpu(), rkc) and torch.equal(vcd.cpu(), rvc)
+
+
+@pytest.mark.parametrize("B,tokens,Hq,Hkv,D,rotary", [(3, 300, 32, 4, 128, 128), (2, 700, 24, 3, 64, 24), (5, 33, 6, 6, 256, 0)])
+def test_appended_chunks_of_more_steps_than_one(B, tokens, Hq, Hkv, D, rotary):
+    """More 16-byte pieces than the append kernel has threads, head counts that are no powers of two, a table that ends inside."""
+    lens = [17, 64, 300, 1, 90][:B]
+    cap = max(lens) + tokens
+    q, kc, vc, kn, vn = _contig_case(B + tokens, B, B, cap, Hq, Hkv, D, tokens, tokens)
+    cl = torch.tensor(lens, dtype=torch.int32)
+    cos, sin = cases.rotary_tables(cap, rotary) if rotary else (None, None)
+    ro, rkc, rvc = orc.kvcache_ref(q, kc, vc, kn, vn, cos, sin, cache_seqlens=cl, causal=True, rotary_interleaved=False)
+    kcd, vcd = kc.to(DEV), vc.to(DEV)
+    out = fa().flash_attn_with_kvcache(dev(q), kcd, vcd, dev(kn), dev(vn), dev(cos), dev(sin), cache_seqlens=dev(cl), causal=True,
+                                       rotary_interleaved=False)
+    assert maxdiff(out, ro) <= util.FWD_TOL
+    assert torch.equal(kcd.cpu(), rkc) and torch.equal(vcd.cpu(), rvc)
