@@ -868,8 +868,12 @@ static OneTile one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
 //   up to 2.5 CTAs per SM        +1 to +15 %
 //   head_dim 64, plain           -2 to -22 % dense (16 x 32 heads x 1024, causal: 205 -> 191 us; no mask, 1531 tokens: 550 -> 518),
 //                                -2 to -11 % packed; +3 to +7 % where part of the exponentials would go to the FMA pipe
-//   others, by the key tiles of a row tile on average: up to 6.5  -2 to -26 % (head_dim 128, 512 x 1024, causal: 245 -> 235;
-//                                packed 17 to 2048, causal: 396 -> 370), 8 and more  0 to +15 %
+//   others, by the key tiles of a row tile on average, where the persistent kernel is the alternative: up to 6.5  -2 to -26 %
+//                                (packed 17 to 2048, causal: 396 -> 370), 8 and more  0 to +15 % (40 packed of 64 to 3000: +5 %)
+//   where the two-tile kernel is (below the persistent one's lengths; dropout): head_dim 64 with options 0 to -13 % at every
+//                                length, no mask -1 to -13 % up to 15 key tiles (8 x 16 x 1152: 111.0 -> 96.6), causal -3 to -9 % up to 8 on
+//                                average (8 x 16 x 1600: 131 -> 123, with a soft cap 6 x 16: 140 -> 130, dropout 139 -> 127, 24 packed
+//                                of 64 to 2040, 32 heads over 8: 458 -> 417; the worst, 1700 tokens, +0.4 %), +2 to +4 % at 8.5
 //   windows, up to 10            -4 to -12 % (32 packed sequences of 256 to 4096, window 1024, ALiBi and soft cap, head_dim
 //                                128: 1686 -> 1621): two thirds of a short window's tiles are masked, and the pair of
 //                                tiles of the other kernels sees one more than either needs
@@ -886,7 +890,11 @@ static bool two_ctas_are_faster(const fa_attn_args& a, const ScoreCfg& cfg, int 
   const int64_t nk = (keys + kBN - 1) / kBN;
   int64_t twice = cfg.causal ? nk + 1 : 2 * nk;
   const int right = cfg.causal ? 0 : cfg.wr;
-  if (cfg.wl < 0 || right < 0) return twice <= 13;
+  if (cfg.wl < 0 || right < 0) {
+    const bool two_tile = cfg.keep != nullptr || persistent_from <= 0 || a.seqlen_k < persistent_from;   // the alternative
+    if (!two_tile) return twice <= 13;
+    return a.head_dim == 64 || twice <= (cfg.causal ? 16 : 30);
+  }
   return std::min<int64_t>(twice, 2 * (((int64_t)cfg.wl + right) / kBN + 2)) <= 20;
 }
 

@@ -79,3 +79,25 @@ def test_packed_two_ctas(monkeypatch, kw, D, dtype):
             assert maxdiff(got[r], want[0]) <= util.tols(dtype)[0], b
     monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
     assert torch.equal(got, run(k, v))
+
+
+@pytest.mark.parametrize("S,D,kw", [(1537, 128, dict(causal=True)), (1920, 128, dict(causal=True)), (1921, 128, dict(causal=True)),
+                                    (1600, 128, dict(causal=True, dropout_p=0.2)), (1920, 128, dict()), (1921, 128, dict()),
+                                    (1600, 128, dict(causal=True, softcap=20.0)), (2047, 64, dict(causal=True, alibi=True)),
+                                    (1530, 64, dict(softcap=20.0))], ids=str)
+def test_below_the_persistent_kernel(monkeypatch, S, D, kw):
+    """Lengths on both sides of the rule where the two-tile kernel is the alternative: equal to it bit for bit."""
+    import random
+    import flash_attn_triton_b200 as fa
+    g = torch.Generator(DEV).manual_seed(S)
+    q, k, v = (torch.randn(2, S, 16, D, device=DEV, dtype=torch.half, generator=g) for _ in range(3))
+    assert enough_tiles(2 * -(-S // 128), 16)
+    opts = slopes(kw)
+
+    def run():
+        random.seed(3)                               # the dropout mask
+        return fa.flash_attn_func(q, k, v, **opts)
+
+    got = run()
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    assert torch.equal(got, run())
