@@ -214,6 +214,21 @@ def test_values_of_cu_seqlens_are_checked(batch, dtype):
     torch.cuda.current_stream().wait_stream(side)
 
 
+@pytest.mark.parametrize("where", ["cpu", DEV])
+@pytest.mark.parametrize("dtype", [torch.int32, torch.int64, torch.int16])
+def test_longest_sequence_as_a_tensor(dtype, where):
+    """max_seqlen as `(cu[1:] - cu[:-1]).max()` leaves it: one that is too small is refused in any type, with dropout too."""
+    q = torch.randn(64, 2, 64, device=DEV, dtype=torch.half)
+    cu = torch.tensor([0, 30, 64], dtype=torch.int32, device=DEV)
+    n = lambda x: torch.tensor(x, dtype=dtype, device=where)
+    want = fa().flash_attn_varlen_func(q, q, q, cu, cu, 34, 34)
+    assert torch.equal(fa().flash_attn_varlen_func(q, q, q, cu, cu, n(34), n(34)), want)
+    for more in (dict(), dict(dropout_p=0.5)):
+        for lengths in ((n(33), n(34)), (n(34), n(33)), (33, n(34))):
+            with pytest.raises(ValueError, match="cover every packed sequence"):
+                fa().flash_attn_varlen_func(q, q, q, cu, cu, *lengths, **more)
+
+
 @pytest.mark.filterwarnings("ignore:The CUDA Graph is empty")
 def test_value_checks_are_refused_under_capture():
     q = torch.randn(64, 2, 64, device=DEV, dtype=torch.half)
