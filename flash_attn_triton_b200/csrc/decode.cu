@@ -38,6 +38,7 @@
 #include <type_traits>
 
 #include "cache_geo.cuh"
+#include "check_slots.h"
 #include "common.cuh"
 
 namespace fa {
@@ -1046,71 +1047,76 @@ int decode_paged(const fa_decode_args& a, cudaStream_t st) {
 // changes as soon as the checks have run, so the host goes on while the attention is still running, without
 // a stream synchronisation.
 // ---------------------------------------------------------------------------------------
-constexpr int kCheckSlots = 256;
+constexpr int kCheckSlots = 256, kTickets = FA_VARLEN_TICKETS;
 alignas(4096) static volatile uint32_t g_check_host[kCheckSlots * 16];      // a cache line per slot
 
 namespace {
-struct CheckSlots {
-  std::mutex mu;
-  int free_list[kCheckSlots], nfree = 0;
-  bool mapped = false;
-  // index of a free slot, or -1 (error set)
-  int acquire(uint32_t** host_dptr) {
-    for (;;) {
-      {
-        std::lock_guard<std::mutex> lock(mu);
-        if (!mapped) {
-          // tried again by the next call where it fails (another thread may be capturing a graph right now)
-          const cudaError_t e = cudaHostRegister(const_cast<uint32_t*>(g_check_host), sizeof(g_check_host),
-                                                 cudaHostRegisterPortable | cudaHostRegisterMapped);
-          if (e != cudaSuccess) {
-            cudaGetLastError();
-            set_error("decode: no mapped host memory for the value checks: %s", cudaGetErrorString(e));
-            return -1;
-          }
-          mapped = true;
-          for (int i = 0; i < kCheckSlots; ++i) free_list[nfree++] = kCheckSlots - 1 - i;
-        }
-        if (nfree > 0) {
-          const int i = free_list[--nfree];
-          void* h = nullptr;
-          if (cudaHostGetDevicePointer(&h, const_cast<uint32_t*>(&g_check_host[i * 16]), 0) != cudaSuccess) {
-            set_error("decode: cudaHostGetDevicePointer: %s", cudaGetErrorString(cudaGetLastError()));
-            free_list[nfree++] = i;
-            return -1;
-          }
-          *host_dptr = static_cast<uint32_t*>(h);
-          g_check_host[i * 16] = 0u;
-          return i;
-        }
-      }
-      sched_yield();                   // as many threads as slots are inside this function
-    }
-  }
-  // Waits until the kernel that was given the slot has written it: only then may another call have it.
-  int await(int i, uint32_t* failed, cudaStream_t st) {
-    volatile uint32_t* word = &g_check_host[i * 16];
-    for (uint32_t it = 1; *word == 0u; ++it) {
-#if defined(__x86_64__)
-      __builtin_ia32_pause();
-#endif
-      if ((it & 0x3fffu) == 0) {       // every few hundred microseconds: has the stream died?
-        const cudaError_t e = cudaStreamQuery(st);
-        if (e == cudaErrorNotReady) continue;
-        if (e != cudaSuccess || *word == 0u) {
-          set_error("decode: value checks did not run: %s", cudaGetErrorString(e));
-          return FA_ERR_LAUNCH;
-        }
-      }
-    }
-    *failed = *word & ~kCheckDone;
-    return FA_OK;
-  }
-  void release(int i) {
+CheckSlots<kCheckSlots, kTickets> g_slots(g_check_host);
+volatile uint32_t* slot_word(int i) { return g_slots.word_of(g_check_host, i); }
+
+// The words as the current device sees them, null (error set) without mapped host memory.  Tried again by the next call where it fails
+// (another thread may be capturing a graph right now).
+uint32_t* check_words() {
+  static std::mutex mu;
+  static bool mapped = false;
+  {
     std::lock_guard<std::mutex> lock(mu);
-    free_list[nfree++] = i;
+    if (!mapped) {
+      const cudaError_t e = cudaHostRegister(const_cast<uint32_t*>(g_check_host), sizeof(g_check_host),
+                                             cudaHostRegisterPortable | cudaHostRegisterMapped);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("no mapped host memory for the value checks: %s", cudaGetErrorString(e));
+        return nullptr;
+      }
+      mapped = true;
+    }
   }
-} g_slots;
+  void* h = nullptr;
+  if (cudaHostGetDevicePointer(&h, const_cast<uint32_t*>(g_check_host), 0) != cudaSuccess) {
+    set_error("value checks: cudaHostGetDevicePointer: %s", cudaGetErrorString(cudaGetLastError()));
+    return nullptr;
+  }
+  return static_cast<uint32_t*>(h);
+}
+
+// Index of a slot, its word at *dptr; -1 (error set) without one.  A call waits for another call's, a ticket does not.
+int take_slot(bool ticket, uint32_t** dptr) {
+  uint32_t* words = check_words();
+  if (words == nullptr) return -1;
+  for (;;) {
+    const int i = g_slots.take(ticket);
+    if (i >= 0) {
+      *dptr = words + i * 16;
+      return i;
+    }
+    if (ticket || i == g_slots.kNever) {
+      set_error(ticket ? "%d tickets of value checks are out" : "no word for the value checks is left", kTickets);
+      return -1;
+    }
+    sched_yield();                     // as many threads as slots are inside this function
+  }
+}
+
+// Waits until the kernel that was given the slot has written it.
+int await_slot(int i, uint32_t* failed, cudaStream_t st) {
+  volatile uint32_t* word = slot_word(i);
+  for (uint32_t it = 1; *word == 0u; ++it) {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+    if ((it & 0x3fffu) == 0) {         // every few hundred microseconds: has the stream died?
+      const cudaError_t e = cudaStreamQuery(st);
+      if (e == cudaErrorNotReady) continue;
+      if (e != cudaSuccess || *word == 0u) {
+        set_error("value checks did not run: %s", cudaGetErrorString(e));
+        return FA_ERR_LAUNCH;
+      }
+    }
+  }
+  *failed = *word & ~kCheckDone;
+  return FA_OK;
+}
 
 // Packed calls: both cu_seqlens arrays, by one CTA.
 __global__ void __launch_bounds__(1024) varlen_check_kernel(const int32_t* cu_q, const int32_t* cu_k, int batch, int64_t total_q,
@@ -1164,20 +1170,20 @@ int varlen_check(const int32_t* cu_q, const int32_t* cu_k, int batch, int64_t to
     return FA_ERR_LAUNCH;
   }
   uint32_t* host = nullptr;
-  const int slot = g_slots.acquire(&host);
+  const int slot = take_slot(true, &host);
   if (slot < 0) return FA_ERR_UNSUPPORTED;
   varlen_check_kernel<<<1, batch > 128 ? 1024 : 128, 0, st>>>(cu_q, cu_k, batch, total_q, total_k, k_at_most, max_q, max_k, host);
   if (int r = check_launch("varlen_check")) {
-    g_slots.release(slot);
+    g_slots.give(slot, false);
     return r;
   }
   *ticket = slot;
   return FA_OK;
 }
 int check_result(int32_t ticket, uint32_t* failed, cudaStream_t st) {
-  FA_REQUIRE(ticket >= 0 && ticket < kCheckSlots, "no such ticket");
-  const int r = g_slots.await(ticket, failed, st);
-  g_slots.release(ticket);
+  FA_REQUIRE(g_slots.hand_in(ticket), "ticket %d is not out", ticket);
+  const int r = await_slot(ticket, failed, st);
+  g_slots.give(ticket, true);
   return r;
 }
 
@@ -1203,7 +1209,7 @@ int decode_paged_checked(const fa_decode_args& a, uint32_t* failed, cudaStream_t
   const bool host_order = k.word && word == nullptr;   // no room for the word: launch nothing before the result is here
   if (host_order) k.inside = false;
   uint32_t* host = nullptr;
-  const int slot = g_slots.acquire(&host);
+  const int slot = take_slot(false, &host);
   if (slot < 0) return FA_ERR_LAUNCH;
   int r = FA_OK;
   bool queued = false;                                 // a kernel that writes the host word is on the stream
@@ -1221,10 +1227,10 @@ int decode_paged_checked(const fa_decode_args& a, uint32_t* failed, cudaStream_t
     }
   }
   if (queued) {
-    const int w = g_slots.await(slot, failed, st);
+    const int w = await_slot(slot, failed, st);
     if (r == FA_OK) r = w;
   }
-  g_slots.release(slot);
+  g_slots.give(slot, queued);
   if (r != FA_OK || *failed || !host_order) return r;
   return k.chunk ? chunk_run(a, k.c, nullptr, nullptr, nullptr, st) : decode_run(a, DecodeCheck{nullptr, nullptr}, st);
 }

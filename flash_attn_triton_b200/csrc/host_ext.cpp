@@ -240,7 +240,7 @@ class VarlenCheck {
       check(r, "fa_varlen_check");
       return;
     }
-    // no mapped host memory: by a copy
+    // no mapped host memory, or too many tickets out: by a copy
     const Tensor hq = cu_q.cpu(), hk = cu_k.cpu();
     const int32_t *a = hq.const_data_ptr<int32_t>(), *b = hk.const_data_ptr<int32_t>();
     if (a[0] != 0 || b[0] != 0) failed_ |= FA_VARLEN_START;

@@ -56,6 +56,10 @@ def test_argument_errors_without_gpu(built):
     d.heads_q, d.heads_kv, d.head_dim, d.batch, d.seqlen_q = 8, 2, 128, 1, 1
     assert lib.fa_decode_paged(ctypes.byref(d), None) == -1
     assert lib.fa_quantize_k_int8(None, None, None, 4, 16, 0, None) == -1
+    failed = ctypes.c_uint32()
+    for ticket in (-1, 0, 5, 1 << 20):                     # never issued
+        assert lib.fa_check_result(ticket, ctypes.byref(failed), None) == -1
+        assert b"not out" in lib.fa_last_error()
 
 
 def test_no_oracle_in_product():

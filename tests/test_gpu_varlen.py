@@ -248,3 +248,34 @@ def test_value_checks_are_refused_under_capture():
     finally:
         fa().set_validation(True)
     assert torch.equal(out, want)
+
+
+def test_tickets_of_value_checks():
+    """As many tickets as there are: the next check is not taken, calls go on, and a ticket is handed in once."""
+    import ctypes as C
+    from flash_attn_triton_b200 import _native as N
+    lib, cu, out = N.lib(), torch.tensor([0, 30, 64], dtype=torch.int32, device=DEV), []
+    q = torch.randn(64, 2, 64, device=DEV, dtype=torch.half)
+    ticket, failed, stream = C.c_int32(), C.c_uint32(), N.stream_ptr(q.device)
+    want = fa().flash_attn_varlen_func(q, q, q, cu, cu, 34, 34)
+
+    def issue(longest):
+        return lib.fa_varlen_check(cu.data_ptr(), cu.data_ptr(), 2, 64, 64, 0, longest, 34, 0, C.byref(ticket), stream)
+
+    for i in range(128):
+        assert issue(34 - i % 2) == 0
+        out.append(ticket.value)
+    assert issue(34) == -2                               # FA_ERR_UNSUPPORTED, without a wait
+    assert torch.equal(fa().flash_attn_varlen_func(q, q, q, cu, cu, 34, 34), want)
+    with pytest.raises(ValueError, match="cover every packed sequence"):
+        fa().flash_attn_varlen_func(q, q, q, cu, cu, 34, 33)
+    lens = torch.tensor([5], dtype=torch.int32, device=DEV)
+    cache = torch.zeros(1, 64, 2, 64, device=DEV, dtype=torch.half)
+    fa().flash_attn_with_kvcache(q[None, :1], cache, cache.clone(), cache_seqlens=lens)      # a call with a word of its own
+    for i, t in enumerate(out):
+        assert lib.fa_check_result(t, C.byref(failed), stream) == 0
+        assert failed.value == (8 if i % 2 else 0)       # FA_VARLEN_LONGEST
+    for t in out:
+        assert lib.fa_check_result(t, C.byref(failed), stream) == -1
+    assert issue(34) == 0
+    assert lib.fa_check_result(ticket.value, C.byref(failed), stream) == 0 and failed.value == 0
