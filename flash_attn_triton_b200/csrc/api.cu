@@ -117,7 +117,7 @@ int fwd_alt_sm100_clear_status();
 int fwd_duo_sm100_clear_status();
 int decode_paged(const fa_decode_args&, cudaStream_t);
 int decode_paged_checked(const fa_decode_args&, uint32_t*, cudaStream_t);
-int varlen_check(const int32_t*, const int32_t*, int, int64_t, int64_t, bool, int64_t, int64_t, int32_t*, cudaStream_t);
+int varlen_check(const int32_t*, const int32_t*, int, int64_t, int64_t, bool, int64_t, int64_t, int, int32_t*, cudaStream_t);
 int check_result(int32_t, uint32_t*, cudaStream_t);
 int decode_num_counters(const fa_decode_args&);
 size_t decode_workspace_bytes(const fa_decode_args&);
@@ -422,7 +422,8 @@ int fa_varlen_check(const int32_t* cu_q, const int32_t* cu_k, int32_t batch, int
                     int64_t max_q, int64_t max_k, int32_t device, int32_t* ticket, void* stream) {
   FA_REQUIRE(cu_q != nullptr && cu_k != nullptr && ticket != nullptr && batch >= 0, "cu_seqlens and ticket are required");
   if (int r = ensure_device(device)) return r;
-  return varlen_check(cu_q, cu_k, batch, total_q, total_k, k_at_most != 0, max_q, max_k, ticket, reinterpret_cast<cudaStream_t>(stream));
+  return varlen_check(cu_q, cu_k, batch, total_q, total_k, k_at_most != 0, max_q, max_k, device, ticket,
+                      reinterpret_cast<cudaStream_t>(stream));
 }
 
 int fa_check_result(int32_t ticket, uint32_t* failed, void* stream) {

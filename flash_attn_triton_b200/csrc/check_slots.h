@@ -20,8 +20,8 @@ template <int kWords, int kTickets> class CheckSlots {
   explicit CheckSlots(volatile uint32_t* base) : base_(base) {
     for (int i = 0; i < kWords; ++i) free_[nfree_++] = kWords - 1 - i;
   }
-  // A word of zero, as a ticket or for the call itself.
-  int take(bool ticket) {
+  // A word of zero, as a ticket (whose kernel runs on `device`) or for the call itself.
+  int take(bool ticket, int device) {
     std::lock_guard<std::mutex> lock(mu_);
     if (ticket && tickets_ == kTickets) return kNone;
     if (nfree_ == 0 && lost_ > 0) find_again();
@@ -29,16 +29,18 @@ template <int kWords, int kTickets> class CheckSlots {
     const int i = free_[--nfree_];
     state_[i] = ticket ? kTicket : kCall;
     tickets_ += ticket;
+    device_[i] = device;
     *word(i) = 0u;
     return i;
   }
   // A ticket becomes a word of the call that hands it in: false where it is not out, so that of two that hand in the
-  // same one gets it.
-  bool hand_in(int i) {
+  // same one gets it.  *device: where its kernel is.
+  bool hand_in(int i, int* device) {
     std::lock_guard<std::mutex> lock(mu_);
     if (i < 0 || i >= kWords || state_[i] != kTicket) return false;
     state_[i] = kCall;
     --tickets_;
+    *device = device_[i];
     return true;
   }
   // Back from the call.  queued: a kernel was given the word.
@@ -69,6 +71,7 @@ template <int kWords, int kTickets> class CheckSlots {
   volatile uint32_t* base_;
   int free_[kWords], nfree_ = 0, tickets_ = 0, lost_ = 0;
   State state_[kWords] = {};
+  int device_[kWords];
 };
 
 }  // namespace fa

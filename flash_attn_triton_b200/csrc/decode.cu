@@ -1081,11 +1081,11 @@ uint32_t* check_words() {
 }
 
 // Index of a slot, its word at *dptr; -1 (error set) without one.  A call waits for another call's, a ticket does not.
-int take_slot(bool ticket, uint32_t** dptr) {
+int take_slot(bool ticket, int device, uint32_t** dptr) {
   uint32_t* words = check_words();
   if (words == nullptr) return -1;
   for (;;) {
-    const int i = g_slots.take(ticket);
+    const int i = g_slots.take(ticket, device);
     if (i >= 0) {
       *dptr = words + i * 16;
       return i;
@@ -1162,7 +1162,7 @@ size_t word_offset(const fa_decode_args& a) { return (decode_workspace_bytes(a) 
 // 24 prompts of 17 to 2048 tokens, 32 heads over 8 of 128, 385 -> 358; of 7 of 67 to 540, 32 heads of 64, 56 -> 31; forward and
 // backward of 14 of 64, 32 heads of 64, 127 -> 92; of 23 of 261 to 522, 16 heads of 128, 268 -> 235.
 int varlen_check(const int32_t* cu_q, const int32_t* cu_k, int batch, int64_t total_q, int64_t total_k, bool k_at_most, int64_t max_q,
-                 int64_t max_k, int32_t* ticket, cudaStream_t st) {
+                 int64_t max_k, int device, int32_t* ticket, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     cudaGetLastError();
@@ -1170,7 +1170,7 @@ int varlen_check(const int32_t* cu_q, const int32_t* cu_k, int batch, int64_t to
     return FA_ERR_LAUNCH;
   }
   uint32_t* host = nullptr;
-  const int slot = take_slot(true, &host);
+  const int slot = take_slot(true, device, &host);
   if (slot < 0) return FA_ERR_UNSUPPORTED;
   varlen_check_kernel<<<1, batch > 128 ? 1024 : 128, 0, st>>>(cu_q, cu_k, batch, total_q, total_k, k_at_most, max_q, max_k, host);
   if (int r = check_launch("varlen_check")) {
@@ -1180,10 +1180,15 @@ int varlen_check(const int32_t* cu_q, const int32_t* cu_k, int batch, int64_t to
   *ticket = slot;
   return FA_OK;
 }
+// The caller's current device may be another by now, and a stream of that device (0 is one of each) would be asked about
+// a kernel that it never had.
 int check_result(int32_t ticket, uint32_t* failed, cudaStream_t st) {
-  FA_REQUIRE(g_slots.hand_in(ticket), "ticket %d is not out", ticket);
-  const int r = await_slot(ticket, failed, st);
+  int device = -1, current = -1;
+  FA_REQUIRE(g_slots.hand_in(ticket, &device), "ticket %d is not out", ticket);
+  int r = cudaGetDevice(&current) == cudaSuccess ? ensure_device(device) : FA_ERR_LAUNCH;
+  if (r == FA_OK) r = await_slot(ticket, failed, st);
   g_slots.give(ticket, true);
+  if (current >= 0 && current != device) cudaSetDevice(current);
   return r;
 }
 
@@ -1209,7 +1214,7 @@ int decode_paged_checked(const fa_decode_args& a, uint32_t* failed, cudaStream_t
   const bool host_order = k.word && word == nullptr;   // no room for the word: launch nothing before the result is here
   if (host_order) k.inside = false;
   uint32_t* host = nullptr;
-  const int slot = take_slot(false, &host);
+  const int slot = take_slot(false, a.device, &host);
   if (slot < 0) return FA_ERR_LAUNCH;
   int r = FA_OK;
   bool queued = false;                                 // a kernel that writes the host word is on the stream

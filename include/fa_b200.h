@@ -243,7 +243,8 @@ int fa_decode_paged_checked(const fa_decode_args* args, uint32_t* failed, void* 
  * cu_seqlens arrays (batch + 1 entries) and gives a ticket; fa_check_result waits until that kernel has run -- not for what
  * is queued behind it -- and returns the checks that did not hold.  Every ticket is handed in exactly once; one that is not
  * out is refused.  FA_ERR_UNSUPPORTED: no mapped host memory, or FA_VARLEN_TICKETS tickets are out in this process; the
- * caller has to look at the values itself.  Not for streams under capture.
+ * caller has to look at the values itself.  Not for streams under capture.  fa_check_result takes the stream of the check and
+ * may be called with any device current.
  */
 #define FA_VARLEN_TICKETS 128
 typedef enum fa_varlen_check_bit {

@@ -13,8 +13,10 @@ using Slots = fa::CheckSlots<8, 4>;
 extern "C" {
 void* make() { for (int i = 0; i < 8; ++i) words[i * 16] = 0u; return new Slots(words); }
 void drop(void* s) { delete static_cast<Slots*>(s); }
-int take(void* s, int ticket) { return static_cast<Slots*>(s)->take(ticket != 0); }
-int hand_in(void* s, int i) { return static_cast<Slots*>(s)->hand_in(i); }
+int take_on(void* s, int ticket, int device) { return static_cast<Slots*>(s)->take(ticket != 0, device); }
+int take(void* s, int ticket) { return take_on(s, ticket, 0); }
+int device_of(void* s, int i) { int d = -1; return static_cast<Slots*>(s)->hand_in(i, &d) ? d : -1; }
+int hand_in(void* s, int i) { return device_of(s, i) >= 0; }
 void give(void* s, int i, int queued) { static_cast<Slots*>(s)->give(i, queued != 0); }
 void answer(int i) { *Slots::word_of(words, i) = 1u; }
 int word(int i) { return (int)*Slots::word_of(words, i); }
@@ -31,8 +33,8 @@ def lib(tmp_path_factory):
                     str(d / "slots.so")], check=True)
     m = C.CDLL(str(d / "slots.so"))
     m.make.restype = C.c_void_p
-    for f in (m.drop, m.take, m.hand_in, m.give):
-        f.argtypes = [C.c_void_p] + [C.c_int] * {"drop": 0, "take": 1, "hand_in": 1, "give": 2}[f.__name__]
+    for f in (m.drop, m.take, m.hand_in, m.give, m.device_of, m.take_on):
+        f.argtypes = [C.c_void_p] + [C.c_int] * {"drop": 0, "take": 1, "hand_in": 1, "give": 2, "device_of": 1, "take_on": 2}[f.__name__]
     return m
 
 
@@ -87,3 +89,14 @@ def test_no_wait_for_words_that_only_tickets_hold(lib, s):
     for _ in range(4):
         lib.give(s, lib.take(s, 0), 1)
     assert lib.take(s, 0) == NEVER
+
+
+def test_a_ticket_knows_its_device(lib, s):
+    """The thread that hands it in may have another device current."""
+    out = {lib.take_on(s, 1, d): d for d in (3, 0, 7)}
+    lib.give(s, lib.take_on(s, 0, 5), 0)
+    for i, d in out.items():
+        lib.answer(i)
+        assert lib.device_of(s, i) == d and lib.device_of(s, i) == -1
+        lib.give(s, i, 1)
+    assert lib.device_of(s, lib.take_on(s, 1, 2)) == 2
