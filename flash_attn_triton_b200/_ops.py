@@ -191,11 +191,11 @@ def varlen_attention(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, s
     """Packed sequences: q (Tq,Hq,D), k/v (Tk,Hkv,D), int32 cu_seqlens on the device; differentiable.  `checks`: the
     values of cu_seqlens are looked at, on the device, before the attention is launched."""
     f = feat or _NO_FEATURES
-    tail = (impl, f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse, checks)
+    tail = (impl, f.dropout_p, f.seed, f.row_stride, f.seqused_q, f.seqused_k, want_lse)
     if _tracing() is not None:
         return _TracedCall.apply(lambda q, k, v, cu_q, cu_k, alibi: N.host().varlen(
-            q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail), q, k, v, cu_q, cu_k, alibi)
-    return N.host().varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, *tail)
+            q, k, v, cu_q, cu_k, max_q, max_k, checks, scale, causal, wl, wr, softcap, alibi, *tail), q, k, v, cu_q, cu_k, alibi)
+    return N.host().varlen(q, k, v, cu_q, cu_k, max_q, max_k, checks, scale, causal, wl, wr, softcap, alibi, *tail)
 
 
 def varlen_forward(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,

@@ -238,6 +238,7 @@ class VarlenCheck {
                                      max_q, max_k, q.device().index(), &ticket_, stream_);
     if (r != FA_ERR_UNSUPPORTED) {
       check(r, "fa_varlen_check");
+      open_ = true;
       return;
     }
     // no mapped host memory, or too many tickets out: by a copy
@@ -250,9 +251,12 @@ class VarlenCheck {
       if (lq > max_q || lk > max_k) failed_ |= FA_VARLEN_LONGEST;
     }
     if (a[n] != q.size(0) || (k_at_most ? b[n] > k.size(0) : b[n] != k.size(0))) failed_ |= FA_VARLEN_COVER;
+    open_ = true;
   }
-  // Raises what the values are refused for.
+  // Raises what the values are refused for, once.
   void finish() {
+    if (!open_) return;
+    open_ = false;
     check(result(), "fa_check_result");
     const char* what = failed_ & FA_VARLEN_START     ? "cu_seqlens arrays must start at zero and contain a batch boundary"
                        : failed_ & FA_VARLEN_ORDER   ? "cu_seqlens arrays must be monotonically non-decreasing"
@@ -282,6 +286,7 @@ class VarlenCheck {
     failed_ |= bad;
     return r;
   }
+  bool open_ = false;              // checks made or under way, the answer not looked at yet
   int32_t ticket_ = -1;
   uint32_t failed_ = 0;
   void* stream_ = nullptr;
@@ -536,9 +541,10 @@ PyObject* py_dense(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// varlen(q, k, v, cu_q, cu_k, max_q, max_k, scale, causal, wl, wr, softcap, alibi, impl,
-//        dropout_p, seed, row_stride, used_q, used_k, want_lse, checks) -> out | (out, lse2)
-// checks: 0 none, 1 the values of cu_seqlens, 2 the same with rows of k and v past the last sequence
+// varlen(q, k, v, cu_q, cu_k, max_q, max_k, checks, scale, causal, wl, wr, softcap, alibi, impl,
+//        dropout_p, seed, row_stride, used_q, used_k, want_lse) -> out | (out, lse2)
+// checks: 0 none, 1 the values of cu_seqlens, 2 the same with rows of k and v past the last sequence.  What they are refused for
+// comes before anything else that the call is refused for.
 PyObject* py_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   Args a{args, n};
@@ -550,26 +556,35 @@ PyObject* py_varlen(PyObject*, PyObject* const* args, Py_ssize_t n) {
   c.cu_k = a.tensor();
   c.max_q = (int)a.integer();
   c.max_k = (int)a.integer();
-  score_params(a, c);
-  c.impl = (int)a.integer();
-  c.dropout_p = a.real();
-  c.seed = (uint64_t)a.integer();
-  c.row_stride = (int)a.integer();
-  c.used_q = a.tensor_or_none();
-  c.used_k = a.tensor_or_none();
-  const bool want_lse = a.truth();
   const int checks = (int)a.integer();
-  Tensor lse;
   VarlenCheck values;
   if (checks != 0) {
     c10::cuda::CUDAGuard guard(in[0].device());
     at::AutoDispatchBelowADInplaceOrView below;
     values.start(in[0], in[1], c.cu_q, c.cu_k, checks == 2, c.max_q, c.max_k);
   }
-  Tensor out = with_grad(c, std::move(in), want_lse, lse, [&](const variable_list& x, bool w, Tensor& o, Tensor& l) {
-    run_forward(c, x, w, o, l, checks != 0 ? &values : nullptr);
-  });
-  return result(out, lse, want_lse);
+  try {
+    score_params(a, c);
+    c.impl = (int)a.integer();
+    c.dropout_p = a.real();
+    c.seed = (uint64_t)a.integer();
+    c.row_stride = (int)a.integer();
+    c.used_q = a.tensor_or_none();
+    c.used_k = a.tensor_or_none();
+    const bool want_lse = a.truth();
+    Tensor lse;
+    Tensor out = with_grad(c, std::move(in), want_lse, lse, [&](const variable_list& x, bool w, Tensor& o, Tensor& l) {
+      run_forward(c, x, w, o, l, &values);
+    });
+    return result(out, lse, want_lse);
+  } catch (python_error& e) {
+    e.persist();
+    values.finish();
+    throw;
+  } catch (...) {
+    values.finish();
+    throw;
+  }
   END_HANDLE_TH_ERRORS
 }
 

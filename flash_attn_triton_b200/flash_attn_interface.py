@@ -465,7 +465,13 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
             checks = _ops.VARLEN_UNCHECKED
     if max_seqlen_q == 0 or max_seqlen_k == 0:
         return q.new_zeros((q.shape[0], q.shape[1], q.shape[2]))
-    alibi = _normalise_alibi(alibi_slopes, batch_size, q.shape[1], q.device)
+    try:
+        alibi = _normalise_alibi(alibi_slopes, batch_size, q.shape[1], q.device)
+        window_left, window_right = window_size[0], window_size[1]
+    except Exception:
+        if checks != _ops.VARLEN_UNCHECKED:      # what the values are refused for comes first
+            _ops.varlen_check(q, k, cu_seqlens_q, cu_seqlens_k, longest_q, longest_k, checks)
+        raise
     out_dtype = q.dtype
     q, k, v = _as_kernel_dtype(q, k, v)
     if softmax_scale is None:
@@ -511,7 +517,7 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
         feat = _ops.Features(dropout_p=dropout_p, seed=random.randrange(2 ** 31 - 1) if dropout_p else 0,
                              row_stride=int(max_seqlen_k), seqused_q=used_q, seqused_k=used_k)
     args = (cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), softmax_scale, causal,
-            window_size[0], window_size[1], softcap, alibi)
+            window_left, window_right, softcap, alibi)
     if return_attn_probs:
         out, lse2 = _ops.varlen_attention(q, k, v, *args, N.IMPL_AUTO, feat, True, checks)
         probs, lse = _ops.varlen_probs(q.detach(), k.detach(), v.detach(), lse2, *args, feat)

@@ -214,6 +214,31 @@ def test_values_of_cu_seqlens_are_checked(batch, dtype):
     torch.cuda.current_stream().wait_stream(side)
 
 
+def test_what_the_values_are_refused_for_comes_first():
+    """Calls that are wrong in two ways: cu_seqlens, and something that is looked at behind them."""
+    import torch.autograd.forward_ad as fwad
+    q = torch.randn(64, 2, 64, device=DEV, dtype=torch.half)
+    good = torch.tensor([0, 30, 64], dtype=torch.int32, device=DEV)
+    bad = torch.tensor([1, 30, 64], dtype=torch.int32, device=DEV)
+    call = lambda cu, x=q, **kw: fa().flash_attn_varlen_func(x, q, q, cu, good, 34, 34, **kw)
+    want = call(good)
+    slopes = torch.ones(3, device=DEV)
+    for kw, own in ((dict(alibi_slopes=slopes), ValueError), (dict(window_size=(3,)), IndexError), (dict(window_size=("a", 1)), TypeError),
+                    (dict(softmax_scale="a"), TypeError)):
+        with pytest.raises(ValueError, match="start at zero"):
+            call(bad, **kw)
+        with pytest.raises(own) as e:
+            call(good, **kw)
+        assert "start at zero" not in str(e.value)
+    with fwad.dual_level():
+        x = fwad.make_dual(q, torch.ones_like(q))
+        with pytest.raises(ValueError, match="start at zero"):
+            call(bad, x)
+        with pytest.raises(NotImplementedError):
+            call(good, x)
+    assert torch.equal(call(good), want)
+
+
 @pytest.mark.parametrize("where", ["cpu", DEV])
 @pytest.mark.parametrize("dtype", [torch.int32, torch.int64, torch.int16])
 def test_longest_sequence_as_a_tensor(dtype, where):
