@@ -24,10 +24,10 @@
 //   same order.
 //   Latency.  A small step is one chain: lengths, piece, tiles and Q, the append, the merge of the warps, the merge of the
 //   pieces.  So Q and the new tokens are read and rotated 16 bytes at a time (they came element by element), what the
-//   append reads is fetched to L1 under the first tiles, the warps write their outputs side by side and add them up after
-//   one barrier (not in four turns), and sixteen pieces are merged per trip to L2.  Kernel time, before -> after (us):
-//   1 x 1900 tokens, 32 heads over 8 of 128: 15.2 -> 12.2; 28 x 66 to 2112, 8 over 2: 20.0 -> 15.9; 47 x 192, 2 new tokens, 32
-//   over 8 of 64: 22.6 -> 17.1; 4 x 600 to 2400, 4 new tokens, 16 over 4 of 128: 34.7 -> 21.1; 17 x 18450, 8 over 2: 68.9 -> 63.5.
+//   append reads is fetched to L1 under the first tiles, and the warps write their outputs side by side and add them up after
+//   one barrier (not in four turns).  Kernel time, before -> after (us): 1 x 1900 tokens, 32 heads over 8 of 128: 15.1 -> 11.9;
+//   28 x 66 to 2112, 8 over 2: 20.0 -> 15.0; 47 x 192, 2 new tokens, 32 over 8 of 64: 22.5 -> 16.8; 4 x 600 to 2400, 4 new
+//   tokens, 16 over 4 of 128: 34.7 -> 20.7; 17 x 18450, 8 over 2: 69.0 -> 63.1.
 //   Value checks of the public call run at the start of the same kernel while the tables are small (one
 //   decode step of a few sequences is bounded by launches: 17 small kernels, a copy and a
 //   synchronisation took 150 us around a 16 us kernel), in decode_check_kernel otherwise.
@@ -142,6 +142,19 @@ __device__ __forceinline__ T rotary_elem(F get, int d, const T* cos, const T* si
   return first ? hsub_rn(hmul_rn(x, c), hmul_rn(y, s)) : hadd_rn(hmul_rn(y, s), hmul_rn(x, c));
 }
 
+// The general case of the next: pairs side by side, halves or tables that 16-byte reads do not fit.  Out of line: eight
+// rotary_elem() in the main loop of decode_kernel cost its registers and its order of loads (head_dim 256, 32 x 8000
+// tokens, 16 heads over 4: 268 -> 233 us).
+template <typename T>
+__device__ __noinline__ uint4 rotary_chunk_any(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
+                                               int interleaved, int rotary_seqlen) {
+  union { uint4 v; T e[8]; } out;
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    out.e[k] = rotary_elem<T>([&](int j) { return x[j]; }, d + k, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+  return out.v;
+}
+
 // 8 elements of a head row, rotated like rotary_elem.
 template <typename T>
 __device__ __forceinline__ uint4 rotary_chunk(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
@@ -150,21 +163,17 @@ __device__ __forceinline__ uint4 rotary_chunk(const T* x, int d, const T* cos, c
   self.v = *reinterpret_cast<const uint4*>(x + d);
   if (cos == nullptr || d >= rotary_dim || pos < 0 || pos >= rotary_seqlen) return self.v;
   const int half = rotary_dim >> 1;
-  if (!interleaved && half % 8 == 0 && ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 15) == 0) {
-    const bool first = d < half;
-    const int i = first ? d : d - half;
-    other.v = *reinterpret_cast<const uint4*>(x + (first ? d + half : d - half));
-    c.v = *reinterpret_cast<const uint4*>(cos + (int64_t)pos * half + i);
-    s.v = *reinterpret_cast<const uint4*>(sin + (int64_t)pos * half + i);
-#pragma unroll
-    for (int k = 0; k < 8; ++k)
-      out.e[k] = first ? hsub_rn(hmul_rn(self.e[k], c.e[k]), hmul_rn(other.e[k], s.e[k]))
-                       : hadd_rn(hmul_rn(other.e[k], s.e[k]), hmul_rn(self.e[k], c.e[k]));
-    return out.v;
-  }
+  if (interleaved || half % 8 != 0 || ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 15) != 0)
+    return rotary_chunk_any<T>(x, d, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+  const bool first = d < half;
+  const int i = first ? d : d - half;
+  other.v = *reinterpret_cast<const uint4*>(x + (first ? d + half : d - half));
+  c.v = *reinterpret_cast<const uint4*>(cos + (int64_t)pos * half + i);
+  s.v = *reinterpret_cast<const uint4*>(sin + (int64_t)pos * half + i);
 #pragma unroll
   for (int k = 0; k < 8; ++k)
-    out.e[k] = rotary_elem<T>([&](int j) { return x[j]; }, d + k, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+    out.e[k] = first ? hsub_rn(hmul_rn(self.e[k], c.e[k]), hmul_rn(other.e[k], s.e[k]))
+                     : hadd_rn(hmul_rn(other.e[k], s.e[k]), hmul_rn(self.e[k], c.e[k]));
   return out.v;
 }
 
@@ -216,9 +225,10 @@ __device__ __forceinline__ SeqTiles seq_tiles(const fa_decode_args& p, const Sco
   return s;
 }
 
-// Elements [d, d + 4) of one output row, merged from the `parts` workspace rows r0, r0 + step, ...  Sixteen
-// pieces are loaded at a time (a small step seldom has more: one trip to L2), their common maximum taken first.
-constexpr int kMergeBatch = 16;
+// Elements [d, d + 4) of one output row, merged from the `parts` workspace rows r0, r0 + step, ...  Eight
+// pieces are loaded at a time, their common maximum taken first.  (Sixteen: longer code in front of few rows, -1 to
+// +7 % of a step's time at every head size -- 2 x 411 tokens, one head of 64: 9.7 -> 10.6 us.)
+constexpr int kMergeBatch = 8;
 template <typename T, int D>
 __device__ __forceinline__ void merge_pieces(const float* ws_o, const float* ws_l, int64_t r0, int64_t step, int parts, int d,
                                              T* og) {

@@ -230,11 +230,11 @@ def test_unchecked_lengths_stay_inside_the_cache(tokens, padded):
         assert torch.equal(t[2, :cap - 1], was[2, :cap - 1]) and torch.equal(t[2, cap - 1], new[1, 0])
 
 
-@pytest.mark.parametrize("pieces", [15, 16, 17, 33])
+@pytest.mark.parametrize("pieces", [7, 8, 9, 16, 17, 33])
 @pytest.mark.parametrize("D,rotary,interleaved,tokens", [(64, 24, False, 1), (64, 24, True, 3), (64, 48, False, 2), (128, 128, False, 2),
                                                          (128, 96, True, 1), (16, 16, False, 4), (256, 256, False, 1)])
 def test_merge_batches_and_rotated_chunks(pieces, D, rotary, interleaved, tokens):
-    """Numbers of pieces around the 16 that are merged at a time; rotary dimensions that end inside a 16-byte chunk, new tokens
+    """Numbers of pieces around the 8 that are merged at a time, and twice that; rotary dimensions that end inside a 16-byte chunk, new tokens
     in the last tile and across two of them.  The cache rows are the reference's arithmetic to the last bit."""
     cap, lens, Hq, Hkv = 2304, [2300 - tokens, 63 if tokens > 1 else 2111, 0], 8, 4
     q, kc, vc, kn, vn = _contig_case(pieces + D + rotary, 3, 3, cap, Hq, Hkv, D, tokens, tokens)
