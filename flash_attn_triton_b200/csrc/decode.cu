@@ -142,29 +142,79 @@ __device__ __forceinline__ T rotary_elem(F get, int d, const T* cos, const T* si
   return first ? hsub_rn(hmul_rn(x, c), hmul_rn(y, s)) : hadd_rn(hmul_rn(y, s), hmul_rn(x, c));
 }
 
-// The general case of the next: pairs side by side, halves or tables that 16-byte reads do not fit.  Out of line: eight
-// rotary_elem() in the main loop of decode_kernel cost its registers and its order of loads (head_dim 256, 32 x 8000
-// tokens, 16 heads over 4: 268 -> 233 us).
+// Whether rotary_chunk() can read 16 (pairs side by side: 8) bytes of the tables at a time.
 template <typename T>
-__device__ __noinline__ uint4 rotary_chunk_any(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
-                                               int interleaved, int rotary_seqlen) {
-  union { uint4 v; T e[8]; } out;
+__device__ __forceinline__ bool rotary_in_chunks(const T* cos, const T* sin, int rotary_dim, int interleaved) {
+  return (rotary_dim & (interleaved ? 7 : 15)) == 0 &&
+         ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & (interleaved ? 7 : 15)) == 0;
+}
+
+// The others: halves that are multiples of 4 by 8 bytes, the rest element by element.
+template <typename T>
+__device__ __forceinline__ uint4 rotary_chunk_any(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
+                                                  int interleaved, int rotary_seqlen) {
+  union { uint4 v; uint2 h[2]; T e[8]; } out;
+  const int half = rotary_dim >> 1;
+  if (!interleaved && half % 4 == 0 && ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 7) == 0) {
+    union Four { uint2 v; T e[4]; };
+    out.v = *reinterpret_cast<const uint4*>(x + d);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int at = d + 4 * h;
+      if (at >= rotary_dim) break;
+      const bool first = at < half;
+      const int64_t i = (int64_t)pos * half + (first ? at : at - half);
+      Four self, other, c, s;
+      self.v = out.h[h];
+      other.v = *reinterpret_cast<const uint2*>(x + (first ? at + half : at - half));
+      c.v = *reinterpret_cast<const uint2*>(cos + i);
+      s.v = *reinterpret_cast<const uint2*>(sin + i);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        self.e[k] = first ? hsub_rn(hmul_rn(self.e[k], c.e[k]), hmul_rn(other.e[k], s.e[k]))
+                          : hadd_rn(hmul_rn(other.e[k], s.e[k]), hmul_rn(self.e[k], c.e[k]));
+      out.h[h] = self.v;
+    }
+    return out.v;
+  }
 #pragma unroll
   for (int k = 0; k < 8; ++k)
     out.e[k] = rotary_elem<T>([&](int j) { return x[j]; }, d + k, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
   return out.v;
 }
-
-// 8 elements of a head row, rotated like rotary_elem.
 template <typename T>
+__device__ __noinline__ uint4 rotary_chunk_call(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
+                                                int interleaved, int rotary_seqlen) {
+  return rotary_chunk_any(x, d, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+}
+
+// 8 elements of a head row, rotated like rotary_elem.  kCall: the general case out of line.  In the main loop of decode_kernel
+// it cost registers and the order of the loads (head_dim 256, 32 x 8000 tokens, 16 heads over 4: 268 us, 233 as a call); a
+// kernel that only rotates and copies is better off without the call (4 x 256 tokens behind 300, 32 heads over 8 of 128, with
+// their attention: 42 us, 46).  Pairs side by side need no row beside the one at hand and half as much of the tables: 8 x 900
+// tokens, 4 new, 16 heads over 4 of 128: element by element 30.4 us, as eight calls 20.6, now 16.6.
+template <typename T, bool kCall>
 __device__ __forceinline__ uint4 rotary_chunk(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
                                               int interleaved, int rotary_seqlen) {
   union { uint4 v; T e[8]; } out, self, other, c, s;
   self.v = *reinterpret_cast<const uint4*>(x + d);
   if (cos == nullptr || d >= rotary_dim || pos < 0 || pos >= rotary_seqlen) return self.v;
+  if (!rotary_in_chunks(cos, sin, rotary_dim, interleaved)) {
+    if (kCall) return rotary_chunk_call(x, d, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+    return rotary_chunk_any(x, d, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+  }
   const int half = rotary_dim >> 1;
-  if (interleaved || half % 8 != 0 || ((reinterpret_cast<uintptr_t>(cos) | reinterpret_cast<uintptr_t>(sin)) & 15) != 0)
-    return rotary_chunk_any<T>(x, d, cos, sin, pos, rotary_dim, interleaved, rotary_seqlen);
+  if (interleaved) {
+    *reinterpret_cast<uint2*>(c.e) = *reinterpret_cast<const uint2*>(cos + (int64_t)pos * half + (d >> 1));
+    *reinterpret_cast<uint2*>(s.e) = *reinterpret_cast<const uint2*>(sin + (int64_t)pos * half + (d >> 1));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const T x0 = self.e[2 * k], x1 = self.e[2 * k + 1];
+      out.e[2 * k] = hsub_rn(hmul_rn(x0, c.e[k]), hmul_rn(x1, s.e[k]));
+      out.e[2 * k + 1] = hadd_rn(hmul_rn(x0, s.e[k]), hmul_rn(x1, c.e[k]));
+    }
+    return out.v;
+  }
   const bool first = d < half;
   const int i = first ? d : d - half;
   other.v = *reinterpret_cast<const uint4*>(x + (first ? d + half : d - half));
@@ -487,7 +537,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
       const int sq = gr / G, gi = gr % G;
       const T* qrow = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + sq * p.q_stride[1] +
                       (int64_t)(hk * G + gi) * p.q_stride[2];
-      val = rotary_chunk<T>(qrow, d, cos, sin, len - p.seqlen_q + sq + pad, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+      val = rotary_chunk<T, true>(qrow, d, cos, sin, len - p.seqlen_q + sq + pad, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
     }
     *reinterpret_cast<uint4*>(sQ + r * P + d) = val;
   }
@@ -552,7 +602,7 @@ __global__ void __launch_bounds__(128, D <= 128 ? 2 : 1)
         const T* kn = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + hk * p.kn_stride[2];
         const T* vn = reinterpret_cast<const T*>(p.v_new) + b * p.vn_stride[0] + tok * p.vn_stride[1] + hk * p.vn_stride[2];
         const uint4 vv = *reinterpret_cast<const uint4*>(vn + d);
-        const uint4 kv = rotary_chunk<T>(kn, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+        const uint4 kv = rotary_chunk<T, true>(kn, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
         *reinterpret_cast<uint4*>(tK + (key - keyw) * P + d) = kv;
         *reinterpret_cast<uint4*>(tV + (key - keyw) * P + d) = vv;
         if (rg == 0 && pos < cache_capacity(p)) {
@@ -798,7 +848,7 @@ __global__ void __launch_bounds__(256, 5) cache_append_kernel(const fa_decode_ar
       const int pos = p.cache_seqlens[b] + n_new - p.seqlen_q + tok + (p.cache_leftpad ? p.cache_leftpad[b] : 0);
       const T* x = reinterpret_cast<const T*>(p.q) + b * p.q_stride[0] + tok * p.q_stride[1] + h * p.q_stride[2];
       *reinterpret_cast<uint4*>(q_out + (int64_t)i * 8) =
-          rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+          rotary_chunk<T, false>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
       continue;
     }
     i -= nq;
@@ -815,7 +865,7 @@ __global__ void __launch_bounds__(256, 5) cache_append_kernel(const fa_decode_ar
     } else {
       const T* x = reinterpret_cast<const T*>(p.k_new) + b * p.kn_stride[0] + tok * p.kn_stride[1] + h * p.kn_stride[2];
       T* dst = reinterpret_cast<T*>(p.k_cache) + cache_row_offset(p, b, pos, page_shift, p.kc_stride) + h * p.kc_stride[2];
-      *reinterpret_cast<uint4*>(dst + d) = rotary_chunk<T>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
+      *reinterpret_cast<uint4*>(dst + d) = rotary_chunk<T, false>(x, d, cos, sin, pos, p.rotary_dim, p.rotary_interleaved, p.rotary_seqlen);
     }
   }
 }

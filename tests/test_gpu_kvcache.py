@@ -262,3 +262,31 @@ def test_appended_chunks_of_more_steps_than_one(B, tokens, Hq, Hkv, D, rotary):
                                        rotary_interleaved=False)
     assert maxdiff(out, ro) <= util.FWD_TOL
     assert torch.equal(kcd.cpu(), rkc) and torch.equal(vcd.cpu(), rvc)
+
+
+@pytest.mark.parametrize("tokens", [2, 40])            # a decode step, and a chunk with an append kernel of its own
+@pytest.mark.parametrize("interleaved", [True, False])
+@pytest.mark.parametrize("shift", [0, 1, 2, 4])        # elements from a 16-byte boundary to the tables
+@pytest.mark.parametrize("D,rotary", [(64, 64), (64, 56), (64, 40), (64, 24), (64, 20), (64, 8), (64, 6), (64, 2), (128, 104), (256, 128)])
+def test_rotary_dimensions_and_table_addresses(D, rotary, shift, interleaved, tokens):
+    """Every way in which rows are read and rotated: 16, 8 or 2 bytes of the tables at a time, by the rotary dimension and by where
+    the tables lie.  The cache rows are the reference's arithmetic to the last bit."""
+    B, Hq, Hkv, lens = 3, 8, 4, [70, 0, 129]
+    cap = max(lens) + tokens
+    q, kc, vc, kn, vn = _contig_case(D + rotary + tokens, B, B, cap, Hq, Hkv, D, tokens, tokens)
+    cl = torch.tensor(lens, dtype=torch.int32)
+    cos, sin = cases.rotary_tables(cap, rotary)
+
+    def placed(t):
+        buf = torch.zeros(t.numel() + 8, dtype=t.dtype, device=DEV)
+        assert buf.data_ptr() % 16 == 0
+        out = buf[shift:shift + t.numel()].view(t.shape)
+        out.copy_(t)
+        return out
+
+    ro, rkc, rvc = orc.kvcache_ref(q, kc, vc, kn, vn, cos, sin, cache_seqlens=cl, causal=True, rotary_interleaved=interleaved)
+    kcd, vcd = kc.to(DEV), vc.to(DEV)
+    out = fa().flash_attn_with_kvcache(dev(q), kcd, vcd, dev(kn), dev(vn), placed(cos), placed(sin), cache_seqlens=dev(cl), causal=True,
+                                       rotary_interleaved=interleaved)
+    assert maxdiff(out, ro) <= util.FWD_TOL
+    assert torch.equal(kcd.cpu(), rkc) and torch.equal(vcd.cpu(), rvc)
