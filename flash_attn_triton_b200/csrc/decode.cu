@@ -33,6 +33,7 @@
 //   synchronisation took 150 us around a 16 us kernel), in decode_check_kernel otherwise.
 #include <sched.h>
 
+#include <atomic>
 #include <cmath>
 #include <mutex>
 #include <type_traits>
@@ -961,10 +962,16 @@ static int launch_rows(const fa_decode_args& a, const ScoreCfg& cfg, const Decod
                          cudaStream_t st) {
   const size_t smem = DecodeSmem<D, kRows>::fixed;
   auto kern = decode_kernel<T, D, kRows>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    set_error("decode: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    return FA_ERR_LAUNCH;
+  // once per kernel and device: a step of one conversation is bounded by the host's part
+  static std::atomic<uint64_t> prepared{0};
+  const uint64_t bit = a.device < 64 ? 1ull << a.device : 0;
+  if ((prepared.load(std::memory_order_relaxed) & bit) == 0) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+      set_error("decode: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      return FA_ERR_LAUNCH;
+    }
+    prepared.fetch_or(bit, std::memory_order_relaxed);
   }
   cudaLaunchConfig_t lc = {};
   cudaLaunchAttribute attr;
@@ -1114,35 +1121,38 @@ namespace {
 CheckSlots<kCheckSlots, kTickets> g_slots(g_check_host);
 volatile uint32_t* slot_word(int i) { return g_slots.word_of(g_check_host, i); }
 
-// The words as the current device sees them, null (error set) without mapped host memory.  Tried again by the next call where it fails
-// (another thread may be capturing a graph right now).
-uint32_t* check_words() {
+// The words as `device`, the current one, sees them; null (error set) without mapped host memory.  Tried again by the next call
+// where it fails (another thread may be capturing a graph right now).
+uint32_t* check_words(int device) {
+  static std::atomic<uint32_t*> words[64];
+  const bool kept = device >= 0 && device < 64;
+  if (kept)
+    if (uint32_t* w = words[device].load(std::memory_order_acquire)) return w;
   static std::mutex mu;
   static bool mapped = false;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!mapped) {
-      const cudaError_t e = cudaHostRegister(const_cast<uint32_t*>(g_check_host), sizeof(g_check_host),
-                                             cudaHostRegisterPortable | cudaHostRegisterMapped);
-      if (e != cudaSuccess) {
-        cudaGetLastError();
-        set_error("no mapped host memory for the value checks: %s", cudaGetErrorString(e));
-        return nullptr;
-      }
-      mapped = true;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!mapped) {
+    const cudaError_t e = cudaHostRegister(const_cast<uint32_t*>(g_check_host), sizeof(g_check_host),
+                                           cudaHostRegisterPortable | cudaHostRegisterMapped);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      set_error("no mapped host memory for the value checks: %s", cudaGetErrorString(e));
+      return nullptr;
     }
+    mapped = true;
   }
   void* h = nullptr;
   if (cudaHostGetDevicePointer(&h, const_cast<uint32_t*>(g_check_host), 0) != cudaSuccess) {
     set_error("value checks: cudaHostGetDevicePointer: %s", cudaGetErrorString(cudaGetLastError()));
     return nullptr;
   }
+  if (kept) words[device].store(static_cast<uint32_t*>(h), std::memory_order_release);
   return static_cast<uint32_t*>(h);
 }
 
 // Index of a slot, its word at *dptr; -1 (error set) without one.  A call waits for another call's, a ticket does not.
 int take_slot(bool ticket, int device, uint32_t** dptr) {
-  uint32_t* words = check_words();
+  uint32_t* words = check_words(device);
   if (words == nullptr) return -1;
   for (;;) {
     const int i = g_slots.take(ticket, device);
