@@ -14,10 +14,11 @@
 // in the in-order tensor pipe.  At head_dim 64 the accumulator leaves 64 columns, which P has to itself: Q K_{j+1}^T follows
 // as soon as the scores of tile j are in registers and runs under their exponentials, where it came behind P V_j, with
 // nothing of this CTA to do meanwhile (us, before -> after: 4 x 32 heads x 1024 x 1531 92.1 -> 88.0, 4 x 16 x 4096 causal 225 -> 219,
-// 8 x 16 x 512 with dropout 25.3 -> 24.3, 24 packed of 64 to 2048 211 -> 206; rows of two or three tiles +-1 %).  Arithmetic, order of the tiles and of the sums are those of the two-tile kernels
+// 8 x 16 x 512 with dropout 25.3 -> 24.3, 24 packed of 64 to 2048 211 -> 206); rows that are too short for that keep P over S
+// (p_over_s_is_faster).  Arithmetic, order of the tiles and of the sums are those of the two-tile kernels
 // (fwd_sm100.cu, fwd_persist_sm100.cu): results are equal bit for bit.
 //
-// TMEM (256 columns): S (128) | O (head_dim) | at head_dim 64 P (64).  Every mbarrier wait is bounded.
+// TMEM (256 columns): S (128) | O (head_dim) | P of its own (64).  Every mbarrier wait is bounded.
 #include <type_traits>
 
 #include "common.cuh"
@@ -52,9 +53,9 @@ struct DShared {
   uint64_t kv_full[4];
   uint64_t kv_empty[4];
   uint64_t s_full;         // scores computed
-  uint64_t s_free;         // head_dim 64: scores in registers (128 arrivals)
+  uint64_t s_free;         // P in columns of its own: scores in registers (128 arrivals)
   // (Barriers that count threads: none may arrive for a phase before the one ahead of it is complete.  For P: the next
-  // scores, which a thread needs first, are issued behind p_ready -- at head_dim 64 behind s_free, but a thread writes
+  // scores, which a thread needs first, are issued behind p_ready -- with kOwnP behind s_free, but a thread writes
   // P only when the P V before, which was issued behind p_ready, has finished.)
   uint64_t p_half;         // the first 64 keys of P written back (128 arrivals)
   uint64_t p_ready;        // P written back (128 arrivals)
@@ -74,15 +75,15 @@ template <> struct DFmt<__nv_bfloat16> { static constexpr int code = 1; };
 }  // namespace
 
 // kDrop: probabilities whose bit in cfg.keep is 0 do not enter P V (they stay in the row sum); the scale of
-// the kept ones goes into the normalisation of the output.
-template <typename T, int D, Feat kFeat, bool kDrop>
+// the kept ones goes into the normalisation of the output.  kOwnP: P in columns of its own (head_dim 64).
+template <typename T, int D, Feat kFeat, bool kDrop, bool kOwnP>
 __global__ void __launch_bounds__(kThreads, 2)
 fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                      const fa_attn_args p, const ScoreCfg cfg, int* const host_status) {
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr bool kPvSplit = !kExtras;     // P V in two key halves (measured: helps the plain variants only)
-  constexpr bool kOwnP = D == 64;         // P in columns of its own
+  static_assert(!kOwnP || D == 64, "at head_dim 128 S and O fill the columns");
   constexpr int kPCol = kOwnP ? kBN + D : 0;
   using C = DCfg<D>;
   constexpr int S = C::kStages;
@@ -220,7 +221,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         static_assert(S == 4, "K tiles take slots 0 and 2, V tiles 1 and 3");
         for (int j = 0; j <= nt && ok; ++j) {
           if (j < nt) {
-            if (j > 0) wwait(&sh->s_free, (j - 1) & 1, 25);
+            if (j > 0) wwait(&sh->s_free, (j - 1) & 1, 26);
             stage = 2 * (j & 1);
             phase = (j >> 1) & 1;
             if (ok) issue_qk();
@@ -413,7 +414,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
 
-      // ---- P = exp2(s - m), row sum, P -> TMEM in place over S ----------------------------
+      // ---- P = exp2(s - m), row sum, P -> TMEM, over S or in columns of its own -------------
       // packed pairs: one FMA, two exponentials, one conversion and one add per two scores
       if (kOwnP && j > 0) {                          // the P V before has read its P (as good as always)
         ok = wait_bar(&sh->o_ready, (j - 1) & 1, sh, 33);
@@ -516,6 +517,22 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 // ---------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------
+// head_dim 64: P in columns of its own, or over S as at head_dim 128?  Rows of one key tile have no next scores to compute
+// early, and rows of two gain what rows of one lose.  Own columns against P over S, 16 heads, two orders of launches:
+//   dense      one tile +2 % (64 x 128: 20.8 -> 21.3 us), causal two tiles 0 to +1 % (64 x 200: 55.5 -> 56.0), causal three 0, no
+//              mask two -2 % (64 x 256: 54.0 -> 52.9), more -1 to -3 %
+//   packed, causal    17 to 256 tokens +1.3 %, 100 to 200 +1.9 %, 17 to 400 +0.3 %, 17 to 640 -0.6 %, 550 to 1100 -2 %
+//   packed, no mask   100 to 200 +1.1 %, 128 to 256 -0.3 %, 250 to 500 -1.4 %
+//   windows    below two key tiles +0.3 to +2 % (16 x 1024, 50 on either side: 81.1 -> 82.6), 300 -1.7 %, 150 on either side 0
+// Of a packed batch only the sum and the longest length are known here.
+static bool p_over_s_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
+  const bool packed = a.cu_seqlens_q != nullptr;
+  const int64_t keys = packed ? (a.total_k / a.batch + a.seqlen_k) / 2 : a.seqlen_k, nk = (keys + kBN - 1) / kBN;
+  if ((cfg.causal ? nk + 1 : 2 * nk) <= (packed ? 4 : 3)) return true;    // twice the key tiles of a row tile
+  const int right = cfg.causal ? 0 : cfg.wr;
+  return cfg.wl >= 0 && right >= 0 && (int64_t)cfg.wl + right < 2 * kBN;
+}
+
 template <typename T, int D>
 static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
   using C = DCfg<D>;
@@ -535,10 +552,17 @@ static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t
     set_error("fwd_duo_sm100: cuTensorMapEncodeTiled failed");
     return FA_ERR_LAUNCH;
   }
-  auto kern = plain.keep != nullptr  ? fwd_duo_sm100_kernel<T, D, Feat::kNone, true>
-              : plain.softcap > 0.f ? fwd_duo_sm100_kernel<T, D, Feat::kCap, false>
-              : plain.has_alibi     ? fwd_duo_sm100_kernel<T, D, Feat::kAlibi, false>
-                                    : fwd_duo_sm100_kernel<T, D, Feat::kNone, false>;
+  auto pick = [&](auto own) {
+    constexpr bool kOwn = decltype(own)::value;
+    return plain.keep != nullptr  ? fwd_duo_sm100_kernel<T, D, Feat::kNone, true, kOwn>
+           : plain.softcap > 0.f ? fwd_duo_sm100_kernel<T, D, Feat::kCap, false, kOwn>
+           : plain.has_alibi     ? fwd_duo_sm100_kernel<T, D, Feat::kAlibi, false, kOwn>
+                                 : fwd_duo_sm100_kernel<T, D, Feat::kNone, false, kOwn>;
+  };
+  auto kern = pick(std::false_type{});
+  if constexpr (D == 64) {
+    if (!p_over_s_is_faster(a, plain)) kern = pick(std::true_type{});
+  }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
   if (e != cudaSuccess) {
     set_error("fwd_duo_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));

@@ -101,3 +101,34 @@ def test_below_the_persistent_kernel(monkeypatch, S, D, kw):
     got = run()
     monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
     assert torch.equal(got, run())
+
+
+@pytest.mark.parametrize("S,kw", [(128, dict()), (129, dict()), (128, dict(causal=True)), (256, dict(causal=True)), (257, dict(causal=True)),
+                                  (256, dict(causal=True, softcap=20.0)), (257, dict(causal=True, alibi=True)), (128, dict(dropout_p=0.2)),
+                                  (256, dict(causal=True, dropout_p=0.2)), (400, dict(causal=True, window_size=(255, 0))),
+                                  (400, dict(causal=True, window_size=(256, 0))), (640, dict(window_size=(100, 155))),
+                                  (640, dict(window_size=(128, 128), softcap=20.0)), (640, dict(window_size=(0, 255), alibi=True))], ids=str)
+@pytest.mark.parametrize("packed", [False, True])
+def test_short_rows(monkeypatch, S, kw, packed):
+    """head_dim 64 on both sides of the rule for P over S: equal to the two-tile kernel bit for bit.  Packed: S on average and longest, the
+    rule has another line there."""
+    import flash_attn_triton_b200 as fa
+    kw = slopes(kw)
+    if packed and "dropout_p" in kw:
+        pytest.skip("packed calls with dropout have another kernel")
+    g = torch.Generator(DEV).manual_seed(S)
+    B, half = 24, 50 if packed else 0
+    assert enough_tiles(B * -(-S // 128), 16)
+    lens = [S - half, S + half] * (B // 2)
+    q, k, v = (torch.randn(sum(lens), 16, 64, device=DEV, dtype=torch.half, generator=g) for _ in range(3))
+    cu = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32)
+
+    def run():
+        random.seed(3)                               # the dropout mask
+        if packed:
+            return fa.flash_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), **kw)
+        return fa.flash_attn_func(*(t.view(B, S, 16, 64) for t in (q, k, v)), **kw)
+
+    got = run()
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    assert torch.equal(got, run())
