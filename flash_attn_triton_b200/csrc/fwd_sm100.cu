@@ -868,15 +868,36 @@ static OneTile one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
 //   up to 2.5 CTAs per SM        +1 to +15 %
 //   head_dim 64, plain           -2 to -22 % dense (16 x 32 heads x 1024, causal: 205 -> 191 us; no mask, 1531 tokens: 550 -> 518),
 //                                -2 to -11 % packed; +3 to +7 % where part of the exponentials would go to the FMA pipe
+//                                (all with P over S; P in columns of its own, fwd_duo_sm100.cu, is another -1 to -4 %)
 //   others, by the key tiles of a row tile on average, where the persistent kernel is the alternative: up to 6.5  -2 to -26 %
 //                                (packed 17 to 2048, causal: 396 -> 370), 8 and more  0 to +15 % (40 packed of 64 to 3000: +5 %)
-//   where the two-tile kernel is (below the persistent one's lengths; dropout): head_dim 64 with options 0 to -13 % at every
-//                                length, no mask -1 to -13 % up to 15 key tiles (8 x 16 x 1152: 111.0 -> 96.6), causal -3 to -9 % up to 8 on
-//                                average (8 x 16 x 1600: 131 -> 123, with a soft cap 6 x 16: 140 -> 130, dropout 139 -> 127, 24 packed
-//                                of 64 to 2040, 32 heads over 8: 458 -> 417; the worst, 1700 tokens, +0.4 %), +2 to +4 % at 8.5
+//   where the two-tile kernel is (below the persistent one's lengths; dropout), see longer_rows_for_two_ctas()
 //   windows, up to 10            -4 to -12 % (32 packed sequences of 256 to 4096, window 1024, ALiBi and soft cap, head_dim
 //                                128: 1686 -> 1621): two thirds of a short window's tiles are masked, and the pair of
 //                                tiles of the other kernels sees one more than either needs
+// Rows of more than 6.5 key tiles on average, up to 15, where the two-tile kernel is the alternative: a call may need a whole wave of
+// either kernel less than of the other, and the two-tile kernel computes an odd number of row tiles as the next even one.
+// Measured against it on 466 random calls (an earlier rule took all of them: everything up to 15 key tiles, causal 8 on average;
+// head_dim 128 and 64 with options, 2.5 to 20 CTAs per SM), and checked on 263 others that it takes: -7 % on average, two above
+// +0.7 %, +1.8 % at most; what the earlier rule took besides, 0 % on average, -6 to +18 %.
+//   dropout, ALiBi, no mask    0 to -25 % everywhere
+//   causal, dense, odd number of row tiles    -1 to -10 % from 3 CTAs per SM on; even 0 to +7 %, packed -6 to +18 %
+//   plain and soft cap, no mask, dense    by the waves: as many as the two-tile kernel +1 to +8 % (plain; soft cap on many waves
+//                              -8 to 0 %), 12 x 8 heads x 1536: 122 -> 127 us; fewer -2 to -25 %, 8 x 8 x 1030: 69 -> 54
+//   the same, packed           up to 10 tiles from 4 CTAs per SM on, up to 13 from 7 on: +1 to -13 %; +1 to +6 % beside that
+static bool longer_rows_for_two_ctas(const fa_attn_args& a, const ScoreCfg& cfg, int64_t nk, int64_t tiles) {
+  const bool packed = a.cu_seqlens_q != nullptr;
+  const int64_t sms = sm_count(a.device), ctas = tiles * a.heads_q;
+  if (nk > 15) return false;
+  if (cfg.causal) return !packed && (a.seqlen_q + kBM - 1) / kBM % 2 == 1 && ctas >= 3 * sms;
+  if (cfg.keep != nullptr || cfg.has_alibi) return true;
+  if (packed) return ctas >= (nk <= 10 ? 4 : 7) * sms && nk <= 13;
+  const int64_t pairs = (int64_t)((a.seqlen_q + 2 * kBM - 1) / (2 * kBM)) * a.batch * a.heads_q, rest = ctas % (2 * sms);
+  // a wave of two CTAs per SM takes 1.02 (soft cap) to 1.06 as long as one of the two-tile kernel, of one CTA three quarters
+  const int64_t waves = 100 * (ctas / (2 * sms)) + (rest == 0 ? 0 : rest <= sms ? 75 : 100);
+  return waves * (cfg.softcap > 0.f ? 102 : 106) <= 100 * 100 * ((pairs + sms - 1) / sms);
+}
+
 static bool two_ctas_are_faster(const fa_attn_args& a, const ScoreCfg& cfg, int persistent_from) {
   const bool packed = a.cu_seqlens_q != nullptr, plain = !cfg.has_alibi && !(cfg.softcap > 0.f);
   const int64_t tiles = packed ? a.total_q / kBM + a.batch / 2 : (int64_t)((a.seqlen_q + kBM - 1) / kBM) * a.batch;
@@ -891,9 +912,9 @@ static bool two_ctas_are_faster(const fa_attn_args& a, const ScoreCfg& cfg, int 
   int64_t twice = cfg.causal ? nk + 1 : 2 * nk;
   const int right = cfg.causal ? 0 : cfg.wr;
   if (cfg.wl < 0 || right < 0) {
+    if (twice <= 13) return true;
     const bool two_tile = cfg.keep != nullptr || persistent_from <= 0 || a.seqlen_k < persistent_from;   // the alternative
-    if (!two_tile) return twice <= 13;
-    return a.head_dim == 64 || twice <= (cfg.causal ? 16 : 30);
+    return two_tile && longer_rows_for_two_ctas(a, cfg, nk, tiles);
   }
   return std::min<int64_t>(twice, 2 * (((int64_t)cfg.wl + right) / kBN + 2)) <= 20;
 }

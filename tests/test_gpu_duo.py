@@ -132,3 +132,35 @@ def test_short_rows(monkeypatch, S, kw, packed):
     got = run()
     monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
     assert torch.equal(got, run())
+
+
+@pytest.mark.parametrize("B,Sq,S,H,D,kw", [
+    (8, 1030, 1030, 8, 128, dict()), (6, 1536, 1536, 8, 128, dict()), (8, 1030, 1030, 8, 64, dict(softcap=20.0)),
+    (4, 1700, 1792, 16, 128, dict(alibi=True)), (7, 1000, 1900, 8, 128, dict(dropout_p=0.1)), (5, 1100, 1700, 16, 128, dict(causal=True)),
+    (5, 1300, 1900, 16, 128, dict(causal=True, softcap=20.0)), (5, 1664, 1664, 16, 64, dict(causal=True, alibi=True)),
+    (5, 1664, 1664, 16, 128, dict(causal=True, dropout_p=0.1)), (-14, 900, 900, 16, 128, dict()), (-14, 1900, 1900, 8, 128, dict(softcap=20.0)),
+    (-14, 1900, 1900, 8, 64, dict(alibi=True))], ids=str)
+def test_longer_rows(monkeypatch, B, Sq, S, H, D, kw):
+    """Seven to fifteen key tiles, on both sides of the rule that goes by the waves of the two kernels, rows and keys of different
+    lengths and (B < 0) packed: equal to the two-tile kernel bit for bit."""
+    import flash_attn_triton_b200 as fa
+    packed, B = B < 0, abs(B)
+    g = torch.Generator(DEV).manual_seed(S)
+    mk = lambda n: torch.randn(n, H, D, device=DEV, dtype=torch.half, generator=g)
+    kw = dict(kw)
+    if kw.pop("alibi", False):
+        kw["alibi_slopes"] = torch.tensor([0.5 ** (i + 1) for i in range(H)], device=DEV)
+    lens = [S - 300 * (i % 2) for i in range(B)] if packed else [S] * B
+    rows = lens if packed else [Sq] * B
+    q, k, v = mk(sum(rows)), mk(sum(lens)), mk(sum(lens))
+    cu = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32)
+
+    def run():
+        random.seed(3)                               # the dropout mask
+        if packed:
+            return fa.flash_attn_varlen_func(q, k, v, cu, cu, S, S, **kw)
+        return fa.flash_attn_func(q.view(B, Sq, H, D), k.view(B, S, H, D), v.view(B, S, H, D), **kw)
+
+    got = run()
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    assert torch.equal(got, run())
