@@ -205,3 +205,63 @@ def test_query_rows_with_infinities_and_zeros(S, D):
     assert torch.equal(out, want)
     mean = v[0, 0].float().mean(0)                   # scores of zero: every key alike
     assert (out[0, 0, :2].float() - mean).abs().max() <= 2e-3
+
+
+def query_rows(D):
+    """Rows of finite fp16 values whose quotients by the row's scale lie next to a rounding boundary (below and above every half from 0.5 to
+    126.5), one row or more for every largest value >= 1 that there is; and random rows."""
+    amax = np.arange(0x3c00, 0x7c00, dtype=np.uint16).view(np.float16)
+    s = amax.astype(np.float32) / np.float32(127.0)
+    halves = (np.arange(127, dtype=np.float64) + 0.5)[None, :] * s[:, None].astype(np.float64)
+    near = np.minimum(halves, amax[:, None].astype(np.float64)).astype(np.float16)
+    near = np.minimum(near, amax[:, None])
+    below = np.minimum(np.maximum(near.view(np.uint16).astype(np.int32) - 1, 0).astype(np.uint16).view(np.float16), amax[:, None])
+    above = np.minimum((near.view(np.uint16) + 1).view(np.float16), amax[:, None])
+    x = np.concatenate([near, below, above], 1)                       # 381 values a row
+    sign = np.where(np.arange(x.shape[1]) % 3 == 0, -1, 1).astype(np.float16)
+    x = x * sign
+    per = D - 1
+    x = np.pad(x, ((0, 0), (0, -x.shape[1] % per))).reshape(len(amax), -1, per)
+    x = np.concatenate([np.repeat(amax[:, None, None], x.shape[1], 1), x], 2).reshape(-1, D)
+    g = np.random.default_rng(D)
+    more = (g.standard_normal((4096, D)) * np.exp(g.uniform(-8, 9, (4096, 1)))).astype(np.float16)
+    more[::7, ::5] = -0.0
+    x = np.concatenate([x, more])
+    assert np.isfinite(x).all()
+    return x[:len(x) // 1024 * 1024]
+
+
+@pytest.mark.parametrize("D", [128, 64])
+def test_query_codes_are_those_of_a_division(D):
+    """The quantiser's quotient (a reciprocal and a correction step) against an fp32 division, where a last-bit error changes the code, as
+    int8 and as 16-bit floats with the sign of a zero."""
+    import ctypes as C
+    from flash_attn_triton_b200 import _native as N
+    x = query_rows(D)
+    r8, rs = orc.quantize_q_rows_ref(torch.from_numpy(x))
+    amax = np.maximum(np.abs(x.astype(np.float32)).max(1, keepdims=True), np.float32(1.0))
+    inverse = np.float32(1.0) / (amax / np.float32(127.0))
+    wrong = np.trunc(np.abs(x.astype(np.float32) * inverse) + np.float32(0.5)) * np.sign(x)
+    assert (wrong.astype(np.int8) != r8.reshape(x.shape)).any()       # a quotient without the correction would be seen
+    heads, S = len(x) // 1024, 1024
+    q = torch.from_numpy(x).to(DEV).view(1, heads, S, D)
+    k, v, o = torch.randn_like(q), torch.randn_like(q), torch.empty_like(q)
+    s_k, s_q = (torch.empty(heads * S, dtype=torch.float32, device=DEV) for _ in range(2))
+    a = N.Int8Args()
+    a.device, a.impl, a.batch, a.heads, a.seqlen, a.head_dim = 0, N.IMPL_AUTO, 1, heads, S, D
+    a.q, a.s_k, a.v, a.o, a.softmax_scale, a.sq_scratch = q.data_ptr(), s_k.data_ptr(), v.data_ptr(), o.data_ptr(), 0.1, s_q.data_ptr()
+    lib, stream = N.lib(), N.stream_ptr(q.device)
+    if D == 64:
+        codes = torch.zeros(lib.fa_int8_codes16_bytes(C.byref(a)), dtype=torch.uint8, device=DEV)
+        assert codes.numel() >= 2 * q.numel()
+        N.check(lib.fa_fwd_int8_codes16(C.byref(a), k.data_ptr(), s_k.data_ptr(), codes.data_ptr(), stream), "fa_fwd_int8_codes16")
+        got = codes.view(torch.float16)[:q.numel()].cpu().numpy().reshape(x.shape)
+        want = np.copysign(r8.reshape(x.shape).astype(np.float16), x)
+        assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
+    else:
+        k8, q8 = torch.zeros_like(q, dtype=torch.int8), torch.zeros_like(q, dtype=torch.int8)
+        N.check(lib.fa_quantize_k_int8(k.data_ptr(), k8.data_ptr(), s_k.data_ptr(), heads * S, D, 0, stream), "fa_quantize_k_int8")
+        a.k8, a.q8_scratch = k8.data_ptr(), q8.data_ptr()
+        N.check(lib.fa_fwd_int8(C.byref(a), stream), "fa_fwd_int8")
+        assert np.array_equal(q8.cpu().numpy().reshape(x.shape), r8.reshape(x.shape))
+    assert np.array_equal(s_q.cpu().numpy().view(np.uint32), rs.reshape(-1).view(np.uint32))
