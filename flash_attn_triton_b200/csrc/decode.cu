@@ -816,12 +816,13 @@ static int decode_row_groups(const fa_decode_args& a) {
 // rows; these calls append and rotate in a kernel of their own and attend on the tensor cores
 // (fwd_alt_sm100.cu), which takes about as long for 128 rows as the kernel above for 16.
 // ---------------------------------------------------------------------------------------
+constexpr int kAppendPerSm = 5;    // CTAs of 256 threads with 48 registers each
 // New keys (rotated) and values into the cache, rotated queries into q_out (batch, tokens, heads, D); a
 // 16-byte chunk per thread and step, HBM-bound.  host / dev: value checks made by every CTA, see decode_kernel.
 // Index: of a chunk.  With 64-bit indices the five divisions of a thread were most of the kernel; and as every CTA makes the
 // checks, there are no more CTAs than run at a time (4 x 256 tokens of 32 heads over 8 of 128: 15.5 -> 10.9 us).
 template <typename T, typename Index>
-__global__ void __launch_bounds__(256, 5) cache_append_kernel(const fa_decode_args p, T* q_out, int page_shift, uint32_t* host,
+__global__ void __launch_bounds__(256, kAppendPerSm) cache_append_kernel(const fa_decode_args p, T* q_out, int page_shift, uint32_t* host,
                                                            uint32_t* dev, bool check_here) {
   if (check_here) {
     const uint32_t bad = decode_checks(p, threadIdx.x, 256);
@@ -1082,7 +1083,7 @@ static int chunk_run(const fa_decode_args& args, const ChunkPlan& c, uint32_t* h
   const int64_t chunks = ((q_out ? (int64_t)a.batch * a.seqlen_q * a.heads_q : 0) + 2ll * a.batch * geo.n_new * a.heads_kv) *
                          (a.head_dim / 8);
   if (chunks > 0 || inside) {
-    const int64_t need = chunks > 0 ? (chunks + 255) / 256 : 1, fit = (int64_t)sm_count(a.device) * 5;
+    const int64_t need = chunks > 0 ? (chunks + 255) / 256 : 1, fit = (int64_t)sm_count(a.device) * kAppendPerSm;
     const unsigned grid = (unsigned)(need < fit ? need : fit);
     const int shift = page_shift_of(a);
     const bool small = chunks < (int64_t)1 << 31;
