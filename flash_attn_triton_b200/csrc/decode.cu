@@ -15,7 +15,7 @@
 //   (16-byte row gathers), so that the warps never wait for one another before they merge at the end.
 //   With 16-row products, a barrier per tile and the score options tested per element the compute of
 //   two CTAs per SM, not the memory, set the pace: 702 to 850 us for a 64-sequence step over
-//   4.3 GB of cache against 664 us now, 0.99 of the measured copy rate (calls in a row, value checks on or off).
+//   4.3 GB of cache against 660 us now, 0.99 of the measured copy rate (calls in a row, value checks on or off: 670).
 //   Append.  The new tokens (k_new rotated, v_new) never come from the cache: the CTA whose tile holds
 //   their positions puts them into the staged tile itself, and the one of row group 0 also writes
 //   them to their cache slots -- one writer per (sequence, kv head, token), no separate launch.
@@ -193,7 +193,7 @@ __device__ __noinline__ uint4 rotary_chunk_call(const T* x, int d, const T* cos,
 // it cost registers and the order of the loads (head_dim 256, 32 x 8000 tokens, 16 heads over 4: 268 us, 233 as a call); a
 // kernel that only rotates and copies is better off without the call (4 x 256 tokens behind 300, 32 heads over 8 of 128, with
 // their attention: 42 us, 46).  Pairs side by side need no row beside the one at hand and half as much of the tables: 8 x 900
-// tokens, 4 new, 16 heads over 4 of 128: element by element 30.4 us, as eight calls 20.6, now 16.6.
+// tokens, 4 new, 16 heads over 4 of 128: a thread per element 30.4 us, eight elements of a thread one by one 20.6, now 16.6.
 template <typename T, bool kCall>
 __device__ __forceinline__ uint4 rotary_chunk(const T* x, int d, const T* cos, const T* sin, int pos, int rotary_dim,
                                               int interleaved, int rotary_seqlen) {
@@ -1229,9 +1229,10 @@ constexpr size_t kWordBytes = 16;
 size_t word_offset(const fa_decode_args& a) { return (decode_workspace_bytes(a) + kWordBytes - 1) / kWordBytes * kWordBytes; }
 }  // namespace
 
-// A copy of both arrays to the host, looked at in Python, cost a packed call 25 to 40 us.  Whole calls, before -> after (us): forward of
-// 24 prompts of 17 to 2048 tokens, 32 heads over 8 of 128, 385 -> 358; of 7 of 67 to 540, 32 heads of 64, 56 -> 31; forward and
-// backward of 14 of 64, 32 heads of 64, 127 -> 92; of 23 of 261 to 522, 16 heads of 128, 268 -> 235.
+// A copy of both arrays to the host, looked at in Python, cost a packed call 17 to 33 us.  Whole calls, before -> after (us): forward of
+// 2 prompts of 30 and 34 tokens, 2 heads of 64, 40 -> 20; of 7 of 67 to 540, 32 heads of 64, 54 -> 35; of 24 of 17 to 2048, 32 heads
+// over 8 of 128, 392 -> 374 (404 -> 389 on another box); forward and backward of 14 of 64, 32 heads of 64, 127 -> 93; of 23 of 261
+// to 522, 16 heads of 128, 257 -> 225.
 int varlen_check(const int32_t* cu_q, const int32_t* cu_k, int batch, int64_t total_q, int64_t total_k, bool k_at_most, int64_t max_q,
                  int64_t max_k, int device, int32_t* ticket, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
