@@ -457,8 +457,10 @@ def flash_attn_varlen_func(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, ma
         # every value check the reference makes (:588-626).  Gathered pages are sized by batch * max_seqlen_k, an upper bound
         # of cu_seqlens_k[-1].  The plain call makes them itself, under its own host work.
         checks = _ops.VARLEN_KV_AT_MOST if paged else _ops.VARLEN_EXACT
-        # (a tensor of one element compares with a number in its own type: 2 ** 31 would wrap around in int32)
-        longest_q, longest_k = (x.item() if isinstance(x, torch.Tensor) else x for x in (max_seqlen_q, max_seqlen_k))
+        longest_q, longest_k = max_seqlen_q, max_seqlen_k
+        if not (type(longest_q) is int and type(longest_k) is int):
+            # a tensor of one element compares with a number in its own type: 2 ** 31 would wrap around in int32
+            longest_q, longest_k = (x.item() if isinstance(x, torch.Tensor) else x for x in (longest_q, longest_k))
         if dropout_p or used_q is not None or used_k is not None or not (0 < longest_q < 2 ** 31) or \
                 not (0 < longest_k < 2 ** 31):
             _ops.varlen_check(q, k, cu_seqlens_q, cu_seqlens_k, min(longest_q, 2 ** 62), min(longest_k, 2 ** 62), checks)
