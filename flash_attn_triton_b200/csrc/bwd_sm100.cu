@@ -27,14 +27,14 @@
 //       P and dS (16-bit) overwrite the fp32 regions of S and dP; S has a second buffer at head_dim 64.
 //   dQ, per key tile k:        S(k+1) -> other S buffer | dQ += dS(k) K(k) | dP(k+1)
 //
-// Roles (384 threads):
-//   warps 0-3 / 4-7  element-wise groups A / B: columns 0..63 / 64..127 of the 128 x 128
-//                    tiles, one TMEM lane (row) per thread
-//   warp 8           TMA producer
-//   warp 9           MMA issuer (uniform control flow, one elected lane issues)
-//   warp 10          dK/dV kernel: loads the per-row statistics (base-2 LSE, delta) of the
+// Roles (384 threads; 640 with score options: see Roles):
+//   element-wise     two groups of four warps, with score options four groups: 64 (32) columns of the
+//                    128 x 128 tiles each, one TMEM lane (row) per thread
+//   producer         TMA loads
+//   issuer           MMAs (uniform control flow, one elected lane issues)
+//   statistics       dK/dV kernel: loads the per-row statistics (base-2 LSE, delta) of the
 //                    streamed query tile and writes them as a 16-column GEMM operand
-//   warp 11          dK/dV kernel: hands the staged dV and dK tiles to the TMA unit
+//   store            dK/dV kernel: hands the staged dV and dK tiles to the TMA unit
 //
 // TMEM, dK/dV kernel: S^T, P^T (128 columns) | dP^T, dS^T (128) | dV (128) | dK (128); at head_dim 64
 //                     S^T, P^T [0] | S^T, P^T [1] | dP^T, dS^T | dV (64) | dK (64).
@@ -66,21 +66,29 @@ __device__ int g_bwd_sm100_status = 0;
 namespace {
 
 constexpr int kT = 128;        // tile edge: rows of Q / keys of K,V per tile
-constexpr int kHalfT = 64;     // columns per element-wise group
-constexpr int kBwdThreads = 384;
+// Roles of the warps with G element-wise warpgroups, each of which takes 128 / G columns of a tile, and the split of the
+// registers (setmaxnreg): the CTA starts with kRegsLaunch per thread; the four service warps drop to kRegsService and the
+// element-wise warps grow to kRegsEw, out of what the CTA was launched with.
+template <int G> struct Roles {
+  static constexpr int kCols = kT / G;             // columns of a 128 x 128 tile per element-wise thread
+  static constexpr int kEwThreads = 128 * G, kEwWarps = 4 * G;
+  static constexpr int kProducer = kEwWarps, kIssuer = kEwWarps + 1, kStats = kEwWarps + 2, kStore = kEwWarps + 3;
+  static constexpr int kThreads = kEwThreads + 128;
+  static constexpr int kRegsLaunch = G == 2 ? 168 : 96;          // what a CTA of kThreads can have
+  static constexpr int kRegsService = G == 2 ? 88 : 64, kRegsEw = G == 2 ? 208 : 104;
+  static_assert(kThreads * kRegsLaunch <= 65536, "registers of an SM");
+  static_assert((kRegsEw - kRegsLaunch) * kEwThreads <= (kRegsLaunch - kRegsService) * 128, "register split");
+};
+// Groups of a variant.  With score options a score takes two special-function results and a dozen other instructions, and
+// two warps per scheduler leave most of their latencies open: with four the exponential phase of dK/dV takes 2.0 k cycles
+// instead of 2.5 k (the special-function unit needs 2.05 k).  dK/dV and dQ, two groups -> four (us), causal: soft cap,
+// 4 x 16 x 2048 of 64 156 -> 139, 118 -> 112; 2 x 16 x 4096 of 128 315 -> 302, 219 -> 207; ALiBi, 4 x 16 x 2048 of 128
+// 150 -> 144, 105 -> 102.  Without options the phase is close to the unit's 1.02 k with two groups (1.35 k), and
+// the larger number of warps delays the MMAs: 4 x 16 x 4096 of 128 864 -> 877, 605 -> 617; 4 x 32 x 1024 x 1531 of 64
+// 137 -> 141, 101 -> 100.  (An arrival per warp instead of per thread: 0 to +1 %.  The LSE of the next tile read under this
+// one's dS phase: +8 to +13 %, spills.  The LSE read next to its use: +4 to +8 %.)
+__host__ __device__ constexpr int ew_groups(Feat f) { return f == Feat::kNone ? 2 : 4; }
 constexpr int kSched = 4;      // depth of the in-CTA ring of work-queue entries
-// Register re-balancing (setmaxnreg): the CTA starts with 168 registers per thread; the four
-// service warps drop to kRegsService and the eight element-wise warps grow to kRegsEw.
-// setmaxnreg.inc blocks until the registers exist, so the split has to satisfy
-// (kRegsEw - 168) * 256 <= (168 - kRegsService) * 128.
-constexpr int kRegsService = 88, kRegsEw = 208;
-// Share of the exponentials of the unmasked fast path that run on the FMA pipe (every n-th).
-#ifndef FA_POLY_BWD
-#define FA_POLY_BWD 0
-#endif
-constexpr int kPolyEvery = FA_POLY_BWD;
-static_assert((kRegsEw - 168) * 256 <= (168 - kRegsService) * 128, "register split");
-
 template <int D> struct BCfg {
   static constexpr int kTileBytes = kT * D * 2;
   static constexpr int kBoxes = D / 64;
@@ -120,8 +128,8 @@ struct BShared {
   uint64_t k_full, k_free;  // dK/dV kernel: the same for K
   uint64_t s_full[2];     // [buffer]: S computed
   uint64_t dp_full;       // dP computed
-  uint64_t p_ready[2];    // dK/dV kernel, [score buffer]: P written back (256 arrivals)
-  uint64_t ds_ready;      // dS written back (256 arrivals)
+  uint64_t p_ready[2];    // dK/dV kernel, [score buffer]: P written back (every element-wise thread)
+  uint64_t ds_ready;      // dS written back (every element-wise thread)
   uint64_t dv_done;       // dK/dV kernel: every dV MMA of the item finished
   uint64_t acc_done;      // every accumulation MMA of the item finished
   uint64_t sched_full[kSched];   // work-queue entry published by the producer thread
@@ -307,15 +315,15 @@ __device__ __forceinline__ void mma_kmajor(uint32_t d_tmem, uint32_t a_smem, uin
 }
 
 // acc(128 x D) += A(128 x 128, fp16 pairs in TMEM) * B(128 rows x D, MN-major smem tile).
-// A is stored as two 32-column blocks (written by the two element-wise groups) at
-// a_tmem and a_tmem + kGroupStride.
-template <int D, int kGroupStride>
+// A is stored by the element-wise groups, each over the first half of its kCols columns.
+template <int D, int kCols>
 __device__ __forceinline__ void mma_from_tmem(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_smem,
                                               uint32_t idesc, bool accumulate, uint32_t leader) {
   const uint64_t db = make_smem_desc(b_smem, kT * 128, 1024);
 #pragma unroll
   for (int kk = 0; kk < kT / 16; ++kk) {
-    const uint32_t a = a_tmem + (kk / 4) * kGroupStride + (kk % 4) * 8;
+    constexpr int kPer = kCols / 16;               // MMAs per group
+    const uint32_t a = a_tmem + (kk / kPer) * kCols + (kk % kPer) * 8;
     mma_f16_ts_lp(d_tmem, a, db + ((kk * 2048) >> 4), idesc, (accumulate || kk > 0) ? 1u : 0u, leader);
   }
 }
@@ -326,22 +334,26 @@ __device__ __forceinline__ void mma_from_tmem(uint32_t d_tmem, uint32_t a_tmem, 
 template <typename T, int kCols>
 __device__ __forceinline__ void drain_acc(uint32_t tsrc, float mul, bool staged, uint32_t stg, int lrow,
                                           int col0, T* grow) {
-  uint32_t r[kCols / 32][32];
+  constexpr int kW = kCols < 32 ? kCols : 32;
+  uint32_t r[kCols / kW][kW];
 #pragma unroll
-  for (int cc = 0; cc < kCols / 32; ++cc) tmem_ld32(tsrc + cc * 32, r[cc]);
+  for (int cc = 0; cc < kCols / kW; ++cc) {
+    if constexpr (kW == 16) tmem_ld16(tsrc + cc * kW, r[cc]);
+    else tmem_ld32(tsrc + cc * kW, r[cc]);
+  }
   tmem_wait_ld();
 #pragma unroll
-  for (int cc = 0; cc < kCols / 32; ++cc) {
+  for (int cc = 0; cc < kCols / kW; ++cc) {
 #pragma unroll
-    for (int i = 0; i < 32; i += 8) {
+    for (int i = 0; i < kW; i += 8) {
       uint4 v;
       v.x = Elem<T>::pack(__uint_as_float(r[cc][i]) * mul, __uint_as_float(r[cc][i + 1]) * mul);
       v.y = Elem<T>::pack(__uint_as_float(r[cc][i + 2]) * mul, __uint_as_float(r[cc][i + 3]) * mul);
       v.z = Elem<T>::pack(__uint_as_float(r[cc][i + 4]) * mul, __uint_as_float(r[cc][i + 5]) * mul);
       v.w = Elem<T>::pack(__uint_as_float(r[cc][i + 6]) * mul, __uint_as_float(r[cc][i + 7]) * mul);
-      const int col = col0 + cc * 32 + i;
+      const int col = col0 + cc * kW + i;
       if (staged) st_shared_v4(sw128_addr(stg + (col / 64) * (kT * 128), lrow, (col % 64) / 8), v);
-      else if (grow != nullptr) *reinterpret_cast<uint4*>(grow + cc * 32 + i) = v;
+      else if (grow != nullptr) *reinterpret_cast<uint4*>(grow + cc * kW + i) = v;
     }
   }
 }
@@ -421,7 +433,7 @@ __device__ __forceinline__ bool dq_item(const fa_attn_args& p, const ScoreCfg& c
 // kDrop: P^T and dS^T are zero where the bit of (key, query row) in cfg.keep is 0, and scaled by
 // dropout_scale, which is folded into the statistics operand (its log2 is added to -lse2).
 template <typename T, int D, Feat kFeat, bool kDrop>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(Roles<ew_groups(kFeat)>::kThreads, 1)
 bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                       const __grid_constant__ CUtensorMap tmdK, const __grid_constant__ CUtensorMap tmdV,
@@ -430,7 +442,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   using C = BCfg<D>;
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr int SQ = C::kStagesQ, SO = C::kStagesO;
-  constexpr int kConsumers = 11;   // warps that read the work queue: 8 element-wise, issuer, statistics, store agent
+  using R = Roles<ew_groups(kFeat)>;
+  constexpr int kEwCols = R::kCols;              // columns per element-wise thread
+  constexpr int kConsumers = R::kEwWarps + 3;   // warps that read the work queue: 8 element-wise, issuer, statistics, store agent
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -456,9 +470,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     mbar_init(smem_u32(&sh->s_full[0]), 1);
     mbar_init(smem_u32(&sh->s_full[1]), 1);
     mbar_init(smem_u32(&sh->dp_full), 1);
-    mbar_init(smem_u32(&sh->p_ready[0]), 256);
-    mbar_init(smem_u32(&sh->p_ready[1]), 256);
-    mbar_init(smem_u32(&sh->ds_ready), 256);
+    mbar_init(smem_u32(&sh->p_ready[0]), R::kEwThreads);
+    mbar_init(smem_u32(&sh->p_ready[1]), R::kEwThreads);
+    mbar_init(smem_u32(&sh->ds_ready), R::kEwThreads);
     mbar_init(smem_u32(&sh->dv_done), 1);
     mbar_init(smem_u32(&sh->acc_done), 1);
     for (int i = 0; i < 4; ++i) {
@@ -471,15 +485,15 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_init(smem_u32(&sh->sched_full[i]), 1);
       mbar_init(smem_u32(&sh->sched_empty[i]), kConsumers);
     }
-    mbar_init(smem_u32(&sh->stg_ready[0]), 256);
-    mbar_init(smem_u32(&sh->stg_ready[1]), 256);
+    mbar_init(smem_u32(&sh->stg_ready[0]), R::kEwThreads);
+    mbar_init(smem_u32(&sh->stg_ready[1]), R::kEwThreads);
     mbar_init(smem_u32(&sh->stg_taken[0]), 1);
     sh->abort_flag = 0;
     fence_barrier_init();
   }
-  stat_write_keys<T>(aug + SQ * kStatBlock, cfg.scale_log2, tid, kBwdThreads);
+  stat_write_keys<T>(aug + SQ * kStatBlock, cfg.scale_log2, tid, R::kThreads);
   fence_proxy_async();
-  if (warp == 8) {
+  if (warp == R::kProducer) {
     tmem_alloc(smem_u32(&sh->tmem_base), 512);
     tmem_relinquish();
   }
@@ -501,9 +515,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   // slot's barriers.  The entries of the LAST tile are released by the store agent (the epilogue stages
   // dK and dV over them), the others by the commits of the issuer.
 
-  if (warp == 8) {
+  if (warp == R::kProducer) {
     // ------------------------------- TMA producer ---------------------------------------
-    reg_dealloc<kRegsService>();
+    reg_dealloc<R::kRegsService>();
     if (lane == 0) {
       prefetch_tmap(&tmQ);
       prefetch_tmap(&tmK);
@@ -555,13 +569,13 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ++wi;
       }
     }
-  } else if (warp == 10) {
+  } else if (warp == R::kStats) {
     // ------------------------------- statistics loader ----------------------------------
     // The loads of the next tile are ISSUED right after the current one has been written and only consumed
     // after the wait for the next slot, so their latency hides behind that wait (nothing reads
     // the registers in between: a scoreboard stall before the poll would serialise the two; the pieces worked
     // out there too cost 4 x 1024 x 1531 of 32 heads of 64 387 -> 488 us).
-    reg_dealloc<kRegsService>();
+    reg_dealloc<R::kRegsService>();
     float rl[kT / 32], rd[kT / 32];                  // statistics of rows lane, lane + 32, ... as loaded
     const float unit = stat_score_unit(cfg.scale_log2);
     auto fetch = [&](const KItem& w, int it) {
@@ -620,7 +634,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       fetched = haven;
       w = sched_get<KItem>(sh, sidx++, true, ok);
     }
-  } else if (warp == 9) {
+  } else if (warp == R::kIssuer) {
     // ------------------------------- MMA issuer -----------------------------------------
     // The GEMMs of tile i+1 follow, in the in-order tensor pipe, the accumulation of tile i that
     // reads the region they overwrite:
@@ -631,7 +645,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     // is complete, because the scores that it needs first, S(i + buffers) after P(i), are issued behind that phase.  With
     // two score buffers that holds per buffer only: a warp can store P(i+1) while another has not stored P(i), so
     // each buffer has a barrier of its own.  For dS: dP(i+1), which dS(i+1) needs, is issued behind dS(i) of all warps.
-    reg_dealloc<kRegsService>();
+    reg_dealloc<R::kRegsService>();
     constexpr uint32_t idesc_s = make_idesc(1, BFmt<T>::code, 0, 0, kT, kT);
     constexpr uint32_t idesc_acc = make_idesc(1, BFmt<T>::code, 0, 1, kT, D);
     const uint32_t leader = elect_one() ? 1u : 0u;
@@ -699,13 +713,13 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const bool more = i < last;
         wq(&sh->p_ready[sbuf(ps)], sphase(ps), 45);
         if (!ok) break;
-        mma_from_tmem<D, kHalfT>(tdV, tS + sbuf(ps) * 128, slotB(ps), idesc_acc, i > 0, leader);   // dV += P(i)^T dO(i)
+        mma_from_tmem<D, kEwCols>(tdV, tS + sbuf(ps) * 128, slotB(ps), idesc_acc, i > 0, leader);   // dV += P(i)^T dO(i)
         // (dO(i)'s other reader, dP(i), precedes in the pipe)
         mma_commit_lp(smem_u32(more ? &sh->empty_b[ps % SO] : &sh->dv_done), leader);
         next_s(i + NB);
         wq(&sh->ds_ready, ps & 1, 46);
         if (!ok) break;
-        mma_from_tmem<D, kHalfT>(tdK, tdP, slotA(ps), idesc_acc, i > 0, leader);                   // dK += dS(i)^T Q(i)
+        mma_from_tmem<D, kEwCols>(tdK, tdP, slotA(ps), idesc_acc, i > 0, leader);                   // dK += dS(i)^T Q(i)
         if (more) mma_commit_lp(smem_u32(&sh->empty_a[ps % SQ]), leader);
         next_dp(i + 1);
       }
@@ -714,11 +728,11 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       ++wi;
     }
     __syncwarp();
-  } else if (warp == 11) {
+  } else if (warp == R::kStore) {
     // ------------------------------- store agent ----------------------------------------
     // The element-wise warps stage dV and dK over the item's last dO and Q tiles; this warp hands them
     // to the TMA unit and releases the two ring entries once the unit has read them.
-    reg_dealloc<kRegsService>();
+    reg_dealloc<R::kRegsService>();
     const uint32_t leader = elect_one() ? 1u : 0u;
     int pos = 0, sidx = 0, wi = 0;
     bool ok = true;
@@ -757,12 +771,12 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     __syncwarp();
   } else {
     // ------------------------------- element-wise groups --------------------------------
-    reg_alloc<kRegsEw>();
+    reg_alloc<R::kRegsEw>();
     const int x = warp >> 2;                         // column half
     const int lrow = (warp & 3) * 32 + lane;         // TMEM lane = key inside the tile
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     // this group's 64 columns; the 16-bit pairs of P, of dS take the first 32 of them
-    const uint32_t tSg = tS + lane_addr + x * kHalfT, tdPx = tdP + lane_addr + x * kHalfT;
+    const uint32_t tSg = tS + lane_addr + x * kEwCols, tdPx = tdP + lane_addr + x * kEwCols;
     bool ok = true;
     int pos = 0, wi = 0, sidx = 0;
     PROF_VARS(16);
@@ -774,16 +788,16 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     while (ok && w.total >= 0) {
       const int key = w.n0 + lrow;
       // each group stores half of the head_dim columns of dV and of dK * softmax_scale
-      constexpr int DH = D / 2;
-      T *gdv = nullptr, *gdk = nullptr;
-      if (key < w.g.k_len) {
-        gdv = reinterpret_cast<T*>(p.dv) + (int64_t)w.g.k_boff * p.dv_stride[0] +
-              (int64_t)(w.g.k_row0 + key) * p.dv_stride[1] + (int64_t)w.hk * p.dv_stride[2] + x * DH;
-        gdk = reinterpret_cast<T*>(p.dk) + (int64_t)w.g.k_boff * p.dk_stride[0] +
-              (int64_t)(w.g.k_row0 + key) * p.dk_stride[1] + (int64_t)w.hk * p.dk_stride[2] + x * DH;
-      }
+      constexpr int DH = D * kEwCols / kT;
+      auto row_of = [&](void* base, const int64_t* stride) -> T* {     // this thread's part of its key's row
+        if (key >= w.g.k_len) return nullptr;
+        return reinterpret_cast<T*>(base) + (int64_t)w.g.k_boff * stride[0] + (int64_t)(w.g.k_row0 + key) * stride[1] +
+               (int64_t)w.hk * stride[2] + x * DH;
+      };
       if (w.total == 0) {
         // no query can see these keys: their gradients are zero
+        T* const gdv = row_of(p.dv, p.dv_stride);
+        T* const gdk = row_of(p.dk, p.dk_stride);
         if (gdv != nullptr) {
 #pragma unroll
           for (int c = 0; c < DH / 8; ++c) {
@@ -802,36 +816,39 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // (the divisions of the other roles would be 0.2 k cycles at the start of every tile here, where nothing hides them)
       int hq = w.hk * G, m = w.m_lo;
       const int m_end = w.m_lo + w.ntiles;
+      float slope = 0.f;
       for (int it = 0; it < w.total && ok; ++it, ++pos) {
         const int stage = pos % SQ;
-        const int q0 = m * kT + x * kHalfT;            // first query row of this thread's columns
-        const float slope = (kExtras && cfg.has_alibi) ? p.alibi_slopes[w.b * p.heads_q + hq] : 0.f;
+        const int q0 = m * kT + x * kEwCols;            // first query row of this thread's columns
+        if (kExtras && m == w.m_lo && cfg.has_alibi) slope = p.alibi_slopes[w.b * p.heads_q + hq];
         if (++m == m_end) {
           m = w.m_lo;
           ++hq;
         }
         bool masked = false;
         if (cfg.causal) masked |= (w.n0 + kT - 1 > q0 + off);
-        if (cfg.wl >= 0) masked |= (w.n0 < q0 + kHalfT - 1 + off - cfg.wl);
+        if (cfg.wl >= 0) masked |= (w.n0 < q0 + kEwCols - 1 + off - cfg.wl);
         if (cfg.wr >= 0) masked |= (w.n0 + kT - 1 > q0 + off + cfg.wr);
 
-        // Only the feature path still needs the LSE per column (it is added after the soft cap);
-        // it is fetched into registers BEFORE the wait for the scores: shared-memory loads issued
-        // while the tensor pipe streams its operands take hundreds of cycles, and here that
-        // latency hides behind the wait.  Otherwise the GEMMs deliver S - lse and dP - delta.
-        float st[kHalfT];                              // -lse
+        // Only the feature variant needs the LSE per column (it is added after the soft cap); otherwise the GEMMs deliver
+        // S - lse and dP - delta.  It is fetched into registers BEFORE the wait for the scores: shared-memory loads issued
+        // while the tensor pipe streams its operands take hundreds of cycles, and here that latency hides behind the wait.
+        float st[kEwCols];                             // -lse
         if (kExtras) {
           ok = bwait(&sh->full_a[stage], (pos / SQ) & 1, sh, 47);
           if (!ok) break;
-          const float4* L4 = reinterpret_cast<const float4*>(&sh->lse[stage][x * kHalfT]);
+          const float4* L4 = reinterpret_cast<const float4*>(&sh->lse[stage][x * kEwCols]);
 #pragma unroll
-          for (int i4 = 0; i4 < kHalfT / 4; ++i4) {
+          for (int i4 = 0; i4 < kEwCols / 4; ++i4) {
             const float4 l4 = L4[i4];
             st[i4 * 4] = l4.x; st[i4 * 4 + 1] = l4.y; st[i4 * 4 + 2] = l4.z; st[i4 * 4 + 3] = l4.w;
           }
         }
-        uint2 keep2;                                   // this thread's 64 bits of the tile, on their way during the wait
-        if (kDrop) keep2 = __ldg(reinterpret_cast<const uint2*>(cfg.keep + key * cfg.keep_words + (q0 >> 5)));
+        uint32_t keep[kEwCols / 32];                   // this thread's bits of the tile, on their way during the wait
+        if (kDrop) {
+#pragma unroll
+          for (int h = 0; h < kEwCols / 32; ++h) keep[h] = __ldg(cfg.keep + key * cfg.keep_words + (q0 >> 5) + h);
+        }
         PROF_T0();
         ok = bwait(&sh->s_full[sbuf(pos)], sphase(pos), sh, 46);
 #ifdef FA_PROF
@@ -839,16 +856,16 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         PROF_T0();
 #endif
         if (!ok) break;
-        SKEW(warp, pos, 0);
+        SKEW(warp, R::kEwWarps, pos, 0);
         tc_fence_after();
 
         // ---- exp phase: P = exp2(score - lse), written back as T pairs ---------------------
-        uint32_t r0[32], r1[32];
+        uint32_t r[kEwCols / 32][32];
         const uint32_t tSx = tSg + sbuf(pos) * 128;
-        tmem_ld32(tSx, r0);
-        tmem_ld32(tSx + 32, r1);
+#pragma unroll
+        for (int h = 0; h < kEwCols / 32; ++h) tmem_ld32(tSx + h * 32, r[h]);
         tmem_wait_ld();
-        float pf[kHalfT];                              // P in fp32, kept for the dS phase
+        float pf[kEwCols];                              // P in fp32, kept for the dS phase
         const float dist0 = (float)(q0 + off - key);   // query position - key position of column 0
         // columns (query rows) of this tile that see this thread's key
         const ColMask cm = make_col_mask(vq_lo - (q0 + off), vq_hi - (q0 + off));
@@ -914,7 +931,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                 pe.y = col_visible(cm, c + 1) ? pe.y : 0.f;
               }
               if (kDrop) {
-                const uint32_t kw = h == 0 ? keep2.x : keep2.y;
+                const uint32_t kw = keep[h];
                 pe.x = (kw >> i) & 1u ? pe.x : 0.f;
                 pe.y = (kw >> (i + 1)) & 1u ? pe.y : 0.f;
               }
@@ -928,12 +945,10 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         // |distance| only where a visible element can lie on the other side of the diagonal
         const bool need_abs = kExtras && !cfg.causal;
         auto run_exp = [&](auto mask_tag) {
-          if (need_abs) {
-            exp_body(0, r0, mask_tag, std::true_type{});
-            exp_body(1, r1, mask_tag, std::true_type{});
-          } else {
-            exp_body(0, r0, mask_tag, std::false_type{});
-            exp_body(1, r1, mask_tag, std::false_type{});
+#pragma unroll
+          for (int h = 0; h < kEwCols / 32; ++h) {
+            if (need_abs) exp_body(h, r[h], mask_tag, std::true_type{});
+            else exp_body(h, r[h], mask_tag, std::false_type{});
           }
         };
         if (masked) run_exp(std::true_type{});
@@ -950,16 +965,16 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ok = bwait(&sh->dp_full, pos & 1, sh, 48);
         PROF_ADD(2);
         if (!ok) break;
-        SKEW(warp, pos, 1);
+        SKEW(warp, R::kEwWarps, pos, 1);
         PROF_T0();
         tc_fence_after();
-        tmem_ld32(tdPx, r0);
-        tmem_ld32(tdPx + 32, r1);
+#pragma unroll
+        for (int h = 0; h < kEwCols / 32; ++h) tmem_ld32(tdPx + h * 32, r[h]);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < kEwCols / 32; ++c) {
           uint32_t pk[16];
-          const uint32_t* rr = c == 0 ? r0 : r1;
+          const uint32_t (&rr)[32] = r[c];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float2 ds = f2mul(make_float2(pf[c * 32 + 2 * i], pf[c * 32 + 2 * i + 1]),
@@ -988,10 +1003,10 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       ok = bwait(&sh->dv_done, wi & 1, sh, 49);
       PROF_ADD(5);
       if (!ok) break;
-      SKEW(warp, wi, 2);
+      SKEW(warp, R::kEwWarps, wi, 2);
       tc_fence_after();
       PROF_T0();
-      drain_acc<T, DH>(tdV + lane_addr + x * DH, 1.f, via_tma, slotB(pos - 1), lrow, x * DH, gdv);
+      drain_acc<T, DH>(tdV + lane_addr + x * DH, 1.f, via_tma, slotB(pos - 1), lrow, x * DH, via_tma ? nullptr : row_of(p.dv, p.dv_stride));
       tc_fence_before();
       if (via_tma) fence_proxy_async();
       // (the agent has seen the previous item's tiles: its barrier is never a whole phase behind)
@@ -999,9 +1014,9 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       mbar_arrive(smem_u32(&sh->stg_ready[0]));
       ok = bwait(&sh->acc_done, wi & 1, sh, 49);
       if (!ok) break;
-      SKEW(warp, wi, 3);
+      SKEW(warp, R::kEwWarps, wi, 3);
       tc_fence_after();
-      drain_acc<T, DH>(tdK + lane_addr + x * DH, cfg.scale, via_tma, slotA(pos - 1), lrow, x * DH, gdk);
+      drain_acc<T, DH>(tdK + lane_addr + x * DH, cfg.scale, via_tma, slotA(pos - 1), lrow, x * DH, via_tma ? nullptr : row_of(p.dk, p.dk_stride));
       tc_fence_before();
       if (via_tma) fence_proxy_async();
       mbar_arrive(smem_u32(&sh->stg_ready[1]));
@@ -1017,7 +1032,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) tmem_dealloc(tmem, 512);
+  if (warp == R::kProducer) tmem_dealloc(tmem, 512);
   if (tid == 0) {
     if (sh->abort_flag == 0) sched_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
@@ -1030,7 +1045,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 // kDrop: dS is zero where the bit of (query row, key) in cfg.keep is 0; the scale of the kept probabilities
 // is folded into the row's LSE.
 template <typename T, int D, Feat kFeat, bool kDrop>
-__global__ void __launch_bounds__(kBwdThreads, 1)
+__global__ void __launch_bounds__(Roles<ew_groups(kFeat)>::kThreads, 1)
 bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                     const __grid_constant__ CUtensorMap tmdQ, const fa_attn_args p, const ScoreCfg cfg,
@@ -1039,7 +1054,9 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   using C = BCfg<D>;
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr int SK = C::kStagesK, SV = C::kStagesV;
-  constexpr int kConsumers = 9;    // warps that read the work queue: 8 element-wise and the issuer
+  using R = Roles<ew_groups(kFeat)>;
+  constexpr int kEwCols = R::kCols;              // columns per element-wise thread
+  constexpr int kConsumers = R::kEwWarps + 1;    // warps that read the work queue: 8 element-wise and the issuer
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -1059,7 +1076,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     mbar_init(smem_u32(&sh->s_full[0]), 1);
     mbar_init(smem_u32(&sh->s_full[1]), 1);
     mbar_init(smem_u32(&sh->dp_full), 1);
-    mbar_init(smem_u32(&sh->ds_ready), 256);
+    mbar_init(smem_u32(&sh->ds_ready), R::kEwThreads);
     mbar_init(smem_u32(&sh->acc_done), 1);
     for (int i = 0; i < 4; ++i) {
       mbar_init(smem_u32(&sh->full_a[i]), 1);
@@ -1071,12 +1088,12 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       mbar_init(smem_u32(&sh->sched_full[i]), 1);
       mbar_init(smem_u32(&sh->sched_empty[i]), kConsumers);
     }
-    mbar_init(smem_u32(&sh->stg_ready[0]), 256);
+    mbar_init(smem_u32(&sh->stg_ready[0]), R::kEwThreads);
     mbar_init(smem_u32(&sh->stg_taken[0]), 1);
     sh->abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 8) {
+  if (warp == R::kProducer) {
     tmem_alloc(smem_u32(&sh->tmem_base), 512);
     tmem_relinquish();
   }
@@ -1090,15 +1107,15 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   // ring B entries V(0) ... V(total-1); the last K entry is released by the epilogue, which
   // stages dQ over it.
 
-  if (warp >= 10) {
-    reg_dealloc<kRegsService>();
-    if (warp == 10 && lane == 0) {
+  if (warp >= R::kStats) {
+    reg_dealloc<R::kRegsService>();
+    if (warp == R::kStats && lane == 0) {
       prefetch_tmap(&tmdQ);
       store_lane<D>(sh, 0, &tmdQ, 1);                 // the store lane of dQ
     }
-  } else if (warp == 8) {
+  } else if (warp == R::kProducer) {
     // ------------------------------- TMA producer ---------------------------------------
-    reg_dealloc<kRegsService>();
+    reg_dealloc<R::kRegsService>();
     if (lane == 0) {
       prefetch_tmap(&tmQ);
       prefetch_tmap(&tmK);
@@ -1153,9 +1170,9 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         ++wi;
       }
     }
-  } else if (warp == 9) {
+  } else if (warp == R::kIssuer) {
     // ------------------------------- MMA issuer -----------------------------------------
-    reg_dealloc<kRegsService>();
+    reg_dealloc<R::kRegsService>();
     constexpr uint32_t idesc_s = make_idesc(1, BFmt<T>::code, 0, 0, kT, kT);
     constexpr uint32_t idesc_acc = make_idesc(1, BFmt<T>::code, 0, 1, kT, D);
     const uint32_t leader = elect_one() ? 1u : 0u;
@@ -1202,7 +1219,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         }
         wq(&sh->ds_ready, tg & 1, 55);                // (dP(k+1), which dS(k+1) needs, is issued behind this phase)
         if (!ok) break;
-        mma_from_tmem<D, kHalfT>(tdQ, tdP, slotK(kpos), idesc_acc, k > 0, leader);        // dQ += dS(k) K(k)
+        mma_from_tmem<D, kEwCols>(tdQ, tdP, slotK(kpos), idesc_acc, k > 0, leader);        // dQ += dS(k) K(k)
         if (more) mma_commit_lp(smem_u32(&sh->empty_a[kpos % SK]), leader);       // (the epilogue releases the last)
         if (more) {
           wq(&sh->full_b[v1pos % SV], (v1pos / SV) & 1, 54);
@@ -1221,12 +1238,12 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     __syncwarp();
   } else {
     // ------------------------------- element-wise groups --------------------------------
-    reg_alloc<kRegsEw>();
+    reg_alloc<R::kRegsEw>();
     const int x = warp >> 2;
     const int lrow = (warp & 3) * 32 + lane;  // TMEM lane = query row inside the tile
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tdPx = tdP + lane_addr + x * kHalfT;
-    constexpr int DH = D / 2;                 // each group stores half of the head_dim columns
+    const uint32_t tdPx = tdP + lane_addr + x * kEwCols;
+    constexpr int DH = D * kEwCols / kT;                 // each group stores half of the head_dim columns
     bool ok = true;
     int posA = 0, wi = 0, tg = 0, sidx = 0;
     // statistics of this thread's row: base-2 LSE (+inf for rows that do not exist or see no
@@ -1280,26 +1297,29 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       visible_k_interval(cfg, qpos, w.g.k_len, vk_lo, vk_hi);
 
       for (int j = 0; j < w.total && ok; ++j, ++tg) {
-        const int k0 = (w.n_hi - 1 - j) * kT + x * kHalfT;   // first key of this thread's columns
-        bool masked = (k0 + kHalfT > w.g.k_len);
-        if (cfg.causal) masked |= (k0 + kHalfT - 1 > w.m0 + off);
+        const int k0 = (w.n_hi - 1 - j) * kT + x * kEwCols;   // first key of this thread's columns
+        bool masked = (k0 + kEwCols > w.g.k_len);
+        if (cfg.causal) masked |= (k0 + kEwCols - 1 > w.m0 + off);
         if (cfg.wl >= 0) masked |= (k0 < w.m0 + kT - 1 + off - cfg.wl);
-        if (cfg.wr >= 0) masked |= (k0 + kHalfT - 1 > w.m0 + off + cfg.wr);
+        if (cfg.wr >= 0) masked |= (k0 + kEwCols - 1 > w.m0 + off + cfg.wr);
 
-        uint2 keep2;                                   // this thread's 64 bits of the tile, on their way during the wait
-        if (kDrop) keep2 = __ldg(reinterpret_cast<const uint2*>(cfg.keep + row * cfg.keep_words + (k0 >> 5)));
+        uint32_t keep[kEwCols / 32];                   // this thread's bits of the tile, on their way during the wait
+        if (kDrop) {
+#pragma unroll
+          for (int h = 0; h < kEwCols / 32; ++h) keep[h] = __ldg(cfg.keep + row * cfg.keep_words + (k0 >> 5) + h);
+        }
         ok = bwait(&sh->s_full[tg & 1], (tg >> 1) & 1, sh, 56);
         if (!ok) break;
-        SKEW(warp, tg, 0);
+        SKEW(warp, R::kEwWarps, tg, 0);
         tc_fence_after();
-        uint32_t r0[32], r1[32];
-        const uint32_t tSx = tS + (tg & 1) * kT + lane_addr + x * kHalfT;
-        tmem_ld32(tSx, r0);
-        tmem_ld32(tSx + 32, r1);
+        uint32_t r[kEwCols / 32][32];
+        const uint32_t tSx = tS + (tg & 1) * kT + lane_addr + x * kEwCols;
+#pragma unroll
+        for (int h = 0; h < kEwCols / 32; ++h) tmem_ld32(tSx + h * 32, r[h]);
         tmem_wait_ld();
         // ---- exp phase: P (times the soft cap's tanh factor) in fp32 registers -------------
         const float dist0 = (float)(qpos - k0);        // query position - key position of column 0
-        float pf[kHalfT];
+        float pf[kEwCols];
         // columns (keys) of this tile that this thread's query row sees
         const ColMask cm = make_col_mask(vk_lo - k0, vk_hi - k0);
         // One body, compiled per masked tile: no branch inside the unrolled loops.
@@ -1314,8 +1334,8 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const float2 one2 = make_float2(1.f, 1.f), none2 = make_float2(-1.f, -1.f), step2 = make_float2(-2.f, -2.f);
             float2 d2 = make_float2(dist0, dist0 - 1.f);
 #pragma unroll
-            for (int i = 0; i < kHalfT; i += 2) {
-              const uint32_t* rr = i < 32 ? r0 : r1;
+            for (int i = 0; i < kEwCols; i += 2) {
+              const uint32_t (&rr)[32] = r[i / 32];
               const float2 sv2 = make_float2(__uint_as_float(rr[i & 31]), __uint_as_float(rr[(i & 31) + 1]));
               const float2 u2 = score_unit_feat2<kCap, kAbs>(fk, sv2, d2);
               const float2 a2 = kCap ? f2fma(u2, cl2, nl2) : f2add(u2, nl2);
@@ -1332,16 +1352,16 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
           } else {
             const float2 c2 = make_float2(cfg.scale_log2, cfg.scale_log2), nl = make_float2(-l2, -l2);
 #pragma unroll
-            for (int i = 0; i < kHalfT; i += 2) {
-              const uint32_t* rr = i < 32 ? r0 : r1;
+            for (int i = 0; i < kEwCols; i += 2) {
+              const uint32_t (&rr)[32] = r[i / 32];
               const float2 a = f2fma(make_float2(__uint_as_float(rr[i & 31]), __uint_as_float(rr[(i & 31) + 1])), c2, nl);
-              float2 pe = ex2_pair<kPolyEvery>(a, i >> 1);
+              float2 pe = make_float2(ex2(a.x), ex2(a.y));
               if (kMask) {
                 pe.x = col_visible(cm, i) ? pe.x : 0.f;
                 pe.y = col_visible(cm, i + 1) ? pe.y : 0.f;
               }
               if (kDrop) {
-                const uint32_t kw = i < 32 ? keep2.x : keep2.y;
+                const uint32_t kw = keep[i / 32];
                 pe.x = (kw >> (i & 31)) & 1u ? pe.x : 0.f;
                 pe.y = (kw >> ((i & 31) + 1)) & 1u ? pe.y : 0.f;
               }
@@ -1361,15 +1381,15 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // ---- dS phase --------------------------------------------------------------------
         ok = bwait(&sh->dp_full, tg & 1, sh, 57);
         if (!ok) break;
-        SKEW(warp, tg, 1);
+        SKEW(warp, R::kEwWarps, tg, 1);
         tc_fence_after();
-        tmem_ld32(tdPx, r0);
-        tmem_ld32(tdPx + 32, r1);
+#pragma unroll
+        for (int h = 0; h < kEwCols / 32; ++h) tmem_ld32(tdPx + h * 32, r[h]);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < kEwCols / 32; ++c) {
           uint32_t pk[16];
-          const uint32_t* rr = c == 0 ? r0 : r1;
+          const uint32_t (&rr)[32] = r[c];
 #pragma unroll
           for (int i = 0; i < 16; ++i) {
             const float2 d = f2add(make_float2(__uint_as_float(rr[2 * i]), __uint_as_float(rr[2 * i + 1])),
@@ -1399,7 +1419,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       const int spos = posA + w.total - 1;
       ok = bwait(&sh->acc_done, wi & 1, sh, 58);
       if (!ok) break;
-      SKEW(warp, wi, 2);
+      SKEW(warp, R::kEwWarps, wi, 2);
       tc_fence_after();
       const bool via_tma = (p.cu_seqlens_q == nullptr) || (w.m0 + kT <= w.g.q_len);
       const uint32_t stg = slotK(spos);
@@ -1415,7 +1435,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     // No more items: the store lane may leave.  Between items the products of the next one wait for every warp, so that none
     // arrives on stg_ready twice in a phase; here the warps wait for one another (all of them get here, whatever `ok` says).
-    asm volatile("bar.sync 1, 256;\n" ::: "memory");
+    asm volatile("bar.sync 1, %0;\n" ::"n"(R::kEwThreads) : "memory");
     if (ok) {
       if (tid == 0) ok = post_store(sh, 0, wi, -1, 0, 0, 0, 0);
       mbar_arrive(smem_u32(&sh->stg_ready[0]));
@@ -1424,7 +1444,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   tc_fence_before();
   __syncthreads();
-  if (warp == 8) tmem_dealloc(tmem, 512);
+  if (warp == R::kProducer) tmem_dealloc(tmem, 512);
   if (tid == 0) {
     if (sh->abort_flag == 0) sched_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
@@ -1481,6 +1501,12 @@ template <typename K> int set_smem_attr(K kern, int bytes, const char* what) {
   return FA_OK;
 }
 
+// threads of a CTA of the plain variants, of those with score options
+int threads_of(bool options) {
+  return options ? Roles<ew_groups(Feat::kCap)>::kThreads : Roles<ew_groups(Feat::kNone)>::kThreads;
+}
+static_assert(ew_groups(Feat::kAlibi) == ew_groups(Feat::kCap), "one size for all options");
+
 // candidates of a launch: blocks x heads x batch must stay a 32-bit count
 bool candidate_count(int64_t blocks, int64_t heads, int64_t batch, int* out) {
   const int64_t n = blocks * heads * batch;
@@ -1526,8 +1552,8 @@ int launch_dkdv(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   unsigned int* queue = work_queue(a.device);
   if (queue == nullptr) return FA_ERR_LAUNCH;
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
-  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytes, st>>>(m.q, m.k, m.v, m.dout, m.dk, m.dv, a, with_order(a, cfg, a.heads_kv), nkb, ncand, queue,
-                                                           host_wait_word(a.device));
+  kern<<<grid, threads_of(cfg.keep == nullptr && extras), BCfg<D>::kSmemBytes, st>>>(
+      m.q, m.k, m.v, m.dout, m.dk, m.dv, a, with_order(a, cfg, a.heads_kv), nkb, ncand, queue, host_wait_word(a.device));
   return check_launch("bwd_dkdv_sm100");
 }
 
@@ -1552,8 +1578,8 @@ int launch_dq(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   unsigned int* queue = work_queue(a.device);
   if (queue == nullptr) return FA_ERR_LAUNCH;
   const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
-  kern<<<grid, kBwdThreads, BCfg<D>::kSmemBytesDq, st>>>(m.q, m.k, m.v, m.dout, m.dq, a, with_order(a, cfg, a.heads_q), nmb, ncand, queue,
-                                                             host_wait_word(a.device));
+  kern<<<grid, threads_of(cfg.keep == nullptr && (cfg.has_alibi || cfg.softcap > 0.f)), BCfg<D>::kSmemBytesDq, st>>>(
+      m.q, m.k, m.v, m.dout, m.dq, a, with_order(a, cfg, a.heads_q), nmb, ncand, queue, host_wait_word(a.device));
   return check_launch("bwd_dq_sm100");
 }
 

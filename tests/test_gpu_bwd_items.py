@@ -57,3 +57,23 @@ def test_packed_items_with_options(softcap, alibi, D):
         assert maxdiff(out[r], ro[0]) <= util.FWD_TOL
         for a, w in zip(grads, rg):
             assert maxdiff(a[r], w[0]) <= util.GRAD_TOL
+
+
+@pytest.mark.parametrize("wl", [0, 31, 32, 95, 127, 161])
+@pytest.mark.parametrize("softcap,alibi", [(20.0, True), (0.0, True), (0.0, False)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_masks_that_end_in_each_column_group(wl, softcap, alibi, D):
+    """Windows and a diagonal that cross the columns of every element-wise thread (64 of a tile, 32 with score options)."""
+    from flash_attn_triton_b200 import _native as N, _ops
+    B, S, H = 2, 417, 2
+    q, k, v, do = cases.dense_case(wl + D, B, S, S, H, H, D)
+    sl = torch.tensor([0.25, 0.0625]) if alibi else None
+    args = (D ** -0.5, True, wl, -1, softcap, None if sl is None else sl.to(DEV).repeat(B, 1), 0)
+    qd, kd, vd, dod = (t.to(DEV) for t in (q, k, v, do))
+    o, lse, _ = _ops.dense_forward(qd, kd, vd, *args, N.IMPL_TCGEN05, "bshd", True)
+    got = _ops.dense_backward(qd, kd, vd, o, lse, dod, *args, N.IMPL_TCGEN05, "bshd")
+    assert N.lib().fa_device_wait_status(0) == 0
+    want = orc.attention_grads_ref(q, k, v, do, softmax_scale=D ** -0.5, causal=True, window=(wl, -1), softcap=softcap,
+                                   alibi_slopes=sl)[2:]
+    for a, r in zip(got, want):
+        assert maxdiff(a, r) <= util.GRAD_TOL
