@@ -592,18 +592,11 @@ template <int kBM> inline dim3 packed_grid(const fa_attn_args& a, ScoreCfg& cfg)
   cfg.packed_list = !((int64_t)per * a.batch <= entries && a.heads_q <= 65535 && a.batch <= 65535);
   return cfg.packed_list ? dim3((unsigned)(entries * a.heads_q)) : dim3(per, a.heads_q, a.batch);
 }
-// The CTA's head, sequence and tile (with a causal mask the last, heaviest tile of a sequence comes first).  Called by whole
-// warps; false when there is no such tile.
+// Head, sequence and tile of entry (t, h) of the list, or of tile t, head h, sequence b without one (with a causal mask the
+// last, heaviest tile of a sequence comes first).  Called by whole warps; false when there is no such tile.
 template <int kBM>
-__device__ __forceinline__ bool packed_tile(const fa_attn_args& p, const ScoreCfg& cfg, int lane, int& h, int& b, SeqInfo& si, int& mt) {
-  int t;
-  if (!cfg.packed_list) {
-    t = blockIdx.x;
-    h = blockIdx.y;
-    b = blockIdx.z;
-  } else {
-    h = blockIdx.x % p.heads_q;                      // the heads of a tile next to one another
-    t = blockIdx.x / p.heads_q;
+__device__ __forceinline__ bool packed_entry(const fa_attn_args& p, const ScoreCfg& cfg, int lane, int t, int& b, SeqInfo& si, int& mt) {
+  if (cfg.packed_list) {
     auto first = [&](int s) { return p.cu_seqlens_q[s] / kBM + s; };
     b = 0;
     for (int n = p.batch; n > 1;) {                  // the last sequence of [b, b + n) that starts at t or before
@@ -619,6 +612,36 @@ __device__ __forceinline__ bool packed_tile(const fa_attn_args& p, const ScoreCf
   const int tiles = (min(si.q_len, p.seqlen_q) + kBM - 1) / kBM;
   mt = cfg.causal ? tiles - 1 - t : t;
   return t >= 0 && t < tiles;
+}
+// The tile of a CTA of packed_grid().
+template <int kBM>
+__device__ __forceinline__ bool packed_tile(const fa_attn_args& p, const ScoreCfg& cfg, int lane, int& h, int& b, SeqInfo& si, int& mt) {
+  int t = blockIdx.x;
+  if (cfg.packed_list) {
+    h = t % p.heads_q;                               // the heads of a tile next to one another
+    t /= p.heads_q;
+  } else {
+    h = blockIdx.y;
+    b = blockIdx.z;
+  }
+  return packed_entry<kBM>(p, cfg, lane, t, b, si, mt);
+}
+// The same for the c-th of its blocks.
+template <int kBM>
+__device__ __forceinline__ bool packed_tile_of(const fa_attn_args& p, const ScoreCfg& cfg, int c, int lane, int& h, int& b,
+                                               SeqInfo& si, int& mt) {
+  int t = c;
+  if (cfg.packed_list) {
+    h = t % p.heads_q;
+    t /= p.heads_q;
+  } else {
+    const int per = (p.seqlen_q + kBM - 1) / kBM;
+    t = c % per;
+    c /= per;
+    h = c % p.heads_q;
+    b = c / p.heads_q;
+  }
+  return packed_entry<kBM>(p, cfg, lane, t, b, si, mt);
 }
 
 }  // namespace fa

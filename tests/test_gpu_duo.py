@@ -164,3 +164,24 @@ def test_longer_rows(monkeypatch, B, Sq, S, H, D, kw):
     got = run()
     monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
     assert torch.equal(got, run())
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(causal=True), dict(softcap=20.0), dict(window_size=(40, 0))], ids=str)
+@pytest.mark.parametrize("D", [64, 128])
+def test_items_one_behind_the_other(monkeypatch, kw, D):
+    """Several items per CTA, of no, one and a few key tiles in turn, whole and ragged: everything is handed on from item to item.  Launches
+    one behind the other find the queue as the first one did."""
+    import flash_attn_triton_b200 as fa
+    rows = [128, 130, 1, 257, 300, 64, 128, 129] * 8
+    keys = [0, 128, 129, 0, 1, 300, 256, 17] * 8
+    assert enough_tiles(sum(-(-n // 128) for n in rows) // 2, 16)
+    g = torch.Generator(DEV).manual_seed(D)
+    mk = lambda n, h: torch.randn(n, h, D, device=DEV, dtype=torch.half, generator=g)
+    q, k, v = mk(sum(rows), 16), mk(sum(keys), 4), mk(sum(keys), 4)
+    cq, ck = (torch.tensor([0] + x, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32) for x in (rows, keys))
+    run = lambda: fa.flash_attn_varlen_func(q, k, v, cq, ck, max(rows), max(keys), **kw)
+    got = [run() for _ in range(3)]
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    want = run()
+    for o in got:
+        assert torch.equal(o, want)
