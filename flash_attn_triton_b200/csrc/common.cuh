@@ -626,10 +626,59 @@ __device__ __forceinline__ bool packed_tile(const fa_attn_args& p, const ScoreCf
   }
   return packed_entry<kBM>(p, cfg, lane, t, b, si, mt);
 }
-// The same for the c-th of its blocks.
+// The c-th of its blocks, for kernels that take them from a queue.  With a mask whose tiles see different numbers of keys the order
+// is that of block_of(): the heaviest tiles of 32 sequences (one per lane), then the second, ..., for `by_weight` heads at a time
+// (0: not so), so that what the CTAs read together stays in L2.  Sequence by sequence, heavy tiles of the last one set the time of a launch,
+// and items of different lengths in turn bring the two CTAs of an SM into each other's exponentials (us, before -> after): 14 sequences of 461, 32
+// heads of 64 67 -> 52, 24 prompts of 17 to 2048, 32 heads over 8 of 128 290 -> 276, 111 of 394 with a window of 1024 and 128 273 -> 215.
+constexpr int kPackedLevels = 64;      // tiles of the longest sequence; the search looks at one level after the other
+inline int packed_by_weight(const fa_attn_args& a, const ScoreCfg& cfg, int bm) {
+  if (!(cfg.causal || cfg.wl >= 0 || cfg.wr >= 0) || (a.seqlen_q + bm - 1) / bm > kPackedLevels) return 0;
+  int kv = a.heads_kv;                 // keys and values of the heads: 32 MB, see fwd_unit_group()
+  while (kv > 1 && (a.heads_kv % kv != 0 || (int64_t)4 * a.total_k * kv * a.head_dim > (int64_t)32 << 20)) --kv;
+  return kv * (a.heads_q / a.heads_kv);
+}
 template <int kBM>
-__device__ __forceinline__ bool packed_tile_of(const fa_attn_args& p, const ScoreCfg& cfg, int c, int lane, int& h, int& b,
-                                               SeqInfo& si, int& mt) {
+__device__ __forceinline__ bool packed_tile_of(const fa_attn_args& p, const ScoreCfg& cfg, int by_weight, int c, int lane,
+                                               int& h, int& b, SeqInfo& si, int& mt) {
+  auto first = [&](int s) { return p.cu_seqlens_q[s] / kBM + s; };       // entry of the list, see above
+  if (by_weight > 0) {
+    h = c % by_weight;
+    c /= by_weight;
+    const int entries = p.total_q / kBM + p.batch;
+    h += c / entries * by_weight;
+    c %= entries;
+    int b0 = 0;                                      // first of the 32 sequences that entry c belongs to
+    for (int n = (p.batch + 31) / 32; n > 1;) {
+      const int step = (n + 31) / 32, at = lane * step;
+      const unsigned before = __ballot_sync(0xffffffffu, at < n && first(32 * (b0 + at)) <= c);
+      const int skip = before != 0u ? (31 - __clz(before)) * step : 0;
+      b0 += skip;
+      n = min(step, n - skip);
+    }
+    b0 *= 32;
+    c -= first(b0);
+    int tiles = 0;
+    if (b0 + lane < p.batch) {
+      si = seq_info(p, b0 + lane);
+      tiles = (min(si.q_len, p.seqlen_q) + kBM - 1) / kBM;
+    }
+    const int most = __reduce_max_sync(0xffffffffu, tiles);
+    const bool down = cfg.causal || cfg.wr >= 0;     // the last tiles see most keys
+    unsigned have = 0u;                              // sequences with a tile mt
+    int i = 0;
+    for (; i < most; ++i) {
+      mt = down ? most - 1 - i : i;
+      have = __ballot_sync(0xffffffffu, tiles > mt);
+      if (c < __popc(have)) break;
+      c -= __popc(have);
+    }
+    if (i == most) return false;                     // (the list has up to 32 entries more than these sequences have tiles)
+    const unsigned mine = __ballot_sync(0xffffffffu, (have >> lane & 1u) != 0u && __popc(have & ((1u << lane) - 1u)) == c);
+    b = b0 + __ffs(mine) - 1;                        // the c-th of them
+    si = seq_info(p, b);
+    return true;
+  }
   int t = c;
   if (cfg.packed_list) {
     h = t % p.heads_q;

@@ -117,18 +117,18 @@ __device__ __forceinline__ Item sched_get(DShared* sh, int idx, bool& ok) {
 }
 
 // Item of candidate c (whole warp); false where there is none.
-__device__ __forceinline__ bool item_of(const fa_attn_args& p, const ScoreCfg& cfg, int c, int lane, Item& w) {
+__device__ __forceinline__ bool item_of(const fa_attn_args& p, const ScoreCfg& cfg, int by_weight, int c, int lane, Item& w) {
   SeqInfo si;
   int mt;
   if (p.cu_seqlens_q != nullptr) {
-    if (!packed_tile_of<kBM>(p, cfg, c, lane, w.h, w.b, si, mt)) return false;
+    if (!packed_tile_of<kBM>(p, cfg, by_weight, c, lane, w.h, w.b, si, mt)) return false;
   } else {
     const int mtiles = (p.seqlen_q + kBM - 1) / kBM;
     int unit;
     block_of(c, mtiles, p.heads_q * p.batch, cfg.unit_group, unit, mt);
     w.h = unit % p.heads_q;
     w.b = unit / p.heads_q;
-    if (cfg.causal) mt = mtiles - 1 - mt;          // heavy tiles first
+    if (cfg.causal || cfg.wr >= 0) mt = mtiles - 1 - mt;   // heavy tiles first
     si = seq_info(p, w.b);
   }
   w.m0 = mt * kBM;
@@ -161,7 +161,7 @@ template <typename T, int D, Feat kFeat, bool kDrop, bool kOwnP>
 __global__ void __launch_bounds__(kThreads, 2)
 fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
-                     const fa_attn_args p, const ScoreCfg cfg, const int ncand, unsigned int* const queue,
+                     const fa_attn_args p, const ScoreCfg cfg, const int ncand, const int by_weight, unsigned int* const queue,
                      int* const host_status) {
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr bool kPvSplit = !kExtras;     // P V in two key halves (measured: helps the plain variants only)
@@ -240,19 +240,18 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     while (ok) {
       if (i + 1 >= 2 * nt) {
         Item w;
-        int c = fidx == 0 ? (int)blockIdx.x : -1;
-        for (;;) {
-          if (c < 0) {
+        int c = blockIdx.x;
+        for (bool drawn = fidx > 0;; drawn = true) {
+          if (drawn) {
             unsigned int u = 0;
-            if (lane == 0) u = queue_draw(queue, ncand);
+            if (lane == 0) u = queue == nullptr ? (c == (int)blockIdx.x && fidx == 1 ? gridDim.x + c : ncand) : queue_draw(queue, ncand);
             c = (int)min(__shfl_sync(0xffffffffu, u, 0), (unsigned int)ncand);
           }
           if (c >= ncand) {
             w.nt = -1;
             break;
           }
-          if (item_of(p, cfg, c, lane, w)) break;
-          c = -1;
+          if (item_of(p, cfg, by_weight, c, lane, w)) break;
         }
         if (fidx == 0) {
           __syncthreads();                             // barriers are set up
@@ -680,7 +679,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   if (warp == 5) tmem_dealloc(tmem, 256);
   if (tid == 0) {
-    if (sh->abort_flag == 0) queue_finish(queue, ncand);
+    if (sh->abort_flag == 0 && queue != nullptr) queue_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }
@@ -741,22 +740,39 @@ static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t
   }
   ScoreCfg cfg = plain;
   int64_t ncand;
+  int by_weight = 0;
   if (packed) {
     const dim3 list = packed_grid<kBM>(a, cfg);
     ncand = (int64_t)list.x * list.y * list.z;
+    by_weight = packed_by_weight(a, cfg, kBM);
+    if (by_weight > 0) ncand = (a.total_q / kBM + (int64_t)a.batch) * a.heads_q;
   } else {
     const int blocks = (a.seqlen_q + kBM - 1) / kBM;
-    cfg.unit_group = blocks == 1 ? 1 : fwd_unit_group(a, cfg);
+    // Windows have the order of a causal mask: tiles that see equally many keys one behind the other.  The two CTAs of an SM then stay
+    // out of phase; with items of one to four tiles in turn they run into each other's exponentials (111 x 16 heads x 512 of 64, window of
+    // 1024 and 0: 230 -> 172 us).
+    ScoreCfg order = cfg;
+    order.causal = cfg.causal || cfg.wl >= 0 || cfg.wr >= 0;
+    cfg.unit_group = blocks == 1 ? 1 : fwd_unit_group(a, order);
     ncand = (int64_t)blocks * a.heads_q * a.batch;
   }
   if (ncand > 0x7fffffff - 4096) {
     set_error("fwd_duo_sm100: too many work items");
     return FA_ERR_UNSUPPORTED;
   }
-  unsigned int* queue = work_queue(a.device);
-  if (queue == nullptr) return FA_ERR_LAUNCH;
   const int grid = (int)std::min<int64_t>(ncand, 2 * (int64_t)sm_count(a.device));
-  kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, (int)ncand, queue, host_wait_word(a.device));
+  // Up to two items per CTA, of one size: no queue, CTA i takes items i and grid + i, so that second items go to CTAs on SMs of their own.
+  // Drawn from the queue, both CTAs of an SM may get one while another SM gets none (us, queue -> so: 8 x 16 x 512 of 64 with dropout 25.6 -> 24.7,
+  // 7 x 16 x 640 of 128 33.1 -> 31.9, 6 packed of 252, 32 heads over 8 of 128 23.0 -> 21.5); with items of different sizes the queue is as
+  // good or better (7 x 16 x 640 of 128, causal 27.4 for 30.4).
+  const int right = cfg.causal ? 0 : cfg.wr;
+  const bool even = (!cfg.causal && cfg.wl < 0 && cfg.wr < 0) || (cfg.wl >= 0 && right >= 0 && (int64_t)cfg.wl + right < 2 * kBN);
+  unsigned int* queue = nullptr;
+  if (ncand > 2 * (int64_t)grid || !even) {
+    queue = work_queue(a.device);
+    if (queue == nullptr) return FA_ERR_LAUNCH;
+  }
+  kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, (int)ncand, by_weight, queue, host_wait_word(a.device));
   return check_launch("fwd_duo_sm100");
 }
 

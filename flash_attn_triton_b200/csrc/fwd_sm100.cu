@@ -861,62 +861,36 @@ static OneTile one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
   return a.head_dim == 128 && 3 * ctas <= nk * sms ? kOneTileByCtas : kNotOneTile;
 }
 
-// Calls for the kernel with two CTAs per SM (fwd_duo_sm100.cu), whose starts and ends lie under each other's work but whose
-// tiles cost more at head_dim 128 (2.9 k cycles of an SM per tile, against 2.1 k: K and V of a CTA pass through two
-// ring slots, and every tile is loaded for 128 rows instead of 256).  Measured against the rule without it, launches
-// interleaved, 32 to 512 heads * batch, 128 to 4096 tokens, and packed batches of 12 to 48 sequences of 17 to 4096:
-//   up to 2.5 CTAs per SM        +1 to +15 %
-//   head_dim 64, plain           -2 to -22 % dense (16 x 32 heads x 1024, causal: 205 -> 191 us; no mask, 1531 tokens: 550 -> 518),
-//                                -2 to -11 % packed; +3 to +7 % where part of the exponentials would go to the FMA pipe
-//                                (all with P over S; P in columns of its own, fwd_duo_sm100.cu, is another -1 to -4 %)
-//   others, by the key tiles of a row tile on average, where the persistent kernel is the alternative: up to 6.5  -2 to -26 %
-//                                (packed 17 to 2048, causal: 396 -> 370), 8 and more  0 to +15 % (40 packed of 64 to 3000: +5 %)
-//   where the two-tile kernel is (below the persistent one's lengths; dropout), see longer_rows_for_two_ctas()
-//   windows, up to 10            -4 to -12 % (32 packed sequences of 256 to 4096, window 1024, ALiBi and soft cap, head_dim
-//                                128: 1686 -> 1621): two thirds of a short window's tiles are masked, and the pair of
-//                                tiles of the other kernels sees one more than either needs
-// Rows of more than 6.5 key tiles on average, up to 15, where the two-tile kernel is the alternative: a call may need a whole wave of
-// either kernel less than of the other, and the two-tile kernel computes an odd number of row tiles as the next even one.
-// Measured against it on 466 random calls (an earlier rule took all of them: everything up to 15 key tiles, causal 8 on average;
-// head_dim 128 and 64 with options, 2.5 to 20 CTAs per SM), and checked on 263 others that it takes: -7 % on average, two above
-// +0.7 %, +1.8 % at most; what the earlier rule took besides, 0 % on average, -6 to +18 %.
-//   dropout, ALiBi, no mask    0 to -25 % everywhere
-//   causal, dense, odd number of row tiles    -1 to -10 % from 3 CTAs per SM on; even 0 to +7 %, packed -6 to +18 %
-//   plain and soft cap, no mask, dense    by the waves: as many as the two-tile kernel +1 to +8 % (plain; soft cap on many waves
-//                              -8 to 0 %), 12 x 8 heads x 1536: 122 -> 127 us; fewer -2 to -25 %, 8 x 8 x 1030: 69 -> 54
-//   the same, packed           up to 10 tiles from 4 CTAs per SM on, up to 13 from 7 on: +1 to -13 %; +1 to +6 % beside that
-static bool longer_rows_for_two_ctas(const fa_attn_args& a, const ScoreCfg& cfg, int64_t nk, int64_t tiles) {
-  const bool packed = a.cu_seqlens_q != nullptr;
-  const int64_t sms = sm_count(a.device), ctas = tiles * a.heads_q;
-  if (nk > 15) return false;
-  if (cfg.causal) return !packed && (a.seqlen_q + kBM - 1) / kBM % 2 == 1 && ctas >= 3 * sms;
-  if (cfg.keep != nullptr || cfg.has_alibi) return true;
-  if (packed) return ctas >= (nk <= 10 ? 4 : 7) * sms && nk <= 13;
-  const int64_t pairs = (int64_t)((a.seqlen_q + 2 * kBM - 1) / (2 * kBM)) * a.batch * a.heads_q, rest = ctas % (2 * sms);
-  // a wave of two CTAs per SM takes 1.02 (soft cap) to 1.06 as long as one of the two-tile kernel, of one CTA three quarters
-  const int64_t waves = 100 * (ctas / (2 * sms)) + (rest == 0 ? 0 : rest <= sms ? 75 : 100);
-  return waves * (cfg.softcap > 0.f ? 102 : 106) <= 100 * 100 * ((pairs + sms - 1) / sms);
-}
-
+// Calls for the kernel with two persistent CTAs per SM (fwd_duo_sm100.cu).  Measured against the rule without it on 1820 random calls of
+// 8 to 32 heads, 1 to 64 sequences of 64 to 8191 tokens, dense and packed:
+//   up to 2.5 CTAs per SM        -20 to +70 %: the other kernels spread fewer tiles better
+//   where the two-tile kernel is the alternative (below the persistent one's lengths; dropout)    -16 % on average, -46 to +6 %; beyond
+//                                that +7 to +26 % on a few packed causal calls of 2.5 to 6 CTAs per SM (before they had packed_by_weight())
+//   where the persistent kernel is
+//     head_dim 64                plain and ALiBi -4 to -19 %, without a mask (part of the exponentials on the FMA pipe there) not taken;
+//                                windows -9 to -32 %; soft cap, causal -2 to -18 % (packed 0 %), no mask, more than 24 tiles +4 %
+//     head_dim 128               by the key tiles of a row tile: up to 6.5 -10 to -25 %; causal, dense: up to 24 tiles long -8 % (0 to -18), longer
+//                                -1 to +4 %; with soft cap up to 48 -4 % (+1 to -12), ALiBi +2 %; windows -13 % (+4 to -24); no mask 0 %;
+//                                packed 0 % (up to 16 tiles and from 8 CTAs per SM on -4 %)
 static bool two_ctas_are_faster(const fa_attn_args& a, const ScoreCfg& cfg, int persistent_from) {
-  const bool packed = a.cu_seqlens_q != nullptr, plain = !cfg.has_alibi && !(cfg.softcap > 0.f);
+  const bool packed = a.cu_seqlens_q != nullptr, cap = cfg.softcap > 0.f;
   const int64_t tiles = packed ? a.total_q / kBM + a.batch / 2 : (int64_t)((a.seqlen_q + kBM - 1) / kBM) * a.batch;
-  if (2 * tiles * a.heads_q <= 5 * (int64_t)sm_count(a.device)) return false;
+  const int64_t sms = sm_count(a.device);
+  if (2 * tiles * a.heads_q <= 5 * sms) return false;
   // the choice between the kernels must not show in the results
   if (cfg.keep == nullptr && persistent_from > 0 && a.seqlen_k >= persistent_from && fwd_poly_pays(a, cfg)) return false;
   if (!packed && a.seqlen_k >= 96 * kBN) return false;                      // one_tile_is_faster()
-  if (plain && a.head_dim == 64) return true;
+  if (cfg.keep != nullptr || persistent_from <= 0 || a.seqlen_k < persistent_from) return true;      // two-tile kernel
   // of a packed batch only the sum and the longest are known here
   const int64_t keys = packed ? (a.total_k / a.batch + a.seqlen_k) / 2 : a.seqlen_k;
   const int64_t nk = (keys + kBN - 1) / kBN;
-  int64_t twice = cfg.causal ? nk + 1 : 2 * nk;
   const int right = cfg.causal ? 0 : cfg.wr;
-  if (cfg.wl < 0 || right < 0) {
-    if (twice <= 13) return true;
-    const bool two_tile = cfg.keep != nullptr || persistent_from <= 0 || a.seqlen_k < persistent_from;   // the alternative
-    return two_tile && longer_rows_for_two_ctas(a, cfg, nk, tiles);
-  }
-  return std::min<int64_t>(twice, 2 * (((int64_t)cfg.wl + right) / kBN + 2)) <= 20;
+  if (cfg.wl >= 0 && right >= 0 && ((int64_t)cfg.wl + right) / kBN + 2 <= 12) return true;
+  if ((cfg.causal ? nk + 1 : 2 * nk) <= 13) return true;
+  if (a.head_dim == 64) return !cap || cfg.causal || nk <= 24;
+  if (cfg.has_alibi) return false;
+  if (packed) return nk <= 16 && tiles * a.heads_q >= 8 * sms;
+  return cfg.causal && nk <= (cap ? 48 : 24);
 }
 
 int fwd_sm100(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {

@@ -185,3 +185,22 @@ def test_items_one_behind_the_other(monkeypatch, kw, D):
     want = run()
     for o in got:
         assert torch.equal(o, want)
+
+
+@pytest.mark.parametrize("n", [3, 32, 33, 70])
+@pytest.mark.parametrize("kw", [dict(causal=True), dict(window_size=(200, 30)), dict(window_size=(100, -1)), dict(window_size=(-1, 60))], ids=str)
+def test_order_by_weight(monkeypatch, n, kw):
+    """Packed batches on both sides of 32 sequences, empty and short ones among them, heads in one group and in several (keys and values above
+    32 MB): every tile is worked on once, whatever the order."""
+    import flash_attn_triton_b200 as fa
+    lens = [(0, 1, 129, 700, 128, 383, 64)[i * i % 7] for i in range(n)]
+    lens[0] = 2000 if n > 3 else 6000
+    H, Hk = (16, 4) if n > 3 else (32, 32)
+    g = torch.Generator(DEV).manual_seed(n)
+    mk = lambda h: torch.randn(sum(lens), h, 128, device=DEV, dtype=torch.half, generator=g)
+    q, k, v = mk(H), mk(Hk), mk(Hk)
+    cu = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32)
+    run = lambda: fa.flash_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), **kw)
+    got = run()
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    assert torch.equal(got, run())
