@@ -54,7 +54,8 @@ constexpr int kThreads = 256;
 constexpr int kRegsSoftmax = 216, kRegsService = 40;
 static_assert(128 * (kRegsSoftmax + kRegsService) <= 128 * kThreads, "register split");
 constexpr int kSched = 4;         // depth of the in-CTA ring of work-queue entries
-constexpr int kConsumers = 6;     // warps that read it: softmax, issuer, store agent
+constexpr int kConsumers = 6;     // warps that read it: softmax, issuer, store agent (INT8: and the one that loads the scales)
+constexpr int kSkSlots = 4;       // INT8: key tiles whose scales are staged ahead
 
 template <int D> struct DCfg {
   static constexpr int kTileBytes = kBN * D * 2;
@@ -62,7 +63,8 @@ template <int D> struct DCfg {
   static constexpr int kBoxes = D / 64;
   static constexpr int kSmemTiles = (1 + kStages) * kTileBytes;
   static constexpr int kSmemBytes = kSmemTiles + 1024 /*align slack*/ + 1024 /*DShared*/;
-  static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
+  static constexpr int kSmemBytesInt8 = kSmemBytes + kSkSlots * kBN * 4;
+  static_assert(2 * (kSmemBytesInt8 + 1024) <= 228 * 1024, "two CTAs per SM");
 };
 
 // A work item: one tile of query rows.  Decoded once, by the producer warp.
@@ -88,6 +90,8 @@ struct DShared {
   uint64_t o_ready;        // the latest P V finished
   uint64_t stg_ready;      // output of an item staged for the store agent (128 arrivals)
   uint64_t stg_taken;      // ... and seen by it
+  uint64_t sk_full[kSkSlots];    // INT8: scales of the tile's keys written (slot: tile % kSkSlots)
+  uint64_t sk_empty[kSkSlots];   // ... read (128 arrivals: a slot is written again behind them)
   uint64_t sched_full[kSched];   // queue entry published by the producer warp
   uint64_t sched_empty[kSched];  // ... read by every consuming warp
   int4 sched_item[kSched][3];
@@ -157,14 +161,17 @@ template <> struct DFmt<__nv_bfloat16> { static constexpr int code = 1; };
 
 // kDrop: probabilities whose bit in cfg.keep is 0 do not enter P V (they stay in the row sum); the scale of
 // the kept ones goes into the normalisation of the output.  kOwnP: P in columns of its own (head_dim 64).
-template <typename T, int D, Feat kFeat, bool kDrop, bool kOwnP>
+// kInt8: INT8 scores on codes held as 16-bit floats (exact sums), sq and sk the scales of the query rows and of the keys, as in fwd_sm100.cu
+// and equal to it bit for bit.  (The form with int32 accumulators, head_dim 128, spilled 290 bytes and was 13 to 22 % slower than there.)
+template <typename T, int D, Feat kFeat, bool kDrop, bool kOwnP, bool kInt8 = false>
 __global__ void __launch_bounds__(kThreads, 2)
 fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmO,
                      const fa_attn_args p, const ScoreCfg cfg, const int ncand, const int by_weight, unsigned int* const queue,
-                     int* const host_status) {
+                     int* const host_status, const float* const sq, const float* const sk) {
   constexpr bool kExtras = kFeat != Feat::kNone, kCap = kFeat == Feat::kCap;
   constexpr bool kPvSplit = !kExtras;     // P V in two key halves (measured: helps the plain variants only)
+  static_assert(!kInt8 || (kFeat == Feat::kNone && !kDrop), "INT8 is plain");
   static_assert(!kOwnP || D == 64, "at head_dim 128 S and O fill the columns");
   constexpr int kPCol = kOwnP ? kBN + D : 0;
   using C = DCfg<D>;
@@ -174,6 +181,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   DShared* sh = reinterpret_cast<DShared*>(tiles + C::kSmemTiles);
   const uint32_t sQ = smem_u32(tiles), sKV = sQ + C::kTileBytes;
+  float* const skt = reinterpret_cast<float*>(tiles + C::kSmemTiles + 1024);     // INT8: [slot][key]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   const int off = p.q_pos_offset;
@@ -192,9 +200,13 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       mbar_init(smem_u32(&sh->p_half), 128);
       mbar_init(smem_u32(&sh->stg_ready), 128);
       mbar_init(smem_u32(&sh->stg_taken), 1);
+      for (int i = 0; kInt8 && i < kSkSlots; ++i) {
+        mbar_init(smem_u32(&sh->sk_full[i]), 1);
+        mbar_init(smem_u32(&sh->sk_empty[i]), 128);
+      }
       for (int i = 0; i < kSched; ++i) {
         mbar_init(smem_u32(&sh->sched_full[i]), 1);
-        mbar_init(smem_u32(&sh->sched_empty[i]), kConsumers);
+        mbar_init(smem_u32(&sh->sched_empty[i]), kConsumers + (kInt8 ? 1 : 0));
       }
       mbar_init(smem_u32(&sh->p_ready), 128);
       for (int i = 0; i < S; ++i) {
@@ -224,6 +236,33 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
   if (warp == 7) {
     reg_dealloc<kRegsService>();
+    if constexpr (kInt8) {
+      // Scales of the keys, times softmax_scale log2(e) (what the softmax warps need with them), a few tiles ahead.
+      int sidx = 0, tc = 0;
+      bool ok = true;
+      for (;;) {
+        const Item w = sched_get(sh, sidx++, ok);
+        if (!ok || w.nt < 0) break;
+        const float* const row = sk + ((int64_t)w.b * p.heads_q + w.h) * p.total_k;
+        for (int j = 0; j < w.nt && ok; ++j, ++tc) {
+          const int slot = tc % kSkSlots;
+          float v[kBN / 32];
+#pragma unroll
+          for (int i = 0; i < kBN / 32; ++i) {
+            const int col = (w.n_hi - 1 - j) * kBN + lane + 32 * i;
+            v[i] = col < w.k_len ? row[col] : 1.f;
+          }
+          ok = wait_bar(&sh->sk_empty[slot], ((tc / kSkSlots) & 1) ^ 1, sh, 12);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+#pragma unroll
+          for (int i = 0; i < kBN / 32; ++i) skt[slot * kBN + lane + 32 * i] = v[i] * (cfg.scale * 1.44269504f);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh->sk_full[slot]));
+        }
+        if (!ok) break;
+      }
+    }
   } else if (warp == 4) {
     // ------------------------------- TMA producer and work queue ------------------------
     // The warp draws and decodes the next item before it waits for the slot of the current one's last V tile: publishing it
@@ -413,6 +452,8 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       if (nt < 0) break;
       const int qpos = m0 + row_in_tile + off;
       const float slope = (kExtras && cfg.has_alibi) ? p.alibi_slopes[entry.b * p.heads_q + entry.h] : 0.f;
+      const float sq_row = kInt8 && m0 + row_in_tile < entry.q_len
+                               ? sq[((int64_t)entry.b * p.heads_q + entry.h) * p.total_k + m0 + row_in_tile] : 1.f;
       float m_used = -INFINITY, l = 0.f;
       const int tq_min = m0 + off, tq_max = tq_min + kBM - 1;
 
@@ -444,7 +485,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           mbar_arrive(smem_u32(&sh->s_free));
         }
 
-        const bool prescaled = kExtras || masked;
+        const bool prescaled = kExtras || masked || kInt8;
         // columns (keys) of this tile that this thread's query row sees (used by masked tiles only)
         ColMask cm;
         if (masked) {
@@ -452,7 +493,34 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           visible_k_interval(cfg, qpos, k_len, vk_lo, vk_hi);
           cm = make_col_mask(vk_lo - k0, vk_hi - k0);
         }
-        if (prescaled) {
+        if constexpr (kInt8) {
+          // score = acc * s_q * (s_k * softmax_scale * log2 e), s_q in the FMA that forms the exponent
+          const int slot = (tc + j) % kSkSlots;
+          ok = wait_bar(&sh->sk_full[slot], ((tc + j) / kSkSlots) & 1, sh, 37);
+          if (!ok) break;
+          const float4* S4 = reinterpret_cast<const float4*>(skt + slot * kBN);
+          auto scale_tile = [&](auto mask_tag) {
+            constexpr bool kMask = decltype(mask_tag)::value;
+#pragma unroll
+            for (int cc = 0; cc < 4; ++cc) {
+#pragma unroll
+              for (int i = 0; i < 32; i += 4) {
+                const float4 s4 = S4[cc * 8 + i / 4];
+                const float2 v01 = f2mul(make_float2(__uint_as_float(r[cc][i]), __uint_as_float(r[cc][i + 1])), make_float2(s4.x, s4.y));
+                const float2 v23 = f2mul(make_float2(__uint_as_float(r[cc][i + 2]), __uint_as_float(r[cc][i + 3])), make_float2(s4.z, s4.w));
+                float v[4] = {v01.x, v01.y, v23.x, v23.y};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  if (kMask) v[e] = col_visible(cm, cc * 32 + i + e) ? v[e] : -INFINITY;
+                  r[cc][i + e] = __float_as_uint(v[e]);
+                }
+              }
+            }
+          };
+          if (masked) scale_tile(std::true_type{});
+          else scale_tile(std::false_type{});
+          mbar_arrive(smem_u32(&sh->sk_empty[slot]));
+        } else if (prescaled) {
           // score pipeline and mask applied once, in place; values end up in the log2 domain.
           // One body, compiled per masked tile: no branch inside the unrolled loops.
           const float dist0 = (float)(qpos - k0);
@@ -543,6 +611,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         // on the plain path, cap log2e for capped scores (stored as tanh), else 1; all >= 0
         const float mul = !prescaled ? cfg.scale_log2 : (kCap ? cfg.softcap * FA_LOG2E : 1.f);
         mx *= mul;
+        if (kInt8) mx *= sq_row;                       // s_q > 0
 
         // ---- lazy rescale ----------------------------------------------------------------
         if (j == 0) {
@@ -583,7 +652,8 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           tc_fence_after();
         }
         if (kDrop && D == 128) keep4 = __ldg(keep_at);
-        const float2 mul2 = make_float2(mul, mul), nm2 = make_float2(-m_safe, -m_safe);
+        const float mul_x = kInt8 ? sq_row : mul;
+        const float2 mul2 = make_float2(mul_x, mul_x), nm2 = make_float2(-m_safe, -m_safe);
         float2 acc2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         auto half_done = [&]() {
           // the first 64 keys of P are complete: the issuer starts P V on them while the
@@ -599,6 +669,13 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           for (int i = 0; i < 32; i += 2) {
             const float2 a = f2fma(make_float2(__uint_as_float(r[cc][i]), __uint_as_float(r[cc][i + 1])), mul2, nm2);
             float2 pe = make_float2(ex2(a.x), ex2(a.y));
+            if constexpr (kInt8) {
+              // l sums the ROUNDED values that enter P V: with outlier keys a row's dominant probability is 2^x relative to a stale
+              // maximum, and its rounding has to cancel in O / l
+              pk[i >> 1] = Elem<T>::pack(pe.x, pe.y);
+              acc2[(i >> 1) & 1] = f2add(acc2[(i >> 1) & 1], Elem<T>::unpack(pk[i >> 1]));
+              continue;
+            }
             acc2[(i >> 1) & 1] = f2add(acc2[(i >> 1) & 1], pe);
             if (kDrop) {
               const uint32_t kw = cc == 0 ? keep4.x : cc == 1 ? keep4.y : cc == 2 ? keep4.z : keep4.w;
@@ -703,41 +780,15 @@ static bool p_over_s_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
   return cfg.wl >= 0 && right >= 0 && (int64_t)cfg.wl + right < 2 * kBN;
 }
 
-template <typename T, int D>
-static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
-  using C = DCfg<D>;
-  const bool packed = a.cu_seqlens_q != nullptr;
-  const int64_t q_rows = packed ? a.total_q : a.seqlen_q, k_rows = packed ? a.total_k : a.seqlen_k;
-  auto map = [&](CUtensorMap* m, const void* base, const int64_t* stride, int heads, int64_t rows) {
-    // dims (innermost first): head_dim, heads, rows, batch
-    const uint64_t dims[4] = {(uint64_t)D, (uint64_t)heads, (uint64_t)rows, (uint64_t)(packed ? 1 : a.batch)};
-    const uint64_t strides[3] = {(uint64_t)stride[2] * 2, (uint64_t)stride[1] * 2,
-                                 (uint64_t)(packed ? rows * stride[1] : stride[0]) * 2};
-    const uint32_t box[4] = {64, 1, 128, 1};
-    return encode_tmap(m, base, 2, 4, dims, strides, box);
-  };
-  CUtensorMap tq, tk, tv, to;
-  if (!map(&tq, a.q, a.q_stride, a.heads_q, q_rows) || !map(&tk, a.k, a.k_stride, a.heads_kv, k_rows) ||
-      !map(&tv, a.v, a.v_stride, a.heads_kv, k_rows) || !map(&to, a.o, a.o_stride, a.heads_q, q_rows)) {
-    set_error("fwd_duo_sm100: cuTensorMapEncodeTiled failed");
-    return FA_ERR_LAUNCH;
-  }
-  auto pick = [&](auto own) {
-    constexpr bool kOwn = decltype(own)::value;
-    return plain.keep != nullptr  ? fwd_duo_sm100_kernel<T, D, Feat::kNone, true, kOwn>
-           : plain.softcap > 0.f ? fwd_duo_sm100_kernel<T, D, Feat::kCap, false, kOwn>
-           : plain.has_alibi     ? fwd_duo_sm100_kernel<T, D, Feat::kAlibi, false, kOwn>
-                                 : fwd_duo_sm100_kernel<T, D, Feat::kNone, false, kOwn>;
-  };
-  auto kern = pick(std::false_type{});
-  if constexpr (D == 64) {
-    if (!p_over_s_is_faster(a, plain)) kern = pick(std::true_type{});
-  }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+template <typename K>
+static int launch_items(K kern, int smem, const CUtensorMap (&tm)[4], const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st,
+                        const float* sq = nullptr, const float* sk = nullptr) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) {
-    set_error("fwd_duo_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
+    set_error("fwd_duo_sm100: cudaFuncSetAttribute(%d): %s", smem, cudaGetErrorString(e));
     return FA_ERR_LAUNCH;
   }
+  const bool packed = a.cu_seqlens_q != nullptr;
   ScoreCfg cfg = plain;
   int64_t ncand;
   int by_weight = 0;
@@ -772,14 +823,52 @@ static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t
     queue = work_queue(a.device);
     if (queue == nullptr) return FA_ERR_LAUNCH;
   }
-  kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, (int)ncand, by_weight, queue, host_wait_word(a.device));
+  kern<<<grid, kThreads, smem, st>>>(tm[0], tm[1], tm[2], tm[3], a, cfg, (int)ncand, by_weight, queue, host_wait_word(a.device), sq, sk);
   return check_launch("fwd_duo_sm100");
+}
+
+template <typename T, int D>
+static int launch_duo(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t st) {
+  using C = DCfg<D>;
+  const bool packed = a.cu_seqlens_q != nullptr;
+  const int64_t q_rows = packed ? a.total_q : a.seqlen_q, k_rows = packed ? a.total_k : a.seqlen_k;
+  auto map = [&](CUtensorMap* m, const void* base, const int64_t* stride, int heads, int64_t rows) {
+    // dims (innermost first): head_dim, heads, rows, batch
+    const uint64_t dims[4] = {(uint64_t)D, (uint64_t)heads, (uint64_t)rows, (uint64_t)(packed ? 1 : a.batch)};
+    const uint64_t strides[3] = {(uint64_t)stride[2] * 2, (uint64_t)stride[1] * 2,
+                                 (uint64_t)(packed ? rows * stride[1] : stride[0]) * 2};
+    const uint32_t box[4] = {64, 1, 128, 1};
+    return encode_tmap(m, base, 2, 4, dims, strides, box);
+  };
+  CUtensorMap tm[4];
+  if (!map(&tm[0], a.q, a.q_stride, a.heads_q, q_rows) || !map(&tm[1], a.k, a.k_stride, a.heads_kv, k_rows) ||
+      !map(&tm[2], a.v, a.v_stride, a.heads_kv, k_rows) || !map(&tm[3], a.o, a.o_stride, a.heads_q, q_rows)) {
+    set_error("fwd_duo_sm100: cuTensorMapEncodeTiled failed");
+    return FA_ERR_LAUNCH;
+  }
+  auto pick = [&](auto own) {
+    constexpr bool kOwn = decltype(own)::value;
+    return plain.keep != nullptr  ? fwd_duo_sm100_kernel<T, D, Feat::kNone, true, kOwn>
+           : plain.softcap > 0.f ? fwd_duo_sm100_kernel<T, D, Feat::kCap, false, kOwn>
+           : plain.has_alibi     ? fwd_duo_sm100_kernel<T, D, Feat::kAlibi, false, kOwn>
+                                 : fwd_duo_sm100_kernel<T, D, Feat::kNone, false, kOwn>;
+  };
+  auto kern = pick(std::false_type{});
+  if constexpr (D == 64) {
+    if (!p_over_s_is_faster(a, plain)) kern = pick(std::true_type{});
+  }
+  return launch_items(kern, C::kSmemBytes, tm, a, plain, st);
 }
 
 int fwd_duo_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
   const bool bf = a.dtype == FA_BF16;
   if (a.head_dim == 64) return bf ? launch_duo<__nv_bfloat16, 64>(a, cfg, st) : launch_duo<__half, 64>(a, cfg, st);
   return bf ? launch_duo<__nv_bfloat16, 128>(a, cfg, st) : launch_duo<__half, 128>(a, cfg, st);
+}
+
+// INT8 forward of head_dim 64 on the maps of its caller (fwd_sm100.cu).
+int fwd_duo_int8(const CUtensorMap (&tm)[4], const fa_attn_args& a, const ScoreCfg& cfg, const float* sq, const float* sk, cudaStream_t st) {
+  return launch_items(fwd_duo_sm100_kernel<__half, 64, Feat::kNone, false, true, true>, DCfg<64>::kSmemBytesInt8, tm, a, cfg, st, sq, sk);
 }
 
 int fwd_duo_sm100_status() {

@@ -834,6 +834,7 @@ int fwd_persist_sm100_clear_status();
 bool fwd_poly_pays(const fa_attn_args& a, const ScoreCfg& cfg);
 int fwd_alt_sm100(const fa_attn_args& a, const ScoreCfg& cfg, bool poly, cudaStream_t st);
 int fwd_duo_sm100(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st);
+int fwd_duo_int8(const CUtensorMap (&tm)[4], const fa_attn_args&, const ScoreCfg&, const float* sq, const float* sk, cudaStream_t);
 
 // Plain dense problems for the one-tile kernel (fwd_alt_sm100.cu): a tile of its costs 1.8 k cycles of an SM
 // where a pair of tiles costs the others 4.3 k, but it has twice as many CTAs to start, drain and balance.
@@ -1003,6 +1004,10 @@ int fwd_int8_codes16(const fa_int8_args& a, const void* q16, const void* k16, cu
   }
   ScoreCfg cfg = make_score_cfg(a.softmax_scale, 0.f, a.causal, -1, -1, false);
   cfg.rescale_at = 0.f;
+  // Above 2.5 tiles of rows per SM the kernel with two persistent CTAs per SM, bit for bit equal (us, two-tile kernel -> so): 2 x 32 heads x 4096,
+  // causal 384 -> 362, 8 x 16 x 1024 131 -> 112, 1 x 8 x 8192, causal 208 -> 176, 8 x 32 x 8192, causal 5538 -> 5097.
+  if (2 * (int64_t)((p.seqlen_q + kBM - 1) / kBM) * p.batch * p.heads_q > 5 * (int64_t)sm_count(p.device))
+    return fwd_duo_int8({tq, tk, tv, to}, p, cfg, a.sq_scratch, a.s_k, st);
   const dim3 grid = dense_grid(p, (a.seqlen + 2 * kBM - 1) / (2 * kBM), cfg);
   auto kern = fwd_sm100_kernel<__half, D, Feat::kNone, 2, false>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);

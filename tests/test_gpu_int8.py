@@ -265,3 +265,18 @@ def test_query_codes_are_those_of_a_division(D):
         N.check(lib.fa_fwd_int8(C.byref(a), stream), "fa_fwd_int8")
         assert np.array_equal(q8.cpu().numpy().reshape(x.shape), r8.reshape(x.shape))
     assert np.array_equal(s_q.cpu().numpy().view(np.uint32), rs.reshape(-1).view(np.uint32))
+
+
+@pytest.mark.parametrize("S", [1024, 1088, 2112])
+@pytest.mark.parametrize("causal", [True, False])
+def test_head_dim_64_entries_do_not_depend_on_the_batch(S, causal):
+    """From 1024 tokens on a batch takes the kernel with two CTAs per SM, one entry of it the two-tile kernel: bit for bit equal."""
+    import flash_attn_triton_b200 as fa
+    B, H = 6, 16
+    assert 2 * B * H * (S // 128) > 5 * torch.cuda.get_device_properties(0).multi_processor_count
+    g = torch.Generator("cuda").manual_seed(S)
+    q, k, v = (torch.randn(B, H, S, 64, device="cuda", dtype=torch.half, generator=g) for _ in range(3))
+    k[:, :, ::37] *= 8                                # outlier keys
+    got = fa.attention_int8(q, k, v, causal=causal)
+    for b in (0, B - 1):
+        assert torch.equal(got[b:b + 1], fa.attention_int8(q[b:b + 1].contiguous(), k[b:b + 1].contiguous(), v[b:b + 1].contiguous(), causal=causal))
