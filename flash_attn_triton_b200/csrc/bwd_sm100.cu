@@ -794,10 +794,15 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         return reinterpret_cast<T*>(base) + (int64_t)w.g.k_boff * stride[0] + (int64_t)(w.g.k_row0 + key) * stride[1] +
                (int64_t)w.hk * stride[2] + x * DH;
       };
+      // Worked out here, under the wait for the first scores, or, with score options, where they are used (the registers are short): for
+      // items of one query tile 1.5 % (60 x 32 heads x 128 of 64, causal 73.5 -> 72.5 us).
+      T *gdv = nullptr, *gdk = nullptr;
+      if (!kExtras || w.total == 0) {
+        gdv = row_of(p.dv, p.dv_stride);
+        gdk = row_of(p.dk, p.dk_stride);
+      }
       if (w.total == 0) {
         // no query can see these keys: their gradients are zero
-        T* const gdv = row_of(p.dv, p.dv_stride);
-        T* const gdk = row_of(p.dk, p.dk_stride);
         if (gdv != nullptr) {
 #pragma unroll
           for (int c = 0; c < DH / 8; ++c) {
@@ -1006,7 +1011,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       SKEW(warp, R::kEwWarps, wi, 2);
       tc_fence_after();
       PROF_T0();
-      drain_acc<T, DH>(tdV + lane_addr + x * DH, 1.f, via_tma, slotB(pos - 1), lrow, x * DH, via_tma ? nullptr : row_of(p.dv, p.dv_stride));
+      drain_acc<T, DH>(tdV + lane_addr + x * DH, 1.f, via_tma, slotB(pos - 1), lrow, x * DH, kExtras && !via_tma ? row_of(p.dv, p.dv_stride) : gdv);
       tc_fence_before();
       if (via_tma) fence_proxy_async();
       // (the agent has seen the previous item's tiles: its barrier is never a whole phase behind)
@@ -1016,7 +1021,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (!ok) break;
       SKEW(warp, R::kEwWarps, wi, 3);
       tc_fence_after();
-      drain_acc<T, DH>(tdK + lane_addr + x * DH, cfg.scale, via_tma, slotA(pos - 1), lrow, x * DH, via_tma ? nullptr : row_of(p.dk, p.dk_stride));
+      drain_acc<T, DH>(tdK + lane_addr + x * DH, cfg.scale, via_tma, slotA(pos - 1), lrow, x * DH, kExtras && !via_tma ? row_of(p.dk, p.dk_stride) : gdk);
       tc_fence_before();
       if (via_tma) fence_proxy_async();
       mbar_arrive(smem_u32(&sh->stg_ready[1]));
