@@ -538,31 +538,28 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           u = sched_draw(queue, ncand);
           continue;
         }
-        // K: its slot is free once the last score GEMM of the previous item has read it
-        if (wi > 0 && !(ok = bwait_relaxed(&sh->k_free, (wi - 1) & 1, sh, 41))) break;
-        mbar_expect_tx(smem_u32(&sh->k_full), C::kTileBytes);
-        load_tile<D>(sK, &tmK, smem_u32(&sh->k_full), w.g.k_row0 + w.n0, w.hk, w.g.k_boff);
-        for (int it = 0; it < w.total; ++it, ++pos) {
-          const int hq = w.hk * G + it / w.ntiles, m = w.m_lo + it % w.ntiles;
+        // Loads in order of use: K Q(0) V dO(0), Q(1) dO(1), ...  K's slot is free once the last score GEMM of the previous item has read it,
+        // V's after its last dP GEMM.  (One copy, see the issuer.)
+        int hq = w.hk * G, m = w.m_lo;
+        const int m_end = w.m_lo + w.ntiles;
+        for (int it = 0; it < w.total && ok; ++it, ++pos) {
           if (it + 1 == w.total) u = sched_draw(queue, ncand);
-          if (!(ok = bwait_relaxed(&sh->empty_a[pos % SQ], ((pos / SQ) & 1) ^ 1, sh, 41))) break;
-          {
-            const uint32_t bar = smem_u32(&sh->full_a[pos % SQ]);
-            mbar_expect_tx(bar, C::kTileBytes);
-            load_tile<D>(slotA(pos), &tmQ, bar, w.g.q_row0 + m * kT, hq, w.g.q_boff);
+#pragma unroll 1
+          for (int e = it == 0 ? 0 : 2; e < 4 && ok; ++e) {
+            const int what = it == 0 ? e : 2 * e - 3;            // 0 K, 1 Q, 2 V, 3 dO
+            const bool q = what == 1, resident = (what & 1) == 0, b = what >= 2;
+            uint64_t* const empty = resident ? (b ? &sh->res_free : &sh->k_free) : q ? &sh->empty_a[pos % SQ] : &sh->empty_b[pos % SO];
+            uint64_t* const full = resident ? (b ? &sh->res_full : &sh->k_full) : q ? &sh->full_a[pos % SQ] : &sh->full_b[pos % SO];
+            const uint32_t parity = resident ? (wi - 1) & 1 : (((q ? pos / SQ : pos / SO) & 1) ^ 1);
+            if (!resident || wi > 0) ok = bwait_relaxed(empty, parity, sh, 41);
+            if (!ok) break;
+            mbar_expect_tx(smem_u32(full), C::kTileBytes);
+            load_tile<D>(resident ? (b ? sV : sK) : q ? slotA(pos) : slotB(pos), resident ? (b ? &tmV : &tmK) : q ? &tmQ : &tmdO, smem_u32(full),
+                         resident ? w.g.k_row0 + w.n0 : w.g.q_row0 + m * kT, resident ? w.hk : hq, resident ? w.g.k_boff : w.g.q_boff);
           }
-          if (it == 0) {
-            // V: after the last dP GEMM of the previous item
-            if (wi > 0 && !(ok = bwait_relaxed(&sh->res_free, (wi - 1) & 1, sh, 41))) break;
-            const uint32_t bar = smem_u32(&sh->res_full);
-            mbar_expect_tx(bar, C::kTileBytes);
-            load_tile<D>(sV, &tmV, bar, w.g.k_row0 + w.n0, w.hk, w.g.k_boff);
-          }
-          if (!(ok = bwait_relaxed(&sh->empty_b[pos % SO], ((pos / SO) & 1) ^ 1, sh, 41))) break;
-          {
-            const uint32_t bar = smem_u32(&sh->full_b[pos % SO]);
-            mbar_expect_tx(bar, C::kTileBytes);
-            load_tile<D>(slotB(pos), &tmdO, bar, w.g.q_row0 + m * kT, hq, w.g.q_boff);
+          if (++m == m_end) {
+            m = w.m_lo;
+            ++hq;
           }
         }
         if (!ok) break;
@@ -619,16 +616,15 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&sh->full_a[stage]));
-        if (it + 1 < w.total) {
-          fetch(w, it + 1);
-        } else {
-          // the entry after this one (published once the loads of this item are issued), if it
-          // has work, gets its first tile fetched ahead
-          const KItem wn = sched_get<KItem>(sh, sidx, false, ok);
+        // the item's next tile, or the first one of the entry after this (published once the loads of this item are issued), if
+        // that has work
+        KItem wf = w;
+        if (it + 1 == w.total) {
+          wf = sched_get<KItem>(sh, sidx, false, ok);
           if (!ok) break;
-          haven = wn.total > 0;
-          if (haven) fetch(wn, 0);
+          haven = wf.total > 0;
         }
+        if (wf.total > 0) fetch(wf, it + 1 < w.total ? it + 1 : 0);
       }
       if (!ok) break;
       fetched = haven;
@@ -691,37 +687,72 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const int tail_m = (p.cu_seqlens_q != nullptr && (w.g.q_len % kT) != 0) ? w.g.q_len / kT : -1;
       const int tail_first = w.g.q_len % kT, m_end = w.m_lo + w.ntiles;
       int ms = w.m_lo, mdp = w.m_lo;                   // query tiles of the next score and dP GEMMs
-      auto next_s = [&](int i) {                       // S(i) of the item, whose tile 0 is at ring position pos
-        if (i > last || !ok) return;
-        issue_s(pos + i, ms == tail_m ? tail_first : kT);
-        if (ok && i == last) mma_commit_lp(smem_u32(&sh->k_free), leader);     // K's last reader
-        ms = (ms + 1 == m_end) ? w.m_lo : ms + 1;
-      };
-      auto next_dp = [&](int i) {
-        if (i > last || !ok) return;
-        issue_dp(pos + i, mdp == tail_m ? tail_first : kT);
-        if (ok && i == last) mma_commit_lp(smem_u32(&sh->res_free), leader);   // V's last reader
-        mdp = (mdp + 1 == m_end) ? w.m_lo : mdp + 1;
-      };
       wq(&sh->k_full, wi & 1, 43);
-      next_s(0);
-      wq(&sh->res_full, wi & 1, 43);
-      next_dp(0);
-      if (NB == 2) next_s(1);
-      for (int i = 0; i < w.total && ok; ++i) {
-        const int ps = pos + i;
-        const bool more = i < last;
-        wq(&sh->p_ready[sbuf(ps)], sphase(ps), 45);
-        if (!ok) break;
-        mma_from_tmem<D, kEwCols>(tdV, tS + sbuf(ps) * 128, slotB(ps), idesc_acc, i > 0, leader);   // dV += P(i)^T dO(i)
-        // (dO(i)'s other reader, dP(i), precedes in the pipe)
-        mma_commit_lp(smem_u32(more ? &sh->empty_b[ps % SO] : &sh->dv_done), leader);
-        next_s(i + NB);
-        wq(&sh->ds_ready, ps & 1, 46);
-        if (!ok) break;
-        mma_from_tmem<D, kEwCols>(tdK, tdP, slotA(ps), idesc_acc, i > 0, leader);                   // dK += dS(i)^T Q(i)
-        if (more) mma_commit_lp(smem_u32(&sh->empty_a[ps % SQ]), leader);
-        next_dp(i + 1);
+      // One copy of each part here, in the producer and in the element-wise warps: a launch that follows other kernels waits for what it
+      // executes first (kernel of 104 -> 84 KB; within a training step, 8 x 16 x 512 of 128, causal 38.0 -> 34.7 us, 2 x 4 x 128 of 64
+      // 8.4 -> 8.0, 60 x 32 x 128 of 64 72.8 -> 67.2).  At head_dim 64, where a tile is half as long, the tests of this form cost longer items 3 to
+      // 10 %: first steps of their own there.
+      if constexpr (NB == 1) {
+        // Step -1 issues the first score and dP GEMMs.
+        for (int i = -NB; i < w.total && ok; ++i) {
+          const int ps = pos + i;
+          if (i >= 0) {
+            wq(&sh->p_ready[sbuf(ps)], sphase(ps), 45);
+            if (!ok) break;
+            mma_from_tmem<D, kEwCols>(tdV, tS + sbuf(ps) * 128, slotB(ps), idesc_acc, i > 0, leader);   // dV += P(i)^T dO(i)
+            // (dO(i)'s other reader, dP(i), precedes in the pipe)
+            mma_commit_lp(smem_u32(i < last ? &sh->empty_b[ps % SO] : &sh->dv_done), leader);
+          }
+          if (i + NB <= last) {
+            issue_s(ps + NB, ms == tail_m ? tail_first : kT);
+            if (ok && i + NB == last) mma_commit_lp(smem_u32(&sh->k_free), leader);      // K's last reader
+            ms = (ms + 1 == m_end) ? w.m_lo : ms + 1;
+          }
+          if (i >= 0) {
+            wq(&sh->ds_ready, ps & 1, 46);
+            if (!ok) break;
+            mma_from_tmem<D, kEwCols>(tdK, tdP, slotA(ps), idesc_acc, i > 0, leader);                   // dK += dS(i)^T Q(i)
+            if (i < last) mma_commit_lp(smem_u32(&sh->empty_a[ps % SQ]), leader);
+          }
+          if (i >= -1 && i < last) {
+            if (i < 0) wq(&sh->res_full, wi & 1, 43);
+            issue_dp(ps + 1, mdp == tail_m ? tail_first : kT);
+            if (ok && i + 1 == last) mma_commit_lp(smem_u32(&sh->res_free), leader);     // V's last reader
+            mdp = (mdp + 1 == m_end) ? w.m_lo : mdp + 1;
+          }
+        }
+      } else {
+        auto next_s = [&](int i) {                       // S(i) of the item, whose tile 0 is at ring position pos
+          if (i > last || !ok) return;
+          issue_s(pos + i, ms == tail_m ? tail_first : kT);
+          if (ok && i == last) mma_commit_lp(smem_u32(&sh->k_free), leader);     // K's last reader
+          ms = (ms + 1 == m_end) ? w.m_lo : ms + 1;
+        };
+        auto next_dp = [&](int i) {
+          if (i > last || !ok) return;
+          issue_dp(pos + i, mdp == tail_m ? tail_first : kT);
+          if (ok && i == last) mma_commit_lp(smem_u32(&sh->res_free), leader);   // V's last reader
+          mdp = (mdp + 1 == m_end) ? w.m_lo : mdp + 1;
+        };
+        next_s(0);
+        wq(&sh->res_full, wi & 1, 43);
+        next_dp(0);
+        if (NB == 2) next_s(1);
+        for (int i = 0; i < w.total && ok; ++i) {
+          const int ps = pos + i;
+          const bool more = i < last;
+          wq(&sh->p_ready[sbuf(ps)], sphase(ps), 45);
+          if (!ok) break;
+          mma_from_tmem<D, kEwCols>(tdV, tS + sbuf(ps) * 128, slotB(ps), idesc_acc, i > 0, leader);   // dV += P(i)^T dO(i)
+          // (dO(i)'s other reader, dP(i), precedes in the pipe)
+          mma_commit_lp(smem_u32(more ? &sh->empty_b[ps % SO] : &sh->dv_done), leader);
+          next_s(i + NB);
+          wq(&sh->ds_ready, ps & 1, 46);
+          if (!ok) break;
+          mma_from_tmem<D, kEwCols>(tdK, tdP, slotA(ps), idesc_acc, i > 0, leader);                   // dK += dS(i)^T Q(i)
+          if (more) mma_commit_lp(smem_u32(&sh->empty_a[ps % SQ]), leader);
+          next_dp(i + 1);
+        }
       }
       pos += w.total;
       if (ok) mma_commit_lp(smem_u32(&sh->acc_done), leader);
@@ -784,8 +815,12 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const long long prof_start = clock64();
 #endif
 
-    KItem w = sched_get<KItem>(sh, sidx++, true, ok);
-    while (ok && w.total >= 0) {
+    KItem w;
+    bool have = false;                               // w was looked at behind the item before it
+    for (;;) {
+      if (!have) w = sched_get<KItem>(sh, sidx++, true, ok);
+      have = false;
+      if (!ok || w.total < 0) break;
       const int key = w.n0 + lrow;
       // each group stores half of the head_dim columns of dV and of dK * softmax_scale
       constexpr int DH = D * kEwCols / kT;
@@ -810,7 +845,6 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             reinterpret_cast<uint4*>(gdk)[c] = make_uint4(0u, 0u, 0u, 0u);
           }
         }
-        w = sched_get<KItem>(sh, sidx++, true, ok);
         continue;
       }
       int vq_lo, vq_hi;                              // query positions that see this thread's key
@@ -1026,6 +1060,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (via_tma) fence_proxy_async();
       mbar_arrive(smem_u32(&sh->stg_ready[1]));
       w = wn;
+      have = true;
       PROF_ADD(6);
       ++wi;
     }
