@@ -52,6 +52,7 @@
 #include <cstdlib>
 #include "bwd_stats.cuh"
 #include "common.cuh"
+#include "queue.cuh"
 #define PROF_TAG bwd
 #include "prof.cuh"
 #include "skew.cuh"
@@ -167,22 +168,17 @@ __device__ __forceinline__ bool bwait_relaxed(uint64_t* bar, uint32_t parity, BS
   return bwait(bar, parity, sh, code);
 }
 
-// Work queue.  A CTA's first candidate is its own index; `counter[0]` hands out the others,
-// `counter[1]` counts the CTAs that have finished; the last one to finish puts both back to zero, so a
-// launch always finds them at zero.  A launch without others (ncand <= gridDim.x) does not touch them.
+// Work queue (queue.cuh).
 // The producer thread draws a candidate (just before the last loads of the current item, so that the
 // round trip to the counter is over when they are issued), decodes it into an item (12 ints: KItem / QItem) and
 // publishes the item to the other roles; entry number i of this CTA travels in ring slot
 // i % kSched.  Candidates outside their sequence are skipped; an item with total < 0 ends the queue.
-__device__ __forceinline__ unsigned int sched_draw(unsigned int* counter, int ncand) {
-  return ncand <= (int)gridDim.x ? (unsigned int)ncand : gridDim.x + atomicAdd(&counter[0], 1u);
-}
 template <typename Item, typename F>
 __device__ __forceinline__ Item sched_publish(BShared* sh, unsigned int* counter, int ncand, unsigned int u, int& fidx,
                                               bool& ok, F decode) {
   static_assert(sizeof(Item) == 48, "an item travels as three 16-byte words");
   Item w;
-  for (;; u = sched_draw(counter, ncand)) {
+  for (;; u = queue_draw(counter, ncand)) {
     if (u >= (unsigned int)ncand) {
       w.total = -1;
       break;
@@ -280,17 +276,6 @@ __device__ __forceinline__ bool post_store(BShared* sh, int x, int n, int addr, 
   sh->stg_msg[x][3] = batch;
   sh->stg_msg[x][4] = (int)release_bar;
   return true;
-}
-
-__device__ __forceinline__ void sched_finish(unsigned int* counter, int ncand) {
-  if (ncand <= (int)gridDim.x) return;
-  __threadfence();
-  const unsigned int done = atomicAdd(&counter[1], 1u);
-  if (done == gridDim.x - 1) {
-    counter[0] = 0u;
-    counter[1] = 0u;
-    __threadfence();
-  }
 }
 
 // TMA loads of one 128 x D tile (D/64 boxes) at (row, head, batch)
@@ -535,7 +520,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         const KItem w = sched_publish<KItem>(sh, queue, ncand, u, fidx, ok, decode);
         if (!ok || w.total < 0) break;
         if (w.total == 0) {
-          u = sched_draw(queue, ncand);
+          u = queue_draw(queue, ncand);
           continue;
         }
         // Loads in order of use: K Q(0) V dO(0), Q(1) dO(1), ...  K's slot is free once the last score GEMM of the previous item has read it,
@@ -543,7 +528,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         int hq = w.hk * G, m = w.m_lo;
         const int m_end = w.m_lo + w.ntiles;
         for (int it = 0; it < w.total && ok; ++it, ++pos) {
-          if (it + 1 == w.total) u = sched_draw(queue, ncand);
+          if (it + 1 == w.total) u = queue_draw(queue, ncand);
 #pragma unroll 1
           for (int e = it == 0 ? 0 : 2; e < 4 && ok; ++e) {
             const int what = it == 0 ? e : 2 * e - 3;            // 0 K, 1 Q, 2 V, 3 dO
@@ -1074,7 +1059,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   if (warp == R::kProducer) tmem_dealloc(tmem, 512);
   if (tid == 0) {
-    if (sh->abort_flag == 0) sched_finish(queue, ncand);
+    if (sh->abort_flag == 0) queue_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }
@@ -1169,7 +1154,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const QItem w = sched_publish<QItem>(sh, queue, ncand, u, fidx, ok, decode);
         if (!ok || w.total < 0) break;
         if (w.total == 0) {
-          u = sched_draw(queue, ncand);
+          u = queue_draw(queue, ncand);
           continue;
         }
         const int hk = w.h / (p.heads_q / p.heads_kv);
@@ -1200,7 +1185,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         };
         ok = load_k(0);
         for (int j = 0; j < w.total && ok; ++j) {
-          if (j + 1 == w.total) u = sched_draw(queue, ncand);
+          if (j + 1 == w.total) u = queue_draw(queue, ncand);
           if (j + 1 < w.total) ok = load_k(j + 1);
           if (ok) ok = load_v(j);
         }
@@ -1487,7 +1472,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   if (warp == R::kProducer) tmem_dealloc(tmem, 512);
   if (tid == 0) {
-    if (sh->abort_flag == 0) sched_finish(queue, ncand);
+    if (sh->abort_flag == 0) queue_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }

@@ -371,15 +371,6 @@ __device__ __forceinline__ void mma_commit_lp(uint32_t bar, uint32_t leader) {
       : "memory");
 }
 
-// Barrier 2 between the start of a CTA's kernel and its roles: the warp that initialises the mbarriers arrives and goes on (its
-// first loads need no one else), the other warps of the `kThreads` wait.
-template <int kThreads> __device__ __forceinline__ void setup_arrive() {
-  asm volatile("barrier.cta.arrive 2, %0;\n" ::"n"(kThreads) : "memory");
-}
-template <int kThreads> __device__ __forceinline__ void setup_sync() {
-  asm volatile("barrier.cta.sync 2, %0;\n" ::"n"(kThreads) : "memory");
-}
-
 // Register re-balancing between warpgroups (all 4 warps of the group execute it together).
 template <int N> __device__ __forceinline__ void reg_alloc() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(N));
