@@ -124,19 +124,8 @@ __device__ __forceinline__ Item sched_get(DShared* sh, int idx, bool& ok) {
 __device__ __forceinline__ bool item_of(const fa_attn_args& p, const ScoreCfg& cfg, int by_weight, int c, int lane, Item& w) {
   SeqInfo si;
   int mt;
-  if (p.cu_seqlens_q != nullptr) {
-    if (!packed_tile_of<kBM>(p, cfg, by_weight, c, lane, w.h, w.b, si, mt)) return false;
-  } else {
-    const int mtiles = (p.seqlen_q + kBM - 1) / kBM;
-    int unit;
-    block_of(c, mtiles, p.heads_q * p.batch, cfg.unit_group, unit, mt);
-    w.h = unit % p.heads_q;
-    w.b = unit / p.heads_q;
-    if (cfg.causal || cfg.wr >= 0) mt = mtiles - 1 - mt;   // heavy tiles first
-    si = seq_info(p, w.b);
-  }
+  if (!item_tile<kBM>(p, cfg, by_weight, c, lane, w.h, w.b, si, mt)) return false;
   w.m0 = mt * kBM;
-  if (w.m0 >= si.q_len) return false;
   w.q_len = si.q_len;
   w.k_len = si.k_len;
   w.q_row0 = (int)si.q_row0;
@@ -270,6 +259,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // (One copy of each part: what a CTA executes first it waits for, and where other kernels have run in between 40 KB more of
     // code were 5 k cycles at the start of a launch.)
     int fidx = 0, pos = 0, qi = 0;
+    unsigned int cand = kNoCandidate;
     bool ok = true;
     auto wwait = [&](uint64_t* bar, uint32_t parity, int code) {
       if (ok) ok = wait_bar(bar, parity, sh, code);
@@ -279,19 +269,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     while (ok) {
       if (i + 1 >= 2 * nt) {
         Item w;
-        int c = blockIdx.x;
-        for (bool drawn = fidx > 0;; drawn = true) {
-          if (drawn) {
-            unsigned int u = 0;
-            if (lane == 0) u = queue == nullptr ? (c == (int)blockIdx.x && fidx == 1 ? gridDim.x + c : ncand) : queue_draw(queue, ncand);
-            c = (int)min(__shfl_sync(0xffffffffu, u, 0), (unsigned int)ncand);
-          }
-          if (c >= ncand) {
-            w.nt = -1;
-            break;
-          }
-          if (item_of(p, cfg, by_weight, c, lane, w)) break;
-        }
+        if (!queue_item(queue, ncand, cand, lane, [&](int c) { return item_of(p, cfg, by_weight, c, lane, w); })) w.nt = -1;
         if (fidx == 0) {
           __syncthreads();                             // barriers are set up
           reg_dealloc<kRegsService>();
@@ -788,25 +766,9 @@ static int launch_items(K kern, int smem, const CUtensorMap (&tm)[4], const fa_a
     set_error("fwd_duo_sm100: cudaFuncSetAttribute(%d): %s", smem, cudaGetErrorString(e));
     return FA_ERR_LAUNCH;
   }
-  const bool packed = a.cu_seqlens_q != nullptr;
   ScoreCfg cfg = plain;
-  int64_t ncand;
-  int by_weight = 0;
-  if (packed) {
-    const dim3 list = packed_grid<kBM>(a, cfg);
-    ncand = (int64_t)list.x * list.y * list.z;
-    by_weight = packed_by_weight(a, cfg, kBM);
-    if (by_weight > 0) ncand = (a.total_q / kBM + (int64_t)a.batch) * a.heads_q;
-  } else {
-    const int blocks = (a.seqlen_q + kBM - 1) / kBM;
-    // Windows have the order of a causal mask: tiles that see equally many keys one behind the other.  The two CTAs of an SM then stay
-    // out of phase; with items of one to four tiles in turn they run into each other's exponentials (111 x 16 heads x 512 of 64, window of
-    // 1024 and 0: 230 -> 172 us).
-    ScoreCfg order = cfg;
-    order.causal = cfg.causal || cfg.wl >= 0 || cfg.wr >= 0;
-    cfg.unit_group = blocks == 1 ? 1 : fwd_unit_group(a, order);
-    ncand = (int64_t)blocks * a.heads_q * a.batch;
-  }
+  int by_weight;
+  const int64_t ncand = item_candidates<kBM>(a, cfg, by_weight);
   if (ncand > 0x7fffffff - 4096) {
     set_error("fwd_duo_sm100: too many work items");
     return FA_ERR_UNSUPPORTED;

@@ -2,12 +2,29 @@
 // `counter[0]` hands out the others, `counter[1]` counts the CTAs that have finished.  The last one to finish puts both back to
 // zero, so a launch always finds them at zero.  A launch without others (ncand <= gridDim.x) does not touch them.
 #pragma once
-#include <cuda_runtime.h>
 
 namespace fa {
 
 __device__ __forceinline__ unsigned int queue_draw(unsigned int* counter, int ncand) {
   return ncand <= (int)gridDim.x ? (unsigned int)ncand : gridDim.x + atomicAdd(&counter[0], 1u);
+}
+
+// The CTA's next item, for a whole warp: candidates are drawn until `decode` takes one; false behind the last.  `last` is the candidate drawn last
+// (kNoCandidate at the start): it stays with the caller between items, whatever became of the candidate.
+// counter null: no queue, CTA i takes i, i + gridDim.x, i + 2 gridDim.x, ...
+constexpr unsigned int kNoCandidate = 0xffffffffu;
+template <typename F>
+__device__ __forceinline__ bool queue_item(unsigned int* counter, int ncand, unsigned int& last, int lane, F decode) {
+  for (;;) {
+    unsigned int u = blockIdx.x;
+    if (last != kNoCandidate) {
+      u = last + gridDim.x;
+      if (counter != nullptr) u = __shfl_sync(0xffffffffu, lane == 0 ? queue_draw(counter, ncand) : 0u, 0);
+    }
+    last = u < (unsigned int)ncand ? u : (unsigned int)ncand;
+    if (last == (unsigned int)ncand) return false;
+    if (decode((int)last)) return true;
+  }
 }
 // One thread of a CTA that has drawn its last candidate.
 __device__ __forceinline__ void queue_finish(unsigned int* counter, int ncand) {

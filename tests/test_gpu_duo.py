@@ -204,3 +204,60 @@ def test_order_by_weight(monkeypatch, n, kw):
     got = run()
     monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
     assert torch.equal(got, run())
+
+
+# With 16 heads on 148 SMs: up to two items per CTA, some of the first ones no tiles (as a list of tiles; with three grid dimensions; short and empty
+# sequences first, last and in between)
+UNEVEN = [[256, 512, 384, 640, 128, 768, 256, 512], [128] * 12 + [256] * 6, [30] * 2 + [252] * 10, [0] + [256] * 12, [256] * 12 + [0, 0, 1],
+          [300, 0, 1, 640, 129, 0, 511, 250, 128, 128, 30, 700]]
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(alibi=True), dict(softcap=20.0), dict(wl=100, wr=60), dict(wl=0, wr=200, softcap=20.0)], ids=str)
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("lens", UNEVEN, ids=len)
+def test_two_items_per_cta_with_gaps(monkeypatch, lens, D, kw):
+    """Every row of O and every LSE is written, as by the two-tile kernel, into buffers that were full of NaN."""
+    import ctypes as C
+    from flash_attn_triton_b200 import _native as N, _ops
+    kw = dict(kw)
+    H, grid = 16, 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    entries, per = sum(lens) // 128 + len(lens), -(-max(lens) // 128)
+    assert grid < min(entries, per * len(lens)) * H <= 2 * grid and enough_tiles(sum(lens) // 128 + len(lens) // 2, H)
+    g = torch.Generator(DEV).manual_seed(D)
+    mk = lambda h: torch.randn(sum(lens), h, D, device=DEV, dtype=torch.half, generator=g)
+    q, k, v = mk(H), mk(4), mk(4)
+    cu = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32)
+    sl = torch.full((len(lens), H), 0.125, device=DEV) if kw.get("alibi") else None
+
+    def run():
+        o, lse = torch.full_like(q, float("nan")), torch.full((H, sum(lens)), float("nan"), device=DEV)
+        a = N.AttnArgs()
+        _ops._fill_common(a, q, k, v, o, _ops._THD, _ops._THD, batch=len(lens), sq=max(lens), sk=max(lens), hq=H, hkv=4, d=D, scale=D ** -0.5,
+                          causal=False, wl=kw.get("wl", -1), wr=kw.get("wr", -1), softcap=kw.get("softcap", 0.0), alibi=sl, q_pos_offset=0,
+                          impl=N.IMPL_AUTO, cu_q=cu, cu_k=cu)
+        a.lse2 = lse.data_ptr()
+        a.lse_stride = N._I64x3(0, 1, sum(lens))
+        N.check(N.lib().fa_varlen_fwd(C.byref(a), C.c_void_p(torch.cuda.current_stream().cuda_stream)), "fa_varlen_fwd")
+        return o, lse
+
+    got = run()
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    want = run()
+    for x, y in zip(got, want):
+        assert not torch.isnan(y).any() and torch.equal(x, y)
+
+
+def test_gradients_of_uneven_sequences():
+    """The unpadded batch of an encoder: no mask, sequences of unequal length."""
+    import flash_attn_triton_b200 as fa
+    lens, H, D = UNEVEN[1], 16, 64
+    q, k, v, do, cu, _ = cases.varlen_case(5, lens, lens, H, H, D)
+    ts = [t.to(DEV).requires_grad_() for t in (q, k, v)]
+    out = fa.flash_attn_varlen_func(*ts, cu.to(DEV), cu.to(DEV), max(lens), max(lens))
+    grads = torch.autograd.grad(out, ts, do.to(DEV))
+    for b in range(0, len(lens), 3):
+        r = slice(int(cu[b]), int(cu[b + 1]))
+        ro, _, *rg = orc.attention_grads_ref(q[None, r], k[None, r], v[None, r], do[None, r])
+        assert maxdiff(out[r], ro[0]) <= util.FWD_TOL
+        for a, w in zip(grads, rg):
+            assert maxdiff(a[r], w[0]) <= util.GRAD_TOL
