@@ -169,6 +169,7 @@ __device__ __forceinline__ bool packed_tile_of(const fa_attn_args& p, const Scor
     }
     b0 *= 32;
     c -= first(b0);
+    if (c < 0) return false;                         // rows before the first sequence
     int tiles = 0;
     if (b0 + lane < p.batch) {
       si = seq_info(p, b0 + lane);

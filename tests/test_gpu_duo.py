@@ -261,3 +261,21 @@ def test_gradients_of_uneven_sequences():
         assert maxdiff(out[r], ro[0]) <= util.FWD_TOL
         for a, w in zip(grads, rg):
             assert maxdiff(a[r], w[0]) <= util.GRAD_TOL
+
+
+def test_rows_before_the_first_sequence():
+    """With the value checks off a first sequence may start behind row 0: the rows before it belong to nobody."""
+    import flash_attn_triton_b200 as fa
+    first, lens, H = 700, [500] * 16, 16
+    assert enough_tiles(len(lens) * 4, H)
+    g = torch.Generator(DEV).manual_seed(1)
+    q, k, v = (torch.randn(first + sum(lens), H, 64, device=DEV, dtype=torch.half, generator=g) for _ in range(3))
+    cu = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32)
+    run = lambda q, k, v, cu: fa.flash_attn_varlen_func(q, k, v, cu, cu, 500, 500, causal=True)
+    want = run(*(t[first:].contiguous() for t in (q, k, v)), cu)
+    fa.set_validation(False)
+    try:
+        got = run(q, k, v, cu + first)
+    finally:
+        fa.set_validation(True)
+    assert torch.equal(got[first:], want)

@@ -139,14 +139,14 @@ def tiles_worked_on(lib, args, mask, grid_of, use_queue, rng):
     return got
 
 
-def call(q_lens, heads, heads_kv, packed, max_q=None, used=None):
+def call(q_lens, heads, heads_kv, packed, max_q=None, used=None, first=0):
     from flash_attn_triton_b200 import _native as N
     a = N.AttnArgs()
     a.batch, a.heads_q, a.heads_kv, a.head_dim = len(q_lens), heads, heads_kv, 128
     a.seqlen_q = a.seqlen_k = max(q_lens) if max_q is None else max_q
     keep = []
     if packed:
-        cu = np.concatenate([[0], np.cumsum(q_lens)]).astype(np.int32)
+        cu = np.concatenate([[first], first + np.cumsum(q_lens)]).astype(np.int32)
         a.total_q = a.total_k = int(cu[-1])
         a.cu_seqlens_q = a.cu_seqlens_k = cu.ctypes.data
         keep.append(cu)
@@ -160,8 +160,8 @@ def call(q_lens, heads, heads_kv, packed, max_q=None, used=None):
 MASKS = {"none": (0, -1, -1), "causal": (1, -1, -1), "narrow": (0, 100, 60), "left": (0, 200, -1), "right": (0, -1, 60)}
 
 
-def check(lib, q_lens, heads, heads_kv, packed, mask, grid_of, use_queue, rng, max_q=None, used=None):
-    a, keep = call(q_lens, heads, heads_kv, packed, max_q, used)
+def check(lib, q_lens, heads, heads_kv, packed, mask, grid_of, use_queue, rng, max_q=None, used=None, first=0):
+    a, keep = call(q_lens, heads, heads_kv, packed, max_q, used, first)
     got = tiles_worked_on(lib, a, MASKS[mask], grid_of, use_queue, rng)
     rows = [min(n, a.seqlen_q) for n in q_lens] if used is None else [min(n, u, a.seqlen_q) for n, u in zip(q_lens, used)]
     want = sorted((h, b, t) for b, n in enumerate(rows) for t in range(-(-n // 128)) for h in range(heads))
@@ -181,6 +181,16 @@ def test_every_tile_once(lib, lens, mask, use_queue):
     rng = random.Random(7)
     for grid_of in (HALF, FEW, lambda n: n):
         check(lib, LENGTHS[lens], 4, 2, True, mask, grid_of, use_queue, rng)
+
+
+@pytest.mark.parametrize("use_queue", [False, True])
+@pytest.mark.parametrize("mask", MASKS)
+@pytest.mark.parametrize("first", [1, 127, 128, 300, 6000])
+def test_rows_before_the_first_sequence(lib, first, mask, use_queue):
+    """A first sequence that does not start at row 0 (refused by the value checks, which a caller may have switched off)."""
+    rng = random.Random(first)
+    for lens in ([300, 0, 129, 64], [200] * 40):
+        check(lib, lens, 4, 2, True, mask, HALF, use_queue, rng, first=first)
 
 
 @pytest.mark.parametrize("seed", range(12))
