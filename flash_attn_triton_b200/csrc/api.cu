@@ -1,10 +1,16 @@
 // C ABI: argument validation, kernel-family dispatch, error strings.  See include/fa_b200.h.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
+#ifdef FA_SKEW
+#include <vector>
+#endif
 
 #include "common.cuh"
+#include "queue_slots.h"
 
 namespace fa {
 
@@ -74,27 +80,66 @@ int* host_wait_word(int device) {
 
 int host_wait_status(int device) { return (device >= 0 && device < 1024) ? g_host_wait[device] : 0; }
 
-static __device__ unsigned int g_work_queues[kWorkQueues][2];
+// Per device: 1024 streams, and 15 k launches in graphs.
+using WorkQueues = QueueSlots<1024, 15 * 1024>;
+static __device__ unsigned int g_work_queues[WorkQueues::kPairs][2];
+constexpr int kQueueDevices = 64;
 
-unsigned int* work_queue(int device) {
-  static unsigned int* base[64] = {nullptr};
-  static std::mutex mu;
-  static unsigned int turn = 0;
-  if (device < 0 || device >= 64) {
-    set_error("device ordinal %d out of range for the work queues", device);
-    return nullptr;
+static WorkQueues g_queue_slots[kQueueDevices];      // (of which the devices in use are in memory)
+static_assert(std::is_trivially_destructible<WorkQueues>::value, "the last graphs may go when the process ends");
+// A graph that a launch was captured into is gone, with all that was made of it.  Called on a thread of the driver: no CUDA call here, and
+// none under the lock that this takes.
+static void give_work_queue(void* where) {
+  const uintptr_t w = reinterpret_cast<uintptr_t>(where);
+  g_queue_slots[w % kQueueDevices].give((int)(w / kQueueDevices));
+}
+#ifdef FA_SKEW
+static int g_debug_no_queues = 0;
+#endif
+static int work_queue_of(int device, cudaStream_t st) {
+  constexpr int kNone = WorkQueues::kNone;
+#ifdef FA_SKEW
+  if (g_debug_no_queues) return kNone;
+#endif
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  cudaGraph_t graph = nullptr;
+  if (cudaStreamGetCaptureInfo_v2(st, &status, nullptr, &graph, nullptr, nullptr) != cudaSuccess) return kNone;
+  if (status == cudaStreamCaptureStatusNone) return cudaStreamGetId(st, &id) == cudaSuccess ? g_queue_slots[device].of_stream(id) : kNone;
+  if (status != cudaStreamCaptureStatusActive) return kNone;
+  const int i = g_queue_slots[device].take();
+  if (i == kNone) return kNone;
+  cudaUserObject_t owner = nullptr;
+  void* const where = reinterpret_cast<void*>((uintptr_t)i * kQueueDevices + device);
+  if (cudaUserObjectCreate(&owner, where, give_work_queue, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+    g_queue_slots[device].give(i);
+    return kNone;
   }
-  std::lock_guard<std::mutex> lock(mu);
-  if (base[device] == nullptr) {
-    void* p = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&p, g_work_queues);
-    if (e != cudaSuccess || p == nullptr) {
-      set_error("cudaGetSymbolAddress(work queues) on device %d: %s", device, cudaGetErrorString(e));
-      return nullptr;
-    }
-    base[device] = static_cast<unsigned int*>(p);
+  if (cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+    cudaUserObjectRelease(owner, 1);                 // gives the pair back
+    return kNone;
   }
-  return base[device] + 2 * (turn++ % kWorkQueues);
+  return i;
+}
+
+int queue_grid(int device, cudaStream_t st, int ncand, int ctas, unsigned int** queue) {
+  *queue = nullptr;
+  if (ncand <= ctas || device < 0 || device >= kQueueDevices) return ncand;
+  static std::atomic<unsigned int*> base[kQueueDevices];
+  unsigned int* p = base[device].load(std::memory_order_acquire);
+  int i = WorkQueues::kNone;
+  if (p == nullptr) {
+    void* at = nullptr;
+    if (cudaGetSymbolAddress(&at, g_work_queues) == cudaSuccess) p = static_cast<unsigned int*>(at);
+    base[device].store(p, std::memory_order_release);
+  }
+  if (p != nullptr) i = work_queue_of(device, st);
+  if (i == WorkQueues::kNone) {
+    cudaGetLastError();
+    return ncand;
+  }
+  *queue = p + 2 * (int64_t)i;
+  return ctas;
 }
 
 // kernel families (defined in the other translation units)
@@ -589,8 +634,9 @@ int fa_device_wait_clear(int device) {
   fwd_alt_sm100_clear_status();
   fwd_duo_sm100_clear_status();
   // a launch whose CTAs gave up has not put its pair of counters back to zero; the next one to get the pair would skip items
-  static const unsigned int zero[kWorkQueues][2] = {};
-  e = cudaMemcpyToSymbol(g_work_queues, zero, sizeof(zero));
+  void* queues = nullptr;
+  e = cudaGetSymbolAddress(&queues, g_work_queues);
+  if (e == cudaSuccess) e = cudaMemset(queues, 0, sizeof(g_work_queues));
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
   if (e != cudaSuccess) {
     set_error("clearing the work queues: %s", cudaGetErrorString(e));
@@ -614,12 +660,17 @@ int fa_mma_peak_probe(int32_t device, int32_t kind, int32_t iters, void* stream)
 }
 
 #ifdef FA_SKEW
-// Side build of the tests: the counters as launches whose CTAs gave up on a wait may leave them.
+// Side build of the tests: the counters as launches whose CTAs gave up on a wait may leave them; launches as where no pair is left; pairs
+// that captured launches have.
 int fa_debug_dirty_queues(unsigned int value) {
-  unsigned int pairs[kWorkQueues][2];
-  for (auto& pair : pairs) pair[0] = pair[1] = value;
-  return (int)cudaMemcpyToSymbol(g_work_queues, pairs, sizeof(pairs));
+  const std::vector<unsigned int> pairs(2 * WorkQueues::kPairs, value);
+  return (int)cudaMemcpyToSymbol(g_work_queues, pairs.data(), sizeof(g_work_queues));
 }
+int fa_debug_no_queues(int on) {
+  g_debug_no_queues = on;
+  return 0;
+}
+int fa_debug_captured_queues(int device) { return g_queue_slots[device].taken(); }
 #endif
 
 int fa_debug_set_wait_status(int32_t device, int32_t code) {

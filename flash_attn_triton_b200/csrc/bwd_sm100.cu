@@ -1059,7 +1059,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   if (warp == R::kProducer) tmem_dealloc(tmem, 512);
   if (tid == 0) {
-    if (sh->abort_flag == 0) queue_finish(queue, ncand);
+    queue_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }
@@ -1472,7 +1472,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   if (warp == R::kProducer) tmem_dealloc(tmem, 512);
   if (tid == 0) {
-    if (sh->abort_flag == 0) queue_finish(queue, ncand);
+    queue_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }
@@ -1575,9 +1575,8 @@ int launch_dkdv(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
     set_error("bwd_dkdv_sm100: too many work items");
     return FA_ERR_UNSUPPORTED;
   }
-  unsigned int* queue = work_queue(a.device);
-  if (queue == nullptr) return FA_ERR_LAUNCH;
-  const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
+  unsigned int* queue;
+  const int grid = queue_grid(a.device, st, ncand, sm_count(a.device), &queue);
   kern<<<grid, threads_of(cfg.keep == nullptr && extras), BCfg<D>::kSmemBytes, st>>>(
       m.q, m.k, m.v, m.dout, m.dk, m.dv, a, with_order(a, cfg, a.heads_kv), nkb, ncand, queue, host_wait_word(a.device));
   return check_launch("bwd_dkdv_sm100");
@@ -1601,9 +1600,8 @@ int launch_dq(const fa_attn_args& a, const ScoreCfg& cfg, cudaStream_t st) {
     set_error("bwd_dq_sm100: too many work items");
     return FA_ERR_UNSUPPORTED;
   }
-  unsigned int* queue = work_queue(a.device);
-  if (queue == nullptr) return FA_ERR_LAUNCH;
-  const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
+  unsigned int* queue;
+  const int grid = queue_grid(a.device, st, ncand, sm_count(a.device), &queue);
   kern<<<grid, threads_of(cfg.keep == nullptr && (cfg.has_alibi || cfg.softcap > 0.f)), BCfg<D>::kSmemBytesDq, st>>>(
       m.q, m.k, m.v, m.dout, m.dq, a, with_order(a, cfg, a.heads_q), nmb, ncand, queue, host_wait_word(a.device));
   return check_launch("bwd_dq_sm100");

@@ -18,19 +18,17 @@ namespace fa {
 void set_error(const char* fmt, ...);
 int check_launch(const char* what);
 int ensure_device(int device);
-int sm_count(int device);
-// Counter pair for one launch of a persistent kernel (work queue: [0] next candidate, [1] CTAs
-// finished; both zero between launches).  Pairs come from a fixed array inside the library and
-// are handed out in rotation, so launches that overlap on the GPU use different pairs as long as
-// fewer than kWorkQueues of them are in flight on one device.  Null (with the error set) on failure.
+int sm_count(int device);  // streaming multiprocessors of `device`
 // Time-outs of bounded device-side waits.  host_wait_word(): the word (in mapped host memory, as
 // a device-visible pointer; null when the mapping is unavailable) that a kernel of `device` sets
 // when one of its waits runs out.  host_wait_status(): its current value, read without touching
 // the GPU; the tcgen05 launchers refuse to launch while it is non-zero.
 int* host_wait_word(int device);
 int host_wait_status(int device);
-constexpr int kWorkQueues = 64;
-unsigned int* work_queue(int device);  // streaming multiprocessors of `device` (the persistent kernels launch one CTA each)
+// Grid of a persistent kernel with work for `ncand` candidates and room for `ctas` CTAs at once, and its counter pair of the work queue
+// (queue.cuh; [0] next candidate, [1] CTAs finished, both zero between launches).  No other launch that can run at the same time has the
+// pair, see queue_slots.h.  Without one -- every candidate has a CTA, or no pair is left, and then a CTA per candidate does it -- *queue is null.
+int queue_grid(int device, cudaStream_t st, int ncand, int ctas, unsigned int** queue);
 
 #define FA_REQUIRE(cond, ...)      \
   do {                             \

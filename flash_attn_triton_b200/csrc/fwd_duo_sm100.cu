@@ -734,7 +734,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
   __syncthreads();
   if (warp == 5) tmem_dealloc(tmem, 256);
   if (tid == 0) {
-    if (sh->abort_flag == 0 && queue != nullptr) queue_finish(queue, ncand);
+    if (queue != nullptr) queue_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
   }
 }
@@ -773,7 +773,7 @@ static int launch_items(K kern, int smem, const CUtensorMap (&tm)[4], const fa_a
     set_error("fwd_duo_sm100: too many work items");
     return FA_ERR_UNSUPPORTED;
   }
-  const int grid = (int)std::min<int64_t>(ncand, 2 * (int64_t)sm_count(a.device));
+  const int ctas = 2 * sm_count(a.device);
   // Up to two items per CTA, of one size: no queue, CTA i takes items i and grid + i, so that second items go to CTAs on SMs of their own.
   // Drawn from the queue, both CTAs of an SM may get one while another SM gets none (us, queue -> so: 8 x 16 x 512 of 64 with dropout 25.6 -> 24.7,
   // 7 x 16 x 640 of 128 33.1 -> 31.9, 6 packed of 252, 32 heads over 8 of 128 23.0 -> 21.5); with items of different sizes the queue is as
@@ -781,10 +781,7 @@ static int launch_items(K kern, int smem, const CUtensorMap (&tm)[4], const fa_a
   const int right = cfg.causal ? 0 : cfg.wr;
   const bool even = (!cfg.causal && cfg.wl < 0 && cfg.wr < 0) || (cfg.wl >= 0 && right >= 0 && (int64_t)cfg.wl + right < 2 * kBN);
   unsigned int* queue = nullptr;
-  if (ncand > 2 * (int64_t)grid || !even) {
-    queue = work_queue(a.device);
-    if (queue == nullptr) return FA_ERR_LAUNCH;
-  }
+  const int grid = even && ncand <= 2 * (int64_t)ctas ? std::min((int)ncand, ctas) : queue_grid(a.device, st, (int)ncand, ctas, &queue);
   kern<<<grid, kThreads, smem, st>>>(tm[0], tm[1], tm[2], tm[3], a, cfg, (int)ncand, by_weight, queue, host_wait_word(a.device), sq, sk);
   return check_launch("fwd_duo_sm100");
 }

@@ -26,6 +26,7 @@
 
 #include <cstdlib>
 #include "common.cuh"
+#include "queue.cuh"
 #include "sm100.cuh"
 
 namespace fa {
@@ -215,13 +216,14 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
       prefetch_tmap(&tmV);
       prefetch_tmap(&tmO);
       int pos = 0, qi = 0, fidx = 0;
-      bool ok = true;
+      bool ok = true, drawn = false;
       while (ok) {
         // draw the next item (as late as possible: all loads of the previous one are issued)
         Geo g;
         int c = -1;
         for (;;) {
-          const unsigned int u = atomicAdd(&queue[0], 1u);
+          const unsigned int u = drawn ? queue_draw(queue, ncand) : blockIdx.x;
+          drawn = true;
           if (u >= (unsigned int)ncand) break;
           if (item_geo(p, cfg, (int)u, npair, g)) {
             c = (int)u;
@@ -702,15 +704,8 @@ fwd_persist_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_c
   __syncthreads();
   if (warp == 8) tmem_dealloc(tmem, 512);
   if (tid == 0) {
+    queue_finish(queue, ncand);
     report_abort(sh->abort_flag, host_status);
-    // the last CTA to finish puts the queue back to zero for the next launch that is given it
-    __threadfence();
-    const unsigned int done = atomicAdd(&queue[1], 1u);
-    if (done == gridDim.x - 1) {
-      queue[0] = 0u;
-      queue[1] = 0u;
-      __threadfence();
-    }
   }
 }
 
@@ -762,8 +757,6 @@ static int launch_p(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t s
     set_error("fwd_persist_sm100: cudaFuncSetAttribute(%d): %s", C::kSmemBytes, cudaGetErrorString(e));
     return FA_ERR_LAUNCH;
   }
-  unsigned int* queue = work_queue(a.device);
-  if (queue == nullptr) return FA_ERR_LAUNCH;
   const int npair = (a.seqlen_q + 2 * kBM - 1) / (2 * kBM);
   const int64_t ncand64 = (int64_t)npair * a.heads_q * a.batch;
   if (ncand64 > (1 << 30)) {
@@ -773,7 +766,8 @@ static int launch_p(const fa_attn_args& a, const ScoreCfg& plain, cudaStream_t s
   const int ncand = (int)ncand64;
   ScoreCfg cfg = plain;
   cfg.unit_group = fwd_unit_group(a, plain);
-  const int grid = ncand < sm_count(a.device) ? ncand : sm_count(a.device);
+  unsigned int* queue;
+  const int grid = queue_grid(a.device, st, ncand, sm_count(a.device), &queue);
   kern<<<grid, kThreads, C::kSmemBytes, st>>>(tq, tk, tv, to, a, cfg, npair, ncand, queue, host_wait_word(a.device));
   return check_launch("fwd_persist_sm100");
 }

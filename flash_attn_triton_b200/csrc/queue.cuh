@@ -1,6 +1,7 @@
 // Work queue of the persistent kernels with a queue entry per CTA at the start: a CTA's first candidate is its own index;
 // `counter[0]` hands out the others, `counter[1]` counts the CTAs that have finished.  The last one to finish puts both back to
-// zero, so a launch always finds them at zero.  A launch without others (ncand <= gridDim.x) does not touch them.
+// zero, so a launch always finds them at zero.  A launch without others (ncand <= gridDim.x) does not touch them.  Which pair a launch
+// has: queue_slots.h.
 #pragma once
 
 namespace fa {
@@ -26,7 +27,7 @@ __device__ __forceinline__ bool queue_item(unsigned int* counter, int ncand, uns
     if (decode((int)last)) return true;
   }
 }
-// One thread of a CTA that has drawn its last candidate.
+// One thread of a CTA that has drawn its last candidate (or has given up on a wait and draws no more).
 __device__ __forceinline__ void queue_finish(unsigned int* counter, int ncand) {
   if (ncand <= (int)gridDim.x) return;
   __threadfence();

@@ -69,11 +69,53 @@ def after_a_failed_wait():
     L = N.lib()
     want = gradients()
     assert L.fa_debug_dirty_queues(3) == 0 and L.fa_device_wait_clear(0) == 0
-    for _ in range(4):                           # more launches than there are queues
+    for _ in range(4):
         got = gradients()
         wrong = [n for n in want if got[n] != want[n]]
         assert not wrong, wrong
     print("queues ok")
+
+
+def without_queues():
+    """Where no pair of counters is left, a CTA per item does the work, with the same results."""
+    from flash_attn_triton_b200 import _native as N
+    L = N.lib()
+    want = gradients()
+    assert L.fa_debug_no_queues(1) == 0
+    got = gradients()
+    wrong = [n for n in want if got[n] != want[n]]
+    assert not wrong, wrong
+    print("no queues ok")
+
+
+def captured_pairs():
+    """The counters of captured launches come back when their graph is gone, not before."""
+    import gc
+    import time
+
+    import flash_attn_triton_b200 as fa
+    from flash_attn_triton_b200 import _native as N
+    L = N.lib()
+    q = torch.randn(12, 256, 16, 64, device=DEV, dtype=torch.half)
+    want = fa.flash_attn_func(q, q, q, causal=True)
+    assert L.fa_debug_captured_queues(0) == 0
+    for _ in range(3):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            outs = [fa.flash_attn_func(q, q, q, causal=True) for _ in range(3)]
+        assert L.fa_debug_captured_queues(0) == 3
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, want) for o in outs) and L.fa_debug_captured_queues(0) == 3
+        del graph, outs
+        gc.collect()
+        for _ in range(100):                     # the driver gives them back on a thread of its own
+            if L.fa_debug_captured_queues(0) == 0:
+                break
+            torch.cuda.synchronize()
+            time.sleep(0.05)
+        assert L.fa_debug_captured_queues(0) == 0
+    print("captured ok")
 
 
 def library():
@@ -102,6 +144,14 @@ def test_late_warps_do_not_change_gradients():
 
 def test_queues_are_cleared_with_the_wait_status():
     assert "queues ok" in child("after_a_failed_wait")
+
+
+def test_results_without_a_queue():
+    assert "no queues ok" in child("without_queues")
+
+
+def test_captured_launches_give_their_queues_back():
+    assert "captured ok" in child("captured_pairs")
 
 
 if __name__ == "__main__":

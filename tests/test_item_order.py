@@ -206,3 +206,25 @@ def test_random_calls(lib, seed):
         B, S = rng.randint(1, 6), rng.randint(1, 700)
         used = None if rng.random() < .5 else [rng.randint(0, S) for _ in range(B)]
         check(lib, [S] * B, rng.choice((1, 3, 8)), 1, False, rng.choice(list(MASKS)), rng.choice((HALF, FEW)), rng.random() < .5, rng, S, used)
+
+
+def test_two_launches_with_one_pair_lose_tiles(lib):
+    """Why launches that run at the same time need counters of their own: the CTAs of two calls in turn, on one pair and on two."""
+    rng = random.Random(1)
+    a, keep = call([700] * 3, 4, 2, True)
+    h, b, mt = C.c_int(), C.c_int(), C.c_int()
+    ncand = lib.candidates(C.byref(a), *MASKS["causal"])
+    lost = {}
+    for pairs in (1, 2):
+        counters = [(C.c_uint * 2)(0, 0) for _ in range(pairs)]
+        last = {(n, cta): C.c_uint(0xffffffff) for n in range(2) for cta in range(5)}
+        got, running = {0: set(), 1: set()}, list(last)
+        while running:
+            n, cta = rng.choice(running)
+            if lib.next_item(5, cta, counters[n % pairs], C.byref(last[n, cta]), C.byref(h), C.byref(b), C.byref(mt)):
+                got[n].add((h.value, b.value, mt.value))
+            else:
+                running.remove((n, cta))
+                lib.finish(5, cta, counters[n % pairs])
+        lost[pairs] = 2 * 3 * 6 * 4 - len(got[0]) - len(got[1])
+    assert ncand > 5 and lost[1] > 0 and lost[2] == 0
