@@ -259,7 +259,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // (One copy of each part: what a CTA executes first it waits for, and where other kernels have run in between 40 KB more of
     // code were 5 k cycles at the start of a launch.)
     int fidx = 0, pos = 0, qi = 0;
-    unsigned int cand = kNoCandidate;
+    int c = blockIdx.x;
     bool ok = true;
     auto wwait = [&](uint64_t* bar, uint32_t parity, int code) {
       if (ok) ok = wait_bar(bar, parity, sh, code);
@@ -269,7 +269,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     while (ok) {
       if (i + 1 >= 2 * nt) {
         Item w;
-        if (!queue_item(queue, ncand, cand, lane, [&](int c) { return item_of(p, cfg, by_weight, c, lane, w); })) w.nt = -1;
+        if (!queue_item(queue, ncand, fidx == 0, c, lane, [&](int u) { return item_of(p, cfg, by_weight, u, lane, w); })) w.nt = -1;
         if (fidx == 0) {
           __syncthreads();                             // barriers are set up
           reg_dealloc<kRegsService>();

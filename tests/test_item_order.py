@@ -52,12 +52,12 @@ static const fa_attn_args* g_a;
 static ScoreCfg g_cfg;
 static int g_by_weight, g_ncand, g_h[32], g_b[32], g_mt[32];
 static unsigned* g_counter;
-static unsigned g_last[32];
-static bool g_found[32];
+static int g_last[32];
+static bool g_first, g_found[32];
 static void lane_main() {
   const int lane = current;
   SeqInfo si;
-  g_found[lane] = queue_item(g_counter, g_ncand, g_last[lane], lane, [&](int c) {
+  g_found[lane] = queue_item(g_counter, g_ncand, g_first, g_last[lane], lane, [&](int c) {
     return item_tile<128>(*g_a, g_cfg, g_by_weight, c, lane, g_h[lane], g_b[lane], si, g_mt[lane]);
   });
   ++done;
@@ -90,12 +90,13 @@ int candidates(const fa_attn_args* a, int causal, int wl, int wr) {
   g_ncand = (int)item_candidates<128>(*a, g_cfg, g_by_weight);
   return g_ncand;
 }
-// The next item of CTA `cta` of `grid`, whose last candidate was *last: 0 behind the last one.  counter: null without a queue.
-int next_item(int grid, int cta, unsigned* counter, unsigned* last, int* h, int* b, int* mt) {
+// The next item of CTA `cta` of `grid`, whose last candidate was *last (-1: none yet): 0 behind the last one.  counter: null without a queue.
+int next_item(int grid, int cta, unsigned* counter, int* last, int* h, int* b, int* mt) {
   gridDim.x = grid;
   blockIdx.x = cta;
   g_counter = counter;
-  for (int i = 0; i < 32; ++i) g_last[i] = *last;
+  g_first = *last < 0;
+  for (int i = 0; i < 32; ++i) g_last[i] = g_first ? cta : *last;
   run_warp();
   for (int i = 1; i < 32; ++i)
     if (g_found[i] != g_found[0] || g_last[i] != g_last[0] || (g_found[0] && (g_h[i] != g_h[0] || g_b[i] != g_b[0] || g_mt[i] != g_mt[0]))) abort();
@@ -122,7 +123,7 @@ def tiles_worked_on(lib, args, mask, grid_of, use_queue, rng):
     ncand = lib.candidates(C.byref(args), *mask)
     grid = grid_of(ncand)
     counter = (C.c_uint * 2)(0, 0)
-    last = [C.c_uint(0xffffffff) for _ in range(grid)]
+    last = [C.c_int(-1) for _ in range(grid)]
     h, b, mt = C.c_int(), C.c_int(), C.c_int()
     got, running = [], list(range(grid))
     while running:
@@ -217,7 +218,7 @@ def test_two_launches_with_one_pair_lose_tiles(lib):
     lost = {}
     for pairs in (1, 2):
         counters = [(C.c_uint * 2)(0, 0) for _ in range(pairs)]
-        last = {(n, cta): C.c_uint(0xffffffff) for n in range(2) for cta in range(5)}
+        last = {(n, cta): C.c_int(-1) for n in range(2) for cta in range(5)}
         got, running = {0: set(), 1: set()}, list(last)
         while running:
             n, cta = rng.choice(running)
