@@ -1460,8 +1460,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
     // No more items: the store lane may leave.  Between items the products of the next one wait for every warp, so that none
     // arrives on stg_ready twice in a phase; here the warps wait for one another (all of them get here, whatever `ok` says).
-    if constexpr (R::kEwThreads == 256) asm volatile("bar.sync 1, 256;\n" ::: "memory");
-    else asm volatile("bar.sync 1, 512;\n" ::: "memory");
+    asm volatile("bar.sync 1, %0;\n" ::"n"(R::kEwThreads) : "memory");
     if (ok) {
       if (tid == 0) ok = post_store(sh, 0, wi, -1, 0, 0, 0, 0);
       mbar_arrive(smem_u32(&sh->stg_ready[0]));

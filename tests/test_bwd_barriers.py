@@ -1,4 +1,4 @@
-"""The barriers between the issuer and the element-wise warps of the backward kernels, as a model on the CPU: warps, issuer
+"""The barriers between the issuer and the element-wise warps of the backward kernels (8, with score options 16), as a model on the CPU: warps, issuer
 and tensor pipe run in random orders with some of them slow, and every step checks that what it reads is complete and that
 what it overwrites has been read."""
 import os
@@ -8,7 +8,7 @@ import re
 import pytest
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "flash_attn_triton_b200", "csrc")
-WARPS = 8
+WARPS = (8, 16)
 
 
 class Fault(AssertionError):
@@ -53,13 +53,13 @@ def run(agents, rng):
             del waits[a]
 
 
-def dkdv(items, buffers, p_barriers, rng):
+def dkdv(items, buffers, p_barriers, rng, warps=8):
     """Tiles of dK/dV: `items` are numbers of query tiles, `buffers` score buffers, `p_barriers` barriers for "P stored"."""
     s_full, dp_full = [Barrier(1) for _ in range(buffers)], Barrier(1)
-    p_ready, ds_ready = [Barrier(WARPS) for _ in range(p_barriers)], Barrier(WARPS)
+    p_ready, ds_ready = [Barrier(warps) for _ in range(p_barriers)], Barrier(warps)
     pipe, closed = [], []
     s_done, dp_done = {}, -1                     # buffer -> tile computed in it
-    loaded_s, stored_p, loaded_dp, stored_ds = ([-1] * WARPS for _ in range(4))
+    loaded_s, stored_p, loaded_dp, stored_ds = ([-1] * warps for _ in range(4))
     total = sum(items)
 
     def tensor_pipe():
@@ -116,14 +116,14 @@ def dkdv(items, buffers, p_barriers, rng):
             stored_ds[w] = i
             ds_ready.arrive()
 
-    run([tensor_pipe(), issuer()] + [warp(w) for w in range(WARPS)], rng)
+    run([tensor_pipe(), issuer()] + [warp(w) for w in range(warps)], rng)
 
 
-def dq_results(items, last_waits, rng):
+def dq_results(items, last_waits, rng, warps=8):
     """Result tiles of the dQ kernel on their way to the store lane; `last_waits`: the warps wait for one another
     before the message that ends it."""
-    ready, taken, products, last = Barrier(WARPS), Barrier(1), Barrier(WARPS), Barrier(WARPS)
-    staged, message = [-1] * WARPS, None
+    ready, taken, products, last = Barrier(warps), Barrier(1), Barrier(warps), Barrier(warps)
+    staged, message = [-1] * warps, None
 
     def store_lane():
         for n in range(items + 1):
@@ -150,7 +150,7 @@ def dq_results(items, last_waits, rng):
                 staged[w] = n
             ready.arrive()
 
-    run([store_lane()] + [warp(w) for w in range(WARPS)], rng)
+    run([store_lane()] + [warp(w) for w in range(warps)], rng)
 
 
 ITEMS = [[5], [1, 1, 1, 1], [3, 2, 1], [2, 7]]
@@ -160,16 +160,25 @@ def kernel_source():
     return open(os.path.join(CSRC, "bwd_sm100.cu")).read()
 
 
+def test_barriers_count_every_element_wise_thread():
+    """Both numbers of groups: what the model takes for granted."""
+    src = kernel_source()
+    counts = re.findall(r"mbar_init\(smem_u32\(&sh->(?:p_ready|ds_ready|stg_ready)(?:\[\d\])?\), (.*?)\);", src)
+    assert len(counts) == 7 and set(counts) == {"R::kEwThreads"}
+    assert "kEwThreads = 128 * G, kEwWarps = 4 * G;" in src and "return f == Feat::kNone ? 2 : 4;" in src
+
+
+@pytest.mark.parametrize("warps", WARPS)
 @pytest.mark.parametrize("items", ITEMS, ids=str)
 @pytest.mark.parametrize("head_dim", [64, 128])
-def test_dkdv_tiles(items, head_dim):
+def test_dkdv_tiles(items, head_dim, warps):
     src = kernel_source()
     buffers = int(re.search(r"kSBuf = D == 64 \? (\d) : (\d);", src).group(1 if head_dim == 64 else 2))
     declared = re.search(r"uint64_t p_ready(?:\[(\d)\])?;", src).group(1)
     per_buffer = "p_ready[sbuf(pos)]" in src and "p_ready[sbuf(ps)], sphase(ps)" in src
     assert not per_buffer or int(declared) >= buffers
     for seed in range(60):
-        dkdv(items, buffers, buffers if per_buffer else 1, random.Random(seed))
+        dkdv(items, buffers, buffers if per_buffer else 1, random.Random(seed), warps)
 
 
 def test_the_model_sees_an_early_phase():
@@ -179,12 +188,13 @@ def test_the_model_sees_an_early_phase():
             dkdv([7], 2, 1, random.Random(seed))
 
 
+@pytest.mark.parametrize("warps", WARPS)
 @pytest.mark.parametrize("items", [0, 1, 2, 5])
-def test_dq_results(items):
+def test_dq_results(items, warps):
     end = kernel_source().split("No more items: the store lane may leave")[-1]
-    last_waits = "bar.sync 1, 256" in end.split("post_store(sh, 0, wi, -1")[0]
+    last_waits = re.search(r'"bar\.sync 1, %0;\\n" ::"n"\(R::kEwThreads\)', end.split("post_store(sh, 0, wi, -1")[0]) is not None
     for seed in range(100):
-        dq_results(items, last_waits, random.Random(seed))
+        dq_results(items, last_waits, random.Random(seed), warps)
 
 
 def test_the_model_sees_a_tile_stored_early():
