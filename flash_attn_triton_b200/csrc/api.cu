@@ -184,6 +184,9 @@ int bwd_sm100_status();
 void fwd_sm100_clear_status();
 void bwd_sm100_clear_status();
 int wait_probe(int device, long long clocks, cudaStream_t st);
+#ifdef FA_SKEW
+int skew_mode_bwd(int), skew_mode_duo(int);
+#endif
 int mma_peak_probe(int device, int kind, int iters, cudaStream_t st);
 
 static bool mult8(const int64_t* s, int n) {
@@ -669,6 +672,11 @@ int fa_debug_dirty_queues(unsigned int value) {
 int fa_debug_no_queues(int on) {
   g_debug_no_queues = on;
   return 0;
+}
+// The warps that are late (skew.cuh).
+int fa_debug_skew(int mode) {
+  const int e = skew_mode_bwd(mode);
+  return e != 0 ? e : skew_mode_duo(mode);
 }
 int fa_debug_captured_queues(int device) { return g_queue_slots[device].taken(); }
 #endif

@@ -55,6 +55,7 @@
 #include "queue.cuh"
 #define PROF_TAG bwd
 #include "prof.cuh"
+#define SKEW_TAG bwd
 #include "skew.cuh"
 #include "sm100.cuh"
 

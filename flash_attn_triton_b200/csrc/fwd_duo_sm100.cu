@@ -37,6 +37,8 @@
 
 #include "common.cuh"
 #include "queue.cuh"
+#define SKEW_TAG duo
+#include "skew.cuh"
 #include "sm100.cuh"
 
 namespace fa {
@@ -241,6 +243,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
             const int col = (w.n_hi - 1 - j) * kBN + lane + 32 * i;
             v[i] = col < w.k_len ? row[col] : 1.f;
           }
+          SKEW(warp, 8, tc, 0);
           ok = wait_bar(&sh->sk_empty[slot], ((tc / kSkSlots) & 1) ^ 1, sh, 12);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
@@ -286,6 +289,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       }
       if (i < 2 * nt) {                                // K_0 V_0 K_1 V_1 ...
         const int slot = pos % S;
+        SKEW(warp, 8, pos, 0);
         wwait(&sh->kv_empty[slot], ((pos / S) & 1) ^ 1, 11);
         if (ok && lane == 0) {
           const uint32_t bar = smem_u32(&sh->kv_full[slot]);
@@ -373,6 +377,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       // (the scores of the item's first tile overwrite those, or P, of the last item's last: read before the
       // epilogue that is now in the softmax warps, and by the P V ahead in the in-order pipe)
       for (int j = 0; j <= nt && ok; ++j) {
+        SKEW(warp, 8, tc + j, 0);
         // P in columns of its own: S(j) goes before P V_{j-1}, while the softmax warps have S(j - 1) in registers
         if (kOwnP && j > 0) wwait(&sh->s_free, (tc + j - 1) & 1, 26);
         if (!kOwnP && j > 0) issue_pv(pos + 2 * j - 1, tc + j - 1, j == 1, j == nt);
@@ -399,6 +404,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       ok = wait_bar(&sh->stg_ready, wi & 1, sh, 62);
       if (!ok) break;
       ++wi;
+      SKEW(warp, 8, wi, 2);
       if (leader) {
         mbar_arrive(smem_u32(&sh->stg_taken));
         if (p.cu_seqlens_q == nullptr || w.m0 + kBM <= w.q_len) {
@@ -451,6 +457,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
 
         ok = wait_bar(&sh->s_full, (tc + j) & 1, sh, 31);
         if (!ok) break;
+        SKEW(warp, 8, tc + j, 0);
         tc_fence_after();
 
         // ---- the 128 scores of this row into registers -------------------------------------
@@ -621,6 +628,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
           }
         }
         const float m_safe = (m_used == -INFINITY) ? 0.f : m_used;
+        SKEW(warp, 8, tc + j, 1);
 
         // ---- P = exp2(s - m), row sum, P -> TMEM, over S or in columns of its own -------------
         // packed pairs: one FMA, two exponentials, one conversion and one add per two scores
@@ -677,6 +685,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
       // row by row instead (the unit would write the neighbour's rows).
       tc += nt;
       pos += 2 * nt;
+      SKEW(warp, 8, wi, 2);
       if (ok && nt > 0) ok = wait_bar(&sh->o_ready, (tc - 1) & 1, sh, 35);
       if (!ok) break;
       tc_fence_after();
@@ -717,6 +726,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
         tc_fence_before();
         if (via_tma) fence_proxy_async();
         // (the agent has seen the previous item's tile: its barrier is never a whole phase behind)
+        SKEW(warp, 8, wi, 3);
         if (wi > 0 && !(ok = wait_bar(&sh->stg_taken, (wi - 1) & 1, sh, 63))) break;
         mbar_arrive(smem_u32(&sh->stg_ready));
         ++wi;

@@ -1,5 +1,5 @@
-"""Backward kernels whose element-wise warps are made to drift apart (csrc/skew.cuh, a build of its own): the gradients stay
-bit for bit those of the shipped build, whichever warps are late."""
+"""Backward kernels whose element-wise warps, and forwards with two CTAs per SM whose warps of all roles are made to drift apart (csrc/skew.cuh, a
+build of its own): results stay bit for bit those of the shipped build, whichever warps are late."""
 import hashlib
 import json
 import os
@@ -54,12 +54,54 @@ def gradients():
     return out
 
 
-def skewed():
+FORWARDS = {                                     # more than 2.5 tiles per SM, several items for each CTA
+    "one tile": dict(B=60, Sq=128, Sk=128),
+    "causal": dict(B=14, Sq=400, Sk=400, causal=True),
+    "odd": dict(B=14, Sq=385, Sk=640),
+    "window": dict(B=10, Sq=700, Sk=700, window_size=(200, 30)),
+    "dropout": dict(B=14, Sq=512, Sk=512, causal=True, dropout_p=0.2),
+    "options": dict(B=14, Sq=384, Sk=384, causal=True, softcap=20.0, alibi=True),
+    "packed": dict(lens=[0, 300, 128, 513, 64, 257, 0, 129, 700, 31, 256, 512] * 4, keys=[128, 0, 300, 128, 513, 64, 257, 0, 129, 700, 31, 256] * 4),
+    "int8": dict(B=6, Sq=1088, Sk=1088, causal=True),
+}
+
+
+def forwards():
+    """Digests of O of every call."""
+    import flash_attn_triton_b200 as fa
+    from flash_attn_triton_b200 import _native as N
+    out = {}
+    for name, call in FORWARDS.items():
+        for D in (64, 128):
+            kw, H = dict(call), 16
+            if kw.pop("alibi", False):
+                kw["alibi_slopes"] = torch.tensor([0.5 ** (i + 1) for i in range(H)], device=DEV)
+            g = torch.Generator(DEV).manual_seed(D)
+            mk = lambda *s: torch.randn(*s, D, device=DEV, dtype=torch.half, generator=g)
+            random.seed(3)                       # the dropout mask
+            if "lens" in kw:
+                lens, keys = kw.pop("lens"), kw.pop("keys")
+                cu, ck = (torch.tensor([0] + x, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32) for x in (lens, keys))
+                o = fa.flash_attn_varlen_func(mk(sum(lens), H), mk(sum(keys), 4), mk(sum(keys), 4), cu, ck, max(lens), max(keys), **kw)
+            else:
+                B, Sq, Sk = kw.pop("B"), kw.pop("Sq"), kw.pop("Sk")
+                assert 2 * B * H * -(-Sq // 128) > 5 * torch.cuda.get_device_properties(0).multi_processor_count
+                if name == "int8":
+                    o = fa.attention_int8(mk(B, H, Sq), mk(B, H, Sk), mk(B, H, Sk), **kw)
+                else:
+                    o = fa.flash_attn_func(mk(B, Sq, H), mk(B, Sk, H), mk(B, Sk, H), **kw)
+            assert torch.isfinite(o).all(), (name, D)
+            out[f"{name}-{D}-o"] = hashlib.sha256(o.cpu().numpy().tobytes()).hexdigest()
+    assert N.lib().fa_device_wait_status(0) == 0
+    return out
+
+
+def skewed(results):
     from flash_attn_triton_b200 import _native as N
     modes = {}
     for mode in range(5):
         assert N.lib().fa_debug_skew(mode) == 0
-        modes[mode] = gradients()
+        modes[mode] = globals()[results]()
     print("digests " + json.dumps(modes))
 
 
@@ -126,17 +168,18 @@ def library():
         subprocess.run([sys.executable, "-m", "flash_attn_triton_b200.build"], cwd=ROOT, env=env, check=True, timeout=900)
 
 
-def child(what):
+def child(*what):
     library()
-    r = subprocess.run([sys.executable, os.path.abspath(__file__), what], capture_output=True, text=True, timeout=600,
+    r = subprocess.run([sys.executable, os.path.abspath(__file__), *what], capture_output=True, text=True, timeout=600,
                        env=dict(os.environ, FA_B200_LIB=LIB, PYTHONPATH=os.pathsep.join(sys.path)))
     assert r.returncode == 0, r.stdout + r.stderr
     return r.stdout
 
 
-def test_late_warps_do_not_change_gradients():
-    modes = json.loads(child("skewed").split("digests ", 1)[1])
-    want = gradients()
+@pytest.mark.parametrize("results", ["gradients", "forwards"])
+def test_late_warps_do_not_change_results(results):
+    modes = json.loads(child("skewed", results).split("digests ", 1)[1])
+    want = globals()[results]()
     for mode, got in modes.items():
         wrong = [n for n in want if got[n] != want[n]]
         assert not wrong, (mode, wrong)
@@ -155,4 +198,4 @@ def test_captured_launches_give_their_queues_back():
 
 
 if __name__ == "__main__":
-    globals()[sys.argv[1]]()
+    globals()[sys.argv[1]](*sys.argv[2:])
