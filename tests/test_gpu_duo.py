@@ -279,3 +279,20 @@ def test_rows_before_the_first_sequence():
     finally:
         fa.set_validation(True)
     assert torch.equal(got[first:], want)
+
+
+@pytest.mark.parametrize("kw", [dict(causal=True), dict(window_size=(200, -1)), dict(window_size=(-1, 60)), dict(causal=True, softcap=20.0)], ids=str)
+@pytest.mark.parametrize("D,H", [(64, 32), (128, 16)])
+def test_order_by_weight_in_groups_of_heads(monkeypatch, D, H, kw):
+    """Keys and values above 32 MB, so that the heads come in groups, in sequences too short for the persistent kernel: every tile is worked
+    on once."""
+    import flash_attn_triton_b200 as fa
+    lens = [1500, 0, 1, 1900, 700, 128, 1031, 64]
+    assert 4 * sum(lens) * H * D > 32 << 20 and max(lens) < 2048 and enough_tiles(sum(lens) // 128, H)
+    g = torch.Generator(DEV).manual_seed(D)
+    q, k, v = (torch.randn(sum(lens), H, D, device=DEV, dtype=torch.half, generator=g) for _ in range(3))
+    cu = torch.tensor([0] + lens, dtype=torch.int32, device=DEV).cumsum(0, dtype=torch.int32)
+    run = lambda: fa.flash_attn_varlen_func(q, k, v, cu, cu, max(lens), max(lens), **kw)
+    got = run()
+    monkeypatch.setenv("FA_B200_FWD_PERSISTENT_FROM", "0")
+    assert torch.equal(got, run())
