@@ -88,7 +88,8 @@ template <int G> struct Roles {
 // 150 -> 144, 105 -> 102.  Without options the phase is close to the unit's 1.02 k with two groups (1.35 k), and
 // the larger number of warps delays the MMAs: 4 x 16 x 4096 of 128 864 -> 877, 605 -> 617; 4 x 32 x 1024 x 1531 of 64
 // 137 -> 141, 101 -> 100.  (An arrival per warp instead of per thread: 0 to +1 %.  The LSE of the next tile read under this
-// one's dS phase: +8 to +13 %, spills.  The LSE read next to its use: +4 to +8 %.)
+// one's dS phase: +8 to +13 %, spills.  The LSE read next to its use: +4 to +8 %.)  dK/dV with soft cap spills 60 (head_dim 64) and 84 bytes a
+// thread, the other variants up to 12.
 __host__ __device__ constexpr int ew_groups(Feat f) { return f == Feat::kNone ? 2 : 4; }
 constexpr int kSched = 4;      // depth of the in-CTA ring of work-queue entries
 template <int D> struct BCfg {
@@ -430,7 +431,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   constexpr int SQ = C::kStagesQ, SO = C::kStagesO;
   using R = Roles<ew_groups(kFeat)>;
   constexpr int kEwCols = R::kCols;              // columns per element-wise thread
-  constexpr int kConsumers = R::kEwWarps + 3;   // warps that read the work queue: 8 element-wise, issuer, statistics, store agent
+  constexpr int kConsumers = R::kEwWarps + 3;   // warps that read the work queue: every element-wise one, issuer, statistics, store agent
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -789,10 +790,10 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   } else {
     // ------------------------------- element-wise groups --------------------------------
     reg_alloc<R::kRegsEw>();
-    const int x = warp >> 2;                         // column half
+    const int x = warp >> 2;                         // group: columns x * kEwCols and on
     const int lrow = (warp & 3) * 32 + lane;         // TMEM lane = key inside the tile
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    // this group's 64 columns; the 16-bit pairs of P, of dS take the first 32 of them
+    // this group's kEwCols columns; the 16-bit pairs of P, of dS take the first half of them
     const uint32_t tSg = tS + lane_addr + x * kEwCols, tdPx = tdP + lane_addr + x * kEwCols;
     bool ok = true;
     int pos = 0, wi = 0, sidx = 0;
@@ -808,7 +809,7 @@ bwd_dkdv_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       have = false;
       if (!ok || w.total < 0) break;
       const int key = w.n0 + lrow;
-      // each group stores half of the head_dim columns of dV and of dK * softmax_scale
+      // each group stores its part of the head_dim columns of dV and of dK * softmax_scale
       constexpr int DH = D * kEwCols / kT;
       auto row_of = [&](void* base, const int64_t* stride) -> T* {     // this thread's part of its key's row
         if (key >= w.g.k_len) return nullptr;
@@ -1082,7 +1083,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   constexpr int SK = C::kStagesK, SV = C::kStagesV;
   using R = Roles<ew_groups(kFeat)>;
   constexpr int kEwCols = R::kCols;              // columns per element-wise thread
-  constexpr int kConsumers = R::kEwWarps + 1;    // warps that read the work queue: 8 element-wise and the issuer
+  constexpr int kConsumers = R::kEwWarps + 1;    // warps that read the work queue: every element-wise one and the issuer
   extern __shared__ unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
@@ -1269,7 +1270,7 @@ bwd_dq_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int lrow = (warp & 3) * 32 + lane;  // TMEM lane = query row inside the tile
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t tdPx = tdP + lane_addr + x * kEwCols;
-    constexpr int DH = D * kEwCols / kT;                 // each group stores half of the head_dim columns
+    constexpr int DH = D * kEwCols / kT;                 // each group stores its part of the head_dim columns
     bool ok = true;
     int posA = 0, wi = 0, tg = 0, sidx = 0;
     // statistics of this thread's row: base-2 LSE (+inf for rows that do not exist or see no

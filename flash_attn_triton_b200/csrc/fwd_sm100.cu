@@ -865,8 +865,9 @@ static OneTile one_tile_is_faster(const fa_attn_args& a, const ScoreCfg& cfg) {
 // Calls for the kernel with two persistent CTAs per SM (fwd_duo_sm100.cu).  Measured against the rule without it on 1820 random calls of
 // 8 to 32 heads, 1 to 64 sequences of 64 to 8191 tokens, dense and packed:
 //   up to 2.5 CTAs per SM        -20 to +70 %: the other kernels spread fewer tiles better
-//   where the two-tile kernel is the alternative (below the persistent one's lengths; dropout)    -16 % on average, -46 to +6 %; beyond
-//                                that +7 to +26 % on a few packed causal calls of 2.5 to 6 CTAs per SM (before they had packed_by_weight())
+//   where the two-tile kernel is the alternative (below the persistent one's lengths; dropout)    -16 % on average, -46 to +6 %; packed causal
+//                                calls of 2.5 to 6 CTAs per SM, with packed_by_weight(), -16 % (head_dim 64: -31 to -5) and -12 % (128: -26 to
+//                                +8; three of 64 calls above +3, with ALiBi or soft cap)
 //   where the persistent kernel is
 //     head_dim 64                plain and ALiBi -4 to -19 %, without a mask (part of the exponentials on the FMA pipe there) not taken;
 //                                windows -9 to -32 %; soft cap, causal -2 to -18 % (packed 0 %), no mask, more than 24 tiles +4 %
