@@ -29,7 +29,7 @@
 //
 // What bounds it: at head_dim 64 the exponentials, which the two CTAs contend for (1.8 k of 3.5 k cycles per tile and CTA, 1.02 k alone);
 // at head_dim 128 the chain P V, Q K, load, maximum, exponentials (1.1 k of 4.5 k are spent waiting for the scores).
-// Spills of the plain variants and those with options 60 to 84 bytes of stores a thread, of INT8 180 (what the compiler prints; it allots 128 registers).
+// Spills of the plain variants and those with options 72 to 96 bytes of stores a thread, of INT8 192 (what the compiler prints; it allots 128 registers).
 // Tried: two threads per row (256 softmax threads of 104 registers, maxima and sums exchanged through shared memory), +2 to +15 %.
 //
 // TMEM (256 columns): S (128) | O (head_dim) | P of its own (64).  Every mbarrier wait is bounded.
@@ -263,7 +263,7 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     // (One copy of each part: what a CTA executes first it waits for, and where other kernels have run in between 40 KB more of
     // code were 5 k cycles at the start of a launch.)
     int fidx = 0, pos = 0, qi = 0;
-    int c = blockIdx.x;
+    int c = blockIdx.x;                                // the candidate looked at last, an item or not
     bool ok = true;
     auto wwait = [&](uint64_t* bar, uint32_t parity, int code) {
       if (ok) ok = wait_bar(bar, parity, sh, code);
@@ -273,7 +273,14 @@ fwd_duo_sm100_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_const
     while (ok) {
       if (i + 1 >= 2 * nt) {
         Item w;
-        if (!queue_item(queue, ncand, fidx == 0, c, lane, [&](int u) { return item_of(p, cfg, by_weight, u, lane, w); })) w.nt = -1;
+        for (bool drawn = fidx > 0;; drawn = true) {
+          if (drawn) c = queue_next(queue, ncand, c, lane);
+          if ((unsigned int)c >= (unsigned int)ncand) {
+            w.nt = -1;
+            break;
+          }
+          if (item_of(p, cfg, by_weight, c, lane, w)) break;
+        }
         if (fidx == 0) {
           __syncthreads();                             // barriers are set up
           reg_dealloc<kRegsService>();

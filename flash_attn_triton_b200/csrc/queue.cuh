@@ -10,20 +10,11 @@ __device__ __forceinline__ unsigned int queue_draw(unsigned int* counter, int nc
   return ncand <= (int)gridDim.x ? (unsigned int)ncand : gridDim.x + atomicAdd(&counter[0], 1u);
 }
 
-// The CTA's next item, for a whole warp: candidates are drawn until `decode` takes one; false behind the last.  c is the candidate looked at
-// last, at first the CTA's index: it stays with the caller between items, whatever became of the candidate.
+// The candidate behind c, the one that this CTA looked at last whatever became of it, for a whole warp; ncand or more: there is none.
 // counter null: no queue, CTA i takes i, i + gridDim.x, i + 2 gridDim.x, ...
-template <typename F>
-__device__ __forceinline__ bool queue_item(unsigned int* counter, int ncand, bool first, int& c, int lane, F decode) {
-  for (bool drawn = !first;; drawn = true) {
-    if (drawn) {
-      unsigned int u = 0;
-      if (lane == 0) u = counter == nullptr ? gridDim.x + c : queue_draw(counter, ncand);
-      c = (int)min(__shfl_sync(0xffffffffu, u, 0), (unsigned int)ncand);
-    }
-    if (c >= ncand) return false;
-    if (decode(c)) return true;
-  }
+__device__ __forceinline__ int queue_next(unsigned int* counter, int ncand, int c, int lane) {
+  if (counter == nullptr) return c + gridDim.x;
+  return (int)__shfl_sync(0xffffffffu, lane == 0 ? queue_draw(counter, ncand) : 0u, 0);
 }
 // One thread of a CTA that has drawn its last candidate (or has given up on a wait and draws no more).
 __device__ __forceinline__ void queue_finish(unsigned int* counter, int ncand) {

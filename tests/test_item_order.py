@@ -1,8 +1,9 @@
-"""Items of the kernels that take them by number (csrc/items.cuh, csrc/queue.cuh), compiled for the CPU with the lanes of a warp in turn:
-every tile of rows is worked on once, whatever the lengths, the order and the way in which the CTAs get their candidates."""
+"""Items of the kernel that takes them by number (csrc/items.cuh, csrc/queue.cuh and the draw in csrc/fwd_duo_sm100.cu), compiled for the CPU with the
+lanes of a warp in turn: every tile of rows is worked on once, whatever the lengths, the order and the way in which the CTAs get their candidates."""
 import ctypes as C
 import os
 import random
+import re
 import subprocess
 
 import numpy as np
@@ -53,13 +54,25 @@ static ScoreCfg g_cfg;
 static int g_by_weight, g_ncand, g_h[32], g_b[32], g_mt[32];
 static unsigned* g_counter;
 static int g_last[32];
-static bool g_first, g_found[32];
+static bool g_found[32];
+static int g_fidx;
+struct Item { int nt; };
 static void lane_main() {
-  const int lane = current;
-  SeqInfo si;
-  g_found[lane] = queue_item(g_counter, g_ncand, g_first, g_last[lane], lane, [&](int c) {
-    return item_tile<128>(*g_a, g_cfg, g_by_weight, c, lane, g_h[lane], g_b[lane], si, g_mt[lane]);
-  });
+  const int lane = current, fidx = g_fidx, ncand = g_ncand, by_weight = g_by_weight;
+  unsigned* const queue = g_counter;
+  const fa_attn_args& p = *g_a;
+  const ScoreCfg& cfg = g_cfg;
+  auto item_of = [](const fa_attn_args& p, const ScoreCfg& cfg, int by_weight, int c, int lane, Item& w) {
+    SeqInfo si;
+    w.nt = 1;
+    return item_tile<128>(p, cfg, by_weight, c, lane, g_h[lane], g_b[lane], si, g_mt[lane]);
+  };
+  int c = g_last[lane];
+  Item w;
+  // from fwd_duo_sm100.cu
+  DRAW
+  g_last[lane] = c;
+  g_found[lane] = w.nt >= 0;
   ++done;
 }
 static void run_warp() {
@@ -95,8 +108,8 @@ int next_item(int grid, int cta, unsigned* counter, int* last, int* h, int* b, i
   gridDim.x = grid;
   blockIdx.x = cta;
   g_counter = counter;
-  g_first = *last < 0;
-  for (int i = 0; i < 32; ++i) g_last[i] = g_first ? cta : *last;
+  g_fidx = *last < 0 ? 0 : 1;
+  for (int i = 0; i < 32; ++i) g_last[i] = g_fidx == 0 ? cta : *last;
   run_warp();
   for (int i = 1; i < 32; ++i)
     if (g_found[i] != g_found[0] || g_last[i] != g_last[0] || (g_found[0] && (g_h[i] != g_h[0] || g_b[i] != g_b[0] || g_mt[i] != g_mt[0]))) abort();
@@ -112,7 +125,9 @@ void finish(int grid, int cta, unsigned* counter) { gridDim.x = grid; blockIdx.x
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
     d = tmp_path_factory.mktemp("items")
-    (d / "items.cpp").write_text(SOURCE)
+    kernel = open(os.path.join(CSRC, "fwd_duo_sm100.cu")).read()
+    draw = re.search(r"int c = blockIdx.x;.*?Item w;\n(.*?)\n        if \(fidx == 0\)", kernel, re.S).group(1)
+    (d / "items.cpp").write_text(SOURCE.replace("DRAW", draw))
     subprocess.run([os.environ.get("CXX", "g++"), "-O1", "-std=c++17", "-fPIC", "-shared", "-I" + CSRC, "-I" + os.path.join(ROOT, "include"),
                     str(d / "items.cpp"), "-o", str(d / "items.so")], check=True)
     return C.CDLL(str(d / "items.so"))
